@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <vector>
 
 #include "ecp_ff.h"
 
@@ -74,6 +75,8 @@ struct DevJob {
   const double *besT, *besC;
   const double *besH;          // Taylor coefficients [i][l <= besHL][6] (batched path)
   const double *besA;          // large-argument polynomial [l][i], stride max(besHL + 1, 6)
+  const long long *besX;       // besH as fixed-point rows [i][l <= besHL][8] (ecp_fixed.h)
+  const long long *besXA;      // besA likewise, [l <= besHL][16]
   // the level schedules' slot tables in global memory as well, for reads
   // whose index differs across a warp (the __constant__ copies serialise those)
   const int *s93, *s92;
@@ -100,33 +103,66 @@ struct DevJob {
   int *status;
   double *mat;
   int *errWord;          // [0] first unit with a warning (atomicMin), [1] input error flags
-  // batched path: work queue and tuning
-  const int *order;              // units by descending estimated cost (null: natural order)
-  const int *orderClass;         // units grouped by (la, lb, L) class, by cost within a class
-  unsigned long long *queueHead; // next queue position (persistent launch); reset per run
-  int gcap;                      // type-1 step-table width cap (doubles per slot per warp)
-  int maxNP;                     // most primitive pairs of a shell pair (shared-memory sizing)
-  int mixed;                     // 1: the fallbacks' tables and sums in double-single (ecp_ff.h)
-  int balance;                   // 1: type-1 groups narrowed so that every warp gets pairs
-  int ctaUnits;                  // >0: a persistent CTA takes at most this many units, then exits
+  // batched path: the plan's orders (pairs; centres by descending L), scratch
+  // between the stages, work lists and their counters (ecp_fast.cu)
+  const int *pairOrders;          // [3][nPairs], by FastConfig::sorted
+  const long long *scrOffs;       // [3][nPairs + 1] scratch bytes before a pair's units
+  const int *chunkPairs;          // first sorted pair of every chunk, order after order
+  const int *ctrOrder;
+  const struct JobPlan *plan;     // host side
+  char *scr;
+  unsigned *counters;
+  // the launch's order and chunk
+  const int *pairOrder, *chunkPair;
+  const long long *scrOff;
+  int chunk, nChunks, chunk0, chunk1;  // queue positions [chunk0, chunk1)
+  long long scrBase;
+  int2 *listT1, *listT2, *listPart;
+  struct T1Fail *listFail;
+  int take;                      // work-list entries a warp takes before it exits
+  int gcap;                      // type-1 step-table width cap (doubles per slot)
+  int balance;                   // 1: narrower type-1 groups for units with few primitive pairs
   // per-(la, lb)-class type-1 settings (index la * (maxLBS + 1) + lb):
   // 0 = the job's gcap and balance, else kClassSet | gcap | balance << 12
   int classCfg[kMaxClasses];
-  unsigned long long *classCycles;  // non-null: clock cycles of each class's units (autotuner)
-  // screening stage (batched path): the queue of units that compute blocks
-  int *live;                     // live units in queue order (null: no screening stage)
-  unsigned long long *liveCount; // their number
+  unsigned long long *classCycles;  // non-null: clock cycles of each class's type-1 groups (autotuner)
+  // screening stage: the queue positions of the units that compute blocks
+  int *live;                     // in queue order (null: no screening stage)
+  int *liveStart;                // per chunk, where its live units start; then their total
   int *screenBlocks;             // per-CTA counts, then offsets, of the screening kernels
+};
+
+// What a shell pair's units take: scratch and work-list bytes of one unit,
+// and its largest numbers of work-list entries.
+struct PairPlan {
+  long long scratch, lists;
+  int groups, batches, parts;
+};
+PairPlan pair_plan(int NP, int la, int lb, int nItems);
+
+// A batched job's queue orders, cut into chunks of consecutive sorted pairs
+// whose units' scratch fits the scratch buffer.
+struct JobPlan {
+  struct Chunk {
+    int p0, p1;                // sorted pairs
+    long long base, scratch;   // scratch offset of p0, bytes of the chunk's units
+    long long groups, batches, parts;
+  };
+  struct Order {
+    std::vector<Chunk> chunks;
+    int chunkAt;               // position of the order in DevJob::chunkPairs
+  } order[3];
+  size_t bytes = 0;            // scratch buffer, work lists included
 };
 
 // Launch configuration of the batched path (picked by the autotuner).
 struct FastConfig {
-  int queue = 1;   // 1: persistent CTAs pulling units from the work queue; 0: a CTA per unit
-  int sorted = 1;  // 1: units by descending estimated cost; 2: class-major; 0: the reference's order
+  int queue = 1;   // 1: the units that compute blocks (with screen); 0: every unit
+  int sorted = 1;  // pairs 1: by descending estimated cost; 2: class-major; 0: the reference's order
   int gcap = 45;   // type-1 step-table width cap; smaller caps fit more CTAs per SM
   int mixed = 0;   // set from the job's mode (ECPGB_MIXED), not tuned
   int balance = 1; // narrower type-1 groups when a unit has few primitive pairs
-  int screen = 1;  // with the queue launch: a screening stage compacts the queue to live units
+  int screen = 1;  // with queue: a screening stage compacts the queue to live units
   // per-(la, lb)-class type-1 cap and balance (DevJob::classCfg); the launch's
   // shared memory is sized by gcap, so a class's cap is at most gcap
   int cls[kMaxClasses] = {};
@@ -212,22 +248,24 @@ int launch_fp64_pipeline(const DevJob &job, cudaStream_t stream, size_t smemByte
 void launch_prologue(const DevJob &job, cudaStream_t stream, bool withF);
 void launch_epilogue(const DevJob &job, cudaStream_t stream);
 
-// Batched path (ecp_fast.cu): same prologue/epilogue, warp-per-primitive-pair
-// unit kernel with level-granular tabulation, Horner-form Bessel rows and a
-// table-driven exp.  Its level schedules are this unit's own __constant__
-// copies.
+// The first three of those kernels and the run's first warning word in one launch.
+void launch_stage1(const DevJob &job, cudaStream_t stream);
+
+// Batched path (ecp_fast.cu): the units in four stages over work lists
+// (plan, small grid, large grid, blocks).  Its level schedules are that file's
+// own __constant__ copies.
 int upload_schedules_fast(const int *s93slot, int s93n, const int *s93lvEnd, const int *s93lvJ,
                           const int *s93lvN, int s93levels, const int *s92slot, int s92n,
                           const int *s92lvEnd, const int *s92lvN, int s92levels, void *stream);
-size_t fast_smem_bytes(int LB, int LE, int gcap, int maxNP);
-// CTAs of the batched unit kernel resident per SM at smemBytes.
-int fast_ctas_per_sm(size_t smemBytes, int queue);
+// Shared memory of the small-grid stage, and its CTAs (one warp) per SM.
+size_t fast_smem_bytes(int LB, int gcap);
+int fast_ctas_per_sm(size_t smemBytes);
 // Sets the batched kernels' function attributes on the current device (call
 // before any graph capture).
 void fast_prepare();
-// Resets the per-run words (warning word, queue head).
+// Resets the per-run words (first warning, input errors).
 void launch_reset(const DevJob &job, cudaStream_t stream);
-int launch_fast_pipeline(const DevJob &job, cudaStream_t stream, size_t smemBytes, const FastConfig &cfg,
-                         cudaEvent_t u0, cudaEvent_t u1);
+int launch_fast_pipeline(const DevJob &job, cudaStream_t stream, const FastConfig &cfg, cudaEvent_t u0,
+                         cudaEvent_t u1);
 
 }  // namespace ecpgb

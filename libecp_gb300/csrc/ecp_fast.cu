@@ -28,16 +28,14 @@
 //     exactly the terms the reference adds to each chi[i][j];
 //   * the precision mode a template parameter: the FP64 kernels carry no
 //     mixed-precision code (instruction fetch is one of the kernel's stalls).
+#include <algorithm>
+
 #include "ecp_device.cuh"
 #include "ecp_fastmath.h"
+#include "ecp_fixed.h"
 
 namespace ecpgb {
 
-constexpr int kWarps = kUnitThreads / 32;
-// CTAs per SM the unit kernels are compiled for (168 registers a thread):
-// with the target stated, the register allocator keeps the spills to a few
-// bytes (without it: 168 registers and 0.8 KB of spill traffic a thread)
-constexpr int kUnitCtasPerSm = 3;
 constexpr int kWalkCap = 128;  // large-grid quadratures per warp and pass
 constexpr int kLargeWords = (kMaxLargeOrder + 1) / 32;  // bitmap words over the large grid (128, even)
 static_assert(kLargeWords * 32 >= kMaxLargeOrder && kLargeWords % 2 == 0, "large-grid bitmap size");
@@ -45,12 +43,6 @@ static_assert(kLargeWords * 32 >= kMaxLargeOrder && kLargeWords % 2 == 0, "large
 
 // --------------------------------------------------------------- helpers
 
-// K_0..K_lmax(z): the branches of src/bessel.c:102-199.  The Taylor branch
-// (z < 16) and the large-argument branch are both one Horner pass per row, in
-// dz over the row's Taylor coefficients or in -1/(2z) over the row's
-// large-argument polynomial, so that lanes on either branch run the same
-// instructions: row l is a polynomial of degree max(5, l) whose coefficients
-// above the branch's own degree are zero.
 // K_0..K_lmax(z) for z < 1e-7: the reference's zeroth-order branch,
 // K_l = (1 - z) z^l / (2l+1)!! by its recurrence (src/bessel.c:118-133).
 static __device__ void bessel_small(int lmax, double z, double *K, int stride) {
@@ -63,47 +55,27 @@ static __device__ void bessel_small(int lmax, double z, double *K, int stride) {
   }
 }
 
-template <bool kMixed>
-static __device__ __noinline__ void bessel_fast(const DevJob &J, int lmax, double z, double *K, int stride) {
-  if (__builtin_expect(z < 1.0E-7, 0)) {  // rare: laid out of line
-    bessel_small(lmax, z, K, stride);
-    return;
-  }
-  const bool asy = z >= 16.0;
-  const int HL1 = J.besHL + 1;
-  double x, mult = 1.0;
-  const double *cf;
-  int cs;
-  if (asy) {
-    mult = 0.5 * __drcp_rn(z);  // = 0.5 / z exactly (scaling by 2^-1)
-    x = -mult;
-    cf = J.besA;
-    cs = HL1 < 6 ? 6 : HL1;
-  } else {
-    const double h = J.besselN / 16;  // integer division, as the reference
-    const int index = (int)floor(z * h + 0.5);
-    x = z - __ldg(J.besZ + index);  // index / h, tabulated
-    cf = J.besH + (size_t)index * HL1 * 6;
-    cs = 6;
-  }
-  for (int l = 0; l <= lmax; l++) {
-    const double *q = cf + l * cs;
-    // Horner from the row's top coefficient (degree l on the large-argument
-    // branch above 5, else 5): no multiply of a zero, no scaling by 1
-    int k = asy && l > 5 ? l : 5;
-    double v = q[k];
-    while (k > 5) {
-      k--;
-      v = fma(v, x, q[k]);
-    }
-#pragma unroll
-    for (int j = 4; j >= 0; j--) v = fma(v, x, q[j]);
-    if (asy) v *= mult;
-    K[l * stride] = v;
-  }
+static __device__ __noinline__ void bessel_fx(const DevJob &J, int lmax, xf z100, xf mul, uint32_t sign, double *K) {
+  fx_bessel_rows(J.besX, J.besXA, J.besHL + 1, lmax, z100, mul, sign, K);
 }
 
-// One row K_l(z), by the same branches as bessel_fast.
+// One ECP term d r^n exp(-a r^2) (R2 = r^2): mantissa and sign; a zero of the
+// smallest exponent (it moves no sum) where the exponential underflows.
+static __device__ inline xf ecp_term_fx(const DevJob &J, int t, double r, xf R, xf R2, uint32_t &sign) {
+  const xf a = xf_mul(xf_from(J.termA[t]), R2);
+  const double d = J.termD[t], n = J.termN[t];
+  sign = sign_of(d);
+  const int sh = a.e + 53;  // a r^2 in Q53
+  const u64 E = sh < 0 ? shr64(a.m, -sh) : (a.m >> (63 - (sh > 63 ? 63 : sh)) ? ~0ull : a.m << sh);
+  if (E > (u64)(700ll << 53)) return {0, -100000};
+  xf v = xf_mul(fx_exp(-(i64)E), xf_from(d));
+  if (n == 0.0) return v;
+  if (n == 1.0) return xf_mul(v, R);
+  if (n == 2.0) return xf_mul(v, R2);
+  return xf_mul(v, xf_from(rpow(r, n)));  // other powers: rare
+}
+
+// One row K_l(z), by the same branches as bessel_fx.
 static __device__ __noinline__ double bessel_row(const DevJob &J, int l, double z) {
   if (__builtin_expect(z < 1.0E-7, 0)) {  // rare: laid out of line
     if (z <= 0) return l == 0 ? 1.0 : 0.0;
@@ -135,25 +107,46 @@ static __device__ __noinline__ double bessel_row(const DevJob &J, int l, double 
 }
 
 // U_l(r) of centre c for the channels l set in mask, in one pass over its
-// terms (src/ecp.c:42-60); the other entries of U are left untouched.
-template <bool kMixed>
+// terms (src/ecp.c:42-60); the other entries of U are left untouched.  A
+// channel's terms are summed with 60-bit mantissas; a channel that comes back
+// after another one is added to in FP64.
 static __device__ __noinline__ void channels_masked(const DevJob &J, int c, double r, unsigned mask, double *U) {
-  double r2 = r * r;
   for (unsigned m = mask; m; m &= m - 1) U[__ffs(m) - 1] = 0.0;
-  int t0 = J.ctrT0[c], t1 = t0 + J.ctrNT[c];
-  for (int t = t0; t < t1; t++) {
-    int l = J.termL[t];
-    if (mask >> l & 1u) U[l] += rpow(r, J.termN[t]) * J.termD[t] * fast_exp(-J.termA[t] * r2);
+  const xf R = xf_from(r), R2 = norm1(xf_mul(R, R));
+  const int t0 = J.ctrT0[c], t1 = t0 + J.ctrNT[c];
+  unsigned seen = 0;
+  for (int t = t0; t < t1;) {
+    const int l = J.termL[t];
+    xf_sum acc;
+    const bool use = mask >> l & 1u;
+    for (; t < t1 && J.termL[t] == l; t++)
+      if (use) {
+        uint32_t sg;
+        const xf v = ecp_term_fx(J, t, r, R, R2, sg);
+        acc.add(v, sg);
+      }
+    if (use) {
+      const double v = acc.value();
+      if (seen >> l & 1u) U[l] += v;
+      else U[l] = v;
+      seen |= 1u << l;
+    }
   }
 }
 
-template <bool kMixed>
-static __device__ __noinline__ double channel(const DevJob &J, int c, int l, double r) {
-  double r2 = r * r, pot = 0.0;
-  int t0 = J.ctrT0[c], t1 = t0 + J.ctrNT[c];
+// U_l(r) as a mantissa, exponent and sign.
+static __device__ __noinline__ xf channel(const DevJob &J, int c, int l, double r, uint32_t &sign) {
+  const xf R = xf_from(r), R2 = norm1(xf_mul(R, R));
+  xf_sum acc;
+  const int t0 = J.ctrT0[c], t1 = t0 + J.ctrNT[c];
   for (int t = t0; t < t1; t++)
-    if (J.termL[t] == l) pot += rpow(r, J.termN[t]) * J.termD[t] * fast_exp(-J.termA[t] * r2);
-  return pot;
+    if (J.termL[t] == l) {
+      uint32_t sg;
+      const xf v = ecp_term_fx(J, t, r, R, R2, sg);
+      acc.add(v, sg);
+    }
+  sign = acc.m < 0 ? 0x80000000u : 0u;
+  return {acc.m < 0 ? (u64)-acc.m : (u64)acc.m, acc.e};
 }
 
 // ------------------------------------------- double-single (mixed path)
@@ -540,91 +533,149 @@ __host__ __device__ inline int t1_items(int lab) {
   for (int l1 = 0; l1 <= lab; l1++) n += l1 / 2 + 1;
   return n;
 }
+// Index of quadrature (l1, l2) in that list.
+__host__ __device__ inline int t1_index(int l1, int l2) { return (l1 + 1) * (l1 + 1) / 4 + ((l1 - l2) >> 1); }
 __host__ __device__ inline int t1_group(int lab, int cap) {
   int g = 32 / t1_items(lab);
   g = g > 8 ? 8 : (g < 1 ? 1 : g);
   // the group's step table (33 slots x g entries of 2 (lab+1) + 1 doubles)
-  // stays within 33 x cap doubles (cap 45: three CTAs per SM at l <= 3, L <= 4)
+  // stays within 33 x cap doubles
   while (g > 1 && g * (2 * lab + 3) > cap) g--;
   return g;
 }
 
-struct FastSmem {
-  int chi, J, T, phase, total;
-  // type-1 per warp (inside phase): pair scalars, S_lm, Q, H, step table
-  int w1Stride, w1Sc, w1Rsh, w1Q, w1H, w1Tab;
-  // type-2 fallback per warp (inside phase)
-  int w2Stride, w2Tab, w2I, w2P, w2Q, w2R, w2Part, tab2Stride;
-  int w2Bits, w2Pend, w2Pref;  // fallback streaming: needed-slot bitmap, pending slots, word prefixes
-  int ppMap;                   // type-2 fallback: FM06 map (i1, i2) of every primitive pair
-  int ppWin;                   // and the point-index interval where its exponent can pass the screen
+// The type-2 fallback deals a unit's primitive pairs to warps in parts of
+// consecutive pairs: at least 4 pairs a part (the list of failed quadratures
+// is decoded once per part) and at most 16 parts (each keeps a partial sum
+// per quadrature).
+__host__ __device__ inline int t2_part_pairs(int NP) {
+  const int n = (NP + 15) / 16;
+  return n < 4 ? 4 : n;
+}
+__host__ __device__ inline int t2_parts(int NP) { return (NP + t2_part_pairs(NP) - 1) / t2_part_pairs(NP); }
+
+// Global scratch of one unit between the stages (byte offsets): a header,
+// per primitive pair the FM06 map (i1, i2) and {break index, window}, the
+// type-1 quadratures [pair][t1_index], the type-2 quadratures of the class's
+// items, their partial sums [part][item] when there are several parts, the
+// bitmap of failed items, and the primitive pairs ordered by kind.
+struct UnitHead {
+  u64 est;   // mixed path: largest |estimate| of a failed small-grid item (bits)
+  int warn;  // 1: a type-1, 2: a type-2 quadrature ran out of levels
+  int pad;
+};
+struct UnitScratch {
+  int map, win, Q, T, part, mask, perm, total;
+};
+__host__ __device__ inline UnitScratch unit_scratch(int NP, int lab, int nItems) {
+  UnitScratch s;
+  int o = (int)sizeof(UnitHead);
+  s.map = o; o += 16 * NP;
+  s.win = o; o += 16 * NP;
+  s.Q = o; o += 8 * NP * t1_items(lab);
+  s.T = o; o += 8 * nItems;
+  s.part = o; o += t2_parts(NP) > 1 ? 8 * t2_parts(NP) * nItems : 0;
+  s.mask = o; o += 4 * ((nItems + 31) / 32);
+  s.perm = o; o += NP;
+  s.total = (o + 15) & ~15;
+  return s;
+}
+// Work-list entries a unit can add: type-1 groups (at most one per pair),
+// type-2 small-grid batches, type-2 parts, failed type-1 pairs.
+struct T1Fail {
+  int pos, k;  // queue position, primitive pair (bit 16: double-single tables)
+  unsigned mask;
+};
+__host__ __device__ inline size_t unit_list_bytes(int NP, int nItems) {
+  return 8 * (size_t)NP + 8 * (size_t)((nItems + 31) / 32) + 8 * (size_t)t2_parts(NP) + sizeof(T1Fail) * (size_t)NP;
+}
+
+PairPlan pair_plan(int NP, int la, int lb, int nItems) {
+  PairPlan p;
+  if (la < 0 || lb < 0) NP = nItems = la = lb = 0;
+  p.scratch = unit_scratch(NP, la + lb, nItems).total;
+  p.lists = (long long)unit_list_bytes(NP, nItems);
+  p.groups = NP;
+  p.batches = (nItems + 31) / 32;
+  p.parts = NP ? t2_parts(NP) : 0;
+  return p;
+}
+
+// A normal-kind primitive pair's scalars in fixed point: s = |P| as S 2^-q,
+// Z = za + zb (mantissa and exponent), 100 s.
+struct PairFx {
+  i64 S;
+  u64 Zm, sm;
+  int Ze, se, q;
 };
 
-__host__ __device__ inline FastSmem fast_layout(int LB, int LE, int cap, int maxNP) {
-  FastSmem s{};
+// Shared memory of the stages, in doubles.  Small grid (one warp a CTA): the
+// group's pair scalars and step table.
+struct SmallSmem {
+  int sc, fx, tab, total;
+};
+__host__ __device__ inline SmallSmem small_layout(int LB, int cap) {
+  SmallSmem s;
+  int tt = 0;
+  for (int lab = 0; lab <= 2 * LB; lab++) {
+    const int w = 33 * t1_group(lab, cap) * (2 * lab + 3);
+    if (w > tt) tt = w;
+  }
+  s.sc = 0;
+  s.fx = 24;  // 3 scalars of up to 8 pairs
+  s.tab = s.fx + 8 * (int)(sizeof(PairFx) / sizeof(double));
+  s.total = s.tab + tt;
+  return s;
+}
+// Large grid (one warp a CTA): type 1 a 32-slot table; type 2 a 32-slot table
+// (U[nE], R[nA], Ka[LBE], Kb[LBE]), the walkers' state, the needed-slot bitmap
+// with word prefixes, the pending slots and the failed items.
+struct LargeSmem {
+  int tab, I, P, Q, R, part, bits, pend, pref, fail, total, tabStride;
+};
+__host__ __device__ inline LargeSmem large_layout(int LB, int LE) {
+  LargeSmem s;
+  const int nA = 2 * LB + 1, nE = LE > 0 ? LE : 1, LBE = LB + nE;
+  s.tabStride = (nE + nA + 2 * LBE) | 1;  // odd: conflict-free lane strides
+  int o = 32 * s.tabStride, t1 = 32 * (2 * nA + 3);
+  s.tab = 0;
+  if (t1 > o) o = t1;
+  s.I = o; o += kWalkCap;
+  s.P = o; o += kWalkCap;
+  s.Q = o; o += kWalkCap;
+  s.R = o; o += kWalkCap;
+  s.part = o; o += kWalkCap;
+  s.bits = o; o += kLargeWords / 2;
+  s.pend = o; o += 32;
+  s.pref = o; o += kLargeWords / 2;
+  s.fail = o; o += kWalkCap / 2;
+  s.total = o;
+  return s;
+}
+// Linking: chi / gamma, the half-shifted block, the radial table T, S_lm of a
+// batch of primitive pairs, their sums W and the combined-index block H.
+constexpr int kLinkBatch = 16;
+struct LinkSmem {
+  int chi, J, T, rsh, dir, W, H, total;
+};
+__host__ __device__ inline LinkSmem link_layout(int LB, int LE) {
+  LinkSmem s;
   const int nA = 2 * LB + 1, nE = LE > 0 ? LE : 1, LBE = LB + nE;
   const int nc = (LB + 1) * (LB + 2) * (LB + 3) / 6, nct = (LB + 1) * (LB + 2) / 2;
   const int ncAB = (2 * LB + 1) * (2 * LB + 2) * (2 * LB + 3) / 6;
-  int rq = 0, tt = 0;  // largest per-warp S_lm/Q and step-table widths over lab <= 2 LB
-  for (int lab = 0; lab <= 2 * LB; lab++) {
-    int g = t1_group(lab, cap), lq = lab + 1;
-    if (g * lq * lq > rq) rq = g * lq * lq;
-    // small-grid steps: 33 slots x g entries of 2 lq + 1; fallback steps: 32
-    // slots of 2 lq + 3
-    if (33 * g * (1 + 2 * lq) > tt) tt = 33 * g * (1 + 2 * lq);
-    if (32 * (3 + 2 * lq) > tt) tt = 32 * (3 + 2 * lq);
-  }
   int o = 0;
   s.chi = o; o += nc * nc;
   s.J = o; o += nct * nc;
   s.T = o; o += nE * LBE * LBE * nA;
-  s.phase = o;
-  s.w1Sc = 0;
-  s.w1Rsh = 48;  // pair scalars: 6 per pair, up to 8 pairs
-  s.w1Q = s.w1Rsh + rq;
-  s.w1H = s.w1Q + rq;
-  s.w1Tab = s.w1H + ncAB;
-  s.w1Stride = s.w1Tab + tt;
-  int t1 = kWarps * s.w1Stride;
-  // type 2 fallback: 32-slot table (w, base, vis, U[nE], R[nA], Ka[LBE], Kb[LBE]) + walker state
-  s.tab2Stride = (3 + nE + nA + 2 * LBE) | 1;  // odd: conflict-free lane strides
-  s.w2Tab = 0;
-  s.w2I = 32 * s.tab2Stride;
-  s.w2P = s.w2I + kWalkCap;
-  s.w2Q = s.w2P + kWalkCap;
-  s.w2R = s.w2Q + kWalkCap;
-  s.w2Part = s.w2R + kWalkCap;
-  s.w2Bits = s.w2Part + kWalkCap;            // kLargeWords uint32
-  s.w2Pend = s.w2Bits + kLargeWords / 2;      // 64 int
-  s.w2Pref = s.w2Pend + 32;                   // kLargeWords int
-  s.w2Stride = s.w2Pref + kLargeWords / 2;
-  s.ppMap = kWarps * s.w2Stride;
-  s.ppWin = s.ppMap + 2 * maxNP;  // 2 ints per pair
-  int t2b = s.ppWin + maxNP;
-  int ph = t1;
-  if (t2b > ph) ph = t2b;
-  s.total = s.phase + ph;
+  s.rsh = o; o += kLinkBatch * nA * nA;
+  s.dir = o; o += kLinkBatch * 3;
+  s.W = o; o += ncAB;
+  s.H = o; o += ncAB;
+  s.total = o;
   return s;
 }
 
-size_t fast_smem_bytes(int LB, int LE, int cap, int maxNP) {
-  return sizeof(double) * (size_t)fast_layout(LB, LE, cap, maxNP).total;
-}
-
-struct FastShared {
-  // type-2 fallback: break index per primitive pair; during type 1 the
-  // primitive pairs ordered by kind (normal, band, zero)
-  int ppBreak[kMaxContraction * kMaxContraction];
-  int t1Count[3];
-  int failIdx[kWalkCap];        // the pass's failed items as (l, l1, l2, l3) bytes
-  unsigned failMask[64];
-  int nFail, nThis, nextBase;
-  int t2Next;                   // next small-grid item to hand out
-  unsigned passMask;            // channels read by this pass's failed quadratures
-  int passL1, passL2, passL3;   // highest Ka, Kb and r^l rows they read
-  int warn;
-  unsigned long long estBits;   // mixed path: largest |estimate| of a failed small-grid item (bits)
-};
+size_t fast_smem_bytes(int LB, int gcap) { return sizeof(double) * (size_t)small_layout(LB, gcap).total; }
 
 // Mixed path: the largest quadrature value for which double-single level
 // sums still decide the large-grid convergence test as FP64 does.  The
@@ -633,6 +684,89 @@ struct FastShared {
 // coarsest levels (N = 256) that noise reaches it for integrals near
 // 2^47 tol 48, so quadratures above 1/8 of that take FP64 tables.
 __device__ inline double ff_limit(double tol) { return 0x1p47 * tol * 6.0; }
+
+// A unit as the stages see it: queue position pos = (sorted pair, centre),
+// the pair's shells and derivative shift, the screened window, its scratch.
+struct Unit {
+  int c, pr, sa, sb, A, B, la, lb, lab, lpa, lpb, pa0, pb0, ws, we, Nb, NP, Lc, cls, nItems;
+  const double *gA, *gB, *pzA, *pcA, *pzB, *pcB;
+  char *scr;
+  UnitScratch L;
+  bool live;
+};
+
+// Unit id of queue position pos (pairs in the plan's order, centres innermost).
+static __device__ inline long long unit_at(const DevJob &J, int pos) {
+  const int c = J.ctrOrder[pos % J.nCentres], pr = J.pairOrder[pos / J.nCentres];
+  return (long long)c * J.nPairs + pr;
+}
+
+// Items of the unit's class over the channels below l.
+static __device__ inline int class_items(const DevJob &J, int ncls, int l) {
+  int n = 0;
+  for (int k = 0; k < l; k++) n += J.itemCnt[ncls + k];
+  return n;
+}
+
+static __device__ inline Unit unit_load(const DevJob &J, int pos) {
+  Unit U;
+  const int ps = pos / J.nCentres, ci = pos % J.nCentres;
+  U.c = J.ctrOrder[ci];
+  U.pr = J.pairOrder[ps];
+  U.sa = J.pairA[U.pr];
+  U.sb = J.pairB[U.pr];
+  U.A = J.shAtom[U.sa];
+  U.B = J.shAtom[U.sb];
+  const int *wa = J.win + ((size_t)U.c * J.nShells + U.sa) * 3, *wb = J.win + ((size_t)U.c * J.nShells + U.sb) * 3;
+  // derivative shift: the shells' l moved by (shifta, shiftb) for the
+  // computation, the blocks handed out with l (lpa, lpb)
+  const UnitShift sh = unit_shift(J, U.pr, J.shL[U.sa], J.shL[U.sb], U.A, U.B, J.ctrAtom[U.c]);
+  U.ws = wa[0] > wb[0] ? wa[0] : wb[0];
+  U.we = wa[1] > wb[1] ? wa[1] : wb[1];
+  U.live = !(wa[2] || wb[2] || sh.skip) && U.ws < U.we;
+  U.la = J.shL[U.sa] + sh.a;
+  U.lb = J.shL[U.sb] + sh.b;
+  U.lab = U.la + U.lb;
+  U.lpa = sh.lpa;
+  U.lpb = sh.lpb;
+  U.pa0 = sh.a > 0 ? sh.a : 0;
+  U.pb0 = sh.b > 0 ? sh.b : 0;
+  U.Nb = J.shK[U.sb];
+  U.NP = J.shK[U.sa] * U.Nb;
+  U.Lc = J.ctrL[U.c];
+  if (!U.live) return U;
+  const int LE = J.maxLECP > 0 ? J.maxLECP : 1;
+  U.cls = U.la * (J.maxLBS + 1) + U.lb;
+  U.nItems = class_items(J, U.cls * LE, U.Lc);
+  U.gA = J.cgeo + ((size_t)U.c * J.nAtoms + U.A) * 4;
+  U.gB = J.cgeo + ((size_t)U.c * J.nAtoms + U.B) * 4;
+  U.pzA = J.primA + J.shP[U.sa];
+  U.pcA = J.primD + J.shP[U.sa];
+  U.pzB = J.primA + J.shP[U.sb];
+  U.pcB = J.primD + J.shP[U.sb];
+  U.L = unit_scratch(U.NP, U.lab, class_items(J, U.cls * LE, LE));
+  U.scr = J.scr + (J.scrOff[ps] - J.scrBase) + (size_t)ci * U.L.total;
+  return U;
+}
+
+// The item q of the unit's class as (l, l1, l2, l3), one byte each (all below 16).
+static __device__ inline int unit_item(const DevJob &J, const Unit &U, int q) {
+  const int ncls = U.cls * (J.maxLECP > 0 ? J.maxLECP : 1);
+  int l = 0;
+  while (q >= J.itemCnt[ncls + l]) { q -= J.itemCnt[ncls + l]; l++; }
+  const int v = J.items[J.itemOff[ncls + l] + q];
+  return l | (v & 255) << 8 | ((v >> 8) & 255) << 16 | (v >> 16) << 24;
+}
+
+// Work lists of a chunk and their counters (zeroed before the chunk).
+enum { kCntT1, kCntT2, kCntFail, kCntPart, kHeadSmall, kHeadLarge, kCounters };
+
+// The next entry of a list for a warp; its index to every lane.
+static __device__ inline int next_item(unsigned *head) {
+  int i = 0;
+  if ((threadIdx.x & 31) == 0) i = (int)atomicAdd(head, 1u);
+  return __shfl_sync(0xffffffffu, i, 0);
+}
 
 // --------------------------------------------------------------- type 1
 
@@ -725,213 +859,217 @@ static __device__ void rsh_column(const DevJob &J, int lmax, int m, double x, do
   }
 }
 
-// A group of G primitive pairs (p0 .. p0+G-1) of the type-1 block, by one
-// warp (src/type1.c:95-302); lane = (pair, quadrature).  Adds the group's terms
-// to the warp's per-combined-index accumulators H.
-// The mixed kernel's type-1 large-grid fallback of one primitive pair kk
-// (src/type1.c:149-196) for the lanes whose small-grid quadrature (l1, l2)
-// failed (`fail`), out of line so that the three pair-kind instances of the
-// group code share one copy of both precisions' tables and walks; est: the
-// lane's last small-grid estimate (the ff_limit guard).  Returns each failed
-// lane's result.
-static __device__ __noinline__ double t1_fallback_mixed(const DevJob &J, double *tab, int c, int Lc, int lab, int kk,
-                                                       double s, bool fail, double est, int l1, int l2, int Nb,
-                                                       const double *pzA, const double *pcA, const double *pzB,
-                                                       const double *pcB, double dAC, double dBC, int ws, int we,
-                                                       int pa0, int pb0, int &warn) {
-  constexpr bool kMixed = true;
-  const int lane = threadIdx.x & 31, lq = lab + 1, O = kSmallOrder, OL = J.largeOrder, TSf = 3 + 2 * lq;
-  const double *uL = J.uL + (size_t)c * O;
-  bool ffp;
-  {
-    const unsigned hi = (unsigned)((unsigned long long)__double_as_longlong(fail ? est : 0.0) >> 32);
-    const unsigned lim = (unsigned)((unsigned long long)__double_as_longlong(ff_limit(J.tol)) >> 32);
-    ffp = __reduce_max_sync(0xffffffffu, hi) < lim;
+// One live entry of the type-1 large-grid tables: K[0..kq] = K_l(s r) and
+// WR[0..rq] = w C2 U_L(r) e^ex r^l; returns whether the entry is not zero.
+static __device__ __noinline__ bool t1_large_entry(const DevJob &J, int c, int Lc, double r, double ex, double w,
+                                                   double C2, double s, int kq, int rq, double *K, double *WR) {
+  const xf R = xf_from(r);
+  uint32_t sign;
+  xf v = channel(J, c, Lc, r, sign);
+  v = xf_mul(xf_mul(fx_exp(fx_q53(ex)), xf_norm(v)),
+             xf_mul(xf_from(C2), xf_from(w)));
+  if (v.m == 0) return false;
+  sign ^= sign_of(C2) ^ sign_of(w);
+  bessel_fx(J, kq, xf_mul(xf_times100(xf_from(s)), R), {0, 0}, 0, K);
+  WR[0] = xf_to_double(v.m, v.e, sign);
+  for (int l = 1; l <= rq; l++) {
+    v = norm1(xf_mul(v, R));
+    WR[l] = xf_to_double(v.m, v.e, sign);
   }
-  const double za = pzA[kk / Nb], ca = zeta_times(pcA[kk / Nb], za, pa0), zb = pzB[kk % Nb],
-               cb = zeta_times(pcB[kk % Nb], zb, pb0);
-  const double z = -za - zb, zd2 = -za * dAC * dAC - zb * dBC * dBC;
-  const double C2 = ca * cb;
-  const ff C2f = ff_from_double(C2), sf = ff_from_double(s);
-  double i1, i2;
-  fm06(za, zb, dAC, dBC, i1, i2);
-  const ff i1f = ff_from_double(i1);
-  // first point past both centres whose exponent is below the screen
-  // (src/type1.c:168-176).  Past both centres the exponent falls as r
-  // grows, so the predicate is monotone in the index: a 32-way search,
-  // first over the last points of 32 chunks, then inside the first chunk
-  // whose last point qualifies.
-  auto brk = [&](int n) {
-    const double r = i1 * J.xLarge[n] + i2, e = (z * r + s) * r + zd2;
-    return r > dAC && r > dBC && e < J.lnAcc1;
-  };
-  const int chunk = (OL + 31) / 32;
-  int nb = OL;
-  {
-    const int n = lane * chunk + chunk - 1 < OL ? lane * chunk + chunk - 1 : OL - 1;
-    const unsigned b = __ballot_sync(0xffffffffu, brk(n));
-    if (b) {
-      const int n0 = (__ffs(b) - 1) * chunk;
-      for (int c0 = n0; c0 < n0 + chunk && c0 < OL; c0 += 32) {
-        const int m = c0 + lane;
-        const unsigned b2 = __ballot_sync(0xffffffffu, m < n0 + chunk && m < OL && brk(m));
-        if (b2) {
-          nb = c0 + __ffs(b2) - 1;
-          break;
-        }
-      }
-    }
-  }
-  const int end = nb - 1;
-  double I2 = 0, p2 = 0, q2 = 0, res2 = 0;
-  bool done2 = !fail;
-  for (int s0 = 0; s0 < OL;) {
-    const int s1 = step_end92(s0) < OL ? step_end92(s0) : OL;
-    // the rows the quadratures still running read
-    const int kq = __reduce_max_sync(0xffffffffu, done2 ? 0 : l2);
-    const int rq = __reduce_max_sync(0xffffffffu, done2 ? 0 : l1);
-    for (int t = s0 + lane; t < s1; t += 32) {
-      int n = __ldg(J.s92 + t);
-      bool upper = t > 0 && ((t - 1) & 1);
-      // entry: K_l rows, then the rows w * C2 U_L e^(..) r^l
-      double *K = tab + (t - s0) * TSf, *WR = K + lq;
-      const double w = J.wLarge[n] * i1;
-      bool any = false;
-      if (n < nb && !(upper && n > end)) {
-        double r = i1 * J.xLarge[n] + i2, ex = (z * r + s) * r + zd2;
-        if (ex >= J.lnAcc1) {
-          if (ffp) {
-            ff *Kf = (ff *)K, *WRf = (ff *)WR;
-            const ff rf = ff_from_double(r);
-            ff v = ff_mul(ff_mul(J.wLf[n], i1f),
-                          ff_mul(C2f, ff_mul(channel_ff(J, c, Lc, rf), ff_exp(ff_from_double(ex)))));
-            any = v.hi != 0.0f;
-            bessel_ff(J, kq, ff_mul(sf, rf), Kf, 1);
-            WRf[0] = v;
-            for (int l = 1; l <= rq; l++) {
-              v = ff_mul(v, rf);
-              WRf[l] = v;
-            }
-          } else {
-            double v = w * (C2 * channel<kMixed>(J, c, Lc, r) * fast_exp(ex));
-            any = v != 0.0;
-            bessel_fast<kMixed>(J, kq, s * r, K, 1);
-            WR[0] = v;
-            for (int l = 1; l <= rq; l++) {
-              v *= r;
-              WR[l] = v;
-            }
-          }
-        }
-      } else if (__builtin_expect(n != nb && !upper && n < O && n >= ws && n < we, 0)) {
-        // beyond the break the reference integrates its small-grid buffers:
-        // exponent and U_L at index n, r^l and K_l at flat offset l*OL + n of
-        // rows written with the small grid's stride
-        double rs = J.xSmall[n], es = (z * rs + s) * rs;
-        if (es >= J.lnAcc1) {
-          const double v = w * (C2 * uL[n] * fast_exp(es));
-          any = v != 0.0;
-          for (int l = 0; l <= lab; l++) {
-            int f = l * OL + n, lr = f / O, nr = f % O;
-            bool ok = lr <= lab && nr >= ws && nr < we;
-            double xr = J.xSmall[nr], pw = 1.0;
-            for (int i = 0; i < lr && ok; i++) pw = xr * pw;
-            WR[l] = ok ? v * pw : 0.0;
-            K[l] = ok ? bessel_row(J, lr, s * xr) : 0.0;
-          }
-          if (ffp)  // the rows as ff, in place (entry l holds row l either way)
-            for (int l = 0; l <= lab; l++) {
-              ((ff *)WR)[l] = ff_from_double(WR[l]);
-              ((ff *)K)[l] = ff_from_double(K[l]);
-            }
-        }
-      }
-      if (!any) {  // zero bits read as 0.0 in FP64 and in ff alike
-        for (int l = 0; l <= kq; l++) K[l] = 0.0;
-        for (int l = 0; l <= rq; l++) WR[l] = 0.0;
-      }
-    }
-    __syncwarp();
-    if (!done2) {
-      auto vis = [&](int t) { return c92_slot[t] <= end; };
-      if (ffp) {
-        auto val = [&](int t) {
-          const ff *e = (const ff *)(tab + (t - s0) * TSf);
-          return ff_mul(e[lq + l1], e[l2]);
-        };
-        psm92_advance_ff(s0, s1, J.tol, val, vis, I2, p2, q2, done2, res2);
-      } else {
-        auto val = [&](int t) {
-          const double *e = tab + (t - s0) * TSf;
-          return e[lq + l1] * e[l2];
-        };
-        psm92_advance(s0, s1, J.tol, val, vis, I2, p2, q2, done2, res2);
-      }
-    }
-    __syncwarp();
-    s0 = s1;
-    if (__all_sync(0xffffffffu, done2)) break;
-  }
-  double out = 0.0;
-  if (fail) {
-    if (!done2) {
-      res2 = 16 * I2 / (3 * (c92_lvN[c92_nLevels - 1] + 1.0));
-      warn = 1;
-    }
-    out = res2;
-  }
-  __syncwarp();
-  return out;
+  return true;
 }
 
+// --------------------------------------------------------- stage 1: the plan
+
+// A unit by one warp: its primitive pairs by kind (kind-major, each kind in
+// pair order), the FM06 map, break index and point window of every pair, its
+// work-list entries; a dead unit is marked skipped.
+constexpr int kPlanThreads = 128;
+__global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
+  const int lane = threadIdx.x & 31;
+  const int idx = blockIdx.x * (kPlanThreads / 32) + (threadIdx.x >> 5);
+  int pos = J.chunk0 + idx;
+  if (J.live) {
+    const int l0 = J.liveStart[J.chunk];
+    if (l0 + idx >= J.liveStart[J.chunk + 1]) return;
+    pos = J.live[l0 + idx];
+  } else if (pos >= J.chunk1) {
+    return;
+  }
+  const Unit U = unit_load(J, pos);
+  if (!U.live) {
+    if (lane == 0) J.status[(size_t)U.c * J.nPairs + U.pr] = kUnitSkipped;
+    return;
+  }
+  const double dAC = U.gA[3], dBC = U.gB[3];
+  const int NP = U.NP, Nb = U.Nb;
+  unsigned char *perm = (unsigned char *)(U.scr + U.L.perm);
+  double2 *map = (double2 *)(U.scr + U.L.map);
+  int4 *win = (int4 *)(U.scr + U.L.win);
+  unsigned *mask = (unsigned *)(U.scr + U.L.mask);
+  for (int w = lane; w < (U.nItems + 31) / 32; w += 32) mask[w] = 0u;
+  if (lane == 0) *(UnitHead *)U.scr = {0ull, 0, 0};
+  int cnt[3] = {0, 0, 0};
+  unsigned kinds = 0;  // the lane's pairs' kinds, 2 bits each (at most 8)
+  for (int k0 = 0, j = 0; k0 < NP; k0 += 32, j++) {
+    const int k = k0 + lane;
+    int kind = 3;
+    if (k < NP) {
+      const double za = U.pzA[k / Nb], zb = U.pzB[k % Nb];
+      const double ca = zeta_times(U.pcA[k / Nb], za, U.pa0), cb = zeta_times(U.pcB[k % Nb], zb, U.pb0);
+      const double C1 = t1_prefactor(za, ca, zb, cb, dAC, dBC);
+      double P[3];
+      for (int i = 0; i < 3; i++) P[i] = 2.0 * (za * U.gA[i] + zb * U.gB[i]);
+      const double s2 = P[0] * P[0] + P[1] * P[1] + P[2] * P[2];
+      kind = C1 == 0.0 ? kPairZero : (fabs(C1) < 0x1p-900 || s2 > 2800.0 * (za + zb)) ? kPairBand : kPairNormal;
+      if (U.nItems > 0) {
+        // break index (bisection: the break predicate is monotone in the
+        // index beyond both centres) and the point-index interval outside
+        // which the pair's exponent stays below the screen by a margin of 1:
+        // the exponent is a parabola in r with its vertex at P, and r grows
+        // with the index
+        double i1, i2;
+        fm06(za, zb, dAC, dBC, i1, i2);
+        auto exq = [&](int n, double &r) {
+          r = i1 * J.xLarge[n] + i2;
+          const double d1 = dAC - r, d2 = dBC - r;
+          return -za * d1 * d1 - zb * d2 * d2;
+        };
+        double r;
+        int lo = 0, hi = J.largeOrder;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          const double e = exq(mid, r);
+          if (r > dAC && r > dBC && e < J.lnAcc2) hi = mid; else lo = mid + 1;
+        }
+        const int brk = lo < J.largeOrder ? lo : INT_MAX;
+        const double thr = J.lnAcc2 - 1.0, V = (za * dAC + zb * dBC) / (za + zb);
+        int a = 0, b = J.largeOrder;
+        while (a < b) {
+          const int mid = (a + b) >> 1;
+          if (i1 * J.xLarge[mid] + i2 >= V) b = mid; else a = mid + 1;
+        }
+        const int nv = a;
+        a = 0;
+        b = nv;
+        while (a < b) {
+          const int mid = (a + b) >> 1;
+          if (exq(mid, r) >= thr) b = mid; else a = mid + 1;
+        }
+        const int nLo = a;
+        a = nv;
+        b = J.largeOrder;
+        while (a < b) {
+          const int mid = (a + b) >> 1;
+          if (exq(mid, r) < thr) b = mid; else a = mid + 1;
+        }
+        map[k] = make_double2(i1, i2);
+        win[k] = make_int4(brk, nLo, a - 1, 0);
+      }
+    }
+    kinds |= (unsigned)kind << (2 * j);
+    for (int kd = 0; kd < 3; kd++) cnt[kd] += __popc(__ballot_sync(0xffffffffu, kind == kd));
+  }
+  int at[3] = {0, cnt[0], cnt[0] + cnt[1]};
+  for (int k0 = 0, j = 0; k0 < NP; k0 += 32, j++) {
+    const int kind = (kinds >> (2 * j)) & 3u;
+    for (int kd = 0; kd < 3; kd++) {
+      const unsigned m = __ballot_sync(0xffffffffu, kind == kd);
+      if (kind == kd) perm[at[kd] + __popc(m & ((1u << lane) - 1u))] = (unsigned char)(k0 + lane);
+      at[kd] += __popc(m);
+    }
+  }
+  // the class's type-1 settings (the autotuner may set them per (la, lb))
+  int gcap = J.gcap, bal = J.balance;
+  if (J.classCfg[U.cls] & kClassSet) {
+    gcap = J.classCfg[U.cls] & 0xfff;
+    bal = (J.classCfg[U.cls] >> 12) & 1;
+  }
+  int G[3], n[3], nGroups = 0;
+  for (int kd = 0; kd < 3; kd++) {
+    G[kd] = t1_group(U.lab, gcap);
+    // balance: a unit with few primitive pairs gives its groups to four warps
+    if (bal) {
+      const int g = (cnt[kd] + 3) / 4;
+      if (g < G[kd]) G[kd] = g > 0 ? g : 1;
+    }
+    n[kd] = (cnt[kd] + G[kd] - 1) / G[kd];
+    nGroups += n[kd];
+  }
+  const int nBatch = (U.nItems + 31) / 32, nPart = U.nItems > 0 ? t2_parts(NP) : 0;
+  int base = 0;
+  if (lane < 3) base = (int)atomicAdd(J.counters + (lane == 0 ? kCntT1 : lane == 1 ? kCntT2 : kCntPart),
+                                      (unsigned)(lane == 0 ? nGroups : lane == 1 ? nBatch : nPart));
+  const int b1 = __shfl_sync(0xffffffffu, base, 0), b2 = __shfl_sync(0xffffffffu, base, 1),
+            b3 = __shfl_sync(0xffffffffu, base, 2);
+  for (int g = lane; g < nGroups; g += 32) {
+    int kd = 0, gj = g, p0 = 0;
+    while (gj >= n[kd]) { gj -= n[kd]; p0 += cnt[kd]; kd++; }
+    p0 += gj * G[kd];
+    const int left = cnt[kd] - gj * G[kd];
+    J.listT1[b1 + g] = make_int2(pos, p0 | (left < G[kd] ? left : G[kd]) << 10 | kd << 16);
+  }
+  for (int q = lane; q < nBatch; q += 32) J.listT2[b2 + q] = make_int2(pos, 32 * q);
+  for (int q = lane; q < nPart; q += 32) J.listPart[b3 + q] = make_int2(pos, q);
+}
+
+// --------------------------------------------------- stage 2: the small grid
+
+// A group of G primitive pairs of one kind (perm[p0 ..]) of a unit's type-1
+// quadratures on the small grid (src/type1.c:95-148), by one warp; lane =
+// (pair, quadrature).  Converged quadratures are written to the unit's Q, the
+// pairs with a failed one to the fallback list.
 template <bool kMixed, int kKind>
-static __device__ void t1_group_run(const DevJob &J, const FastSmem &L, double *W, int c, int Lc,
-                                    int la, int lb, const int *perm, int p0, int G, int Nb, const double *pzA,
-                                    const double *pcA, const double *pzB, const double *pcB,
-                                    const double *gA, const double *gB, int ws, int we, int pa0, int pb0,
-                                    int &warn) {
-  const int lane = threadIdx.x & 31, lab = la + lb, lq = lab + 1, O = kSmallOrder;
+static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem &L, double *sm, int pos, int p0,
+                                int G) {
+  const int lane = threadIdx.x & 31, lab = U.lab, lq = lab + 1, O = kSmallOrder, Nb = U.Nb, ws = U.ws, we = U.we;
   // odd entry strides: lanes touching neighbouring entries hit distinct banks
-  const int OL = J.largeOrder, TSs = 1 + 2 * lq, TSf = 3 + 2 * lq, RQ = lq * lq, nq = t1_items(lab);
-  double *sc = W + L.w1Sc, *rsh = W + L.w1Rsh, *Q = W + L.w1Q, *H = W + L.w1H, *tab = W + L.w1Tab;
-  const double dAC = gA[3], dBC = gB[3];
-  const double *uL = J.uL + (size_t)c * O;
-  // (1) per pair: k-vector, its spherical coordinates, the prefactor
+  const int TS = 1 + 2 * lq, nq = t1_items(lab);
+  const u64 thr = (u64)(i64)(-J.lnAcc1 * 0x1p53);
+  double *sc = sm + L.sc, *tab = sm + L.tab;
+  PairFx *fx = (PairFx *)(sm + L.fx);
+  const unsigned char *perm = (const unsigned char *)(U.scr + U.L.perm);
+  const double *uL = J.uL + (size_t)U.c * O;
+  // (1) per pair: |P| (as src/util.c:75-106), the prefactor, -za - zb
+  __syncwarp();
   if (lane < G) {
-    int k = perm[p0 + lane];
+    const int k = perm[p0 + lane];
     // derivative blocks: coefficients times zeta^max(0, shift) (src/type1.c:239-246)
-    double za = pzA[k / Nb], ca = zeta_times(pcA[k / Nb], za, pa0), zb = pzB[k % Nb],
-           cb = zeta_times(pcB[k % Nb], zb, pb0);
+    const double za = U.pzA[k / Nb], ca = zeta_times(U.pcA[k / Nb], za, U.pa0), zb = U.pzB[k % Nb],
+                 cb = zeta_times(U.pcB[k % Nb], zb, U.pb0);
     double P[3];
-    for (int i = 0; i < 3; i++) P[i] = 2.0 * (za * gA[i] + zb * gB[i]);
-    sc[lane * 6 + 0] = sqrt(P[0] * P[0] + P[1] * P[1] + P[2] * P[2]);  // |P|, as src/util.c:75-106
-    direction(P, sc[lane * 6 + 1], sc[lane * 6 + 2], sc[lane * 6 + 5]);
-    sc[lane * 6 + 3] = t1_prefactor(za, ca, zb, cb, dAC, dBC);
-    sc[lane * 6 + 4] = -za - zb;
+    for (int i = 0; i < 3; i++) P[i] = 2.0 * (za * U.gA[i] + zb * U.gB[i]);
+    const double s = sqrt(P[0] * P[0] + P[1] * P[1] + P[2] * P[2]);
+    sc[lane * 3 + 0] = s;
+    sc[lane * 3 + 1] = t1_prefactor(za, ca, zb, cb, U.gA[3], U.gB[3]);
+    sc[lane * 3 + 2] = -za - zb;
+    if (kKind == kPairNormal) {
+      // s and Z r (r inside the window) as integers times 2^q, both below 2^62
+      const xf S = xf_from(s), Z = xf_from(za + zb), s100 = xf_times100(S);
+      const int zr = Z.e + xf_from(J.xSmall[we - 1]).e + 64, q = -3 - (S.e > zr ? S.e : zr);
+      fx[lane] = {(i64)shr64(S.m, -(S.e + q)), Z.m, s100.m, Z.e, s100.e, q};
+    }
   }
   __syncwarp();
-  // (2) S_lm of every pair, one (pair, m) column per lane
-  if (lane < G * lq) {
-    int g = lane / lq, m = lane % lq;
-    rsh_column(J, lab, m, sc[g * 6 + 1], sc[g * 6 + 2], sc[g * 6 + 5], rsh + g * RQ);
-  }
-  for (int e = lane; e < G * RQ; e += 32) Q[e] = 0.0;
-  __syncwarp();
-  // (3) small grid, PS93: lane = (pair g, quadrature (l1, l2))
+  // (2) PS93: lane = (pair g, quadrature (l1, l2))
   const bool mine = lane < G * nq;
-  const int g = mine ? lane / nq : 0;
+  const int g = mine ? lane / nq : 0, qi = mine ? lane % nq : 0;
   int l1 = 0, l2 = 0;
   {
-    int rem = mine ? lane % nq : 0;
+    int rem = qi;
     while (l1 <= lab && rem >= l1 / 2 + 1) { rem -= l1 / 2 + 1; l1++; }
     l2 = l1 - 2 * rem;
   }
+  double *Qout = (double *)(U.scr + U.L.Q) + (size_t)perm[p0 + g] * nq + qi;
   double I = 0, p = 0, q = 0;
   bool done = !mine;
   int k = 0, cnt = 0;
   if constexpr (kKind == kPairZero) {
-    // converged quadratures add 0 to Q; failed ones go to the fallback
-    if (mine) done = t1_zero_walk(J, sc[g * 6], sc[g * 6 + 4], ws, we);
+    // converged quadratures give 0; failed ones go to the fallback
+    if (mine) {
+      done = t1_zero_walk(J, sc[g * 3], sc[g * 3 + 2], ws, we);
+      if (done) *Qout = 0.0;
+    }
   } else
   for (int s0 = 0; s0 < O;) {
     const int s1 = step_end93(s0) < O ? step_end93(s0) : O;
@@ -968,39 +1106,50 @@ static __device__ void t1_group_run(const DevJob &J, const FastSmem &L, double *
     for (int e = lane; e < nIn * nLive; e += 32) {
       const int i = slot_of(e);
       const int gg = live_pair(e, i), t = __ldg(J.byN93 + s0 + lo + i), n = __ldg(J.s93 + t);
-      double *ent = tab + ((t - s0) * G + gg) * TSs;
-      const double s = sc[gg * 6];
-      double *WR = ent + lq;
+      double *ent = tab + ((t - s0) * G + gg) * TS, *WR = ent + lq;
+      const double s = sc[gg * 3], C1 = sc[gg * 3 + 1];
       if constexpr (kKind == kPairBand) {
         // row l: (C1 r^l) U; the walk multiplies by K, exp(e) and w in turn
-        const double r = J.xSmall[n], e = t1_exponent(sc[gg * 6 + 4], s, r), C1 = sc[gg * 6 + 3];
-        bessel_fast<kMixed>(J, lab, s * r, ent, 1);
+        const double r = J.xSmall[n], ex = t1_exponent(sc[gg * 3 + 2], s, r);
+        bessel_fx(J, lab, xf_mul(xf_times100(xf_from(s)), xf_from(r)), {0, 0}, 0, ent);
         double R = 1.0;
         for (int l = 0; l <= lab; l++) {
           if (l) R = __dmul_rn(r, R);
           WR[l] = __dmul_rn(__dmul_rn(C1, R), uL[n]);
         }
-        ent[2 * lq] = e >= J.lnAcc1 ? fast_exp(e) : 0.0;
+        ent[2 * lq] = ex >= J.lnAcc1 ? fast_exp(ex) : 0.0;
       } else {
-        double r = J.xSmall[n], ex = (sc[gg * 6 + 4] * r + s) * r;
-        ex = ex >= J.lnAcc1 ? fast_exp(ex) : 0.0;
-        const double wB = J.wSmall[n] * (sc[gg * 6 + 3] * uL[n] * ex);
-        bessel_fast<kMixed>(J, lab, s * r, ent, 1);
-        double v = wB;
-        WR[0] = v;
-        for (int l = 1; l <= lab; l++) {
-          v *= r;
-          WR[l] = v;
+        // the table row in integers: e = (s - Z r) r in Q53, then
+        // w C1 U_L exp(e) r^l with 60-bit mantissas
+        const double w = J.wSmall[n], u = uL[n];
+        const xf R = xf_from(J.xSmall[n]);
+        const PairFx F = fx[gg];
+        const u64 zr = shr64(mul_hi(F.Zm, R.m), -(F.Ze + R.e + 64 + F.q));
+        const i64 tt = F.S - (i64)zr;
+        u64 E = mul_hi(tt < 0 ? (u64)-tt : (u64)tt, R.m);
+        const int sh = 117 - F.q + R.e;
+        E = sh <= 0 ? shr64(E, -sh) : (E >> (63 - (sh > 63 ? 63 : sh)) ? ~0ull >> 1 : E << sh);
+        if (tt < 0 && E > thr) {  // below the screen
+          for (int l = 0; l < 2 * lq; l++) ent[l] = 0.0;
+        } else {
+          xf v = xf_mul(xf_mul(fx_exp(tt < 0 ? -(i64)E : (i64)E), xf_from(C1)), xf_mul(xf_from(w), xf_from(u)));
+          const uint32_t sign = sign_of(w) ^ sign_of(u) ^ sign_of(C1);
+          bessel_fx(J, lab, xf_mul({F.sm, F.se}, R), {0, 0}, 0, ent);
+          WR[0] = xf_to_double(v.m, v.e, sign);
+          for (int l = 1; l <= lab; l++) {
+            v = norm1(xf_mul(v, R));
+            WR[l] = xf_to_double(v.m, v.e, sign);
+          }
         }
       }
     }
     for (int e = lane; e < (ns - nIn) * nLive; e += 32) {
       const int i = slot_of(e), t = __ldg(J.byN93 + s0 + (i < lo ? i : i + nIn));
-      double *ent = tab + ((t - s0) * G + live_pair(e, i)) * TSs;
+      double *ent = tab + ((t - s0) * G + live_pair(e, i)) * TS;
       for (int l = 0; l <= 2 * lq; l++) ent[l] = 0.0;
     }
     __syncwarp();
-    auto ent_of = [&](int t) { return tab + ((t - s0) * G + g) * TSs; };
+    auto ent_of = [&](int t) { return tab + ((t - s0) * G + g) * TS; };
     // band kind: w * ((((C1 r^l1) U) K_l2) exp(e)), each product rounded
     auto wf = [&](int t, int n) {
       const double *e = ent_of(t);
@@ -1047,7 +1196,7 @@ static __device__ void t1_group_run(const DevJob &J, const FastSmem &L, double *
           q = (1 - j) * q + j * I;
           if (cnt > 0 && 16 * d < J.tol * (3 * n)) {
             done = true;
-            Q[g * RQ + l1 * lq + l2] += 16 * q / (3 * n);
+            *Qout = 16 * q / (3 * n);
           }
         }
         k++;
@@ -1059,215 +1208,254 @@ static __device__ void t1_group_run(const DevJob &J, const FastSmem &L, double *
     s0 = s1;
     if (__all_sync(0xffffffffu, done)) break;
   }
-  // (4) large-grid fallback, one pair of the group at a time, for the
-  //     quadratures that did not converge (src/type1.c:149-196)
-  const bool failed = mine && !done;
+  // (3) the pairs with a failed quadrature, to the large grid
+  const unsigned fail = __ballot_sync(0xffffffffu, mine && !done);
+  if (!fail) return;
+  // mixed path: double-single tables only where the sums of the pair's failed
+  // quadratures can take the reference's decisions (ff_limit, judged on their
+  // last small-grid estimates, by the high words); larger integrals in FP64
+  unsigned est = 0, lim = 0;
+  if constexpr (kMixed) {
+    est = mine && !done ? (unsigned)((u64)__double_as_longlong(fabs(16 * q / (3 * c93_lvN[c93_nLevels - 1]))) >> 32) : 0u;
+    lim = (unsigned)((u64)__double_as_longlong(ff_limit(J.tol)) >> 32);
+  }
   for (int gg = 0; gg < G; gg++) {
-    const bool fail = failed && g == gg;
-    if (!__ballot_sync(0xffffffffu, fail)) continue;
-    // mixed path: the pair's tables in double-single only where the sums of
-    // its failed quadratures can take the reference's decisions (ff_limit,
-    // judged on their last small-grid estimates); larger integrals in FP64
-    if constexpr (kMixed) {
-      const double est = fail ? fabs(16 * q / (3 * c93_lvN[c93_nLevels - 1])) : 0.0;
-      const double r = t1_fallback_mixed(J, tab, c, Lc, lab, perm[p0 + gg], sc[gg * 6], fail, est, l1, l2, Nb, pzA,
-                                         pcA, pzB, pcB, dAC, dBC, ws, we, pa0, pb0, warn);
-      if (fail) Q[g * RQ + l1 * lq + l2] += r;
-      __syncwarp();
+    const unsigned m = fail >> (gg * nq) & (nq >= 32 ? ~0u : (1u << nq) - 1u);
+    if (!m) continue;
+    int ffp = 0;
+    if constexpr (kMixed) ffp = __reduce_max_sync(0xffffffffu, g == gg ? est : 0u) < lim;
+    if (lane == 0) J.listFail[atomicAdd(J.counters + kCntFail, 1u)] = {pos, perm[p0 + gg] | ffp << 16, m};
+  }
+}
+
+// A batch of 32 type-2 small-grid quadratures (src/type2.c:337-387), one per
+// lane: F tables (derivative runs max(0, shift), src/type2.c:563-564) and the
+// r^k U_l table read through L2, FP64 integrand in every mode.
+template <bool kMixed>
+static __device__ void t2_small(const DevJob &J, const Unit &U, int q0) {
+  const int q = q0 + (threadIdx.x & 31), O = kSmallOrder;
+  if (q >= U.nItems) return;
+  const int nF = J.nF, nk = J.nk, LE = J.maxLECP > 0 ? J.maxLECP : 1, nRuns = J.nRuns > 0 ? J.nRuns : 1;
+  const int v = unit_item(J, U, q), l = v & 255, l1 = (v >> 8) & 255, l2 = (v >> 16) & 255, l3 = v >> 24;
+  const double *Fa = J.F + (((size_t)U.c * J.nShells + U.sa) * nRuns + U.pa0) * O * nF + l1;
+  const double *Fb = J.F + (((size_t)U.c * J.nShells + U.sb) * nRuns + U.pb0) * O * nF + l2;
+  const double *Ut = J.utab + (size_t)U.c * O * LE * nk + l * nk + l3;
+  double res;
+  const bool ok = ps93_walk_fast(J.wSmall, U.ws, U.we, J.tol,
+                                 [&](int n) {
+                                   return __ldg(Fa + n * nF) * __ldg(Fb + n * nF) * __ldg(Ut + (size_t)n * LE * nk);
+                                 },
+                                 res);
+  if (ok) ((double *)(U.scr + U.L.T))[q] = res;
+  else {
+    atomicOr((unsigned *)(U.scr + U.L.mask) + (q >> 5), 1u << (q & 31));
+    if (kMixed) atomicMax(&((UnitHead *)U.scr)->est, (u64)__double_as_longlong(fabs(res)));
+  }
+}
+
+// One warp a CTA; each takes up to J.take entries of the type-1 groups, then
+// of the type-2 batches (one kind of work at a time on the whole GPU).
+template <bool kMixed>
+__global__ void __launch_bounds__(32, 16) k_unit_small(DevJob J) {
+  extern __shared__ double sm[];
+  const SmallSmem L = small_layout(J.maxLBS, J.gcap);
+  const int n1 = (int)J.counters[kCntT1], n = n1 + (int)J.counters[kCntT2];
+  for (int taken = 0; taken < J.take; taken++) {
+    const int i = next_item(J.counters + kHeadSmall);
+    if (i >= n) return;
+    const int2 it = i < n1 ? J.listT1[i] : J.listT2[i - n1];
+    const Unit U = unit_load(J, it.x);
+    if (i >= n1) {
+      t2_small<kMixed>(J, U, it.y);
       continue;
     }
-    constexpr bool ffp = false;
-    const int kk = perm[p0 + gg];
-    const double za = pzA[kk / Nb], ca = zeta_times(pcA[kk / Nb], za, pa0), zb = pzB[kk % Nb],
-                 cb = zeta_times(pcB[kk % Nb], zb, pb0);
-    const double s = sc[gg * 6], z = -za - zb, zd2 = -za * dAC * dAC - zb * dBC * dBC;
-    const double C2 = ca * cb;
-    const ff C2f = ff_from_double(C2), sf = ff_from_double(s);
-    double i1, i2;
-    fm06(za, zb, dAC, dBC, i1, i2);
-    const ff i1f = ff_from_double(i1);
-    // first point past both centres whose exponent is below the screen
-    // (src/type1.c:168-176).  Past both centres the exponent falls as r
-    // grows, so the predicate is monotone in the index: a 32-way search,
-    // first over the last points of 32 chunks, then inside the first chunk
-    // whose last point qualifies.
-    auto brk = [&](int n) {
-      const double r = i1 * J.xLarge[n] + i2, e = (z * r + s) * r + zd2;
-      return r > dAC && r > dBC && e < J.lnAcc1;
-    };
-    const int chunk = (OL + 31) / 32;
-    int nb = OL;
-    {
-      const int n = lane * chunk + chunk - 1 < OL ? lane * chunk + chunk - 1 : OL - 1;
-      const unsigned b = __ballot_sync(0xffffffffu, brk(n));
-      if (b) {
-        const int n0 = (__ffs(b) - 1) * chunk;
-        for (int c0 = n0; c0 < n0 + chunk && c0 < OL; c0 += 32) {
-          const int m = c0 + lane;
-          const unsigned b2 = __ballot_sync(0xffffffffu, m < n0 + chunk && m < OL && brk(m));
-          if (b2) {
-            nb = c0 + __ffs(b2) - 1;
-            break;
-          }
+    const long long t0 = J.classCycles ? clock64() : 0;
+    const int p0 = it.y & 1023, G = (it.y >> 10) & 63, kind = it.y >> 16;
+    if (kind == kPairNormal) t1_small<kMixed, kPairNormal>(J, U, L, sm, it.x, p0, G);
+    else if (kind == kPairBand) t1_small<kMixed, kPairBand>(J, U, L, sm, it.x, p0, G);
+    else t1_small<kMixed, kPairZero>(J, U, L, sm, it.x, p0, G);
+    if (J.classCycles && threadIdx.x == 0) atomicAdd(&J.classCycles[U.cls], (u64)(clock64() - t0));
+  }
+}
+
+// --------------------------------------------------- stage 3: the large grid
+
+// The large-grid quadratures of one primitive pair whose small-grid ones
+// (mask, by t1_index) failed (src/type1.c:149-196), one per lane.
+template <bool kMixed>
+static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int kk, bool ffp, unsigned mask) {
+  const int lane = threadIdx.x & 31, lab = U.lab, lq = lab + 1, O = kSmallOrder, OL = J.largeOrder, TSf = 3 + 2 * lq;
+  const int Nb = U.Nb, ws = U.ws, we = U.we, c = U.c, Lc = U.Lc;
+  const double *uL = J.uL + (size_t)c * O;
+  const double dAC = U.gA[3], dBC = U.gB[3];
+  const bool fail = mask >> lane & 1u;
+  int l1 = 0, l2 = 0;
+  {
+    int rem = lane;
+    while (l1 <= lab && rem >= l1 / 2 + 1) { rem -= l1 / 2 + 1; l1++; }
+    l2 = l1 - 2 * rem;
+  }
+  const double za = U.pzA[kk / Nb], ca = zeta_times(U.pcA[kk / Nb], za, U.pa0), zb = U.pzB[kk % Nb],
+               cb = zeta_times(U.pcB[kk % Nb], zb, U.pb0);
+  double P[3];
+  for (int i = 0; i < 3; i++) P[i] = 2.0 * (za * U.gA[i] + zb * U.gB[i]);
+  const double s = sqrt(P[0] * P[0] + P[1] * P[1] + P[2] * P[2]);
+  const double z = -za - zb, zd2 = -za * dAC * dAC - zb * dBC * dBC;
+  const double C2 = ca * cb;
+  double i1, i2;
+  fm06(za, zb, dAC, dBC, i1, i2);
+  const ff C2f = ff_from_double(C2), sf = ff_from_double(s), i1f = ff_from_double(i1);
+  // first point past both centres whose exponent is below the screen
+  // (src/type1.c:168-176).  Past both centres the exponent falls as r
+  // grows, so the predicate is monotone in the index: a 32-way search,
+  // first over the last points of 32 chunks, then inside the first chunk
+  // whose last point qualifies.
+  auto brk = [&](int n) {
+    const double r = i1 * J.xLarge[n] + i2, e = (z * r + s) * r + zd2;
+    return r > dAC && r > dBC && e < J.lnAcc1;
+  };
+  const int chunk = (OL + 31) / 32;
+  int nb = OL;
+  {
+    const int n = lane * chunk + chunk - 1 < OL ? lane * chunk + chunk - 1 : OL - 1;
+    const unsigned b = __ballot_sync(0xffffffffu, brk(n));
+    if (b) {
+      const int n0 = (__ffs(b) - 1) * chunk;
+      for (int c0 = n0; c0 < n0 + chunk && c0 < OL; c0 += 32) {
+        const int m = c0 + lane;
+        const unsigned b2 = __ballot_sync(0xffffffffu, m < n0 + chunk && m < OL && brk(m));
+        if (b2) {
+          nb = c0 + __ffs(b2) - 1;
+          break;
         }
       }
     }
-    const int end = nb - 1;
-    double I2 = 0, p2 = 0, q2 = 0, res2 = 0;
-    bool done2 = !fail;
-    for (int s0 = 0; s0 < OL;) {
-      const int s1 = step_end92(s0) < OL ? step_end92(s0) : OL;
-      // the rows the quadratures still running read
-      const int kq = __reduce_max_sync(0xffffffffu, done2 ? 0 : l2);
-      const int rq = __reduce_max_sync(0xffffffffu, done2 ? 0 : l1);
-      for (int t = s0 + lane; t < s1; t += 32) {
-        int n = __ldg(J.s92 + t);
-        bool upper = t > 0 && ((t - 1) & 1);
-        // entry: K_l rows, then the rows w * C2 U_L e^(..) r^l
-        double *K = tab + (t - s0) * TSf, *WR = K + lq;
-        const double w = J.wLarge[n] * i1;
-        bool any = false;
-        if (n < nb && !(upper && n > end)) {
-          double r = i1 * J.xLarge[n] + i2, ex = (z * r + s) * r + zd2;
-          if (ex >= J.lnAcc1) {
-            if (ffp) {
-              ff *Kf = (ff *)K, *WRf = (ff *)WR;
-              const ff rf = ff_from_double(r);
-              ff v = ff_mul(ff_mul(J.wLf[n], i1f),
-                            ff_mul(C2f, ff_mul(channel_ff(J, c, Lc, rf), ff_exp(ff_from_double(ex)))));
-              any = v.hi != 0.0f;
-              bessel_ff(J, kq, ff_mul(sf, rf), Kf, 1);
-              WRf[0] = v;
-              for (int l = 1; l <= rq; l++) {
-                v = ff_mul(v, rf);
-                WRf[l] = v;
-              }
-            } else {
-              double v = w * (C2 * channel<kMixed>(J, c, Lc, r) * fast_exp(ex));
-              any = v != 0.0;
-              bessel_fast<kMixed>(J, kq, s * r, K, 1);
-              WR[0] = v;
-              for (int l = 1; l <= rq; l++) {
-                v *= r;
-                WR[l] = v;
-              }
+  }
+  const int end = nb - 1;
+  double I2 = 0, p2 = 0, q2 = 0, res2 = 0;
+  bool done2 = !fail;
+  for (int s0 = 0; s0 < OL;) {
+    const int s1 = step_end92(s0) < OL ? step_end92(s0) : OL;
+    // the rows the quadratures still running read
+    const int kq = __reduce_max_sync(0xffffffffu, done2 ? 0 : l2);
+    const int rq = __reduce_max_sync(0xffffffffu, done2 ? 0 : l1);
+    for (int t = s0 + lane; t < s1; t += 32) {
+      int n = __ldg(J.s92 + t);
+      bool upper = t > 0 && ((t - 1) & 1);
+      // entry: K_l rows, then the rows w * C2 U_L e^(..) r^l
+      double *K = tab + (t - s0) * TSf, *WR = K + lq;
+      const double w = J.wLarge[n] * i1;
+      bool any = false;
+      if (n < nb && !(upper && n > end)) {
+        double r = i1 * J.xLarge[n] + i2, ex = (z * r + s) * r + zd2;
+        if (ex >= J.lnAcc1) {
+          if (kMixed && ffp) {
+            ff *Kf = (ff *)K, *WRf = (ff *)WR;
+            const ff rf = ff_from_double(r);
+            ff v = ff_mul(ff_mul(J.wLf[n], i1f),
+                          ff_mul(C2f, ff_mul(channel_ff(J, c, Lc, rf), ff_exp(ff_from_double(ex)))));
+            any = v.hi != 0.0f;
+            bessel_ff(J, kq, ff_mul(sf, rf), Kf, 1);
+            WRf[0] = v;
+            for (int l = 1; l <= rq; l++) {
+              v = ff_mul(v, rf);
+              WRf[l] = v;
             }
+          } else {
+            any = t1_large_entry(J, c, Lc, r, ex, w, C2, s, kq, rq, K, WR);
           }
-        } else if (__builtin_expect(n != nb && !upper && n < O && n >= ws && n < we, 0)) {
-          // beyond the break the reference integrates its small-grid buffers:
-          // exponent and U_L at index n, r^l and K_l at flat offset l*OL + n of
-          // rows written with the small grid's stride
-          double rs = J.xSmall[n], es = (z * rs + s) * rs;
-          if (es >= J.lnAcc1) {
-            const double v = w * (C2 * uL[n] * fast_exp(es));
-            any = v != 0.0;
+        }
+      } else if (__builtin_expect(n != nb && !upper && n < O && n >= ws && n < we, 0)) {
+        // beyond the break the reference integrates its small-grid buffers:
+        // exponent and U_L at index n, r^l and K_l at flat offset l*OL + n of
+        // rows written with the small grid's stride
+        double rs = J.xSmall[n], es = (z * rs + s) * rs;
+        if (es >= J.lnAcc1) {
+          const double v = w * (C2 * uL[n] * fast_exp(es));
+          any = v != 0.0;
+          for (int l = 0; l <= lab; l++) {
+            int f = l * OL + n, lr = f / O, nr = f % O;
+            bool ok = lr <= lab && nr >= ws && nr < we;
+            double xr = J.xSmall[nr], pw = 1.0;
+            for (int i = 0; i < lr && ok; i++) pw = xr * pw;
+            WR[l] = ok ? v * pw : 0.0;
+            K[l] = ok ? bessel_row(J, lr, s * xr) : 0.0;
+          }
+          if (kMixed && ffp)  // the rows as ff, in place (entry l holds row l either way)
             for (int l = 0; l <= lab; l++) {
-              int f = l * OL + n, lr = f / O, nr = f % O;
-              bool ok = lr <= lab && nr >= ws && nr < we;
-              double xr = J.xSmall[nr], pw = 1.0;
-              for (int i = 0; i < lr && ok; i++) pw = xr * pw;
-              WR[l] = ok ? v * pw : 0.0;
-              K[l] = ok ? bessel_row(J, lr, s * xr) : 0.0;
+              ((ff *)WR)[l] = ff_from_double(WR[l]);
+              ((ff *)K)[l] = ff_from_double(K[l]);
             }
-            if (ffp)  // the rows as ff, in place (entry l holds row l either way)
-              for (int l = 0; l <= lab; l++) {
-                ((ff *)WR)[l] = ff_from_double(WR[l]);
-                ((ff *)K)[l] = ff_from_double(K[l]);
-              }
-          }
-        }
-        if (!any) {  // zero bits read as 0.0 in FP64 and in ff alike
-          for (int l = 0; l <= kq; l++) K[l] = 0.0;
-          for (int l = 0; l <= rq; l++) WR[l] = 0.0;
         }
       }
-      __syncwarp();
-      if (!done2) {
-        auto vis = [&](int t) { return c92_slot[t] <= end; };
-        if (ffp) {
-          auto val = [&](int t) {
-            const ff *e = (const ff *)(tab + (t - s0) * TSf);
-            return ff_mul(e[lq + l1], e[l2]);
-          };
-          psm92_advance_ff(s0, s1, J.tol, val, vis, I2, p2, q2, done2, res2);
-        } else {
-          auto val = [&](int t) {
-            const double *e = tab + (t - s0) * TSf;
-            return e[lq + l1] * e[l2];
-          };
-          psm92_advance(s0, s1, J.tol, val, vis, I2, p2, q2, done2, res2);
-        }
+      if (!any) {  // zero bits read as 0.0 in FP64 and in ff alike
+        for (int l = 0; l <= kq; l++) K[l] = 0.0;
+        for (int l = 0; l <= rq; l++) WR[l] = 0.0;
       }
-      __syncwarp();
-      s0 = s1;
-      if (__all_sync(0xffffffffu, done2)) break;
-    }
-    if (fail) {
-      if (!done2) {
-        res2 = 16 * I2 / (3 * (c92_lvN[c92_nLevels - 1] + 1.0));
-        warn = 1;
-      }
-      Q[g * RQ + l1 * lq + l2] += res2;
     }
     __syncwarp();
-  }
-  __syncwarp();
-  // (5) H[p] += sum_l (sum_m S_lm poly2sph[p][lm]) Q[|p|][l], pair by pair in
-  //     order (src/type1.c:323-345)
-  const int dd = J.tmDim + 1, tmW = (J.tmDim + 1) * (J.tmDim + 1);
-  const int ncab = (lab + 1) * (lab + 2) * (lab + 3) / 6;
-  for (int pi = lane; pi < ncab; pi += 32) {
-    const int *ex = J.ijk + 3 * pi;
-    const int lmax = ex[0] + ex[1] + ex[2];
-    const int prow = J.ijkIdx[(ex[0] * dd + ex[1]) * dd + ex[2]];
-    double acc = H[pi];
-    for (int gg = 0; gg < G; gg++) {
-      const double *rs = rsh + gg * RQ, *Qg = Q + gg * RQ;
-      for (int l = lmax; l >= 0; l -= 2) {
-        double factor = 0.0;
-        for (int m = 0; m < 2 * l + 1; m++) factor += rs[l * l + m] * J.p2s[(size_t)prow * tmW + l * l + m];
-        acc += factor * Qg[lmax * lq + l];
+    if (!done2) {
+      auto vis = [&](int t) { return c92_slot[t] <= end; };
+      if (kMixed && ffp) {
+        auto val = [&](int t) {
+          const ff *e = (const ff *)(tab + (t - s0) * TSf);
+          return ff_mul(e[lq + l1], e[l2]);
+        };
+        psm92_advance_ff(s0, s1, J.tol, val, vis, I2, p2, q2, done2, res2);
+      } else {
+        auto val = [&](int t) {
+          const double *e = tab + (t - s0) * TSf;
+          return e[lq + l1] * e[l2];
+        };
+        psm92_advance(s0, s1, J.tol, val, vis, I2, p2, q2, done2, res2);
       }
     }
-    H[pi] = acc;
+    __syncwarp();
+    s0 = s1;
+    if (__all_sync(0xffffffffu, done2)) break;
+  }
+  if (fail) {
+    if (!done2) {
+      res2 = 16 * I2 / (3 * (c92_lvN[c92_nLevels - 1] + 1.0));
+      atomicOr(&((UnitHead *)U.scr)->warn, 1);
+    }
+    ((double *)(U.scr + U.L.Q))[(size_t)kk * t1_items(lab) + lane] = res2;
   }
   __syncwarp();
 }
 
-// --------------------------------------------------------------- type 2
-
 // One primitive pair of the type-2 large-grid fallback, by one warp
-// (src/type2.c:418-528): integrates the pass's failed items and adds each
-// result to the warp's partial sums.
+// (src/type2.c:418-528): integrates the pass's failed items (decoded in
+// `fail`) and adds each result to the partial sums.  mb: the latest break of
+// the earlier pairs, beyond which no earlier pair's buffers are reused.
+struct T2Pass {
+  int nf;            // failed items of the pass
+  unsigned mask;     // channels they read
+  int l1, l2, l3;    // highest Ka, Kb and r^l rows
+};
 template <bool kMixed>
-static __device__ void t2_pair(const DevJob &J, const FastSmem &L, double *W, const FastShared &S,
-                               int k, int Nb, int nf, int c, int Lc, int la, int lb, const double *pzA,
-                               const double *pcA, const double *pzB, const double *pcB, double dAC,
-                               double dBC, int ncls, int pa0, int pb0, const double *map, const int *win,
-                               bool useFF, int &warn) {
+static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &L, double *sm, const T2Pass &S,
+                               int k, int mb, const double2 *map, const int4 *win, bool useFF, int &warn) {
   // mixed path: useFF picks the double-single tables and sums for this pass
   // (one copy of the common code for both precisions)
   const bool inFF = kMixed && useFF;
-  const int lane = threadIdx.x & 31, nA = 2 * J.maxLBS + 1;
+  const int lane = threadIdx.x & 31, nA = 2 * J.maxLBS + 1, Nb = U.Nb, c = U.c, nf = S.nf;
   const int LE = J.maxLECP > 0 ? J.maxLECP : 1, LBE = J.maxLBS + LE, OL = J.largeOrder;
-  const int TS = L.tab2Stride;
-  double *tab = W + L.w2Tab, *sI = W + L.w2I, *sP = W + L.w2P, *sQ = W + L.w2Q, *sR = W + L.w2R;
-  double *part = W + L.w2Part;
-  unsigned *needBits = (unsigned *)(W + L.w2Bits);
-  int *pend = (int *)(W + L.w2Pend), *pref = (int *)(W + L.w2Pref);
-  const double za = pzA[k / Nb], ca = pcA[k / Nb], zb = pzB[k % Nb], cb = pcB[k % Nb];
+  const int TS = L.tabStride;
+  const double *pzA = U.pzA, *pzB = U.pzB;
+  const double dAC = U.gA[3], dBC = U.gB[3];
+  double *tab = sm + L.tab, *sI = sm + L.I, *sP = sm + L.P, *sQ = sm + L.Q, *sR = sm + L.R, *part = sm + L.part;
+  const int *fail = (const int *)(sm + L.fail);
+  unsigned *needBits = (unsigned *)(sm + L.bits);
+  int *pend = (int *)(sm + L.pend), *pref = (int *)(sm + L.pref);
+  const double za = pzA[k / Nb], ca = U.pcA[k / Nb], zb = pzB[k % Nb], cb = U.pcB[k % Nb];
   // derivative blocks: the product times zeta_a^max(0, shifta), then
   // zeta_b^max(0, shiftb) (src/type2.c:456-462)
-  const double Ck = zeta_times(zeta_times(ca * cb, za, pa0), zb, pb0);
-  const double i1 = map[2 * k], i2 = map[2 * k + 1];
+  const double Ck = zeta_times(zeta_times(ca * cb, za, U.pa0), zb, U.pb0);
+  const double i1 = map[k].x, i2 = map[k].y;
   const ff i1f = ff_from_double(i1), Ckf = ff_from_double(Ck);
-  const int nb = S.ppBreak[k], end = nb == INT_MAX ? OL - 1 : nb - 1;
-  const int nLo = win[2 * k], nHi = win[2 * k + 1];
-  // the latest break of the earlier pairs: beyond it no earlier pair's
-  // buffers are reused
-  int mb = -1;
-  for (int j = lane; j < k; j += 32) mb = S.ppBreak[j] > mb ? S.ppBreak[j] : mb;
-  mb = __reduce_max_sync(0xffffffffu, mb);
+  const int4 wk = win[k];
+  const int nb = wk.x, end = nb == INT_MAX ? OL - 1 : nb - 1, nLo = wk.y, nHi = wk.z;
   for (int q = lane; q < nf; q += 32) { sI[q] = 0; sP[q] = 0; sQ[q] = 0; sR[q] = 0; }
   for (int w = lane; w < (OL + 31) / 32; w += 32) needBits[w] = 0u;
   __syncwarp();
@@ -1281,12 +1469,12 @@ static __device__ void t2_pair(const DevJob &J, const FastSmem &L, double *W, co
     if (n < nb) owner = k;
     else if (__builtin_expect(n != nb && !upper, 0)) {
       for (int j = k - 1; j >= 0; j--)
-        if (S.ppBreak[j] >= n) { owner = j; break; }
-      if (owner >= 0 && S.ppBreak[owner] == n) owner = -1;
+        if (win[j].x >= n) { owner = j; break; }
+      if (owner >= 0 && win[owner].x == n) owner = -1;
     }
     if (owner < 0) return;
     const double zaj = owner == k ? za : pzA[owner / Nb], zbj = owner == k ? zb : pzB[owner % Nb];
-    r = map[2 * owner] * J.xLarge[n] + map[2 * owner + 1];
+    r = map[owner].x * J.xLarge[n] + map[owner].y;
     const double d1 = dAC - r, d2 = dBC - r;
     ex = -zaj * d1 * d1 - zbj * d2 * d2;
   };
@@ -1299,8 +1487,8 @@ static __device__ void t2_pair(const DevJob &J, const FastSmem &L, double *W, co
   int cpos = 0, wpos = 0, nPend = 0;
   // channels and rows the quadratures still running read (the pass's to
   // begin with, narrowed after every walk)
-  unsigned pMask = S.passMask;
-  int pL1 = S.passL1, pL2 = S.passL2, pL3 = S.passL3;
+  unsigned pMask = S.mask;
+  int pL1 = S.l1, pL2 = S.l2, pL3 = S.l3;
   const unsigned below = (1u << lane) - 1u;
   while (wpos < OL) {
     while (nPend < 32 && cpos < OL) {
@@ -1348,10 +1536,10 @@ static __device__ void t2_pair(const DevJob &J, const FastSmem &L, double *W, co
       double *e = tab + lane * TS;
       if (inFF) {
         // the same rows in double-single
-        ff *U = (ff *)(e + 3), *R = U + LE, *Ka = R + nA, *Kb = Ka + LBE;
+        ff *Uc = (ff *)e, *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
         const ff rf = ff_from_double(r);
         const ff wB = ff_mul(ff_mul(J.wLf[n], i1f), ff_mul(Ckf, ff_exp(ff_from_double(ex))));
-        channels_ff(J, c, rf, pMask, U);
+        channels_ff(J, c, rf, pMask, Uc);
 #pragma unroll 1
         for (int side = 0; side < 2; side++)
           bessel_ff(J, side ? pL2 : pL1, ff_mul(ff_from_double(side ? 2.0 * zbj * dBC : 2.0 * zaj * dAC), rf),
@@ -1360,18 +1548,29 @@ static __device__ void t2_pair(const DevJob &J, const FastSmem &L, double *W, co
         R[0] = {1.0f, 0.0f};
         for (int l = 1; l <= pL3; l++) R[l] = ff_mul(rf, R[l - 1]);
       } else {
-        double *U = e + 3, *R = U + LE, *Ka = R + nA, *Kb = Ka + LBE;
+        double *Uc = e, *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
         // Ka rows carry the weight and prefactor: w * Ck * e^(..) * K_l1
-        const double wB = (J.wLarge[n] * i1) * (Ck * fast_exp(ex));
+        const double w = J.wLarge[n];
+        const xf Rx = xf_from(r),
+                 wB = xf_mul(fx_exp(fx_q53(ex)), xf_mul(xf_mul(xf_from(w), xf_from(i1)), xf_from(Ck)));
+        // (a zero prefactor as a zero of the smallest exponent: mul.m = 0 means 1)
+        const xf mul = wB.m ? norm1(wB) : xf{1, -100000};
+        const uint32_t sign = sign_of(w) ^ sign_of(Ck);
         // only the channels and rows this pass's quadratures read
-        channels_masked<kMixed>(J, c, r, pMask, U);
+        channels_masked(J, c, r, pMask, Uc);
         // the rows of both centres through one copy of the Bessel code
 #pragma unroll 1
-        for (int side = 0; side < 2; side++)
-          bessel_fast<kMixed>(J, side ? pL2 : pL1, side ? 2.0 * zbj * dBC * r : 2.0 * zaj * dAC * r, side ? Kb : Ka, 1);
-        for (int l = 0; l <= pL1; l++) Ka[l] *= wB;
+        for (int side = 0; side < 2; side++) {
+          const xf f = xf_mul(xf_from(side ? zbj : zaj), xf_from(side ? dBC : dAC));  // times 2: exponent + 1
+          bessel_fx(J, side ? pL2 : pL1, xf_mul(xf_times100({f.m, f.e + 1}), Rx), side ? xf{0, 0} : mul,
+                    side ? 0u : sign, side ? Kb : Ka);
+        }
         R[0] = 1.0;
-        for (int l = 1; l <= pL3; l++) R[l] = r * R[l - 1];
+        xf p = {1ull << 63, -63};
+        for (int l = 1; l <= pL3; l++) {
+          p = norm1(xf_mul(p, Rx));
+          R[l] = xf_to_double(p.m, p.e, 0);
+        }
       }
     }
     if (lane == 0) {  // entry of slot t: queued slots in [wpos, t)
@@ -1389,7 +1588,7 @@ static __device__ void t2_pair(const DevJob &J, const FastSmem &L, double *W, co
     for (int q = lane, qi = 0; q < nf; q += 32, qi++) {
       if (doneBits[qi] & (1u << lane)) continue;
       // the pass's item, decoded once when the pass was listed
-      const int v = S.failIdx[q], l = v & 255, l1 = (v >> 8) & 255, l2 = (v >> 16) & 255, l3 = v >> 24;
+      const int v = fail[q], l = v & 255, l1 = (v >> 8) & 255, l2 = (v >> 16) & 255, l3 = v >> 24;
       auto entry = [&](int t) {  // a queued slot's table entry
         const unsigned word = needBits[t >> 5], bit = 1u << (t & 31);
         return tab + (pref[t >> 5] + __popc(word & (bit - 1u))) * TS;
@@ -1399,15 +1598,15 @@ static __device__ void t2_pair(const DevJob &J, const FastSmem &L, double *W, co
       bool done = false;
       if (inFF) {
         auto val = [&](int t) {
-          const ff *U = (const ff *)(entry(t) + 3), *R = U + LE, *Ka = R + nA, *Kb = Ka + LBE;
-          return ff_mul(ff_mul(ff_mul(Ka[l1], Kb[l2]), U[l]), R[l3]);
+          const ff *Uc = (const ff *)entry(t), *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
+          return ff_mul(ff_mul(ff_mul(Ka[l1], Kb[l2]), Uc[l]), R[l3]);
         };
         psm92_sparse_ff(wpos, b, needBits, J.tol, val, vis, I, p, qv, done, res);
       } else {
         auto val = [&](int t) {
           const double *e = entry(t);
-          const double *U = e + 3, *R = U + LE, *Ka = R + nA, *Kb = Ka + LBE;
-          return Ka[l1] * Kb[l2] * U[l] * R[l3];
+          const double *Uc = e, *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
+          return Ka[l1] * Kb[l2] * Uc[l] * R[l3];
         };
         psm92_sparse(wpos, b, needBits, J.tol, val, vis, I, p, qv, done, res);
       }
@@ -1444,199 +1643,198 @@ static __device__ void t2_pair(const DevJob &J, const FastSmem &L, double *W, co
   __syncwarp();
 }
 
-// --------------------------------------------------------------- the kernel
-
-// One unit (centre c, shell pair pr) by the whole CTA.  Every thread enters
-// and leaves together (the early exits are CTA-uniform).
+// The failed type-2 quadratures of a unit over the primitive pairs of one part
+// (src/type2.c:418-528), in passes of up to kWalkCap of them.
 template <bool kMixed>
-static __device__ void unit_fast(const DevJob &J, const long long u, FastShared &S, double *sm) {
-  const int c = (int)(u / J.nPairs), pr = (int)(u % J.nPairs);
-  const int sa = J.pairA[pr], sb = J.pairB[pr], tid = threadIdx.x, NT = blockDim.x;
-  const int warp = tid >> 5;
-  const int *wa = J.win + ((size_t)c * J.nShells + sa) * 3;
-  const int *wb = J.win + ((size_t)c * J.nShells + sb) * 3;
-  // derivative shift: the shells' l moved by (shifta, shiftb) for the
-  // computation, the blocks handed out with l (lpa, lpb)
-  const UnitShift sh = unit_shift(J, pr, J.shL[sa], J.shL[sb], J.shAtom[sa], J.shAtom[sb], J.ctrAtom[c]);
-  if (wa[2] || wb[2] || sh.skip) {
-    if (tid == 0) J.status[u] = kUnitSkipped;
-    return;
-  }
-  const int ws = wa[0] > wb[0] ? wa[0] : wb[0];
-  const int we = wa[1] > wb[1] ? wa[1] : wb[1];
-  if (!(ws < we)) {
-    if (tid == 0) J.status[u] = kUnitSkipped;
-    return;
-  }
-  const FastSmem Lm = fast_layout(J.maxLBS, J.maxLECP, J.gcap, J.maxNP);
-  const int A = J.shAtom[sa], B = J.shAtom[sb], la = J.shL[sa] + sh.a, lb = J.shL[sb] + sh.b, lab = la + lb;
-  // the class's type-1 settings (the autotuner may set them per (la, lb))
-  const int cls = la * (J.maxLBS + 1) + lb;
-  int gcapU = J.gcap, balU = J.balance;
-  if (J.classCfg[cls] & kClassSet) {
-    gcapU = J.classCfg[cls] & 0xfff;
-    balU = (J.classCfg[cls] >> 12) & 1;
-  }
-  const long long tc0 = J.classCycles ? clock64() : 0;
-  const int lpa = sh.lpa, lpb = sh.lpb, pa0 = sh.a > 0 ? sh.a : 0, pb0 = sh.b > 0 ? sh.b : 0;
-  const int nA = 2 * J.maxLBS + 1, LE = J.maxLECP > 0 ? J.maxLECP : 1, LBE = J.maxLBS + LE;
-  const int Lc = J.ctrL[c], nca = NCUM(la), ncb = NCUM(lb), O = kSmallOrder;
-  const size_t cA = (size_t)c * J.nAtoms + A, cB = (size_t)c * J.nAtoms + B;
-  const double *gA = J.cgeo + cA * 4, *gB = J.cgeo + cB * 4;
-  const double dAC = gA[3], dBC = gB[3];
-  const double *pzA = J.primA + J.shP[sa], *pcA = J.primD + J.shP[sa];
-  const double *pzB = J.primA + J.shP[sb], *pcB = J.primD + J.shP[sb];
-  const int Na = J.shK[sa], Nb = J.shK[sb], NP = Na * Nb;
-  double *chi = sm + Lm.chi, *Jsh = sm + Lm.J, *T = sm + Lm.T, *ph = sm + Lm.phase;
-  double *out1 = J.out + (size_t)c * J.centreStride + J.pairOff[pr];
-  double *out2 = out1 + NCART(lpa) * NCART(lpb);
-  int warn1 = 0, warn2 = 0;
-  // type-2 small-grid quadratures (src/type2.c:337-387): the items of the
-  // unit's class, their F tables (derivative runs max(0, shift),
-  // src/type2.c:563-564) and r^k U_l table read through L2
-  const int nF = J.nF, nk = J.nk;
-  const int nRuns = J.nRuns > 0 ? J.nRuns : 1;
-  const double *gFa = J.F + (((size_t)c * J.nShells + sa) * nRuns + pa0) * O * nF;
-  const double *gFb = J.F + (((size_t)c * J.nShells + sb) * nRuns + pb0) * O * nF;
-  const double *Ut = J.utab + (size_t)c * O * LE * nk;
-  const int ncls = (la * (J.maxLBS + 1) + lb) * LE;
-  int nItems = 0;
-  for (int l = 0; l < Lc; l++) nItems += J.itemCnt[ncls + l];
-  auto item = [&](int q, int &l, int &l1, int &l2, int &l3) {
-    l = 0;
-    while (q >= J.itemCnt[ncls + l]) { q -= J.itemCnt[ncls + l]; l++; }
-    int v = J.items[J.itemOff[ncls + l] + q];
-    l1 = v & 255; l2 = (v >> 8) & 255; l3 = v >> 16;
-  };
-  auto tidx = [&](int l, int l1, int l2, int l3) { return ((l * LBE + l1) * LBE + l2) * nA + l3; };
-  auto small_item = [&](int q) {
-    int l, l1, l2, l3;
-    item(q, l, l1, l2, l3);
-    double res;
-    // FP64 integrand in every mode: the reference's test
-    const bool ok = ps93_walk_fast(J.wSmall, ws, we, J.tol,
-                                   [&](int n) {
-                                     return __ldg(gFa + n * nF + l1) * __ldg(gFb + n * nF + l2) *
-                                            __ldg(Ut + ((size_t)n * LE + l) * nk + l3);
-                                   },
-                                   res);
-    if (ok) T[tidx(l, l1, l2, l3)] = res;
-    else {
-      atomicOr(&S.failMask[q >> 5], 1u << (q & 31));
-      atomicAdd(&S.nFail, 1);
-      if (kMixed) atomicMax(&S.estBits, (unsigned long long)__double_as_longlong(fabs(res)));
+static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem &L, double *sm, int part) {
+  const int lane = threadIdx.x & 31, nIt = U.nItems, LE = J.maxLECP > 0 ? J.maxLECP : 1;
+  const unsigned *mask = (const unsigned *)(U.scr + U.L.mask);
+  int *fail = (int *)(sm + L.fail);
+  double *sum = sm + L.part;
+  const int pp = t2_part_pairs(U.NP), k0 = part * pp, k1 = k0 + pp < U.NP ? k0 + pp : U.NP;
+  const bool single = t2_parts(U.NP) == 1;
+  // partial sums of the part, or the results themselves when it is the only one
+  double *dst = single ? (double *)(U.scr + U.L.T)
+                       : (double *)(U.scr + U.L.part) + (size_t)part * class_items(J, U.cls * LE, LE);
+  // mixed path: double-single tables only where their sums can take the
+  // reference's decisions (ff_limit); larger integrals in FP64
+  const bool useFF = kMixed && __longlong_as_double((i64)((const UnitHead *)U.scr)->est) < ff_limit(J.tol);
+  const double2 *map = (const double2 *)(U.scr + U.L.map);
+  const int4 *win = (const int4 *)(U.scr + U.L.win);
+  // the latest break of the pairs before the part: beyond it no earlier
+  // pair's buffers are reused
+  int mb0 = -1;
+  for (int j = lane; j < k0; j += 32) mb0 = win[j].x > mb0 ? win[j].x : mb0;
+  mb0 = __reduce_max_sync(0xffffffffu, mb0);
+  int q0 = 0;
+  while (q0 < nIt) {
+    // the pass's items, decoded once
+    int nf = 0;
+    unsigned pMask = 0;
+    int m1 = 0, m2 = 0, m3 = 0;
+    const int first = q0;
+    for (; q0 < nIt; q0 += 32) {
+      const unsigned m = mask[q0 >> 5];
+      if (nf + __popc(m) > kWalkCap) break;
+      if (m >> lane & 1u) {
+        const int v = unit_item(J, U, q0 + lane);
+        fail[nf + __popc(m & ((1u << lane) - 1u))] = v;
+        pMask |= 1u << (v & 255);
+        m1 = m1 > ((v >> 8) & 255) ? m1 : (v >> 8) & 255;
+        m2 = m2 > ((v >> 16) & 255) ? m2 : (v >> 16) & 255;
+        m3 = m3 > (v >> 24) ? m3 : v >> 24;
+      }
+      nf += __popc(m);
     }
-  };
-  for (int e = tid; e < LE * LBE * LBE * nA; e += NT) T[e] = 0.0;
-  for (int e = tid; e < 64; e += NT) S.failMask[e] = 0;
-  if (tid == 0) {
-    S.warn = 0;
-    S.nFail = 0;
-    S.t2Next = 0;
-    S.estBits = 0ull;
-  }
-  __syncthreads();
-
-  // ---------------------------------------------------------- type 1
-  {
-    double *W = ph + warp * Lm.w1Stride;
-    const int ncab = (lab + 1) * (lab + 2) * (lab + 3) / 6;
-    for (int e = tid & 31; e < ncab; e += 32) W[Lm.w1H + e] = 0.0;
+    if (nf == 0) continue;
+    T2Pass S;
+    S.nf = nf;
+    S.mask = __reduce_or_sync(0xffffffffu, pMask);
+    S.l1 = __reduce_max_sync(0xffffffffu, m1);
+    S.l2 = __reduce_max_sync(0xffffffffu, m2);
+    S.l3 = __reduce_max_sync(0xffffffffu, m3);
+    for (int q = lane; q < nf; q += 32) sum[q] = 0.0;
     __syncwarp();
-    // primitive pairs by kind (normal, band, zero), each kind in pair order
-    int *perm = S.ppBreak;
-    if (warp == 0) {
-      const int lane = tid & 31;
-      int base[3] = {0, 0, 0};
-      for (int k0 = 0; k0 < NP; k0 += 32) {
-        const int k = k0 + lane;
-        int kind = -1;
-        if (k < NP) {
-          const double za = pzA[k / Nb], ca = zeta_times(pcA[k / Nb], za, pa0), zb = pzB[k % Nb],
-                       cb = zeta_times(pcB[k % Nb], zb, pb0);
-          const double C1 = t1_prefactor(za, ca, zb, cb, dAC, dBC);
-          double P[3];
-          for (int i = 0; i < 3; i++) P[i] = 2.0 * (za * gA[i] + zb * gB[i]);
-          const double s2 = P[0] * P[0] + P[1] * P[1] + P[2] * P[2];
-          kind = C1 == 0.0 ? kPairZero : (C1 < 0x1p-900 || s2 > 2800.0 * (za + zb)) ? kPairBand : kPairNormal;
-        }
-        // first pass: counts only
-        for (int kd = 0; kd < 3; kd++) base[kd] += __popc(__ballot_sync(0xffffffffu, kind == kd));
+    int mb = mb0, warn = 0;
+    for (int k = k0; k < k1; k++) {
+      t2_pair<kMixed>(J, U, L, sm, S, k, mb, map, win, useFF, warn);
+      mb = win[k].x > mb ? win[k].x : mb;
+    }
+    if (warn) atomicOr(&((UnitHead *)U.scr)->warn, 2);
+    int at = 0;
+    for (int w = first; w < q0; w += 32) {
+      const unsigned m = mask[w >> 5];
+      if (m >> lane & 1u) dst[w + lane] = sum[at + __popc(m & ((1u << lane) - 1u))];
+      at += __popc(m);
+    }
+    __syncwarp();
+  }
+}
+
+// One warp a CTA; the type-2 parts first (the longer ones), then the failed
+// type-1 pairs.
+template <bool kMixed>
+__global__ void __launch_bounds__(32, 12) k_unit_large(DevJob J) {
+  extern __shared__ double sm[];
+  const LargeSmem L = large_layout(J.maxLBS, J.maxLECP);
+  const int n2 = (int)J.counters[kCntPart], n = n2 + (int)J.counters[kCntFail];
+  for (int taken = 0; taken < J.take; taken++) {
+    const int i = next_item(J.counters + kHeadLarge);
+    if (i >= n) return;
+    if (i < n2) {
+      const int2 it = J.listPart[i];
+      const Unit U = unit_load(J, it.x);
+      t2_large<kMixed>(J, U, L, sm, it.y);
+    } else {
+      const T1Fail it = J.listFail[i - n2];
+      const Unit U = unit_load(J, it.pos);
+      t1_large<kMixed>(J, U, sm + L.tab, it.k & 0xffff, it.k >> 16, it.mask);
+    }
+  }
+}
+
+// -------------------------------------------------------- stage 4: the blocks
+
+// One unit a CTA: the type-1 block from the quadratures of its primitive
+// pairs (src/type1.c:323-345), the type-2 block from its radial table
+// (src/type2.c:583-623), both shifted onto A and B (src/util.c:247-334).
+constexpr int kLinkThreads = 128;
+__global__ void __launch_bounds__(kLinkThreads) k_unit_link(DevJob J) {
+  extern __shared__ double sm[];
+  int pos = J.chunk0 + blockIdx.x;
+  if (J.live) {
+    const int l0 = J.liveStart[J.chunk];
+    if (l0 + (int)blockIdx.x >= J.liveStart[J.chunk + 1]) return;
+    pos = J.live[l0 + blockIdx.x];
+  }
+  const Unit U = unit_load(J, pos);
+  if (!U.live) return;
+  const LinkSmem Lm = link_layout(J.maxLBS, J.maxLECP);
+  const int tid = threadIdx.x, NT = kLinkThreads, la = U.la, lb = U.lb, lab = U.lab, lq = lab + 1, lpa = U.lpa,
+            lpb = U.lpb, nca = NCUM(la), ncb = NCUM(lb), Lc = U.Lc, Nb = U.Nb;
+  const int nA = 2 * J.maxLBS + 1, LE = J.maxLECP > 0 ? J.maxLECP : 1, LBE = J.maxLBS + LE;
+  const size_t cA = (size_t)U.c * J.nAtoms + U.A, cB = (size_t)U.c * J.nAtoms + U.B;
+  double *chi = sm + Lm.chi, *Jsh = sm + Lm.J, *T = sm + Lm.T, *rsh = sm + Lm.rsh, *dir = sm + Lm.dir,
+         *W = sm + Lm.W, *H = sm + Lm.H;
+  double *out1 = J.out + (size_t)U.c * J.centreStride + J.pairOff[U.pr];
+  double *out2 = out1 + NCART(lpa) * NCART(lpb);
+  const int dd = J.tmDim + 1, tmW = (J.tmDim + 1) * (J.tmDim + 1), RQ = lq * lq, nq = t1_items(lab);
+  // type 1: W[L][l][m] = sum over the primitive pairs of S_lm Q[L][l] (the
+  // pairs in order), then H[p] = sum_lm poly2sph[p][lm] W[|p|][l][m]: the
+  // angular coefficients once per unit instead of once per pair
+  {
+    const double *Q = (const double *)(U.scr + U.L.Q);
+    const int nW = NCUM(lab);  // sum over L of (L+1)(L+2)/2 entries (l, m)
+    for (int e = tid; e < nW; e += NT) W[e] = 0.0;
+    for (int b0 = 0; b0 < U.NP; b0 += kLinkBatch) {
+      const int nb = U.NP - b0 < kLinkBatch ? U.NP - b0 : kLinkBatch;
+      __syncthreads();
+      if (tid < nb) {
+        const int k = b0 + tid;
+        const double za = U.pzA[k / Nb], zb = U.pzB[k % Nb];
+        double P[3];
+        for (int i = 0; i < 3; i++) P[i] = 2.0 * (za * U.gA[i] + zb * U.gB[i]);
+        direction(P, dir[3 * tid], dir[3 * tid + 1], dir[3 * tid + 2]);
       }
-      if (lane == 0) { S.t1Count[0] = base[0]; S.t1Count[1] = base[1]; S.t1Count[2] = base[2]; }
-      int pos[3] = {0, base[0], base[0] + base[1]};
-      for (int k0 = 0; k0 < NP; k0 += 32) {
-        const int k = k0 + lane;
-        int kind = -1;
-        if (k < NP) {
-          const double za = pzA[k / Nb], ca = zeta_times(pcA[k / Nb], za, pa0), zb = pzB[k % Nb],
-                       cb = zeta_times(pcB[k % Nb], zb, pb0);
-          const double C1 = t1_prefactor(za, ca, zb, cb, dAC, dBC);
-          double P[3];
-          for (int i = 0; i < 3; i++) P[i] = 2.0 * (za * gA[i] + zb * gB[i]);
-          const double s2 = P[0] * P[0] + P[1] * P[1] + P[2] * P[2];
-          kind = C1 == 0.0 ? kPairZero : (C1 < 0x1p-900 || s2 > 2800.0 * (za + zb)) ? kPairBand : kPairNormal;
-        }
-        for (int kd = 0; kd < 3; kd++) {
-          const unsigned m = __ballot_sync(0xffffffffu, kind == kd);
-          if (kind == kd) perm[pos[kd] + __popc(m & ((1u << lane) - 1u))] = k;
-          pos[kd] += __popc(m);
-        }
+      __syncthreads();
+      for (int e = tid; e < nb * lq; e += NT) {
+        const int g = e / lq, m = e % lq;
+        rsh_column(J, lab, m, dir[3 * g], dir[3 * g + 1], dir[3 * g + 2], rsh + g * RQ);
+      }
+      __syncthreads();
+      for (int e = tid; e < nW; e += NT) {
+        int Lm1 = 0;
+        while (NCUM(Lm1) <= e) Lm1++;
+        int r = e - NCUM(Lm1 - 1), l = Lm1;
+        while (r >= 2 * l + 1) { r -= 2 * l + 1; l -= 2; }
+        const double *q = Q + (size_t)b0 * nq + t1_index(Lm1, l), *s = rsh + l * l + r;
+        double v = W[e];
+        for (int g = 0; g < nb; g++) v += s[g * RQ] * q[(size_t)g * nq];
+        W[e] = v;
       }
     }
     __syncthreads();
-    // groups of each kind, dealt to the warps round-robin over all kinds
-    int Gk[3], nG[3], nGroups = 0;
-    for (int kd = 0; kd < 3; kd++) {
-      const int n = S.t1Count[kd];
-      int G = t1_group(lab, gcapU);
-      // balance: with few primitive pairs, narrower groups keep all warps busy
-      if (balU) {
-        const int Gb = (n + kWarps - 1) / kWarps;
-        if (Gb < G) G = Gb > 0 ? Gb : 1;
+    for (int pi = tid; pi < nW; pi += NT) {
+      const int *ex = J.ijk + 3 * pi;
+      const int lmax = ex[0] + ex[1] + ex[2];
+      const double *p2s = J.p2s + (size_t)J.ijkIdx[(ex[0] * dd + ex[1]) * dd + ex[2]] * tmW;
+      const double *w = W + NCUM(lmax - 1);
+      double acc = 0.0;
+      for (int l = lmax; l >= 0; l -= 2) {
+        for (int m = 0; m < 2 * l + 1; m++) acc += p2s[l * l + m] * w[m];
+        w += 2 * l + 1;
       }
-      Gk[kd] = G;
-      nG[kd] = (n + G - 1) / G;
-      nGroups += nG[kd];
-    }
-    for (int gi = warp; gi < nGroups; gi += kWarps) {
-      int kd = 0, gj = gi, off = 0;
-      while (gj >= nG[kd]) { gj -= nG[kd]; off += S.t1Count[kd]; kd++; }
-      const int p0 = off + gj * Gk[kd], n = S.t1Count[kd] - gj * Gk[kd], G = n < Gk[kd] ? n : Gk[kd];
-      if (kd == kPairNormal)
-        t1_group_run<kMixed, kPairNormal>(J, Lm, W, c, Lc, la, lb, perm, p0, G, Nb, pzA, pcA, pzB, pcB, gA, gB,
-                                          ws, we, pa0, pb0, warn1);
-      else if (kd == kPairBand)
-        t1_group_run<kMixed, kPairBand>(J, Lm, W, c, Lc, la, lb, perm, p0, G, Nb, pzA, pcA, pzB, pcB, gA, gB,
-                                        ws, we, pa0, pb0, warn1);
-      else
-        t1_group_run<kMixed, kPairZero>(J, Lm, W, c, Lc, la, lb, perm, p0, G, Nb, pzA, pcA, pzB, pcB, gA, gB,
-                                        ws, we, pa0, pb0, warn1);
-    }
-    // the type-2 small-grid quadratures, 32 at a time to whichever warp is
-    // through with its type-1 groups (each writes its own entry of T: the
-    // result does not depend on the warp)
-    for (;;) {
-      int q0 = 0;
-      if ((tid & 31) == 0) q0 = atomicAdd(&S.t2Next, 32);
-      q0 = __shfl_sync(0xffffffffu, q0, 0);
-      if (q0 >= nItems) break;
-      if (q0 + (tid & 31) < nItems) small_item(q0 + (tid & 31));
+      H[pi] = acc;
     }
     __syncthreads();
-    // chi[i][j] = sum over warps of H[index(a_i + b_j)]
-    const int dd = J.tmDim + 1;
     for (int e = tid; e < nca * ncb; e += NT) {
       const int *ei = J.ijk + 3 * (e / ncb), *ej = J.ijk + 3 * (e % ncb);
-      int pi = J.ijkIdx[((ei[0] + ej[0]) * dd + (ei[1] + ej[1])) * dd + ei[2] + ej[2]];
-      double v = 0.0;
-      for (int w = 0; w < kWarps; w++) v += ph[w * Lm.w1Stride + Lm.w1H + pi];
-      chi[e] = v;
+      chi[e] = H[J.ijkIdx[((ei[0] + ej[0]) * dd + (ei[1] + ej[1])) * dd + ei[2] + ej[2]]];
     }
-    __syncthreads();
   }
+  // the radial table of type 2
+  auto tidx = [&](int l, int l1, int l2, int l3) { return ((l * LBE + l1) * LBE + l2) * nA + l3; };
+  for (int e = tid; e < LE * LBE * LBE * nA; e += NT) T[e] = 0.0;
+  __syncthreads();
+  {
+    const double *Tq = (const double *)(U.scr + U.L.T), *part = (const double *)(U.scr + U.L.part);
+    const unsigned *mask = (const unsigned *)(U.scr + U.L.mask);
+    const int nParts = t2_parts(U.NP), nIt = class_items(J, U.cls * LE, LE);
+    for (int q = tid; q < U.nItems; q += NT) {
+      double v;
+      if (nParts > 1 && (mask[q >> 5] >> (q & 31) & 1u)) {
+        v = 0.0;
+        for (int p = 0; p < nParts; p++) v += part[(size_t)p * nIt + q];
+      } else {
+        v = Tq[q];
+      }
+      const int it = unit_item(J, U, q);
+      T[tidx(it & 255, (it >> 8) & 255, (it >> 16) & 255, it >> 24)] = v;
+    }
+  }
+  __syncthreads();
   auto poly_shift = [&](double norm, double *dst) {  // src/util.c:247-334
-    const int D = J.uspD, dd = J.tmDim + 1, nta = NCART(lpa), ntb = NCART(lpb);
+    const int D = J.uspD, nta = NCART(lpa), ntb = NCART(lpb);
     const double *uA = J.usp + cA * D * D * D, *uB = J.usp + cB * D * D * D;
     for (int e = tid; e < nta * ncb; e += NT) {
       int c1 = e / ncb, q = e % ncb;
@@ -1680,107 +1878,6 @@ static __device__ void unit_fast(const DevJob &J, const long long u, FastShared 
   };
   const double norm1 = 4.0 * kPi, norm2 = norm1 * norm1;
   poly_shift(norm1, out1);
-
-  // ---------------------------------------------------------- type 2
-  // (the small-grid quadratures ran beside the type-1 groups)
-  if (S.nFail > 0) {
-    // break index of every primitive pair (bisection: the break predicate is
-    // monotone in the index beyond both centres)
-    double *map = ph + Lm.ppMap;
-    int *win = (int *)(ph + Lm.ppWin);
-    for (int k = tid; k < NP; k += NT) {
-      double za = pzA[k / Nb], zb = pzB[k % Nb], i1, i2;
-      fm06(za, zb, dAC, dBC, i1, i2);
-      map[2 * k] = i1;
-      map[2 * k + 1] = i2;
-      int lo = 0, hi = J.largeOrder;
-      while (lo < hi) {
-        int mid = (lo + hi) >> 1;
-        double r = i1 * J.xLarge[mid] + i2, d1 = dAC - r, d2 = dBC - r;
-        double e = -za * d1 * d1 - zb * d2 * d2;
-        if (r > dAC && r > dBC && e < J.lnAcc2) hi = mid; else lo = mid + 1;
-      }
-      S.ppBreak[k] = lo < J.largeOrder ? lo : INT_MAX;
-      // point-index interval outside which this pair's exponent stays below
-      // the screen by a margin of 1: the exponent is a parabola in r with
-      // its vertex at P and r grows with the index
-      const double thr = J.lnAcc2 - 1.0, P = (za * dAC + zb * dBC) / (za + zb);
-      auto exq = [&](int n) {
-        const double r = i1 * J.xLarge[n] + i2, d1 = dAC - r, d2 = dBC - r;
-        return -za * d1 * d1 - zb * d2 * d2;
-      };
-      int a = 0, bb = J.largeOrder;
-      while (a < bb) {
-        const int mid = (a + bb) >> 1;
-        if (i1 * J.xLarge[mid] + i2 >= P) bb = mid; else a = mid + 1;
-      }
-      const int nv = a;
-      a = 0;
-      bb = nv;
-      while (a < bb) {
-        const int mid = (a + bb) >> 1;
-        if (exq(mid) >= thr) bb = mid; else a = mid + 1;
-      }
-      win[2 * k] = a;
-      a = nv;
-      bb = J.largeOrder;
-      while (a < bb) {
-        const int mid = (a + bb) >> 1;
-        if (exq(mid) < thr) bb = mid; else a = mid + 1;
-      }
-      win[2 * k + 1] = a - 1;
-    }
-    if (tid == 0) S.nextBase = 0;
-    __syncthreads();
-    // passes of up to kWalkCap failed items.  Thread 0 writes the pass's
-    // list, count and resume point before the barrier; every thread reads
-    // the count after it, and thread 0 writes again only after the pass's
-    // last barrier, so no thread can see the next pass's values early.
-    for (;;) {
-      if (tid == 0) {
-        int nf = 0, q = S.nextBase;
-        unsigned mask = 0;
-        int m1 = 0, m2 = 0, m3 = 0;
-        for (; q < nItems && nf < kWalkCap; q++)
-          if (S.failMask[q >> 5] & (1u << (q & 31))) {
-            int l, l1, l2, l3;
-            item(q, l, l1, l2, l3);
-            // the item's (l, l1, l2, l3), one byte each (all below 16)
-            S.failIdx[nf++] = l | l1 << 8 | l2 << 16 | l3 << 24;
-            mask |= 1u << l;
-            m1 = l1 > m1 ? l1 : m1;
-            m2 = l2 > m2 ? l2 : m2;
-            m3 = l3 > m3 ? l3 : m3;
-          }
-        S.nThis = nf;
-        S.nextBase = q;
-        S.passMask = mask;
-        S.passL1 = m1;
-        S.passL2 = m2;
-        S.passL3 = m3;
-      }
-      __syncthreads();
-      const int nf = S.nThis;
-      if (nf == 0) break;  // no failed item left
-      double *W = ph + warp * Lm.w2Stride;
-      for (int q = tid & 31; q < nf; q += 32) W[Lm.w2Part + q] = 0.0;
-      __syncwarp();
-      // mixed path: double-single tables only where their sums can take the
-      // reference's decisions (ff_limit); larger integrals in FP64
-      const bool ff2 = kMixed && __longlong_as_double((long long)S.estBits) < ff_limit(J.tol);
-      for (int k = warp; k < NP; k += kWarps)
-        t2_pair<kMixed>(J, Lm, W, S, k, Nb, nf, c, Lc, la, lb, pzA, pcA, pzB, pcB, dAC, dBC, ncls, pa0, pb0,
-                        ph + Lm.ppMap, (const int *)(ph + Lm.ppWin), ff2, warn2);
-      __syncthreads();
-      for (int q = tid; q < nf; q += NT) {
-        double v = 0.0;
-        for (int w = 0; w < kWarps; w++) v += ph[w * Lm.w2Stride + Lm.w2Part + q];
-        const int it = S.failIdx[q];
-        T[tidx(it & 255, (it >> 8) & 255, (it >> 16) & 255, it >> 24)] = v;
-      }
-      __syncthreads();
-    }
-  }
   // gamma (src/type2.c:583-623)
   {
     const double *angA = J.ang + cA * J.angLam * J.angLM * J.angC;
@@ -1811,14 +1908,12 @@ static __device__ void unit_fast(const DevJob &J, const long long u, FastShared 
   }
   __syncthreads();
   poly_shift(norm2, out2);
-  if (warn1) atomicOr(&S.warn, 1);
-  if (warn2) atomicOr(&S.warn, 2);
-  __syncthreads();
   if (tid == 0) {
-    int st = (S.warn & 1) ? kUnitWarnType1 : (S.warn & 2) ? kUnitWarnType2 : kUnitDone;
+    const int warn = ((const UnitHead *)U.scr)->warn;
+    const long long u = (long long)U.c * J.nPairs + U.pr;
+    const int st = (warn & 1) ? kUnitWarnType1 : (warn & 2) ? kUnitWarnType2 : kUnitDone;
     J.status[u] = st;
     if (st != kUnitDone) atomicMin(&J.errWord[0], (int)u);
-    if (J.classCycles) atomicAdd(&J.classCycles[cls], (unsigned long long)(clock64() - tc0));
   }
 }
 
@@ -1849,10 +1944,13 @@ __global__ void __launch_bounds__(128) k_shell_F_fast(DevJob J) {
         for (int p = 0; p < J.shK[s]; p++) {
           double zeta = pa[p], da = pd[p];
           for (int k = 0; k < run; k++) da *= zeta;
-          bessel_fast<false>(J, lmaxA, 2.0 * zeta * dAC * r, K, 1);
           double e = dAC - r;
-          e = fast_exp(-zeta * e * e);
-          for (int i = 0; i <= lmaxA; i++) acc[i] += da * K[i] * e;
+          e = -zeta * e * e;
+          const xf v = e > -700.0 ? xf_mul(fx_exp(fx_q53(e)), xf_from(da)) : xf{0, 0};
+          if (v.m == 0) continue;
+          const xf f = xf_mul(xf_from(zeta), xf_from(dAC));
+          bessel_fx(J, lmaxA, xf_mul(xf_times100({f.m, f.e + 1}), xf_from(r)), v, sign_of(da), K);
+          for (int i = 0; i <= lmaxA; i++) acc[i] += K[i];
         }
       }
       for (int i = 0; i < nF; i++) F[(size_t)n * nF + i] = acc[i];
@@ -1860,45 +1958,12 @@ __global__ void __launch_bounds__(128) k_shell_F_fast(DevJob J) {
   }
 }
 
-// The unit at queue position i (cost order, or the reference's order).
-__device__ inline long long queue_unit(const DevJob &J, long long i) { return J.order ? J.order[i] : i; }
-
-// A CTA per unit; blockIdx.x is a queue position.
-template <bool kMixed>
-__global__ void __launch_bounds__(kUnitThreads, kUnitCtasPerSm) k_unit_fast(DevJob J) {
-  extern __shared__ double sm[];
-  __shared__ FastShared S;
-  const long long i = blockIdx.x;
-  unit_fast<kMixed>(J, J.order ? (long long)J.order[i] : i, S, sm);
-}
-
-// Persistent CTAs (as many as fit on the GPU) pulling queue positions from
-// one counter: the costliest units start first and the cheap ones fill the
-// tail, whatever order the hardware would dispatch CTAs in.
-template <bool kMixed>
-__global__ void __launch_bounds__(kUnitThreads, kUnitCtasPerSm) k_unit_queue(DevJob J) {
-  extern __shared__ double sm[];
-  __shared__ FastShared S;
-  __shared__ long long next;
-  // with the screening stage the queue holds the live units only
-  const long long n = J.live ? (long long)*J.liveCount : (long long)J.nCentres * J.nPairs;
-  // ctaUnits > 0: a CTA takes at most that many units and exits, so that
-  // the SMs free up for other launches (the request server's jobs)
-  for (int taken = 0; J.ctaUnits <= 0 || taken < J.ctaUnits; taken++) {
-    if (threadIdx.x == 0) next = (long long)atomicAdd(J.queueHead, 1ull);
-    __syncthreads();
-    const long long i = next;
-    if (i >= n) break;
-    unit_fast<kMixed>(J, J.live ? (long long)J.live[i] : queue_unit(J, i), S, sm);
-    __syncthreads();  // shared state is rewritten by the next unit
-  }
-}
-
 // ---------------------------------------------------------- screening stage
 
-// True when unit u computes blocks: the unit kernels' own early exits (the
-// screened windows of src/libecp.c:296-330 and the derivative skip rules).
-static __device__ bool unit_live(const DevJob &J, long long u) {
+constexpr int kScreenThreads = 256;
+
+static __device__ bool unit_live(const DevJob &J, int pos) {
+  const long long u = unit_at(J, pos);
   const int c = (int)(u / J.nPairs), pr = (int)(u % J.nPairs);
   const int sa = J.pairA[pr], sb = J.pairB[pr];
   const int *wa = J.win + ((size_t)c * J.nShells + sa) * 3;
@@ -1908,20 +1973,18 @@ static __device__ bool unit_live(const DevJob &J, long long u) {
   return (wa[0] > wb[0] ? wa[0] : wb[0]) < (wa[1] > wb[1] ? wa[1] : wb[1]);
 }
 
-constexpr int kScreenThreads = 256;
-
-// Live units per CTA chunk of the queue.
+// Live units (those that compute blocks: the screened windows of
+// src/libecp.c:296-330 and the derivative skips) per CTA chunk of the queue.
 __global__ void __launch_bounds__(kScreenThreads) k_screen_count(DevJob J, long long n) {
   const long long i = (long long)blockIdx.x * kScreenThreads + threadIdx.x;
-  const int live = i < n && unit_live(J, queue_unit(J, i));
-  const int cnt = __syncthreads_count(live);
+  const int cnt = __syncthreads_count(i < n && unit_live(J, (int)i));
   if (threadIdx.x == 0) J.screenBlocks[blockIdx.x] = cnt;
 }
 
-// Exclusive scan of the per-CTA counts (one CTA); the total is the live count.
+// Exclusive scan of the per-CTA counts (one CTA); the total ends the last chunk.
 __global__ void __launch_bounds__(1024) k_screen_scan(DevJob J, int nBlocks) {
   __shared__ int v[1024];
-  __shared__ long long base;
+  __shared__ int base;
   if (threadIdx.x == 0) base = 0;
   __syncthreads();
   for (int b0 = 0; b0 < nBlocks; b0 += 1024) {
@@ -1935,34 +1998,37 @@ __global__ void __launch_bounds__(1024) k_screen_scan(DevJob J, int nBlocks) {
       v[threadIdx.x] += y;
       __syncthreads();
     }
-    if (b < nBlocks) J.screenBlocks[b] = (int)(base + v[threadIdx.x] - x);
+    if (b < nBlocks) J.screenBlocks[b] = base + v[threadIdx.x] - x;
     __syncthreads();
     if (threadIdx.x == 1023) base += v[1023];
     __syncthreads();
   }
-  if (threadIdx.x == 0) *J.liveCount = (unsigned long long)base;
+  if (threadIdx.x == 0) J.liveStart[J.nChunks] = base;
 }
 
-// Stable compaction of the live units; the others are marked skipped here.
+// Stable compaction of the live units' queue positions; the others are marked
+// skipped here.  A chunk's first position notes where its live units start.
 __global__ void __launch_bounds__(kScreenThreads) k_screen_scatter(DevJob J, long long n) {
   __shared__ int warpCnt[kScreenThreads / 32];
   const long long i = (long long)blockIdx.x * kScreenThreads + threadIdx.x;
-  const long long u = i < n ? queue_unit(J, i) : -1;
-  const bool live = u >= 0 && unit_live(J, u);
+  const bool live = i < n && unit_live(J, (int)i);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned m = __ballot_sync(0xffffffffu, live);
   if (lane == 0) warpCnt[warp] = __popc(m);
   __syncthreads();
-  int pos = J.screenBlocks[blockIdx.x] + __popc(m & ((1u << lane) - 1u));
-  for (int w = 0; w < warp; w++) pos += warpCnt[w];
-  if (live) J.live[pos] = (int)u;
-  else if (u >= 0) J.status[u] = kUnitSkipped;
+  if (i >= n) return;
+  int at = J.screenBlocks[blockIdx.x] + __popc(m & ((1u << lane) - 1u));
+  for (int w = 0; w < warp; w++) at += warpCnt[w];
+  if (live) J.live[at] = (int)i;
+  else J.status[unit_at(J, (int)i)] = kUnitSkipped;
+  if ((int)i % J.nCentres == 0)
+    for (int k = 0; k < J.nChunks; k++)
+      if (J.chunkPair[k] == (int)i / J.nCentres) J.liveStart[k] = at;
 }
 
-__global__ void k_reset(int *errWord, unsigned long long *queueHead) {
+__global__ void k_reset(int *errWord) {
   errWord[0] = INT_MAX;
   errWord[1] = 0;
-  if (queueHead) *queueHead = 0ull;
 }
 
 // --------------------------------------------------------------- launchers
@@ -1992,74 +2058,84 @@ void fast_prepare() {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || attr[dev]) return;
-  for (const void *k : {(const void *)k_unit_fast<false>, (const void *)k_unit_queue<false>,
-                        (const void *)k_unit_fast<true>, (const void *)k_unit_queue<true>}) {
+  for (const void *k : {(const void *)k_unit_small<false>, (const void *)k_unit_small<true>,
+                        (const void *)k_unit_large<false>, (const void *)k_unit_large<true>,
+                        (const void *)k_unit_link}) {
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    // the whole unified L1/shared array as shared memory: three CTAs of
-    // <= 72 KB per SM
+    // most of the unified L1/shared array as shared memory
     cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   }
   attr[dev] = true;
 }
 
-int fast_ctas_per_sm(size_t smemBytes, int queue) {
+int fast_ctas_per_sm(size_t smemBytes) {
   fast_prepare();
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, queue ? (const void *)k_unit_queue<false> : (const void *)k_unit_fast<false>,
-                                                    kUnitThreads, smemBytes) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, (const void *)k_unit_small<false>, 32, smemBytes) != cudaSuccess)
     return 0;
   return n;
 }
 
-void launch_reset(const DevJob &J, cudaStream_t st) { k_reset<<<1, 1, 0, st>>>(J.errWord, J.queueHead); }
+void launch_reset(const DevJob &J, cudaStream_t st) { k_reset<<<1, 1, 0, st>>>(J.errWord); }
 
-int launch_fast_pipeline(const DevJob &J, cudaStream_t st, size_t smemBytes, const FastConfig &cfg,
-                         cudaEvent_t u0, cudaEvent_t u1) {
+int launch_fast_pipeline(const DevJob &J, cudaStream_t st, const FastConfig &cfg, cudaEvent_t u0, cudaEvent_t u1) {
   fast_prepare();
-  if (smemBytes > 200 * 1024) return 3;
   DevJob Jc = J;
   Jc.gcap = cfg.gcap;
-  Jc.mixed = cfg.mixed;
   Jc.balance = cfg.balance;
   for (int i = 0; i < kMaxClasses; i++) Jc.classCfg[i] = cfg.cls[i];
   Jc.classCycles = cfg.classCycles;
-  if (!cfg.sorted) Jc.order = nullptr;
-  else if (cfg.sorted == 2 && J.orderClass) Jc.order = J.orderClass;
-  const bool screen = cfg.queue && cfg.screen && J.queueHead && J.live && J.liveCount && J.screenBlocks;
+  const JobPlan::Order &ord = J.plan->order[cfg.sorted];
+  Jc.pairOrder = J.pairOrders + (size_t)cfg.sorted * J.nPairs;
+  Jc.scrOff = J.scrOffs + (size_t)cfg.sorted * (J.nPairs + 1);
+  Jc.chunkPair = J.chunkPairs + ord.chunkAt;
+  Jc.nChunks = (int)ord.chunks.size();
+  const size_t sSmall = fast_smem_bytes(J.maxLBS, cfg.gcap);
+  const size_t sLarge = sizeof(double) * (size_t)large_layout(J.maxLBS, J.maxLECP).total;
+  const size_t sLink = sizeof(double) * (size_t)link_layout(J.maxLBS, J.maxLECP).total;
+  if (sSmall > 200 * 1024 || sLarge > 200 * 1024 || sLink > 200 * 1024) return 3;
+  const bool screen = cfg.queue && cfg.screen;
   if (!screen) Jc.live = nullptr;
-  launch_prologue(Jc, st, false);
-  {
-    DevJob Jf = Jc;
-    Jf.mixed = 0;  // the F tables stay FP64 in every mode
-    k_shell_F_fast<<<dim3(J.nShells, J.nCentres), 128, 0, st>>>(Jf);
-  }
-  long long nUnits = (long long)J.nCentres * J.nPairs;
-  if (screen && nUnits > 0) {  // screening stage: the queue of live units
+  launch_stage1(Jc, st);
+  k_shell_F_fast<<<dim3(J.nShells, J.nCentres), 128, 0, st>>>(Jc);
+  const long long nUnits = (long long)J.nCentres * J.nPairs;
+  if (screen && nUnits > 0) {  // screening stage: the live units' positions
     const long long nb = (nUnits + kScreenThreads - 1) / kScreenThreads;
     k_screen_count<<<(unsigned)nb, kScreenThreads, 0, st>>>(Jc, nUnits);
     k_screen_scan<<<1, 1024, 0, st>>>(Jc, (int)nb);
     k_screen_scatter<<<(unsigned)nb, kScreenThreads, 0, st>>>(Jc, nUnits);
   }
   if (u0) record_timing(u0, st);
-  if (nUnits > 0) {
-    if (cfg.queue && J.queueHead) {
-      int dev = 0, sms = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      int per = fast_ctas_per_sm(smemBytes, 1);
-      long long grid = (long long)sms * (per > 0 ? per : 1);
-      if (J.ctaUnits > 0) {  // bounded CTAs: enough of them for every unit
-        const long long need = (nUnits + J.ctaUnits - 1) / J.ctaUnits;
-        grid = need > grid ? need : grid;
-        if (grid > (1LL << 30)) grid = 1LL << 30;
-      }
-      if (grid > nUnits) grid = nUnits;
-      if (cfg.mixed) k_unit_queue<true><<<(unsigned)grid, kUnitThreads, smemBytes, st>>>(Jc);
-      else k_unit_queue<false><<<(unsigned)grid, kUnitThreads, smemBytes, st>>>(Jc);
-    } else {
-      if (cfg.mixed) k_unit_fast<true><<<(unsigned)nUnits, kUnitThreads, smemBytes, st>>>(Jc);
-      else k_unit_fast<false><<<(unsigned)nUnits, kUnitThreads, smemBytes, st>>>(Jc);
-    }
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  for (int k = 0; k < Jc.nChunks; k++) {
+    const JobPlan::Chunk &ch = ord.chunks[k];
+    Jc.chunk = k;
+    Jc.chunk0 = ch.p0 * J.nCentres;
+    Jc.chunk1 = ch.p1 * J.nCentres;
+    Jc.scrBase = ch.base;
+    char *lists = J.scr + ch.scratch;
+    Jc.listT1 = (int2 *)lists;
+    Jc.listT2 = Jc.listT1 + ch.groups;
+    Jc.listPart = Jc.listT2 + ch.batches;
+    Jc.listFail = (T1Fail *)(Jc.listPart + ch.parts);
+    cudaMemsetAsync(Jc.counters, 0, sizeof(unsigned) * kCounters, st);
+    const long long n = (long long)Jc.chunk1 - Jc.chunk0;
+    k_unit_plan<<<(unsigned)((n + 3) / 4), kPlanThreads, 0, st>>>(Jc);
+    // entries a warp takes: 8 where there are many (fewer CTAs to start), one
+    // where there are few (every SM gets work)
+    auto take = [&](long long items) { return (int)std::min(8ll, std::max(1ll, items / (64ll * sms))); };
+    const long long nSmall = ch.groups + ch.batches, nLarge = ch.parts + ch.groups;
+    Jc.take = take(nSmall);
+    const unsigned gSmall = (unsigned)std::max(1ll, (nSmall + Jc.take - 1) / Jc.take);
+    if (cfg.mixed) k_unit_small<true><<<gSmall, 32, sSmall, st>>>(Jc);
+    else k_unit_small<false><<<gSmall, 32, sSmall, st>>>(Jc);
+    Jc.take = take(nLarge);
+    const unsigned gLarge = (unsigned)std::max(1ll, (nLarge + Jc.take - 1) / Jc.take);
+    if (cfg.mixed) k_unit_large<true><<<gLarge, 32, sLarge, st>>>(Jc);
+    else k_unit_large<false><<<gLarge, 32, sLarge, st>>>(Jc);
+    k_unit_link<<<(unsigned)n, kLinkThreads, sLink, st>>>(Jc);
   }
   if (u1) record_timing(u1, st);
   launch_epilogue(Jc, st);

@@ -1,0 +1,273 @@
+// ecp_fixed.h -- 64-bit integer-mantissa arithmetic of the batched path.
+//
+// GB300's FP64 pipe takes one warp instruction per 16 to 19 cycles and SM,
+// whatever the number of active lanes, and holds a warp for 64 cycles per
+// dependent operation; the integer pipes take one warp instruction per cycle
+// and SM quarter at 4 to 6 cycles of latency.  The tabulations of the batched
+// kernels (Bessel rows, exponentials, powers, prefactors) therefore run on
+// the integer pipes with 64-bit mantissas -- eleven bits more than FP64 -- and
+// round once, to double, where a table entry is written.
+//
+// Two forms:
+//   xf        an unsigned 64-bit mantissa and a binary exponent, value m * 2^e.
+//             Products keep the high 64 bits (mul_hi, below 3 units short) and
+//             are not renormalised, so a product loses at most one leading
+//             bit; norm1() wins one back.
+//   fixed     a signed 64-bit integer at a scale the context knows (Horner
+//             passes, exponents in Q53).
+// Everything here is integer arithmetic (one float reciprocal seeds fx_recip
+// on either side), so host and device agree bit for bit; tests/test_fixed.py
+// measures the errors on the host against 200-bit arithmetic.
+#pragma once
+#include <cstdint>
+#include <cstring>
+
+#include "ecp_fastmath.h"
+
+namespace ecpgb {
+
+using u64 = unsigned long long;
+using i64 = long long;
+
+struct xf {
+  u64 m;
+  int e;
+};
+
+ECPGB_HD int clz64(u64 v) {
+#ifdef __CUDA_ARCH__
+  return __clzll((i64)v);
+#else
+  return v ? __builtin_clzll(v) : 64;
+#endif
+}
+
+// High 64 bits of a * b, up to 2 units below the exact value: three 32-bit
+// products instead of four.
+ECPGB_HD u64 mul_hi(u64 a, u64 b) {
+  const uint32_t a0 = (uint32_t)a, a1 = (uint32_t)(a >> 32), b0 = (uint32_t)b, b1 = (uint32_t)(b >> 32);
+  return (u64)a1 * b1 + (((u64)a1 * b0) >> 32) + (((u64)a0 * b1) >> 32);
+}
+
+// A multiplier 0 <= x < 2^63 split for mul_hi_s: high word, signed low word.
+struct fxmul {
+  int hi, lo;
+};
+ECPGB_HD fxmul fx_split(u64 x) {
+  const int lo = (int)(uint32_t)x;
+  return {(int)(uint32_t)(x >> 32) - (lo >> 31), lo};
+}
+// v * x / 2^64 for signed v and a split x, within 2 units: the low word of x
+// is taken signed so that every 32-bit product has one kind of operands.
+ECPGB_HD i64 mul_hi_s(i64 v, fxmul x) {
+  const int v1 = (int)(v >> 32);
+  const uint32_t v0 = (uint32_t)v;
+  return (i64)v1 * x.hi + (i64)(((u64)v0 * (uint32_t)x.hi) >> 32) + (((i64)v1 * x.lo) >> 32);
+}
+
+// A finite non-negative double (a subnormal counts as 0); the sign is ignored.
+ECPGB_HD xf xf_from(double x) {
+  const u64 b = (u64)dbits(x);
+  const int be = (int)(b >> 52) & 0x7ff;
+  return {be ? (b << 11) | (1ull << 63) : 0ull, be - (1023 + 63)};
+}
+// The sign bit of a double, in the high word's position.
+ECPGB_HD uint32_t sign_of(double x) { return (uint32_t)((u64)dbits(x) >> 32) & 0x80000000u; }
+
+ECPGB_HD xf xf_mul(xf a, xf b) { return {mul_hi(a.m, b.m), a.e + b.e + 64}; }
+// Wins back the leading bit a product of normalised mantissas may have lost.
+ECPGB_HD xf norm1(xf a) {
+  if ((i64)a.m >= 0) {
+    a.m += a.m;
+    a.e -= 1;
+  }
+  return a;
+}
+
+// Leading bit to the top (a zero stays zero).
+ECPGB_HD xf xf_norm(xf a) {
+  const int lz = clz64(a.m | 1u);
+  return {a.m << lz, a.e - lz};
+}
+
+// m * 2^e rounded to the nearest double, with a sign; 0 below the normal range.
+ECPGB_HD double xf_to_double(u64 m, int e, uint32_t sign) {
+  const int lz = clz64(m);
+  const int be = e + 63 + 1023 - lz;  // biased exponent
+  m <<= (lz & 63);
+  const u64 b = ((u64)(uint32_t)be << 52) + ((m << 1) >> 12) + ((m >> 10) & 1u);
+  return lz < 64 && be > 0 ? bits_d((i64)(b | (u64)sign << 32)) : 0.0;
+}
+
+// v >> s for s >= 0 (0 from 64 on).
+ECPGB_HD u64 shr64(u64 v, int s) { return s > 63 ? 0ull : v >> s; }
+
+#ifdef __CUDACC__
+static __device__ const u64 kExp2Fixed[ECPGB_EXP2_N] = ECPGB_EXP2_TABLE62;
+#endif
+static const u64 kExp2FixedHost[ECPGB_EXP2_N] = ECPGB_EXP2_TABLE62;
+
+// exp(E / 2^53) for |E| < 2^63 (arguments within +-1023): Tang's table method
+// as in fast_exp, in fixed point.  n = floor of E * 512/ln2 (up to 1/64 below
+// the exact quotient: r then ends slightly above ln2/512), r = E - n ln2/512
+// in Q62 from a 94-bit ln2/512, exp(r) to degree 5 with each term in as many
+// bits as its weight needs, times 2^(j/512) with 62 bits.  Error below 2^-58
+// of the result.
+ECPGB_HD xf fx_exp(i64 E) {
+  const int Eh = (int)(E >> 32);  // Q21
+  // 512/ln2 in Q20; the bias (1/128 of a step) covers its error and Eh's
+  const i64 prod = (i64)Eh * 774541002 - (1ll << 34);
+  const int n = (int)(prod >> 41);
+  const i64 nl = n;
+  u64 r = ((u64)E << 9) - (u64)nl * ECPGB_LN2_512_Q62 - (u64)((nl * (i64)ECPGB_LN2_512_Q94LO) >> 32);
+  const u64 X = r << 11;  // r * 2^9 in Q64, r < 2^-9.5
+  const uint32_t X32 = (uint32_t)(X >> 32);
+  const uint32_t u4 = 178956971u + (uint32_t)(((u64)X32 * 69905u) >> 32);          // 1/24 + r/120, Q32
+  const uint32_t u3 = 715827883u + ((uint32_t)(((u64)X32 * u4) >> 32) >> 9);       // 1/6 + r u4, Q32
+  const u64 u2 = (1ull << 63) + (((u64)X32 * u3) >> 9);                            // 1/2 + r u3, Q64
+  const u64 u1 = (1ull << 63) + (mul_hi(X, u2) >> 10);                             // 1 + r u2, Q63
+  const u64 p = mul_hi(X, u1) >> 8;                                                // exp(r) - 1, Q64
+#ifdef __CUDA_ARCH__
+  const u64 s = __ldg(&kExp2Fixed[n & (ECPGB_EXP2_N - 1)]);
+#else
+  const u64 s = kExp2FixedHost[n & (ECPGB_EXP2_N - 1)];
+#endif
+  return {s + mul_hi(s, p), (n >> ECPGB_EXP2_LOG2N) - 62};
+}
+
+// 1/x for a mantissa x in [2^63, 2^64): 2^126 / x within 2^-60 of it, by two
+// Newton steps from a float reciprocal.
+ECPGB_HD u64 fx_recip(u64 x) {
+  const float f = (float)(uint32_t)(x >> 40) * 0x1p-23f;
+#ifdef __CUDA_ARCH__
+  const float g = __frcp_rn(f);
+#else
+  const float g = 1.0f / f;
+#endif
+  const u64 y0 = (u64)(uint32_t)(g * 0x1p31f);  // Q31, 23 bits
+  // t = x y0 in Q62, d = 1 - t
+  const u64 t0 = (x >> 32) * y0 + (((x & 0xffffffffull) * y0) >> 32);
+  const i64 d0 = (i64)((1ull << 62) - t0);  // Q62, about 40 bits
+  u64 y = (y0 << 32) + (u64)(((i64)y0 * (d0 >> 8)) >> 22);
+  const i64 d1 = (i64)((1ull << 62) - mul_hi(x, y));  // Q62, about 18 bits
+  y += (u64)(((i64)(y >> 32) * d1) >> 30);
+  return y;  // Q63
+}
+
+// Table reads: 16 bytes (the rows are 16-byte aligned) and 8 bytes.
+struct fxpair {
+  i64 x, y;
+};
+ECPGB_HD fxpair ld_pair(const i64 *p) {
+#ifdef __CUDA_ARCH__
+  const longlong2 v = __ldg((const longlong2 *)p);
+  return {v.x, v.y};
+#else
+  return {p[0], p[1]};
+#endif
+}
+ECPGB_HD i64 ld_one(const i64 *p) {
+#ifdef __CUDA_ARCH__
+  return __ldg(p);
+#else
+  return *p;
+#endif
+}
+
+// 100 z for z = f * r, f already times 100 (xf_times100): the argument of fx_bessel_rows.
+ECPGB_HD xf xf_times100(xf f) { return {mul_hi(f.m, 100ull << 57), f.e + 7}; }
+
+// K_0..K_lmax(z), each times mul (mul.m = 0: times 1) with the sign bit
+// `sign`, rounded to double.  z100 = 100 z (the reference's table step is 1/100).
+// The branches of src/bessel.c:102-199 in fixed point: the 5-term Taylor
+// polynomial about the nearest table point (z < 16) and the large-argument
+// polynomial are both one Horner pass per row over 64-bit coefficients
+// (besX, besXA), so lanes on either branch run the same instructions.  The
+// small-argument branch (z < 1e-7) agrees with the first table point's
+// polynomial to 1e-14 of K_0 and needs no code; z = 0 gives exactly (1, 0, ...).
+ECPGB_HD void fx_bessel_rows(const i64 *besX, const i64 *besXA, int HL1, int lmax, xf z100, xf mul, uint32_t sign,
+                             double *K) {
+  if (__builtin_expect(z100.m == 0, 0)) {  // rare: a shell on the ECP centre
+    K[0] = mul.m ? xf_to_double(mul.m, mul.e, sign) : 1.0;
+    for (int l = 1; l <= lmax; l++) K[l] = 0.0;
+    return;
+  }
+  z100 = xf_norm(z100);
+  const int sh = -(z100.e + 52);  // 100 z in Q52 = z100.m >> sh; sh < 0 only above 1600
+  u64 W = sh < 0 ? ~0ull : shr64(z100.m, sh);
+  const bool asy = W >= 1600ull << 52;
+  const i64 *q;
+  int rowStride, scaleAt;
+  u64 X;
+  xf am = {0, 0};
+  if (asy) {
+    am.m = mul_hi(fx_recip(z100.m), 50ull << 58);  // a = 1/(2z) = 50 / z100
+    am.e = -120 - z100.e;
+    const int s = am.e + 68;  // 16 a in Q64
+    X = s > 0 ? am.m << 1 : shr64(am.m, -s);
+    X = X < (1ull << 63) - 1 ? X : (1ull << 63) - 1;
+    q = besXA;
+    rowStride = 16;
+    scaleAt = 15;
+  } else {
+    W += 1ull << 51;
+    X = (W & ((1ull << 52) - 1)) << 11;
+    q = besX + (size_t)(W >> 52) * HL1 * 8;
+    rowStride = 8;
+    scaleAt = 6;
+  }
+  const fxmul x = fx_split(X);
+  for (int l = 0; l <= lmax; l++, q += rowStride) {
+    i64 v = 0;
+    for (int k = asy ? l : 5; k > 5; k--) v = ld_one(q + k) + mul_hi_s(v, x);
+    const fxpair c45 = ld_pair(q + 4), c23 = ld_pair(q + 2), c01 = ld_pair(q);
+    v = c45.y + mul_hi_s(v, x);
+    v = c45.x + mul_hi_s(v, x);
+    v = c23.y + mul_hi_s(v, x);
+    v = c23.x + mul_hi_s(v, x);
+    v = c01.y + mul_hi_s(v, x);
+    v = c01.x + mul_hi_s(v, x);
+    xf k = xf_norm({v > 0 ? (u64)v : 0ull, -(int)ld_one(q + scaleAt)});
+    if (asy) k = xf_mul(k, am);
+    if (mul.m) k = xf_mul(k, mul);
+    K[l] = xf_to_double(k.m, k.e, sign);
+  }
+}
+
+// x in Q53 (fixed point) for |x| < 1023; saturates beyond.
+ECPGB_HD i64 fx_q53(double x) {
+  const u64 b = (u64)dbits(x);
+  const int e = (int)(b >> 52) & 0x7ff;
+  const u64 m = (b & ((1ull << 52) - 1)) | (1ull << 52);
+  const int sh = e - 1022;  // value = m 2^(e - 1075)
+  const i64 v = sh > 10 ? 0x7fe0000000000000ll : sh >= 0 ? (i64)(m << sh) : (i64)shr64(m, -sh);
+  return (i64)b < 0 ? -v : v;
+}
+
+// A signed sum of terms +-m 2^e: 60-bit mantissa, aligned to the larger
+// exponent, never renormalised upwards (cancelled bits stay cancelled).
+struct xf_sum {
+  i64 m = 0;
+  int e = -100000;
+  ECPGB_HD void add(xf t, uint32_t sign) {
+    i64 tm = (i64)(t.m >> 4);
+    t.e += 4;
+    if (sign) tm = -tm;
+    const int d = e - t.e;
+    if (d >= 0) tm >>= (d > 63 ? 63 : d);
+    else {
+      m >>= (d < -63 ? 63 : -d);
+      e = t.e;
+    }
+    m += tm;
+    if ((m ^ (m << 1)) < 0) {  // room for the next term
+      m >>= 1;
+      e++;
+    }
+  }
+  ECPGB_HD double value() const {
+    return xf_to_double(m < 0 ? (u64)-m : (u64)m, e, m < 0 ? 0x80000000u : 0u);
+  }
+};
+
+}  // namespace ecpgb

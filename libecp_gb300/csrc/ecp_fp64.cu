@@ -30,8 +30,7 @@ namespace ecpgb {
 
 // ------------------------------------------------------------- small kernels
 
-__global__ void k_radius(DevJob J) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
+static __device__ void radius_of(const DevJob &J, int s) {
   if (s >= J.nShells) return;
   const double *a = J.primA + J.shP[s], *d = J.primD + J.shP[s];
   double zeta = a[0], c = fabs(d[0]);
@@ -42,11 +41,13 @@ __global__ void k_radius(DevJob J) {
   J.radius[s] = r < 0 ? -1.0 : sqrt(r);
 }
 
-__global__ void __launch_bounds__(128) k_centre(DevJob J) {
+__global__ void k_radius(DevJob J) { radius_of(J, blockIdx.x * blockDim.x + threadIdx.x); }
+
+static __device__ void centre_of(const DevJob &J, int c) {
   extern __shared__ double sU[];  // (L+1) x 383
   __shared__ int sEnd[kMaxLEcp + 1];
   __shared__ int sBest;
-  const int c = blockIdx.x, L = J.ctrL[c], O = kSmallOrder;
+  const int L = J.ctrL[c], O = kSmallOrder;
   for (int n = threadIdx.x; n < O; n += blockDim.x) {
     double r = J.xSmall[n];
     for (int l = 0; l <= L; l++) sU[l * O + n] = eval_ecp(J, c, l, r);
@@ -82,10 +83,11 @@ __global__ void __launch_bounds__(128) k_centre(DevJob J) {
   if (threadIdx.x == 0) J.gridEnd[c] = end;
 }
 
-__global__ void __launch_bounds__(64) k_centre_atom(DevJob J) {
+__global__ void __launch_bounds__(128) k_centre(DevJob J) { centre_of(J, blockIdx.x); }
+
+static __device__ void centre_atom_of(const DevJob &J, int A, int c) {
   __shared__ double rsh[169];
   __shared__ double g[4];
-  const int A = blockIdx.x, c = blockIdx.y;
   const int C = J.ctrAtom[c];
   // the atom's largest l, plus the derivative order whose shifts raise it
   // (src/libecp.c:285-286, :292-293)
@@ -128,6 +130,23 @@ __global__ void __launch_bounds__(64) k_centre_atom(DevJob J) {
       v += rsh[lam * lam + mu] * J.omega[(size_t)lm * inc2 + (lam * lam + mu) * inc1 + cart];
     J.ang[((ca * J.angLam + lam) * J.angLM + lm) * J.angC + cart] = v;
   }
+}
+
+__global__ void __launch_bounds__(64) k_centre_atom(DevJob J) { centre_atom_of(J, blockIdx.x, blockIdx.y); }
+
+// The three stages above in one launch (the batched path): centres, (centre,
+// atom) pairs, then shells 128 a CTA.  errWord[1] is cleared before the launch
+// (the shells set it), errWord[0] here.
+__global__ void __launch_bounds__(128) k_stage1(DevJob J) {
+  int b = blockIdx.x;
+  if (b == 0 && threadIdx.x == 0) J.errWord[0] = INT_MAX;
+  if (b < J.nCentres) {
+    centre_of(J, b);
+    return;
+  }
+  b -= J.nCentres;
+  if (b < J.nCentres * J.nAtoms) centre_atom_of(J, b % J.nAtoms, b / J.nAtoms);
+  else radius_of(J, (b - J.nCentres * J.nAtoms) * 128 + threadIdx.x);
 }
 
 __global__ void __launch_bounds__(128) k_shell_F(DevJob J) {
@@ -737,6 +756,12 @@ void launch_prologue(const DevJob &J, cudaStream_t st, bool withF) {
   k_centre<<<J.nCentres, 128, sizeof(double) * kSmallOrder * (kMaxLEcp + 1), st>>>(J);
   k_centre_atom<<<dim3(J.nAtoms, J.nCentres), 64, 0, st>>>(J);
   if (withF) k_shell_F<<<dim3(J.nShells, J.nCentres), 128, 0, st>>>(J);
+}
+
+void launch_stage1(const DevJob &J, cudaStream_t st) {
+  cudaMemsetAsync(J.errWord + 1, 0, sizeof(int), st);
+  k_stage1<<<J.nCentres * (1 + J.nAtoms) + (J.nShells + 127) / 128, 128,
+             sizeof(double) * kSmallOrder * (kMaxLEcp + 1), st>>>(J);
 }
 
 void launch_epilogue(const DevJob &J, cudaStream_t st) {

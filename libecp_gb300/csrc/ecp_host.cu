@@ -218,6 +218,7 @@ struct DevTables {
   DBuf<double> xs, ws, xl, wl, besT, besC, besH, besA, besZ, shNorm, p2s, fac, dfac, omega, c2s;
   DBuf<int> ijk, ijkIdx, itemOff, itemCnt, items, s93, s92;
   DBuf<short> byN93;
+  DBuf<long long> besX, besXA;  // fixed-point Bessel rows
   int nItemsMax = 0;
 };
 
@@ -297,7 +298,8 @@ struct Engine {
               t->ijkIdx.upload(h.ijkIndex, stream) && t->besH.upload(h.besselH, stream) && t->besA.upload(h.besselA, stream) && t->besHf.upload(h.besselHf, stream) &&
               t->besAf.upload(h.besselAf, stream) && t->besZf.upload(h.besselZf, stream) &&
               t->xlf.upload(h.xlf, stream) && t->wlf.upload(h.wlf, stream) &&
-              t->besZ.upload(h.besselZ, stream) &&
+              t->besZ.upload(h.besselZ, stream) && t->besX.upload(h.besselX, stream) &&
+              t->besXA.upload(h.besselXA, stream) &&
               t->c2s.upload(h.cart2sph, stream) && t->s93.upload(h.s93.slot, stream) &&
               t->s92.upload(h.s92.slot, stream) && t->byN93.upload(by_point_order(h.s93.slot), stream) &&
               t->shNorm.upload(h.shNorm, stream);
@@ -426,103 +428,148 @@ void free_retired_pinned() {
 
 bool valid_mode(int mode) { return mode == ECPGB_FP64 || mode == ECPGB_FAST || mode == ECPGB_MIXED; }
 
-// The class-major work queue: units grouped by their (la, lb, L) class --
-// largest la + lb first, then la, then the centre's L descending -- and
-// within a class by descending estimated cost, ties in the reference's order.
-// Concurrent CTAs then mostly run units of one class, i.e. the same code
-// paths and table widths.  Empty when the units do not fit 31-bit indices.
-static void unit_order_class(const Parsed &P, std::vector<int> &order) {
-  order.clear();
-  const long long n = (long long)P.nCentres * P.nPairs;
-  if (n <= 0 || n >= INT_MAX) return;
-  // two stable counting sorts (least significant key first): by descending
-  // cost, then by class
-  std::vector<int> pc(P.nPairs), cc(P.nCentres), pcls(P.nPairs);
-  int maxP = 0, maxC = 0, LB = 0, LE = 0;
-  for (int c = 0; c < P.nCentres; c++) { cc[c] = P.ctrL[c] + 2; maxC = std::max(maxC, cc[c]); LE = std::max(LE, P.ctrL[c]); }
-  for (int p = 0; p < P.nPairs; p++) {
-    const int a = P.pairA[p], b = P.pairB[p];
-    pc[p] = P.shK[a] * P.shK[b] * (P.shL[a] + P.shL[b] + 2);
-    maxP = std::max(maxP, pc[p]);
-    LB = std::max(LB, std::max(P.shL[a], P.shL[b]));
-  }
-  const long long nCost = (long long)maxP * maxC + 1;
-  if (nCost > (1 << 24)) return;
-  const int W1 = LB + 1, W2 = LE + 1, nCls = (2 * LB + 1) * W1 * W2;
-  for (int p = 0; p < P.nPairs; p++) {
-    const int la = P.shL[P.pairA[p]], lb = P.shL[P.pairB[p]];
-    pcls[p] = ((2 * LB - la - lb) * W1 + (LB - la)) * W2;  // + (LE - L) per centre
-  }
-  std::vector<int> tmp(n);
-  std::vector<int> start(std::max<long long>(nCost, nCls) + 1);
-  // pass 1: by descending cost, ties in the reference's order
-  std::fill(start.begin(), start.begin() + nCost + 1, 0);
-  for (int c = 0; c < P.nCentres; c++)
-    for (int p = 0; p < P.nPairs; p++) start[nCost - 1 - (long long)pc[p] * cc[c]]++;
-  for (long long k = 0, acc = 0; k <= nCost; k++) { const int v = start[k]; start[k] = (int)acc; acc += v; }
-  for (int c = 0; c < P.nCentres; c++)
-    for (int p = 0; p < P.nPairs; p++) tmp[start[nCost - 1 - (long long)pc[p] * cc[c]]++] = c * P.nPairs + p;
-  // pass 2: by class, stable
-  auto cls = [&](int u) { const int c = u / P.nPairs; return pcls[u % P.nPairs] + (LE - P.ctrL[c]); };
-  std::fill(start.begin(), start.begin() + nCls + 1, 0);
-  for (long long i = 0; i < n; i++) start[cls(tmp[i])]++;
-  for (int k = 0, acc = 0; k <= nCls; k++) { const int v = start[k]; start[k] = acc; acc += v; }
-  order.resize(n);
-  for (long long i = 0; i < n; i++) order[start[cls(tmp[i])]++] = tmp[i];
+// Items of the type-2 radial table per (la, lb) over channels l < L.
+static int class_item_count(int la, int lb, int L) {
+  static const std::vector<int> n = [] {
+    std::vector<int> v, tmp;
+    for (int a = 0; a <= kMaxLBasis; a++)
+      for (int b = 0; b <= kMaxLBasis; b++) {
+        int tot = 0;
+        for (int l = 0; l < kMaxLEcp; l++) {
+          used_triples(a, b, l, tmp);
+          v.push_back(tot += (int)tmp.size());
+        }
+      }
+    return v;
+  }();
+  return L > 0 ? n[(la * (kMaxLBasis + 1) + lb) * kMaxLEcp + L - 1] : 0;
 }
 
-// The work queue of the batched path: units by descending estimated cost,
-// primitive pairs x (la + lb + 2) x (L + 2), ties in the reference's order
-// (a stable counting sort).  Empty when the units do not fit 31-bit indices.
-static void unit_order(const Parsed &P, std::vector<int> &order) {
-  order.clear();
-  const long long n = (long long)P.nCentres * P.nPairs;
-  if (n <= 0 || n >= INT_MAX) return;
-  std::vector<int> pk(P.nPairs), ck(P.nCentres);
-  int maxP = 0, maxC = 0;
+// The l of a pair entry's shells after its derivative shift (may be -1).
+static void shifted_l(const Parsed &P, int p, int &la, int &lb) {
+  int ha = 0, hb = 0;
+  if (P.deriv) shift_pair(P.deriv, P.pairShift[p], ha, hb);
+  la = P.shL[P.pairA[p]] + ha;
+  lb = P.shL[P.pairB[p]] + hb;
+}
+
+static PairPlan plan_of_pair(const Parsed &P, int p) {
+  int la, lb;
+  shifted_l(P, p, la, lb);
+  const int LE = P.maxLECP > 0 ? P.maxLECP : 1;
+  return pair_plan(P.shK[P.pairA[p]] * P.shK[P.pairB[p]], la, lb, la < 0 || lb < 0 ? 0 : class_item_count(la, lb, LE));
+}
+
+// Scratch of a batched job with chunks of at most `cap` bytes (at least one
+// pair's units a chunk).
+static size_t scratch_bytes(const Parsed &P, size_t cap) {
+  size_t tot = 0, one = 0;
   for (int p = 0; p < P.nPairs; p++) {
-    int a = P.pairA[p], b = P.pairB[p];
-    pk[p] = P.shK[a] * P.shK[b] * (P.shL[a] + P.shL[b] + 2);
-    maxP = std::max(maxP, pk[p]);
+    const PairPlan q = plan_of_pair(P, p);
+    const size_t b = (size_t)P.nCentres * (q.scratch + q.lists);
+    tot += b;
+    one = std::max(one, b);
   }
-  for (int c = 0; c < P.nCentres; c++) {
-    ck[c] = P.ctrL[c] + 2;
-    maxC = std::max(maxC, ck[c]);
+  return std::min(tot, std::max(cap, one));
+}
+
+// The queue orders of a batched job -- shell pairs in the reference's order,
+// by descending estimated cost, and class-major (largest la + lb first, then
+// la; within a class by that cost), ties in the reference's order; every
+// pair's units consecutive, centres by descending L -- and their chunks.
+static void make_plan(const Parsed &P, size_t cap, JobPlan &plan, std::vector<int> &orders,
+                      std::vector<long long> &offs, std::vector<int> &chunkPairs, std::vector<int> &ctr) {
+  const int n = P.nPairs;
+  std::vector<int> cost(n), cls(n);
+  std::vector<PairPlan> pp(n);
+  for (int p = 0; p < n; p++) {
+    const int a = P.pairA[p], b = P.pairB[p], la = P.shL[a], lb = P.shL[b];
+    cost[p] = P.shK[a] * P.shK[b] * (la + lb + 2);
+    cls[p] = (2 * kMaxLBasis - la - lb) * (kMaxLBasis + 1) + kMaxLBasis - la;
+    pp[p] = plan_of_pair(P, p);
   }
-  const long long nk = (long long)maxP * maxC + 1;
-  if (nk > (1 << 24)) return;
-  std::vector<int> start(nk + 1, 0);
-  for (int c = 0; c < P.nCentres; c++)
-    for (int p = 0; p < P.nPairs; p++) start[nk - 1 - pk[p] * ck[c]]++;
-  int acc = 0;
-  for (long long k = 0; k <= nk; k++) {
-    int v = start[k];
-    start[k] = acc;
-    acc += v;
+  ctr.resize(P.nCentres);
+  for (int c = 0; c < P.nCentres; c++) ctr[c] = c;
+  std::stable_sort(ctr.begin(), ctr.end(), [&](int a, int b) { return P.ctrL[a] > P.ctrL[b]; });
+  orders.resize(3 * (size_t)n);
+  offs.resize(3 * (size_t)(n + 1));
+  chunkPairs.clear();
+  plan.bytes = 0;
+  // a stable counting sort by cost serves both sorted orders
+  std::vector<int> byCost(n), start;
+  int top = 0;
+  for (int p = 0; p < n; p++) top = std::max(top, cost[p]);
+  start.assign(top + 2, 0);
+  for (int p = 0; p < n; p++) start[top - cost[p] + 1]++;
+  for (int k = 0; k <= top; k++) start[k + 1] += start[k];
+  for (int p = 0; p < n; p++) byCost[start[top - cost[p]]++] = p;
+  for (int o = 0; o < 3; o++) {
+    int *ord = orders.data() + (size_t)o * n;
+    if (o == 0) {
+      for (int p = 0; p < n; p++) ord[p] = p;
+    } else if (o == 1) {
+      std::copy(byCost.begin(), byCost.end(), ord);
+    } else {
+      std::vector<int> st((2 * kMaxLBasis + 1) * (kMaxLBasis + 1) + 1, 0);
+      for (int p = 0; p < n; p++) st[cls[p] + 1]++;
+      for (size_t k = 1; k < st.size(); k++) st[k] += st[k - 1];
+      for (int i = 0; i < n; i++) ord[st[cls[byCost[i]]]++] = byCost[i];
+    }
+    long long *off = offs.data() + (size_t)o * (n + 1);
+    JobPlan::Order &O = plan.order[o];
+    O.chunks.clear();
+    O.chunkAt = (int)chunkPairs.size();
+    long long at = 0, lists = 0;
+    JobPlan::Chunk ch{0, 0, 0, 0, 0, 0, 0};
+    const long long nc = P.nCentres;
+    auto close = [&](int p) {
+      ch.p1 = p;
+      ch.scratch = at - ch.base;
+      O.chunks.push_back(ch);
+      chunkPairs.push_back(ch.p0);
+      plan.bytes = std::max(plan.bytes, (size_t)(ch.scratch + lists));
+      ch = {p, 0, at, 0, 0, 0, 0};
+      lists = 0;
+    };
+    for (int i = 0; i < n; i++) {
+      const PairPlan &q = pp[ord[i]];
+      if (i > ch.p0 && (size_t)(at - ch.base + lists + nc * (q.scratch + q.lists)) > cap) close(i);
+      off[i] = at;
+      at += nc * q.scratch;
+      lists += nc * q.lists;
+      ch.groups += nc * q.groups;
+      ch.batches += nc * q.batches;
+      ch.parts += nc * q.parts;
+    }
+    off[n] = at;
+    if (n) close(n);
   }
-  order.resize(n);
-  for (int c = 0; c < P.nCentres; c++)
-    for (int p = 0; p < P.nPairs; p++) order[start[nk - 1 - pk[p] * ck[c]]++] = c * P.nPairs + p;
 }
 
 // Packs the inputs into the pinned staging buffer, copies them to the device
 // and fills the DevJob's input and work pointers.
-size_t job_device_bytes(const Parsed &P, int mode) {
+size_t job_device_bytes(const Parsed &P, int mode, size_t budget, size_t *scratchCap) {
   const size_t nc = P.nCentres, ns = P.nShells, na = P.nAtoms, O = kSmallOrder;
   const size_t LE = P.maxLECP > 0 ? P.maxLECP : 1, LB = P.maxLBS + P.deriv;
   const size_t nk = std::max(LB + LE, 2 * LB) + 1, nF = LB + LE + 1, D = LB + 1;  // table ranks (upper bounds)
   const size_t angLam = P.maxLECP + LB + 1, angC = (LB + 1) * (LB + 2) * (LB + 3) / 6;
   size_t in = 8 * (P.geom.size() + P.primA.size() + P.primD.size() + 3 * P.termL.size() + P.pairOff.size()) +
               4 * (5 * P.shL.size() + P.atomMaxL.size() + 4 * P.ctrAtom.size() + P.termL.size() + 3 * P.pairA.size()) +
-              (mode != ECPGB_FP64 ? 8 * nc * P.nPairs : 0) + (mode == ECPGB_MIXED ? 16 * P.termL.size() : 0) +
+              (mode != ECPGB_FP64 ? 36 * (P.nPairs + 1) + 4 * nc : 0) + (mode == ECPGB_MIXED ? 16 * P.termL.size() : 0) +
               24 * 256;
   size_t work = 8 * (ns + nc * O * LE * nk + nc * O + nc * ns * (1 + P.deriv) * O * nF + nc * na * 4 + nc * na * D * D * D +
                      nc * na * angLam * LE * LE * angC + nc * (size_t)P.centreStride + (size_t)P.dim * P.dim) +
                 4 * (nc + nc * ns * 3 + nc * (size_t)P.nPairs + 2) + 8;
-  return in + work;
+  if (mode == ECPGB_FP64) return in + work;
+  // the scratch between the stages takes what the budget leaves: a job whose
+  // other buffers fit is never refused for it
+  const size_t base = in + work, cap = base < budget ? std::min(kScratchCap, budget - base) : 0;
+  if (scratchCap) *scratchCap = cap;
+  return base > budget ? base : std::min(budget, base + scratch_bytes(P, cap));
 }
 
-int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int mode, cudaStream_t stream) {
+int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int mode, cudaStream_t stream,
+              size_t scratchCap) {
   const HostTables &h = T->host;
   std::memset(&J, 0, sizeof J);
   J.nAtoms = P.nAtoms; J.nShells = P.nShells; J.nPrims = P.nPrims; J.nCentres = P.nCentres;
@@ -535,7 +582,6 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.angC = ncum(h.maxLBS);
   J.uspD = h.maxLBS + 1;
   J.largeOrder = (int)h.xl.size();
-  for (int k : P.shK) J.maxNP = std::max(J.maxNP, k * k);
   J.tol = P.tol; J.acc = P.acc;
   J.lnAcc1 = std::log(P.acc) - 2;
   J.lnAcc2 = std::log(1.0E-14) - 2;
@@ -559,12 +605,11 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
          iTL = add(P.termL.data(), 4 * P.termL.size()), iPrA = add(P.pairA.data(), 4 * P.pairA.size()),
          iPrB = add(P.pairB.data(), 4 * P.pairB.size()), iPO = add(P.pairOff.data(), 8 * P.pairOff.size()),
          iPS = add(P.pairShift.data(), 4 * P.pairShift.size());
-  std::vector<int> order, orderClass;
-  if (mode != ECPGB_FP64) {
-    unit_order(P, order);
-    unit_order_class(P, orderClass);
-  }
-  size_t iOrd = add(order.data(), 4 * order.size()), iOrdC = add(orderClass.data(), 4 * orderClass.size());
+  std::vector<int> orders, chunkPairs, ctr;
+  std::vector<long long> offs;
+  if (mode != ECPGB_FP64) make_plan(P, scratchCap, B.plan, orders, offs, chunkPairs, ctr);
+  size_t iOrd = add(orders.data(), 4 * orders.size()), iOff = add(offs.data(), 8 * offs.size()),
+         iChk = add(chunkPairs.data(), 4 * chunkPairs.size()), iCtr = add(ctr.data(), 4 * ctr.size());
   // the ECP terms' exponents and coefficients as float pairs (mixed path)
   std::vector<float> tAf, tDf;
   if (mode == ECPGB_MIXED) {
@@ -593,8 +638,6 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.termDf = mode == ECPGB_MIXED ? (const ff *)dp(iTDf) : nullptr;
   J.deriv = P.deriv;
   J.nRuns = 1 + P.deriv;
-  J.order = order.empty() ? nullptr : (const int *)dp(iOrd);
-  J.orderClass = orderClass.empty() ? nullptr : (const int *)dp(iOrdC);
   J.centreStride = P.centreStride;
   // --- tables
   J.itemOff = T->itemOff.p; J.itemCnt = T->itemCnt.p; J.items = T->items.p;
@@ -608,28 +651,40 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
             B.cgeo.ensure(nc * na * 4 + 1) && B.usp.ensure(nc * na * J.uspD * J.uspD * J.uspD + 1) &&
             B.ang.ensure(nc * na * (size_t)J.angLam * J.angLM * J.angC + 1) &&
             B.out.ensure(nc * (size_t)P.centreStride + 1) && B.status.ensure(nc * (size_t)P.nPairs + 1) &&
-            B.mat.ensure((size_t)P.dim * P.dim + 1) && B.err.ensure(2) && B.head.ensure(1);
+            B.mat.ensure((size_t)P.dim * P.dim + 1) && B.err.ensure(16);
   if (!ok) {
     set_error("device allocation failed for the job's work arrays");
     return -1;
   }
   J.radius = B.radius.p; J.utab = B.utab.p; J.uL = B.uL.p; J.gridEnd = B.gridEnd.p; J.win = B.win.p;
   J.F = B.F.p; J.cgeo = B.cgeo.p; J.usp = B.usp.p; J.ang = B.ang.p; J.out = B.out.p;
-  J.status = B.status.p; J.mat = B.mat.p; J.errWord = B.err.p; J.queueHead = B.head.p;
-  if (mode != ECPGB_FP64) {  // screening stage buffers of the batched path
+  J.status = B.status.p; J.mat = B.mat.p; J.errWord = B.err.p;
+  if (mode != ECPGB_FP64) {  // the batched path's plan, scratch and screening stage
     const size_t nu = nc * (size_t)P.nPairs;
-    if (!B.live.ensure(nu + 1) || !B.screenBlocks.ensure(nu / 256 + 2) || !B.liveCount.ensure(1)) {
-      set_error("device allocation failed for the screening stage");
+    size_t chunks = 0;
+    for (const JobPlan::Order &o : B.plan.order) chunks = std::max(chunks, o.chunks.size());
+    if (!B.live.ensure(nu + 1) || !B.screenBlocks.ensure(nu / 256 + 2) || !B.liveStart.ensure(chunks + 1) ||
+        !B.scr.ensure(B.plan.bytes + 16)) {
+      set_error("device allocation failed for the batched path's scratch");
       return -1;
     }
     J.live = B.live.p;
-    J.liveCount = B.liveCount.p;
+    J.liveStart = B.liveStart.p;
     J.screenBlocks = B.screenBlocks.p;
+    J.scr = B.scr.p;
+    J.counters = (unsigned *)(B.err.p + 2);
+    J.plan = &B.plan;
+    J.pairOrders = (const int *)dp(iOrd);
+    J.scrOffs = (const long long *)dp(iOff);
+    J.chunkPairs = (const int *)dp(iChk);
+    J.ctrOrder = (const int *)dp(iCtr);
   }
   J.gcap = FastConfig{}.gcap;
   J.besH = T->besH.p;
   J.besA = T->besA.p;
   J.besZ = T->besZ.p;
+  J.besX = T->besX.p;
+  J.besXA = T->besXA.p;
   J.besHf = (const ff *)T->besHf.p;
   J.besAf = (const ff *)T->besAf.p;
   J.besZf = (const ff *)T->besZf.p;
@@ -638,7 +693,6 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.s93 = T->s93.p;
   J.s92 = T->s92.p;
   J.byN93 = T->byN93.p;
-  J.mixed = mode == ECPGB_MIXED;
   J.besHL = h.besselHL;
   J.shNorm = T->shNorm.p;
   UnitSmem L = unit_smem_layout(h.maxLBS, h.maxLECP, h.nF);
@@ -650,14 +704,14 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
 // batched path with launch configuration cfg).
 int run_pipeline(JobBuffers &B, const DevJob &J, int mode, cudaEvent_t u0, cudaEvent_t u1,
                  const FastConfig *cfg, cudaStream_t stream) {
-  launch_reset(J, stream);
   CUDA_OK(cudaMemsetAsync(B.mat.p, 0, sizeof(double) * (size_t)J.dim * J.dim, stream));
   int rc;
   if (mode == ECPGB_FAST || mode == ECPGB_MIXED) {
     FastConfig c = cfg ? *cfg : engine().config_for(J.maxLBS, J.maxLECP);
     c.mixed = mode == ECPGB_MIXED;
-    rc = launch_fast_pipeline(J, stream, fast_smem_bytes(J.maxLBS, J.maxLECP, c.gcap, J.maxNP), c, u0, u1);
+    rc = launch_fast_pipeline(J, stream, c, u0, u1);
   } else {
+    launch_reset(J, stream);
     rc = launch_fp64_pipeline(J, stream, B.smem, u0, u1);
   }
   if (rc) {
@@ -1089,7 +1143,7 @@ int job_tune(void *vj, ecpgb_launch_config *chosen, ecpgb_launch_config *trials,
   FastConfig bestCfg = R->cfg;
   int n = 0;
   for (const FastConfig &c : cand) {
-    if (fast_ctas_per_sm(fast_smem_bytes(R->J.maxLBS, R->J.maxLECP, c.gcap, R->J.maxNP), c.queue) < 1) continue;
+    if (fast_ctas_per_sm(fast_smem_bytes(R->J.maxLBS, c.gcap)) < 1) continue;
     float tot = 0;
     for (int r = 0; r < 3; r++) {
       cudaMemsetAsync(E.flush.p, r & 0xff, flushBytes, E.stream);
@@ -1196,7 +1250,7 @@ int job_config(void *vj, const ecpgb_launch_config *cfg, ecpgb_launch_config *ou
     c.gcap = cfg->gcap;
     c.balance = cfg->balance ? 1 : 0;
     c.screen = cfg->screen ? 1 : 0;
-    if (fast_ctas_per_sm(fast_smem_bytes(R->J.maxLBS, R->J.maxLECP, c.gcap, R->J.maxNP), c.queue) < 1) {
+    if (fast_ctas_per_sm(fast_smem_bytes(R->J.maxLBS, c.gcap)) < 1) {
       set_error("configuration does not fit on an SM");
       return 1;
     }
@@ -1257,11 +1311,14 @@ long long job_units(const void *vj, long long *emitted) {
 }
 
 int job_launches(const void *vj) {
-  // reset, four per-job stages, the unit kernel, the AO scatter (order 0), and
-  // with the batched queue launch the three screening kernels
   const auto *R = (const ResidentJob *)vj;
-  int n = 6 + (R->P.deriv ? 0 : 1);
-  if (R->mode != ECPGB_FP64 && R->cfg.queue && R->cfg.screen) n += 3;
+  const int scatter = R->P.deriv ? 0 : 1;
+  // reset, four per-job stages, the unit kernel, the AO scatter (order 0)
+  if (R->mode == ECPGB_FP64) return 6 + scatter;
+  // two per-job stages, with the compacted queue the three screening kernels,
+  // the four unit stages per chunk, the scatter
+  int n = 2 + 4 * (int)R->B.plan.order[R->cfg.sorted].chunks.size() + scatter;
+  if (R->cfg.queue && R->cfg.screen) n += 3;
   return n;
 }
 

@@ -130,8 +130,9 @@ struct JobBuffers {
   DBuf<char> in;
   DBuf<double> radius, utab, uL, F, cgeo, usp, ang, out, mat;
   DBuf<int> gridEnd, win, status, err;
-  DBuf<unsigned long long> head, liveCount;
-  DBuf<int> live, screenBlocks;  // screening stage of the batched path
+  DBuf<int> live, screenBlocks, liveStart;  // screening stage of the batched path
+  DBuf<char> scr;                // its scratch between the unit stages
+  JobPlan plan;
   DBuf<double> sout;       // spherical blocks
   DBuf<long long> sphOff;  // their per-entry offsets
   PinnedBuf pinned, pinnedOut;
@@ -141,17 +142,15 @@ struct JobBuffers {
   JobBuffers() { cudaMallocHost((void **)&pinnedErr, 4 * sizeof(int)); }
   // device bytes held by the buffers
   size_t device_bytes() const {
-    return in.cap + 8 * (radius.cap + utab.cap + uL.cap + F.cap + cgeo.cap + usp.cap + ang.cap + out.cap + mat.cap) +
-           4 * (gridEnd.cap + win.cap + status.cap + err.cap + live.cap + screenBlocks.cap) +
-           8 * (head.cap + liveCount.cap);
+    return in.cap + scr.cap + 8 * (radius.cap + utab.cap + uL.cap + F.cap + cgeo.cap + usp.cap + ang.cap + out.cap + mat.cap) +
+           4 * (gridEnd.cap + win.cap + status.cap + err.cap + live.cap + screenBlocks.cap + liveStart.cap);
   }
   // Releases the device buffers (ordered on stream s); they grow again on use.
   void release(cudaStream_t s) {
     in.release(s);
     for (DBuf<double> *b : {&radius, &utab, &uL, &F, &cgeo, &usp, &ang, &out, &mat, &sout}) b->release(s);
-    for (DBuf<int> *b : {&gridEnd, &win, &status, &err, &live, &screenBlocks}) b->release(s);
-    head.release(s);
-    liveCount.release(s);
+    for (DBuf<int> *b : {&gridEnd, &win, &status, &err, &live, &screenBlocks, &liveStart}) b->release(s);
+    scr.release(s);
     sphOff.release(s);
   }
   ~JobBuffers() {
@@ -196,13 +195,17 @@ bool valid_mode(int mode);
 struct DevTables;
 // Packs P's inputs into B's pinned buffer, copies them to the device on
 // `stream` and fills J (B's buffers grow as needed).
-int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int mode, cudaStream_t stream);
+// A batched job's units run in chunks whose scratch stays within scratchCap.
+constexpr size_t kScratchCap = 512ull << 20;
+int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int mode, cudaStream_t stream,
+              size_t scratchCap = kScratchCap);
 // Resets the run's words and launches the pipeline of the mode on `stream`;
 // cfg null = the tuned configuration for the job's (l, L).
 int run_pipeline(JobBuffers &B, const DevJob &J, int mode, cudaEvent_t u0, cudaEvent_t u1,
                  const FastConfig *cfg, cudaStream_t stream);
-// Device bytes a job of P will hold (inputs and work arrays).
-size_t job_device_bytes(const Parsed &P, int mode);
+// Device bytes a job of P will hold (inputs, work arrays, scratch) where at
+// most `budget` may be held; scratchCap: the scratch cap to stage it with.
+size_t job_device_bytes(const Parsed &P, int mode, size_t budget, size_t *scratchCap);
 // With the engine lock held: the tables of the request and, unless requests
 // in flight pin other level schedules (returns 4: retry after they finish),
 // its schedules made current and pinned.  0 ok, 1 error.

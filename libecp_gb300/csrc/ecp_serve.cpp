@@ -11,12 +11,12 @@
 //     others are running overlap on the device;
 //   * completion is read from the slot's last event; the matrix is copied out
 //     of the pinned buffer and the slot is free again;
-//   * continuous batching at unit granularity: in the batched modes a served
-//     job's persistent CTAs each take at most kServeCtaUnits units and exit,
-//     so no job holds the SMs for its whole duration, and jobs below
-//     kSmallUnits units run on high-priority streams, whose pending CTAs the
-//     hardware places before those of the large jobs -- a small request that
-//     arrives while a large one runs starts within one CTA's units.
+//   * continuous batching below the unit: in the batched modes a job's CTAs
+//     are single warps that take a few work-list entries each and exit, so no
+//     job holds the SMs for its whole duration, and jobs below kSmallUnits
+//     units run on high-priority streams, whose pending CTAs the hardware
+//     places before those of the large jobs -- a small request that arrives
+//     while a large one runs starts within one CTA's entries.
 // The basis-independent tables live in the engine and are shared by every
 // job; the level schedules are __constant__ data, so jobs in flight pin them
 // and a job whose large grid differs waits until the pins are released.
@@ -42,7 +42,6 @@ namespace ecpgb {
 
 namespace {
 
-constexpr int kServeCtaUnits = 8;            // units a served job's CTA takes before it exits
 constexpr long long kSmallUnits = 100000;    // (centre, pair) units below which a job is small
 
 double now_ms() {
@@ -54,6 +53,7 @@ struct Request {
   long long id = 0;
   Parsed P;
   size_t need = 0;  // device bytes estimate
+  size_t scratchCap = kScratchCap;
   int state = 0;    // 0 queued, 1 running, 2 done, 3 failed
   int rc = 0;       // like ecpgb_getIntegrals: 0 ok, 2 unit warnings, 1 failure
   std::string err;
@@ -122,9 +122,8 @@ struct Server {
     // buffer growth ordered on the slot's stream: admitting a job never
     // waits for the jobs running on the other slots
     alloc_stream() = s.stream;
-    bool ok = stage_job(r->P, T, s.B, s.J, mode, s.stream) == 0;
+    bool ok = stage_job(r->P, T, s.B, s.J, mode, s.stream, r->scratchCap) == 0;
     alloc_stream() = nullptr;
-    s.J.ctaUnits = kServeCtaUnits;
     ok = ok && cudaEventRecord(s.e0, s.stream) == cudaSuccess;
     ok = ok && run_pipeline(s.B, s.J, mode, nullptr, nullptr, nullptr, s.stream) == 0;
     const size_t mb = sizeof(double) * (size_t)r->P.dim * r->P.dim;
@@ -305,7 +304,7 @@ long long server_submit(void *sv, const ecpgb_system &s) {
     set_error("job has no units");
     return -1;
   }
-  r->need = job_device_bytes(r->P, S->mode);
+  r->need = job_device_bytes(r->P, S->mode, S->budget, &r->scratchCap);
   r->tSubmit = now_ms();
   std::lock_guard<std::mutex> lk(S->mu);
   if (S->stop) {

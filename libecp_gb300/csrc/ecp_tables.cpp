@@ -5,6 +5,7 @@
 // same table values the reference computes.
 #include "ecp_tables.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 
@@ -392,6 +393,7 @@ void build_tables(const TableKey &key, HostTables &t) {
   if (t.maxLECP > 0) omega_table(t);
   else t.omega.assign(1, 0.0);
   bessel_horner(t);
+  bessel_fixed(t);
   const int W = t.tmDim + 1;
   t.shNorm.assign((size_t)W * W, 0.0);
   for (int l = 0; l < W; l++) {
@@ -450,6 +452,50 @@ void bessel_horner(HostTables &t) {
   split_pairs(t.besselH, t.besselHf);
   split_pairs(t.besselA, t.besselAf);
   split_pairs(t.besselZ, t.besselZf);
+}
+
+// Integer coefficients of one polynomial in X in [0, 1/2]: the largest scale
+// at which every Horner value sum_{j >= k} c_j X^{j-k} stays below 2^62.
+static void fixed_row(const long double *c, int deg, long long *out, long long &scale) {
+  long double top = 0.0L, s = 0.0L;
+  for (int k = deg; k >= 0; k--) {
+    s = 0.5L * s + std::fabs(c[k]);
+    top = std::max(top, s);
+  }
+  scale = 0;
+  if (!(top > 1e-300L)) {
+    for (int k = 0; k <= deg; k++) out[k] = 0;
+    return;
+  }
+  scale = 61 - std::ilogb(top);
+  for (int k = 0; k <= deg; k++) out[k] = std::llroundl(std::ldexp(c[k], (int)scale));
+}
+
+void bessel_fixed(HostTables &t) {
+  const int N = t.besselN + 1, HL = t.besselHL, AS = HL + 1 < 6 ? 6 : HL + 1;
+  const long double h = 16.0L / t.besselN;
+  t.besselX.assign((size_t)N * (HL + 1) * 8, 0);
+  for (int i = 0; i < N; i++)
+    for (int l = 0; l <= HL; l++) {
+      const double *q = &t.besselH[((size_t)i * (HL + 1) + l) * 6];
+      // sum_j q_j (h (2 X - 1/2))^j in powers of X
+      long double c[6] = {0, 0, 0, 0, 0, 0}, d[6];
+      for (int j = 5; j >= 0; j--) {  // c = c * (2 h X - h/2) + q_j
+        for (int k = 5; k >= 0; k--) d[k] = (k ? 2 * h * c[k - 1] : 0.0L) - 0.5L * h * c[k];
+        for (int k = 0; k < 6; k++) c[k] = d[k];
+        c[0] += q[j];
+      }
+      long long *out = &t.besselX[((size_t)i * (HL + 1) + l) * 8];
+      fixed_row(c, 5, out, out[6]);
+    }
+  t.besselXA.assign((size_t)(HL + 1) * 16, 0);
+  for (int l = 0; l <= HL; l++) {
+    long double c[16] = {0}, f = 1.0L;
+    const int deg = l > 5 ? l : 5;
+    for (int i = 0; i <= l; i++, f *= -1.0L / 16.0L) c[i] = t.besselA[(size_t)l * AS + i] * f;
+    long long *out = &t.besselXA[(size_t)l * 16];
+    fixed_row(c, deg, out, out[15]);
+  }
 }
 
 void used_triples(int la, int lb, int l, std::vector<int> &out) {

@@ -80,6 +80,13 @@ struct HostTables {
   // max(besselHL + 1, 6), zero beyond i = l.  The coefficients are the integers (l+i)!/((l-i)! i!), the
   // reference's running product divided by i!, so they are exact in FP64.
   std::vector<double> besselA;
+  // The polynomials of besselH and besselA as 64-bit integers for Horner passes
+  // in fixed point (ecp_fixed.h), both in a variable X in [0, 1/2]:
+  // besselX [i][l][8]: X = x / 2, z = z_i + (x - 1/2) h, h = 16/besselN, degree
+  // 5, coefficients in [0..5]; besselXA [l][16]: X = 16 a, coefficients with
+  // their signs in [0..l].  A row's value is v * 2^-scale, the scale in [6]
+  // ([15] of besselXA).
+  std::vector<long long> besselX, besselXA;
   // mixed-precision path: the tables above split into float pairs (hi, lo)
   // with hi + lo = the double to 48 bits (ecp_ff.h), interleaved
   std::vector<float> besselHf, besselAf, besselZf, xlf, wlf;
@@ -96,6 +103,7 @@ struct HostTables {
 // Builds every table for the key.  status != 0 reports a failure.
 void build_tables(const TableKey &key, HostTables &t);
 void bessel_horner(HostTables &t);
+void bessel_fixed(HostTables &t);
 void split_pairs(const std::vector<double> &d, std::vector<float> &out);
 
 // Used triples (l1, l2, l3) of the type-2 radial table for one (la, lb, l):

@@ -5,6 +5,8 @@
   ln2/512 split as L1 + L2, L1 with 32 significant bits (so n * L1 is exact
   for |n| < 2^21), L2 the nearest double to ln2/512 - L1;
   512/ln2 rounded to nearest.
+  For the fixed-point exp (ecp_fixed.h): 2^(j/512) and ln2/512 as integers
+  scaled by 2^62, and what the latter's rounding leaves, scaled by 2^94.
 
 Run from anywhere: python libecp_gb300/csrc/gen_exp2_table.py [output]
 (default output: ecp_exp2_table.h beside this script).
@@ -41,6 +43,16 @@ def main() -> None:
     ]
     for i in range(0, N, 4):
         lines.append("    " + ", ".join(v.hex() for v in vals[i:i + 4]) + ", \\")
+    lines.append("  }")
+    l62 = int(mpmath.nint(step * 2 ** 62))
+    lo = int(mpmath.nint((step * mpmath.mpf(2) ** 62 - l62) * 2 ** 32))
+    assert abs(lo) <= 2 ** 31 - 1
+    lines += [f"#define ECPGB_LN2_512_Q62 {l62}ull  // ln2/512 * 2^62",
+              f"#define ECPGB_LN2_512_Q94LO ({lo})  // the rest, * 2^94",
+              "#define ECPGB_EXP2_TABLE62 \\", "  { \\"]
+    fixed = [int(mpmath.nint(mpmath.power(2, mpmath.mpf(j) / N + 62))) for j in range(N)]
+    for i in range(0, N, 4):
+        lines.append("    " + ", ".join(f"{v}ull" for v in fixed[i:i + 4]) + ", \\")
     lines.append("  }")
     out = sys.argv[1] if len(sys.argv) > 1 else os.path.join(os.path.dirname(os.path.abspath(__file__)),
                                                              "ecp_exp2_table.h")
