@@ -59,20 +59,25 @@ static __device__ __noinline__ void bessel_fx(const DevJob &J, int lmax, xf z100
   fx_bessel_rows(J.besX, J.besXA, J.besHL + 1, lmax, z100, mul, sign, K);
 }
 
-// One ECP term d r^n exp(-a r^2) (R2 = r^2): mantissa and sign; a zero of the
-// smallest exponent (it moves no sum) where the exponential underflows.
-static __device__ inline xf ecp_term_fx(const DevJob &J, int t, double r, xf R, xf R2, uint32_t &sign) {
-  const xf a = xf_mul(xf_from(J.termA[t]), R2);
-  const double d = J.termD[t], n = J.termN[t];
-  sign = sign_of(d);
+// Adds one ECP term d r^n exp(-a r^2) (R2 = r^2) to a channel's sum.  A term
+// below 2^-70 of what the sum holds is left out (the sum carries 60 bits), and
+// one whose exponential underflows.
+static __device__ inline void ecp_term_fx(const DevJob &J, int t, double r, xf R, xf R2, xf_sum &acc) {
+  const xf a = xf_mul(xf_from(J.termA[t]), R2), D = xf_from(J.termD[t]);
+  const double n = J.termN[t];
   const int sh = a.e + 53;  // a r^2 in Q53
   const u64 E = sh < 0 ? shr64(a.m, -sh) : (a.m >> (63 - (sh > 63 ? 63 : sh)) ? ~0ull : a.m << sh);
-  if (E > (u64)(700ll << 53)) return {0, -100000};
-  xf v = xf_mul(fx_exp(-(i64)E), xf_from(d));
-  if (n == 0.0) return v;
-  if (n == 1.0) return xf_mul(v, R);
-  if (n == 2.0) return xf_mul(v, R2);
-  return xf_mul(v, xf_from(rpow(r, n)));  // other powers: rare
+  if (E > (u64)(700ll << 53)) return;
+  // 2^b above the term, b = log2 |d| + log2 r^n - a r^2 log2 e rounded up
+  // (n <= 2; r^n otherwise unknown: never left out)
+  const int rn = n == 0.0 ? 0 : n == 1.0 ? R.e + 64 : n == 2.0 ? R2.e + 64 : 100000;
+  const int b = D.e + 64 + rn - (int)(((u64)(uint32_t)(E >> 32) * 1477) >> 31);
+  if (b < acc.e - 10 + (63 - clz64((u64)(acc.m < 0 ? -acc.m : acc.m) | 1u)) - 60) return;
+  xf v = xf_mul(fx_exp(-(i64)E), D);
+  if (n == 1.0) v = xf_mul(v, R);
+  else if (n == 2.0) v = xf_mul(v, R2);
+  else if (n != 0.0) v = xf_mul(v, xf_from(rpow(r, n)));  // other powers: rare
+  acc.add(v, sign_of(J.termD[t]));
 }
 
 // One row K_l(z), by the same branches as bessel_fx.
@@ -115,16 +120,14 @@ static __device__ __noinline__ void channels_masked(const DevJob &J, int c, doub
   const xf R = xf_from(r), R2 = norm1(xf_mul(R, R));
   const int t0 = J.ctrT0[c], t1 = t0 + J.ctrNT[c];
   unsigned seen = 0;
+#pragma unroll 1
   for (int t = t0; t < t1;) {
     const int l = J.termL[t];
     xf_sum acc;
     const bool use = mask >> l & 1u;
+#pragma unroll 1
     for (; t < t1 && J.termL[t] == l; t++)
-      if (use) {
-        uint32_t sg;
-        const xf v = ecp_term_fx(J, t, r, R, R2, sg);
-        acc.add(v, sg);
-      }
+      if (use) ecp_term_fx(J, t, r, R, R2, acc);
     if (use) {
       const double v = acc.value();
       if (seen >> l & 1u) U[l] += v;
@@ -139,12 +142,9 @@ static __device__ __noinline__ xf channel(const DevJob &J, int c, int l, double 
   const xf R = xf_from(r), R2 = norm1(xf_mul(R, R));
   xf_sum acc;
   const int t0 = J.ctrT0[c], t1 = t0 + J.ctrNT[c];
+#pragma unroll 1
   for (int t = t0; t < t1; t++)
-    if (J.termL[t] == l) {
-      uint32_t sg;
-      const xf v = ecp_term_fx(J, t, r, R, R2, sg);
-      acc.add(v, sg);
-    }
+    if (J.termL[t] == l) ecp_term_fx(J, t, r, R, R2, acc);
   sign = acc.m < 0 ? 0x80000000u : 0u;
   return {acc.m < 0 ? (u64)-acc.m : (u64)acc.m, acc.e};
 }
@@ -311,71 +311,104 @@ static __device__ inline void fm06(double za, double zb, double dAC, double dBC,
 static __device__ inline int step_end93(int s0) { return s0 == 0 ? 33 : s0 + 32; }
 static __device__ inline int step_end92(int s0) { return s0 == 0 ? 31 : s0 + 32; }
 
+// Level constants of both rules as doubles (3 n, 3 N): no conversion per level.
+static __constant__ double c93_3n[32], c92_3N[32];
+
+// The factors of an integrand value, from table entries: mantissa, exponent
+// and sign of a double.
+struct xfs {
+  xf v;
+  uint32_t s;
+};
+static __device__ inline xfs xfs_from(double x) { return {xf_from(x), sign_of(x)}; }
+static __device__ inline xfs operator*(xfs a, xfs b) { return {xf_mul(a.v, b.v), a.s ^ b.s}; }
+
+// A level's end of the PSM92 walk (src/gc_integrators.c:39-86): true when the
+// level's test accepts, with the result.
+static __device__ inline bool psm92_level(int k, double tol16, double I, double p, double q, double &res) {
+  const double N3 = c92_3N[k], e = I - p;
+  // 16 e^2 <= 3 N |I - q| tol
+  if (!(e * e <= N3 * fabs(I - q) * tol16)) return false;
+  res = 16 * I / N3;
+  return true;
+}
+
 // PSM92 walker (src/gc_integrators.c:39-86) over slots [s0, s1) of the
-// large-grid schedule; `val(pos)` = w * f at slot pos; `vis(pos)` whether the
-// (upper) point counts.  State in I, p, q; returns through done/res.
-template <class V, class Vis>
-static __device__ inline void psm92_advance(int s0, int s1, double tol, V val, Vis vis,
+// large-grid schedule; add(pos, sum) adds w * f at slot pos; vis(pos) whether
+// the (upper) point counts.  A level is summed with 60-bit mantissas on the
+// integer pipes and added to the FP64 running sum at its end (and at the end
+// of the slots walked, so that I is complete between calls).
+template <class Add, class Vis>
+static __device__ inline void psm92_advance(int s0, int s1, double tol, Add add, Vis vis,
                                             double &I, double &p, double &q, bool &done, double &res) {
-  int pos = s0;
-  if (pos == 0) {
-    I = val(0);
-    p = I;
-    pos = 1;
-  }
-  int k = level_of(pos);
-  while (pos < s1 && !done) {
-    int lvStart = k == 0 ? 1 : c92_lvEnd[k - 1];
-    if (pos == lvStart) {
+  // one copy of the integrand code: slot 0 is a level of its own
+  xf_sum sum;
+  int k = s0 == 0 ? -1 : level_of(s0);
+  int lvStart = k <= 0 ? 1 : c92_lvEnd[k - 1], lvEnd = k < 0 ? 1 : c92_lvEnd[k];
+#pragma unroll 1
+  for (int t = s0; t < s1 && !done; t++) {
+    if (t == lvStart && k >= 0) {
       q = 2 * p;
       p = 2 * I;
     }
-    double T = 0.0;
-    T += val(pos);
-    if (vis(pos + 1)) T += val(pos + 1);
-    I += T;
-    pos += 2;
-    if (pos == c92_lvEnd[k]) {
-      double N = c92_lvN[k] + 1.0, e = I - p;
-      if (16 * e * e <= 3 * N * fabs(I - q) * tol) {
-        res = 16 * I / (3 * N);
-        done = true;
-      }
+    if ((t & 1) || t == 0 || vis(t)) add(t, sum);  // even slots (after 0) are the upper points
+    if (t + 1 == lvEnd) {
+      I += sum.value();
+      sum = xf_sum();
+      if (k < 0) p = I;
+      else done = psm92_level(k, tol * 0.0625, I, p, q, res);
       k++;
+      lvStart = lvEnd;
+      lvEnd = c92_lvEnd[k];  // k <= the level count, inside the 32-entry table
     }
   }
+  if (sum.m) I += sum.value();
 }
 
 // PS93 walk of ps93_walk (src/gc_integrators.c:157-217) with the error test
-// 16 d / (3 n) < tol written as 16 d < tol 3 n: no divide per level (the
-// same decision but within an ulp of the threshold).
-template <class Fn>
-static __device__ bool ps93_walk_fast(const double *w, int start, int end, double tol, Fn f, double &res) {
-  int mid = c93_slot[0], a = c93_slot[1], b = c93_slot[2];
-  double p = w[mid] * f(mid);
-  double q = w[a] * f(a) + w[b] * f(b);
-  double I = p + q;
-  int pos = 3;
-  for (int k = 0; k < c93_nLevels; k++) {
-    int j = c93_lvJ[k], cnt = 0, e = c93_lvEnd[k];
-    for (; pos < e; pos += 2) {
-      int lo = c93_slot[pos], hi = c93_slot[pos + 1];
-      double T = 0.0;
-      if (lo >= start) { T += w[lo] * f(lo); cnt++; }
-      if (hi <= end) { T += w[hi] * f(hi); cnt++; }
-      I += T;
-    }
-    int n = c93_lvN[k];
-    p += (1 - j) * (I - q);
-    const double d = fabs((1 - j) * (q - 3 * p / 2) + j * (I - 2 * q));
-    q = (1 - j) * q + j * I;
-    if (cnt == 0) continue;
-    if (16 * d < tol * (3 * n)) {
-      res = 16 * q / (3 * n);
-      return true;
-    }
+// 16 d / (3 n) < tol written as d < tol 3 n / 16: no divide per level (the
+// same decision but within an ulp of the threshold); add(n, sum) adds w * f at
+// point n.  Levels are summed as in psm92_advance.  A level's update and
+// test: true when it accepts (cnt points counted).
+static __device__ inline bool ps93_level(int k, double tol16, int cnt, double I, double &p, double &q, double &res) {
+  const double n3 = c93_3n[k];
+  double d;
+  if (c93_lvJ[k]) {
+    d = fabs(I - 2 * q);
+    q = I;
+  } else {
+    p += I - q;
+    d = fabs(q - 3 * p / 2);
   }
-  res = 16 * q / (3 * c93_lvN[c93_nLevels - 1]);  // the last estimate (mixed path: its size)
+  if (cnt == 0 || !(d < tol16 * n3)) return false;
+  res = 16 * q / n3;
+  return true;
+}
+template <class Add>
+static __device__ bool ps93_walk_fast(int start, int end, double tol, Add add, double &res) {
+  // one copy of the integrand code: slot 0 and slots 1, 2 are levels of
+  // their own (-2, -1)
+  xf_sum sum;
+  double p = 0, q = 0, I = 0;
+  int k = -2, lvEnd = 1, cnt = 0;
+#pragma unroll 1
+  for (int t = 0;; t++) {
+    const int n = c93_slot[t];
+    // (the integrand is 0 outside [start, end))
+    if (n >= start && n < end) add(n, sum);
+    cnt += (t & 1) ? n >= start : n <= end;
+    if (t + 1 < lvEnd) continue;
+    const double v = sum.value();
+    sum = xf_sum();
+    I += v;
+    if (k == -2) p = v;
+    else if (k == -1) q = v;
+    else if (ps93_level(k, tol * 0.0625, cnt, I, p, q, res)) return true;
+    if (++k >= c93_nLevels) break;
+    lvEnd = k < 0 ? 3 : c93_lvEnd[k];
+    cnt = 0;
+  }
+  res = 16 * q / c93_3n[c93_nLevels - 1];  // the last estimate (mixed path: its size)
   return false;
 }
 
@@ -383,54 +416,42 @@ static __device__ bool ps93_walk_fast(const double *w, int start, int end, doubl
 // other slots integrate to exactly zero, so (lower, upper) pairs without a set
 // bit are skipped -- adding 0.0 changes no sum -- while every level end is
 // still visited in order for the convergence test.
-template <class V, class Vis>
-static __device__ inline void psm92_sparse(int s0, int s1, const unsigned *bits, double tol, V val,
+template <class Add, class Vis>
+static __device__ inline void psm92_sparse(int s0, int s1, const unsigned *bits, double tol, Add add,
                                            Vis vis, double &I, double &p, double &q, bool &done, double &res) {
-  auto has = [&](int t) { return (bits[t >> 5] >> (t & 31)) & 1u; };
   int pos = s0;
-  if (pos == 0) {
-    I = has(0) ? val(0) : 0.0;
-    p = I;
-    pos = 1;
-  }
-  int k = level_of(pos);
+  xf_sum sum;
+  int k = s0 == 0 ? -1 : level_of(s0);
+#pragma unroll 1
   while (pos < s1 && !done) {
-    const int lvStart = k == 0 ? 1 : c92_lvEnd[k - 1];
-    if (pos == lvStart) {
+    const int lvStart = k <= 0 ? 1 : c92_lvEnd[k - 1], lvE = k < 0 ? 1 : c92_lvEnd[k];
+    if (pos == lvStart && k >= 0) {
       q = 2 * p;
       p = 2 * I;
     }
-    const int lvE = c92_lvEnd[k], stop = lvE < s1 ? lvE : s1;
-    while (true) {
-      int t = stop;  // first set bit in [pos, stop)
-      for (int w = pos >> 5; (w << 5) < stop; w++) {
-        unsigned word = bits[w];
-        if (w == (pos >> 5)) word &= ~0u << (pos & 31);
-        if (word) {
-          t = (w << 5) + __ffs(word) - 1;
-          break;
-        }
+    const int stop = lvE < s1 ? lvE : s1;
+    // every set bit in [pos, stop)
+#pragma unroll 1
+    for (int w = pos >> 5; (w << 5) < stop; w++) {
+      unsigned word = bits[w];
+      if (w == (pos >> 5)) word &= ~0u << (pos & 31);
+      if ((w << 5) + 32 > stop) word &= ~(~0u << (stop & 31));
+#pragma unroll 1
+      for (; word; word &= word - 1u) {
+        const int t = (w << 5) + __ffs(word) - 1;
+        if ((t & 1) || t == 0 || vis(t)) add(t, sum);  // even slots (after 0) are the upper points
       }
-      if (t >= stop) {
-        pos = stop;
-        break;
-      }
-      const int ps = (t - 1) | 1;  // the (lower, upper) pair holding t
-      double T = 0.0;
-      if (has(ps)) T += val(ps);
-      if (has(ps + 1) && vis(ps + 1)) T += val(ps + 1);
-      I += T;
-      pos = ps + 2;
     }
+    pos = stop;
     if (pos == lvE) {
-      double N = c92_lvN[k] + 1.0, e = I - p;
-      if (16 * e * e <= 3 * N * fabs(I - q) * tol) {
-        res = 16 * I / (3 * N);
-        done = true;
-      }
+      I += sum.value();
+      sum = xf_sum();
+      if (k < 0) p = I;
+      else done = psm92_level(k, tol * 0.0625, I, p, q, res);
       k++;
     }
   }
+  if (sum.m) I += sum.value();
 }
 
 // psm92_advance with val(pos) in ff: each level summed with a compensated
@@ -585,6 +606,8 @@ __host__ __device__ inline UnitScratch unit_scratch(int NP, int lab, int nItems)
 struct T1Fail {
   int pos, k;  // queue position, primitive pair (bit 16: double-single tables)
   unsigned mask;
+  int pad;
+  double s;  // |P|
 };
 __host__ __device__ inline size_t unit_list_bytes(int NP, int nItems) {
   return 8 * (size_t)NP + 8 * (size_t)((nItems + 31) / 32) + 8 * (size_t)t2_parts(NP) + sizeof(T1Fail) * (size_t)NP;
@@ -631,7 +654,7 @@ __host__ __device__ inline SmallSmem small_layout(int LB, int cap) {
 // (U[nE], R[nA], Ka[LBE], Kb[LBE]), the walkers' state, the needed-slot bitmap
 // with word prefixes, the pending slots and the failed items.
 struct LargeSmem {
-  int tab, I, P, Q, R, part, bits, pend, pref, fail, total, tabStride;
+  int tab, I, P, Q, part, bits, pend, pref, fail, total, tabStride;
 };
 __host__ __device__ inline LargeSmem large_layout(int LB, int LE) {
   LargeSmem s;
@@ -643,7 +666,6 @@ __host__ __device__ inline LargeSmem large_layout(int LB, int LE) {
   s.I = o; o += kWalkCap;
   s.P = o; o += kWalkCap;
   s.Q = o; o += kWalkCap;
-  s.R = o; o += kWalkCap;
   s.part = o; o += kWalkCap;
   s.bits = o; o += kLargeWords / 2;
   s.pend = o; o += 32;
@@ -872,6 +894,7 @@ static __device__ __noinline__ bool t1_large_entry(const DevJob &J, int c, int L
   sign ^= sign_of(C2) ^ sign_of(w);
   bessel_fx(J, kq, xf_mul(xf_times100(xf_from(s)), R), {0, 0}, 0, K);
   WR[0] = xf_to_double(v.m, v.e, sign);
+#pragma unroll 1
   for (int l = 1; l <= rq; l++) {
     v = norm1(xf_mul(v, R));
     WR[l] = xf_to_double(v.m, v.e, sign);
@@ -907,10 +930,12 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
   double2 *map = (double2 *)(U.scr + U.L.map);
   int4 *win = (int4 *)(U.scr + U.L.win);
   unsigned *mask = (unsigned *)(U.scr + U.L.mask);
+#pragma unroll 1
   for (int w = lane; w < (U.nItems + 31) / 32; w += 32) mask[w] = 0u;
   if (lane == 0) *(UnitHead *)U.scr = {0ull, 0, 0};
   int cnt[3] = {0, 0, 0};
   unsigned kinds = 0;  // the lane's pairs' kinds, 2 bits each (at most 8)
+#pragma unroll 1
   for (int k0 = 0, j = 0; k0 < NP; k0 += 32, j++) {
     const int k = k0 + lane;
     int kind = 3;
@@ -922,14 +947,14 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
       for (int i = 0; i < 3; i++) P[i] = 2.0 * (za * U.gA[i] + zb * U.gB[i]);
       const double s2 = P[0] * P[0] + P[1] * P[1] + P[2] * P[2];
       kind = C1 == 0.0 ? kPairZero : (fabs(C1) < 0x1p-900 || s2 > 2800.0 * (za + zb)) ? kPairBand : kPairNormal;
+      double i1, i2;
+      fm06(za, zb, dAC, dBC, i1, i2);
+      map[k] = make_double2(i1, i2);
       if (U.nItems > 0) {
-        // break index (bisection: the break predicate is monotone in the
-        // index beyond both centres) and the point-index interval outside
-        // which the pair's exponent stays below the screen by a margin of 1:
-        // the exponent is a parabola in r with its vertex at P, and r grows
-        // with the index
-        double i1, i2;
-        fm06(za, zb, dAC, dBC, i1, i2);
+        // break index, and the point-index interval in which the pair's
+        // exponent passes the screen, by bisection: past both centres the
+        // exponent falls with the index; it is a parabola in r with its vertex
+        // at V, and r grows with the index
         auto exq = [&](int n, double &r) {
           r = i1 * J.xLarge[n] + i2;
           const double d1 = dAC - r, d2 = dBC - r;
@@ -943,7 +968,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
           if (r > dAC && r > dBC && e < J.lnAcc2) hi = mid; else lo = mid + 1;
         }
         const int brk = lo < J.largeOrder ? lo : INT_MAX;
-        const double thr = J.lnAcc2 - 1.0, V = (za * dAC + zb * dBC) / (za + zb);
+        const double V = (za * dAC + zb * dBC) / (za + zb);
         int a = 0, b = J.largeOrder;
         while (a < b) {
           const int mid = (a + b) >> 1;
@@ -954,16 +979,15 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
         b = nv;
         while (a < b) {
           const int mid = (a + b) >> 1;
-          if (exq(mid, r) >= thr) b = mid; else a = mid + 1;
+          if (exq(mid, r) >= J.lnAcc2) b = mid; else a = mid + 1;
         }
         const int nLo = a;
         a = nv;
         b = J.largeOrder;
         while (a < b) {
           const int mid = (a + b) >> 1;
-          if (exq(mid, r) < thr) b = mid; else a = mid + 1;
+          if (exq(mid, r) < J.lnAcc2) b = mid; else a = mid + 1;
         }
-        map[k] = make_double2(i1, i2);
         win[k] = make_int4(brk, nLo, a - 1, 0);
       }
     }
@@ -971,6 +995,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
     for (int kd = 0; kd < 3; kd++) cnt[kd] += __popc(__ballot_sync(0xffffffffu, kind == kd));
   }
   int at[3] = {0, cnt[0], cnt[0] + cnt[1]};
+#pragma unroll 1
   for (int k0 = 0, j = 0; k0 < NP; k0 += 32, j++) {
     const int kind = (kinds >> (2 * j)) & 3u;
     for (int kd = 0; kd < 3; kd++) {
@@ -1002,6 +1027,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
                                       (unsigned)(lane == 0 ? nGroups : lane == 1 ? nBatch : nPart));
   const int b1 = __shfl_sync(0xffffffffu, base, 0), b2 = __shfl_sync(0xffffffffu, base, 1),
             b3 = __shfl_sync(0xffffffffu, base, 2);
+#pragma unroll 1
   for (int g = lane; g < nGroups; g += 32) {
     int kd = 0, gj = g, p0 = 0;
     while (gj >= n[kd]) { gj -= n[kd]; p0 += cnt[kd]; kd++; }
@@ -1009,7 +1035,9 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
     const int left = cnt[kd] - gj * G[kd];
     J.listT1[b1 + g] = make_int2(pos, p0 | (left < G[kd] ? left : G[kd]) << 10 | kd << 16);
   }
+#pragma unroll 1
   for (int q = lane; q < nBatch; q += 32) J.listT2[b2 + q] = make_int2(pos, 32 * q);
+#pragma unroll 1
   for (int q = lane; q < nPart; q += 32) J.listPart[b3 + q] = make_int2(pos, q);
 }
 
@@ -1062,8 +1090,10 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
   }
   double *Qout = (double *)(U.scr + U.L.Q) + (size_t)perm[p0 + g] * nq + qi;
   double I = 0, p = 0, q = 0;
+  xf_sum sum;    // the running level (normal kind)
+  double T = 0;  // the running slot pair (band kind)
   bool done = !mine;
-  int k = 0, cnt = 0;
+  int k = -2, cnt = 0, lvEnd = 1;
   if constexpr (kKind == kPairZero) {
     // converged quadratures give 0; failed ones go to the fallback
     if (mine) {
@@ -1071,6 +1101,7 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
       if (done) *Qout = 0.0;
     }
   } else
+#pragma unroll 1
   for (int s0 = 0; s0 < O;) {
     const int s1 = step_end93(s0) < O ? step_end93(s0) : O;
     // slot entry: [0, lq) K_l(s r), [lq, 2lq) w * C1 U_L e^(..) r^l; zero
@@ -1090,6 +1121,7 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
     unsigned live = 0;
     {
       const unsigned run = __ballot_sync(0xffffffffu, !done), qm = nq >= 32 ? ~0u : (1u << nq) - 1u;
+#pragma unroll 1
       for (int gg = 0; gg < G; gg++)
         if (run >> (gg * nq) & qm) live |= 1u << gg;
     }
@@ -1099,10 +1131,12 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
     // multiply-shift: ceil(2^16 / d) is exact for d <= 8 and e < 8192
     // (e < 33 * 8 here) -- no integer divide in the loops
     unsigned packed = 0;
+#pragma unroll 1
     for (unsigned m = live, j = 0; m; m &= m - 1u, j++) packed |= (unsigned)(__ffs(m) - 1) << (4 * j);
     const unsigned dmag = nLive > 0 ? (65536u + (unsigned)nLive - 1u) / (unsigned)nLive : 0u;
     auto slot_of = [&](int e) { return (int)(((unsigned)e * dmag) >> 16); };
     auto live_pair = [&](int e, int i) { return (int)((packed >> (4 * (e - i * nLive))) & 15u); };
+#pragma unroll 1
     for (int e = lane; e < nIn * nLive; e += 32) {
       const int i = slot_of(e);
       const int gg = live_pair(e, i), t = __ldg(J.byN93 + s0 + lo + i), n = __ldg(J.s93 + t);
@@ -1113,6 +1147,7 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
         const double r = J.xSmall[n], ex = t1_exponent(sc[gg * 3 + 2], s, r);
         bessel_fx(J, lab, xf_mul(xf_times100(xf_from(s)), xf_from(r)), {0, 0}, 0, ent);
         double R = 1.0;
+#pragma unroll 1
         for (int l = 0; l <= lab; l++) {
           if (l) R = __dmul_rn(r, R);
           WR[l] = __dmul_rn(__dmul_rn(C1, R), uL[n]);
@@ -1130,12 +1165,14 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
         const int sh = 117 - F.q + R.e;
         E = sh <= 0 ? shr64(E, -sh) : (E >> (63 - (sh > 63 ? 63 : sh)) ? ~0ull >> 1 : E << sh);
         if (tt < 0 && E > thr) {  // below the screen
+#pragma unroll 1
           for (int l = 0; l < 2 * lq; l++) ent[l] = 0.0;
         } else {
           xf v = xf_mul(xf_mul(fx_exp(tt < 0 ? -(i64)E : (i64)E), xf_from(C1)), xf_mul(xf_from(w), xf_from(u)));
           const uint32_t sign = sign_of(w) ^ sign_of(u) ^ sign_of(C1);
           bessel_fx(J, lab, xf_mul({F.sm, F.se}, R), {0, 0}, 0, ent);
           WR[0] = xf_to_double(v.m, v.e, sign);
+#pragma unroll 1
           for (int l = 1; l <= lab; l++) {
             v = norm1(xf_mul(v, R));
             WR[l] = xf_to_double(v.m, v.e, sign);
@@ -1143,9 +1180,11 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
         }
       }
     }
+#pragma unroll 1
     for (int e = lane; e < (ns - nIn) * nLive; e += 32) {
       const int i = slot_of(e), t = __ldg(J.byN93 + s0 + (i < lo ? i : i + nIn));
       double *ent = tab + ((t - s0) * G + live_pair(e, i)) * TS;
+#pragma unroll 1
       for (int l = 0; l <= 2 * lq; l++) ent[l] = 0.0;
     }
     __syncwarp();
@@ -1155,54 +1194,44 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
       const double *e = ent_of(t);
       return __dmul_rn(J.wSmall[n], __dmul_rn(__dmul_rn(e[lq + l1], e[l2]), e[2 * lq]));
     };
-    int t = s0;
-    if (t == 0) {
+    // one copy of the integrand code: slot 0 and slots 1, 2 are levels of
+    // their own (-2, -1)
+#pragma unroll 1
+    for (int t = s0; t < s1; t++) {
+      const int n = c93_slot[t];
+      // the points inside the window (the entries outside it are zero)
+      if (!done && n >= ws && n < we) {
+        if constexpr (kKind == kPairBand) T = __dadd_rn(T, wf(t, n));
+        else {
+          const double *e = ent_of(t);
+          const xfs v = xfs_from(e[lq + l1]) * xfs_from(e[l2]);
+          sum.add(v.v, v.s);
+        }
+      }
+      cnt += (t & 1) ? n >= ws : n <= we;
+      if constexpr (kKind == kPairBand)
+        if (t > 2 && !(t & 1)) {  // the reference's order: pair by pair
+          I += T;
+          T = 0.0;
+        }
+      if (t + 1 < lvEnd) continue;
       if (!done) {
-        if constexpr (kKind == kPairBand) {
-          p = wf(0, c93_slot[0]);
-          q = __dadd_rn(wf(1, c93_slot[1]), wf(2, c93_slot[2]));
-        } else {
-          const double *e0 = ent_of(0), *e1 = ent_of(1), *e2 = ent_of(2);
-          p = e0[lq + l1] * e0[l2];
-          q = fma(e2[lq + l1], e2[l2], e1[lq + l1] * e1[l2]);
+        double v = T;
+        if constexpr (kKind == kPairNormal) v = sum.value();
+        sum = xf_sum();
+        T = 0.0;
+        I += v;
+        double res;
+        if (k == -2) p = v;
+        else if (k == -1) q = v;
+        else if (ps93_level(k, J.tol * 0.0625, cnt, I, p, q, res)) {
+          done = true;
+          *Qout = res;
         }
-        I = p + q;
       }
-      t = 3;
-    }
-    // the current level's first and end slot, read once per level
-    int lvStart = k == 0 ? 3 : c93_lvEnd[k - 1], lvEnd = c93_lvEnd[k];
-    while (t < s1) {
-      if (t == lvStart) cnt = 0;
-      int lo = c93_slot[t], hi = c93_slot[t + 1];
-      double T = 0.0;
-      if constexpr (kKind == kPairBand) {
-        if (lo >= ws) { if (!done) T = wf(t, lo); cnt++; }
-        if (hi <= we) { if (!done) T = __dadd_rn(T, wf(t + 1, hi)); cnt++; }
-      } else {
-        if (lo >= ws) { if (!done) { const double *e = ent_of(t); T = e[lq + l1] * e[l2]; } cnt++; }
-        if (hi <= we) { if (!done) { const double *e = ent_of(t + 1); T = fma(e[lq + l1], e[l2], T); } cnt++; }
-      }
-      if (!done) I += T;
-      t += 2;
-      if (t == lvEnd) {
-        int j = c93_lvJ[k], n = c93_lvN[k];
-        if (!done) {
-          p += (1 - j) * (I - q);
-          // the reference's error estimate is 16 d / (3 n); tested as
-          // 16 d < tol 3 n (no divide; the same decision but within an ulp
-          // of the threshold)
-          const double d = fabs((1 - j) * (q - 3 * p / 2) + j * (I - 2 * q));
-          q = (1 - j) * q + j * I;
-          if (cnt > 0 && 16 * d < J.tol * (3 * n)) {
-            done = true;
-            *Qout = 16 * q / (3 * n);
-          }
-        }
-        k++;
-        lvStart = lvEnd;
-        lvEnd = c93_lvEnd[k];  // k <= the level count, inside the 32-entry table
-      }
+      k++;
+      lvEnd = k < 0 ? 3 : c93_lvEnd[k];  // k <= the level count, inside the 32-entry table
+      cnt = 0;
     }
     __syncwarp();
     s0 = s1;
@@ -1216,21 +1245,22 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
   // last small-grid estimates, by the high words); larger integrals in FP64
   unsigned est = 0, lim = 0;
   if constexpr (kMixed) {
-    est = mine && !done ? (unsigned)((u64)__double_as_longlong(fabs(16 * q / (3 * c93_lvN[c93_nLevels - 1]))) >> 32) : 0u;
+    est = mine && !done ? (unsigned)((u64)__double_as_longlong(fabs(16 * q / c93_3n[c93_nLevels - 1])) >> 32) : 0u;
     lim = (unsigned)((u64)__double_as_longlong(ff_limit(J.tol)) >> 32);
   }
+#pragma unroll 1
   for (int gg = 0; gg < G; gg++) {
     const unsigned m = fail >> (gg * nq) & (nq >= 32 ? ~0u : (1u << nq) - 1u);
     if (!m) continue;
     int ffp = 0;
     if constexpr (kMixed) ffp = __reduce_max_sync(0xffffffffu, g == gg ? est : 0u) < lim;
-    if (lane == 0) J.listFail[atomicAdd(J.counters + kCntFail, 1u)] = {pos, perm[p0 + gg] | ffp << 16, m};
+    if (lane == 0) J.listFail[atomicAdd(J.counters + kCntFail, 1u)] = {pos, perm[p0 + gg] | ffp << 16, m, 0, sc[gg * 3]};
   }
 }
 
 // A batch of 32 type-2 small-grid quadratures (src/type2.c:337-387), one per
 // lane: F tables (derivative runs max(0, shift), src/type2.c:563-564) and the
-// r^k U_l table read through L2, FP64 integrand in every mode.
+// r^k U_l table read through L2, 64-bit mantissas in every mode.
 template <bool kMixed>
 static __device__ void t2_small(const DevJob &J, const Unit &U, int q0) {
   const int q = q0 + (threadIdx.x & 31), O = kSmallOrder;
@@ -1241,9 +1271,11 @@ static __device__ void t2_small(const DevJob &J, const Unit &U, int q0) {
   const double *Fb = J.F + (((size_t)U.c * J.nShells + U.sb) * nRuns + U.pb0) * O * nF + l2;
   const double *Ut = J.utab + (size_t)U.c * O * LE * nk + l * nk + l3;
   double res;
-  const bool ok = ps93_walk_fast(J.wSmall, U.ws, U.we, J.tol,
-                                 [&](int n) {
-                                   return __ldg(Fa + n * nF) * __ldg(Fb + n * nF) * __ldg(Ut + (size_t)n * LE * nk);
+  const bool ok = ps93_walk_fast(U.ws, U.we, J.tol,
+                                 [&](int n, xf_sum &a) {
+                                   const xfs f = (xfs_from(__ldg(Fa + n * nF)) * xfs_from(__ldg(Fb + n * nF))) *
+                                                 (xfs_from(__ldg(Ut + (size_t)n * LE * nk)) * xfs_from(J.wSmall[n]));
+                                   a.add(f.v, f.s);
                                  },
                                  res);
   if (ok) ((double *)(U.scr + U.L.T))[q] = res;
@@ -1256,10 +1288,11 @@ static __device__ void t2_small(const DevJob &J, const Unit &U, int q0) {
 // One warp a CTA; each takes up to J.take entries of the type-1 groups, then
 // of the type-2 batches (one kind of work at a time on the whole GPU).
 template <bool kMixed>
-__global__ void __launch_bounds__(32, 16) k_unit_small(DevJob J) {
+__global__ void __launch_bounds__(32, 20) k_unit_small(DevJob J) {
   extern __shared__ double sm[];
   const SmallSmem L = small_layout(J.maxLBS, J.gcap);
   const int n1 = (int)J.counters[kCntT1], n = n1 + (int)J.counters[kCntT2];
+#pragma unroll 1
   for (int taken = 0; taken < J.take; taken++) {
     const int i = next_item(J.counters + kHeadSmall);
     if (i >= n) return;
@@ -1283,7 +1316,7 @@ __global__ void __launch_bounds__(32, 16) k_unit_small(DevJob J) {
 // The large-grid quadratures of one primitive pair whose small-grid ones
 // (mask, by t1_index) failed (src/type1.c:149-196), one per lane.
 template <bool kMixed>
-static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int kk, bool ffp, unsigned mask) {
+static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int kk, bool ffp, unsigned mask, double s) {
   const int lane = threadIdx.x & 31, lab = U.lab, lq = lab + 1, O = kSmallOrder, OL = J.largeOrder, TSf = 3 + 2 * lq;
   const int Nb = U.Nb, ws = U.ws, we = U.we, c = U.c, Lc = U.Lc;
   const double *uL = J.uL + (size_t)c * O;
@@ -1297,13 +1330,10 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int
   }
   const double za = U.pzA[kk / Nb], ca = zeta_times(U.pcA[kk / Nb], za, U.pa0), zb = U.pzB[kk % Nb],
                cb = zeta_times(U.pcB[kk % Nb], zb, U.pb0);
-  double P[3];
-  for (int i = 0; i < 3; i++) P[i] = 2.0 * (za * U.gA[i] + zb * U.gB[i]);
-  const double s = sqrt(P[0] * P[0] + P[1] * P[1] + P[2] * P[2]);
   const double z = -za - zb, zd2 = -za * dAC * dAC - zb * dBC * dBC;
   const double C2 = ca * cb;
-  double i1, i2;
-  fm06(za, zb, dAC, dBC, i1, i2);
+  const double2 map = ((const double2 *)(U.scr + U.L.map))[kk];
+  const double i1 = map.x, i2 = map.y;
   const ff C2f = ff_from_double(C2), sf = ff_from_double(s), i1f = ff_from_double(i1);
   // first point past both centres whose exponent is below the screen
   // (src/type1.c:168-176).  Past both centres the exponent falls as r
@@ -1321,6 +1351,7 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int
     const unsigned b = __ballot_sync(0xffffffffu, brk(n));
     if (b) {
       const int n0 = (__ffs(b) - 1) * chunk;
+#pragma unroll 1
       for (int c0 = n0; c0 < n0 + chunk && c0 < OL; c0 += 32) {
         const int m = c0 + lane;
         const unsigned b2 = __ballot_sync(0xffffffffu, m < n0 + chunk && m < OL && brk(m));
@@ -1334,11 +1365,13 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int
   const int end = nb - 1;
   double I2 = 0, p2 = 0, q2 = 0, res2 = 0;
   bool done2 = !fail;
+#pragma unroll 1
   for (int s0 = 0; s0 < OL;) {
     const int s1 = step_end92(s0) < OL ? step_end92(s0) : OL;
     // the rows the quadratures still running read
     const int kq = __reduce_max_sync(0xffffffffu, done2 ? 0 : l2);
     const int rq = __reduce_max_sync(0xffffffffu, done2 ? 0 : l1);
+#pragma unroll 1
     for (int t = s0 + lane; t < s1; t += 32) {
       int n = __ldg(J.s92 + t);
       bool upper = t > 0 && ((t - 1) & 1);
@@ -1357,6 +1390,7 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int
             any = v.hi != 0.0f;
             bessel_ff(J, kq, ff_mul(sf, rf), Kf, 1);
             WRf[0] = v;
+#pragma unroll 1
             for (int l = 1; l <= rq; l++) {
               v = ff_mul(v, rf);
               WRf[l] = v;
@@ -1373,15 +1407,18 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int
         if (es >= J.lnAcc1) {
           const double v = w * (C2 * uL[n] * fast_exp(es));
           any = v != 0.0;
+#pragma unroll 1
           for (int l = 0; l <= lab; l++) {
             int f = l * OL + n, lr = f / O, nr = f % O;
             bool ok = lr <= lab && nr >= ws && nr < we;
             double xr = J.xSmall[nr], pw = 1.0;
+#pragma unroll 1
             for (int i = 0; i < lr && ok; i++) pw = xr * pw;
             WR[l] = ok ? v * pw : 0.0;
             K[l] = ok ? bessel_row(J, lr, s * xr) : 0.0;
           }
           if (kMixed && ffp)  // the rows as ff, in place (entry l holds row l either way)
+#pragma unroll 1
             for (int l = 0; l <= lab; l++) {
               ((ff *)WR)[l] = ff_from_double(WR[l]);
               ((ff *)K)[l] = ff_from_double(K[l]);
@@ -1389,7 +1426,9 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int
         }
       }
       if (!any) {  // zero bits read as 0.0 in FP64 and in ff alike
+#pragma unroll 1
         for (int l = 0; l <= kq; l++) K[l] = 0.0;
+#pragma unroll 1
         for (int l = 0; l <= rq; l++) WR[l] = 0.0;
       }
     }
@@ -1403,11 +1442,12 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int
         };
         psm92_advance_ff(s0, s1, J.tol, val, vis, I2, p2, q2, done2, res2);
       } else {
-        auto val = [&](int t) {
+        auto add = [&](int t, xf_sum &a) {
           const double *e = tab + (t - s0) * TSf;
-          return e[lq + l1] * e[l2];
+          const xfs v = xfs_from(e[lq + l1]) * xfs_from(e[l2]);
+          a.add(v.v, v.s);
         };
-        psm92_advance(s0, s1, J.tol, val, vis, I2, p2, q2, done2, res2);
+        psm92_advance(s0, s1, J.tol, add, vis, I2, p2, q2, done2, res2);
       }
     }
     __syncwarp();
@@ -1416,7 +1456,7 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int
   }
   if (fail) {
     if (!done2) {
-      res2 = 16 * I2 / (3 * (c92_lvN[c92_nLevels - 1] + 1.0));
+      res2 = 16 * I2 / c92_3N[c92_nLevels - 1];
       atomicOr(&((UnitHead *)U.scr)->warn, 1);
     }
     ((double *)(U.scr + U.L.Q))[(size_t)kk * t1_items(lab) + lane] = res2;
@@ -1444,7 +1484,7 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
   const int TS = L.tabStride;
   const double *pzA = U.pzA, *pzB = U.pzB;
   const double dAC = U.gA[3], dBC = U.gB[3];
-  double *tab = sm + L.tab, *sI = sm + L.I, *sP = sm + L.P, *sQ = sm + L.Q, *sR = sm + L.R, *part = sm + L.part;
+  double *tab = sm + L.tab, *sI = sm + L.I, *sP = sm + L.P, *sQ = sm + L.Q, *part = sm + L.part;
   const int *fail = (const int *)(sm + L.fail);
   unsigned *needBits = (unsigned *)(sm + L.bits);
   int *pend = (int *)(sm + L.pend), *pref = (int *)(sm + L.pref);
@@ -1452,11 +1492,13 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
   // derivative blocks: the product times zeta_a^max(0, shifta), then
   // zeta_b^max(0, shiftb) (src/type2.c:456-462)
   const double Ck = zeta_times(zeta_times(ca * cb, za, U.pa0), zb, U.pb0);
-  const double i1 = map[k].x, i2 = map[k].y;
+  const double i1 = map[k].x;
   const ff i1f = ff_from_double(i1), Ckf = ff_from_double(Ck);
   const int4 wk = win[k];
   const int nb = wk.x, end = nb == INT_MAX ? OL - 1 : nb - 1, nLo = wk.y, nHi = wk.z;
-  for (int q = lane; q < nf; q += 32) { sI[q] = 0; sP[q] = 0; sQ[q] = 0; sR[q] = 0; }
+#pragma unroll 1
+  for (int q = lane; q < nf; q += 32) { sI[q] = 0; sP[q] = 0; sQ[q] = 0; }
+#pragma unroll 1
   for (int w = lane; w < (OL + 31) / 32; w += 32) needBits[w] = 0u;
   __syncwarp();
   // Whose tables slot t reads (the reference's reused buffers): this pair's
@@ -1468,6 +1510,7 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
     owner = -1;
     if (n < nb) owner = k;
     else if (__builtin_expect(n != nb && !upper, 0)) {
+#pragma unroll 1
       for (int j = k - 1; j >= 0; j--)
         if (win[j].x >= n) { owner = j; break; }
       if (owner >= 0 && win[owner].x == n) owner = -1;
@@ -1497,11 +1540,8 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
       if (t < c1) {
         const int n = __ldg(J.s92 + t);
         if (n < nb) {
-          // this pair's own point: only inside its interval can the exponent pass
-          if (n >= nLo && n <= nHi) {
-            const double r = i1 * J.xLarge[n] + i2, d1 = dAC - r, d2 = dBC - r;
-            need = -za * d1 * d1 - zb * d2 * d2 >= J.lnAcc2;
-          }
+          // this pair's own point: the exponent passes inside its interval
+          need = n >= nLo && n <= nHi;
         } else if (n <= mb && n != nb && !(t > 0 && ((t - 1) & 1))) {
           int owner;
           double r, ex;
@@ -1544,8 +1584,10 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
         for (int side = 0; side < 2; side++)
           bessel_ff(J, side ? pL2 : pL1, ff_mul(ff_from_double(side ? 2.0 * zbj * dBC : 2.0 * zaj * dAC), rf),
                     side ? Kb : Ka, 1);
+#pragma unroll 1
         for (int l = 0; l <= pL1; l++) Ka[l] = ff_mul(Ka[l], wB);
         R[0] = {1.0f, 0.0f};
+#pragma unroll 1
         for (int l = 1; l <= pL3; l++) R[l] = ff_mul(rf, R[l - 1]);
       } else {
         double *Uc = e, *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
@@ -1567,6 +1609,7 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
         }
         R[0] = 1.0;
         xf p = {1ull << 63, -63};
+#pragma unroll 1
         for (int l = 1; l <= pL3; l++) {
           p = norm1(xf_mul(p, Rx));
           R[l] = xf_to_double(p.m, p.e, 0);
@@ -1576,6 +1619,7 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
     if (lane == 0) {  // entry of slot t: queued slots in [wpos, t)
       const int w0 = wpos >> 5, w1 = (b - 1) >> 5;
       int acc = -__popc(needBits[w0] & ((1u << (wpos & 31)) - 1u));
+#pragma unroll 1
       for (int w = w0; w <= w1; w++) {
         pref[w] = acc;
         acc += __popc(needBits[w]);
@@ -1585,6 +1629,7 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
     bool all = true;
     unsigned nMask = 0u;
     int n1 = 0, n2 = 0, n3 = 0;
+#pragma unroll 1
     for (int q = lane, qi = 0; q < nf; q += 32, qi++) {
       if (doneBits[qi] & (1u << lane)) continue;
       // the pass's item, decoded once when the pass was listed
@@ -1603,15 +1648,15 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
         };
         psm92_sparse_ff(wpos, b, needBits, J.tol, val, vis, I, p, qv, done, res);
       } else {
-        auto val = [&](int t) {
-          const double *e = entry(t);
-          const double *Uc = e, *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
-          return Ka[l1] * Kb[l2] * Uc[l] * R[l3];
+        auto add = [&](int t, xf_sum &a) {
+          const double *Uc = entry(t), *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
+          const xfs v = (xfs_from(Ka[l1]) * xfs_from(Kb[l2])) * (xfs_from(Uc[l]) * xfs_from(R[l3]));
+          a.add(v.v, v.s);
         };
-        psm92_sparse(wpos, b, needBits, J.tol, val, vis, I, p, qv, done, res);
+        psm92_sparse(wpos, b, needBits, J.tol, add, vis, I, p, qv, done, res);
       }
       sI[q] = I; sP[q] = p; sQ[q] = qv;
-      if (done) { sR[q] = res; doneBits[qi] |= 1u << lane; }
+      if (done) { sI[q] = res; doneBits[qi] |= 1u << lane; }
       else {
         all = false;
         nMask |= 1u << l;
@@ -1635,10 +1680,11 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
     __syncwarp();
     if (__all_sync(0xffffffffu, all)) break;
   }
-  const double Nlast = c92_lvN[c92_nLevels - 1] + 1.0;
+  const double N3 = c92_3N[c92_nLevels - 1];
+#pragma unroll 1
   for (int q = lane, qi = 0; q < nf; q += 32, qi++) {
-    if (doneBits[qi] & (1u << lane)) part[q] += sR[q];
-    else { part[q] += 16 * sI[q] / (3 * Nlast); warn = 1; }
+    if (doneBits[qi] & (1u << lane)) part[q] += sI[q];
+    else { part[q] += 16 * sI[q] / N3; warn = 1; }
   }
   __syncwarp();
 }
@@ -1664,6 +1710,7 @@ static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem 
   // the latest break of the pairs before the part: beyond it no earlier
   // pair's buffers are reused
   int mb0 = -1;
+#pragma unroll 1
   for (int j = lane; j < k0; j += 32) mb0 = win[j].x > mb0 ? win[j].x : mb0;
   mb0 = __reduce_max_sync(0xffffffffu, mb0);
   int q0 = 0;
@@ -1673,6 +1720,7 @@ static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem 
     unsigned pMask = 0;
     int m1 = 0, m2 = 0, m3 = 0;
     const int first = q0;
+#pragma unroll 1
     for (; q0 < nIt; q0 += 32) {
       const unsigned m = mask[q0 >> 5];
       if (nf + __popc(m) > kWalkCap) break;
@@ -1693,15 +1741,18 @@ static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem 
     S.l1 = __reduce_max_sync(0xffffffffu, m1);
     S.l2 = __reduce_max_sync(0xffffffffu, m2);
     S.l3 = __reduce_max_sync(0xffffffffu, m3);
+#pragma unroll 1
     for (int q = lane; q < nf; q += 32) sum[q] = 0.0;
     __syncwarp();
     int mb = mb0, warn = 0;
+#pragma unroll 1
     for (int k = k0; k < k1; k++) {
       t2_pair<kMixed>(J, U, L, sm, S, k, mb, map, win, useFF, warn);
       mb = win[k].x > mb ? win[k].x : mb;
     }
     if (warn) atomicOr(&((UnitHead *)U.scr)->warn, 2);
     int at = 0;
+#pragma unroll 1
     for (int w = first; w < q0; w += 32) {
       const unsigned m = mask[w >> 5];
       if (m >> lane & 1u) dst[w + lane] = sum[at + __popc(m & ((1u << lane) - 1u))];
@@ -1714,10 +1765,11 @@ static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem 
 // One warp a CTA; the type-2 parts first (the longer ones), then the failed
 // type-1 pairs.
 template <bool kMixed>
-__global__ void __launch_bounds__(32, 12) k_unit_large(DevJob J) {
+__global__ void __launch_bounds__(32, 16) k_unit_large(DevJob J) {
   extern __shared__ double sm[];
   const LargeSmem L = large_layout(J.maxLBS, J.maxLECP);
   const int n2 = (int)J.counters[kCntPart], n = n2 + (int)J.counters[kCntFail];
+#pragma unroll 1
   for (int taken = 0; taken < J.take; taken++) {
     const int i = next_item(J.counters + kHeadLarge);
     if (i >= n) return;
@@ -1728,7 +1780,7 @@ __global__ void __launch_bounds__(32, 12) k_unit_large(DevJob J) {
     } else {
       const T1Fail it = J.listFail[i - n2];
       const Unit U = unit_load(J, it.pos);
-      t1_large<kMixed>(J, U, sm + L.tab, it.k & 0xffff, it.k >> 16, it.mask);
+      t1_large<kMixed>(J, U, sm + L.tab, it.k & 0xffff, it.k >> 16, it.mask, it.s);
     }
   }
 }
@@ -1765,7 +1817,9 @@ __global__ void __launch_bounds__(kLinkThreads) k_unit_link(DevJob J) {
   {
     const double *Q = (const double *)(U.scr + U.L.Q);
     const int nW = NCUM(lab);  // sum over L of (L+1)(L+2)/2 entries (l, m)
+#pragma unroll 1
     for (int e = tid; e < nW; e += NT) W[e] = 0.0;
+#pragma unroll 1
     for (int b0 = 0; b0 < U.NP; b0 += kLinkBatch) {
       const int nb = U.NP - b0 < kLinkBatch ? U.NP - b0 : kLinkBatch;
       __syncthreads();
@@ -1777,11 +1831,13 @@ __global__ void __launch_bounds__(kLinkThreads) k_unit_link(DevJob J) {
         direction(P, dir[3 * tid], dir[3 * tid + 1], dir[3 * tid + 2]);
       }
       __syncthreads();
+#pragma unroll 1
       for (int e = tid; e < nb * lq; e += NT) {
         const int g = e / lq, m = e % lq;
         rsh_column(J, lab, m, dir[3 * g], dir[3 * g + 1], dir[3 * g + 2], rsh + g * RQ);
       }
       __syncthreads();
+#pragma unroll 1
       for (int e = tid; e < nW; e += NT) {
         int Lm1 = 0;
         while (NCUM(Lm1) <= e) Lm1++;
@@ -1789,24 +1845,29 @@ __global__ void __launch_bounds__(kLinkThreads) k_unit_link(DevJob J) {
         while (r >= 2 * l + 1) { r -= 2 * l + 1; l -= 2; }
         const double *q = Q + (size_t)b0 * nq + t1_index(Lm1, l), *s = rsh + l * l + r;
         double v = W[e];
+#pragma unroll 1
         for (int g = 0; g < nb; g++) v += s[g * RQ] * q[(size_t)g * nq];
         W[e] = v;
       }
     }
     __syncthreads();
+#pragma unroll 1
     for (int pi = tid; pi < nW; pi += NT) {
       const int *ex = J.ijk + 3 * pi;
       const int lmax = ex[0] + ex[1] + ex[2];
       const double *p2s = J.p2s + (size_t)J.ijkIdx[(ex[0] * dd + ex[1]) * dd + ex[2]] * tmW;
       const double *w = W + NCUM(lmax - 1);
       double acc = 0.0;
+#pragma unroll 1
       for (int l = lmax; l >= 0; l -= 2) {
+#pragma unroll 1
         for (int m = 0; m < 2 * l + 1; m++) acc += p2s[l * l + m] * w[m];
         w += 2 * l + 1;
       }
       H[pi] = acc;
     }
     __syncthreads();
+#pragma unroll 1
     for (int e = tid; e < nca * ncb; e += NT) {
       const int *ei = J.ijk + 3 * (e / ncb), *ej = J.ijk + 3 * (e % ncb);
       chi[e] = H[J.ijkIdx[((ei[0] + ej[0]) * dd + (ei[1] + ej[1])) * dd + ei[2] + ej[2]]];
@@ -1814,16 +1875,19 @@ __global__ void __launch_bounds__(kLinkThreads) k_unit_link(DevJob J) {
   }
   // the radial table of type 2
   auto tidx = [&](int l, int l1, int l2, int l3) { return ((l * LBE + l1) * LBE + l2) * nA + l3; };
+#pragma unroll 1
   for (int e = tid; e < LE * LBE * LBE * nA; e += NT) T[e] = 0.0;
   __syncthreads();
   {
     const double *Tq = (const double *)(U.scr + U.L.T), *part = (const double *)(U.scr + U.L.part);
     const unsigned *mask = (const unsigned *)(U.scr + U.L.mask);
     const int nParts = t2_parts(U.NP), nIt = class_items(J, U.cls * LE, LE);
+#pragma unroll 1
     for (int q = tid; q < U.nItems; q += NT) {
       double v;
       if (nParts > 1 && (mask[q >> 5] >> (q & 31) & 1u)) {
         v = 0.0;
+#pragma unroll 1
         for (int p = 0; p < nParts; p++) v += part[(size_t)p * nIt + q];
       } else {
         v = Tq[q];
@@ -1836,14 +1900,18 @@ __global__ void __launch_bounds__(kLinkThreads) k_unit_link(DevJob J) {
   auto poly_shift = [&](double norm, double *dst) {  // src/util.c:247-334
     const int D = J.uspD, nta = NCART(lpa), ntb = NCART(lpb);
     const double *uA = J.usp + cA * D * D * D, *uB = J.usp + cB * D * D * D;
+#pragma unroll 1
     for (int e = tid; e < nta * ncb; e += NT) {
       int c1 = e / ncb, q = e % ncb;
       const int *ex = J.ijk + 3 * (NCUM(lpa - 1) + c1);
       double v = 0.0;
+#pragma unroll 1
       for (int x = 0; x <= ex[0]; x++) {
         double bx = binom_tab(ex[0], x);
+#pragma unroll 1
         for (int y = 0; y <= ex[1]; y++) {
           double by = bx * binom_tab(ex[1], y);
+#pragma unroll 1
           for (int zz = 0; zz <= ex[2]; zz++) {
             double bz = by * binom_tab(ex[2], zz);
             double factor = bz * uA[((ex[0] - x) * D + (ex[1] - y)) * D + (ex[2] - zz)];
@@ -1855,14 +1923,18 @@ __global__ void __launch_bounds__(kLinkThreads) k_unit_link(DevJob J) {
       Jsh[e] = v;
     }
     __syncthreads();
+#pragma unroll 1
     for (int e = tid; e < nta * ntb; e += NT) {
       int c1 = e / ntb, c2 = e % ntb;
       const int *ex = J.ijk + 3 * (NCUM(lpb - 1) + c2);
       double v = 0.0;
+#pragma unroll 1
       for (int x = 0; x <= ex[0]; x++) {
         double bx = binom_tab(ex[0], x);
+#pragma unroll 1
         for (int y = 0; y <= ex[1]; y++) {
           double by = bx * binom_tab(ex[1], y);
+#pragma unroll 1
           for (int zz = 0; zz <= ex[2]; zz++) {
             double bz = by * binom_tab(ex[2], zz);
             double factor = bz * uB[((ex[0] - x) * D + (ex[1] - y)) * D + (ex[2] - zz)];
@@ -1883,20 +1955,25 @@ __global__ void __launch_bounds__(kLinkThreads) k_unit_link(DevJob J) {
     const double *angA = J.ang + cA * J.angLam * J.angLM * J.angC;
     const double *angB = J.ang + cB * J.angLam * J.angLM * J.angC;
     const int LMd = J.angLM, AC = J.angC;
+#pragma unroll 1
     for (int e = tid; e < nca * ncb; e += NT) {
       int pidx = e / ncb, qidx = e % ncb, alpha = 0, beta = 0;
       while (NCUM(alpha) <= pidx) alpha++;
       while (NCUM(beta) <= qidx) beta++;
       double g = 0.0;
+#pragma unroll 1
       for (int l = 0; l < Lc; l++) {
         int ll1 = l - alpha, p1 = (alpha + l) % 2;
         if (p1 > ll1) ll1 = p1;
         int ll2 = l - beta, p2 = (beta + l) % 2;
         if (p2 > ll2) ll2 = p2;
         double tmp = 0.0;
+#pragma unroll 1
         for (int l1 = ll1; l1 <= la + l; l1 += 2)
+#pragma unroll 1
           for (int l2 = ll2; l2 <= lb + l; l2 += 2) {
             double factor = 0.0;
+#pragma unroll 1
             for (int m = 0; m < 2 * l + 1; m++)
               factor += angA[((size_t)l1 * LMd + l * l + m) * AC + pidx] * angB[((size_t)l2 * LMd + l * l + m) * AC + qidx];
             tmp += factor * T[tidx(l, l1, l2, alpha + beta)];
@@ -1933,16 +2010,21 @@ __global__ void __launch_bounds__(128) k_shell_F_fast(DevJob J) {
   // coefficients times zeta^run (src/type2.c:229, :263-290)
   const int nF = J.nF, nRuns = J.nRuns > 0 ? J.nRuns : 1;
   const double *pa = J.primA + J.shP[s], *pd = J.primD + J.shP[s];
+#pragma unroll 1
   for (int run = 0; run < nRuns; run++) {
     const int lmaxA = J.maxLECP - 1 + J.shL[s] + run;
     double *F = J.F + (((size_t)c * J.nShells + s) * nRuns + run) * O * nF;
+#pragma unroll 1
     for (int n = threadIdx.x; n < O; n += blockDim.x) {
       double acc[kMaxRows], K[kMaxRows];
+#pragma unroll 1
       for (int i = 0; i < nF; i++) acc[i] = 0.0;
       if (!sw[2] && n >= sw[0] && n < sw[1] && lmaxA >= 0) {
         double r = J.xSmall[n];
+#pragma unroll 1
         for (int p = 0; p < J.shK[s]; p++) {
           double zeta = pa[p], da = pd[p];
+#pragma unroll 1
           for (int k = 0; k < run; k++) da *= zeta;
           double e = dAC - r;
           e = -zeta * e * e;
@@ -1950,9 +2032,11 @@ __global__ void __launch_bounds__(128) k_shell_F_fast(DevJob J) {
           if (v.m == 0) continue;
           const xf f = xf_mul(xf_from(zeta), xf_from(dAC));
           bessel_fx(J, lmaxA, xf_mul(xf_times100({f.m, f.e + 1}), xf_from(r)), v, sign_of(da), K);
+#pragma unroll 1
           for (int i = 0; i <= lmaxA; i++) acc[i] += K[i];
         }
       }
+#pragma unroll 1
       for (int i = 0; i < nF; i++) F[(size_t)n * nF + i] = acc[i];
     }
   }
@@ -1987,6 +2071,7 @@ __global__ void __launch_bounds__(1024) k_screen_scan(DevJob J, int nBlocks) {
   __shared__ int base;
   if (threadIdx.x == 0) base = 0;
   __syncthreads();
+#pragma unroll 1
   for (int b0 = 0; b0 < nBlocks; b0 += 1024) {
     const int b = b0 + threadIdx.x;
     const int x = b < nBlocks ? J.screenBlocks[b] : 0;
@@ -2018,10 +2103,12 @@ __global__ void __launch_bounds__(kScreenThreads) k_screen_scatter(DevJob J, lon
   __syncthreads();
   if (i >= n) return;
   int at = J.screenBlocks[blockIdx.x] + __popc(m & ((1u << lane) - 1u));
+#pragma unroll 1
   for (int w = 0; w < warp; w++) at += warpCnt[w];
   if (live) J.live[at] = (int)i;
   else J.status[unit_at(J, (int)i)] = kUnitSkipped;
   if ((int)i % J.nCentres == 0)
+#pragma unroll 1
     for (int k = 0; k < J.nChunks; k++)
       if (J.chunkPair[k] == (int)i / J.nCentres) J.liveStart[k] = at;
 }
@@ -2048,6 +2135,13 @@ int upload_schedules_fast(const int *s93slot, int s93n, const int *s93lvEnd, con
   cudaMemcpyToSymbolAsync(c92_lvN, s92lvN, sizeof(int) * s92levels, 0, cudaMemcpyHostToDevice, st);
   cudaMemcpyToSymbolAsync(c92_nLevels, &s92levels, sizeof(int), 0, cudaMemcpyHostToDevice, st);
   cudaMemcpyToSymbolAsync(c92_order, &s92n, sizeof(int), 0, cudaMemcpyHostToDevice, st);
+  double n93[32] = {}, n92[32] = {};
+#pragma unroll 1
+  for (int k = 0; k < s93levels; k++) n93[k] = 3.0 * s93lvN[k];
+#pragma unroll 1
+  for (int k = 0; k < s92levels; k++) n92[k] = 3.0 * (s92lvN[k] + 1.0);
+  cudaMemcpyToSymbolAsync(c93_3n, n93, sizeof n93, 0, cudaMemcpyHostToDevice, st);
+  cudaMemcpyToSymbolAsync(c92_3N, n92, sizeof n92, 0, cudaMemcpyHostToDevice, st);
   cudaStreamSynchronize(st);
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
@@ -2058,6 +2152,7 @@ void fast_prepare() {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || attr[dev]) return;
+#pragma unroll 1
   for (const void *k : {(const void *)k_unit_small<false>, (const void *)k_unit_small<true>,
                         (const void *)k_unit_large<false>, (const void *)k_unit_large<true>,
                         (const void *)k_unit_link}) {
@@ -2083,6 +2178,7 @@ int launch_fast_pipeline(const DevJob &J, cudaStream_t st, const FastConfig &cfg
   DevJob Jc = J;
   Jc.gcap = cfg.gcap;
   Jc.balance = cfg.balance;
+#pragma unroll 1
   for (int i = 0; i < kMaxClasses; i++) Jc.classCfg[i] = cfg.cls[i];
   Jc.classCycles = cfg.classCycles;
   const JobPlan::Order &ord = J.plan->order[cfg.sorted];
@@ -2109,6 +2205,7 @@ int launch_fast_pipeline(const DevJob &J, cudaStream_t st, const FastConfig &cfg
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+#pragma unroll 1
   for (int k = 0; k < Jc.nChunks; k++) {
     const JobPlan::Chunk &ch = ord.chunks[k];
     Jc.chunk = k;

@@ -26,6 +26,12 @@
 
 namespace ecpgb {
 
+#ifdef __CUDA_ARCH__
+#define ECPGB_NOUNROLL _Pragma("unroll 1")
+#else
+#define ECPGB_NOUNROLL
+#endif
+
 using u64 = unsigned long long;
 using i64 = long long;
 
@@ -217,8 +223,10 @@ ECPGB_HD void fx_bessel_rows(const i64 *besX, const i64 *besXA, int HL1, int lma
     scaleAt = 6;
   }
   const fxmul x = fx_split(X);
+ECPGB_NOUNROLL
   for (int l = 0; l <= lmax; l++, q += rowStride) {
     i64 v = 0;
+ECPGB_NOUNROLL
     for (int k = asy ? l : 5; k > 5; k--) v = ld_one(q + k) + mul_hi_s(v, x);
     const fxpair c45 = ld_pair(q + 4), c23 = ld_pair(q + 2), c01 = ld_pair(q);
     v = c45.y + mul_hi_s(v, x);
@@ -246,24 +254,20 @@ ECPGB_HD i64 fx_q53(double x) {
 
 // A signed sum of terms +-m 2^e: 60-bit mantissa, aligned to the larger
 // exponent, never renormalised upwards (cancelled bits stay cancelled).
+// Branch-free, so that lanes of different exponents stay together.
 struct xf_sum {
   i64 m = 0;
   int e = -100000;
   ECPGB_HD void add(xf t, uint32_t sign) {
     i64 tm = (i64)(t.m >> 4);
-    t.e += 4;
+    const int te = t.e + 4, d = e - te;
+    const int sa = d < 0 ? (d < -63 ? 63 : -d) : 0, st = d > 0 ? (d > 63 ? 63 : d) : 0;
     if (sign) tm = -tm;
-    const int d = e - t.e;
-    if (d >= 0) tm >>= (d > 63 ? 63 : d);
-    else {
-      m >>= (d < -63 ? 63 : -d);
-      e = t.e;
-    }
-    m += tm;
-    if ((m ^ (m << 1)) < 0) {  // room for the next term
-      m >>= 1;
-      e++;
-    }
+    m = (m >> sa) + (tm >> st);
+    e = d < 0 ? te : e;
+    const int over = (int)((uint32_t)((u64)(m ^ (m << 1)) >> 63));  // room for the next term
+    m >>= over;
+    e += over;
   }
   ECPGB_HD double value() const {
     return xf_to_double(m < 0 ? (u64)-m : (u64)m, e, m < 0 ? 0x80000000u : 0u);
