@@ -1,6 +1,6 @@
 """Builds libecp_gb300/libecp_gb300.so for sm_103a (in-tree, no cmake).
 
-Each translation unit compiles in parallel with nvcc; the FP64 kernels get
+Each translation unit compiles in parallel with nvcc; the plain FP64 kernels get
 --fmad=false so their arithmetic rounds like the reference's C.  Objects go to
 libecp_gb300/_build/ (git-ignored); the shared object lands next to this file.
 """
@@ -22,6 +22,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # (source, extra flags)
 UNITS = [
     ("ecp_fp64.cu", ["--fmad=false"]),
+    ("ecp_exact.cu", ["--fmad=false"]),
     ("ecp_host.cu", []),
     ("ecp_peaks.cu", []),
     ("ecp_tables.cpp", []),
@@ -44,7 +45,7 @@ def nvcc() -> str:
 def _compile(src: str, extra: list[str]) -> str:
     obj = os.path.join(BUILD, os.path.splitext(src)[0] + ".o")
     path = os.path.join(CSRC, src)
-    deps = [path] + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".h")] + \
+    deps = [path] + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))] + \
         [os.path.join(ROOT, "include", f) for f in os.listdir(os.path.join(ROOT, "include"))]
     if os.path.exists(obj) and os.path.getmtime(obj) >= max(os.path.getmtime(d) for d in deps):
         return obj

@@ -73,6 +73,7 @@ struct DevJob {
   // tables
   const double *xSmall, *wSmall, *xLarge, *wLarge;
   const double *besT, *besC;
+  const double *besD;          // derivative rows D^k K_l(z_i), [i][l <= besHL][6] (plain path; null: recurrence)
   const double *besH;          // Taylor coefficients [i][l <= besHL][6] (batched path)
   const double *besA;          // large-argument polynomial [l][i], stride max(besHL + 1, 6)
   const long long *besX;       // besH as fixed-point rows [i][l <= besHL][8] (ecp_fixed.h)
@@ -119,6 +120,7 @@ struct DevJob {
   long long scrBase;
   int2 *listT1, *listT2, *listPart;
   struct T1Fail *listFail;
+  bool exact;                    // plain path (one primitive pair a type-2 part)
   int take;                      // work-list entries a warp takes before it exits
   int gcap;                      // type-1 step-table width cap (doubles per slot)
   int balance;                   // 1: narrower type-1 groups for units with few primitive pairs
@@ -138,7 +140,7 @@ struct PairPlan {
   long long scratch, lists;
   int groups, batches, parts;
 };
-PairPlan pair_plan(int NP, int la, int lb, int nItems);
+PairPlan pair_plan(int NP, int la, int lb, int nItems, bool exact);
 
 // A batched job's queue orders, cut into chunks of consecutive sorted pairs
 // whose units' scratch fits the scratch buffer.
@@ -250,6 +252,18 @@ void launch_epilogue(const DevJob &job, cudaStream_t stream);
 
 // The first three of those kernels and the run's first warning word in one launch.
 void launch_stage1(const DevJob &job, cudaStream_t stream);
+
+void launch_shell_F(const DevJob &job, cudaStream_t stream);
+// The Bessel table's derivative rows (DevJob::besD), written to D.
+void launch_bessel_rows(const DevJob &job, double *D, cudaStream_t stream);
+
+// Plain path (ecp_exact.cu): the operations of launch_fp64_pipeline's kernels
+// in the batched path's stages, with that file's own __constant__ schedules.
+int upload_schedules_exact(const int *s93slot, int s93n, const int *s93lvEnd, const int *s93lvJ,
+                           const int *s93lvN, int s93levels, const int *s92slot, int s92n,
+                           const int *s92lvEnd, const int *s92lvN, int s92levels, void *stream);
+void exact_prepare();
+int launch_exact_pipeline(const DevJob &job, cudaStream_t stream, cudaEvent_t u0, cudaEvent_t u1);
 
 // Batched path (ecp_fast.cu): the units in four stages over work lists
 // (plan, small grid, large grid, blocks).  Its level schedules are that file's

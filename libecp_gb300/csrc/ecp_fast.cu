@@ -30,16 +30,9 @@
 //     mixed-precision code (instruction fetch is one of the kernel's stalls).
 #include <algorithm>
 
-#include "ecp_device.cuh"
-#include "ecp_fastmath.h"
-#include "ecp_fixed.h"
+#include "ecp_stages.cuh"
 
 namespace ecpgb {
-
-constexpr int kWalkCap = 128;  // large-grid quadratures per warp and pass
-constexpr int kLargeWords = (kMaxLargeOrder + 1) / 32;  // bitmap words over the large grid (128, even)
-static_assert(kLargeWords * 32 >= kMaxLargeOrder && kLargeWords % 2 == 0, "large-grid bitmap size");
-
 
 // --------------------------------------------------------------- helpers
 
@@ -244,75 +237,6 @@ static __device__ __noinline__ ff channel_ff(const DevJob &J, int c, int l, ff r
   return pot;
 }
 
-// Small-grid prefactor of a type-1 primitive pair, C1 = ca cb exp(zd2) with
-// zd2 = -za dAC^2 - zb dBC^2 (src/type1.c:235-246), rounded as the reference
-// rounds it (no contraction), so that every evaluation of it agrees.
-static __device__ inline double t1_prefactor(double za, double ca, double zb, double cb, double dAC, double dBC) {
-  const double zd2 = __dsub_rn(__dmul_rn(__dmul_rn(-za, dAC), dAC), __dmul_rn(__dmul_rn(zb, dBC), dBC));
-  return __dmul_rn(__dmul_rn(ca, cb), fast_exp(zd2));
-}
-
-// Kinds of type-1 primitive pairs.  The reference's small-grid integrand is
-// C1 r^l U K exp(e), e = (z r + s) r, multiplied left to right
-// (src/type1.c:79-88).
-//  * normal: C1 >= 2^-900 and e <= s^2 / (4 (za + zb)) < 700: no partial
-//    product of a non-negligible term underflows and exp(e) cannot overflow,
-//    so the integrand can be regrouped (prefactor, weight and r^l in one
-//    table row);
-//  * band: C1 below 2^-900 but not 0, or exp(e) may overflow: partial
-//    products underflow (or overflow) where a regrouped product would not, so
-//    the integrand is evaluated in the reference's order;
-//  * zero: C1 = 0, so every integrand value is 0 * (finite) = 0, or NaN where
-//    exp(e) overflows -- no table is needed.
-constexpr int kPairNormal = 0, kPairBand = 1, kPairZero = 2;
-constexpr double kLnDblMax = 0x1.62e42fefa39efp+9;  // exp overflows above it
-
-// e = (z r + s) r as the reference rounds it.
-static __device__ inline double t1_exponent(double z, double s, double r) {
-  return __dmul_rn(__dadd_rn(__dmul_rn(z, r), s), r);
-}
-
-// A zero-kind pair's PS93 walk (src/gc_integrators.c:157-217) with an
-// integrand that is 0 except NaN at window points whose exp(e) overflows:
-// the first level that counts a point converges to 0 unless a NaN has been
-// summed by then, after which no level converges.
-static __device__ __noinline__ bool t1_zero_walk(const DevJob &J, double s, double z, int ws, int we) {
-  auto nan_at = [&](int n) {
-    if (n < ws || n >= we) return false;
-    const double e = t1_exponent(z, s, J.xSmall[n]);
-    return e >= J.lnAcc1 && e > kLnDblMax;
-  };
-  bool nan = nan_at(c93_slot[0]) || nan_at(c93_slot[1]) || nan_at(c93_slot[2]);
-  int pos = 3;
-  for (int k = 0; k < c93_nLevels; k++) {
-    const int e = c93_lvEnd[k];
-    int cnt = 0;
-    for (; pos < e; pos += 2) {
-      const int lo = c93_slot[pos], hi = c93_slot[pos + 1];
-      if (lo >= ws) { nan = nan || nan_at(lo); cnt++; }
-      if (hi <= we) { nan = nan || nan_at(hi); cnt++; }
-    }
-    if (cnt > 0) return !nan;
-  }
-  return false;
-}
-
-// FM06 map parameters (src/gc_integrators.c:317-331).
-static __device__ inline void fm06(double za, double zb, double dAC, double dBC, double &i1, double &i2) {
-  double zp = za + zb, P = (za * dAC + zb * dBC) / zp;
-  double sigma = 1.0 / sqrt(zp), t = P - 7.0 * sigma;
-  double rmin = (t > 0.0) ? t : 0.0, rmax = P + 9.0 * sigma;
-  i1 = 0.5 * (rmax - rmin);
-  i2 = 0.5 * (rmax + rmin);
-}
-
-// Schedule steps: step 0 = the head plus 15 (lower, upper) pairs, every later
-// step 16 pairs.  For the large grid step 0 ends exactly at level 3.
-static __device__ inline int step_end93(int s0) { return s0 == 0 ? 33 : s0 + 32; }
-static __device__ inline int step_end92(int s0) { return s0 == 0 ? 31 : s0 + 32; }
-
-// Level constants of both rules as doubles (3 n, 3 N): no conversion per level.
-static __constant__ double c93_3n[32], c92_3N[32];
 
 // The factors of an integrand value, from table entries: mantissa, exponent
 // and sign of a double.
@@ -544,157 +468,15 @@ static __device__ inline void psm92_sparse_ff(int s0, int s1, const unsigned *bi
   I += acc.value();
 }
 
-// --------------------------------------------------------------- layout
-
-// Quadratures per primitive pair in the type-1 block ((l1, l2), l2 = l1,
-// l1-2, ...; src/type1.c:189-202), and primitive pairs packed per warp so
-// that most lanes carry a quadrature.
-__host__ __device__ inline int t1_items(int lab) {
-  int n = 0;
-  for (int l1 = 0; l1 <= lab; l1++) n += l1 / 2 + 1;
-  return n;
-}
-// Index of quadrature (l1, l2) in that list.
-__host__ __device__ inline int t1_index(int l1, int l2) { return (l1 + 1) * (l1 + 1) / 4 + ((l1 - l2) >> 1); }
-__host__ __device__ inline int t1_group(int lab, int cap) {
-  int g = 32 / t1_items(lab);
-  g = g > 8 ? 8 : (g < 1 ? 1 : g);
-  // the group's step table (33 slots x g entries of 2 (lab+1) + 1 doubles)
-  // stays within 33 x cap doubles
-  while (g > 1 && g * (2 * lab + 3) > cap) g--;
-  return g;
-}
-
-// The type-2 fallback deals a unit's primitive pairs to warps in parts of
-// consecutive pairs: at least 4 pairs a part (the list of failed quadratures
-// is decoded once per part) and at most 16 parts (each keeps a partial sum
-// per quadrature).
-__host__ __device__ inline int t2_part_pairs(int NP) {
-  const int n = (NP + 15) / 16;
-  return n < 4 ? 4 : n;
-}
-__host__ __device__ inline int t2_parts(int NP) { return (NP + t2_part_pairs(NP) - 1) / t2_part_pairs(NP); }
-
-// Global scratch of one unit between the stages (byte offsets): a header,
-// per primitive pair the FM06 map (i1, i2) and {break index, window}, the
-// type-1 quadratures [pair][t1_index], the type-2 quadratures of the class's
-// items, their partial sums [part][item] when there are several parts, the
-// bitmap of failed items, and the primitive pairs ordered by kind.
-struct UnitHead {
-  u64 est;   // mixed path: largest |estimate| of a failed small-grid item (bits)
-  int warn;  // 1: a type-1, 2: a type-2 quadrature ran out of levels
-  int pad;
-};
-struct UnitScratch {
-  int map, win, Q, T, part, mask, perm, total;
-};
-__host__ __device__ inline UnitScratch unit_scratch(int NP, int lab, int nItems) {
-  UnitScratch s;
-  int o = (int)sizeof(UnitHead);
-  s.map = o; o += 16 * NP;
-  s.win = o; o += 16 * NP;
-  s.Q = o; o += 8 * NP * t1_items(lab);
-  s.T = o; o += 8 * nItems;
-  s.part = o; o += t2_parts(NP) > 1 ? 8 * t2_parts(NP) * nItems : 0;
-  s.mask = o; o += 4 * ((nItems + 31) / 32);
-  s.perm = o; o += NP;
-  s.total = (o + 15) & ~15;
-  return s;
-}
-// Work-list entries a unit can add: type-1 groups (at most one per pair),
-// type-2 small-grid batches, type-2 parts, failed type-1 pairs.
-struct T1Fail {
-  int pos, k;  // queue position, primitive pair (bit 16: double-single tables)
-  unsigned mask;
-  int pad;
-  double s;  // |P|
-};
-__host__ __device__ inline size_t unit_list_bytes(int NP, int nItems) {
-  return 8 * (size_t)NP + 8 * (size_t)((nItems + 31) / 32) + 8 * (size_t)t2_parts(NP) + sizeof(T1Fail) * (size_t)NP;
-}
-
-PairPlan pair_plan(int NP, int la, int lb, int nItems) {
+PairPlan pair_plan(int NP, int la, int lb, int nItems, bool exact) {
   PairPlan p;
   if (la < 0 || lb < 0) NP = nItems = la = lb = 0;
-  p.scratch = unit_scratch(NP, la + lb, nItems).total;
-  p.lists = (long long)unit_list_bytes(NP, nItems);
+  p.scratch = unit_scratch(NP, la + lb, nItems, exact).total;
+  p.lists = (long long)unit_list_bytes(NP, nItems, exact);
   p.groups = NP;
   p.batches = (nItems + 31) / 32;
-  p.parts = NP ? t2_parts(NP) : 0;
+  p.parts = NP ? t2_parts(NP, exact) : 0;
   return p;
-}
-
-// A normal-kind primitive pair's scalars in fixed point: s = |P| as S 2^-q,
-// Z = za + zb (mantissa and exponent), 100 s.
-struct PairFx {
-  i64 S;
-  u64 Zm, sm;
-  int Ze, se, q;
-};
-
-// Shared memory of the stages, in doubles.  Small grid (one warp a CTA): the
-// group's pair scalars and step table.
-struct SmallSmem {
-  int sc, fx, tab, total;
-};
-__host__ __device__ inline SmallSmem small_layout(int LB, int cap) {
-  SmallSmem s;
-  int tt = 0;
-  for (int lab = 0; lab <= 2 * LB; lab++) {
-    const int w = 33 * t1_group(lab, cap) * (2 * lab + 3);
-    if (w > tt) tt = w;
-  }
-  s.sc = 0;
-  s.fx = 24;  // 3 scalars of up to 8 pairs
-  s.tab = s.fx + 8 * (int)(sizeof(PairFx) / sizeof(double));
-  s.total = s.tab + tt;
-  return s;
-}
-// Large grid (one warp a CTA): type 1 a 32-slot table; type 2 a 32-slot table
-// (U[nE], R[nA], Ka[LBE], Kb[LBE]), the walkers' state, the needed-slot bitmap
-// with word prefixes, the pending slots and the failed items.
-struct LargeSmem {
-  int tab, I, P, Q, part, bits, pend, pref, fail, total, tabStride;
-};
-__host__ __device__ inline LargeSmem large_layout(int LB, int LE) {
-  LargeSmem s;
-  const int nA = 2 * LB + 1, nE = LE > 0 ? LE : 1, LBE = LB + nE;
-  s.tabStride = (nE + nA + 2 * LBE) | 1;  // odd: conflict-free lane strides
-  int o = 32 * s.tabStride, t1 = 32 * (2 * nA + 3);
-  s.tab = 0;
-  if (t1 > o) o = t1;
-  s.I = o; o += kWalkCap;
-  s.P = o; o += kWalkCap;
-  s.Q = o; o += kWalkCap;
-  s.part = o; o += kWalkCap;
-  s.bits = o; o += kLargeWords / 2;
-  s.pend = o; o += 32;
-  s.pref = o; o += kLargeWords / 2;
-  s.fail = o; o += kWalkCap / 2;
-  s.total = o;
-  return s;
-}
-// Linking: chi / gamma, the half-shifted block, the radial table T, S_lm of a
-// batch of primitive pairs, their sums W and the combined-index block H.
-constexpr int kLinkBatch = 16;
-struct LinkSmem {
-  int chi, J, T, rsh, dir, W, H, total;
-};
-__host__ __device__ inline LinkSmem link_layout(int LB, int LE) {
-  LinkSmem s;
-  const int nA = 2 * LB + 1, nE = LE > 0 ? LE : 1, LBE = LB + nE;
-  const int nc = (LB + 1) * (LB + 2) * (LB + 3) / 6, nct = (LB + 1) * (LB + 2) / 2;
-  const int ncAB = (2 * LB + 1) * (2 * LB + 2) * (2 * LB + 3) / 6;
-  int o = 0;
-  s.chi = o; o += nc * nc;
-  s.J = o; o += nct * nc;
-  s.T = o; o += nE * LBE * LBE * nA;
-  s.rsh = o; o += kLinkBatch * nA * nA;
-  s.dir = o; o += kLinkBatch * 3;
-  s.W = o; o += ncAB;
-  s.H = o; o += ncAB;
-  s.total = o;
-  return s;
 }
 
 size_t fast_smem_bytes(int LB, int gcap) { return sizeof(double) * (size_t)small_layout(LB, gcap).total; }
@@ -707,112 +489,7 @@ size_t fast_smem_bytes(int LB, int gcap) { return sizeof(double) * (size_t)small
 // 2^47 tol 48, so quadratures above 1/8 of that take FP64 tables.
 __device__ inline double ff_limit(double tol) { return 0x1p47 * tol * 6.0; }
 
-// A unit as the stages see it: queue position pos = (sorted pair, centre),
-// the pair's shells and derivative shift, the screened window, its scratch.
-struct Unit {
-  int c, pr, sa, sb, A, B, la, lb, lab, lpa, lpb, pa0, pb0, ws, we, Nb, NP, Lc, cls, nItems;
-  const double *gA, *gB, *pzA, *pcA, *pzB, *pcB;
-  char *scr;
-  UnitScratch L;
-  bool live;
-};
-
-// Unit id of queue position pos (pairs in the plan's order, centres innermost).
-static __device__ inline long long unit_at(const DevJob &J, int pos) {
-  const int c = J.ctrOrder[pos % J.nCentres], pr = J.pairOrder[pos / J.nCentres];
-  return (long long)c * J.nPairs + pr;
-}
-
-// Items of the unit's class over the channels below l.
-static __device__ inline int class_items(const DevJob &J, int ncls, int l) {
-  int n = 0;
-  for (int k = 0; k < l; k++) n += J.itemCnt[ncls + k];
-  return n;
-}
-
-static __device__ inline Unit unit_load(const DevJob &J, int pos) {
-  Unit U;
-  const int ps = pos / J.nCentres, ci = pos % J.nCentres;
-  U.c = J.ctrOrder[ci];
-  U.pr = J.pairOrder[ps];
-  U.sa = J.pairA[U.pr];
-  U.sb = J.pairB[U.pr];
-  U.A = J.shAtom[U.sa];
-  U.B = J.shAtom[U.sb];
-  const int *wa = J.win + ((size_t)U.c * J.nShells + U.sa) * 3, *wb = J.win + ((size_t)U.c * J.nShells + U.sb) * 3;
-  // derivative shift: the shells' l moved by (shifta, shiftb) for the
-  // computation, the blocks handed out with l (lpa, lpb)
-  const UnitShift sh = unit_shift(J, U.pr, J.shL[U.sa], J.shL[U.sb], U.A, U.B, J.ctrAtom[U.c]);
-  U.ws = wa[0] > wb[0] ? wa[0] : wb[0];
-  U.we = wa[1] > wb[1] ? wa[1] : wb[1];
-  U.live = !(wa[2] || wb[2] || sh.skip) && U.ws < U.we;
-  U.la = J.shL[U.sa] + sh.a;
-  U.lb = J.shL[U.sb] + sh.b;
-  U.lab = U.la + U.lb;
-  U.lpa = sh.lpa;
-  U.lpb = sh.lpb;
-  U.pa0 = sh.a > 0 ? sh.a : 0;
-  U.pb0 = sh.b > 0 ? sh.b : 0;
-  U.Nb = J.shK[U.sb];
-  U.NP = J.shK[U.sa] * U.Nb;
-  U.Lc = J.ctrL[U.c];
-  if (!U.live) return U;
-  const int LE = J.maxLECP > 0 ? J.maxLECP : 1;
-  U.cls = U.la * (J.maxLBS + 1) + U.lb;
-  U.nItems = class_items(J, U.cls * LE, U.Lc);
-  U.gA = J.cgeo + ((size_t)U.c * J.nAtoms + U.A) * 4;
-  U.gB = J.cgeo + ((size_t)U.c * J.nAtoms + U.B) * 4;
-  U.pzA = J.primA + J.shP[U.sa];
-  U.pcA = J.primD + J.shP[U.sa];
-  U.pzB = J.primA + J.shP[U.sb];
-  U.pcB = J.primD + J.shP[U.sb];
-  U.L = unit_scratch(U.NP, U.lab, class_items(J, U.cls * LE, LE));
-  U.scr = J.scr + (J.scrOff[ps] - J.scrBase) + (size_t)ci * U.L.total;
-  return U;
-}
-
-// The item q of the unit's class as (l, l1, l2, l3), one byte each (all below 16).
-static __device__ inline int unit_item(const DevJob &J, const Unit &U, int q) {
-  const int ncls = U.cls * (J.maxLECP > 0 ? J.maxLECP : 1);
-  int l = 0;
-  while (q >= J.itemCnt[ncls + l]) { q -= J.itemCnt[ncls + l]; l++; }
-  const int v = J.items[J.itemOff[ncls + l] + q];
-  return l | (v & 255) << 8 | ((v >> 8) & 255) << 16 | (v >> 16) << 24;
-}
-
-// Work lists of a chunk and their counters (zeroed before the chunk).
-enum { kCntT1, kCntT2, kCntFail, kCntPart, kHeadSmall, kHeadLarge, kCounters };
-
-// The next entry of a list for a warp; its index to every lane.
-static __device__ inline int next_item(unsigned *head) {
-  int i = 0;
-  if ((threadIdx.x & 31) == 0) i = (int)atomicAdd(head, 1u);
-  return __shfl_sync(0xffffffffu, i, 0);
-}
-
 // --------------------------------------------------------------- type 1
-
-// 1/k, k <= 24 (the Legendre recurrence's divisor l - m)
-static __device__ const double kRecip[25] = {0.0,        1.0,        1.0 / 2,  1.0 / 3,  1.0 / 4,
-                                             1.0 / 5,    1.0 / 6,    1.0 / 7,  1.0 / 8,  1.0 / 9,
-                                             1.0 / 10,   1.0 / 11,   1.0 / 12, 1.0 / 13, 1.0 / 14,
-                                             1.0 / 15,   1.0 / 16,   1.0 / 17, 1.0 / 18, 1.0 / 19,
-                                             1.0 / 20,   1.0 / 21,   1.0 / 22, 1.0 / 23, 1.0 / 24};
-
-// Binomial coefficients C(n, k), n <= 15, as exact doubles: the values
-// fac[n] / (fac[n-k] fac[k]) of src/util.c:247-334 (exact integers), looked
-// up instead of divided out per term.
-struct BinomTable {
-  double v[16][16];
-  constexpr BinomTable() : v() {
-    for (int n = 0; n < 16; n++) {
-      v[n][0] = 1.0;
-      for (int k = 1; k <= n; k++) v[n][k] = v[n - 1][k - 1] + (k < n ? v[n - 1][k] : 0.0);
-    }
-  }
-};
-static __device__ const BinomTable kBinom;
-static __device__ inline double binom_tab(int n, int k) { return __ldg(&kBinom.v[n][k]); }
 
 // Direction of the k-vector P as (cos theta, cos phi, sin phi), the values
 // src/util.c:75-106 and src/spherical_harmonics.c:16-114 produce through
@@ -900,145 +577,6 @@ static __device__ __noinline__ bool t1_large_entry(const DevJob &J, int c, int L
     WR[l] = xf_to_double(v.m, v.e, sign);
   }
   return true;
-}
-
-// --------------------------------------------------------- stage 1: the plan
-
-// A unit by one warp: its primitive pairs by kind (kind-major, each kind in
-// pair order), the FM06 map, break index and point window of every pair, its
-// work-list entries; a dead unit is marked skipped.
-constexpr int kPlanThreads = 128;
-__global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
-  const int lane = threadIdx.x & 31;
-  const int idx = blockIdx.x * (kPlanThreads / 32) + (threadIdx.x >> 5);
-  int pos = J.chunk0 + idx;
-  if (J.live) {
-    const int l0 = J.liveStart[J.chunk];
-    if (l0 + idx >= J.liveStart[J.chunk + 1]) return;
-    pos = J.live[l0 + idx];
-  } else if (pos >= J.chunk1) {
-    return;
-  }
-  const Unit U = unit_load(J, pos);
-  if (!U.live) {
-    if (lane == 0) J.status[(size_t)U.c * J.nPairs + U.pr] = kUnitSkipped;
-    return;
-  }
-  const double dAC = U.gA[3], dBC = U.gB[3];
-  const int NP = U.NP, Nb = U.Nb;
-  unsigned char *perm = (unsigned char *)(U.scr + U.L.perm);
-  double2 *map = (double2 *)(U.scr + U.L.map);
-  int4 *win = (int4 *)(U.scr + U.L.win);
-  unsigned *mask = (unsigned *)(U.scr + U.L.mask);
-#pragma unroll 1
-  for (int w = lane; w < (U.nItems + 31) / 32; w += 32) mask[w] = 0u;
-  if (lane == 0) *(UnitHead *)U.scr = {0ull, 0, 0};
-  int cnt[3] = {0, 0, 0};
-  unsigned kinds = 0;  // the lane's pairs' kinds, 2 bits each (at most 8)
-#pragma unroll 1
-  for (int k0 = 0, j = 0; k0 < NP; k0 += 32, j++) {
-    const int k = k0 + lane;
-    int kind = 3;
-    if (k < NP) {
-      const double za = U.pzA[k / Nb], zb = U.pzB[k % Nb];
-      const double ca = zeta_times(U.pcA[k / Nb], za, U.pa0), cb = zeta_times(U.pcB[k % Nb], zb, U.pb0);
-      const double C1 = t1_prefactor(za, ca, zb, cb, dAC, dBC);
-      double P[3];
-      for (int i = 0; i < 3; i++) P[i] = 2.0 * (za * U.gA[i] + zb * U.gB[i]);
-      const double s2 = P[0] * P[0] + P[1] * P[1] + P[2] * P[2];
-      kind = C1 == 0.0 ? kPairZero : (fabs(C1) < 0x1p-900 || s2 > 2800.0 * (za + zb)) ? kPairBand : kPairNormal;
-      double i1, i2;
-      fm06(za, zb, dAC, dBC, i1, i2);
-      map[k] = make_double2(i1, i2);
-      if (U.nItems > 0) {
-        // break index, and the point-index interval in which the pair's
-        // exponent passes the screen, by bisection: past both centres the
-        // exponent falls with the index; it is a parabola in r with its vertex
-        // at V, and r grows with the index
-        auto exq = [&](int n, double &r) {
-          r = i1 * J.xLarge[n] + i2;
-          const double d1 = dAC - r, d2 = dBC - r;
-          return -za * d1 * d1 - zb * d2 * d2;
-        };
-        double r;
-        int lo = 0, hi = J.largeOrder;
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          const double e = exq(mid, r);
-          if (r > dAC && r > dBC && e < J.lnAcc2) hi = mid; else lo = mid + 1;
-        }
-        const int brk = lo < J.largeOrder ? lo : INT_MAX;
-        const double V = (za * dAC + zb * dBC) / (za + zb);
-        int a = 0, b = J.largeOrder;
-        while (a < b) {
-          const int mid = (a + b) >> 1;
-          if (i1 * J.xLarge[mid] + i2 >= V) b = mid; else a = mid + 1;
-        }
-        const int nv = a;
-        a = 0;
-        b = nv;
-        while (a < b) {
-          const int mid = (a + b) >> 1;
-          if (exq(mid, r) >= J.lnAcc2) b = mid; else a = mid + 1;
-        }
-        const int nLo = a;
-        a = nv;
-        b = J.largeOrder;
-        while (a < b) {
-          const int mid = (a + b) >> 1;
-          if (exq(mid, r) < J.lnAcc2) b = mid; else a = mid + 1;
-        }
-        win[k] = make_int4(brk, nLo, a - 1, 0);
-      }
-    }
-    kinds |= (unsigned)kind << (2 * j);
-    for (int kd = 0; kd < 3; kd++) cnt[kd] += __popc(__ballot_sync(0xffffffffu, kind == kd));
-  }
-  int at[3] = {0, cnt[0], cnt[0] + cnt[1]};
-#pragma unroll 1
-  for (int k0 = 0, j = 0; k0 < NP; k0 += 32, j++) {
-    const int kind = (kinds >> (2 * j)) & 3u;
-    for (int kd = 0; kd < 3; kd++) {
-      const unsigned m = __ballot_sync(0xffffffffu, kind == kd);
-      if (kind == kd) perm[at[kd] + __popc(m & ((1u << lane) - 1u))] = (unsigned char)(k0 + lane);
-      at[kd] += __popc(m);
-    }
-  }
-  // the class's type-1 settings (the autotuner may set them per (la, lb))
-  int gcap = J.gcap, bal = J.balance;
-  if (J.classCfg[U.cls] & kClassSet) {
-    gcap = J.classCfg[U.cls] & 0xfff;
-    bal = (J.classCfg[U.cls] >> 12) & 1;
-  }
-  int G[3], n[3], nGroups = 0;
-  for (int kd = 0; kd < 3; kd++) {
-    G[kd] = t1_group(U.lab, gcap);
-    // balance: a unit with few primitive pairs gives its groups to four warps
-    if (bal) {
-      const int g = (cnt[kd] + 3) / 4;
-      if (g < G[kd]) G[kd] = g > 0 ? g : 1;
-    }
-    n[kd] = (cnt[kd] + G[kd] - 1) / G[kd];
-    nGroups += n[kd];
-  }
-  const int nBatch = (U.nItems + 31) / 32, nPart = U.nItems > 0 ? t2_parts(NP) : 0;
-  int base = 0;
-  if (lane < 3) base = (int)atomicAdd(J.counters + (lane == 0 ? kCntT1 : lane == 1 ? kCntT2 : kCntPart),
-                                      (unsigned)(lane == 0 ? nGroups : lane == 1 ? nBatch : nPart));
-  const int b1 = __shfl_sync(0xffffffffu, base, 0), b2 = __shfl_sync(0xffffffffu, base, 1),
-            b3 = __shfl_sync(0xffffffffu, base, 2);
-#pragma unroll 1
-  for (int g = lane; g < nGroups; g += 32) {
-    int kd = 0, gj = g, p0 = 0;
-    while (gj >= n[kd]) { gj -= n[kd]; p0 += cnt[kd]; kd++; }
-    p0 += gj * G[kd];
-    const int left = cnt[kd] - gj * G[kd];
-    J.listT1[b1 + g] = make_int2(pos, p0 | (left < G[kd] ? left : G[kd]) << 10 | kd << 16);
-  }
-#pragma unroll 1
-  for (int q = lane; q < nBatch; q += 32) J.listT2[b2 + q] = make_int2(pos, 32 * q);
-#pragma unroll 1
-  for (int q = lane; q < nPart; q += 32) J.listPart[b3 + q] = make_int2(pos, q);
 }
 
 // --------------------------------------------------- stage 2: the small grid
@@ -1697,8 +1235,8 @@ static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem 
   const unsigned *mask = (const unsigned *)(U.scr + U.L.mask);
   int *fail = (int *)(sm + L.fail);
   double *sum = sm + L.part;
-  const int pp = t2_part_pairs(U.NP), k0 = part * pp, k1 = k0 + pp < U.NP ? k0 + pp : U.NP;
-  const bool single = t2_parts(U.NP) == 1;
+  const int pp = t2_part_pairs(U.NP, false), k0 = part * pp, k1 = k0 + pp < U.NP ? k0 + pp : U.NP;
+  const bool single = t2_parts(U.NP, false) == 1;
   // partial sums of the part, or the results themselves when it is the only one
   double *dst = single ? (double *)(U.scr + U.L.T)
                        : (double *)(U.scr + U.L.part) + (size_t)part * class_items(J, U.cls * LE, LE);
@@ -1767,7 +1305,7 @@ static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem 
 template <bool kMixed>
 __global__ void __launch_bounds__(32, 16) k_unit_large(DevJob J) {
   extern __shared__ double sm[];
-  const LargeSmem L = large_layout(J.maxLBS, J.maxLECP);
+  const LargeSmem L = large_layout(J.maxLBS, J.maxLECP, false);
   const int n2 = (int)J.counters[kCntPart], n = n2 + (int)J.counters[kCntFail];
 #pragma unroll 1
   for (int taken = 0; taken < J.take; taken++) {
@@ -1790,7 +1328,6 @@ __global__ void __launch_bounds__(32, 16) k_unit_large(DevJob J) {
 // One unit a CTA: the type-1 block from the quadratures of its primitive
 // pairs (src/type1.c:323-345), the type-2 block from its radial table
 // (src/type2.c:583-623), both shifted onto A and B (src/util.c:247-334).
-constexpr int kLinkThreads = 128;
 __global__ void __launch_bounds__(kLinkThreads) k_unit_link(DevJob J) {
   extern __shared__ double sm[];
   int pos = J.chunk0 + blockIdx.x;
@@ -1802,14 +1339,8 @@ __global__ void __launch_bounds__(kLinkThreads) k_unit_link(DevJob J) {
   const Unit U = unit_load(J, pos);
   if (!U.live) return;
   const LinkSmem Lm = link_layout(J.maxLBS, J.maxLECP);
-  const int tid = threadIdx.x, NT = kLinkThreads, la = U.la, lb = U.lb, lab = U.lab, lq = lab + 1, lpa = U.lpa,
-            lpb = U.lpb, nca = NCUM(la), ncb = NCUM(lb), Lc = U.Lc, Nb = U.Nb;
-  const int nA = 2 * J.maxLBS + 1, LE = J.maxLECP > 0 ? J.maxLECP : 1, LBE = J.maxLBS + LE;
-  const size_t cA = (size_t)U.c * J.nAtoms + U.A, cB = (size_t)U.c * J.nAtoms + U.B;
-  double *chi = sm + Lm.chi, *Jsh = sm + Lm.J, *T = sm + Lm.T, *rsh = sm + Lm.rsh, *dir = sm + Lm.dir,
-         *W = sm + Lm.W, *H = sm + Lm.H;
-  double *out1 = J.out + (size_t)U.c * J.centreStride + J.pairOff[U.pr];
-  double *out2 = out1 + NCART(lpa) * NCART(lpb);
+  const int tid = threadIdx.x, NT = kLinkThreads, lab = U.lab, lq = lab + 1, Nb = U.Nb;
+  double *rsh = sm + Lm.rsh, *dir = sm + Lm.dir, *W = sm + Lm.W, *H = sm + Lm.H;
   const int dd = J.tmDim + 1, tmW = (J.tmDim + 1) * (J.tmDim + 1), RQ = lq * lq, nq = t1_items(lab);
   // type 1: W[L][l][m] = sum over the primitive pairs of S_lm Q[L][l] (the
   // pairs in order), then H[p] = sum_lm poly2sph[p][lm] W[|p|][l][m]: the
@@ -1867,131 +1398,8 @@ __global__ void __launch_bounds__(kLinkThreads) k_unit_link(DevJob J) {
       H[pi] = acc;
     }
     __syncthreads();
-#pragma unroll 1
-    for (int e = tid; e < nca * ncb; e += NT) {
-      const int *ei = J.ijk + 3 * (e / ncb), *ej = J.ijk + 3 * (e % ncb);
-      chi[e] = H[J.ijkIdx[((ei[0] + ej[0]) * dd + (ei[1] + ej[1])) * dd + ei[2] + ej[2]]];
-    }
   }
-  // the radial table of type 2
-  auto tidx = [&](int l, int l1, int l2, int l3) { return ((l * LBE + l1) * LBE + l2) * nA + l3; };
-#pragma unroll 1
-  for (int e = tid; e < LE * LBE * LBE * nA; e += NT) T[e] = 0.0;
-  __syncthreads();
-  {
-    const double *Tq = (const double *)(U.scr + U.L.T), *part = (const double *)(U.scr + U.L.part);
-    const unsigned *mask = (const unsigned *)(U.scr + U.L.mask);
-    const int nParts = t2_parts(U.NP), nIt = class_items(J, U.cls * LE, LE);
-#pragma unroll 1
-    for (int q = tid; q < U.nItems; q += NT) {
-      double v;
-      if (nParts > 1 && (mask[q >> 5] >> (q & 31) & 1u)) {
-        v = 0.0;
-#pragma unroll 1
-        for (int p = 0; p < nParts; p++) v += part[(size_t)p * nIt + q];
-      } else {
-        v = Tq[q];
-      }
-      const int it = unit_item(J, U, q);
-      T[tidx(it & 255, (it >> 8) & 255, (it >> 16) & 255, it >> 24)] = v;
-    }
-  }
-  __syncthreads();
-  auto poly_shift = [&](double norm, double *dst) {  // src/util.c:247-334
-    const int D = J.uspD, nta = NCART(lpa), ntb = NCART(lpb);
-    const double *uA = J.usp + cA * D * D * D, *uB = J.usp + cB * D * D * D;
-#pragma unroll 1
-    for (int e = tid; e < nta * ncb; e += NT) {
-      int c1 = e / ncb, q = e % ncb;
-      const int *ex = J.ijk + 3 * (NCUM(lpa - 1) + c1);
-      double v = 0.0;
-#pragma unroll 1
-      for (int x = 0; x <= ex[0]; x++) {
-        double bx = binom_tab(ex[0], x);
-#pragma unroll 1
-        for (int y = 0; y <= ex[1]; y++) {
-          double by = bx * binom_tab(ex[1], y);
-#pragma unroll 1
-          for (int zz = 0; zz <= ex[2]; zz++) {
-            double bz = by * binom_tab(ex[2], zz);
-            double factor = bz * uA[((ex[0] - x) * D + (ex[1] - y)) * D + (ex[2] - zz)];
-            if (fabs(factor) <= J.acc) continue;
-            v += factor * chi[J.ijkIdx[(x * dd + y) * dd + zz] * ncb + q];
-          }
-        }
-      }
-      Jsh[e] = v;
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int e = tid; e < nta * ntb; e += NT) {
-      int c1 = e / ntb, c2 = e % ntb;
-      const int *ex = J.ijk + 3 * (NCUM(lpb - 1) + c2);
-      double v = 0.0;
-#pragma unroll 1
-      for (int x = 0; x <= ex[0]; x++) {
-        double bx = binom_tab(ex[0], x);
-#pragma unroll 1
-        for (int y = 0; y <= ex[1]; y++) {
-          double by = bx * binom_tab(ex[1], y);
-#pragma unroll 1
-          for (int zz = 0; zz <= ex[2]; zz++) {
-            double bz = by * binom_tab(ex[2], zz);
-            double factor = bz * uB[((ex[0] - x) * D + (ex[1] - y)) * D + (ex[2] - zz)];
-            if (fabs(factor) <= J.acc) continue;
-            factor *= norm;
-            v += factor * Jsh[c1 * ncb + J.ijkIdx[(x * dd + y) * dd + zz]];
-          }
-        }
-      }
-      dst[e] = v;
-    }
-    __syncthreads();
-  };
-  const double norm1 = 4.0 * kPi, norm2 = norm1 * norm1;
-  poly_shift(norm1, out1);
-  // gamma (src/type2.c:583-623)
-  {
-    const double *angA = J.ang + cA * J.angLam * J.angLM * J.angC;
-    const double *angB = J.ang + cB * J.angLam * J.angLM * J.angC;
-    const int LMd = J.angLM, AC = J.angC;
-#pragma unroll 1
-    for (int e = tid; e < nca * ncb; e += NT) {
-      int pidx = e / ncb, qidx = e % ncb, alpha = 0, beta = 0;
-      while (NCUM(alpha) <= pidx) alpha++;
-      while (NCUM(beta) <= qidx) beta++;
-      double g = 0.0;
-#pragma unroll 1
-      for (int l = 0; l < Lc; l++) {
-        int ll1 = l - alpha, p1 = (alpha + l) % 2;
-        if (p1 > ll1) ll1 = p1;
-        int ll2 = l - beta, p2 = (beta + l) % 2;
-        if (p2 > ll2) ll2 = p2;
-        double tmp = 0.0;
-#pragma unroll 1
-        for (int l1 = ll1; l1 <= la + l; l1 += 2)
-#pragma unroll 1
-          for (int l2 = ll2; l2 <= lb + l; l2 += 2) {
-            double factor = 0.0;
-#pragma unroll 1
-            for (int m = 0; m < 2 * l + 1; m++)
-              factor += angA[((size_t)l1 * LMd + l * l + m) * AC + pidx] * angB[((size_t)l2 * LMd + l * l + m) * AC + qidx];
-            tmp += factor * T[tidx(l, l1, l2, alpha + beta)];
-          }
-        g += tmp;
-      }
-      chi[e] = g;
-    }
-  }
-  __syncthreads();
-  poly_shift(norm2, out2);
-  if (tid == 0) {
-    const int warn = ((const UnitHead *)U.scr)->warn;
-    const long long u = (long long)U.c * J.nPairs + U.pr;
-    const int st = (warn & 1) ? kUnitWarnType1 : (warn & 2) ? kUnitWarnType2 : kUnitDone;
-    J.status[u] = st;
-    if (st != kUnitDone) atomicMin(&J.errWord[0], (int)u);
-  }
+  link_finish(J, U, Lm, sm);
 }
 
 // The screening window and F table of every (shell, centre) -- k_shell_F of
@@ -2045,17 +1453,6 @@ __global__ void __launch_bounds__(128) k_shell_F_fast(DevJob J) {
 // ---------------------------------------------------------- screening stage
 
 constexpr int kScreenThreads = 256;
-
-static __device__ bool unit_live(const DevJob &J, int pos) {
-  const long long u = unit_at(J, pos);
-  const int c = (int)(u / J.nPairs), pr = (int)(u % J.nPairs);
-  const int sa = J.pairA[pr], sb = J.pairB[pr];
-  const int *wa = J.win + ((size_t)c * J.nShells + sa) * 3;
-  const int *wb = J.win + ((size_t)c * J.nShells + sb) * 3;
-  const UnitShift sh = unit_shift(J, pr, J.shL[sa], J.shL[sb], J.shAtom[sa], J.shAtom[sb], J.ctrAtom[c]);
-  if (wa[2] || wb[2] || sh.skip) return false;
-  return (wa[0] > wb[0] ? wa[0] : wb[0]) < (wa[1] > wb[1] ? wa[1] : wb[1]);
-}
 
 // Live units (those that compute blocks: the screened windows of
 // src/libecp.c:296-330 and the derivative skips) per CTA chunk of the queue.
@@ -2123,27 +1520,8 @@ __global__ void k_reset(int *errWord) {
 int upload_schedules_fast(const int *s93slot, int s93n, const int *s93lvEnd, const int *s93lvJ,
                           const int *s93lvN, int s93levels, const int *s92slot, int s92n,
                           const int *s92lvEnd, const int *s92lvN, int s92levels, void *stream) {
-  if (s93n > kSmallOrder || s92n > kMaxLargeOrder || s93levels > 32 || s92levels > 32) return 1;
-  cudaStream_t st = (cudaStream_t)stream;
-  cudaMemcpyToSymbolAsync(c93_slot, s93slot, sizeof(int) * s93n, 0, cudaMemcpyHostToDevice, st);
-  cudaMemcpyToSymbolAsync(c93_lvEnd, s93lvEnd, sizeof(int) * s93levels, 0, cudaMemcpyHostToDevice, st);
-  cudaMemcpyToSymbolAsync(c93_lvJ, s93lvJ, sizeof(int) * s93levels, 0, cudaMemcpyHostToDevice, st);
-  cudaMemcpyToSymbolAsync(c93_lvN, s93lvN, sizeof(int) * s93levels, 0, cudaMemcpyHostToDevice, st);
-  cudaMemcpyToSymbolAsync(c93_nLevels, &s93levels, sizeof(int), 0, cudaMemcpyHostToDevice, st);
-  cudaMemcpyToSymbolAsync(c92_slot, s92slot, sizeof(int) * s92n, 0, cudaMemcpyHostToDevice, st);
-  cudaMemcpyToSymbolAsync(c92_lvEnd, s92lvEnd, sizeof(int) * s92levels, 0, cudaMemcpyHostToDevice, st);
-  cudaMemcpyToSymbolAsync(c92_lvN, s92lvN, sizeof(int) * s92levels, 0, cudaMemcpyHostToDevice, st);
-  cudaMemcpyToSymbolAsync(c92_nLevels, &s92levels, sizeof(int), 0, cudaMemcpyHostToDevice, st);
-  cudaMemcpyToSymbolAsync(c92_order, &s92n, sizeof(int), 0, cudaMemcpyHostToDevice, st);
-  double n93[32] = {}, n92[32] = {};
-#pragma unroll 1
-  for (int k = 0; k < s93levels; k++) n93[k] = 3.0 * s93lvN[k];
-#pragma unroll 1
-  for (int k = 0; k < s92levels; k++) n92[k] = 3.0 * (s92lvN[k] + 1.0);
-  cudaMemcpyToSymbolAsync(c93_3n, n93, sizeof n93, 0, cudaMemcpyHostToDevice, st);
-  cudaMemcpyToSymbolAsync(c92_3N, n92, sizeof n92, 0, cudaMemcpyHostToDevice, st);
-  cudaStreamSynchronize(st);
-  return cudaGetLastError() == cudaSuccess ? 0 : 2;
+  return upload_stage_schedules(s93slot, s93n, s93lvEnd, s93lvJ, s93lvN, s93levels, s92slot, s92n, s92lvEnd, s92lvN,
+                                s92levels, stream);
 }
 
 void fast_prepare() {
@@ -2181,13 +1559,9 @@ int launch_fast_pipeline(const DevJob &J, cudaStream_t st, const FastConfig &cfg
 #pragma unroll 1
   for (int i = 0; i < kMaxClasses; i++) Jc.classCfg[i] = cfg.cls[i];
   Jc.classCycles = cfg.classCycles;
-  const JobPlan::Order &ord = J.plan->order[cfg.sorted];
-  Jc.pairOrder = J.pairOrders + (size_t)cfg.sorted * J.nPairs;
-  Jc.scrOff = J.scrOffs + (size_t)cfg.sorted * (J.nPairs + 1);
-  Jc.chunkPair = J.chunkPairs + ord.chunkAt;
-  Jc.nChunks = (int)ord.chunks.size();
+  const JobPlan::Order &ord = use_order(Jc, cfg.sorted);
   const size_t sSmall = fast_smem_bytes(J.maxLBS, cfg.gcap);
-  const size_t sLarge = sizeof(double) * (size_t)large_layout(J.maxLBS, J.maxLECP).total;
+  const size_t sLarge = sizeof(double) * (size_t)large_layout(J.maxLBS, J.maxLECP, false).total;
   const size_t sLink = sizeof(double) * (size_t)link_layout(J.maxLBS, J.maxLECP).total;
   if (sSmall > 200 * 1024 || sLarge > 200 * 1024 || sLink > 200 * 1024) return 3;
   const bool screen = cfg.queue && cfg.screen;
@@ -2202,38 +1576,18 @@ int launch_fast_pipeline(const DevJob &J, cudaStream_t st, const FastConfig &cfg
     k_screen_scatter<<<(unsigned)nb, kScreenThreads, 0, st>>>(Jc, nUnits);
   }
   if (u0) record_timing(u0, st);
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-#pragma unroll 1
-  for (int k = 0; k < Jc.nChunks; k++) {
-    const JobPlan::Chunk &ch = ord.chunks[k];
-    Jc.chunk = k;
-    Jc.chunk0 = ch.p0 * J.nCentres;
-    Jc.chunk1 = ch.p1 * J.nCentres;
-    Jc.scrBase = ch.base;
-    char *lists = J.scr + ch.scratch;
-    Jc.listT1 = (int2 *)lists;
-    Jc.listT2 = Jc.listT1 + ch.groups;
-    Jc.listPart = Jc.listT2 + ch.batches;
-    Jc.listFail = (T1Fail *)(Jc.listPart + ch.parts);
-    cudaMemsetAsync(Jc.counters, 0, sizeof(unsigned) * kCounters, st);
-    const long long n = (long long)Jc.chunk1 - Jc.chunk0;
-    k_unit_plan<<<(unsigned)((n + 3) / 4), kPlanThreads, 0, st>>>(Jc);
-    // entries a warp takes: 8 where there are many (fewer CTAs to start), one
-    // where there are few (every SM gets work)
-    auto take = [&](long long items) { return (int)std::min(8ll, std::max(1ll, items / (64ll * sms))); };
-    const long long nSmall = ch.groups + ch.batches, nLarge = ch.parts + ch.groups;
-    Jc.take = take(nSmall);
-    const unsigned gSmall = (unsigned)std::max(1ll, (nSmall + Jc.take - 1) / Jc.take);
-    if (cfg.mixed) k_unit_small<true><<<gSmall, 32, sSmall, st>>>(Jc);
-    else k_unit_small<false><<<gSmall, 32, sSmall, st>>>(Jc);
-    Jc.take = take(nLarge);
-    const unsigned gLarge = (unsigned)std::max(1ll, (nLarge + Jc.take - 1) / Jc.take);
-    if (cfg.mixed) k_unit_large<true><<<gLarge, 32, sLarge, st>>>(Jc);
-    else k_unit_large<false><<<gLarge, 32, sLarge, st>>>(Jc);
-    k_unit_link<<<(unsigned)n, kLinkThreads, sLink, st>>>(Jc);
-  }
+  launch_chunks(Jc, ord, st, [&](const DevJob &C, unsigned units, unsigned gSmall, int takeSmall, unsigned gLarge,
+                                 int takeLarge) {
+    DevJob K = C;
+    k_unit_plan<false><<<(units + 3) / 4, kPlanThreads, 0, st>>>(K);
+    K.take = takeSmall;
+    if (cfg.mixed) k_unit_small<true><<<gSmall, 32, sSmall, st>>>(K);
+    else k_unit_small<false><<<gSmall, 32, sSmall, st>>>(K);
+    K.take = takeLarge;
+    if (cfg.mixed) k_unit_large<true><<<gLarge, 32, sLarge, st>>>(K);
+    else k_unit_large<false><<<gLarge, 32, sLarge, st>>>(K);
+    k_unit_link<<<units, kLinkThreads, sLink, st>>>(K);
+  });
   if (u1) record_timing(u1, st);
   launch_epilogue(Jc, st);
   cudaError_t e = cudaGetLastError();

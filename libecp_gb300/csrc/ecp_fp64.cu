@@ -14,7 +14,9 @@
 //                   src/util.c:215-243), per (centre, atom)
 //   k_shell_F       basis-set screening window and F table
 //                   (src/type2.c:149-180, :223-310), per (centre, shell)
-//   k_unit          one CTA per (centre, shell pair) unit: type-1 block
+//   k_unit          one CTA per (centre, shell pair) unit, for the entry point
+//                   that allocates nothing (the stages of ecp_exact.cu, bit
+//                   for bit the same, need scratch): type-1 block
 //                   (src/type1.c:95-302), type-2 block (src/type2.c:337-631),
 //                   binomial shift (src/util.c:247-334)
 //   k_scatter       upper-triangle accumulation into the AO matrix
@@ -149,6 +151,26 @@ __global__ void __launch_bounds__(128) k_stage1(DevJob J) {
   else radius_of(J, (b - J.nCentres * J.nAtoms) * 128 + threadIdx.x);
 }
 
+// The derivative rows of every Bessel table point (src/bessel.c:195-212), by
+// the operations of bessel_eval; one thread a point.
+__global__ void k_bessel_rows(DevJob J, double *D) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, HL = J.besHL;
+  if (i > J.besselN) return;
+  double d[kMaxRows], prev[kMaxRows];
+  const int top = HL + 5;
+  const double *row = J.besT + (size_t)i * (J.tabL + 1);
+  double *out = D + (size_t)i * (HL + 1) * 6;
+  for (int l = 0; l <= top; l++) d[l] = row[l];
+  for (int l = 0; l <= HL; l++) out[l * 6] = d[l];
+  for (int k = 1; k <= 5; k++) {
+    const int ti = top - k;
+    for (int j = 0; j <= ti + 1; j++) prev[j] = d[j];
+    d[0] = prev[1] - prev[0];
+    for (int j = 1; j <= ti; j++) d[j] = J.besC[j] * (prev[j - 1] - prev[j + 1]) - prev[j] + prev[j + 1];
+    for (int l = 0; l <= HL; l++) out[l * 6 + k] = d[l];
+  }
+}
+
 __global__ void __launch_bounds__(128) k_shell_F(DevJob J) {
   __shared__ int sw[3];
   const int s = blockIdx.x, c = blockIdx.y, O = kSmallOrder;
@@ -173,7 +195,7 @@ __global__ void __launch_bounds__(128) k_shell_F(DevJob J) {
         for (int p = 0; p < J.shK[s]; p++) {
           double zeta = pa[p], da = pd[p];
           for (int k = 0; k < run; k++) da *= zeta;
-          bessel_eval(J, lmaxA, 2.0 * zeta * dAC * r, K, 1);
+          bessel_rows(J, lmaxA, 2.0 * zeta * dAC * r, K);
           double e = dAC - r;
           e = exp(-zeta * e * e);
           for (int i = 0; i <= lmaxA; i++) acc[i] += da * K[i] * e;
@@ -756,6 +778,14 @@ void launch_prologue(const DevJob &J, cudaStream_t st, bool withF) {
   k_centre<<<J.nCentres, 128, sizeof(double) * kSmallOrder * (kMaxLEcp + 1), st>>>(J);
   k_centre_atom<<<dim3(J.nAtoms, J.nCentres), 64, 0, st>>>(J);
   if (withF) k_shell_F<<<dim3(J.nShells, J.nCentres), 128, 0, st>>>(J);
+}
+
+void launch_shell_F(const DevJob &J, cudaStream_t st) {
+  k_shell_F<<<dim3(J.nShells, J.nCentres), 128, 0, st>>>(J);
+}
+
+void launch_bessel_rows(const DevJob &J, double *D, cudaStream_t st) {
+  k_bessel_rows<<<(J.besselN + 128) / 128, 128, 0, st>>>(J, D);
 }
 
 void launch_stage1(const DevJob &J, cudaStream_t st) {

@@ -3,8 +3,7 @@
 //
 // One run of a job on the engine's stream:
 //   one H2D copy of all inputs (packed into a pinned staging buffer), memsets
-//   of the AO matrix / block buffer / error words, the six-kernel FP64
-//   pipeline, one D2H copy of the result (matrix or blocks) and the error
+//   of the AO matrix / block buffer / error words, the mode's pipeline, one D2H copy of the result (matrix or blocks) and the error
 //   words.  Tables (grids, Bessel table, angular table, ...) are built once
 //   per key on the host and stay resident on the device.
 #include <cuda_runtime.h>
@@ -219,6 +218,7 @@ struct DevTables {
   DBuf<int> ijk, ijkIdx, itemOff, itemCnt, items, s93, s92;
   DBuf<short> byN93;
   DBuf<long long> besX, besXA;  // fixed-point Bessel rows
+  DBuf<double> besD;            // derivative rows (plain path)
   int nItemsMax = 0;
 };
 
@@ -303,6 +303,19 @@ struct Engine {
               t->c2s.upload(h.cart2sph, stream) && t->s93.upload(h.s93.slot, stream) &&
               t->s92.upload(h.s92.slot, stream) && t->byN93.upload(by_point_order(h.s93.slot), stream) &&
               t->shNorm.upload(h.shNorm, stream);
+    // the Bessel table's derivative rows, by the device's own operations
+    ok = ok && t->besD.ensure((size_t)(h.besselN + 1) * (h.besselHL + 1) * 6);
+    if (ok) {
+      DevJob J;
+      std::memset(&J, 0, sizeof J);
+      J.besT = t->besT.p;
+      J.besC = t->besC.p;
+      J.tabL = h.tabL;
+      J.besselN = h.besselN;
+      J.besHL = h.besselHL;
+      launch_bessel_rows(J, t->besD.p, stream);
+      ok = cudaStreamSynchronize(stream) == cudaSuccess;
+    }
     // used-triple lists per (la, lb, l)
     int LB = h.maxLBS, LE = h.maxLECP > 0 ? h.maxLECP : 1;
     std::vector<int> off, cnt, items, tmp;
@@ -355,7 +368,7 @@ struct Engine {
       if (schedOwner == t) return 0;
     }
     const HostTables &h = t->host;
-    int rc = upload_schedules(h.s93.slot.data(), (int)h.s93.slot.size(), h.s93.lvEnd.data(),
+    int rc = upload_schedules_exact(h.s93.slot.data(), (int)h.s93.slot.size(), h.s93.lvEnd.data(),
                               h.s93.lvJ.data(), h.s93.lvN.data(), h.s93.nLevels, h.s92.slot.data(),
                               (int)h.s92.slot.size(), h.s92.lvEnd.data(), h.s92.lvN.data(),
                               h.s92.nLevels, stream);
@@ -453,19 +466,20 @@ static void shifted_l(const Parsed &P, int p, int &la, int &lb) {
   lb = P.shL[P.pairB[p]] + hb;
 }
 
-static PairPlan plan_of_pair(const Parsed &P, int p) {
+static PairPlan plan_of_pair(const Parsed &P, int p, bool exact) {
   int la, lb;
   shifted_l(P, p, la, lb);
   const int LE = P.maxLECP > 0 ? P.maxLECP : 1;
-  return pair_plan(P.shK[P.pairA[p]] * P.shK[P.pairB[p]], la, lb, la < 0 || lb < 0 ? 0 : class_item_count(la, lb, LE));
+  return pair_plan(P.shK[P.pairA[p]] * P.shK[P.pairB[p]], la, lb, la < 0 || lb < 0 ? 0 : class_item_count(la, lb, LE),
+                   exact);
 }
 
-// Scratch of a batched job with chunks of at most `cap` bytes (at least one
+// Scratch of a job with chunks of at most `cap` bytes (at least one
 // pair's units a chunk).
-static size_t scratch_bytes(const Parsed &P, size_t cap) {
+static size_t scratch_bytes(const Parsed &P, size_t cap, bool exact) {
   size_t tot = 0, one = 0;
   for (int p = 0; p < P.nPairs; p++) {
-    const PairPlan q = plan_of_pair(P, p);
+    const PairPlan q = plan_of_pair(P, p, exact);
     const size_t b = (size_t)P.nCentres * (q.scratch + q.lists);
     tot += b;
     one = std::max(one, b);
@@ -473,11 +487,11 @@ static size_t scratch_bytes(const Parsed &P, size_t cap) {
   return std::min(tot, std::max(cap, one));
 }
 
-// The queue orders of a batched job -- shell pairs in the reference's order,
+// The queue orders of a job -- shell pairs in the reference's order,
 // by descending estimated cost, and class-major (largest la + lb first, then
 // la; within a class by that cost), ties in the reference's order; every
 // pair's units consecutive, centres by descending L -- and their chunks.
-static void make_plan(const Parsed &P, size_t cap, JobPlan &plan, std::vector<int> &orders,
+static void make_plan(const Parsed &P, size_t cap, bool exact, JobPlan &plan, std::vector<int> &orders,
                       std::vector<long long> &offs, std::vector<int> &chunkPairs, std::vector<int> &ctr) {
   const int n = P.nPairs;
   std::vector<int> cost(n), cls(n);
@@ -486,7 +500,7 @@ static void make_plan(const Parsed &P, size_t cap, JobPlan &plan, std::vector<in
     const int a = P.pairA[p], b = P.pairB[p], la = P.shL[a], lb = P.shL[b];
     cost[p] = P.shK[a] * P.shK[b] * (la + lb + 2);
     cls[p] = (2 * kMaxLBasis - la - lb) * (kMaxLBasis + 1) + kMaxLBasis - la;
-    pp[p] = plan_of_pair(P, p);
+    pp[p] = plan_of_pair(P, p, exact);
   }
   ctr.resize(P.nCentres);
   for (int c = 0; c < P.nCentres; c++) ctr[c] = c;
@@ -555,17 +569,16 @@ size_t job_device_bytes(const Parsed &P, int mode, size_t budget, size_t *scratc
   const size_t angLam = P.maxLECP + LB + 1, angC = (LB + 1) * (LB + 2) * (LB + 3) / 6;
   size_t in = 8 * (P.geom.size() + P.primA.size() + P.primD.size() + 3 * P.termL.size() + P.pairOff.size()) +
               4 * (5 * P.shL.size() + P.atomMaxL.size() + 4 * P.ctrAtom.size() + P.termL.size() + 3 * P.pairA.size()) +
-              (mode != ECPGB_FP64 ? 36 * (P.nPairs + 1) + 4 * nc : 0) + (mode == ECPGB_MIXED ? 16 * P.termL.size() : 0) +
+              36 * (P.nPairs + 1) + 4 * nc + (mode == ECPGB_MIXED ? 16 * P.termL.size() : 0) +
               24 * 256;
   size_t work = 8 * (ns + nc * O * LE * nk + nc * O + nc * ns * (1 + P.deriv) * O * nF + nc * na * 4 + nc * na * D * D * D +
                      nc * na * angLam * LE * LE * angC + nc * (size_t)P.centreStride + (size_t)P.dim * P.dim) +
                 4 * (nc + nc * ns * 3 + nc * (size_t)P.nPairs + 2) + 8;
-  if (mode == ECPGB_FP64) return in + work;
   // the scratch between the stages takes what the budget leaves: a job whose
   // other buffers fit is never refused for it
   const size_t base = in + work, cap = base < budget ? std::min(kScratchCap, budget - base) : 0;
   if (scratchCap) *scratchCap = cap;
-  return base > budget ? base : std::min(budget, base + scratch_bytes(P, cap));
+  return base > budget ? base : std::min(budget, base + scratch_bytes(P, cap, mode == ECPGB_FP64));
 }
 
 int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int mode, cudaStream_t stream,
@@ -607,7 +620,7 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
          iPS = add(P.pairShift.data(), 4 * P.pairShift.size());
   std::vector<int> orders, chunkPairs, ctr;
   std::vector<long long> offs;
-  if (mode != ECPGB_FP64) make_plan(P, scratchCap, B.plan, orders, offs, chunkPairs, ctr);
+  make_plan(P, scratchCap, mode == ECPGB_FP64, B.plan, orders, offs, chunkPairs, ctr);
   size_t iOrd = add(orders.data(), 4 * orders.size()), iOff = add(offs.data(), 8 * offs.size()),
          iChk = add(chunkPairs.data(), 4 * chunkPairs.size()), iCtr = add(ctr.data(), 4 * ctr.size());
   // the ECP terms' exponents and coefficients as float pairs (mixed path)
@@ -659,13 +672,14 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.radius = B.radius.p; J.utab = B.utab.p; J.uL = B.uL.p; J.gridEnd = B.gridEnd.p; J.win = B.win.p;
   J.F = B.F.p; J.cgeo = B.cgeo.p; J.usp = B.usp.p; J.ang = B.ang.p; J.out = B.out.p;
   J.status = B.status.p; J.mat = B.mat.p; J.errWord = B.err.p;
-  if (mode != ECPGB_FP64) {  // the batched path's plan, scratch and screening stage
+  {  // the plan, the scratch and the batched path's screening stage
     const size_t nu = nc * (size_t)P.nPairs;
     size_t chunks = 0;
     for (const JobPlan::Order &o : B.plan.order) chunks = std::max(chunks, o.chunks.size());
-    if (!B.live.ensure(nu + 1) || !B.screenBlocks.ensure(nu / 256 + 2) || !B.liveStart.ensure(chunks + 1) ||
+    if ((mode != ECPGB_FP64 && !(B.live.ensure(nu + 1) && B.screenBlocks.ensure(nu / 256 + 2) &&
+                                 B.liveStart.ensure(chunks + 1))) ||
         !B.scr.ensure(B.plan.bytes + 16)) {
-      set_error("device allocation failed for the batched path's scratch");
+      set_error("device allocation failed for the job's scratch");
       return -1;
     }
     J.live = B.live.p;
@@ -674,6 +688,7 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
     J.scr = B.scr.p;
     J.counters = (unsigned *)(B.err.p + 2);
     J.plan = &B.plan;
+    J.exact = mode == ECPGB_FP64;
     J.pairOrders = (const int *)dp(iOrd);
     J.scrOffs = (const long long *)dp(iOff);
     J.chunkPairs = (const int *)dp(iChk);
@@ -684,6 +699,7 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.besA = T->besA.p;
   J.besZ = T->besZ.p;
   J.besX = T->besX.p;
+  J.besD = T->besD.p;
   J.besXA = T->besXA.p;
   J.besHf = (const ff *)T->besHf.p;
   J.besAf = (const ff *)T->besAf.p;
@@ -695,8 +711,6 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.byN93 = T->byN93.p;
   J.besHL = h.besselHL;
   J.shNorm = T->shNorm.p;
-  UnitSmem L = unit_smem_layout(h.maxLBS, h.maxLECP, h.nF);
-  B.smem = sizeof(double) * (size_t)L.total;
   return 0;
 }
 
@@ -711,8 +725,7 @@ int run_pipeline(JobBuffers &B, const DevJob &J, int mode, cudaEvent_t u0, cudaE
     c.mixed = mode == ECPGB_MIXED;
     rc = launch_fast_pipeline(J, stream, c, u0, u1);
   } else {
-    launch_reset(J, stream);
-    rc = launch_fp64_pipeline(J, stream, B.smem, u0, u1);
+    rc = launch_exact_pipeline(J, stream, u0, u1);
   }
   if (rc) {
     if (rc >= kLaunchErrorBase) set_error("kernel launch failed: %s", cudaGetErrorString((cudaError_t)(rc - kLaunchErrorBase)));
@@ -993,7 +1006,8 @@ static int capture_graph(Engine &E, ResidentJob *R) {
   if (R->graph) return 0;
   if (!R->gu0) cudaEventCreate(&R->gu0);
   if (!R->gu1) cudaEventCreate(&R->gu1);
-  if (R->mode != ECPGB_FP64) fast_prepare();  // function attributes before capture
+  fast_prepare();  // function attributes before capture
+  exact_prepare();
   cudaGraph_t g = nullptr;
   CUDA_OK(cudaStreamBeginCapture(E.stream, cudaStreamCaptureModeThreadLocal));
   int rc = run_pipeline(R->B, R->J, R->mode, R->gu0, R->gu1, &R->cfg, E.stream);
@@ -1313,12 +1327,11 @@ long long job_units(const void *vj, long long *emitted) {
 int job_launches(const void *vj) {
   const auto *R = (const ResidentJob *)vj;
   const int scatter = R->P.deriv ? 0 : 1;
-  // reset, four per-job stages, the unit kernel, the AO scatter (order 0)
-  if (R->mode == ECPGB_FP64) return 6 + scatter;
-  // two per-job stages, with the compacted queue the three screening kernels,
-  // the four unit stages per chunk, the scatter
-  int n = 2 + 4 * (int)R->B.plan.order[R->cfg.sorted].chunks.size() + scatter;
-  if (R->cfg.queue && R->cfg.screen) n += 3;
+  // two per-job stages, the four unit stages per chunk, the AO scatter (order
+  // 0), and with the batched path's compacted queue the three screening kernels
+  const FastConfig cfg = R->mode == ECPGB_FP64 ? FastConfig{} : R->cfg;
+  int n = 2 + 4 * (int)R->B.plan.order[cfg.sorted].chunks.size() + scatter;
+  if (R->mode != ECPGB_FP64 && cfg.queue && cfg.screen) n += 3;
   return n;
 }
 

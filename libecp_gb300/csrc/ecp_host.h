@@ -131,13 +131,12 @@ struct JobBuffers {
   DBuf<double> radius, utab, uL, F, cgeo, usp, ang, out, mat;
   DBuf<int> gridEnd, win, status, err;
   DBuf<int> live, screenBlocks, liveStart;  // screening stage of the batched path
-  DBuf<char> scr;                // its scratch between the unit stages
+  DBuf<char> scr;                // scratch between the unit stages
   JobPlan plan;
   DBuf<double> sout;       // spherical blocks
   DBuf<long long> sphOff;  // their per-entry offsets
   PinnedBuf pinned, pinnedOut;
   int *pinnedErr = nullptr;
-  size_t smem = 0, smemFast = 0;
   long long h2dBytes = 0;
   JobBuffers() { cudaMallocHost((void **)&pinnedErr, 4 * sizeof(int)); }
   // device bytes held by the buffers
@@ -195,7 +194,7 @@ bool valid_mode(int mode);
 struct DevTables;
 // Packs P's inputs into B's pinned buffer, copies them to the device on
 // `stream` and fills J (B's buffers grow as needed).
-// A batched job's units run in chunks whose scratch stays within scratchCap.
+// A job's units run in chunks whose scratch stays within scratchCap.
 constexpr size_t kScratchCap = 512ull << 20;
 int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int mode, cudaStream_t stream,
               size_t scratchCap = kScratchCap);
