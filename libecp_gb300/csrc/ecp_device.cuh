@@ -283,6 +283,46 @@ static __device__ void real_sph(const DevJob &J, int lmax, double theta, double 
 #undef PL
 }
 
+// Column m of real_sph (the entries l = m..lmax of +-m), operation by
+// operation, with J.shNorm's normalisation (the same values, tabulated):
+// x = cos(theta), and sin, cos of phi.
+static __device__ void real_sph_column(const DevJob &J, int lmax, int m, double x, double phi, double sphi, double cphi,
+                                       double *rsh) {
+  const int W = J.tmDim + 1;
+  double sm = 0.0, cm = 1.0;
+  if (m > 0 && 0.0 != phi) {
+    sm = sphi;
+    cm = cphi;
+    for (int i = 2; i <= m; i++) {
+      const double sn = sphi * cm + cphi * sm, cn = cphi * cm - sphi * sm;
+      sm = sn;
+      cm = cn;
+    }
+  }
+  const bool pole = 1.0 == x || -1.0 == x;
+  double P1 = 0.0, P2 = 0.0;
+  for (int l = m; l <= lmax; l++) {
+    double P;
+    if (pole) P = m > 0 ? 0.0 : l == 0 ? 1.0 : 1.0 == x ? 1.0 : -P1;
+    else if (l == 0) P = 1.0;
+    else if (l == m) {
+      const double s1 = sqrt(1.0 - x * x);
+      double s = s1;
+      for (int i = 2; i <= m; i++) s = s * s1;
+      P = s * J.dfac[2 * l - 1];
+    } else if (l == m + 1) P = x * (2 * m + 1) * P1;
+    else P = (x * (2 * l - 1) * P1 - (l + m - 1) * P2) / (l - m);
+    P2 = P1;
+    P1 = P;
+    const double v = J.shNorm[l * W + m] * P;
+    if (m == 0) rsh[l * l + l] = v / sqrt(2.0);
+    else {
+      rsh[l * l + l - m] = v * sm;
+      rsh[l * l + l + m] = v * cm;
+    }
+  }
+}
+
 // Squared radius where c r^l exp(-zeta r^2) = cutoff; -1 if Newton fails
 // (src/util.c:134-172, where the reference asserts).
 static __device__ double gto_radius(double c, double zeta, int l, double cutoff) {

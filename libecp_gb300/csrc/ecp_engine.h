@@ -31,6 +31,7 @@ constexpr int kSmallOrder = 383;       // PS93(128) abscissae
 constexpr int kMaxLargeOrder = 4095;   // PSM92 abscissae (largeGridOrder < 8192)
 constexpr int kMaxContraction = 16;    // primitives per shell
 constexpr int kUnitThreads = 128;      // threads per unit CTA
+constexpr int kPointThreads = 384;     // per-job stages: a thread per small-grid point
 constexpr int kChunkPairs = 64;        // (lower, upper) pairs per fallback chunk
 constexpr int kMaxWalkers = 512;       // large-grid quadratures integrated per pass
 
@@ -120,7 +121,7 @@ struct DevJob {
   long long scrBase;
   int2 *listT1, *listT2, *listPart;
   struct T1Fail *listFail;
-  bool exact;                    // plain path (one primitive pair a type-2 part)
+  bool few, single;              // few primitive pairs in all; one primitive pair a type-2 part
   int take;                      // work-list entries a warp takes before it exits
   int gcap;                      // type-1 step-table width cap (doubles per slot)
   int balance;                   // 1: narrower type-1 groups for units with few primitive pairs
@@ -140,7 +141,7 @@ struct PairPlan {
   long long scratch, lists;
   int groups, batches, parts;
 };
-PairPlan pair_plan(int NP, int la, int lb, int nItems, bool exact);
+PairPlan pair_plan(int NP, int la, int lb, int nItems, bool single);
 
 // A batched job's queue orders, cut into chunks of consecutive sorted pairs
 // whose units' scratch fits the scratch buffer.

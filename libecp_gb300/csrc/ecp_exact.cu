@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(kLinkThreads) k_exact_link(DevJob J) {
   if (!U.live) return;
   const LinkSmem Lm = link_layout(J.maxLBS, J.maxLECP);
   const int tid = threadIdx.x, NT = kLinkThreads, lab = U.lab, lq = lab + 1, Nb = U.Nb, RQ = lq * lq;
-  double *rsh = sm + Lm.rsh, *H = sm + Lm.H;
+  double *rsh = sm + Lm.rsh, *dir = sm + Lm.dir, *H = sm + Lm.H;
   const int dd = J.tmDim + 1, tmW = (J.tmDim + 1) * (J.tmDim + 1), nq = t1_items(lab), nH = NCUM(lab);
   const double *Q = (const double *)(U.scr + U.L.Q);
 #pragma unroll 1
@@ -629,13 +629,24 @@ __global__ void __launch_bounds__(kLinkThreads) k_exact_link(DevJob J) {
   for (int b0 = 0; b0 < U.NP; b0 += kLinkBatch) {
     const int nb = U.NP - b0 < kLinkBatch ? U.NP - b0 : kLinkBatch;
     __syncthreads();
-    if (tid < nb) {
-      const int k = b0 + tid;
+    // cos(theta), phi and its sine and cosine, then S_lm a column a thread
+    if ((tid & 31) < nb && tid < 96) {
+      const int g = tid & 31, k = b0 + g;
       const double za = U.pzA[k / Nb], zb = U.pzB[k % Nb];
       double P[3], S[3];
       for (int i = 0; i < 3; i++) P[i] = 2.0 * (za * U.gA[i] + zb * U.gB[i]);
       to_spherical(P, S);
-      real_sph(J, lab, S[1], S[2], rsh + tid * RQ);
+      if (tid < 32) {
+        dir[4 * g] = cos(S[1]);
+        dir[4 * g + 1] = S[2];
+      } else if (tid < 64) dir[4 * g + 2] = sin(S[2]);
+      else dir[4 * g + 3] = cos(S[2]);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int e = tid; e < nb * lq; e += NT) {
+      const double *d = dir + 4 * (e / lq);
+      real_sph_column(J, lab, e % lq, d[0], d[1], d[2], d[3], rsh + (e / lq) * RQ);
     }
     __syncthreads();
 #pragma unroll 1
@@ -659,7 +670,7 @@ __global__ void __launch_bounds__(kLinkThreads) k_exact_link(DevJob J) {
     }
   }
   __syncthreads();
-  link_finish(J, U, Lm, sm);
+  link_finish<true>(J, U, Lm, sm);
 }
 
 // --------------------------------------------------------------- launchers

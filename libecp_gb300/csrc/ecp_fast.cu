@@ -468,14 +468,14 @@ static __device__ inline void psm92_sparse_ff(int s0, int s1, const unsigned *bi
   I += acc.value();
 }
 
-PairPlan pair_plan(int NP, int la, int lb, int nItems, bool exact) {
+PairPlan pair_plan(int NP, int la, int lb, int nItems, bool single) {
   PairPlan p;
   if (la < 0 || lb < 0) NP = nItems = la = lb = 0;
-  p.scratch = unit_scratch(NP, la + lb, nItems, exact).total;
-  p.lists = (long long)unit_list_bytes(NP, nItems, exact);
+  p.scratch = unit_scratch(NP, la + lb, nItems, single).total;
+  p.lists = (long long)unit_list_bytes(NP, nItems, single);
   p.groups = NP;
   p.batches = (nItems + 31) / 32;
-  p.parts = NP ? t2_parts(NP, exact) : 0;
+  p.parts = NP ? t2_parts(NP, single) : 0;
   return p;
 }
 
@@ -1235,8 +1235,8 @@ static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem 
   const unsigned *mask = (const unsigned *)(U.scr + U.L.mask);
   int *fail = (int *)(sm + L.fail);
   double *sum = sm + L.part;
-  const int pp = t2_part_pairs(U.NP, false), k0 = part * pp, k1 = k0 + pp < U.NP ? k0 + pp : U.NP;
-  const bool single = t2_parts(U.NP, false) == 1;
+  const int pp = t2_part_pairs(U.NP, J.single), k0 = part * pp, k1 = k0 + pp < U.NP ? k0 + pp : U.NP;
+  const bool single = t2_parts(U.NP, J.single) == 1;
   // partial sums of the part, or the results themselves when it is the only one
   double *dst = single ? (double *)(U.scr + U.L.T)
                        : (double *)(U.scr + U.L.part) + (size_t)part * class_items(J, U.cls * LE, LE);
@@ -1399,13 +1399,13 @@ __global__ void __launch_bounds__(kLinkThreads) k_unit_link(DevJob J) {
     }
     __syncthreads();
   }
-  link_finish(J, U, Lm, sm);
+  link_finish<false>(J, U, Lm, sm);
 }
 
 // The screening window and F table of every (shell, centre) -- k_shell_F of
 // the drop-in path (src/type2.c:223-310, src/type2.c:149-180) with the
 // batched path's Bessel rows and exp; FP64 in every mode.
-__global__ void __launch_bounds__(128) k_shell_F_fast(DevJob J) {
+__global__ void __launch_bounds__(kPointThreads) k_shell_F_fast(DevJob J) {
   __shared__ int sw[3];
   const int s = blockIdx.x, c = blockIdx.y, O = kSmallOrder;
   const int C = J.ctrAtom[c], A = J.shAtom[s];
@@ -1567,7 +1567,7 @@ int launch_fast_pipeline(const DevJob &J, cudaStream_t st, const FastConfig &cfg
   const bool screen = cfg.queue && cfg.screen;
   if (!screen) Jc.live = nullptr;
   launch_stage1(Jc, st);
-  k_shell_F_fast<<<dim3(J.nShells, J.nCentres), 128, 0, st>>>(Jc);
+  k_shell_F_fast<<<dim3(J.nShells, J.nCentres), kPointThreads, 0, st>>>(Jc);
   const long long nUnits = (long long)J.nCentres * J.nPairs;
   if (screen && nUnits > 0) {  // screening stage: the live units' positions
     const long long nb = (nUnits + kScreenThreads - 1) / kScreenThreads;

@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(128) k_centre(DevJob J) { centre_of(J, blockId
 
 static __device__ void centre_atom_of(const DevJob &J, int A, int c) {
   __shared__ double rsh[169];
-  __shared__ double g[4];
+  __shared__ double g[4], ang[2], trig[3];
   const int C = J.ctrAtom[c];
   // the atom's largest l, plus the derivative order whose shifts raise it
   // (src/libecp.c:285-286, :292-293)
@@ -103,7 +103,13 @@ static __device__ void centre_atom_of(const DevJob &J, int A, int c) {
     g[3] = sqrt(x * x + y * y + z * z);
     for (int i = 0; i < 4; i++) J.cgeo[ca * 4 + i] = g[i];
     to_spherical(v, S);
-    if (lmax >= 0) real_sph(J, lmax, S[1], S[2], rsh);
+    ang[0] = S[1];
+    ang[1] = S[2];
+  }
+  // the polynomials by another warp meanwhile
+  if (threadIdx.x == 32) {
+    const double *rC = J.geom + 3 * C, *rA = J.geom + 3 * A;
+    const double v[3] = {rA[0] - rC[0], rA[1] - rC[1], rA[2] - rC[2]};
     // (-x)^i (-y)^j (-z)^k, i+j+k <= lA (src/util.c:215-243)
     int D = J.uspD;
     double *t = J.usp + ca * D * D * D;
@@ -118,6 +124,20 @@ static __device__ void centre_atom_of(const DevJob &J, int A, int c) {
           t[(i * D + j) * D + k] = px * py * pz;
         }
       }
+    }
+  }
+  __syncthreads();
+  // S_lm column by column (one thread each); theta's and phi's functions on
+  // different warps
+  if (threadIdx.x == 0) trig[0] = cos(ang[0]);
+  if (threadIdx.x == 32) trig[1] = sin(ang[1]);
+  if (threadIdx.x == 64 % blockDim.x) trig[2] = cos(ang[1]);
+  __syncthreads();
+  if (lmax >= 0) {
+    if (J.shNorm) {
+      if ((int)threadIdx.x <= lmax) real_sph_column(J, lmax, threadIdx.x, trig[0], ang[1], trig[1], trig[2], rsh);
+    } else if (threadIdx.x == 0) {
+      real_sph(J, lmax, ang[0], ang[1], rsh);
     }
   }
   __syncthreads();
@@ -137,9 +157,9 @@ static __device__ void centre_atom_of(const DevJob &J, int A, int c) {
 __global__ void __launch_bounds__(64) k_centre_atom(DevJob J) { centre_atom_of(J, blockIdx.x, blockIdx.y); }
 
 // The three stages above in one launch (the batched path): centres, (centre,
-// atom) pairs, then shells 128 a CTA.  errWord[1] is cleared before the launch
+// atom) pairs, then the shells.  errWord[1] is cleared before the launch
 // (the shells set it), errWord[0] here.
-__global__ void __launch_bounds__(128) k_stage1(DevJob J) {
+__global__ void __launch_bounds__(kPointThreads) k_stage1(DevJob J) {
   int b = blockIdx.x;
   if (b == 0 && threadIdx.x == 0) J.errWord[0] = INT_MAX;
   if (b < J.nCentres) {
@@ -148,7 +168,7 @@ __global__ void __launch_bounds__(128) k_stage1(DevJob J) {
   }
   b -= J.nCentres;
   if (b < J.nCentres * J.nAtoms) centre_atom_of(J, b % J.nAtoms, b / J.nAtoms);
-  else radius_of(J, (b - J.nCentres * J.nAtoms) * 128 + threadIdx.x);
+  else radius_of(J, (b - J.nCentres * J.nAtoms) * kPointThreads + threadIdx.x);
 }
 
 // The derivative rows of every Bessel table point (src/bessel.c:195-212), by
@@ -171,7 +191,7 @@ __global__ void k_bessel_rows(DevJob J, double *D) {
   }
 }
 
-__global__ void __launch_bounds__(128) k_shell_F(DevJob J) {
+__global__ void __launch_bounds__(kPointThreads) k_shell_F(DevJob J) {
   __shared__ int sw[3];
   const int s = blockIdx.x, c = blockIdx.y, O = kSmallOrder;
   const int C = J.ctrAtom[c], A = J.shAtom[s];
@@ -777,11 +797,11 @@ void launch_prologue(const DevJob &J, cudaStream_t st, bool withF) {
   k_radius<<<(J.nShells + 127) / 128, 128, 0, st>>>(J);
   k_centre<<<J.nCentres, 128, sizeof(double) * kSmallOrder * (kMaxLEcp + 1), st>>>(J);
   k_centre_atom<<<dim3(J.nAtoms, J.nCentres), 64, 0, st>>>(J);
-  if (withF) k_shell_F<<<dim3(J.nShells, J.nCentres), 128, 0, st>>>(J);
+  if (withF) k_shell_F<<<dim3(J.nShells, J.nCentres), kPointThreads, 0, st>>>(J);
 }
 
 void launch_shell_F(const DevJob &J, cudaStream_t st) {
-  k_shell_F<<<dim3(J.nShells, J.nCentres), 128, 0, st>>>(J);
+  k_shell_F<<<dim3(J.nShells, J.nCentres), kPointThreads, 0, st>>>(J);
 }
 
 void launch_bessel_rows(const DevJob &J, double *D, cudaStream_t st) {
@@ -790,7 +810,7 @@ void launch_bessel_rows(const DevJob &J, double *D, cudaStream_t st) {
 
 void launch_stage1(const DevJob &J, cudaStream_t st) {
   cudaMemsetAsync(J.errWord + 1, 0, sizeof(int), st);
-  k_stage1<<<J.nCentres * (1 + J.nAtoms) + (J.nShells + 127) / 128, 128,
+  k_stage1<<<J.nCentres * (1 + J.nAtoms) + (J.nShells + kPointThreads - 1) / kPointThreads, kPointThreads,
              sizeof(double) * kSmallOrder * (kMaxLEcp + 1), st>>>(J);
 }
 

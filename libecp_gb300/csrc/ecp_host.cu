@@ -466,20 +466,31 @@ static void shifted_l(const Parsed &P, int p, int &la, int &lb) {
   lb = P.shL[P.pairB[p]] + hb;
 }
 
-static PairPlan plan_of_pair(const Parsed &P, int p, bool exact) {
+static PairPlan plan_of_pair(const Parsed &P, int p, bool single) {
   int la, lb;
   shifted_l(P, p, la, lb);
   const int LE = P.maxLECP > 0 ? P.maxLECP : 1;
   return pair_plan(P.shK[P.pairA[p]] * P.shK[P.pairB[p]], la, lb, la < 0 || lb < 0 ? 0 : class_item_count(la, lb, LE),
-                   exact);
+                   single);
+}
+
+// Jobs of at most kFewPairs primitive pairs over all units: every warp of the
+// GPU gets at most a few work-list entries and the longest one sets a stage's
+// time, so an entry is one primitive pair (the 702-pair example's large-grid
+// stage takes 0.25 instead of 0.52 ms).
+constexpr long long kFewPairs = 4864;  // 32 a streaming multiprocessor
+static bool few_pairs(const Parsed &P) {
+  long long n = 0;
+  for (int p = 0; p < P.nPairs; p++) n += (long long)P.nCentres * P.shK[P.pairA[p]] * P.shK[P.pairB[p]];
+  return n <= kFewPairs;
 }
 
 // Scratch of a job with chunks of at most `cap` bytes (at least one
 // pair's units a chunk).
-static size_t scratch_bytes(const Parsed &P, size_t cap, bool exact) {
+static size_t scratch_bytes(const Parsed &P, size_t cap, bool single) {
   size_t tot = 0, one = 0;
   for (int p = 0; p < P.nPairs; p++) {
-    const PairPlan q = plan_of_pair(P, p, exact);
+    const PairPlan q = plan_of_pair(P, p, single);
     const size_t b = (size_t)P.nCentres * (q.scratch + q.lists);
     tot += b;
     one = std::max(one, b);
@@ -491,7 +502,7 @@ static size_t scratch_bytes(const Parsed &P, size_t cap, bool exact) {
 // by descending estimated cost, and class-major (largest la + lb first, then
 // la; within a class by that cost), ties in the reference's order; every
 // pair's units consecutive, centres by descending L -- and their chunks.
-static void make_plan(const Parsed &P, size_t cap, bool exact, JobPlan &plan, std::vector<int> &orders,
+static void make_plan(const Parsed &P, size_t cap, bool single, JobPlan &plan, std::vector<int> &orders,
                       std::vector<long long> &offs, std::vector<int> &chunkPairs, std::vector<int> &ctr) {
   const int n = P.nPairs;
   std::vector<int> cost(n), cls(n);
@@ -500,7 +511,7 @@ static void make_plan(const Parsed &P, size_t cap, bool exact, JobPlan &plan, st
     const int a = P.pairA[p], b = P.pairB[p], la = P.shL[a], lb = P.shL[b];
     cost[p] = P.shK[a] * P.shK[b] * (la + lb + 2);
     cls[p] = (2 * kMaxLBasis - la - lb) * (kMaxLBasis + 1) + kMaxLBasis - la;
-    pp[p] = plan_of_pair(P, p, exact);
+    pp[p] = plan_of_pair(P, p, single);
   }
   ctr.resize(P.nCentres);
   for (int c = 0; c < P.nCentres; c++) ctr[c] = c;
@@ -578,7 +589,7 @@ size_t job_device_bytes(const Parsed &P, int mode, size_t budget, size_t *scratc
   // other buffers fit is never refused for it
   const size_t base = in + work, cap = base < budget ? std::min(kScratchCap, budget - base) : 0;
   if (scratchCap) *scratchCap = cap;
-  return base > budget ? base : std::min(budget, base + scratch_bytes(P, cap, mode == ECPGB_FP64));
+  return base > budget ? base : std::min(budget, base + scratch_bytes(P, cap, mode == ECPGB_FP64 || few_pairs(P)));
 }
 
 int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int mode, cudaStream_t stream,
@@ -620,7 +631,7 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
          iPS = add(P.pairShift.data(), 4 * P.pairShift.size());
   std::vector<int> orders, chunkPairs, ctr;
   std::vector<long long> offs;
-  make_plan(P, scratchCap, mode == ECPGB_FP64, B.plan, orders, offs, chunkPairs, ctr);
+  make_plan(P, scratchCap, mode == ECPGB_FP64 || few_pairs(P), B.plan, orders, offs, chunkPairs, ctr);
   size_t iOrd = add(orders.data(), 4 * orders.size()), iOff = add(offs.data(), 8 * offs.size()),
          iChk = add(chunkPairs.data(), 4 * chunkPairs.size()), iCtr = add(ctr.data(), 4 * ctr.size());
   // the ECP terms' exponents and coefficients as float pairs (mixed path)
@@ -688,7 +699,8 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
     J.scr = B.scr.p;
     J.counters = (unsigned *)(B.err.p + 2);
     J.plan = &B.plan;
-    J.exact = mode == ECPGB_FP64;
+    J.few = few_pairs(P);
+    J.single = J.few || mode == ECPGB_FP64;
     J.pairOrders = (const int *)dp(iOrd);
     J.scrOffs = (const long long *)dp(iOff);
     J.chunkPairs = (const int *)dp(iChk);

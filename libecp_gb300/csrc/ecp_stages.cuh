@@ -114,14 +114,15 @@ __host__ __device__ inline int t1_group(int lab, int cap) {
 // The type-2 fallback deals a unit's primitive pairs to warps in parts of
 // consecutive pairs: at least 4 pairs a part (the list of failed quadratures
 // is decoded once per part) and at most 16 parts (each keeps a partial sum
-// per quadrature).  The plain path (exact) keeps every pair's result, so that
-// they are added in the reference's order: one pair a part.
-__host__ __device__ inline int t2_part_pairs(int NP, bool exact) {
+// per quadrature).  One pair a part (`single`) on the plain path, which keeps
+// every pair's result and adds them in the reference's order, and for jobs of
+// few primitive pairs, where the longest part sets the time.
+__host__ __device__ inline int t2_part_pairs(int NP, bool single) {
   const int n = (NP + 15) / 16;
-  return exact ? 1 : n < 4 ? 4 : n;
+  return single ? 1 : n < 4 ? 4 : n;
 }
-__host__ __device__ inline int t2_parts(int NP, bool exact) {
-  const int n = t2_part_pairs(NP, exact);
+__host__ __device__ inline int t2_parts(int NP, bool single) {
+  const int n = t2_part_pairs(NP, single);
   return (NP + n - 1) / n;
 }
 
@@ -138,14 +139,14 @@ struct UnitHead {
 struct UnitScratch {
   int map, win, Q, T, part, mask, perm, total;
 };
-__host__ __device__ inline UnitScratch unit_scratch(int NP, int lab, int nItems, bool exact) {
+__host__ __device__ inline UnitScratch unit_scratch(int NP, int lab, int nItems, bool single) {
   UnitScratch s;
   int o = (int)sizeof(UnitHead);
   s.map = o; o += 16 * NP;
   s.win = o; o += 16 * NP;
   s.Q = o; o += 8 * NP * t1_items(lab);
   s.T = o; o += 8 * nItems;
-  s.part = o; o += t2_parts(NP, exact) > 1 ? 8 * t2_parts(NP, exact) * nItems : 0;
+  s.part = o; o += t2_parts(NP, single) > 1 ? 8 * t2_parts(NP, single) * nItems : 0;
   s.mask = o; o += 4 * ((nItems + 31) / 32);
   s.perm = o; o += NP;
   s.total = (o + 15) & ~15;
@@ -159,8 +160,8 @@ struct T1Fail {
   int pad;
   double s;  // |P|
 };
-__host__ __device__ inline size_t unit_list_bytes(int NP, int nItems, bool exact) {
-  return 8 * (size_t)NP + 8 * (size_t)((nItems + 31) / 32) + 8 * (size_t)t2_parts(NP, exact) + sizeof(T1Fail) * (size_t)NP;
+__host__ __device__ inline size_t unit_list_bytes(int NP, int nItems, bool single) {
+  return 8 * (size_t)NP + 8 * (size_t)((nItems + 31) / 32) + 8 * (size_t)t2_parts(NP, single) + sizeof(T1Fail) * (size_t)NP;
 }
 
 // A normal-kind primitive pair's scalars in fixed point: s = |P| as S 2^-q,
@@ -215,10 +216,12 @@ __host__ __device__ inline LargeSmem large_layout(int LB, int LE, bool exact) {
   return s;
 }
 // Linking: chi / gamma, the half-shifted block, the radial table T, S_lm of a
-// batch of primitive pairs, their sums W and the combined-index block H.
+// batch of primitive pairs, the shift factors, the S_lm sums W and the
+// combined-index block H.
 constexpr int kLinkBatch = 16;
+constexpr int kShiftTerms = 12;  // most (x+1)(y+1)(z+1) over x + y + z = l <= 4
 struct LinkSmem {
-  int chi, J, T, rsh, dir, W, H, total;
+  int chi, J, T, rsh, fac, dir, W, H, total;
 };
 __host__ __device__ inline LinkSmem link_layout(int LB, int LE) {
   LinkSmem s;
@@ -229,8 +232,12 @@ __host__ __device__ inline LinkSmem link_layout(int LB, int LE) {
   s.chi = o; o += nc * nc;
   s.J = o; o += nct * nc;
   s.T = o; o += nE * LBE * LBE * nA;
-  s.rsh = o; o += kLinkBatch * nA * nA;
-  s.dir = o; o += kLinkBatch * 3;
+  {  // S_lm of a batch, later the half-contracted gamma of one (l, alpha)
+    const int r = kLinkBatch * nA * nA, y = (2 * nE - 1) * (LB + 1) * nc;
+    s.rsh = o; o += r > y ? r : y;
+  }
+  s.fac = o; o += 2 * kShiftTerms * nct;
+  s.dir = o; o += kLinkBatch * 4;
   s.W = o; o += ncAB;
   s.H = o; o += ncAB;
   s.total = o;
@@ -296,7 +303,7 @@ static __device__ inline Unit unit_load(const DevJob &J, int pos) {
   U.pcA = J.primD + J.shP[U.sa];
   U.pzB = J.primA + J.shP[U.sb];
   U.pcB = J.primD + J.shP[U.sb];
-  U.L = unit_scratch(U.NP, U.lab, class_items(J, U.cls * LE, LE), J.exact);
+  U.L = unit_scratch(U.NP, U.lab, class_items(J, U.cls * LE, LE), J.single);
   U.scr = J.scr + (J.scrOff[ps] - J.scrBase) + (size_t)ci * U.L.total;
   return U;
 }
@@ -456,7 +463,8 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
   }
   int G[3], n[3], nGroups = 0;
   for (int kd = 0; kd < 3; kd++) {
-    G[kd] = t1_group(U.lab, gcap);
+    // (one pair a group in jobs of few pairs, as the type-2 parts)
+    G[kd] = J.few ? 1 : t1_group(U.lab, gcap);
     // balance: a unit with few primitive pairs gives its groups to four warps
     if (bal) {
       const int g = (cnt[kd] + 3) / 4;
@@ -465,7 +473,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
     n[kd] = (cnt[kd] + G[kd] - 1) / G[kd];
     nGroups += n[kd];
   }
-  const int nBatch = (U.nItems + 31) / 32, nPart = U.nItems > 0 ? t2_parts(NP, kExact) : 0;
+  const int nBatch = (U.nItems + 31) / 32, nPart = U.nItems > 0 ? t2_parts(NP, J.single) : 0;
   int base = 0;
   if (lane < 3) base = (int)atomicAdd(J.counters + (lane == 0 ? kCntT1 : lane == 1 ? kCntT2 : kCntPart),
                                       (unsigned)(lane == 0 ? nGroups : lane == 1 ? nBatch : nPart));
@@ -489,6 +497,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
 // table (type 2, src/type2.c:583-623), both shifted onto A and B
 // (src/util.c:247-334), and its status.
 constexpr int kLinkThreads = 128;
+template <bool kExact>
 static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSmem &Lm, double *sm) {
   const int tid = threadIdx.x, NT = kLinkThreads, la = U.la, lb = U.lb, lpa = U.lpa, lpb = U.lpb, nca = NCUM(la),
             ncb = NCUM(lb), Lc = U.Lc;
@@ -511,7 +520,7 @@ static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSme
   {
     const double *Tq = (const double *)(U.scr + U.L.T), *part = (const double *)(U.scr + U.L.part);
     const unsigned *mask = (const unsigned *)(U.scr + U.L.mask);
-    const int nParts = t2_parts(U.NP, J.exact), nIt = class_items(J, U.cls * LE, LE);
+    const int nParts = t2_parts(U.NP, J.single), nIt = class_items(J, U.cls * LE, LE);
 #pragma unroll 1
     for (int q = tid; q < U.nItems; q += NT) {
       double v;
@@ -527,94 +536,190 @@ static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSme
     }
   }
   __syncthreads();
-  auto poly_shift = [&](double norm, double *dst) {  // src/util.c:247-334
+  const double norm1 = 4.0 * kPi, norm2 = norm1 * norm1;
+  if constexpr (kExact) {
+    auto poly_shift = [&](double norm, double *dst) {  // src/util.c:247-334
+      const int D = J.uspD, nta = NCART(lpa), ntb = NCART(lpb);
+      const double *uA = J.usp + cA * D * D * D, *uB = J.usp + cB * D * D * D;
+#pragma unroll 1
+      for (int e = tid; e < nta * ncb; e += NT) {
+        int c1 = e / ncb, q = e % ncb;
+        const int *ex = J.ijk + 3 * (NCUM(lpa - 1) + c1);
+        double v = 0.0;
+#pragma unroll 1
+        for (int x = 0; x <= ex[0]; x++) {
+          double bx = binom_tab(ex[0], x);
+#pragma unroll 1
+          for (int y = 0; y <= ex[1]; y++) {
+            double by = bx * binom_tab(ex[1], y);
+#pragma unroll 1
+            for (int zz = 0; zz <= ex[2]; zz++) {
+              double bz = by * binom_tab(ex[2], zz);
+              double factor = bz * uA[((ex[0] - x) * D + (ex[1] - y)) * D + (ex[2] - zz)];
+              if (fabs(factor) <= J.acc) continue;
+              v += factor * chi[J.ijkIdx[(x * dd + y) * dd + zz] * ncb + q];
+            }
+          }
+        }
+        Jsh[e] = v;
+      }
+      __syncthreads();
+#pragma unroll 1
+      for (int e = tid; e < nta * ntb; e += NT) {
+        int c1 = e / ntb, c2 = e % ntb;
+        const int *ex = J.ijk + 3 * (NCUM(lpb - 1) + c2);
+        double v = 0.0;
+#pragma unroll 1
+        for (int x = 0; x <= ex[0]; x++) {
+          double bx = binom_tab(ex[0], x);
+#pragma unroll 1
+          for (int y = 0; y <= ex[1]; y++) {
+            double by = bx * binom_tab(ex[1], y);
+#pragma unroll 1
+            for (int zz = 0; zz <= ex[2]; zz++) {
+              double bz = by * binom_tab(ex[2], zz);
+              double factor = bz * uB[((ex[0] - x) * D + (ex[1] - y)) * D + (ex[2] - zz)];
+              if (fabs(factor) <= J.acc) continue;
+              factor *= norm;
+              v += factor * Jsh[c1 * ncb + J.ijkIdx[(x * dd + y) * dd + zz]];
+            }
+          }
+        }
+        dst[e] = v;
+      }
+      __syncthreads();
+    };
+    poly_shift(norm1, out1);
+    // gamma (src/type2.c:583-623)
+    {
+      const double *angA = J.ang + cA * J.angLam * J.angLM * J.angC;
+      const double *angB = J.ang + cB * J.angLam * J.angLM * J.angC;
+      const int LMd = J.angLM, AC = J.angC;
+#pragma unroll 1
+      for (int e = tid; e < nca * ncb; e += NT) {
+        int pidx = e / ncb, qidx = e % ncb, alpha = 0, beta = 0;
+        while (NCUM(alpha) <= pidx) alpha++;
+        while (NCUM(beta) <= qidx) beta++;
+        double g = 0.0;
+#pragma unroll 1
+        for (int l = 0; l < Lc; l++) {
+          int ll1 = l - alpha, p1 = (alpha + l) % 2;
+          if (p1 > ll1) ll1 = p1;
+          int ll2 = l - beta, p2 = (beta + l) % 2;
+          if (p2 > ll2) ll2 = p2;
+          double tmp = 0.0;
+#pragma unroll 1
+          for (int l1 = ll1; l1 <= la + l; l1 += 2)
+#pragma unroll 1
+            for (int l2 = ll2; l2 <= lb + l; l2 += 2) {
+              double factor = 0.0;
+#pragma unroll 1
+              for (int m = 0; m < 2 * l + 1; m++)
+                factor += angA[((size_t)l1 * LMd + l * l + m) * AC + pidx] * angB[((size_t)l2 * LMd + l * l + m) * AC + qidx];
+              tmp += factor * T[tidx(l, l1, l2, alpha + beta)];
+            }
+          g += tmp;
+        }
+        chi[e] = g;
+      }
+    }
+    __syncthreads();
+    poly_shift(norm2, out2);
+  } else {
+    // the shift's factors binomial * (-R)^(e - x) once per unit, a row of up to
+    // 12 per Cartesian function, l <= 4 (0 where the reference skips one); then both
+    // blocks' shifts are one multiply-add a term
+    double *fA = sm + Lm.fac, *fB = fA + NCART(lpa) * kShiftTerms;
     const int D = J.uspD, nta = NCART(lpa), ntb = NCART(lpb);
     const double *uA = J.usp + cA * D * D * D, *uB = J.usp + cB * D * D * D;
 #pragma unroll 1
-    for (int e = tid; e < nta * ncb; e += NT) {
-      int c1 = e / ncb, q = e % ncb;
-      const int *ex = J.ijk + 3 * (NCUM(lpa - 1) + c1);
-      double v = 0.0;
+    for (int e = tid; e < (nta + ntb) * kShiftTerms; e += NT) {
+      const bool b = e >= nta * kShiftTerms;
+      const int f = b ? e - nta * kShiftTerms : e, c1 = f / kShiftTerms, i = f % kShiftTerms;
+      const int *ex = J.ijk + 3 * (NCUM((b ? lpb : lpa) - 1) + c1);
+      const int ny = ex[1] + 1, nz = ex[2] + 1;
+      if (i >= (ex[0] + 1) * ny * nz) continue;
+      const int x = i / (ny * nz), y = i / nz % ny, z = i % nz;
+      const double v = binom_tab(ex[0], x) * binom_tab(ex[1], y) * binom_tab(ex[2], z) *
+                       (b ? uB : uA)[((ex[0] - x) * D + (ex[1] - y)) * D + (ex[2] - z)];
+      fA[e] = fabs(v) <= J.acc ? 0.0 : v;
+    }
+    auto shift = [&](double norm, double *dst) {
 #pragma unroll 1
-      for (int x = 0; x <= ex[0]; x++) {
-        double bx = binom_tab(ex[0], x);
+      for (int pass = 0; pass < 2; pass++) {
+        // J = shift_A chi, then dst = norm J shift_B^T
+        const double *fac = pass ? fB : fA;
+        const int l = pass ? lpb : lpa, nOut = pass ? nta * ntb : nta * ncb, w = pass ? ntb : ncb;
 #pragma unroll 1
-        for (int y = 0; y <= ex[1]; y++) {
-          double by = bx * binom_tab(ex[1], y);
+        for (int e = tid; e < nOut; e += NT) {
+          const int i = e / w, j = e % w, c1 = pass ? j : i;
+          const int *ex = J.ijk + 3 * (NCUM(l - 1) + c1);
+          const double *f = fac + c1 * kShiftTerms, *src = pass ? Jsh + i * ncb : chi + j;
+          const int step = pass ? 1 : ncb;
+          double v = 0.0;
 #pragma unroll 1
-          for (int zz = 0; zz <= ex[2]; zz++) {
-            double bz = by * binom_tab(ex[2], zz);
-            double factor = bz * uA[((ex[0] - x) * D + (ex[1] - y)) * D + (ex[2] - zz)];
-            if (fabs(factor) <= J.acc) continue;
-            v += factor * chi[J.ijkIdx[(x * dd + y) * dd + zz] * ncb + q];
+          for (int x = 0; x <= ex[0]; x++)
+#pragma unroll 1
+            for (int y = 0; y <= ex[1]; y++)
+#pragma unroll 1
+              for (int z = 0; z <= ex[2]; z++, f++)
+                if (*f != 0.0) v = fma(*f, src[J.ijkIdx[(x * dd + y) * dd + z] * step], v);
+          if (pass) dst[e] = norm * v;
+          else Jsh[e] = v;
+        }
+        __syncthreads();
+      }
+    };
+    __syncthreads();
+    shift(norm1, out1);
+    // gamma (src/type2.c:583-623), for every channel l and bra degree alpha in
+    // two steps: Y[m][l1][q] = sum over l2 of Omega_B T, then the sum over
+    // (m, l1) of Omega_A Y -- the radial table enters once per (l1, q) instead of
+    // once per (p, q).  Omega_A vanishes for l1 > l + alpha.
+    {
+      const double *angA = J.ang + cA * J.angLam * J.angLM * J.angC;
+      const double *angB = J.ang + cB * J.angLam * J.angLM * J.angC;
+      const int LMd = J.angLM, AC = J.angC;
+      double *Y = sm + Lm.rsh;
+#pragma unroll 1
+      for (int e = tid; e < nca * ncb; e += NT) chi[e] = 0.0;
+#pragma unroll 1
+      for (int l = 0; l < Lc; l++)
+#pragma unroll 1
+        for (int alpha = 0; alpha <= la; alpha++) {
+          const int lo1 = l > alpha ? l - alpha : (alpha + l) & 1, n1 = (l + alpha - lo1) / 2 + 1, M = 2 * l + 1;
+          __syncthreads();
+#pragma unroll 1
+          for (int e = tid; e < M * n1 * ncb; e += NT) {
+            const int q = e % ncb, r = e / ncb, l1 = lo1 + 2 * (r % n1), m = r / n1;
+            int beta = 0;
+            while (NCUM(beta) <= q) beta++;
+            const int lo2 = l > beta ? l - beta : (beta + l) & 1;
+            const double *B = angB + ((size_t)lo2 * LMd + l * l + m) * AC + q;
+            const double *t = T + tidx(l, l1, lo2, alpha + beta);
+            double v = 0.0;
+#pragma unroll 1
+            for (int l2 = lo2; l2 <= l + beta; l2 += 2, B += 2 * (size_t)LMd * AC, t += 2 * nA) v = fma(*B, *t, v);
+            Y[e] = v;
+          }
+          __syncthreads();
+          const int p0 = NCUM(alpha - 1);
+#pragma unroll 1
+          for (int e = tid; e < NCART(alpha) * ncb; e += NT) {
+            const int p = p0 + e / ncb, q = e % ncb;
+            double v = 0.0;
+#pragma unroll 1
+            for (int m = 0; m < M; m++)
+#pragma unroll 1
+              for (int i = 0; i < n1; i++)
+                v = fma(angA[((size_t)(lo1 + 2 * i) * LMd + l * l + m) * AC + p], Y[(m * n1 + i) * ncb + q], v);
+            chi[p * ncb + q] += v;
           }
         }
-      }
-      Jsh[e] = v;
     }
     __syncthreads();
-#pragma unroll 1
-    for (int e = tid; e < nta * ntb; e += NT) {
-      int c1 = e / ntb, c2 = e % ntb;
-      const int *ex = J.ijk + 3 * (NCUM(lpb - 1) + c2);
-      double v = 0.0;
-#pragma unroll 1
-      for (int x = 0; x <= ex[0]; x++) {
-        double bx = binom_tab(ex[0], x);
-#pragma unroll 1
-        for (int y = 0; y <= ex[1]; y++) {
-          double by = bx * binom_tab(ex[1], y);
-#pragma unroll 1
-          for (int zz = 0; zz <= ex[2]; zz++) {
-            double bz = by * binom_tab(ex[2], zz);
-            double factor = bz * uB[((ex[0] - x) * D + (ex[1] - y)) * D + (ex[2] - zz)];
-            if (fabs(factor) <= J.acc) continue;
-            factor *= norm;
-            v += factor * Jsh[c1 * ncb + J.ijkIdx[(x * dd + y) * dd + zz]];
-          }
-        }
-      }
-      dst[e] = v;
-    }
-    __syncthreads();
-  };
-  const double norm1 = 4.0 * kPi, norm2 = norm1 * norm1;
-  poly_shift(norm1, out1);
-  // gamma (src/type2.c:583-623)
-  {
-    const double *angA = J.ang + cA * J.angLam * J.angLM * J.angC;
-    const double *angB = J.ang + cB * J.angLam * J.angLM * J.angC;
-    const int LMd = J.angLM, AC = J.angC;
-#pragma unroll 1
-    for (int e = tid; e < nca * ncb; e += NT) {
-      int pidx = e / ncb, qidx = e % ncb, alpha = 0, beta = 0;
-      while (NCUM(alpha) <= pidx) alpha++;
-      while (NCUM(beta) <= qidx) beta++;
-      double g = 0.0;
-#pragma unroll 1
-      for (int l = 0; l < Lc; l++) {
-        int ll1 = l - alpha, p1 = (alpha + l) % 2;
-        if (p1 > ll1) ll1 = p1;
-        int ll2 = l - beta, p2 = (beta + l) % 2;
-        if (p2 > ll2) ll2 = p2;
-        double tmp = 0.0;
-#pragma unroll 1
-        for (int l1 = ll1; l1 <= la + l; l1 += 2)
-#pragma unroll 1
-          for (int l2 = ll2; l2 <= lb + l; l2 += 2) {
-            double factor = 0.0;
-#pragma unroll 1
-            for (int m = 0; m < 2 * l + 1; m++)
-              factor += angA[((size_t)l1 * LMd + l * l + m) * AC + pidx] * angB[((size_t)l2 * LMd + l * l + m) * AC + qidx];
-            tmp += factor * T[tidx(l, l1, l2, alpha + beta)];
-          }
-        g += tmp;
-      }
-      chi[e] = g;
-    }
+    shift(norm2, out2);
   }
-  __syncthreads();
-  poly_shift(norm2, out2);
   if (tid == 0) {
     const int warn = ((const UnitHead *)U.scr)->warn;
     const long long u = (long long)U.c * J.nPairs + U.pr;
