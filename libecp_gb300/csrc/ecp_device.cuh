@@ -164,6 +164,7 @@ static __constant__ int c_shiftB[3][10] = {{0}, {0, 0, +1, -1}, {0, 0, +1, -1, +
 // c times z, n times in a row: the reference's zeta^n derivative factors
 // (src/type1.c:239-246, src/type2.c:459-462); n <= 0 leaves c.
 static __device__ inline double zeta_times(double c, double z, int n) {
+#pragma unroll 1
   for (int k = 0; k < n; k++) c *= z;
   return c;
 }

@@ -161,10 +161,10 @@ struct JobPlan {
 // Launch configuration of the batched path (picked by the autotuner).
 struct FastConfig {
   int queue = 1;   // 1: the units that compute blocks (with screen); 0: every unit
-  int sorted = 1;  // pairs 1: by descending estimated cost; 2: class-major; 0: the reference's order
-  int gcap = 45;   // type-1 step-table width cap; smaller caps fit more CTAs per SM
+  int sorted = 2;  // pairs 1: by descending estimated cost; 2: class-major; 0: the reference's order
+  int gcap = 33;   // type-1 step-table width cap; smaller caps fit more warps per SM
   int mixed = 0;   // set from the job's mode (ECPGB_MIXED), not tuned
-  int balance = 1; // narrower type-1 groups when a unit has few primitive pairs
+  int balance = 0; // 1: narrower type-1 groups when a unit has few primitive pairs
   int screen = 1;  // with queue: a screening stage compacts the queue to live units
   // per-(la, lb)-class type-1 cap and balance (DevJob::classCfg); the launch's
   // shared memory is sized by gcap, so a class's cap is at most gcap

@@ -52,6 +52,9 @@ static __device__ __noinline__ void bessel_fx(const DevJob &J, int lmax, xf z100
   fx_bessel_rows(J.besX, J.besXA, J.besHL + 1, lmax, z100, mul, sign, K);
 }
 
+// Powers of r other than 0, 1, 2: rare, out of line.
+static __device__ __noinline__ double rpow_rare(double r, double n) { return rpow(r, n); }
+
 // Adds one ECP term d r^n exp(-a r^2) (R2 = r^2) to a channel's sum.  A term
 // below 2^-70 of what the sum holds is left out (the sum carries 60 bits), and
 // one whose exponential underflows.
@@ -65,11 +68,11 @@ static __device__ inline void ecp_term_fx(const DevJob &J, int t, double r, xf R
   // (n <= 2; r^n otherwise unknown: never left out)
   const int rn = n == 0.0 ? 0 : n == 1.0 ? R.e + 64 : n == 2.0 ? R2.e + 64 : 100000;
   const int b = D.e + 64 + rn - (int)(((u64)(uint32_t)(E >> 32) * 1477) >> 31);
-  if (b < acc.e - 10 + (63 - clz64((u64)(acc.m < 0 ? -acc.m : acc.m) | 1u)) - 60) return;
+  if (b < acc.v.e + (63 - clz64((u64)(acc.v.m < 0 ? -acc.v.m : acc.v.m) | 1u)) - 70) return;
   xf v = xf_mul(fx_exp(-(i64)E), D);
   if (n == 1.0) v = xf_mul(v, R);
   else if (n == 2.0) v = xf_mul(v, R2);
-  else if (n != 0.0) v = xf_mul(v, xf_from(rpow(r, n)));  // other powers: rare
+  else if (n != 0.0) v = xf_mul(v, xf_from(rpow_rare(r, n)));
   acc.add(v, sign_of(J.termD[t]));
 }
 
@@ -122,7 +125,7 @@ static __device__ __noinline__ void channels_masked(const DevJob &J, int c, doub
     for (; t < t1 && J.termL[t] == l; t++)
       if (use) ecp_term_fx(J, t, r, R, R2, acc);
     if (use) {
-      const double v = acc.value();
+      const double v = xs_to_double(acc.v);
       if (seen >> l & 1u) U[l] += v;
       else U[l] = v;
       seen |= 1u << l;
@@ -138,8 +141,8 @@ static __device__ __noinline__ xf channel(const DevJob &J, int c, int l, double 
 #pragma unroll 1
   for (int t = t0; t < t1; t++)
     if (J.termL[t] == l) ecp_term_fx(J, t, r, R, R2, acc);
-  sign = acc.m < 0 ? 0x80000000u : 0u;
-  return {acc.m < 0 ? (u64)-acc.m : (u64)acc.m, acc.e};
+  sign = acc.v.m < 0 ? 0x80000000u : 0u;
+  return xs_abs(acc.v);
 }
 
 // ------------------------------------------- double-single (mixed path)
@@ -238,144 +241,107 @@ static __device__ __noinline__ ff channel_ff(const DevJob &J, int c, int l, ff r
 }
 
 
-// The factors of an integrand value, from table entries: mantissa, exponent
-// and sign of a double.
-struct xfs {
-  xf v;
-  uint32_t s;
+// A level's constants of both rules, in shared memory: tol 3 n / 16 and 16 / (3 n).
+constexpr int kMaxLevels = 16;
+struct LevelTab {
+  u64 cm[kMaxLevels], rm[kMaxLevels];
+  int ce[kMaxLevels], re[kMaxLevels];
 };
-static __device__ inline xfs xfs_from(double x) { return {xf_from(x), sign_of(x)}; }
-static __device__ inline xfs operator*(xfs a, xfs b) { return {xf_mul(a.v, b.v), a.s ^ b.s}; }
-
-// A level's end of the PSM92 walk (src/gc_integrators.c:39-86): true when the
-// level's test accepts, with the result.
-static __device__ inline bool psm92_level(int k, double tol16, double I, double p, double q, double &res) {
-  const double N3 = c92_3N[k], e = I - p;
-  // 16 e^2 <= 3 N |I - q| tol
-  if (!(e * e <= N3 * fabs(I - q) * tol16)) return false;
-  res = 16 * I / N3;
-  return true;
-}
-
-// PSM92 walker (src/gc_integrators.c:39-86) over slots [s0, s1) of the
-// large-grid schedule; add(pos, sum) adds w * f at slot pos; vis(pos) whether
-// the (upper) point counts.  A level is summed with 60-bit mantissas on the
-// integer pipes and added to the FP64 running sum at its end (and at the end
-// of the slots walked, so that I is complete between calls).
-template <class Add, class Vis>
-static __device__ inline void psm92_advance(int s0, int s1, double tol, Add add, Vis vis,
-                                            double &I, double &p, double &q, bool &done, double &res) {
-  // one copy of the integrand code: slot 0 is a level of its own
-  xf_sum sum;
-  int k = s0 == 0 ? -1 : level_of(s0);
-  int lvStart = k <= 0 ? 1 : c92_lvEnd[k - 1], lvEnd = k < 0 ? 1 : c92_lvEnd[k];
-#pragma unroll 1
-  for (int t = s0; t < s1 && !done; t++) {
-    if (t == lvStart && k >= 0) {
-      q = 2 * p;
-      p = 2 * I;
-    }
-    if ((t & 1) || t == 0 || vis(t)) add(t, sum);  // even slots (after 0) are the upper points
-    if (t + 1 == lvEnd) {
-      I += sum.value();
-      sum = xf_sum();
-      if (k < 0) p = I;
-      else done = psm92_level(k, tol * 0.0625, I, p, q, res);
-      k++;
-      lvStart = lvEnd;
-      lvEnd = c92_lvEnd[k];  // k <= the level count, inside the 32-entry table
-    }
+static __device__ inline void level_tab(LevelTab &T, const double *n3, int levels, double tol) {
+  const int k = threadIdx.x & 31;
+  if (k < levels && k < kMaxLevels) {
+    const xf c = xf_norm(xf_mul(xf_from(n3[k]), xf_from(tol)));
+    const xf r = xf_from(1.0 / n3[k]);  // the quotient's rounding: half an ulp
+    T.cm[k] = c.m;
+    T.ce[k] = c.e - 4;
+    T.rm[k] = r.m;
+    T.re[k] = r.e + 4;
   }
-  if (sum.m) I += sum.value();
+  __syncwarp();
 }
 
-// PS93 walk of ps93_walk (src/gc_integrators.c:157-217) with the error test
-// 16 d / (3 n) < tol written as d < tol 3 n / 16: no divide per level (the
-// same decision but within an ulp of the threshold); add(n, sum) adds w * f at
-// point n.  Levels are summed as in psm92_advance.  A level's update and
-// test: true when it accepts (cnt points counted).
-static __device__ inline bool ps93_level(int k, double tol16, int cnt, double I, double &p, double &q, double &res) {
-  const double n3 = c93_3n[k];
-  double d;
+// Table entries are doubles that are never subnormal; a zero counts as
+// 2^-1023.  Mantissa, biased exponent (of a positive entry) and high word.
+static __device__ inline u64 ent_m(double x) { return ((u64)dbits(x) << 11) | (1ull << 63); }
+static __device__ inline uint32_t ent_h(double x) { return (uint32_t)((u64)dbits(x) >> 32); }
+constexpr int kEntBias = 1023 + 63;
+
+// xs_add and xs_times out of line: the level ends use them several times, and
+// one copy keeps the kernels' loops in the instruction cache.
+static __device__ __noinline__ xs xs_plus(xs a, xs b) { return xs_add(a, b); }
+static __device__ __noinline__ double xs_scaled(xs a, xf c) { return xs_times(a, c); }
+
+// A quadrature's state between levels: the running sum now, and at the ends
+// of the last two levels.
+struct Psm92 {
+  xs I, I1, I2;
+};
+// After slot 0: p = I, so q = 2 p = 4 (I / 2) on the first level.
+static __device__ inline void psm92_head(Psm92 &S) {
+  S.I1 = S.I;
+  S.I2 = xs_shl(S.I, -1);
+}
+// A level's end of the PSM92 walk (src/gc_integrators.c:39-86), T its sum: p =
+// 2 I1 and q = 4 I2 there, and the test is 16 e^2 <= 3 N |I - q| tol.
+static __device__ inline bool psm92_end(Psm92 &S, const LevelTab &L, int k) {
+  const xs e = xs_plus(S.I, xs_shl(xs_neg(S.I1), 1)), d = xs_plus(S.I, xs_shl(xs_neg(S.I2), 2));
+  S.I2 = S.I1;
+  S.I1 = S.I;
+  const xf a = xs_abs(e), b = norm1(xf_mul(xs_abs(d), {L.cm[k], L.ce[k]}));
+  return a.m == 0 || xf_le(norm1(xf_mul(a, a)), b);
+}
+static __device__ inline double psm92_result(const Psm92 &S, const LevelTab &L, int k) {
+  return xs_scaled(S.I1, {L.rm[k], L.re[k]});
+}
+
+// State of the PS93 walk (src/gc_integrators.c:157-217) and its level end: true
+// when the level's test 16 d / (3 n) < tol accepts (cnt points counted).
+struct Ps93 {
+  xs I, p, q;
+};
+static __device__ inline bool ps93_end(Ps93 &S, const LevelTab &L, int k, int cnt) {
+  xs d;
   if (c93_lvJ[k]) {
-    d = fabs(I - 2 * q);
-    q = I;
+    d = xs_plus(S.I, xs_shl(xs_neg(S.q), 1));
+    S.q = S.I;
   } else {
-    p += I - q;
-    d = fabs(q - 3 * p / 2);
+    S.p = xs_plus(S.p, xs_plus(S.I, xs_neg(S.q)));
+    const xs h = xs_plus(S.p, xs_shl(S.p, -1));  // 3 p / 2
+    d = xs_plus(S.q, xs_neg(h));
   }
-  if (cnt == 0 || !(d < tol16 * n3)) return false;
-  res = 16 * q / n3;
-  return true;
+  return cnt > 0 && xf_lt(xs_abs(d), {L.cm[k], L.ce[k]});
 }
-template <class Add>
-static __device__ bool ps93_walk_fast(int start, int end, double tol, Add add, double &res) {
-  // one copy of the integrand code: slot 0 and slots 1, 2 are levels of
-  // their own (-2, -1)
-  xf_sum sum;
-  double p = 0, q = 0, I = 0;
-  int k = -2, lvEnd = 1, cnt = 0;
-#pragma unroll 1
-  for (int t = 0;; t++) {
-    const int n = c93_slot[t];
-    // (the integrand is 0 outside [start, end))
-    if (n >= start && n < end) add(n, sum);
-    cnt += (t & 1) ? n >= start : n <= end;
-    if (t + 1 < lvEnd) continue;
-    const double v = sum.value();
-    sum = xf_sum();
-    I += v;
-    if (k == -2) p = v;
-    else if (k == -1) q = v;
-    else if (ps93_level(k, tol * 0.0625, cnt, I, p, q, res)) return true;
-    if (++k >= c93_nLevels) break;
-    lvEnd = k < 0 ? 3 : c93_lvEnd[k];
-    cnt = 0;
-  }
-  res = 16 * q / c93_3n[c93_nLevels - 1];  // the last estimate (mixed path: its size)
-  return false;
+static __device__ inline double ps93_result(const Ps93 &S, const LevelTab &L, int k) {
+  return xs_scaled(S.q, {L.rm[k], L.re[k]});
 }
 
-// psm92_advance over the slots [s0, s1) whose bit is set in `bits`; the
-// other slots integrate to exactly zero, so (lower, upper) pairs without a set
-// bit are skipped -- adding 0.0 changes no sum -- while every level end is
-// still visited in order for the convergence test.
-template <class Add, class Vis>
-static __device__ inline void psm92_sparse(int s0, int s1, const unsigned *bits, double tol, Add add,
-                                           Vis vis, double &I, double &p, double &q, bool &done, double &res) {
-  int pos = s0;
-  xf_sum sum;
-  int k = s0 == 0 ? -1 : level_of(s0);
+// Lanes of a warp dealt to n running quadratures: P = 2^b lanes each, so that
+// a run of points is summed by P lanes side by side (the sums of 57-bit
+// integers then combine by shuffles).
+struct LaneDeal {
+  int P;     // lanes per quadrature
+  int rank;  // the quadrature this lane works for, n or more: none
+  int part;  // which of its P lanes
+};
+static __device__ inline LaneDeal deal_lanes(int n) {
+  const int b = n > 16 ? 0 : n > 8 ? 1 : n > 4 ? 2 : 3, lane = threadIdx.x & 31;
+  return {1 << b, lane >> b, lane & ((1 << b) - 1)};
+}
+static __device__ inline xs combine(xs a, int P) {
 #pragma unroll 1
-  while (pos < s1 && !done) {
-    const int lvStart = k <= 0 ? 1 : c92_lvEnd[k - 1], lvE = k < 0 ? 1 : c92_lvEnd[k];
-    if (pos == lvStart && k >= 0) {
-      q = 2 * p;
-      p = 2 * I;
-    }
-    const int stop = lvE < s1 ? lvE : s1;
-    // every set bit in [pos, stop)
-#pragma unroll 1
-    for (int w = pos >> 5; (w << 5) < stop; w++) {
-      unsigned word = bits[w];
-      if (w == (pos >> 5)) word &= ~0u << (pos & 31);
-      if ((w << 5) + 32 > stop) word &= ~(~0u << (stop & 31));
-#pragma unroll 1
-      for (; word; word &= word - 1u) {
-        const int t = (w << 5) + __ffs(word) - 1;
-        if ((t & 1) || t == 0 || vis(t)) add(t, sum);  // even slots (after 0) are the upper points
-      }
-    }
-    pos = stop;
-    if (pos == lvE) {
-      I += sum.value();
-      sum = xf_sum();
-      if (k < 0) p = I;
-      else done = psm92_level(k, tol * 0.0625, I, p, q, res);
-      k++;
-    }
+  for (int o = 1; o < P; o <<= 1) {
+    xs b;
+    b.m = __shfl_xor_sync(0xffffffffu, a.m, o);
+    b.e = __shfl_xor_sync(0xffffffffu, a.e, o);
+    a = xs_plus(a, b);
   }
-  if (sum.m) I += sum.value();
+  return a;
+}
+static __device__ inline xs from_lane(xs a, int src) {
+  xs b;
+  b.m = __shfl_sync(0xffffffffu, a.m, src);
+  b.e = __shfl_sync(0xffffffffu, a.e, src);
+  return b;
 }
 
 // psm92_advance with val(pos) in ff: each level summed with a compensated
@@ -415,57 +381,36 @@ static __device__ inline void psm92_advance_ff(int s0, int s1, double tol, V val
   I += acc.value();
 }
 
-// psm92_sparse with val(pos) in ff, levels summed as in psm92_advance_ff.
-template <class V, class Vis>
-static __device__ inline void psm92_sparse_ff(int s0, int s1, const unsigned *bits, double tol, V val, Vis vis,
-                                              double &I, double &p, double &q, bool &done, double &res) {
-  auto has = [&](int t) { return (bits[t >> 5] >> (t & 31)) & 1u; };
-  int pos = s0;
-  if (pos == 0) {
-    I = has(0) ? ff_to_double(val(0)) : 0.0;
-    p = I;
-    pos = 1;
-  }
-  int k = level_of(pos);
-  ff_acc acc;
+// psm92_advance_ff over the queued slots pend[0 .. nE), which lie in [s0, s1);
+// val(i) of entry i.
+template <class V>
+static __device__ inline void psm92_queue_ff(int s0, int s1, const int *pend, int nE, double tol, V val, double &I,
+                                             double &p, double &q, bool &done, double &res) {
+  int i = 0, pos = s0, k = s0 == 0 ? -1 : level_of(s0);
+#pragma unroll 1
   while (pos < s1 && !done) {
-    const int lvStart = k == 0 ? 1 : c92_lvEnd[k - 1];
-    if (pos == lvStart) {
+    const int lvStart = k <= 0 ? 1 : c92_lvEnd[k - 1], lvE = k < 0 ? 1 : c92_lvEnd[k];
+    if (pos == lvStart && k >= 0) {
       q = 2 * p;
       p = 2 * I;
     }
-    const int lvE = c92_lvEnd[k], stop = lvE < s1 ? lvE : s1;
-    while (true) {
-      int t = stop;  // first set bit in [pos, stop)
-      for (int w = pos >> 5; (w << 5) < stop; w++) {
-        unsigned word = bits[w];
-        if (w == (pos >> 5)) word &= ~0u << (pos & 31);
-        if (word) {
-          t = (w << 5) + __ffs(word) - 1;
-          break;
-        }
-      }
-      if (t >= stop) {
-        pos = stop;
-        break;
-      }
-      const int ps = (t - 1) | 1;  // the (lower, upper) pair holding t
-      if (has(ps)) acc.add(val(ps));
-      if (has(ps + 1) && vis(ps + 1)) acc.add(val(ps + 1));
-      pos = ps + 2;
-    }
+    pos = lvE < s1 ? lvE : s1;
+    ff_acc acc;
+#pragma unroll 1
+    for (; i < nE && pend[i] < pos; i++) acc.add(val(i));
+    I += acc.value();
     if (pos == lvE) {
-      I += acc.value();
-      acc = ff_acc();
-      double N = c92_lvN[k] + 1.0, e = I - p;
-      if (16 * e * e <= 3 * N * fabs(I - q) * tol) {
-        res = 16 * I / (3 * N);
-        done = true;
+      if (k < 0) p = I;
+      else {
+        const double N3 = c92_3N[k], e = I - p;
+        if (16 * e * e <= N3 * fabs(I - q) * tol) {
+          res = 16 * I / N3;
+          done = true;
+        }
       }
       k++;
     }
   }
-  I += acc.value();
 }
 
 PairPlan pair_plan(int NP, int la, int lb, int nItems, bool single) {
@@ -565,7 +510,7 @@ static __device__ __noinline__ bool t1_large_entry(const DevJob &J, int c, int L
   const xf R = xf_from(r);
   uint32_t sign;
   xf v = channel(J, c, Lc, r, sign);
-  v = xf_mul(xf_mul(fx_exp(fx_q53(ex)), xf_norm(v)),
+  v = xf_mul(xf_mul(fx_exp(fx_q53(ex)), v),
              xf_mul(xf_from(C2), xf_from(w)));
   if (v.m == 0) return false;
   sign ^= sign_of(C2) ^ sign_of(w);
@@ -581,13 +526,34 @@ static __device__ __noinline__ bool t1_large_entry(const DevJob &J, int c, int L
 
 // --------------------------------------------------- stage 2: the small grid
 
+// A primitive pair's scalars for the small grid, out of line (one copy for the
+// kinds): |P| (as src/util.c:75-106), the prefactor, -za - zb, and for the
+// normal kind s and Z r (r inside the window) as integers times 2^q, both
+// below 2^62.
+static __device__ __noinline__ void t1_pair_setup(const DevJob &J, const Unit &U, int k, double *sc, PairFx *fx) {
+  const int i = k / U.Nb, j = k - i * U.Nb;
+  // derivative blocks: coefficients times zeta^max(0, shift) (src/type1.c:239-246)
+  const double za = U.pzA[i], ca = zeta_times(U.pcA[i], za, U.pa0), zb = U.pzB[j], cb = zeta_times(U.pcB[j], zb, U.pb0);
+  double P[3];
+  for (int x = 0; x < 3; x++) P[x] = 2.0 * (za * U.gA[x] + zb * U.gB[x]);
+  const double s = sqrt(P[0] * P[0] + P[1] * P[1] + P[2] * P[2]);
+  sc[0] = s;
+  sc[1] = t1_prefactor(za, ca, zb, cb, U.gA[3], U.gB[3]);
+  sc[2] = -za - zb;
+  if (fx) {
+    const xf S = xf_from(s), Z = xf_from(za + zb), s100 = xf_times100(S);
+    const int zr = Z.e + xf_from(J.xSmall[U.we - 1]).e + 64, q = -3 - (S.e > zr ? S.e : zr);
+    *fx = {(i64)shr64(S.m, -(S.e + q)), Z.m, s100.m, Z.e, s100.e, q};
+  }
+}
+
 // A group of G primitive pairs of one kind (perm[p0 ..]) of a unit's type-1
 // quadratures on the small grid (src/type1.c:95-148), by one warp; lane =
 // (pair, quadrature).  Converged quadratures are written to the unit's Q, the
 // pairs with a failed one to the fallback list.
 template <bool kMixed, int kKind>
-static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem &L, double *sm, int pos, int p0,
-                                int G) {
+static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem &L, double *sm, const LevelTab &V,
+                                int pos, int p0, int G) {
   const int lane = threadIdx.x & 31, lab = U.lab, lq = lab + 1, O = kSmallOrder, Nb = U.Nb, ws = U.ws, we = U.we;
   // odd entry strides: lanes touching neighbouring entries hit distinct banks
   const int TS = 1 + 2 * lq, nq = t1_items(lab);
@@ -596,26 +562,8 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
   PairFx *fx = (PairFx *)(sm + L.fx);
   const unsigned char *perm = (const unsigned char *)(U.scr + U.L.perm);
   const double *uL = J.uL + (size_t)U.c * O;
-  // (1) per pair: |P| (as src/util.c:75-106), the prefactor, -za - zb
   __syncwarp();
-  if (lane < G) {
-    const int k = perm[p0 + lane];
-    // derivative blocks: coefficients times zeta^max(0, shift) (src/type1.c:239-246)
-    const double za = U.pzA[k / Nb], ca = zeta_times(U.pcA[k / Nb], za, U.pa0), zb = U.pzB[k % Nb],
-                 cb = zeta_times(U.pcB[k % Nb], zb, U.pb0);
-    double P[3];
-    for (int i = 0; i < 3; i++) P[i] = 2.0 * (za * U.gA[i] + zb * U.gB[i]);
-    const double s = sqrt(P[0] * P[0] + P[1] * P[1] + P[2] * P[2]);
-    sc[lane * 3 + 0] = s;
-    sc[lane * 3 + 1] = t1_prefactor(za, ca, zb, cb, U.gA[3], U.gB[3]);
-    sc[lane * 3 + 2] = -za - zb;
-    if (kKind == kPairNormal) {
-      // s and Z r (r inside the window) as integers times 2^q, both below 2^62
-      const xf S = xf_from(s), Z = xf_from(za + zb), s100 = xf_times100(S);
-      const int zr = Z.e + xf_from(J.xSmall[we - 1]).e + 64, q = -3 - (S.e > zr ? S.e : zr);
-      fx[lane] = {(i64)shr64(S.m, -(S.e + q)), Z.m, s100.m, Z.e, s100.e, q};
-    }
-  }
+  if (lane < G) t1_pair_setup(J, U, perm[p0 + lane], sc + lane * 3, kKind == kPairNormal ? fx + lane : nullptr);
   __syncwarp();
   // (2) PS93: lane = (pair g, quadrature (l1, l2))
   const bool mine = lane < G * nq;
@@ -627,9 +575,10 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
     l2 = l1 - 2 * rem;
   }
   double *Qout = (double *)(U.scr + U.L.Q) + (size_t)perm[p0 + g] * nq + qi;
-  double I = 0, p = 0, q = 0;
-  xf_sum sum;    // the running level (normal kind)
-  double T = 0;  // the running slot pair (band kind)
+  double I = 0, p = 0, q = 0, T = 0;  // band kind, T the running slot pair
+  Ps93 S;                             // normal kind
+  xs lev;                             // its running level
+  int *quad = (int *)(sm + L.quad);   // the running quadratures, by rank
   bool done = !mine;
   int k = -2, cnt = 0, lvEnd = 1;
   if constexpr (kKind == kPairZero) {
@@ -726,50 +675,102 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
       for (int l = 0; l <= 2 * lq; l++) ent[l] = 0.0;
     }
     __syncwarp();
-    auto ent_of = [&](int t) { return tab + ((t - s0) * G + g) * TS; };
-    // band kind: w * ((((C1 r^l1) U) K_l2) exp(e)), each product rounded
-    auto wf = [&](int t, int n) {
-      const double *e = ent_of(t);
-      return __dmul_rn(J.wSmall[n], __dmul_rn(__dmul_rn(e[lq + l1], e[l2]), e[2 * lq]));
-    };
-    // one copy of the integrand code: slot 0 and slots 1, 2 are levels of
-    // their own (-2, -1)
+    if constexpr (kKind == kPairBand) {
+      // w * ((((C1 r^l1) U) K_l2) exp(e)), each product rounded; slot 0 and
+      // slots 1, 2 are levels of their own (-2, -1)
 #pragma unroll 1
-    for (int t = s0; t < s1; t++) {
-      const int n = c93_slot[t];
-      // the points inside the window (the entries outside it are zero)
-      if (!done && n >= ws && n < we) {
-        if constexpr (kKind == kPairBand) T = __dadd_rn(T, wf(t, n));
-        else {
-          const double *e = ent_of(t);
-          const xfs v = xfs_from(e[lq + l1]) * xfs_from(e[l2]);
-          sum.add(v.v, v.s);
+      for (int t = s0; t < s1; t++) {
+        const int n = c93_slot[t];
+        if (!done && n >= ws && n < we) {
+          const double *e = tab + ((t - s0) * G + g) * TS;
+          T = __dadd_rn(T, __dmul_rn(J.wSmall[n], __dmul_rn(__dmul_rn(e[lq + l1], e[l2]), e[2 * lq])));
         }
-      }
-      cnt += (t & 1) ? n >= ws : n <= we;
-      if constexpr (kKind == kPairBand)
+        cnt += (t & 1) ? n >= ws : n <= we;
         if (t > 2 && !(t & 1)) {  // the reference's order: pair by pair
           I += T;
           T = 0.0;
         }
-      if (t + 1 < lvEnd) continue;
-      if (!done) {
-        double v = T;
-        if constexpr (kKind == kPairNormal) v = sum.value();
-        sum = xf_sum();
-        T = 0.0;
-        I += v;
-        double res;
-        if (k == -2) p = v;
-        else if (k == -1) q = v;
-        else if (ps93_level(k, J.tol * 0.0625, cnt, I, p, q, res)) {
-          done = true;
-          *Qout = res;
+        if (t + 1 < lvEnd) continue;
+        if (!done) {
+          if (k == -2) p = T;
+          else if (k == -1) {
+            q = T;
+            I = p + q;
+          } else {
+            const double n3 = c93_3n[k];
+            double d;
+            if (c93_lvJ[k]) {
+              d = fabs(I - 2 * q);
+              q = I;
+            } else {
+              p += I - q;
+              d = fabs(q - 3 * p / 2);
+            }
+            if (cnt > 0 && d < J.tol * 0.0625 * n3) {
+              done = true;
+              *Qout = 16 * q / n3;
+            }
+          }
         }
+        T = 0.0;
+        k++;
+        lvEnd = k < 0 ? 3 : c93_lvEnd[k];  // k <= the level count, inside the 32-entry table
+        cnt = 0;
       }
-      k++;
-      lvEnd = k < 0 ? 3 : c93_lvEnd[k];  // k <= the level count, inside the 32-entry table
-      cnt = 0;
+    } else {
+      // runs of slots of one level, the lanes dealt to the running quadratures
+      const unsigned act = __ballot_sync(0xffffffffu, !done);
+      const LaneDeal D = deal_lanes(__popc(act));
+      const int mine_rank = __popc(act & ((1u << lane) - 1u));
+      if (!done) quad[mine_rank] = g | l1 << 8 | l2 << 16;
+      __syncwarp();
+      const bool work = D.rank < __popc(act);
+      const int qd = work ? quad[D.rank] : 0;
+      const double *eW = tab + (qd & 255) * TS + lq + ((qd >> 8) & 255), *eK = tab + (qd & 255) * TS + (qd >> 16);
+#pragma unroll 1
+      for (int t = s0; t < s1;) {
+        const int te = lvEnd < s1 ? lvEnd : s1;
+        {  // points counted (t < te <= t + 33)
+          const int n = t + lane < te ? __ldg(J.s93 + t + lane) : 0;
+          const bool c = t + lane < te && (((t + lane) & 1) ? n >= ws : n <= we);
+          cnt += __popc(__ballot_sync(0xffffffffu, c));
+          if (te - t > 32) cnt += ((te - 1) & 1) ? c93_slot[te - 1] >= ws : c93_slot[te - 1] <= we;
+        }
+        xf_run run;
+#pragma unroll 1
+        for (int x = t + D.part; x < te; x += D.P) {
+          const int n = __ldg(J.s93 + x);
+          // the points inside the window (the entries outside it are zero)
+          if (work && n >= ws && n < we) {
+            const size_t o = (size_t)(x - s0) * G * TS;
+            const double a = eW[o], b = eK[o];
+            run.add({mul_hi(ent_m(a), ent_m(b)), (int)((ent_h(a) >> 20) & 0x7ff) + (int)(ent_h(b) >> 20) + 64 - 2 * kEntBias},
+                    ent_h(a));
+          }
+        }
+        xs sum = combine(run.sum(), D.P);
+        sum = from_lane(sum, (mine_rank * D.P) & 31);
+        lev = xs_plus(lev, sum);
+        t = te;
+        if (t < lvEnd) break;
+        if (!done) {
+          if (k == -2) S.p = lev;
+          else if (k == -1) {
+            S.q = lev;
+            S.I = xs_plus(S.p, S.q);
+          } else {
+            S.I = xs_plus(S.I, lev);
+            if (ps93_end(S, V, k, cnt)) {
+              done = true;
+              *Qout = ps93_result(S, V, k);
+            }
+          }
+        }
+        lev = xs();
+        k++;
+        lvEnd = k < 0 ? 3 : c93_lvEnd[k];
+        cnt = 0;
+      }
     }
     __syncwarp();
     s0 = s1;
@@ -783,7 +784,8 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
   // last small-grid estimates, by the high words); larger integrals in FP64
   unsigned est = 0, lim = 0;
   if constexpr (kMixed) {
-    est = mine && !done ? (unsigned)((u64)__double_as_longlong(fabs(16 * q / c93_3n[c93_nLevels - 1])) >> 32) : 0u;
+    const double last = kKind == kPairNormal ? ps93_result(S, V, c93_nLevels - 1) : 16 * q / c93_3n[c93_nLevels - 1];
+    est = mine && !done ? (unsigned)((u64)__double_as_longlong(fabs(last)) >> 32) : 0u;
     lim = (unsigned)((u64)__double_as_longlong(ff_limit(J.tol)) >> 32);
   }
 #pragma unroll 1
@@ -800,7 +802,7 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
 // lane: F tables (derivative runs max(0, shift), src/type2.c:563-564) and the
 // r^k U_l table read through L2, 64-bit mantissas in every mode.
 template <bool kMixed>
-static __device__ void t2_small(const DevJob &J, const Unit &U, int q0) {
+static __device__ void t2_small(const DevJob &J, const Unit &U, const LevelTab &V, int q0) {
   const int q = q0 + (threadIdx.x & 31), O = kSmallOrder;
   if (q >= U.nItems) return;
   const int nF = J.nF, nk = J.nk, LE = J.maxLECP > 0 ? J.maxLECP : 1, nRuns = J.nRuns > 0 ? J.nRuns : 1;
@@ -808,19 +810,46 @@ static __device__ void t2_small(const DevJob &J, const Unit &U, int q0) {
   const double *Fa = J.F + (((size_t)U.c * J.nShells + U.sa) * nRuns + U.pa0) * O * nF + l1;
   const double *Fb = J.F + (((size_t)U.c * J.nShells + U.sb) * nRuns + U.pb0) * O * nF + l2;
   const double *Ut = J.utab + (size_t)U.c * O * LE * nk + l * nk + l3;
-  double res;
-  const bool ok = ps93_walk_fast(U.ws, U.we, J.tol,
-                                 [&](int n, xf_sum &a) {
-                                   const xfs f = (xfs_from(__ldg(Fa + n * nF)) * xfs_from(__ldg(Fb + n * nF))) *
-                                                 (xfs_from(__ldg(Ut + (size_t)n * LE * nk)) * xfs_from(J.wSmall[n]));
-                                   a.add(f.v, f.s);
-                                 },
-                                 res);
-  if (ok) ((double *)(U.scr + U.L.T))[q] = res;
-  else {
-    atomicOr((unsigned *)(U.scr + U.L.mask) + (q >> 5), 1u << (q & 31));
-    if (kMixed) atomicMax(&((UnitHead *)U.scr)->est, (u64)__double_as_longlong(fabs(res)));
+  // slot 0 and slots 1, 2 are levels of their own (-2, -1)
+  Ps93 S;
+  xs lev;
+  xf_run run;
+  int k = -2, lvEnd = 1, cnt = 0;
+#pragma unroll 1
+  for (int t = 0;; t++) {
+    const int n = c93_slot[t];
+    // (the integrand is 0 outside the window)
+    if (n >= U.ws && n < U.we) {
+      const xf a = xf_mul(xf_from(__ldg(Fa + n * nF)), xf_from(__ldg(Fb + n * nF)));
+      const double u = __ldg(Ut + (size_t)n * LE * nk);
+      run.add(xf_mul(a, xf_mul(xf_from(u), xf_from(J.wSmall[n]))),
+              ent_h(__ldg(Fa + n * nF)) ^ ent_h(__ldg(Fb + n * nF)) ^ ent_h(u));
+    }
+    cnt += (t & 1) ? n >= U.ws : n <= U.we;
+    if ((t & 31) == 31 || t + 1 == lvEnd) {
+      lev = xs_plus(lev, run.sum());
+      run = xf_run();
+    }
+    if (t + 1 < lvEnd) continue;
+    if (k == -2) S.p = lev;
+    else if (k == -1) {
+      S.q = lev;
+      S.I = xs_plus(S.p, S.q);
+    } else {
+      S.I = xs_plus(S.I, lev);
+      if (ps93_end(S, V, k, cnt)) {
+        ((double *)(U.scr + U.L.T))[q] = ps93_result(S, V, k);
+        return;
+      }
+    }
+    lev = xs();
+    if (++k >= c93_nLevels) break;
+    lvEnd = k < 0 ? 3 : c93_lvEnd[k];
+    cnt = 0;
   }
+  atomicOr((unsigned *)(U.scr + U.L.mask) + (q >> 5), 1u << (q & 31));
+  if (kMixed)
+    atomicMax(&((UnitHead *)U.scr)->est, (u64)__double_as_longlong(fabs(ps93_result(S, V, c93_nLevels - 1))));
 }
 
 // One warp a CTA; each takes up to J.take entries of the type-1 groups, then
@@ -828,6 +857,8 @@ static __device__ void t2_small(const DevJob &J, const Unit &U, int q0) {
 template <bool kMixed>
 __global__ void __launch_bounds__(32, 20) k_unit_small(DevJob J) {
   extern __shared__ double sm[];
+  __shared__ LevelTab V;
+  level_tab(V, c93_3n, c93_nLevels, J.tol);
   const SmallSmem L = small_layout(J.maxLBS, J.gcap);
   const int n1 = (int)J.counters[kCntT1], n = n1 + (int)J.counters[kCntT2];
 #pragma unroll 1
@@ -837,14 +868,14 @@ __global__ void __launch_bounds__(32, 20) k_unit_small(DevJob J) {
     const int2 it = i < n1 ? J.listT1[i] : J.listT2[i - n1];
     const Unit U = unit_load(J, it.x);
     if (i >= n1) {
-      t2_small<kMixed>(J, U, it.y);
+      t2_small<kMixed>(J, U, V, it.y);
       continue;
     }
     const long long t0 = J.classCycles ? clock64() : 0;
     const int p0 = it.y & 1023, G = (it.y >> 10) & 63, kind = it.y >> 16;
-    if (kind == kPairNormal) t1_small<kMixed, kPairNormal>(J, U, L, sm, it.x, p0, G);
-    else if (kind == kPairBand) t1_small<kMixed, kPairBand>(J, U, L, sm, it.x, p0, G);
-    else t1_small<kMixed, kPairZero>(J, U, L, sm, it.x, p0, G);
+    if (kind == kPairNormal) t1_small<kMixed, kPairNormal>(J, U, L, sm, V, it.x, p0, G);
+    else if (kind == kPairBand) t1_small<kMixed, kPairBand>(J, U, L, sm, V, it.x, p0, G);
+    else t1_small<kMixed, kPairZero>(J, U, L, sm, V, it.x, p0, G);
     if (J.classCycles && threadIdx.x == 0) atomicAdd(&J.classCycles[U.cls], (u64)(clock64() - t0));
   }
 }
@@ -854,7 +885,10 @@ __global__ void __launch_bounds__(32, 20) k_unit_small(DevJob J) {
 // The large-grid quadratures of one primitive pair whose small-grid ones
 // (mask, by t1_index) failed (src/type1.c:149-196), one per lane.
 template <bool kMixed>
-static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int kk, bool ffp, unsigned mask, double s) {
+static __device__ void t1_large(const DevJob &J, const Unit &U, const LargeSmem &Ls, double *sm, const LevelTab &V,
+                                int kk, bool ffp, unsigned mask, double s) {
+  double *tab = sm + Ls.tab;
+  int *quad = (int *)(sm + Ls.fail);  // the running quadratures, by rank
   const int lane = threadIdx.x & 31, lab = U.lab, lq = lab + 1, O = kSmallOrder, OL = J.largeOrder, TSf = 3 + 2 * lq;
   const int Nb = U.Nb, ws = U.ws, we = U.we, c = U.c, Lc = U.Lc;
   const double *uL = J.uL + (size_t)c * O;
@@ -901,22 +935,24 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int
     }
   }
   const int end = nb - 1;
-  double I2 = 0, p2 = 0, q2 = 0, res2 = 0;
+  double I2 = 0, p2 = 0, q2 = 0, res2 = 0;  // double-single sums (mixed path)
+  Psm92 S;
   bool done2 = !fail;
+  int k = -1, lvEnd = 1;
 #pragma unroll 1
   for (int s0 = 0; s0 < OL;) {
     const int s1 = step_end92(s0) < OL ? step_end92(s0) : OL;
     // the rows the quadratures still running read
     const int kq = __reduce_max_sync(0xffffffffu, done2 ? 0 : l2);
     const int rq = __reduce_max_sync(0xffffffffu, done2 ? 0 : l1);
-#pragma unroll 1
-    for (int t = s0 + lane; t < s1; t += 32) {
+    bool any = false;  // the lane's slot has an entry that is not zero
+    if (s0 + lane < s1) {
+      const int t = s0 + lane;
       int n = __ldg(J.s92 + t);
       bool upper = t > 0 && ((t - 1) & 1);
       // entry: K_l rows, then the rows w * C2 U_L e^(..) r^l
       double *K = tab + (t - s0) * TSf, *WR = K + lq;
       const double w = J.wLarge[n] * i1;
-      bool any = false;
       if (n < nb && !(upper && n > end)) {
         double r = i1 * J.xLarge[n] + i2, ex = (z * r + s) * r + zd2;
         if (ex >= J.lnAcc1) {
@@ -963,29 +999,57 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int
             }
         }
       }
-      if (!any) {  // zero bits read as 0.0 in FP64 and in ff alike
+      if (kMixed && ffp && !any) {  // zero bits read as 0.0 in ff
 #pragma unroll 1
         for (int l = 0; l <= kq; l++) K[l] = 0.0;
 #pragma unroll 1
         for (int l = 0; l <= rq; l++) WR[l] = 0.0;
       }
     }
+    const unsigned live = __ballot_sync(0xffffffffu, any);
     __syncwarp();
-    if (!done2) {
-      auto vis = [&](int t) { return c92_slot[t] <= end; };
-      if (kMixed && ffp) {
+    if (kMixed && ffp) {
+      if (!done2) {
+        auto vis = [&](int t) { return c92_slot[t] <= end; };
         auto val = [&](int t) {
           const ff *e = (const ff *)(tab + (t - s0) * TSf);
           return ff_mul(e[lq + l1], e[l2]);
         };
         psm92_advance_ff(s0, s1, J.tol, val, vis, I2, p2, q2, done2, res2);
-      } else {
-        auto add = [&](int t, xf_sum &a) {
-          const double *e = tab + (t - s0) * TSf;
-          const xfs v = xfs_from(e[lq + l1]) * xfs_from(e[l2]);
-          a.add(v.v, v.s);
-        };
-        psm92_advance(s0, s1, J.tol, add, vis, I2, p2, q2, done2, res2);
+      }
+    } else {
+      // runs of slots of one level, the lanes dealt to the running
+      // quadratures (entries of points that do not count are zero)
+      const unsigned act = __ballot_sync(0xffffffffu, !done2);
+      const LaneDeal D = deal_lanes(__popc(act));
+      const int mine_rank = __popc(act & ((1u << lane) - 1u));
+      if (!done2) quad[mine_rank] = l1 | l2 << 16;
+      __syncwarp();
+      const bool work = D.rank < __popc(act);
+      const int qd = work ? quad[D.rank] : 0;
+      const double *eW = tab + lq + (qd & 0xffff), *eK = tab + (qd >> 16);
+#pragma unroll 1
+      for (int t = s0; t < s1;) {
+        const int te = lvEnd < s1 ? lvEnd : s1;
+        xf_run run;
+#pragma unroll 1
+        for (int x = t + D.part; x < te; x += D.P)
+          if (work && (live >> (x - s0) & 1u)) {
+            const double a = eW[(x - s0) * TSf], b = eK[(x - s0) * TSf];
+            run.add({mul_hi(ent_m(a), ent_m(b)), (int)((ent_h(a) >> 20) & 0x7ff) + (int)(ent_h(b) >> 20) + 64 - 2 * kEntBias},
+                    ent_h(a));
+          }
+        xs sum = combine(run.sum(), D.P);
+        S.I = xs_plus(S.I, from_lane(sum, (mine_rank * D.P) & 31));
+        t = te;
+        if (t < lvEnd) break;
+        if (k < 0) psm92_head(S);
+        else if (!done2 && psm92_end(S, V, k)) {
+          done2 = true;
+          res2 = psm92_result(S, V, k);
+        }
+        k++;
+        lvEnd = c92_lvEnd[k];  // k <= the level count, inside the 32-entry table
       }
     }
     __syncwarp();
@@ -994,7 +1058,7 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int
   }
   if (fail) {
     if (!done2) {
-      res2 = 16 * I2 / c92_3N[c92_nLevels - 1];
+      res2 = kMixed && ffp ? 16 * I2 / c92_3N[c92_nLevels - 1] : psm92_result(S, V, c92_nLevels - 1);
       atomicOr(&((UnitHead *)U.scr)->warn, 1);
     }
     ((double *)(U.scr + U.L.Q))[(size_t)kk * t1_items(lab) + lane] = res2;
@@ -1006,26 +1070,32 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, double *tab, int
 // (src/type2.c:418-528): integrates the pass's failed items (decoded in
 // `fail`) and adds each result to the partial sums.  mb: the latest break of
 // the earlier pairs, beyond which no earlier pair's buffers are reused.
+constexpr short kNoExp = -32000;  // the exponent of a sum without terms
+static __device__ inline short exp16(int e) { return (short)(e < kNoExp ? kNoExp : e); }
 struct T2Pass {
   int nf;            // failed items of the pass
   unsigned mask;     // channels they read
   int l1, l2, l3;    // highest Ka, Kb and r^l rows
 };
 template <bool kMixed>
-static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &L, double *sm, const T2Pass &S,
-                               int k, int mb, const double2 *map, const int4 *win, bool useFF, int &warn) {
+static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &L, double *sm, const LevelTab &V,
+                               const T2Pass &S0, int k, int mb, const double2 *map, const int4 *win, bool useFF, int &warn) {
   // mixed path: useFF picks the double-single tables and sums for this pass
   // (one copy of the common code for both precisions)
   const bool inFF = kMixed && useFF;
-  const int lane = threadIdx.x & 31, nA = 2 * J.maxLBS + 1, Nb = U.Nb, c = U.c, nf = S.nf;
+  const int lane = threadIdx.x & 31, nA = 2 * J.maxLBS + 1, Nb = U.Nb, c = U.c, nf = S0.nf;
   const int LE = J.maxLECP > 0 ? J.maxLECP : 1, LBE = J.maxLBS + LE, OL = J.largeOrder;
   const int TS = L.tabStride;
   const double *pzA = U.pzA, *pzB = U.pzB;
   const double dAC = U.gA[3], dBC = U.gB[3];
-  double *tab = sm + L.tab, *sI = sm + L.I, *sP = sm + L.P, *sQ = sm + L.Q, *part = sm + L.part;
+  double *tab = sm + L.tab, *part = sm + L.part;
+  // an item's state: three mantissas (or, in double-single, I, p, q) and the
+  // exponents, 16 bits each
+  i64 *s0m = (i64 *)(sm + L.I), *s1m = (i64 *)(sm + L.P), *s2m = (i64 *)(sm + L.Q);
+  short4 *sE = (short4 *)(sm + L.E);
   const int *fail = (const int *)(sm + L.fail);
-  unsigned *needBits = (unsigned *)(sm + L.bits);
-  int *pend = (int *)(sm + L.pend), *pref = (int *)(sm + L.pref);
+  unsigned char *act = (unsigned char *)(sm + L.act);  // the running items
+  int *pend = (int *)(sm + L.pend);
   const double za = pzA[k / Nb], ca = U.pcA[k / Nb], zb = pzB[k % Nb], cb = U.pcB[k % Nb];
   // derivative blocks: the product times zeta_a^max(0, shifta), then
   // zeta_b^max(0, shiftb) (src/type2.c:456-462)
@@ -1033,11 +1103,13 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
   const double i1 = map[k].x;
   const ff i1f = ff_from_double(i1), Ckf = ff_from_double(Ck);
   const int4 wk = win[k];
-  const int nb = wk.x, end = nb == INT_MAX ? OL - 1 : nb - 1, nLo = wk.y, nHi = wk.z;
+  const int nb = wk.x, nLo = wk.y, nHi = wk.z;
 #pragma unroll 1
-  for (int q = lane; q < nf; q += 32) { sI[q] = 0; sP[q] = 0; sQ[q] = 0; }
-#pragma unroll 1
-  for (int w = lane; w < (OL + 31) / 32; w += 32) needBits[w] = 0u;
+  for (int q = lane; q < nf; q += 32) {
+    act[q] = (unsigned char)q;
+    s0m[q] = s1m[q] = s2m[q] = 0;  // (also 0.0)
+    sE[q] = make_short4(kNoExp, kNoExp, kNoExp, 0);
+  }
   __syncwarp();
   // Whose tables slot t reads (the reference's reused buffers): this pair's
   // below its break; beyond it, on the lower half, the last earlier pair
@@ -1064,12 +1136,11 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
   // the needed ones queued, and each pass evaluates 32 queued slots, one per
   // lane, before the quadratures walk every slot up to the first one still
   // queued.
-  unsigned doneBits[kWalkCap / 32] = {0u, 0u, 0u, 0u};
-  int cpos = 0, wpos = 0, nPend = 0;
+  int cpos = 0, wpos = 0, nPend = 0, nAct = nf;
   // channels and rows the quadratures still running read (the pass's to
   // begin with, narrowed after every walk)
-  unsigned pMask = S.mask;
-  int pL1 = S.l1, pL2 = S.l2, pL3 = S.l3;
+  unsigned pMask = S0.mask;
+  int pL1 = S0.l1, pL2 = S0.l2, pL3 = S0.l3;
   const unsigned below = (1u << lane) - 1u;
   while (wpos < OL) {
     while (nPend < 32 && cpos < OL) {
@@ -1088,22 +1159,13 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
         }
       }
       const unsigned m = __ballot_sync(0xffffffffu, need);
-      if (need) {
-        pend[nPend + __popc(m & below)] = t;
-        atomicOr(&needBits[t >> 5], 1u << (t & 31));
-      }
+      if (need) pend[nPend + __popc(m & below)] = t;
       nPend += __popc(m);
       cpos = c1;
     }
     __syncwarp();
-    // this pass: the first queued slots, and the walk's end: an odd slot
-    // (whole (lower, upper) pairs) that no queued slot precedes
-    int nE = nPend < 32 ? nPend : 32, b = cpos;
-    if (nPend > 32) {
-      b = pend[32];
-      if (!(b & 1)) b -= 1;
-      while (nE > 0 && pend[nE - 1] >= b) nE--;
-    }
+    // this pass: the first queued slots, and the walk's end
+    const int nE = nPend < 32 ? nPend : 32, b = nPend > 32 ? pend[32] : cpos;
     if (lane < nE) {
       const int t = pend[lane], n = __ldg(J.s92 + t);
       int owner;
@@ -1154,55 +1216,93 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
         }
       }
     }
-    if (lane == 0) {  // entry of slot t: queued slots in [wpos, t)
-      const int w0 = wpos >> 5, w1 = (b - 1) >> 5;
-      int acc = -__popc(needBits[w0] & ((1u << (wpos & 31)) - 1u));
-#pragma unroll 1
-      for (int w = w0; w <= w1; w++) {
-        pref[w] = acc;
-        acc += __popc(needBits[w]);
-      }
-    }
+    const int myPend = lane < nE ? pend[lane] : INT_MAX;
     __syncwarp();
-    bool all = true;
     unsigned nMask = 0u;
-    int n1 = 0, n2 = 0, n3 = 0;
+    int n1 = 0, n2 = 0, n3 = 0, left = 0;
+    // the running items, 32 at a time, the last ones by several lanes each
 #pragma unroll 1
-    for (int q = lane, qi = 0; q < nf; q += 32, qi++) {
-      if (doneBits[qi] & (1u << lane)) continue;
+    for (int i0 = 0; i0 < nAct;) {
+      const LaneDeal D = deal_lanes(nAct - i0);
+      const bool work = i0 + D.rank < nAct;
+      const int q = work ? act[i0 + D.rank] : 0;
       // the pass's item, decoded once when the pass was listed
       const int v = fail[q], l = v & 255, l1 = (v >> 8) & 255, l2 = (v >> 16) & 255, l3 = v >> 24;
-      auto entry = [&](int t) {  // a queued slot's table entry
-        const unsigned word = needBits[t >> 5], bit = 1u << (t & 31);
-        return tab + (pref[t >> 5] + __popc(word & (bit - 1u))) * TS;
-      };
-      auto vis = [&](int t) { return c92_slot[t] <= end; };  // an upper slot
-      double I = sI[q], p = sP[q], qv = sQ[q], res = 0;
-      bool done = false;
+      bool done = !work;
+      double res = 0;
       if (inFF) {
-        auto val = [&](int t) {
-          const ff *Uc = (const ff *)entry(t), *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
+        double I = __longlong_as_double(s0m[q]), p = __longlong_as_double(s1m[q]), qv = __longlong_as_double(s2m[q]);
+        auto val = [&](int i) {
+          const ff *Uc = (const ff *)(tab + i * TS), *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
           return ff_mul(ff_mul(ff_mul(Ka[l1], Kb[l2]), Uc[l]), R[l3]);
         };
-        psm92_sparse_ff(wpos, b, needBits, J.tol, val, vis, I, p, qv, done, res);
+        psm92_queue_ff(wpos, b, pend, nE, J.tol, val, I, p, qv, done, res);
+        __syncwarp();
+        if (work && D.part == 0) {
+          s0m[q] = __double_as_longlong(done ? res : I);
+          s1m[q] = __double_as_longlong(p);
+          s2m[q] = __double_as_longlong(qv);
+        }
       } else {
-        auto add = [&](int t, xf_sum &a) {
-          const double *Uc = entry(t), *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
-          const xfs v = (xfs_from(Ka[l1]) * xfs_from(Kb[l2])) * (xfs_from(Uc[l]) * xfs_from(R[l3]));
-          a.add(v.v, v.s);
-        };
-        psm92_sparse(wpos, b, needBits, J.tol, add, vis, I, p, qv, done, res);
+        const short4 e = sE[q];
+        Psm92 S;
+        S.I = {s0m[q], e.x};
+        S.I1 = {s1m[q], e.y};
+        S.I2 = {s2m[q], e.z};
+        const double *eA = tab + LE + nA + l1, *eB = tab + LE + nA + LBE + l2, *eU = tab + l, *eR = tab + LE + l3;
+        int i = 0, pos = wpos, k = wpos == 0 ? -1 : level_of(wpos);
+#pragma unroll 1
+        while (pos < b) {
+          const int lvE = k < 0 ? 1 : c92_lvEnd[k];
+          pos = lvE < b ? lvE : b;
+          const int ie = __popc(__ballot_sync(0xffffffffu, myPend < pos));
+          xf_run run;
+#pragma unroll 1
+          for (int x = i + D.part; x < ie; x += D.P) {
+            const double a = eA[x * TS], bb = eB[x * TS], u = eU[x * TS], r = eR[x * TS];
+            run.add({mul_hi(mul_hi(ent_m(a), ent_m(bb)), mul_hi(ent_m(u), ent_m(r))),
+                     (int)((ent_h(a) >> 20) & 0x7ff) + (int)((ent_h(u) >> 20) & 0x7ff) + (int)(ent_h(bb) >> 20) +
+                         (int)(ent_h(r) >> 20) + 3 * 64 - 4 * kEntBias},
+                    ent_h(a) ^ ent_h(u));
+          }
+          i = ie;
+          S.I = xs_plus(S.I, combine(run.sum(), D.P));
+          if (pos == lvE) {
+            if (k < 0) psm92_head(S);
+            else if (!done && psm92_end(S, V, k)) {
+              done = true;
+              res = psm92_result(S, V, k);
+            }
+            k++;
+          }
+          if (__all_sync(0xffffffffu, done)) break;
+        }
+        __syncwarp();
+        if (work && D.part == 0) {
+          s0m[q] = done ? __double_as_longlong(res) : S.I.m;
+          s1m[q] = S.I1.m;
+          s2m[q] = S.I2.m;
+          sE[q] = make_short4(exp16(S.I.e), exp16(S.I1.e), exp16(S.I2.e), 0);
+        }
       }
-      sI[q] = I; sP[q] = p; sQ[q] = qv;
-      if (done) { sI[q] = res; doneBits[qi] |= 1u << lane; }
-      else {
-        all = false;
+      if (!done) {
         nMask |= 1u << l;
         n1 = l1 > n1 ? l1 : n1;
         n2 = l2 > n2 ? l2 : n2;
         n3 = l3 > n3 ? l3 : n3;
       }
+      // keep the items still running (the list shrinks in place); a finished
+      // one adds its result
+      const bool keep = work && D.part == 0 && !done;
+      const unsigned km = __ballot_sync(0xffffffffu, keep);
+      if (work && D.part == 0 && done) part[q] += res;
+      __syncwarp();
+      if (keep) act[left + __popc(km & below)] = (unsigned char)q;
+      left += __popc(km);
+      i0 += 32 / D.P;
+      __syncwarp();
     }
+    nAct = left;
     pMask = __reduce_or_sync(0xffffffffu, nMask);
     pL1 = __reduce_max_sync(0xffffffffu, n1);
     pL2 = __reduce_max_sync(0xffffffffu, n2);
@@ -1216,13 +1316,19 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
     nPend = rest;
     wpos = b;
     __syncwarp();
-    if (__all_sync(0xffffffffu, all)) break;
+    if (nAct == 0) break;
   }
-  const double N3 = c92_3N[c92_nLevels - 1];
+  // out of levels: the full-grid estimate stands and the unit is flagged
 #pragma unroll 1
-  for (int q = lane, qi = 0; q < nf; q += 32, qi++) {
-    if (doneBits[qi] & (1u << lane)) part[q] += sI[q];
-    else { part[q] += 16 * sI[q] / N3; warn = 1; }
+  for (int i = lane; i < nAct; i += 32) {
+    const int q = act[i];
+    if (inFF) part[q] += 16 * __longlong_as_double(s0m[q]) / c92_3N[c92_nLevels - 1];
+    else {
+      Psm92 S;
+      S.I1 = {s1m[q], sE[q].y};
+      part[q] += psm92_result(S, V, c92_nLevels - 1);
+    }
+    warn = 1;
   }
   __syncwarp();
 }
@@ -1230,7 +1336,8 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
 // The failed type-2 quadratures of a unit over the primitive pairs of one part
 // (src/type2.c:418-528), in passes of up to kWalkCap of them.
 template <bool kMixed>
-static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem &L, double *sm, int part) {
+static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem &L, double *sm, const LevelTab &V,
+                                int part) {
   const int lane = threadIdx.x & 31, nIt = U.nItems, LE = J.maxLECP > 0 ? J.maxLECP : 1;
   const unsigned *mask = (const unsigned *)(U.scr + U.L.mask);
   int *fail = (int *)(sm + L.fail);
@@ -1285,7 +1392,7 @@ static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem 
     int mb = mb0, warn = 0;
 #pragma unroll 1
     for (int k = k0; k < k1; k++) {
-      t2_pair<kMixed>(J, U, L, sm, S, k, mb, map, win, useFF, warn);
+      t2_pair<kMixed>(J, U, L, sm, V, S, k, mb, map, win, useFF, warn);
       mb = win[k].x > mb ? win[k].x : mb;
     }
     if (warn) atomicOr(&((UnitHead *)U.scr)->warn, 2);
@@ -1305,6 +1412,8 @@ static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem 
 template <bool kMixed>
 __global__ void __launch_bounds__(32, 16) k_unit_large(DevJob J) {
   extern __shared__ double sm[];
+  __shared__ LevelTab V;
+  level_tab(V, c92_3N, c92_nLevels, J.tol);
   const LargeSmem L = large_layout(J.maxLBS, J.maxLECP, false);
   const int n2 = (int)J.counters[kCntPart], n = n2 + (int)J.counters[kCntFail];
 #pragma unroll 1
@@ -1314,11 +1423,11 @@ __global__ void __launch_bounds__(32, 16) k_unit_large(DevJob J) {
     if (i < n2) {
       const int2 it = J.listPart[i];
       const Unit U = unit_load(J, it.x);
-      t2_large<kMixed>(J, U, L, sm, it.y);
+      t2_large<kMixed>(J, U, L, sm, V, it.y);
     } else {
       const T1Fail it = J.listFail[i - n2];
       const Unit U = unit_load(J, it.pos);
-      t1_large<kMixed>(J, U, sm + L.tab, it.k & 0xffff, it.k >> 16, it.mask, it.s);
+      t1_large<kMixed>(J, U, L, sm, V, it.k & 0xffff, it.k >> 16, it.mask, it.s);
     }
   }
 }

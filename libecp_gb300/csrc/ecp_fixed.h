@@ -193,20 +193,18 @@ ECPGB_HD xf xf_times100(xf f) { return {mul_hi(f.m, 100ull << 57), f.e + 7}; }
 // polynomial to 1e-14 of K_0 and needs no code; z = 0 gives exactly (1, 0, ...).
 ECPGB_HD void fx_bessel_rows(const i64 *besX, const i64 *besXA, int HL1, int lmax, xf z100, xf mul, uint32_t sign,
                              double *K) {
-  if (__builtin_expect(z100.m == 0, 0)) {  // rare: a shell on the ECP centre
-    K[0] = mul.m ? xf_to_double(mul.m, mul.e, sign) : 1.0;
-    for (int l = 1; l <= lmax; l++) K[l] = 0.0;
-    return;
-  }
   z100 = xf_norm(z100);
   const int sh = -(z100.e + 52);  // 100 z in Q52 = z100.m >> sh; sh < 0 only above 1600
   u64 W = sh < 0 ? ~0ull : shr64(z100.m, sh);
   const bool asy = W >= 1600ull << 52;
-  const i64 *q;
-  int rowStride, scaleAt;
+  const i64 *q = besX;
+  int rowStride = 8, scaleAt = 6;
   u64 X;
-  xf am = {0, 0};
+  // one multiplier for every row (1, exactly, where there is none): no copies
+  // of the row loop for its cases
+  xf c = mul.m ? mul : xf{1ull << 63, -63};
   if (asy) {
+    xf am;
     am.m = mul_hi(fx_recip(z100.m), 50ull << 58);  // a = 1/(2z) = 50 / z100
     am.e = -120 - z100.e;
     const int s = am.e + 68;  // 16 a in Q64
@@ -215,12 +213,11 @@ ECPGB_HD void fx_bessel_rows(const i64 *besX, const i64 *besXA, int HL1, int lma
     q = besXA;
     rowStride = 16;
     scaleAt = 15;
+    c = xf_norm(xf_mul(am, c));
   } else {
     W += 1ull << 51;
     X = (W & ((1ull << 52) - 1)) << 11;
-    q = besX + (size_t)(W >> 52) * HL1 * 8;
-    rowStride = 8;
-    scaleAt = 6;
+    q += (size_t)(W >> 52) * HL1 * 8;
   }
   const fxmul x = fx_split(X);
 ECPGB_NOUNROLL
@@ -235,9 +232,10 @@ ECPGB_NOUNROLL
     v = c23.x + mul_hi_s(v, x);
     v = c01.y + mul_hi_s(v, x);
     v = c01.x + mul_hi_s(v, x);
-    xf k = xf_norm({v > 0 ? (u64)v : 0ull, -(int)ld_one(q + scaleAt)});
-    if (asy) k = xf_mul(k, am);
-    if (mul.m) k = xf_mul(k, mul);
+    // (z = 0, a shell on the ECP centre: exactly 1, 0, 0, ...)
+    if (z100.m == 0) v = l == 0 ? 1ll << 62 : 0;
+    const int e = z100.m == 0 ? -62 : -(int)ld_one(q + scaleAt);
+    const xf k = xf_mul(xf_norm({v > 0 ? (u64)v : 0ull, e}), c);
     K[l] = xf_to_double(k.m, k.e, sign);
   }
 }
@@ -252,25 +250,64 @@ ECPGB_HD i64 fx_q53(double x) {
   return (i64)b < 0 ? -v : v;
 }
 
-// A signed sum of terms +-m 2^e: 60-bit mantissa, aligned to the larger
-// exponent, never renormalised upwards (cancelled bits stay cancelled).
-// Branch-free, so that lanes of different exponents stay together.
-struct xf_sum {
+// A signed number m * 2^e, |m| < 2^62: the running values of a quadrature.
+// Sums align to the larger exponent and are never renormalised upwards
+// (cancelled bits stay cancelled); an empty sum has the smallest exponent.
+struct xs {
   i64 m = 0;
   int e = -100000;
+};
+// Back below 2^62 after a sum.
+ECPGB_HD xs xs_fit(xs a) {
+  const int over = (int)((uint32_t)((u64)(a.m ^ (a.m << 1)) >> 63));
+  return {a.m >> over, a.e + over};
+}
+ECPGB_HD xs xs_add(xs a, xs b) {
+  const int d = a.e - b.e;
+  const int sa = d < 0 ? (d < -63 ? 63 : -d) : 0, sb = d > 0 ? (d > 63 ? 63 : d) : 0;
+  return xs_fit({(a.m >> sa) + (b.m >> sb), d < 0 ? b.e : a.e});
+}
+ECPGB_HD xs xs_neg(xs a) { return {-a.m, a.e}; }
+ECPGB_HD xs xs_shl(xs a, int k) { return {a.m, a.e + k}; }  // a 2^k
+ECPGB_HD xf xs_abs(xs a) { return xf_norm({a.m < 0 ? (u64)-a.m : (u64)a.m, a.e}); }
+ECPGB_HD double xs_to_double(xs a) {
+  return xf_to_double(a.m < 0 ? (u64)-a.m : (u64)a.m, a.e, a.m < 0 ? 0x80000000u : 0u);
+}
+// a * c rounded to double (c positive).
+ECPGB_HD double xs_times(xs a, xf c) {
+  const xf v = xf_mul(xs_abs(a), c);
+  return xf_to_double(v.m, v.e, a.m < 0 ? 0x80000000u : 0u);
+}
+// a <= b and a < b for normalised (or zero) a, b.
+ECPGB_HD bool xf_le(xf a, xf b) { return a.m == 0 || (b.m != 0 && (a.e < b.e || (a.e == b.e && a.m <= b.m))); }
+ECPGB_HD bool xf_lt(xf a, xf b) { return !xf_le(b, a); }
+
+// A run of terms +-m 2^e: 57-bit mantissas, room for 63 terms before xs_fit.
+struct xf_run {
+  i64 m = 0;
+  int e = -100000;
+  // sign: any word whose top bit is the term's sign
   ECPGB_HD void add(xf t, uint32_t sign) {
-    i64 tm = (i64)(t.m >> 4);
-    const int te = t.e + 4, d = e - te;
-    const int sa = d < 0 ? (d < -63 ? 63 : -d) : 0, st = d > 0 ? (d > 63 ? 63 : d) : 0;
-    if (sign) tm = -tm;
-    m = (m >> sa) + (tm >> st);
-    e = d < 0 ? te : e;
-    const int over = (int)((uint32_t)((u64)(m ^ (m << 1)) >> 63));  // room for the next term
-    m >>= over;
-    e += over;
+    const i64 s = (i64)(int)sign >> 31;
+    const i64 tm = ((i64)(t.m >> 7) ^ s) - s;
+    const int te = t.e + 7, d = e - te;
+    if (d < 0) {  // a larger term: the sum moves
+      m >>= (d < -63 ? 63 : -d);
+      e = te;
+      m += tm;
+    } else {
+      m += tm >> (d > 63 ? 63 : d);
+    }
   }
-  ECPGB_HD double value() const {
-    return xf_to_double(m < 0 ? (u64)-m : (u64)m, e, m < 0 ? 0x80000000u : 0u);
+  ECPGB_HD xs sum() const { return xs_fit({m, e}); }
+};
+
+// A signed sum of any number of terms (the ECP channels).
+struct xf_sum {
+  xs v;
+  ECPGB_HD void add(xf t, uint32_t sign) {
+    const i64 tm = (i64)(t.m >> 4);
+    v = xs_add(v, {sign ? -tm : tm, t.e + 4});
   }
 };
 

@@ -175,7 +175,7 @@ struct PairFx {
 // Shared memory of the stages, in doubles.  Small grid (one warp a CTA): the
 // group's pair scalars and step table.
 struct SmallSmem {
-  int sc, fx, tab, total;
+  int sc, fx, quad, tab, total;
 };
 __host__ __device__ inline SmallSmem small_layout(int LB, int cap) {
   SmallSmem s;
@@ -186,7 +186,8 @@ __host__ __device__ inline SmallSmem small_layout(int LB, int cap) {
   }
   s.sc = 0;
   s.fx = 24;  // 3 scalars of up to 8 pairs
-  s.tab = s.fx + 8 * (int)(sizeof(PairFx) / sizeof(double));
+  s.quad = s.fx + 8 * (int)(sizeof(PairFx) / sizeof(double));  // 32 ints
+  s.tab = s.quad + 16;
   s.total = s.tab + tt;
   return s;
 }
@@ -195,10 +196,10 @@ __host__ __device__ inline SmallSmem small_layout(int LB, int cap) {
 // the weight), the walkers' state, the needed-slot bitmap
 // with word prefixes, the pending slots and the failed items.
 struct LargeSmem {
-  int tab, I, P, Q, part, bits, pend, pref, fail, total, tabStride;
+  int tab, I, P, Q, E, part, act, bits, pend, pref, fail, total, tabStride;
 };
 __host__ __device__ inline LargeSmem large_layout(int LB, int LE, bool exact) {
-  LargeSmem s;
+  LargeSmem s{};
   const int nA = 2 * LB + 1, nE = LE > 0 ? LE : 1, LBE = LB + nE;
   s.tabStride = (nE + nA + 2 * LBE + (exact ? 2 : 0)) | 1;  // odd: conflict-free lane strides
   int o = 32 * s.tabStride, t1 = 32 * (2 * nA + 3);
@@ -208,9 +209,14 @@ __host__ __device__ inline LargeSmem large_layout(int LB, int LE, bool exact) {
   s.P = o; o += kWalkCap;
   s.Q = o; o += kWalkCap;
   s.part = o; o += kWalkCap;
-  s.bits = o; o += kLargeWords / 2;
   s.pend = o; o += 32;
-  s.pref = o; o += kLargeWords / 2;
+  if (exact) {  // needed-slot bitmap and word prefixes
+    s.bits = o; o += kLargeWords / 2;
+    s.pref = o; o += kLargeWords / 2;
+  } else {  // exponents and list of the running items
+    s.E = o; o += kWalkCap;
+    s.act = o; o += kWalkCap / 8;
+  }
   s.fail = o; o += kWalkCap / 2;
   s.total = o;
   return s;
