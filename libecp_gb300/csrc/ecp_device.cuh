@@ -205,6 +205,12 @@ static __device__ inline double rpow(double r, double n) {
 // U_l(r) of centre c (src/ecp.c:42-60).
 static __device__ double eval_ecp(const DevJob &J, int c, int l, double r) {
   double pot = 0.0, r2 = r * r;
+  if (J.chanT0) {  // the channel's terms, in order
+    const int *ch = J.chanT0 + c * (kMaxLEcp + 2) + l;
+#pragma unroll 1
+    for (int t = ch[0], t1 = ch[1]; t < t1; t++) pot += rpow(r, J.termN[t]) * J.termD[t] * exp(-J.termA[t] * r2);
+    return pot;
+  }
   int t0 = J.ctrT0[c], t1 = t0 + J.ctrNT[c];
   for (int t = t0; t < t1; t++)
     if (J.termL[t] == l) pot += rpow(r, J.termN[t]) * J.termD[t] * exp(-J.termA[t] * r2);

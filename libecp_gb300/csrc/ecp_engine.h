@@ -63,6 +63,8 @@ struct DevJob {
   const double *primA, *primD;
   const int *ctrAtom, *ctrL, *ctrT0, *ctrNT;
   const int *termL;
+  const int *chanT0;           // per centre, the first term of channels l = 0..kMaxLEcp, then the end
+                               // (terms sorted by l; null: none)
   const double *termN, *termD, *termA;
   const int *pairA, *pairB;
   const int *pairShift;        // derivative shift index of each pair entry (null: none)

@@ -52,6 +52,40 @@ static __device__ __noinline__ void bessel_fx(const DevJob &J, int lmax, xf z100
   fx_bessel_rows(J.besX, J.besXA, J.besHL + 1, lmax, z100, mul, sign, K);
 }
 
+// The rows for the type-1 tables, K_l / c = K[l] 2^base with one base for the
+// even rows (K_0 normalised) and one for the odd rows (K_1 normalised): a
+// quadrature (l1, l2) and those it is added to read rows of one parity.
+struct RowBase {
+  xf c;
+  int even, odd;
+};
+static __device__ __noinline__ RowBase bessel_rows2(const DevJob &J, int lmax, xf z100, u64 *K) {
+  RowBase b;
+  int base[2] = {0, 0};
+  b.c = fx_bessel(J.besX, J.besXA, J.besHL + 1, lmax, z100, [&](int l, u64 v, int scale) {
+    if (l < 2) {
+      const int n = clz64(v | 1u);
+      K[l] = v << n;
+      if (l == 0) base[0] = base[1] = -scale - n;
+      else if (v) base[1] = -scale - n;
+    } else {
+      const int sh = (l & 1 ? base[1] : base[0]) + scale;  // K_l <= K_(l-2)
+      K[l] = sh < 0 ? v << -sh : shr64(v, sh);
+    }
+  });
+  b.even = base[0];
+  b.odd = base[1];
+  return b;
+}
+// The rows as normalised mantissas and exponents for the type-2 tables.
+static __device__ __noinline__ xf bessel_me(const DevJob &J, int lmax, xf z100, u64 *K, short *E) {
+  return fx_bessel(J.besX, J.besXA, J.besHL + 1, lmax, z100, [&](int l, u64 v, int scale) {
+    const xf k = xf_norm({v, -scale});
+    K[l] = k.m;
+    E[l] = (short)k.e;
+  });
+}
+
 // Powers of r other than 0, 1, 2: rare, out of line.
 static __device__ __noinline__ double rpow_rare(double r, double n) { return rpow(r, n); }
 
@@ -107,40 +141,14 @@ static __device__ __noinline__ double bessel_row(const DevJob &J, int l, double 
   return fma(v, dz, q[0]);
 }
 
-// U_l(r) of centre c for the channels l set in mask, in one pass over its
-// terms (src/ecp.c:42-60); the other entries of U are left untouched.  A
-// channel's terms are summed with 60-bit mantissas; a channel that comes back
-// after another one is added to in FP64.
-static __device__ __noinline__ void channels_masked(const DevJob &J, int c, double r, unsigned mask, double *U) {
-  for (unsigned m = mask; m; m &= m - 1) U[__ffs(m) - 1] = 0.0;
-  const xf R = xf_from(r), R2 = norm1(xf_mul(R, R));
-  const int t0 = J.ctrT0[c], t1 = t0 + J.ctrNT[c];
-  unsigned seen = 0;
-#pragma unroll 1
-  for (int t = t0; t < t1;) {
-    const int l = J.termL[t];
-    xf_sum acc;
-    const bool use = mask >> l & 1u;
-#pragma unroll 1
-    for (; t < t1 && J.termL[t] == l; t++)
-      if (use) ecp_term_fx(J, t, r, R, R2, acc);
-    if (use) {
-      const double v = xs_to_double(acc.v);
-      if (seen >> l & 1u) U[l] += v;
-      else U[l] = v;
-      seen |= 1u << l;
-    }
-  }
-}
-
-// U_l(r) as a mantissa, exponent and sign.
+// U_l(r) of centre c (src/ecp.c:42-60): its terms of channel l, summed with
+// 60-bit mantissas; normalised, with its sign.
 static __device__ __noinline__ xf channel(const DevJob &J, int c, int l, double r, uint32_t &sign) {
   const xf R = xf_from(r), R2 = norm1(xf_mul(R, R));
   xf_sum acc;
-  const int t0 = J.ctrT0[c], t1 = t0 + J.ctrNT[c];
+  const int *ch = J.chanT0 + c * (kMaxLEcp + 2) + l, t1 = ch[1];
 #pragma unroll 1
-  for (int t = t0; t < t1; t++)
-    if (J.termL[t] == l) ecp_term_fx(J, t, r, R, R2, acc);
+  for (int t = ch[0]; t < t1; t++) ecp_term_fx(J, t, r, R, R2, acc);
   sign = acc.v.m < 0 ? 0x80000000u : 0u;
   return xs_abs(acc.v);
 }
@@ -260,11 +268,7 @@ static __device__ inline void level_tab(LevelTab &T, const double *n3, int level
   __syncwarp();
 }
 
-// Table entries are doubles that are never subnormal; a zero counts as
-// 2^-1023.  Mantissa, biased exponent (of a positive entry) and high word.
-static __device__ inline u64 ent_m(double x) { return ((u64)dbits(x) << 11) | (1ull << 63); }
 static __device__ inline uint32_t ent_h(double x) { return (uint32_t)((u64)dbits(x) >> 32); }
-constexpr int kEntBias = 1023 + 63;
 
 // xs_add and xs_times out of line: the level ends use them several times, and
 // one copy keeps the kernels' loops in the instruction cache.
@@ -503,25 +507,52 @@ static __device__ void rsh_column(const DevJob &J, int lmax, int m, double x, do
   }
 }
 
-// One live entry of the type-1 large-grid tables: K[0..kq] = K_l(s r) and
-// WR[0..rq] = w C2 U_L(r) e^ex r^l; returns whether the entry is not zero.
-static __device__ __noinline__ bool t1_large_entry(const DevJob &J, int c, int Lc, double r, double ex, double w,
-                                                   double C2, double s, int kq, int rq, double *K, double *WR) {
+// Type-1 table entries, 2 lq + 1 words: K_l (bessel_rows2), then normalised
+// mantissas of v r^l, then the exponents: of row l times K_l2's parity,
+// e + l er - (leading bits won back up to row l) - (l odd: odd).
+struct EntInfo {
+  int e;       // 2 e + sign
+  int packed;  // er (8 bits, signed), odd (8 bits), a bit per row whose product was shifted
+};
+constexpr EntInfo kNoEntry = {-2000000, 0};
+// A point past the break: the entry holds doubles.
+constexpr int kStaleEntry = INT_MIN;
+static __device__ inline EntInfo t1_entry_rows(u64 *WR, xf v, const RowBase &b, xf R, uint32_t sign, int lmax) {
+  v = xf_norm(xf_mul(v, b.c));
+  u64 m = v.m;
+  WR[0] = m;
+  unsigned won = 0;
+#pragma unroll 1
+  for (int l = 1; l <= lmax; l++) {
+    m = mul_hi(m, R.m);
+    if ((i64)m >= 0) {
+      m += m;
+      won |= 1u << l;
+    }
+    WR[l] = m;
+  }
+  const int odd = b.even - b.odd;
+  return {(v.e + b.even + 64) * 2 + (int)(sign >> 31), ((R.e + 64) & 255) | (odd > 255 ? 255 : odd) << 8 | (int)(won << 16)};
+}
+// The product of row l1 and K_l2 of an entry into a run.
+static __device__ inline void t1_entry_add(xf_run &run, u64 wr, u64 k, EntInfo f, int l1) {
+  const int er = (int)(signed char)f.packed, odd = l1 & 1 ? (f.packed >> 8) & 255 : 0;
+  run.add({mul_hi(wr, k), (f.e >> 1) + l1 * er - odd - __popc((unsigned)f.packed >> 16 & ((2u << l1) - 1u))},
+          (uint32_t)f.e << 31);
+}
+
+// One live entry of the type-1 large-grid tables: K_l(s r) and w C2 U_L(r) e^ex
+// r^l; kNoEntry where it is zero.
+static __device__ __noinline__ EntInfo t1_large_entry(const DevJob &J, int c, int Lc, double r, double ex, double w,
+                                                      double C2, double s, int kq, int rq, u64 *K, u64 *WR) {
   const xf R = xf_from(r);
   uint32_t sign;
   xf v = channel(J, c, Lc, r, sign);
-  v = xf_mul(xf_mul(fx_exp(fx_q53(ex)), v),
-             xf_mul(xf_from(C2), xf_from(w)));
-  if (v.m == 0) return false;
+  v = xf_mul(xf_mul(fx_exp(fx_q53(ex)), v), xf_mul(xf_from(C2), xf_from(w)));
+  if (v.m == 0) return kNoEntry;
   sign ^= sign_of(C2) ^ sign_of(w);
-  bessel_fx(J, kq, xf_mul(xf_times100(xf_from(s)), R), {0, 0}, 0, K);
-  WR[0] = xf_to_double(v.m, v.e, sign);
-#pragma unroll 1
-  for (int l = 1; l <= rq; l++) {
-    v = norm1(xf_mul(v, R));
-    WR[l] = xf_to_double(v.m, v.e, sign);
-  }
-  return true;
+  const RowBase b = bessel_rows2(J, kq, xf_mul(xf_times100(xf_from(s)), R), K);
+  return t1_entry_rows(WR, v, b, R, sign, rq);
 }
 
 // --------------------------------------------------- stage 2: the small grid
@@ -554,7 +585,7 @@ static __device__ __noinline__ void t1_pair_setup(const DevJob &J, const Unit &U
 template <bool kMixed, int kKind>
 static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem &L, double *sm, const LevelTab &V,
                                 int pos, int p0, int G) {
-  const int lane = threadIdx.x & 31, lab = U.lab, lq = lab + 1, O = kSmallOrder, Nb = U.Nb, ws = U.ws, we = U.we;
+  const int lane = threadIdx.x & 31, lab = U.lab, lq = lab + 1, O = kSmallOrder, ws = U.ws, we = U.we;
   // odd entry strides: lanes touching neighbouring entries hit distinct banks
   const int TS = 1 + 2 * lq, nq = t1_items(lab);
   const u64 thr = (u64)(i64)(-J.lnAcc1 * 0x1p53);
@@ -651,28 +682,14 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
         u64 E = mul_hi(tt < 0 ? (u64)-tt : (u64)tt, R.m);
         const int sh = 117 - F.q + R.e;
         E = sh <= 0 ? shr64(E, -sh) : (E >> (63 - (sh > 63 ? 63 : sh)) ? ~0ull >> 1 : E << sh);
-        if (tt < 0 && E > thr) {  // below the screen
-#pragma unroll 1
-          for (int l = 0; l < 2 * lq; l++) ent[l] = 0.0;
-        } else {
-          xf v = xf_mul(xf_mul(fx_exp(tt < 0 ? -(i64)E : (i64)E), xf_from(C1)), xf_mul(xf_from(w), xf_from(u)));
-          const uint32_t sign = sign_of(w) ^ sign_of(u) ^ sign_of(C1);
-          bessel_fx(J, lab, xf_mul({F.sm, F.se}, R), {0, 0}, 0, ent);
-          WR[0] = xf_to_double(v.m, v.e, sign);
-#pragma unroll 1
-          for (int l = 1; l <= lab; l++) {
-            v = norm1(xf_mul(v, R));
-            WR[l] = xf_to_double(v.m, v.e, sign);
-          }
+        EntInfo info = kNoEntry;  // below the screen
+        if (tt >= 0 || E <= thr) {
+          const xf v = xf_mul(xf_mul(fx_exp(tt < 0 ? -(i64)E : (i64)E), xf_from(C1)), xf_mul(xf_from(w), xf_from(u)));
+          const RowBase b = bessel_rows2(J, lab, xf_mul({F.sm, F.se}, R), (u64 *)ent);
+          info = t1_entry_rows((u64 *)WR, v, b, R, sign_of(w) ^ sign_of(u) ^ sign_of(C1), lab);
         }
+        *(EntInfo *)(ent + 2 * lq) = info;
       }
-    }
-#pragma unroll 1
-    for (int e = lane; e < (ns - nIn) * nLive; e += 32) {
-      const int i = slot_of(e), t = __ldg(J.byN93 + s0 + (i < lo ? i : i + nIn));
-      double *ent = tab + ((t - s0) * G + live_pair(e, i)) * TS;
-#pragma unroll 1
-      for (int l = 0; l <= 2 * lq; l++) ent[l] = 0.0;
     }
     __syncwarp();
     if constexpr (kKind == kPairBand) {
@@ -726,7 +743,9 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
       __syncwarp();
       const bool work = D.rank < __popc(act);
       const int qd = work ? quad[D.rank] : 0;
-      const double *eW = tab + (qd & 255) * TS + lq + ((qd >> 8) & 255), *eK = tab + (qd & 255) * TS + (qd >> 16);
+      const int q1 = (qd >> 8) & 255;
+      const u64 *eT = (const u64 *)tab + (qd & 255) * TS;
+      const int oW = lq + q1, oK = qd >> 16;
 #pragma unroll 1
       for (int t = s0; t < s1;) {
         const int te = lvEnd < s1 ? lvEnd : s1;
@@ -742,10 +761,8 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
           const int n = __ldg(J.s93 + x);
           // the points inside the window (the entries outside it are zero)
           if (work && n >= ws && n < we) {
-            const size_t o = (size_t)(x - s0) * G * TS;
-            const double a = eW[o], b = eK[o];
-            run.add({mul_hi(ent_m(a), ent_m(b)), (int)((ent_h(a) >> 20) & 0x7ff) + (int)(ent_h(b) >> 20) + 64 - 2 * kEntBias},
-                    ent_h(a));
+            const u64 *e = eT + (x - s0) * G * TS;
+            t1_entry_add(run, e[oW], e[oK], *(const EntInfo *)(e + 2 * lq), q1);
           }
         }
         xs sum = combine(run.sum(), D.P);
@@ -950,7 +967,7 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, const LargeSmem 
       const int t = s0 + lane;
       int n = __ldg(J.s92 + t);
       bool upper = t > 0 && ((t - 1) & 1);
-      // entry: K_l rows, then the rows w * C2 U_L e^(..) r^l
+      // (mixed path's double-single entries: K_l rows, then w * C2 U_L e^(..) r^l)
       double *K = tab + (t - s0) * TSf, *WR = K + lq;
       const double w = J.wLarge[n] * i1;
       if (n < nb && !(upper && n > end)) {
@@ -970,7 +987,9 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, const LargeSmem 
               WRf[l] = v;
             }
           } else {
-            any = t1_large_entry(J, c, Lc, r, ex, w, C2, s, kq, rq, K, WR);
+            const EntInfo info = t1_large_entry(J, c, Lc, r, ex, w, C2, s, kq, rq, (u64 *)K, (u64 *)WR);
+            *(EntInfo *)(K + 2 * lq) = info;
+            any = info.e != kNoEntry.e;
           }
         }
       } else if (__builtin_expect(n != nb && !upper && n < O && n >= ws && n < we, 0)) {
@@ -988,15 +1007,16 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, const LargeSmem 
             double xr = J.xSmall[nr], pw = 1.0;
 #pragma unroll 1
             for (int i = 0; i < lr && ok; i++) pw = xr * pw;
-            WR[l] = ok ? v * pw : 0.0;
-            K[l] = ok ? bessel_row(J, lr, s * xr) : 0.0;
-          }
-          if (kMixed && ffp)  // the rows as ff, in place (entry l holds row l either way)
-#pragma unroll 1
-            for (int l = 0; l <= lab; l++) {
-              ((ff *)WR)[l] = ff_from_double(WR[l]);
-              ((ff *)K)[l] = ff_from_double(K[l]);
+            const double wr = ok ? v * pw : 0.0, kr = ok ? bessel_row(J, lr, s * xr) : 0.0;
+            if (kMixed && ffp) {
+              ((ff *)WR)[l] = ff_from_double(wr);
+              ((ff *)K)[l] = ff_from_double(kr);
+            } else {
+              WR[l] = wr;
+              K[l] = kr;
             }
+          }
+          if (!(kMixed && ffp)) *(EntInfo *)(K + 2 * lq) = {kStaleEntry, 0};
         }
       }
       if (kMixed && ffp && !any) {  // zero bits read as 0.0 in ff
@@ -1027,7 +1047,7 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, const LargeSmem 
       __syncwarp();
       const bool work = D.rank < __popc(act);
       const int qd = work ? quad[D.rank] : 0;
-      const double *eW = tab + lq + (qd & 0xffff), *eK = tab + (qd >> 16);
+      const int q1 = qd & 0xffff, oW = lq + q1, oK = qd >> 16;
 #pragma unroll 1
       for (int t = s0; t < s1;) {
         const int te = lvEnd < s1 ? lvEnd : s1;
@@ -1035,9 +1055,14 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, const LargeSmem 
 #pragma unroll 1
         for (int x = t + D.part; x < te; x += D.P)
           if (work && (live >> (x - s0) & 1u)) {
-            const double a = eW[(x - s0) * TSf], b = eK[(x - s0) * TSf];
-            run.add({mul_hi(ent_m(a), ent_m(b)), (int)((ent_h(a) >> 20) & 0x7ff) + (int)(ent_h(b) >> 20) + 64 - 2 * kEntBias},
-                    ent_h(a));
+            const u64 *e = (const u64 *)tab + (x - s0) * TSf;
+            const EntInfo f = *(const EntInfo *)(e + 2 * lq);
+            if (__builtin_expect(f.e == kStaleEntry, 0)) {
+              const double a = ((const double *)e)[oW], b = ((const double *)e)[oK];
+              run.add(xf_mul(xf_from(a), xf_from(b)), ent_h(a) ^ ent_h(b));
+            } else {
+              t1_entry_add(run, e[oW], e[oK], f, q1);
+            }
           }
         xs sum = combine(run.sum(), D.P);
         S.I = xs_plus(S.I, from_lane(sum, (mine_rank * D.P) & 31));
@@ -1085,7 +1110,7 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
   const bool inFF = kMixed && useFF;
   const int lane = threadIdx.x & 31, nA = 2 * J.maxLBS + 1, Nb = U.Nb, c = U.c, nf = S0.nf;
   const int LE = J.maxLECP > 0 ? J.maxLECP : 1, LBE = J.maxLBS + LE, OL = J.largeOrder;
-  const int TS = L.tabStride;
+  const int TS = L.tabStride, ES = L.expStride;
   const double *pzA = U.pzA, *pzB = U.pzB;
   const double dAC = U.gA[3], dBC = U.gB[3];
   double *tab = sm + L.tab, *part = sm + L.part;
@@ -1190,29 +1215,40 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
 #pragma unroll 1
         for (int l = 1; l <= pL3; l++) R[l] = ff_mul(rf, R[l - 1]);
       } else {
-        double *Uc = e, *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
-        // Ka rows carry the weight and prefactor: w * Ck * e^(..) * K_l1
+        // mantissas of w Ck e^ex U_l, r^l, K_l1 and K_l2, the
+        // exponents in 16 bits, U's with its sign
+        u64 *Um = (u64 *)e, *R = Um + LE, *Ka = R + nA, *Kb = Ka + LBE;
+        short *Ue = (short *)(tab + 32 * TS) + lane * ES, *Ae = Ue + LE, *Be = Ae + LBE, *Re = Be + LBE;
         const double w = J.wLarge[n];
-        const xf Rx = xf_from(r),
-                 wB = xf_mul(fx_exp(fx_q53(ex)), xf_mul(xf_mul(xf_from(w), xf_from(i1)), xf_from(Ck)));
-        // (a zero prefactor as a zero of the smallest exponent: mul.m = 0 means 1)
-        const xf mul = wB.m ? norm1(wB) : xf{1, -100000};
-        const uint32_t sign = sign_of(w) ^ sign_of(Ck);
-        // only the channels and rows this pass's quadratures read
-        channels_masked(J, c, r, pMask, Uc);
+        const xf Rx = xf_from(r);
+        xf wB = xf_mul(fx_exp(fx_q53(ex)), xf_mul(xf_mul(xf_from(w), xf_from(i1)), xf_from(Ck)));
         // the rows of both centres through one copy of the Bessel code
 #pragma unroll 1
         for (int side = 0; side < 2; side++) {
           const xf f = xf_mul(xf_from(side ? zbj : zaj), xf_from(side ? dBC : dAC));  // times 2: exponent + 1
-          bessel_fx(J, side ? pL2 : pL1, xf_mul(xf_times100({f.m, f.e + 1}), Rx), side ? xf{0, 0} : mul,
-                    side ? 0u : sign, side ? Kb : Ka);
+          const xf c = bessel_me(J, side ? pL2 : pL1, xf_mul(xf_times100({f.m, f.e + 1}), Rx), side ? Kb : Ka,
+                                 side ? Be : Ae);
+          wB = norm1(xf_mul(wB, c));
         }
-        R[0] = 1.0;
+        wB = xf_norm(wB);
+        // only the channels and rows this pass's quadratures read
+#pragma unroll 1
+        for (unsigned m = pMask; m; m &= m - 1u) {
+          const int l = __ffs(m) - 1;
+          uint32_t sign;
+          const xf u = norm1(xf_mul(channel(J, c, l, r, sign), wB));
+          sign ^= sign_of(w) ^ sign_of(Ck);
+          Um[l] = u.m;
+          Ue[l] = (short)((u.m && u.e > -16000 ? u.e * 2 : -32000) + (int)(sign >> 31));
+        }
         xf p = {1ull << 63, -63};
+        R[0] = p.m;
+        Re[0] = (short)p.e;
 #pragma unroll 1
         for (int l = 1; l <= pL3; l++) {
           p = norm1(xf_mul(p, Rx));
-          R[l] = xf_to_double(p.m, p.e, 0);
+          R[l] = p.m;
+          Re[l] = (short)p.e;
         }
       }
     }
@@ -1249,7 +1285,10 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
         S.I = {s0m[q], e.x};
         S.I1 = {s1m[q], e.y};
         S.I2 = {s2m[q], e.z};
-        const double *eA = tab + LE + nA + l1, *eB = tab + LE + nA + LBE + l2, *eU = tab + l, *eR = tab + LE + l3;
+        const u64 *eU = (const u64 *)tab + l, *eR = (const u64 *)tab + LE + l3, *eA = (const u64 *)tab + LE + nA + l1,
+                  *eB = (const u64 *)tab + LE + nA + LBE + l2;
+        const short *xT = (const short *)(tab + 32 * TS);
+        const int xA = LE + l1, xB = LE + LBE + l2, xR = LE + 2 * LBE + l3;
         int i = 0, pos = wpos, k = wpos == 0 ? -1 : level_of(wpos);
 #pragma unroll 1
         while (pos < b) {
@@ -1259,11 +1298,11 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
           xf_run run;
 #pragma unroll 1
           for (int x = i + D.part; x < ie; x += D.P) {
-            const double a = eA[x * TS], bb = eB[x * TS], u = eU[x * TS], r = eR[x * TS];
-            run.add({mul_hi(mul_hi(ent_m(a), ent_m(bb)), mul_hi(ent_m(u), ent_m(r))),
-                     (int)((ent_h(a) >> 20) & 0x7ff) + (int)((ent_h(u) >> 20) & 0x7ff) + (int)(ent_h(bb) >> 20) +
-                         (int)(ent_h(r) >> 20) + 3 * 64 - 4 * kEntBias},
-                    ent_h(a) ^ ent_h(u));
+            const short *xe = xT + x * ES;
+            const int ue = xe[l];
+            run.add({mul_hi(mul_hi(eA[x * TS], eB[x * TS]), mul_hi(eU[x * TS], eR[x * TS])),
+                     (ue >> 1) + xe[xA] + xe[xB] + xe[xR] + 3 * 64},
+                    (uint32_t)ue << 31);
           }
           i = ie;
           S.I = xs_plus(S.I, combine(run.sum(), D.P));

@@ -183,16 +183,17 @@ ECPGB_HD i64 ld_one(const i64 *p) {
 // 100 z for z = f * r, f already times 100 (xf_times100): the argument of fx_bessel_rows.
 ECPGB_HD xf xf_times100(xf f) { return {mul_hi(f.m, 100ull << 57), f.e + 7}; }
 
-// K_0..K_lmax(z), each times mul (mul.m = 0: times 1) with the sign bit
-// `sign`, rounded to double.  z100 = 100 z (the reference's table step is 1/100).
-// The branches of src/bessel.c:102-199 in fixed point: the 5-term Taylor
-// polynomial about the nearest table point (z < 16) and the large-argument
-// polynomial are both one Horner pass per row over 64-bit coefficients
-// (besX, besXA), so lanes on either branch run the same instructions.  The
-// small-argument branch (z < 1e-7) agrees with the first table point's
-// polynomial to 1e-14 of K_0 and needs no code; z = 0 gives exactly (1, 0, ...).
-ECPGB_HD void fx_bessel_rows(const i64 *besX, const i64 *besXA, int HL1, int lmax, xf z100, xf mul, uint32_t sign,
-                             double *K) {
+// K_0..K_lmax(z) in fixed point: row(l, v, scale) gets K_l / c = v 2^-scale,
+// 0 <= v < 2^62, and the call returns c (1, or 1/(2z) for large z).  z100 =
+// 100 z (the reference's table step is 1/100).  The branches of
+// src/bessel.c:102-199: the 5-term Taylor polynomial about the nearest table
+// point (z < 16) and the large-argument polynomial are both one Horner pass
+// per row over 64-bit coefficients (besX, besXA), so lanes on either branch
+// run the same instructions.  The small-argument branch (z < 1e-7) agrees with
+// the first table point's polynomial to 1e-14 of K_0 and needs no code; z = 0
+// gives exactly (1, 0, ...).
+template <class Row>
+ECPGB_HD xf fx_bessel(const i64 *besX, const i64 *besXA, int HL1, int lmax, xf z100, Row row) {
   z100 = xf_norm(z100);
   const int sh = -(z100.e + 52);  // 100 z in Q52 = z100.m >> sh; sh < 0 only above 1600
   u64 W = sh < 0 ? ~0ull : shr64(z100.m, sh);
@@ -200,20 +201,16 @@ ECPGB_HD void fx_bessel_rows(const i64 *besX, const i64 *besXA, int HL1, int lma
   const i64 *q = besX;
   int rowStride = 8, scaleAt = 6;
   u64 X;
-  // one multiplier for every row (1, exactly, where there is none): no copies
-  // of the row loop for its cases
-  xf c = mul.m ? mul : xf{1ull << 63, -63};
+  xf c = {1ull << 63, -63};
   if (asy) {
-    xf am;
-    am.m = mul_hi(fx_recip(z100.m), 50ull << 58);  // a = 1/(2z) = 50 / z100
-    am.e = -120 - z100.e;
-    const int s = am.e + 68;  // 16 a in Q64
-    X = s > 0 ? am.m << 1 : shr64(am.m, -s);
+    c.m = mul_hi(fx_recip(z100.m), 50ull << 58);  // 1/(2z) = 50 / z100
+    c.e = -120 - z100.e;
+    const int s = c.e + 68;  // 16 / (2z) in Q64
+    X = s > 0 ? c.m << 1 : shr64(c.m, -s);
     X = X < (1ull << 63) - 1 ? X : (1ull << 63) - 1;
     q = besXA;
     rowStride = 16;
     scaleAt = 15;
-    c = xf_norm(xf_mul(am, c));
   } else {
     W += 1ull << 51;
     X = (W & ((1ull << 52) - 1)) << 11;
@@ -233,10 +230,24 @@ ECPGB_NOUNROLL
     v = c01.y + mul_hi_s(v, x);
     v = c01.x + mul_hi_s(v, x);
     // (z = 0, a shell on the ECP centre: exactly 1, 0, 0, ...)
-    if (z100.m == 0) v = l == 0 ? 1ll << 62 : 0;
-    const int e = z100.m == 0 ? -62 : -(int)ld_one(q + scaleAt);
-    const xf k = xf_mul(xf_norm({v > 0 ? (u64)v : 0ull, e}), c);
-    K[l] = xf_to_double(k.m, k.e, sign);
+    const bool zero = z100.m == 0;
+    if (zero) v = l == 0 ? (1ll << 62) - 1 : 0;
+    row(l, (u64)(v > 0 ? v : 0), zero ? 62 : (int)ld_one(q + scaleAt));
+  }
+  return c;
+}
+
+// The rows as doubles, each times mul (mul.m = 0: times 1) with the sign bit `sign`.
+ECPGB_HD void fx_bessel_rows(const i64 *besX, const i64 *besXA, int HL1, int lmax, xf z100, xf mul, uint32_t sign,
+                             double *K) {
+  xf k[16];
+  xf c = fx_bessel(besX, besXA, HL1, lmax, z100, [&](int l, u64 v, int scale) { k[l] = xf_norm({v, -scale}); });
+  if (mul.m) c = xf_norm(xf_mul(c, mul));
+  const bool one = c.m == 1ull << 63;  // a power of two: exact
+ECPGB_NOUNROLL
+  for (int l = 0; l <= lmax; l++) {
+    const xf v = one ? xf{k[l].m, k[l].e + c.e + 63} : xf_mul(k[l], c);
+    K[l] = z100.m == 0 && l == 0 ? xf_to_double(c.m, c.e, sign) : xf_to_double(v.m, v.e, sign);
   }
 }
 

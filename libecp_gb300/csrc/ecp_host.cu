@@ -133,6 +133,24 @@ int parse_system(const ecpgb_system &s, Parsed &P) {
     P.ctrL.push_back(L);
     P.ctrT0.push_back(t0);
     P.ctrNT.push_back((int)P.termL.size() - t0);
+    // the centre's terms by channel, each channel's in the caller's order (a
+    // channel's sum takes them in that order)
+    const int n = (int)P.termL.size() - t0;
+    std::vector<int> at(n), L0 = std::vector<int>(P.termL.begin() + t0, P.termL.end());
+    for (int i = 0; i < n; i++) at[i] = i;
+    std::stable_sort(at.begin(), at.end(), [&](int x, int y) { return L0[x] < L0[y]; });
+    auto sorted = [&](std::vector<double> &v) {
+      const std::vector<double> u(v.begin() + t0, v.end());
+      for (int i = 0; i < n; i++) v[t0 + i] = u[at[i]];
+    };
+    sorted(P.termN);
+    sorted(P.termD);
+    sorted(P.termA);
+    for (int i = 0; i < n; i++) P.termL[t0 + i] = L0[at[i]];
+    for (int l = 0, t = t0; l <= kMaxLEcp + 1; l++) {
+      while (t < t0 + n && P.termL[t] < l) t++;
+      P.chanT0.push_back(t);
+    }
     P.maxLECP = std::max(P.maxLECP, L);
   }
   P.nCentres = (int)P.ctrAtom.size();
@@ -580,7 +598,7 @@ size_t job_device_bytes(const Parsed &P, int mode, size_t budget, size_t *scratc
   const size_t angLam = P.maxLECP + LB + 1, angC = (LB + 1) * (LB + 2) * (LB + 3) / 6;
   size_t in = 8 * (P.geom.size() + P.primA.size() + P.primD.size() + 3 * P.termL.size() + P.pairOff.size()) +
               4 * (5 * P.shL.size() + P.atomMaxL.size() + 4 * P.ctrAtom.size() + P.termL.size() + 3 * P.pairA.size()) +
-              36 * (P.nPairs + 1) + 4 * nc + (mode == ECPGB_MIXED ? 16 * P.termL.size() : 0) +
+              36 * (P.nPairs + 1) + 4 * nc + 4 * P.chanT0.size() + (mode == ECPGB_MIXED ? 16 * P.termL.size() : 0) +
               24 * 256;
   size_t work = 8 * (ns + nc * O * LE * nk + nc * O + nc * ns * (1 + P.deriv) * O * nF + nc * na * 4 + nc * na * D * D * D +
                      nc * na * angLam * LE * LE * angC + nc * (size_t)P.centreStride + (size_t)P.dim * P.dim) +
@@ -628,7 +646,7 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
          iCT = add(P.ctrT0.data(), 4 * P.ctrT0.size()), iCN = add(P.ctrNT.data(), 4 * P.ctrNT.size()),
          iTL = add(P.termL.data(), 4 * P.termL.size()), iPrA = add(P.pairA.data(), 4 * P.pairA.size()),
          iPrB = add(P.pairB.data(), 4 * P.pairB.size()), iPO = add(P.pairOff.data(), 8 * P.pairOff.size()),
-         iPS = add(P.pairShift.data(), 4 * P.pairShift.size());
+         iPS = add(P.pairShift.data(), 4 * P.pairShift.size()), iCh = add(P.chanT0.data(), 4 * P.chanT0.size());
   std::vector<int> orders, chunkPairs, ctr;
   std::vector<long long> offs;
   make_plan(P, scratchCap, mode == ECPGB_FP64 || few_pairs(P), B.plan, orders, offs, chunkPairs, ctr);
@@ -658,6 +676,7 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.ctrNT = (const int *)dp(iCN); J.termL = (const int *)dp(iTL); J.pairA = (const int *)dp(iPrA);
   J.pairB = (const int *)dp(iPrB); J.pairOff = (const long long *)dp(iPO);
   J.pairShift = (const int *)dp(iPS);
+  J.chanT0 = (const int *)dp(iCh);
   J.termAf = mode == ECPGB_MIXED ? (const ff *)dp(iTAf) : nullptr;
   J.termDf = mode == ECPGB_MIXED ? (const ff *)dp(iTDf) : nullptr;
   J.deriv = P.deriv;

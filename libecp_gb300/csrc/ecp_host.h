@@ -28,7 +28,7 @@ struct Parsed {
   double tol = 1e-12, acc = 1e-14;
   std::vector<double> geom, primA, primD, termN, termD, termA;
   std::vector<int> shL, shK, shP, shAtom, shAO, shLocal, atomMaxL, atomShell0;
-  std::vector<int> ctrAtom, ctrL, ctrT0, ctrNT, termL, pairA, pairB, pairShift;
+  std::vector<int> ctrAtom, ctrL, ctrT0, ctrNT, termL, chanT0, pairA, pairB, pairShift;
   std::vector<long long> pairOff;
   long long centreStride = 0;
 };

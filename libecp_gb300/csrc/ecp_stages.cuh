@@ -196,13 +196,15 @@ __host__ __device__ inline SmallSmem small_layout(int LB, int cap) {
 // the weight), the walkers' state, the needed-slot bitmap
 // with word prefixes, the pending slots and the failed items.
 struct LargeSmem {
-  int tab, I, P, Q, E, part, act, bits, pend, pref, fail, total, tabStride;
+  int tab, I, P, Q, E, part, act, bits, pend, pref, fail, total, tabStride, expStride;
 };
 __host__ __device__ inline LargeSmem large_layout(int LB, int LE, bool exact) {
   LargeSmem s{};
   const int nA = 2 * LB + 1, nE = LE > 0 ? LE : 1, LBE = LB + nE;
   s.tabStride = (nE + nA + 2 * LBE + (exact ? 2 : 0)) | 1;  // odd: conflict-free lane strides
-  int o = 32 * s.tabStride, t1 = 32 * (2 * nA + 3);
+  // 16-bit exponents of U, Ka, Kb and r^l (batched path): an odd number of words a lane
+  s.expStride = 2 * (((nE + 2 * LBE + nA + 1) / 2) | 1);
+  int o = 32 * s.tabStride + (exact ? 0 : 8 * s.expStride), t1 = 32 * (2 * nA + 3);
   s.tab = 0;
   if (t1 > o) o = t1;
   s.I = o; o += kWalkCap;
