@@ -56,6 +56,7 @@ struct DevJob {
   int angLam, angLM, angC;     // per (centre, atom) angular table dims
   int uspD;                    // unit-sphere polynomial table side (maxLBS + 1)
   int largeOrder;
+  int t2Rows;                  // most table rows a batch of type-2 quadratures reads
   double tol, acc, lnAcc1, lnAcc2;
   // inputs
   const double *geom;
@@ -275,7 +276,7 @@ int upload_schedules_fast(const int *s93slot, int s93n, const int *s93lvEnd, con
                           const int *s93lvN, int s93levels, const int *s92slot, int s92n,
                           const int *s92lvEnd, const int *s92lvN, int s92levels, void *stream);
 // Shared memory of the small-grid stage, and its CTAs (one warp) per SM.
-size_t fast_smem_bytes(int LB, int gcap);
+size_t fast_smem_bytes(int LB, int t2Rows, int gcap);
 int fast_ctas_per_sm(size_t smemBytes);
 // Sets the batched kernels' function attributes on the current device (call
 // before any graph capture).

@@ -194,7 +194,7 @@ static __device__ void x2_small(const DevJob &J, const Unit &U, int q0) {
 
 __global__ void __launch_bounds__(32, 16) k_exact_small(DevJob J) {
   extern __shared__ double sm[];
-  const SmallSmem L = small_layout(J.maxLBS, J.gcap);
+  const SmallSmem L = small_layout(J.maxLBS, 0, J.gcap);
   const int n1 = (int)J.counters[kCntT1], n = n1 + (int)J.counters[kCntT2];
 #pragma unroll 1
   for (int taken = 0; taken < J.take; taken++) {
@@ -614,12 +614,12 @@ __global__ void __launch_bounds__(32, 14) k_exact_large(DevJob J) {
 
 // Type-1 block (src/type1.c:266-295): per primitive pair in order, S_lm of its
 // k-vector and the terms of every combined Cartesian index.
-__global__ void __launch_bounds__(kLinkThreads) k_exact_link(DevJob J) {
+__global__ void __launch_bounds__(kLinkThreadsMax) k_exact_link(DevJob J) {
   extern __shared__ double sm[];
   const Unit U = unit_load(J, J.chunk0 + blockIdx.x);
   if (!U.live) return;
   const LinkSmem Lm = link_layout(J.maxLBS, J.maxLECP);
-  const int tid = threadIdx.x, NT = kLinkThreads, lab = U.lab, lq = lab + 1, Nb = U.Nb, RQ = lq * lq;
+  const int tid = threadIdx.x, NT = blockDim.x, lab = U.lab, lq = lab + 1, Nb = U.Nb, RQ = lq * lq;
   double *rsh = sm + Lm.rsh, *dir = sm + Lm.dir, *H = sm + Lm.H;
   const int dd = J.tmDim + 1, tmW = (J.tmDim + 1) * (J.tmDim + 1), nq = t1_items(lab), nH = NCUM(lab);
   const double *Q = (const double *)(U.scr + U.L.Q);
@@ -702,7 +702,7 @@ int launch_exact_pipeline(const DevJob &J, cudaStream_t st, cudaEvent_t u0, cuda
   Jc.balance = FastConfig{}.balance;
   Jc.live = nullptr;
   const JobPlan::Order &ord = use_order(Jc, FastConfig{}.sorted);
-  const size_t sSmall = sizeof(double) * (size_t)small_layout(J.maxLBS, Jc.gcap).total;
+  const size_t sSmall = sizeof(double) * (size_t)small_layout(J.maxLBS, 0, Jc.gcap).total;
   const size_t sLarge = sizeof(double) * (size_t)large_layout(J.maxLBS, J.maxLECP, true).total;
   const size_t sLink = sizeof(double) * (size_t)link_layout(J.maxLBS, J.maxLECP).total;
   if (sSmall > 200 * 1024 || sLarge > 200 * 1024 || sLink > 200 * 1024) return 3;
@@ -717,7 +717,7 @@ int launch_exact_pipeline(const DevJob &J, cudaStream_t st, cudaEvent_t u0, cuda
     k_exact_small<<<gSmall, 32, sSmall, st>>>(K);
     K.take = takeLarge;
     k_exact_large<<<gLarge, 32, sLarge, st>>>(K);
-    k_exact_link<<<units, kLinkThreads, sLink, st>>>(K);
+    k_exact_link<<<units, link_threads(sLink), sLink, st>>>(K);
   });
   if (u1) record_timing(u1, st);
   launch_epilogue(Jc, st);

@@ -93,21 +93,23 @@ static __device__ __noinline__ double rpow_rare(double r, double n) { return rpo
 // below 2^-70 of what the sum holds is left out (the sum carries 60 bits), and
 // one whose exponential underflows.
 static __device__ inline void ecp_term_fx(const DevJob &J, int t, double r, xf R, xf R2, xf_sum &acc) {
-  const xf a = xf_mul(xf_from(J.termA[t]), R2), D = xf_from(J.termD[t]);
-  const double n = J.termN[t];
+  const xf a = xf_mul(xf_from(__ldg(J.termA + t)), R2);
+  const double d = __ldg(J.termD + t);
+  const xf D = xf_from(d);
+  // n by its bits (a comparison of doubles is an FP64-pipe instruction)
+  const u64 nb = (u64)dbits(__ldg(J.termN + t));
+  const int n = nb == 0 ? 0 : nb == 0x3ff0000000000000ull ? 1 : nb == 0x4000000000000000ull ? 2 : 3;
   const int sh = a.e + 53;  // a r^2 in Q53
   const u64 E = sh < 0 ? shr64(a.m, -sh) : (a.m >> (63 - (sh > 63 ? 63 : sh)) ? ~0ull : a.m << sh);
   if (E > (u64)(700ll << 53)) return;
   // 2^b above the term, b = log2 |d| + log2 r^n - a r^2 log2 e rounded up
   // (n <= 2; r^n otherwise unknown: never left out)
-  const int rn = n == 0.0 ? 0 : n == 1.0 ? R.e + 64 : n == 2.0 ? R2.e + 64 : 100000;
+  const int rn = n == 0 ? 0 : n == 1 ? R.e + 64 : n == 2 ? R2.e + 64 : 100000;
   const int b = D.e + 64 + rn - (int)(((u64)(uint32_t)(E >> 32) * 1477) >> 31);
   if (b < acc.v.e + (63 - clz64((u64)(acc.v.m < 0 ? -acc.v.m : acc.v.m) | 1u)) - 70) return;
   xf v = xf_mul(fx_exp(-(i64)E), D);
-  if (n == 1.0) v = xf_mul(v, R);
-  else if (n == 2.0) v = xf_mul(v, R2);
-  else if (n != 0.0) v = xf_mul(v, xf_from(rpow_rare(r, n)));
-  acc.add(v, sign_of(J.termD[t]));
+  if (n) v = xf_mul(v, n == 1 ? R : n == 2 ? R2 : xf_from(rpow_rare(r, bits_d((i64)nb))));
+  acc.add(v, sign_of(d));
 }
 
 // One row K_l(z), by the same branches as bessel_fx.
@@ -428,7 +430,7 @@ PairPlan pair_plan(int NP, int la, int lb, int nItems, bool single) {
   return p;
 }
 
-size_t fast_smem_bytes(int LB, int gcap) { return sizeof(double) * (size_t)small_layout(LB, gcap).total; }
+size_t fast_smem_bytes(int LB, int t2Rows, int gcap) { return sizeof(double) * (size_t)small_layout(LB, t2Rows, gcap).total; }
 
 // Mixed path: the largest quadrature value for which double-single level
 // sums still decide the large-grid convergence test as FP64 does.  The
@@ -815,58 +817,121 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
   }
 }
 
-// A batch of 32 type-2 small-grid quadratures (src/type2.c:337-387), one per
-// lane: F tables (derivative runs max(0, shift), src/type2.c:563-564) and the
-// r^k U_l table read through L2, 64-bit mantissas in every mode.
+// A batch of up to 32 type-2 small-grid quadratures (src/type2.c:337-387), by
+// one warp.  32 slots at a time, a slot a lane, the rows that the batch reads of
+// both F tables (derivative runs max(0, shift), src/type2.c:563-564) and of the
+// weighted r^k U_l table are laid out as mantissas and 16-bit exponents (4 e +
+// sign: three signs fit the low bits of a sum), so a point costs a quadrature
+// two products and one sum.  The lanes are dealt to the running quadratures,
+// again whenever half of them have converged.
 template <bool kMixed>
-static __device__ void t2_small(const DevJob &J, const Unit &U, const LevelTab &V, int q0) {
-  const int q = q0 + (threadIdx.x & 31), O = kSmallOrder;
-  if (q >= U.nItems) return;
-  const int nF = J.nF, nk = J.nk, LE = J.maxLECP > 0 ? J.maxLECP : 1, nRuns = J.nRuns > 0 ? J.nRuns : 1;
-  const int v = unit_item(J, U, q), l = v & 255, l1 = (v >> 8) & 255, l2 = (v >> 16) & 255, l3 = v >> 24;
-  const double *Fa = J.F + (((size_t)U.c * J.nShells + U.sa) * nRuns + U.pa0) * O * nF + l1;
-  const double *Fb = J.F + (((size_t)U.c * J.nShells + U.sb) * nRuns + U.pb0) * O * nF + l2;
-  const double *Ut = J.utab + (size_t)U.c * O * LE * nk + l * nk + l3;
-  // slot 0 and slots 1, 2 are levels of their own (-2, -1)
+static __device__ void t2_small(const DevJob &J, const Unit &U, const LevelTab &V, u64 *tab, int *quad, int q0) {
+  const int lane = threadIdx.x & 31, O = kSmallOrder, nF = J.nF, nk = J.nk, LE = J.maxLECP > 0 ? J.maxLECP : 1,
+            nRuns = J.nRuns > 0 ? J.nRuns : 1, ws = U.ws, we = U.we;
+  int n = U.nItems - q0 < 32 ? U.nItems - q0 : 32;
+  LaneDeal D = deal_lanes(n);
+  bool done = D.rank >= n;
+  int q = q0 + (done ? 0 : D.rank);
+  const int item = unit_item(J, U, q), il = item & 255, i1 = (item >> 8) & 255, i2 = (item >> 16) & 255, i3 = item >> 24;
+  // the batch's rows: l1 in [a0, a0 + nA), l2 in [b0, b0 + nB), l3 < n3 of
+  // channels [u0, u0 + nU)
+  const int a0 = __reduce_min_sync(0xffffffffu, i1), nA = __reduce_max_sync(0xffffffffu, i1) - a0 + 1;
+  const int b0 = __reduce_min_sync(0xffffffffu, i2), nB = __reduce_max_sync(0xffffffffu, i2) - b0 + 1;
+  const int u0 = __reduce_min_sync(0xffffffffu, il), nU = __reduce_max_sync(0xffffffffu, il) - u0 + 1;
+  const int n3 = __reduce_max_sync(0xffffffffu, i3) + 1;
+  const int rows = nA + nB + nU * n3, TS = (rows + (rows + 3) / 4) | 1;
+  int at = (i1 - a0) | (nA + i2 - b0) << 8 | (nA + nB + (il - u0) * n3 + i3) << 16;  // the quadrature's rows
+  const double *Fa = J.F + (((size_t)U.c * J.nShells + U.sa) * nRuns + U.pa0) * O * nF + a0;
+  const double *Fb = J.F + (((size_t)U.c * J.nShells + U.sb) * nRuns + U.pb0) * O * nF + b0;
+  const double *Ut = J.utab + (size_t)U.c * O * LE * nk + u0 * nk;
   Ps93 S;
   xs lev;
-  xf_run run;
-  int k = -2, lvEnd = 1, cnt = 0;
+  int k = -2, cnt = 0, lvEnd = 1;  // slot 0 and slots 1, 2 are levels of their own (-2, -1)
 #pragma unroll 1
-  for (int t = 0;; t++) {
-    const int n = c93_slot[t];
-    // (the integrand is 0 outside the window)
-    if (n >= U.ws && n < U.we) {
-      const xf a = xf_mul(xf_from(__ldg(Fa + n * nF)), xf_from(__ldg(Fb + n * nF)));
-      const double u = __ldg(Ut + (size_t)n * LE * nk);
-      run.add(xf_mul(a, xf_mul(xf_from(u), xf_from(J.wSmall[n]))),
-              ent_h(__ldg(Fa + n * nF)) ^ ent_h(__ldg(Fb + n * nF)) ^ ent_h(u));
-    }
-    cnt += (t & 1) ? n >= U.ws : n <= U.we;
-    if ((t & 31) == 31 || t + 1 == lvEnd) {
-      lev = xs_plus(lev, run.sum());
-      run = xf_run();
-    }
-    if (t + 1 < lvEnd) continue;
-    if (k == -2) S.p = lev;
-    else if (k == -1) {
-      S.q = lev;
-      S.I = xs_plus(S.p, S.q);
-    } else {
-      S.I = xs_plus(S.I, lev);
-      if (ps93_end(S, V, k, cnt)) {
-        ((double *)(U.scr + U.L.T))[q] = ps93_result(S, V, k);
-        return;
+  for (int s0 = 0; s0 < O; s0 += 32) {
+    const int s1 = s0 + 32 < O ? s0 + 32 : O;
+    const int m = s0 + lane < s1 ? __ldg(J.s93 + s0 + lane) : 0;
+    const bool in = s0 + lane < s1 && m >= ws && m < we;  // (the integrand is 0 outside the window)
+    const unsigned inw = __ballot_sync(0xffffffffu, in);
+    const unsigned counts = __ballot_sync(0xffffffffu, s0 + lane < s1 && ((lane & 1) ? m >= ws : m <= we));
+    __syncwarp();
+    if (in) {
+      u64 *M = tab + lane * TS;
+      short *E = (short *)(M + rows);
+      const xf w = xf_from(J.wSmall[m]);
+      int i = 0;
+#pragma unroll 1
+      for (int g = 0; g < 2 + nU; g++) {
+        const double *src = g == 0 ? Fa + (size_t)m * nF : g == 1 ? Fb + (size_t)m * nF : Ut + ((size_t)m * LE + g - 2) * nk;
+        const int cntR = g == 0 ? nA : g == 1 ? nB : n3;
+#pragma unroll 1
+        for (int r = 0; r < cntR; r++, i++) {
+          const double x = __ldg(src + r);
+          xf v = xf_from(x);
+          if (g >= 2) v = norm1(xf_mul(v, w));
+          M[i] = v.m;
+          E[i] = (short)(v.e * 4 + (int)(sign_of(x) >> 31));
+        }
       }
     }
-    lev = xs();
-    if (++k >= c93_nLevels) break;
-    lvEnd = k < 0 ? 3 : c93_lvEnd[k];
-    cnt = 0;
+    __syncwarp();
+#pragma unroll 1
+    for (int t = s0; t < s1;) {
+      const int te = lvEnd < s1 ? lvEnd : s1;
+      const unsigned bits = (te - s0 >= 32 ? ~0u : (1u << (te - s0)) - 1u) & ~0u << (t - s0);
+      cnt += __popc(counts & bits);
+      const int ra = at & 255, rb = (at >> 8) & 255, ru = at >> 16;
+      xf_run run;
+#pragma unroll 1
+      for (int x = t + D.part; x < te; x += D.P)
+        if (inw >> (x - s0) & 1u) {
+          const u64 *M = tab + (x - s0) * TS;
+          const short *E = (const short *)(M + rows);
+          const int e = E[ra] + E[rb] + E[ru];
+          run.add({mul_hi(mul_hi(M[ra], M[rb]), M[ru]), (e >> 2) + 128}, (uint32_t)e << 31);
+        }
+      lev = xs_plus(lev, combine(run.sum(), D.P));
+      t = te;
+      if (t < lvEnd) break;
+      if (k == -2) S.p = lev;
+      else if (k == -1) {
+        S.q = lev;
+        S.I = xs_plus(S.p, S.q);
+      } else {
+        S.I = xs_plus(S.I, lev);
+        if (!done && ps93_end(S, V, k, cnt)) {
+          done = true;
+          if (D.part == 0) ((double *)(U.scr + U.L.T))[q] = ps93_result(S, V, k);
+        }
+      }
+      lev = xs();
+      cnt = 0;
+      k++;
+      lvEnd = k < 0 ? 3 : c93_lvEnd[k];  // k <= the level count, inside the 32-entry table
+      const unsigned act = __ballot_sync(0xffffffffu, !done && D.part == 0);
+      n = __popc(act);
+      if (n == 0) return;
+      const LaneDeal N = deal_lanes(n);
+      if (N.P != D.P) {  // the running quadratures move to the first lanes
+        if (!done && D.part == 0) quad[__popc(act & ((1u << lane) - 1u))] = lane;
+        __syncwarp();
+        const int src = N.rank < n ? quad[N.rank] : 0;
+        __syncwarp();
+        D = N;
+        done = D.rank >= n;
+        q = __shfl_sync(0xffffffffu, q, src);
+        at = __shfl_sync(0xffffffffu, at, src);
+        S.I = from_lane(S.I, src);
+        S.p = from_lane(S.p, src);
+        S.q = from_lane(S.q, src);
+      }
+    }
   }
-  atomicOr((unsigned *)(U.scr + U.L.mask) + (q >> 5), 1u << (q & 31));
-  if (kMixed)
-    atomicMax(&((UnitHead *)U.scr)->est, (u64)__double_as_longlong(fabs(ps93_result(S, V, c93_nLevels - 1))));
+  if (!done && D.part == 0) {
+    atomicOr((unsigned *)(U.scr + U.L.mask) + (q >> 5), 1u << (q & 31));
+    if (kMixed)
+      atomicMax(&((UnitHead *)U.scr)->est, (u64)__double_as_longlong(fabs(ps93_result(S, V, c93_nLevels - 1))));
+  }
 }
 
 // One warp a CTA; each takes up to J.take entries of the type-1 groups, then
@@ -876,7 +941,7 @@ __global__ void __launch_bounds__(32, 20) k_unit_small(DevJob J) {
   extern __shared__ double sm[];
   __shared__ LevelTab V;
   level_tab(V, c93_3n, c93_nLevels, J.tol);
-  const SmallSmem L = small_layout(J.maxLBS, J.gcap);
+  const SmallSmem L = small_layout(J.maxLBS, J.t2Rows, J.gcap);
   const int n1 = (int)J.counters[kCntT1], n = n1 + (int)J.counters[kCntT2];
 #pragma unroll 1
   for (int taken = 0; taken < J.take; taken++) {
@@ -885,7 +950,7 @@ __global__ void __launch_bounds__(32, 20) k_unit_small(DevJob J) {
     const int2 it = i < n1 ? J.listT1[i] : J.listT2[i - n1];
     const Unit U = unit_load(J, it.x);
     if (i >= n1) {
-      t2_small<kMixed>(J, U, V, it.y);
+      t2_small<kMixed>(J, U, V, (u64 *)(sm + L.tab), (int *)(sm + L.quad), it.y);
       continue;
     }
     const long long t0 = J.classCycles ? clock64() : 0;
@@ -1139,7 +1204,7 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
   // Whose tables slot t reads (the reference's reused buffers): this pair's
   // below its break; beyond it, on the lower half, the last earlier pair
   // whose loop reached that point; and the point, exponent of that pair.
-  auto locate = [&](int t, int &owner, double &r, double &ex) {
+  auto locate = [&](int t, int &owner, double &r, i64 &E) {
     const int n = __ldg(J.s92 + t);
     const bool upper = t > 0 && ((t - 1) & 1);
     owner = -1;
@@ -1153,9 +1218,10 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
     if (owner < 0) return;
     const double zaj = owner == k ? za : pzA[owner / Nb], zbj = owner == k ? zb : pzB[owner % Nb];
     r = map[owner].x * J.xLarge[n] + map[owner].y;
-    const double d1 = dAC - r, d2 = dBC - r;
-    ex = -zaj * d1 * d1 - zbj * d2 * d2;
+    // za (dAC - r)^2 + zb (dBC - r)^2 in Q53, saturating
+    E = -(i64)(fx_gauss(zaj, dAC - r) + fx_gauss(zbj, dBC - r));
   };
+  const i64 thr = fx_q53(J.lnAcc2);
   // A slot needs its tables only where they are not negligible; the others
   // integrate to exactly zero.  Slots are classified step by step (cheap),
   // the needed ones queued, and each pass evaluates 32 queued slots, one per
@@ -1178,9 +1244,10 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
           need = n >= nLo && n <= nHi;
         } else if (n <= mb && n != nb && !(t > 0 && ((t - 1) & 1))) {
           int owner;
-          double r, ex;
-          locate(t, owner, r, ex);
-          need = owner >= 0 && ex >= J.lnAcc2;
+          double r;
+          i64 E;
+          locate(t, owner, r, E);
+          need = owner >= 0 && E >= thr;
         }
       }
       const unsigned m = __ballot_sync(0xffffffffu, need);
@@ -1194,8 +1261,9 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
     if (lane < nE) {
       const int t = pend[lane], n = __ldg(J.s92 + t);
       int owner;
-      double r, ex;
-      locate(t, owner, r, ex);
+      double r;
+      i64 E;
+      locate(t, owner, r, E);
       // the pair's own exponents (no integer divide) unless a stale slot
       const double zaj = owner == k ? za : pzA[owner / Nb], zbj = owner == k ? zb : pzB[owner % Nb];
       double *e = tab + lane * TS;
@@ -1203,7 +1271,7 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
         // the same rows in double-single
         ff *Uc = (ff *)e, *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
         const ff rf = ff_from_double(r);
-        const ff wB = ff_mul(ff_mul(J.wLf[n], i1f), ff_mul(Ckf, ff_exp(ff_from_double(ex))));
+        const ff wB = ff_mul(ff_mul(J.wLf[n], i1f), ff_mul(Ckf, ff_exp(ff_from_double((double)E * 0x1p-53))));
         channels_ff(J, c, rf, pMask, Uc);
 #pragma unroll 1
         for (int side = 0; side < 2; side++)
@@ -1221,7 +1289,7 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
         short *Ue = (short *)(tab + 32 * TS) + lane * ES, *Ae = Ue + LE, *Be = Ae + LBE, *Re = Be + LBE;
         const double w = J.wLarge[n];
         const xf Rx = xf_from(r);
-        xf wB = xf_mul(fx_exp(fx_q53(ex)), xf_mul(xf_mul(xf_from(w), xf_from(i1)), xf_from(Ck)));
+        xf wB = xf_mul(fx_exp(E), xf_mul(xf_mul(xf_from(w), xf_from(i1)), xf_from(Ck)));
         // the rows of both centres through one copy of the Bessel code
 #pragma unroll 1
         for (int side = 0; side < 2; side++) {
@@ -1476,7 +1544,7 @@ __global__ void __launch_bounds__(32, 16) k_unit_large(DevJob J) {
 // One unit a CTA: the type-1 block from the quadratures of its primitive
 // pairs (src/type1.c:323-345), the type-2 block from its radial table
 // (src/type2.c:583-623), both shifted onto A and B (src/util.c:247-334).
-__global__ void __launch_bounds__(kLinkThreads) k_unit_link(DevJob J) {
+__global__ void __launch_bounds__(kLinkThreadsMax) k_unit_link(DevJob J) {
   extern __shared__ double sm[];
   int pos = J.chunk0 + blockIdx.x;
   if (J.live) {
@@ -1487,7 +1555,7 @@ __global__ void __launch_bounds__(kLinkThreads) k_unit_link(DevJob J) {
   const Unit U = unit_load(J, pos);
   if (!U.live) return;
   const LinkSmem Lm = link_layout(J.maxLBS, J.maxLECP);
-  const int tid = threadIdx.x, NT = kLinkThreads, lab = U.lab, lq = lab + 1, Nb = U.Nb;
+  const int tid = threadIdx.x, NT = blockDim.x, lab = U.lab, lq = lab + 1, Nb = U.Nb;
   double *rsh = sm + Lm.rsh, *dir = sm + Lm.dir, *W = sm + Lm.W, *H = sm + Lm.H;
   const int dd = J.tmDim + 1, tmW = (J.tmDim + 1) * (J.tmDim + 1), RQ = lq * lq, nq = t1_items(lab);
   // type 1: W[L][l][m] = sum over the primitive pairs of S_lm Q[L][l] (the
@@ -1708,7 +1776,7 @@ int launch_fast_pipeline(const DevJob &J, cudaStream_t st, const FastConfig &cfg
   for (int i = 0; i < kMaxClasses; i++) Jc.classCfg[i] = cfg.cls[i];
   Jc.classCycles = cfg.classCycles;
   const JobPlan::Order &ord = use_order(Jc, cfg.sorted);
-  const size_t sSmall = fast_smem_bytes(J.maxLBS, cfg.gcap);
+  const size_t sSmall = fast_smem_bytes(J.maxLBS, J.t2Rows, cfg.gcap);
   const size_t sLarge = sizeof(double) * (size_t)large_layout(J.maxLBS, J.maxLECP, false).total;
   const size_t sLink = sizeof(double) * (size_t)link_layout(J.maxLBS, J.maxLECP).total;
   if (sSmall > 200 * 1024 || sLarge > 200 * 1024 || sLink > 200 * 1024) return 3;
@@ -1734,7 +1802,7 @@ int launch_fast_pipeline(const DevJob &J, cudaStream_t st, const FastConfig &cfg
     K.take = takeLarge;
     if (cfg.mixed) k_unit_large<true><<<gLarge, 32, sLarge, st>>>(K);
     else k_unit_large<false><<<gLarge, 32, sLarge, st>>>(K);
-    k_unit_link<<<units, kLinkThreads, sLink, st>>>(K);
+    k_unit_link<<<units, link_threads(sLink), sLink, st>>>(K);
   });
   if (u1) record_timing(u1, st);
   launch_epilogue(Jc, st);

@@ -261,6 +261,14 @@ ECPGB_HD i64 fx_q53(double x) {
   return (i64)b < 0 ? -v : v;
 }
 
+// z d^2 in Q53 (z > 0), saturating at 2^62.
+ECPGB_HD u64 fx_gauss(double z, double d) {
+  const xf D = xf_from(d), v = xf_mul(xf_from(z), xf_mul(D, D));
+  const int sh = v.e + 53;
+  const u64 E = sh <= 0 ? shr64(v.m, -sh) : (v.m >> (63 - (sh > 63 ? 63 : sh)) ? ~0ull : v.m << sh);
+  return E < 1ull << 62 ? E : 1ull << 62;
+}
+
 // A signed number m * 2^e, |m| < 2^62: the running values of a quadrature.
 // Sums align to the larger exponent and are never renormalised upwards
 // (cancelled bits stay cancelled); an empty sum has the smallest exponent.

@@ -237,7 +237,7 @@ struct DevTables {
   DBuf<short> byN93;
   DBuf<long long> besX, besXA;  // fixed-point Bessel rows
   DBuf<double> besD;            // derivative rows (plain path)
-  int nItemsMax = 0;
+  int nItemsMax = 0, t2Rows = 0;
 };
 
 // The small-grid schedule's slots step by step (33, then 32 at a time) in
@@ -348,6 +348,24 @@ struct Engine {
           tot += (int)tmp.size();
         }
         t->nItemsMax = std::max(t->nItemsMax, tot);
+        // rows that a batch of up to 32 consecutive items reads of the two F
+        // tables and of the r^k U_l table (a centre's items are a prefix)
+        const size_t first = items.size() - tot;
+        for (int q0 = 0; q0 < tot; q0 += 32) {
+          int lo[3] = {99, 99, 99}, hi[3] = {0, 0, 0}, n3 = 0;
+          for (int q = q0; q < std::min(tot, q0 + 32); q++) {
+            const int v = items[first + q];
+            int l = 0;
+            for (int at = cnt[cnt.size() - LE]; q >= at; at += cnt[cnt.size() - LE + l]) l++;
+            const int x[3] = {l, v & 255, (v >> 8) & 255};
+            for (int i = 0; i < 3; i++) {
+              lo[i] = std::min(lo[i], x[i]);
+              hi[i] = std::max(hi[i], x[i]);
+            }
+            n3 = std::max(n3, (v >> 16) + 1);
+          }
+          t->t2Rows = std::max(t->t2Rows, hi[1] - lo[1] + 1 + hi[2] - lo[2] + 1 + (hi[0] - lo[0] + 1) * n3);
+        }
       }
     ok = ok && t->itemOff.upload(off, stream) && t->itemCnt.upload(cnt, stream) &&
          t->items.upload(items, stream);
@@ -624,6 +642,7 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.angC = ncum(h.maxLBS);
   J.uspD = h.maxLBS + 1;
   J.largeOrder = (int)h.xl.size();
+  J.t2Rows = T->t2Rows;
   J.tol = P.tol; J.acc = P.acc;
   J.lnAcc1 = std::log(P.acc) - 2;
   J.lnAcc2 = std::log(1.0E-14) - 2;
@@ -1188,7 +1207,7 @@ int job_tune(void *vj, ecpgb_launch_config *chosen, ecpgb_launch_config *trials,
   FastConfig bestCfg = R->cfg;
   int n = 0;
   for (const FastConfig &c : cand) {
-    if (fast_ctas_per_sm(fast_smem_bytes(R->J.maxLBS, c.gcap)) < 1) continue;
+    if (fast_ctas_per_sm(fast_smem_bytes(R->J.maxLBS, R->J.t2Rows, c.gcap)) < 1) continue;
     float tot = 0;
     for (int r = 0; r < 3; r++) {
       cudaMemsetAsync(E.flush.p, r & 0xff, flushBytes, E.stream);
@@ -1295,7 +1314,7 @@ int job_config(void *vj, const ecpgb_launch_config *cfg, ecpgb_launch_config *ou
     c.gcap = cfg->gcap;
     c.balance = cfg->balance ? 1 : 0;
     c.screen = cfg->screen ? 1 : 0;
-    if (fast_ctas_per_sm(fast_smem_bytes(R->J.maxLBS, c.gcap)) < 1) {
+    if (fast_ctas_per_sm(fast_smem_bytes(R->J.maxLBS, R->J.t2Rows, c.gcap)) < 1) {
       set_error("configuration does not fit on an SM");
       return 1;
     }

@@ -177,9 +177,10 @@ struct PairFx {
 struct SmallSmem {
   int sc, fx, quad, tab, total;
 };
-__host__ __device__ inline SmallSmem small_layout(int LB, int cap) {
+__host__ __device__ inline SmallSmem small_layout(int LB, int rows, int cap) {
   SmallSmem s;
-  int tt = 0;
+  // type 2 (batched path): 32 slots of the most rows a batch reads
+  int tt = 32 * ((rows + (rows + 3) / 4) | 1);
   for (int lab = 0; lab <= 2 * LB; lab++) {
     const int w = 33 * t1_group(lab, cap) * (2 * lab + 3);
     if (w > tt) tt = w;
@@ -504,10 +505,13 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
 // The blocks of a unit from its combined-index block H (type 1) and its radial
 // table (type 2, src/type2.c:583-623), both shifted onto A and B
 // (src/util.c:247-334), and its status.
-constexpr int kLinkThreads = 128;
+constexpr int kLinkThreadsMax = 256;
+// Threads a CTA: 256 where the shared memory (g shells) lets only a few CTAs
+// share a multiprocessor.
+static inline int link_threads(size_t smem) { return smem > 40 * 1024 ? 256 : 128; }
 template <bool kExact>
 static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSmem &Lm, double *sm) {
-  const int tid = threadIdx.x, NT = kLinkThreads, la = U.la, lb = U.lb, lpa = U.lpa, lpb = U.lpb, nca = NCUM(la),
+  const int tid = threadIdx.x, NT = blockDim.x, la = U.la, lb = U.lb, lpa = U.lpa, lpb = U.lpb, nca = NCUM(la),
             ncb = NCUM(lb), Lc = U.Lc;
   const int nA = 2 * J.maxLBS + 1, LE = J.maxLECP > 0 ? J.maxLECP : 1, LBE = J.maxLBS + LE;
   const size_t cA = (size_t)U.c * J.nAtoms + U.A, cB = (size_t)U.c * J.nAtoms + U.B;
