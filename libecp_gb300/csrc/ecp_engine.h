@@ -124,6 +124,7 @@ struct DevJob {
   long long scrBase;
   int2 *listT1, *listT2, *listPart;
   struct T1Fail *listFail;
+  bool plain;                    // runs the plain path's stages
   bool few, single;              // few primitive pairs in all; one primitive pair a type-2 part
   int take;                      // work-list entries a warp takes before it exits
   int gcap;                      // type-1 step-table width cap (doubles per slot)

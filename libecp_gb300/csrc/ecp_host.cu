@@ -521,6 +521,22 @@ static bool few_pairs(const Parsed &P) {
   return n <= kFewPairs;
 }
 
+// Whether a batched job runs the plain path's stages.  The batched path's
+// integer arithmetic takes finite inputs of the magnitudes that basis sets and
+// potentials have, decaying primitives and thresholds below 1; outside that
+// (NaN, infinities, ECP exponents below 0, ...) FP64 decides what comes out.
+static bool plain_stages(const Parsed &P, int mode) {
+  if (mode == ECPGB_FP64) return true;
+  auto within = [](const std::vector<double> &v, double lo, double hi) {
+    for (double x : v)
+      if (!(x >= lo && x <= hi)) return false;
+    return true;
+  };
+  return !(within(P.primA, 1e-30, 1e30) && within(P.primD, -1e60, 1e60) && within(P.termA, 0.0, 1e30) &&
+           within(P.termD, -1e100, 1e100) && within(P.termN, -16.0, 16.0) && P.acc >= 1e-300 && P.acc <= 1.0 &&
+           P.tol >= 1e-300 && P.tol <= 1e100);
+}
+
 // Scratch of a job with chunks of at most `cap` bytes (at least one
 // pair's units a chunk).
 static size_t scratch_bytes(const Parsed &P, size_t cap, bool single) {
@@ -625,13 +641,16 @@ size_t job_device_bytes(const Parsed &P, int mode, size_t budget, size_t *scratc
   // other buffers fit is never refused for it
   const size_t base = in + work, cap = base < budget ? std::min(kScratchCap, budget - base) : 0;
   if (scratchCap) *scratchCap = cap;
-  return base > budget ? base : std::min(budget, base + scratch_bytes(P, cap, mode == ECPGB_FP64 || few_pairs(P)));
+  return base > budget ? base : std::min(budget, base + scratch_bytes(P, cap, plain_stages(P, mode) || few_pairs(P)));
 }
 
 int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int mode, cudaStream_t stream,
               size_t scratchCap) {
   const HostTables &h = T->host;
   std::memset(&J, 0, sizeof J);
+  J.plain = plain_stages(P, mode);
+  J.few = few_pairs(P);
+  J.single = J.few || J.plain;
   J.nAtoms = P.nAtoms; J.nShells = P.nShells; J.nPrims = P.nPrims; J.nCentres = P.nCentres;
   J.nPairs = P.nPairs; J.dim = P.dim;
   J.maxLECP = h.maxLECP; J.maxLBS = h.maxLBS; J.maxLambda = h.maxLambda; J.nk = h.nk; J.nF = h.nF;
@@ -737,8 +756,6 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
     J.scr = B.scr.p;
     J.counters = (unsigned *)(B.err.p + 2);
     J.plan = &B.plan;
-    J.few = few_pairs(P);
-    J.single = J.few || mode == ECPGB_FP64;
     J.pairOrders = (const int *)dp(iOrd);
     J.scrOffs = (const long long *)dp(iOff);
     J.chunkPairs = (const int *)dp(iChk);
@@ -770,7 +787,7 @@ int run_pipeline(JobBuffers &B, const DevJob &J, int mode, cudaEvent_t u0, cudaE
                  const FastConfig *cfg, cudaStream_t stream) {
   CUDA_OK(cudaMemsetAsync(B.mat.p, 0, sizeof(double) * (size_t)J.dim * J.dim, stream));
   int rc;
-  if (mode == ECPGB_FAST || mode == ECPGB_MIXED) {
+  if (!J.plain) {
     FastConfig c = cfg ? *cfg : engine().config_for(J.maxLBS, J.maxLECP);
     c.mixed = mode == ECPGB_MIXED;
     rc = launch_fast_pipeline(J, stream, c, u0, u1);
@@ -1194,7 +1211,7 @@ int job_tune(void *vj, ecpgb_launch_config *chosen, ecpgb_launch_config *trials,
   cand.push_back(mk(0, 0, 45, 1));
   cand.push_back(mk(1, 1, 45, 0));
   for (int gcap : {45, 64}) cand.push_back(mk(1, 2, gcap, 1));
-  cand.push_back(mk(1, 2, 45, 0));
+  cand.push_back(FastConfig{});
   FastConfig noScreen = mk(1, 1, 45, 1);
   noScreen.screen = 0;
   cand.push_back(noScreen);
@@ -1296,7 +1313,7 @@ int job_tune(void *vj, ecpgb_launch_config *chosen, ecpgb_launch_config *trials,
   if (nTrials) *nTrials = n < maxTrials ? n : maxTrials;
   R->cfg = bestCfg;
   R->drop_graph();
-  E.tuned[{R->J.maxLBS, R->J.maxLECP}] = bestCfg;
+  if (!R->J.plain) E.tuned[{R->J.maxLBS, R->J.maxLECP}] = bestCfg;
   if (chosen) *chosen = to_c(bestCfg, best);
   return 0;
 }
@@ -1379,9 +1396,9 @@ int job_launches(const void *vj) {
   const int scatter = R->P.deriv ? 0 : 1;
   // two per-job stages, the four unit stages per chunk, the AO scatter (order
   // 0), and with the batched path's compacted queue the three screening kernels
-  const FastConfig cfg = R->mode == ECPGB_FP64 ? FastConfig{} : R->cfg;
+  const FastConfig cfg = R->J.plain ? FastConfig{} : R->cfg;
   int n = 2 + 4 * (int)R->B.plan.order[cfg.sorted].chunks.size() + scatter;
-  if (R->mode != ECPGB_FP64 && cfg.queue && cfg.screen) n += 3;
+  if (!R->J.plain && cfg.queue && cfg.screen) n += 3;
   return n;
 }
 

@@ -90,3 +90,28 @@ def test_plain_stages_equal_the_single_kernel_bit_for_bit(eg, name):
     s = PLAIN[name]()
     rc, I, _ = eg.get_integrals_info(s, mode=eg.ECPGB_FP64)
     assert np.array_equal(np.triu(I), np.triu(_noalloc(eg, s)))
+
+
+ODD = {
+    "nan_coefficient": lambda s: s.dBS.__setitem__(0, np.nan),
+    "infinite_ecp_coefficient": lambda s: s.dECP.__setitem__(1, np.inf),
+    "growing_potential": lambda s: s.aECP.__setitem__(1, -0.01),
+    "huge_coefficient": lambda s: s.dBS.__setitem__(0, 1e200),
+    "high_power": lambda s: s.nECP.__setitem__(0, 24.0),
+    "loose_accuracy": lambda s: setattr(s, "accuracy", 10.0),
+}
+
+
+@pytest.mark.parametrize("mode_name", ["ECPGB_FAST", "ECPGB_MIXED"])
+@pytest.mark.parametrize("name", list(ODD))
+def test_inputs_outside_the_integer_range_take_the_plain_stages(eg, mode_name, name):
+    s = W.example_like(0)
+    ODD[name](s)
+    ref, got = eg.blocks(s, mode=eg.ECPGB_FP64), eg.blocks(s, mode=getattr(eg, mode_name))
+    assert np.array_equal(ref[0], got[0]) and np.array_equal(ref[1], got[1], equal_nan=True)
+    launches = []
+    for mode in (eg.ECPGB_FP64, getattr(eg, mode_name)):
+        job = eg.Job(s, mode=mode)
+        launches.append(job.launches_per_run())
+        job.close()
+    assert launches[0] == launches[1]
