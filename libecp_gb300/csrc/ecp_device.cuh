@@ -144,14 +144,24 @@ static __device__ __noinline__ void bessel_rows(const DevJob &J, int lmax, doubl
 // whether the shell is screened out entirely (src/type2.c:149-180), written
 // to J.win and to w[3]; dAC = |C - A|.  One thread computes it.
 static __device__ void shell_window(const DevJob &J, int s, int c, double dAC, int *w) {
-  int end = J.gridEnd[c], j;
-  double R = J.radius[s], rmin = dAC - R, rmax = dAC + R;
-  for (j = end; j >= 0; j--)
-    if (J.xSmall[j] < rmin) break;
-  w[0] = j + 1;
-  for (j = end; j >= 0; j--)
-    if (J.xSmall[j] <= rmax) break;
-  w[1] = (j < 0 || J.xSmall[j] > rmax) ? -1 : j;
+  const int end = J.gridEnd[c];
+  const double R = J.radius[s], rmin = dAC - R, rmax = dAC + R;
+  // points 0 .. end below rmin, and up to rmax (xSmall ascends)
+  int lo = 0, hi = end + 1;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (J.xSmall[mid] < rmin) lo = mid + 1;
+    else hi = mid;
+  }
+  w[0] = lo;
+  lo = 0;
+  hi = end + 1;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (J.xSmall[mid] <= rmax) lo = mid + 1;
+    else hi = mid;
+  }
+  w[1] = lo - 1;
   w[2] = !(w[1] >= w[0]) || R < 0;
   int *g = J.win + ((size_t)c * J.nShells + s) * 3;
   g[0] = w[0]; g[1] = w[1]; g[2] = w[2];

@@ -31,7 +31,8 @@ constexpr int kSmallOrder = 383;       // PS93(128) abscissae
 constexpr int kMaxLargeOrder = 4095;   // PSM92 abscissae (largeGridOrder < 8192)
 constexpr int kMaxContraction = 16;    // primitives per shell
 constexpr int kUnitThreads = 128;      // threads per unit CTA
-constexpr int kPointThreads = 384;     // per-job stages: a thread per small-grid point
+constexpr int kPointThreads = 384;     // F tables: a thread per small-grid point
+constexpr int kStageThreads = 128;     // the other per-job stages
 constexpr int kChunkPairs = 64;        // (lower, upper) pairs per fallback chunk
 constexpr int kMaxWalkers = 512;       // large-grid quadratures integrated per pass
 
@@ -101,6 +102,7 @@ struct DevJob {
   double *radius;
   double *utab, *uL;
   int *gridEnd;
+  unsigned *tickets;     // per centre: finished CTAs of its potential's items (0 between runs)
   int *win;
   double *F;
   double *cgeo, *usp, *ang;
@@ -259,6 +261,8 @@ void launch_epilogue(const DevJob &job, cudaStream_t stream);
 void launch_stage1(const DevJob &job, cudaStream_t stream);
 
 void launch_shell_F(const DevJob &job, cudaStream_t stream);
+// Threads a CTA of the F-table kernels.
+int point_threads(const DevJob &job);
 // The Bessel table's derivative rows (DevJob::besD), written to D.
 void launch_bessel_rows(const DevJob &job, double *D, cudaStream_t stream);
 

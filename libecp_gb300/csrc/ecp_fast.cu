@@ -1638,8 +1638,8 @@ __global__ void __launch_bounds__(kPointThreads) k_shell_F_fast(DevJob J) {
   for (int run = 0; run < nRuns; run++) {
     const int lmaxA = J.maxLECP - 1 + J.shL[s] + run;
     double *F = J.F + (((size_t)c * J.nShells + s) * nRuns + run) * O * nF;
-#pragma unroll 1
-    for (int n = threadIdx.x; n < O; n += blockDim.x) {
+    const int n = blockIdx.z * blockDim.x + threadIdx.x;
+    if (n < O) {
       double acc[kMaxRows], K[kMaxRows];
 #pragma unroll 1
       for (int i = 0; i < nF; i++) acc[i] = 0.0;
@@ -1783,7 +1783,8 @@ int launch_fast_pipeline(const DevJob &J, cudaStream_t st, const FastConfig &cfg
   const bool screen = cfg.queue && cfg.screen;
   if (!screen) Jc.live = nullptr;
   launch_stage1(Jc, st);
-  k_shell_F_fast<<<dim3(J.nShells, J.nCentres), kPointThreads, 0, st>>>(Jc);
+  const int nt = point_threads(J);
+  k_shell_F_fast<<<dim3(J.nShells, J.nCentres, (kSmallOrder + nt - 1) / nt), nt, 0, st>>>(Jc);
   const long long nUnits = (long long)J.nCentres * J.nPairs;
   if (screen && nUnits > 0) {  // screening stage: the live units' positions
     const long long nb = (nUnits + kScreenThreads - 1) / kScreenThreads;

@@ -45,47 +45,57 @@ static __device__ void radius_of(const DevJob &J, int s) {
 
 __global__ void k_radius(DevJob J) { radius_of(J, blockIdx.x * blockDim.x + threadIdx.x); }
 
-static __device__ void centre_of(const DevJob &J, int c) {
-  extern __shared__ double sU[];  // (L+1) x 383
+// U_l (channel l, small-grid point n) of centre c, item i = l * 383 + n: the
+// local part to uL, the others to their first slot in utab (centre_finish).
+static __device__ void centre_item(const DevJob &J, int c, int i) {
+  const int L = J.ctrL[c], O = kSmallOrder, l = i / O, n = i - l * O;
+  if (l > L) return;
+  const int LE = J.maxLECP > 0 ? J.maxLECP : 1;
+  const double u = eval_ecp(J, c, l, J.xSmall[n]);
+  if (l == L) J.uL[(size_t)c * O + n] = u;
+  else J.utab[(((size_t)c * O + n) * LE + l) * J.nk] = u;
+}
+
+// The channels' grid ends and the table U_l r^k, by one CTA once every item of
+// the centre is written (by other CTAs too: read past L1).
+static __device__ void centre_finish(const DevJob &J, int c) {
   __shared__ int sEnd[kMaxLEcp + 1];
   __shared__ int sBest;
-  const int L = J.ctrL[c], O = kSmallOrder;
-  for (int n = threadIdx.x; n < O; n += blockDim.x) {
-    double r = J.xSmall[n];
-    for (int l = 0; l <= L; l++) sU[l * O + n] = eval_ecp(J, c, l, r);
-  }
-  __syncthreads();
+  const int L = J.ctrL[c], O = kSmallOrder, LE = J.maxLECP > 0 ? J.maxLECP : 1, nk = J.nk;
+  double *tab = J.utab + (size_t)c * O * LE * nk;
   int end = O - 1;
   for (int l = 0; l < L; l++) {
     if (threadIdx.x == 0) sBest = -1;
     __syncthreads();
     int best = -1;
     for (int i = threadIdx.x; i <= end; i += blockDim.x)
-      if (fabs(sU[l * O + i]) > 1.0E-14) best = i;
+      if (fabs(__ldcg(tab + ((size_t)i * LE + l) * nk)) > 1.0E-14) best = i;
     if (best >= 0) atomicMax(&sBest, best);
     __syncthreads();
     end = sBest;
     if (threadIdx.x == 0) sEnd[l] = end;
     __syncthreads();
   }
-  const int LE = J.maxLECP > 0 ? J.maxLECP : 1, nk = J.nk;
-  for (int n = threadIdx.x; n < O; n += blockDim.x) {
-    double r = J.xSmall[n];
-    double *dst = J.utab + ((size_t)c * O + n) * LE * nk;
-    for (int l = 0; l < LE; l++) {
-      double v = (l < L && n <= sEnd[l]) ? sU[l * O + n] : 0.0;
-      bool live = (l < L && n <= sEnd[l]);
-      for (int k = 0; k < nk; k++) {
-        dst[l * nk + k] = live ? v : 0.0;
-        v = v * r;
-      }
+  for (int i = threadIdx.x; i < O * LE; i += blockDim.x) {
+    const int l = i / O, n = i - l * O;
+    const double r = J.xSmall[n];
+    double *dst = tab + ((size_t)n * LE + l) * nk;
+    const bool live = l < L && n <= sEnd[l];
+    double v = live ? __ldcg(dst) : 0.0;
+    for (int k = 0; k < nk; k++) {
+      dst[k] = live ? v : 0.0;
+      v = v * r;
     }
-    J.uL[(size_t)c * O + n] = sU[L * O + n];
   }
   if (threadIdx.x == 0) J.gridEnd[c] = end;
 }
 
-__global__ void __launch_bounds__(128) k_centre(DevJob J) { centre_of(J, blockIdx.x); }
+__global__ void __launch_bounds__(128) k_centre(DevJob J) {
+  const int c = blockIdx.x;
+  for (int i = threadIdx.x; i < (J.ctrL[c] + 1) * kSmallOrder; i += blockDim.x) centre_item(J, c, i);
+  __syncthreads();
+  centre_finish(J, c);
+}
 
 static __device__ void centre_atom_of(const DevJob &J, int A, int c) {
   __shared__ double rsh[169];
@@ -156,19 +166,32 @@ static __device__ void centre_atom_of(const DevJob &J, int A, int c) {
 
 __global__ void __launch_bounds__(64) k_centre_atom(DevJob J) { centre_atom_of(J, blockIdx.x, blockIdx.y); }
 
-// The three stages above in one launch (the batched path): centres, (centre,
-// atom) pairs, then the shells.  errWord[1] is cleared before the launch
-// (the shells set it), errWord[0] here.
-__global__ void __launch_bounds__(kPointThreads) k_stage1(DevJob J) {
+// The three stages above in one launch: centres, (centre, atom) pairs, then the
+// shells.  errWord[1] is cleared before the launch (the shells set it),
+// errWord[0] here.  A centre's points are a chain of exponentials on the FP64
+// pipe, one per term: a thread an item (channel, point) on `centreCtas` CTAs, the
+// last of which to finish makes the table (12-shell matrix: 34 instead of 46 us,
+// where a CTA had a whole centre; the radii's Newton steps are the rest).
+__global__ void __launch_bounds__(kStageThreads) k_stage1(DevJob J, int centreCtas) {
+  __shared__ bool last;
   int b = blockIdx.x;
   if (b == 0 && threadIdx.x == 0) J.errWord[0] = INT_MAX;
-  if (b < J.nCentres) {
-    centre_of(J, b);
+  if (b < J.nCentres * centreCtas) {
+    const int c = b / centreCtas;
+    centre_item(J, c, (b - c * centreCtas) * kStageThreads + threadIdx.x);
+    __threadfence();
+    __syncthreads();
+    // (wraps to 0 for the next run)
+    if (threadIdx.x == 0) last = (int)atomicInc(J.tickets + c, (unsigned)centreCtas - 1u) == centreCtas - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    centre_finish(J, c);
     return;
   }
-  b -= J.nCentres;
+  b -= J.nCentres * centreCtas;
   if (b < J.nCentres * J.nAtoms) centre_atom_of(J, b % J.nAtoms, b / J.nAtoms);
-  else radius_of(J, (b - J.nCentres * J.nAtoms) * kPointThreads + threadIdx.x);
+  else radius_of(J, (b - J.nCentres * J.nAtoms) * kStageThreads + threadIdx.x);
 }
 
 // The derivative rows of every Bessel table point (src/bessel.c:195-212), by
@@ -191,6 +214,7 @@ __global__ void k_bessel_rows(DevJob J, double *D) {
   }
 }
 
+// One thread a point, gridDim.z CTAs a (shell, centre).
 __global__ void __launch_bounds__(kPointThreads) k_shell_F(DevJob J) {
   __shared__ int sw[3];
   const int s = blockIdx.x, c = blockIdx.y, O = kSmallOrder;
@@ -207,7 +231,8 @@ __global__ void __launch_bounds__(kPointThreads) k_shell_F(DevJob J) {
   for (int run = 0; run < nRuns; run++) {
     const int lmaxA = J.maxLECP - 1 + J.shL[s] + run;
     double *F = J.F + (((size_t)c * J.nShells + s) * nRuns + run) * O * nF;
-    for (int n = threadIdx.x; n < O; n += blockDim.x) {
+    const int n = blockIdx.z * blockDim.x + threadIdx.x;
+    if (n < O) {
       double acc[kMaxRows], K[kMaxRows];
       for (int i = 0; i < nF; i++) acc[i] = 0.0;
       if (!sw[2] && n >= sw[0] && n < sw[1] && lmaxA >= 0) {
@@ -791,17 +816,23 @@ int launch_fp64_pipeline(const DevJob &J, cudaStream_t st, size_t smemBytes, cud
   return e == cudaSuccess ? 0 : kLaunchErrorBase + (int)e;
 }
 
+// Few CTAs leave SMs idle and the slowest sets the time: 32 points a CTA there
+// (12 shells: 27 instead of 51 us batched, 35 instead of 72 plain); with more the
+// window search and the centre's distance are worth sharing.
+int point_threads(const DevJob &J) { return (long long)J.nShells * J.nCentres <= 256 ? 32 : kPointThreads; }
+
+void launch_shell_F(const DevJob &J, cudaStream_t st) {
+  const int nt = point_threads(J);
+  k_shell_F<<<dim3(J.nShells, J.nCentres, (kSmallOrder + nt - 1) / nt), nt, 0, st>>>(J);
+}
+
 // Per-job stages before and after the unit kernel; shared by both paths
 // (the batched path launches its own F-table kernel: withF false).
 void launch_prologue(const DevJob &J, cudaStream_t st, bool withF) {
   k_radius<<<(J.nShells + 127) / 128, 128, 0, st>>>(J);
-  k_centre<<<J.nCentres, 128, sizeof(double) * kSmallOrder * (kMaxLEcp + 1), st>>>(J);
+  k_centre<<<J.nCentres, 128, 0, st>>>(J);
   k_centre_atom<<<dim3(J.nAtoms, J.nCentres), 64, 0, st>>>(J);
-  if (withF) k_shell_F<<<dim3(J.nShells, J.nCentres), kPointThreads, 0, st>>>(J);
-}
-
-void launch_shell_F(const DevJob &J, cudaStream_t st) {
-  k_shell_F<<<dim3(J.nShells, J.nCentres), kPointThreads, 0, st>>>(J);
+  if (withF) launch_shell_F(J, st);
 }
 
 void launch_bessel_rows(const DevJob &J, double *D, cudaStream_t st) {
@@ -810,8 +841,8 @@ void launch_bessel_rows(const DevJob &J, double *D, cudaStream_t st) {
 
 void launch_stage1(const DevJob &J, cudaStream_t st) {
   cudaMemsetAsync(J.errWord + 1, 0, sizeof(int), st);
-  k_stage1<<<J.nCentres * (1 + J.nAtoms) + (J.nShells + kPointThreads - 1) / kPointThreads, kPointThreads,
-             sizeof(double) * kSmallOrder * (kMaxLEcp + 1), st>>>(J);
+  const int cc = ((J.maxLECP + 1) * kSmallOrder + kStageThreads - 1) / kStageThreads;
+  k_stage1<<<J.nCentres * (cc + J.nAtoms) + (J.nShells + kStageThreads - 1) / kStageThreads, kStageThreads, 0, st>>>(J, cc);
 }
 
 void launch_epilogue(const DevJob &J, cudaStream_t st) {

@@ -632,8 +632,8 @@ size_t job_device_bytes(const Parsed &P, int mode, size_t budget, size_t *scratc
   const size_t angLam = P.maxLECP + LB + 1, angC = (LB + 1) * (LB + 2) * (LB + 3) / 6;
   size_t in = 8 * (P.geom.size() + P.primA.size() + P.primD.size() + 3 * P.termL.size() + P.pairOff.size()) +
               4 * (5 * P.shL.size() + P.atomMaxL.size() + 4 * P.ctrAtom.size() + P.termL.size() + 3 * P.pairA.size()) +
-              36 * (P.nPairs + 1) + 4 * nc + 4 * P.chanT0.size() + (mode == ECPGB_MIXED ? 16 * P.termL.size() : 0) +
-              24 * 256;
+              36 * (P.nPairs + 1) + 8 * nc + 4 * P.chanT0.size() + (mode == ECPGB_MIXED ? 16 * P.termL.size() : 0) +
+              32 * 256;
   size_t work = 8 * (ns + nc * O * LE * nk + nc * O + nc * ns * (1 + P.deriv) * O * nF + nc * na * 4 + nc * na * D * D * D +
                      nc * na * angLam * LE * LE * angC + nc * (size_t)P.centreStride + (size_t)P.dim * P.dim) +
                 4 * (nc + nc * ns * 3 + nc * (size_t)P.nPairs + 2) + 8;
@@ -687,9 +687,11 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
          iPS = add(P.pairShift.data(), 4 * P.pairShift.size()), iCh = add(P.chanT0.data(), 4 * P.chanT0.size());
   std::vector<int> orders, chunkPairs, ctr;
   std::vector<long long> offs;
-  make_plan(P, scratchCap, mode == ECPGB_FP64 || few_pairs(P), B.plan, orders, offs, chunkPairs, ctr);
+  make_plan(P, scratchCap, J.single, B.plan, orders, offs, chunkPairs, ctr);
   size_t iOrd = add(orders.data(), 4 * orders.size()), iOff = add(offs.data(), 8 * offs.size()),
          iChk = add(chunkPairs.data(), 4 * chunkPairs.size()), iCtr = add(ctr.data(), 4 * ctr.size());
+  const std::vector<unsigned> zeros(P.nCentres);
+  size_t iTk = add(zeros.data(), 4 * zeros.size());
   // the ECP terms' exponents and coefficients as float pairs (mixed path)
   std::vector<float> tAf, tDf;
   if (mode == ECPGB_MIXED) {
@@ -715,6 +717,7 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.pairB = (const int *)dp(iPrB); J.pairOff = (const long long *)dp(iPO);
   J.pairShift = (const int *)dp(iPS);
   J.chanT0 = (const int *)dp(iCh);
+  J.tickets = (unsigned *)dp(iTk);
   J.termAf = mode == ECPGB_MIXED ? (const ff *)dp(iTAf) : nullptr;
   J.termDf = mode == ECPGB_MIXED ? (const ff *)dp(iTDf) : nullptr;
   J.deriv = P.deriv;
