@@ -73,6 +73,12 @@ static __device__ __noinline__ bool t1_zero_walk(const DevJob &J, double s, doub
   return false;
 }
 
+// The bits of a double as an integer that orders like it.
+static __device__ inline long long ordered_bits(double x) {
+  const long long b = __double_as_longlong(x);
+  return b ^ (long long)((unsigned long long)(b >> 63) >> 1);
+}
+
 // FM06 map parameters (src/gc_integrators.c:317-331).
 static __device__ inline void fm06(double za, double zb, double dAC, double dBC, double &i1, double &i2) {
   double zp = za + zb, P = (za * dAC + zb * dBC) / zp;
@@ -410,45 +416,69 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
       map[k] = make_double2(i1, i2);
       if (U.nItems > 0) {
         // break index, and the point-index interval in which the pair's
-        // exponent passes the screen, by bisection: past both centres the
-        // exponent falls with the index; it is a parabola in r with its vertex
-        // at V, and r grows with the index.  (The plain path tests every slot of
-        // the interval itself: a margin of 1.)
-        const double thr = kExact ? J.lnAcc2 - 1.0 : J.lnAcc2;
-        auto exq = [&](int n, double &r) {
-          r = i1 * J.xLarge[n] + i2;
-          const double d1 = dAC - r, d2 = dBC - r;
-          return -za * d1 * d1 - zb * d2 * d2;
-        };
-        double r;
-        int lo = 0, hi = J.largeOrder;
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          const double e = exq(mid, r);
-          if (r > dAC && r > dBC && e < J.lnAcc2) hi = mid; else lo = mid + 1;
-        }
-        const int brk = lo < J.largeOrder ? lo : INT_MAX;
+        // exponent passes the screen: past both centres the exponent falls with
+        // the index; it is a parabola in r with its vertex at V, and r grows with
+        // the index.
         const double V = (za * dAC + zb * dBC) / (za + zb);
-        int a = 0, b = J.largeOrder;
-        while (a < b) {
-          const int mid = (a + b) >> 1;
-          if (i1 * J.xLarge[mid] + i2 >= V) b = mid; else a = mid + 1;
+        if constexpr (!kExact) {
+          // r within h of the vertex, -zp h^2 - mu = the threshold: two bisections of
+          // the abscissae, whose bits are compared as integers (five of the
+          // exponent, at eight FP64 operations a step, were most of this kernel: 190
+          // -> 69 us for 6048 units)
+          const double zp = za + zb, mu = za * zb / zp * (dAC - dBC) * (dAC - dBC), q = (-J.lnAcc2 - mu) / zp;
+          const double h = sqrt(q > 0.0 ? q : 0.0), m = 1.0 / i1;
+          // first point with x >= b, or x > b
+          auto first = [&](double b, bool after) {
+            const long long key = ordered_bits(b) + (after ? 1 : 0);
+            int lo = 0, hi = J.largeOrder;
+            while (lo < hi) {
+              const int mid = (lo + hi) >> 1;
+              if (ordered_bits(J.xLarge[mid]) >= key) hi = mid; else lo = mid + 1;
+            }
+            return lo;
+          };
+          const int n0 = first((V - h - i2) * m, false), n1 = first((V + h - i2) * m, true),
+                    n2 = first(((dAC > dBC ? dAC : dBC) - i2) * m, true);
+          const int brk = q >= 0.0 && n1 > n2 ? n1 : n2;
+          win[k] = q >= 0.0 ? make_int4(brk < J.largeOrder ? brk : INT_MAX, n0, n1 - 1, 0)
+                            : make_int4(brk < J.largeOrder ? brk : INT_MAX, 1, 0, 0);
+        } else {
+          // (the stage tests every slot of the interval itself: a margin of 1)
+          const double thr = J.lnAcc2 - 1.0;
+          auto exq = [&](int n, double &r) {
+            r = i1 * J.xLarge[n] + i2;
+            const double d1 = dAC - r, d2 = dBC - r;
+            return -za * d1 * d1 - zb * d2 * d2;
+          };
+          double r;
+          int lo = 0, hi = J.largeOrder;
+          while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            const double e = exq(mid, r);
+            if (r > dAC && r > dBC && e < J.lnAcc2) hi = mid; else lo = mid + 1;
+          }
+          const int brk = lo < J.largeOrder ? lo : INT_MAX;
+          int a = 0, b = J.largeOrder;
+          while (a < b) {
+            const int mid = (a + b) >> 1;
+            if (i1 * J.xLarge[mid] + i2 >= V) b = mid; else a = mid + 1;
+          }
+          const int nv = a;
+          a = 0;
+          b = nv;
+          while (a < b) {
+            const int mid = (a + b) >> 1;
+            if (exq(mid, r) >= thr) b = mid; else a = mid + 1;
+          }
+          const int nLo = a;
+          a = nv;
+          b = J.largeOrder;
+          while (a < b) {
+            const int mid = (a + b) >> 1;
+            if (exq(mid, r) < thr) b = mid; else a = mid + 1;
+          }
+          win[k] = make_int4(brk, nLo, a - 1, 0);
         }
-        const int nv = a;
-        a = 0;
-        b = nv;
-        while (a < b) {
-          const int mid = (a + b) >> 1;
-          if (exq(mid, r) >= thr) b = mid; else a = mid + 1;
-        }
-        const int nLo = a;
-        a = nv;
-        b = J.largeOrder;
-        while (a < b) {
-          const int mid = (a + b) >> 1;
-          if (exq(mid, r) < thr) b = mid; else a = mid + 1;
-        }
-        win[k] = make_int4(brk, nLo, a - 1, 0);
       }
     }
     kinds |= (unsigned)kind << (2 * j);
