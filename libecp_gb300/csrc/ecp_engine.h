@@ -86,7 +86,7 @@ struct DevJob {
   // the level schedules' slot tables in global memory as well, for reads
   // whose index differs across a warp (the __constant__ copies serialise those)
   const int *s93, *s92;
-  const short *byN93;          // small-grid slots step by step in ascending point order
+  const int *byN93;            // small-grid slots (with point << 16) step by step in ascending point order
   // mixed path: tables as float pairs (ecp_ff.h)
   const ff *besHf, *besAf, *besZf;  // besH, besA, besZ
   const ff *xLf, *wLf;              // large grid abscissae and weights

@@ -79,8 +79,8 @@ static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem 
   for (int s0 = 0; s0 < O;) {
     const int s1 = step_end93(s0) < O ? step_end93(s0) : O, ns = s1 - s0;
     // the step's in-window slots are the run [lo, hi) of its by-point order
-    const int m0 = lane < ns ? __ldg(J.s93 + __ldg(J.byN93 + s0 + lane)) : INT_MAX;
-    const int m1 = lane + 32 < ns ? __ldg(J.s93 + __ldg(J.byN93 + s0 + lane + 32)) : INT_MAX;
+    const int m0 = lane < ns ? __ldg(J.byN93 + s0 + lane) >> 16 : INT_MAX;
+    const int m1 = lane + 32 < ns ? __ldg(J.byN93 + s0 + lane + 32) >> 16 : INT_MAX;
     const int lo = __popc(__ballot_sync(0xffffffffu, m0 < ws)) + __popc(__ballot_sync(0xffffffffu, m1 < ws));
     const int hi = __popc(__ballot_sync(0xffffffffu, m0 < we)) + __popc(__ballot_sync(0xffffffffu, m1 < we));
     const int nIn = hi - lo;
@@ -93,8 +93,8 @@ static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem 
     const int nLive = __popc(live);
 #pragma unroll 1
     for (int e = lane; e < nIn * nLive; e += 32) {
-      const int i = e / nLive, gg = __fns(live, 0, e - i * nLive + 1), t = __ldg(J.byN93 + s0 + lo + i),
-                n = __ldg(J.s93 + t);
+      const int i = e / nLive, gg = __fns(live, 0, e - i * nLive + 1), tn = __ldg(J.byN93 + s0 + lo + i),
+                t = tn & 0xffff, n = tn >> 16;
       // entry: K_l, then (C1 r^l) U, then the exponential
       double *ent = tab + ((t - s0) * G + gg) * TS, *WR = ent + lq;
       const double r = J.xSmall[n], s = sc[gg * 3], C1 = sc[gg * 3 + 1], ex = (sc[gg * 3 + 2] * r + s) * r, u = uL[n];

@@ -630,8 +630,8 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
     const int ns = s1 - s0;
     int lo, hi;
     {
-      const int n0 = lane < ns ? __ldg(J.s93 + __ldg(J.byN93 + s0 + lane)) : INT_MAX;
-      const int n1 = lane + 32 < ns ? __ldg(J.s93 + __ldg(J.byN93 + s0 + lane + 32)) : INT_MAX;
+      const int n0 = lane < ns ? __ldg(J.byN93 + s0 + lane) >> 16 : INT_MAX;
+      const int n1 = lane + 32 < ns ? __ldg(J.byN93 + s0 + lane + 32) >> 16 : INT_MAX;
       lo = __popc(__ballot_sync(0xffffffffu, n0 < ws)) + __popc(__ballot_sync(0xffffffffu, n1 < ws));
       hi = __popc(__ballot_sync(0xffffffffu, n0 < we)) + __popc(__ballot_sync(0xffffffffu, n1 < we));
     }
@@ -659,7 +659,7 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
 #pragma unroll 1
     for (int e = lane; e < nIn * nLive; e += 32) {
       const int i = slot_of(e);
-      const int gg = live_pair(e, i), t = __ldg(J.byN93 + s0 + lo + i), n = __ldg(J.s93 + t);
+      const int gg = live_pair(e, i), tn = __ldg(J.byN93 + s0 + lo + i), t = tn & 0xffff, n = tn >> 16;
       double *ent = tab + ((t - s0) * G + gg) * TS, *WR = ent + lq;
       const double s = sc[gg * 3], C1 = sc[gg * 3 + 1];
       if constexpr (kKind == kPairBand) {
@@ -737,6 +737,17 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
         cnt = 0;
       }
     } else {
+      // the step's slots inside the window, and those that count as points
+      u64 inw, counts;
+      {
+        const int t = s0 + lane, n = t < s1 ? __ldg(J.s93 + t) : 0, n32 = c93_slot[32];
+        inw = __ballot_sync(0xffffffffu, t < s1 && n >= ws && n < we);
+        counts = __ballot_sync(0xffffffffu, t < s1 && ((t & 1) ? n >= ws : n <= we));
+        if (s0 == 0) {  // the first step's 33rd slot
+          inw |= (u64)(n32 >= ws && n32 < we) << 32;
+          counts |= (u64)(n32 <= we) << 32;
+        }
+      }
       // runs of slots of one level, the lanes dealt to the running quadratures
       const unsigned act = __ballot_sync(0xffffffffu, !done);
       const LaneDeal D = deal_lanes(__popc(act));
@@ -751,22 +762,16 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
 #pragma unroll 1
       for (int t = s0; t < s1;) {
         const int te = lvEnd < s1 ? lvEnd : s1;
-        {  // points counted (t < te <= t + 33)
-          const int n = t + lane < te ? __ldg(J.s93 + t + lane) : 0;
-          const bool c = t + lane < te && (((t + lane) & 1) ? n >= ws : n <= we);
-          cnt += __popc(__ballot_sync(0xffffffffu, c));
-          if (te - t > 32) cnt += ((te - 1) & 1) ? c93_slot[te - 1] >= ws : c93_slot[te - 1] <= we;
-        }
+        const u64 bits = ((1ull << (te - s0)) - 1ull) & ~0ull << (t - s0);
+        cnt += __popcll(counts & bits);
         xf_run run;
 #pragma unroll 1
-        for (int x = t + D.part; x < te; x += D.P) {
-          const int n = __ldg(J.s93 + x);
+        for (int x = t + D.part; x < te; x += D.P)
           // the points inside the window (the entries outside it are zero)
-          if (work && n >= ws && n < we) {
+          if (work && (inw >> (x - s0) & 1u)) {
             const u64 *e = eT + (x - s0) * G * TS;
             t1_entry_add(run, e[oW], e[oK], *(const EntInfo *)(e + 2 * lq), q1);
           }
-        }
         xs sum = combine(run.sum(), D.P);
         sum = from_lane(sum, (mine_rank * D.P) & 31);
         lev = xs_plus(lev, sum);

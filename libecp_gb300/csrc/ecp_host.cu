@@ -233,23 +233,23 @@ struct DevTables {
   HostTables host;
   DBuf<float> besHf, besAf, besZf, xlf, wlf;  // float pairs (mixed path)
   DBuf<double> xs, ws, xl, wl, besT, besC, besH, besA, besZ, shNorm, p2s, fac, dfac, omega, c2s;
-  DBuf<int> ijk, ijkIdx, itemOff, itemCnt, items, s93, s92;
-  DBuf<short> byN93;
+  DBuf<int> ijk, ijkIdx, itemOff, itemCnt, items, s93, s92, byN93;
   DBuf<long long> besX, besXA;  // fixed-point Bessel rows
   DBuf<double> besD;            // derivative rows (plain path)
   int nItemsMax = 0, t2Rows = 0;
 };
 
 // The small-grid schedule's slots step by step (33, then 32 at a time) in
-// ascending order of their grid point (the batched kernel's type-1 steps).
-static std::vector<short> by_point_order(const std::vector<int> &slot) {
+// ascending order of their grid point (the unit kernels' type-1 steps), slot |
+// point << 16.
+static std::vector<int> by_point_order(const std::vector<int> &slot) {
   const int n = (int)slot.size();
-  std::vector<short> out(n);
+  std::vector<int> out(n);
   for (int s0 = 0; s0 < n;) {
     int s1 = s0 == 0 ? 33 : s0 + 32;
     if (s1 > n) s1 = n;
-    for (int t = s0; t < s1; t++) out[t] = (short)t;
-    std::sort(out.begin() + s0, out.begin() + s1, [&](short a, short b) { return slot[a] < slot[b]; });
+    for (int t = s0; t < s1; t++) out[t] = t | slot[t] << 16;
+    std::sort(out.begin() + s0, out.begin() + s1);
     s0 = s1;
   }
   return out;
