@@ -68,6 +68,7 @@ struct DevJob {
   const int *chanT0;           // per centre, the first term of channels l = 0..kMaxLEcp, then the end
                                // (terms sorted by l; null: none)
   const double *termN, *termD, *termA;
+  const struct FxTerm *termFx;   // the terms in integer form (batched path)
   const int *pairA, *pairB;
   const int *pairShift;        // derivative shift index of each pair entry (null: none)
   int deriv, nRuns;            // derivative order; F-table runs (1 + order; 0 reads as 1)

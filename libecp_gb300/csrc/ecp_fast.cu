@@ -89,29 +89,6 @@ static __device__ __noinline__ xf bessel_me(const DevJob &J, int lmax, xf z100, 
 // Powers of r other than 0, 1, 2: rare, out of line.
 static __device__ __noinline__ double rpow_rare(double r, double n) { return rpow(r, n); }
 
-// Adds one ECP term d r^n exp(-a r^2) (R2 = r^2) to a channel's sum.  A term
-// below 2^-70 of what the sum holds is left out (the sum carries 60 bits), and
-// one whose exponential underflows.
-static __device__ inline void ecp_term_fx(const DevJob &J, int t, double r, xf R, xf R2, xf_sum &acc) {
-  const xf a = xf_mul(xf_from(__ldg(J.termA + t)), R2);
-  const double d = __ldg(J.termD + t);
-  const xf D = xf_from(d);
-  // n by its bits (a comparison of doubles is an FP64-pipe instruction)
-  const u64 nb = (u64)dbits(__ldg(J.termN + t));
-  const int n = nb == 0 ? 0 : nb == 0x3ff0000000000000ull ? 1 : nb == 0x4000000000000000ull ? 2 : 3;
-  const int sh = a.e + 53;  // a r^2 in Q53
-  const u64 E = sh < 0 ? shr64(a.m, -sh) : (a.m >> (63 - (sh > 63 ? 63 : sh)) ? ~0ull : a.m << sh);
-  if (E > (u64)(700ll << 53)) return;
-  // 2^b above the term, b = log2 |d| + log2 r^n - a r^2 log2 e rounded up
-  // (n <= 2; r^n otherwise unknown: never left out)
-  const int rn = n == 0 ? 0 : n == 1 ? R.e + 64 : n == 2 ? R2.e + 64 : 100000;
-  const int b = D.e + 64 + rn - (int)(((u64)(uint32_t)(E >> 32) * 1477) >> 31);
-  if (b < acc.v.e + (63 - clz64((u64)(acc.v.m < 0 ? -acc.v.m : acc.v.m) | 1u)) - 70) return;
-  xf v = xf_mul(fx_exp(-(i64)E), D);
-  if (n) v = xf_mul(v, n == 1 ? R : n == 2 ? R2 : xf_from(rpow_rare(r, bits_d((i64)nb))));
-  acc.add(v, sign_of(d));
-}
-
 // One row K_l(z), by the same branches as bessel_fx.
 static __device__ __noinline__ double bessel_row(const DevJob &J, int l, double z) {
   if (__builtin_expect(z < 1.0E-7, 0)) {  // rare: laid out of line
@@ -144,15 +121,32 @@ static __device__ __noinline__ double bessel_row(const DevJob &J, int l, double 
 }
 
 // U_l(r) of centre c (src/ecp.c:42-60): its terms of channel l, summed with
-// 60-bit mantissas; normalised, with its sign.
+// 60-bit mantissas; normalised, with its sign.  A term below 2^-70 of the
+// largest one before it is left out, and one whose exponential underflows.
 static __device__ __noinline__ xf channel(const DevJob &J, int c, int l, double r, uint32_t &sign) {
   const xf R = xf_from(r), R2 = norm1(xf_mul(R, R));
-  xf_sum acc;
+  xs acc;
+  int top = -100000;  // every term so far is below 2^top
   const int *ch = J.chanT0 + c * (kMaxLEcp + 2) + l, t1 = ch[1];
 #pragma unroll 1
-  for (int t = ch[0]; t < t1; t++) ecp_term_fx(J, t, r, R, R2, acc);
-  sign = acc.v.m < 0 ? 0x80000000u : 0u;
-  return xs_abs(acc.v);
+  for (int t = ch[0]; t < t1; t++) {
+    const FxTerm T = J.termFx[t];
+    const xf a = xf_mul({T.am, T.ae}, R2);
+    const u64 E = shr64(a.m, -(a.e + 53));  // a r^2 in Q53
+    if (a.e + 53 > 0 || E > (u64)(700ll << 53)) continue;
+    // 2^b above the term, b = log2 |d| + log2 r^n - a r^2 log2 e rounded up
+    // (n <= 2; r^n otherwise unknown: never left out)
+    const xf Rn = T.n == 1 ? R : R2;
+    const int b = T.de + 64 - (int)(((u64)(uint32_t)(E >> 32) * 1477) >> 31) + (T.n == 0 ? 0 : T.n < 3 ? Rn.e + 64 : 100000);
+    if (b < top - 70) continue;
+    xf v = xf_mul(fx_exp(-(i64)E), {T.dm, T.de});
+    if (T.n) v = xf_mul(v, T.n < 3 ? Rn : xf_from(rpow_rare(r, J.termN[t])));
+    top = v.e + 64 > top ? v.e + 64 : top;
+    const i64 m = (i64)(v.m >> 4), s = (i64)(int)T.sign >> 31;
+    acc = xs_add(acc, {(m ^ s) - s, v.e + 4});
+  }
+  sign = acc.m < 0 ? 0x80000000u : 0u;
+  return xs_abs(acc);
 }
 
 // ------------------------------------------- double-single (mixed path)
@@ -974,8 +968,8 @@ __global__ void __launch_bounds__(32, 20) k_unit_small(DevJob J) {
 template <bool kMixed>
 static __device__ void t1_large(const DevJob &J, const Unit &U, const LargeSmem &Ls, double *sm, const LevelTab &V,
                                 int kk, bool ffp, unsigned mask, double s) {
-  double *tab = sm + Ls.tab;
-  int *quad = (int *)(sm + Ls.fail);  // the running quadratures, by rank
+  double *tab = sm + Ls.tab + (threadIdx.x >> 5) * Ls.tabT1;
+  int *quad = (int *)(sm + Ls.fail) + (threadIdx.x >> 5) * 32;  // the running quadratures, by rank
   const int lane = threadIdx.x & 31, lab = U.lab, lq = lab + 1, O = kSmallOrder, OL = J.largeOrder, TSf = 3 + 2 * lq;
   const int Nb = U.Nb, ws = U.ws, we = U.we, c = U.c, Lc = U.Lc;
   const double *uL = J.uL + (size_t)c * O;
@@ -1161,10 +1155,43 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, const LargeSmem 
   __syncwarp();
 }
 
-// One primitive pair of the type-2 large-grid fallback, by one warp
-// (src/type2.c:418-528): integrates the pass's failed items (decoded in
+template <int kWarps>
+static __device__ inline void cta_sync() {
+  if constexpr (kWarps > 1) __syncthreads();
+  else __syncwarp();
+}
+
+// Whose tables a slot past a pair's break reads: the last earlier pair whose loop
+// reached the point n (-1: none, or it broke off there), and its bra primitive.
+struct StalePair {
+  int owner, i;
+};
+static __device__ __noinline__ StalePair stale_pair(const int4 *win, int k, int n, int Nb) {
+#pragma unroll 1
+  for (int j = k - 1; j >= 0; j--)
+    if (win[j].x >= n) return {win[j].x == n ? -1 : j, j / Nb};
+  return {-1, 0};
+}
+
+// -(za (dA - r)^2 + zb (dB - r)^2) in Q53, saturating.
+static __device__ __noinline__ i64 t2_exponent(double za, double zb, double dA, double dB, double r) {
+  u64 E = 0;
+#pragma unroll 1
+  for (int side = 0; side < 2; side++) E += fx_gauss(side ? zb : za, (side ? dB : dA) - r);
+  return -(i64)E;
+}
+// 100 times the Bessel argument 2 zeta d r without its r.
+static __device__ __noinline__ xf t2_argument(double zeta, double d) {
+  const xf z = xf_mul(xf_from(zeta), xf_from(d));
+  return xf_times100({z.m, z.e + 1});
+}
+
+// One primitive pair of the type-2 large-grid fallback, by the CTA's one or two
+// warps (src/type2.c:418-528): integrates the pass's failed items (decoded in
 // `fail`) and adds each result to the partial sums.  mb: the latest break of
-// the earlier pairs, beyond which no earlier pair's buffers are reused.
+// the earlier pairs, beyond which no earlier pair's buffers are reused.  Two
+// warps share the tables (one the Bessel rows, the other the potential and the
+// powers) and halve the items; each keeps the queue of slots for itself.
 constexpr short kNoExp = -32000;  // the exponent of a sum without terms
 static __device__ inline short exp16(int e) { return (short)(e < kNoExp ? kNoExp : e); }
 struct T2Pass {
@@ -1172,13 +1199,13 @@ struct T2Pass {
   unsigned mask;     // channels they read
   int l1, l2, l3;    // highest Ka, Kb and r^l rows
 };
-template <bool kMixed>
+template <bool kMixed, int kWarps>
 static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &L, double *sm, const LevelTab &V,
                                const T2Pass &S0, int k, int mb, const double2 *map, const int4 *win, bool useFF, int &warn) {
   // mixed path: useFF picks the double-single tables and sums for this pass
   // (one copy of the common code for both precisions)
   const bool inFF = kMixed && useFF;
-  const int lane = threadIdx.x & 31, nA = 2 * J.maxLBS + 1, Nb = U.Nb, c = U.c, nf = S0.nf;
+  const int lane = threadIdx.x & 31, warp = kWarps > 1 ? threadIdx.x >> 5 : 0, nA = 2 * J.maxLBS + 1, Nb = U.Nb, c = U.c, nf = S0.nf;
   const int LE = J.maxLECP > 0 ? J.maxLECP : 1, LBE = J.maxLBS + LE, OL = J.largeOrder;
   const int TS = L.tabStride, ES = L.expStride;
   const double *pzA = U.pzA, *pzB = U.pzB;
@@ -1189,19 +1216,23 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
   i64 *s0m = (i64 *)(sm + L.I), *s1m = (i64 *)(sm + L.P), *s2m = (i64 *)(sm + L.Q);
   short4 *sE = (short4 *)(sm + L.E);
   const int *fail = (const int *)(sm + L.fail);
-  unsigned char *act = (unsigned char *)(sm + L.act);  // the running items
-  int *pend = (int *)(sm + L.pend);
+  unsigned char *act = (unsigned char *)(sm + L.act) + warp * (kWalkCap / 2);  // the warp's running items
+  int *pend = (int *)(sm + L.pend) + warp * 64;
+  int *red = (int *)(sm + L.red);
+  (void)red;
   const double za = pzA[k / Nb], ca = U.pcA[k / Nb], zb = pzB[k % Nb], cb = U.pcB[k % Nb];
   // derivative blocks: the product times zeta_a^max(0, shifta), then
   // zeta_b^max(0, shiftb) (src/type2.c:456-462)
   const double Ck = zeta_times(zeta_times(ca * cb, za, U.pa0), zb, U.pb0);
   const double i1 = map[k].x;
+  const double iCk = i1 * Ck;
   const ff i1f = ff_from_double(i1), Ckf = ff_from_double(Ck);
   const int4 wk = win[k];
   const int nb = wk.x, nLo = wk.y, nHi = wk.z;
 #pragma unroll 1
-  for (int q = lane; q < nf; q += 32) {
-    act[q] = (unsigned char)q;
+  for (int i = lane; i * kWarps + warp < nf; i += 32) {
+    const int q = i * kWarps + warp;
+    act[i] = (unsigned char)q;
     s0m[q] = s1m[q] = s2m[q] = 0;  // (also 0.0)
     sE[q] = make_short4(kNoExp, kNoExp, kNoExp, 0);
   }
@@ -1209,30 +1240,29 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
   // Whose tables slot t reads (the reference's reused buffers): this pair's
   // below its break; beyond it, on the lower half, the last earlier pair
   // whose loop reached that point; and the point, exponent of that pair.
-  auto locate = [&](int t, int &owner, double &r, i64 &E) {
+  auto locate = [&](int t, int &owner, double &r, double &zaj, double &zbj) {
     const int n = __ldg(J.s92 + t);
     const bool upper = t > 0 && ((t - 1) & 1);
-    owner = -1;
-    if (n < nb) owner = k;
-    else if (__builtin_expect(n != nb && !upper, 0)) {
-#pragma unroll 1
-      for (int j = k - 1; j >= 0; j--)
-        if (win[j].x >= n) { owner = j; break; }
-      if (owner >= 0 && win[owner].x == n) owner = -1;
+    owner = k;
+    zaj = za;
+    zbj = zb;
+    if (__builtin_expect(n >= nb, 0)) {
+      const StalePair p = n != nb && !upper ? stale_pair(win, k, n, Nb) : StalePair{-1, 0};
+      owner = p.owner;
+      if (owner < 0) return;
+      zaj = pzA[p.i];
+      zbj = pzB[owner - p.i * Nb];
     }
-    if (owner < 0) return;
-    const double zaj = owner == k ? za : pzA[owner / Nb], zbj = owner == k ? zb : pzB[owner % Nb];
     r = map[owner].x * J.xLarge[n] + map[owner].y;
-    // za (dAC - r)^2 + zb (dBC - r)^2 in Q53, saturating
-    E = -(i64)(fx_gauss(zaj, dAC - r) + fx_gauss(zbj, dBC - r));
   };
+  auto exponent = [&](double zaj, double zbj, double r) { return t2_exponent(zaj, zbj, dAC, dBC, r); };
   const i64 thr = fx_q53(J.lnAcc2);
   // A slot needs its tables only where they are not negligible; the others
   // integrate to exactly zero.  Slots are classified step by step (cheap),
   // the needed ones queued, and each pass evaluates 32 queued slots, one per
   // lane, before the quadratures walk every slot up to the first one still
   // queued.
-  int cpos = 0, wpos = 0, nPend = 0, nAct = nf;
+  int cpos = 0, wpos = 0, nPend = 0, nAct = (nf + kWarps - 1 - warp) / kWarps;
   // channels and rows the quadratures still running read (the pass's to
   // begin with, narrowed after every walk)
   unsigned pMask = S0.mask;
@@ -1249,10 +1279,9 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
           need = n >= nLo && n <= nHi;
         } else if (n <= mb && n != nb && !(t > 0 && ((t - 1) & 1))) {
           int owner;
-          double r;
-          i64 E;
-          locate(t, owner, r, E);
-          need = owner >= 0 && E >= thr;
+          double r, zaj, zbj;
+          locate(t, owner, r, zaj, zbj);
+          need = owner >= 0 && exponent(zaj, zbj, r) >= thr;
         }
       }
       const unsigned m = __ballot_sync(0xffffffffu, need);
@@ -1266,43 +1295,59 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
     if (lane < nE) {
       const int t = pend[lane], n = __ldg(J.s92 + t);
       int owner;
-      double r;
-      i64 E;
-      locate(t, owner, r, E);
-      // the pair's own exponents (no integer divide) unless a stale slot
-      const double zaj = owner == k ? za : pzA[owner / Nb], zbj = owner == k ? zb : pzB[owner % Nb];
+      double r, zaj, zbj;
+      locate(t, owner, r, zaj, zbj);
       double *e = tab + lane * TS;
-      if (inFF) {
-        // the same rows in double-single
-        ff *Uc = (ff *)e, *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
-        const ff rf = ff_from_double(r);
-        const ff wB = ff_mul(ff_mul(J.wLf[n], i1f), ff_mul(Ckf, ff_exp(ff_from_double((double)E * 0x1p-53))));
-        channels_ff(J, c, rf, pMask, Uc);
+      xf f = {1ull << 63, -63};  // the Bessel rows' common factors (large arguments)
+      // the Bessel rows of both centres, then the rest: a warp each, or both by one
 #pragma unroll 1
-        for (int side = 0; side < 2; side++)
-          bessel_ff(J, side ? pL2 : pL1, ff_mul(ff_from_double(side ? 2.0 * zbj * dBC : 2.0 * zaj * dAC), rf),
-                    side ? Kb : Ka, 1);
+      for (int role = warp; role < 2; role += kWarps) {
+        if (inFF) {
+          // the same rows in double-single
+          ff *Uc = (ff *)e, *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
+          const ff rf = ff_from_double(r);
+          if (role == 0) {
 #pragma unroll 1
-        for (int l = 0; l <= pL1; l++) Ka[l] = ff_mul(Ka[l], wB);
-        R[0] = {1.0f, 0.0f};
+            for (int side = 0; side < 2; side++)
+              bessel_ff(J, side ? pL2 : pL1, ff_mul(ff_from_double(side ? 2.0 * zbj * dBC : 2.0 * zaj * dAC), rf),
+                        side ? Kb : Ka, 1);
+          } else {
+            const ff wB = ff_mul(ff_mul(J.wLf[n], i1f),
+                                 ff_mul(Ckf, ff_exp(ff_from_double((double)exponent(zaj, zbj, r) * 0x1p-53))));
+            channels_ff(J, c, rf, pMask, Uc);
 #pragma unroll 1
-        for (int l = 1; l <= pL3; l++) R[l] = ff_mul(rf, R[l - 1]);
-      } else {
+            for (unsigned m = pMask; m; m &= m - 1u) Uc[__ffs(m) - 1] = ff_mul(Uc[__ffs(m) - 1], wB);
+            R[0] = {1.0f, 0.0f};
+#pragma unroll 1
+            for (int l = 1; l <= pL3; l++) R[l] = ff_mul(rf, R[l - 1]);
+          }
+          continue;
+        }
         // mantissas of w Ck e^ex U_l, r^l, K_l1 and K_l2, the
         // exponents in 16 bits, U's with its sign
         u64 *Um = (u64 *)e, *R = Um + LE, *Ka = R + nA, *Kb = Ka + LBE;
         short *Ue = (short *)(tab + 32 * TS) + lane * ES, *Ae = Ue + LE, *Be = Ae + LBE, *Re = Be + LBE;
-        const double w = J.wLarge[n];
         const xf Rx = xf_from(r);
-        xf wB = xf_mul(fx_exp(E), xf_mul(xf_mul(xf_from(w), xf_from(i1)), xf_from(Ck)));
-        // the rows of both centres through one copy of the Bessel code
+        if (role == 0) {
+          // through one copy of the Bessel code
 #pragma unroll 1
-        for (int side = 0; side < 2; side++) {
-          const xf f = xf_mul(xf_from(side ? zbj : zaj), xf_from(side ? dBC : dAC));  // times 2: exponent + 1
-          const xf c = bessel_me(J, side ? pL2 : pL1, xf_mul(xf_times100({f.m, f.e + 1}), Rx), side ? Kb : Ka,
-                                 side ? Be : Ae);
-          wB = norm1(xf_mul(wB, c));
+          for (int side = 0; side < 2; side++) {
+            const xf z = t2_argument(side ? zbj : zaj, side ? dBC : dAC);
+            f = norm1(xf_mul(f, bessel_me(J, side ? pL2 : pL1, xf_mul(z, Rx), side ? Kb : Ka, side ? Be : Ae)));
+          }
+          if constexpr (kWarps > 1) {  // the other warp has the potential
+#pragma unroll 1
+            for (int l = 0; l <= pL2; l++) {
+              const xf v = norm1(xf_mul({Kb[l], Be[l]}, f));
+              Kb[l] = v.m;
+              Be[l] = (short)v.e;
+            }
+          }
+          continue;
         }
+        const double w = J.wLarge[n] * iCk;
+        xf wB = xf_mul(fx_exp(exponent(zaj, zbj, r)), xf_from(w));
+        if constexpr (kWarps == 1) wB = xf_mul(norm1(wB), f);
         wB = xf_norm(wB);
         // only the channels and rows this pass's quadratures read
 #pragma unroll 1
@@ -1310,7 +1355,7 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
           const int l = __ffs(m) - 1;
           uint32_t sign;
           const xf u = norm1(xf_mul(channel(J, c, l, r, sign), wB));
-          sign ^= sign_of(w) ^ sign_of(Ck);
+          sign ^= sign_of(w);
           Um[l] = u.m;
           Ue[l] = (short)((u.m && u.e > -16000 ? u.e * 2 : -32000) + (int)(sign >> 31));
         }
@@ -1326,7 +1371,7 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
       }
     }
     const int myPend = lane < nE ? pend[lane] : INT_MAX;
-    __syncwarp();
+    cta_sync<kWarps>();
     unsigned nMask = 0u;
     int n1 = 0, n2 = 0, n3 = 0, left = 0;
     // the running items, 32 at a time, the last ones by several lanes each
@@ -1419,6 +1464,16 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
     pL1 = __reduce_max_sync(0xffffffffu, n1);
     pL2 = __reduce_max_sync(0xffffffffu, n2);
     pL3 = __reduce_max_sync(0xffffffffu, n3);
+    // both warps' channels (the low byte) and rows, and the end of their walks
+    if constexpr (kWarps > 1) {
+      if (lane == 0) red[warp] = (int)(pMask | (unsigned)pL1 << 8 | (unsigned)pL2 << 16 | (unsigned)pL3 << 24);
+      cta_sync<kWarps>();
+      const unsigned o = (unsigned)red[warp ^ 1];
+      pMask |= o & 255u;
+      pL1 = pL1 > (int)(o >> 8 & 255u) ? pL1 : (int)(o >> 8 & 255u);
+      pL2 = pL2 > (int)(o >> 16 & 255u) ? pL2 : (int)(o >> 16 & 255u);
+      pL3 = pL3 > (int)(o >> 24) ? pL3 : (int)(o >> 24);
+    }
     // drop the evaluated slots from the queue
     const int rest = nPend - nE;
     const int keep0 = lane < rest ? pend[nE + lane] : 0, keep1 = lane + 32 < rest ? pend[nE + lane + 32] : 0;
@@ -1428,7 +1483,7 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
     nPend = rest;
     wpos = b;
     __syncwarp();
-    if (nAct == 0) break;
+    if (pMask == 0u) break;  // no quadrature running
   }
   // out of levels: the full-grid estimate stands and the unit is flagged
 #pragma unroll 1
@@ -1447,7 +1502,7 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
 
 // The failed type-2 quadratures of a unit over the primitive pairs of one part
 // (src/type2.c:418-528), in passes of up to kWalkCap of them.
-template <bool kMixed>
+template <bool kMixed, int kWarps>
 static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem &L, double *sm, const LevelTab &V,
                                 int part) {
   const int lane = threadIdx.x & 31, nIt = U.nItems, LE = J.maxLECP > 0 ? J.maxLECP : 1;
@@ -1483,7 +1538,7 @@ static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem 
       if (nf + __popc(m) > kWalkCap) break;
       if (m >> lane & 1u) {
         const int v = unit_item(J, U, q0 + lane);
-        fail[nf + __popc(m & ((1u << lane) - 1u))] = v;
+        if (threadIdx.x < 32) fail[nf + __popc(m & ((1u << lane) - 1u))] = v;
         pMask |= 1u << (v & 255);
         m1 = m1 > ((v >> 8) & 255) ? m1 : (v >> 8) & 255;
         m2 = m2 > ((v >> 16) & 255) ? m2 : (v >> 16) & 255;
@@ -1499,48 +1554,62 @@ static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem 
     S.l2 = __reduce_max_sync(0xffffffffu, m2);
     S.l3 = __reduce_max_sync(0xffffffffu, m3);
 #pragma unroll 1
-    for (int q = lane; q < nf; q += 32) sum[q] = 0.0;
-    __syncwarp();
+    for (int q = threadIdx.x; q < nf; q += blockDim.x) sum[q] = 0.0;
+    cta_sync<kWarps>();
     int mb = mb0, warn = 0;
 #pragma unroll 1
     for (int k = k0; k < k1; k++) {
-      t2_pair<kMixed>(J, U, L, sm, V, S, k, mb, map, win, useFF, warn);
+      t2_pair<kMixed, kWarps>(J, U, L, sm, V, S, k, mb, map, win, useFF, warn);
       mb = win[k].x > mb ? win[k].x : mb;
     }
     if (warn) atomicOr(&((UnitHead *)U.scr)->warn, 2);
+    cta_sync<kWarps>();
     int at = 0;
 #pragma unroll 1
     for (int w = first; w < q0; w += 32) {
       const unsigned m = mask[w >> 5];
-      if (m >> lane & 1u) dst[w + lane] = sum[at + __popc(m & ((1u << lane) - 1u))];
+      if (threadIdx.x < 32 && (m >> lane & 1u)) dst[w + lane] = sum[at + __popc(m & ((1u << lane) - 1u))];
       at += __popc(m);
     }
-    __syncwarp();
+    cta_sync<kWarps>();
   }
 }
 
-// One warp a CTA; the type-2 parts first (the longer ones), then the failed
-// type-1 pairs.
-template <bool kMixed>
-__global__ void __launch_bounds__(32, 16) k_unit_large(DevJob J) {
+// The type-2 parts first (the longer ones), one at a time by the whole CTA, then
+// the failed type-1 pairs, one a warp.
+template <bool kMixed, int kWarps>
+__global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) k_unit_large(DevJob J) {
   extern __shared__ double sm[];
   __shared__ LevelTab V;
+  __shared__ int drawn;
+  (void)drawn;
   level_tab(V, c92_3N, c92_nLevels, J.tol);
   const LargeSmem L = large_layout(J.maxLBS, J.maxLECP, false);
   const int n2 = (int)J.counters[kCntPart], n = n2 + (int)J.counters[kCntFail];
+  int i = n2, taken = 0;
 #pragma unroll 1
-  for (int taken = 0; taken < J.take; taken++) {
-    const int i = next_item(J.counters + kHeadLarge);
-    if (i >= n) return;
-    if (i < n2) {
-      const int2 it = J.listPart[i];
-      const Unit U = unit_load(J, it.x);
-      t2_large<kMixed>(J, U, L, sm, V, it.y);
+  for (; taken < J.take; taken++) {
+    if constexpr (kWarps > 1) {
+      if (threadIdx.x == 0) drawn = (int)atomicAdd(J.counters + kHeadLarge, 1u);
+      __syncthreads();
+      i = drawn;
+      __syncthreads();
     } else {
-      const T1Fail it = J.listFail[i - n2];
-      const Unit U = unit_load(J, it.pos);
-      t1_large<kMixed>(J, U, L, sm, V, it.k & 0xffff, it.k >> 16, it.mask, it.s);
+      i = next_item(J.counters + kHeadLarge);
     }
+    if (i >= n2) break;
+    const int2 it = J.listPart[i];
+    const Unit U = unit_load(J, it.x);
+    t2_large<kMixed, kWarps>(J, U, L, sm, V, it.y);
+  }
+#pragma unroll 1
+  for (; taken < J.take; taken++, i = n) {
+    // (the first warp goes on with the entry drawn above)
+    if (i >= n || threadIdx.x >= 32) i = next_item(J.counters + kHeadLarge);
+    if (i >= n) return;
+    const T1Fail it = J.listFail[i - n2];
+    const Unit U = unit_load(J, it.pos);
+    t1_large<kMixed>(J, U, L, sm, V, it.k & 0xffff, it.k >> 16, it.mask, it.s);
   }
 }
 
@@ -1753,7 +1822,8 @@ void fast_prepare() {
   if (dev < 0 || dev >= 64 || attr[dev]) return;
 #pragma unroll 1
   for (const void *k : {(const void *)k_unit_small<false>, (const void *)k_unit_small<true>,
-                        (const void *)k_unit_large<false>, (const void *)k_unit_large<true>,
+                        (const void *)k_unit_large<false, 1>, (const void *)k_unit_large<true, 1>,
+                        (const void *)k_unit_large<false, 2>, (const void *)k_unit_large<true, 2>,
                         (const void *)k_unit_link}) {
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     // most of the unified L1/shared array as shared memory
@@ -1806,8 +1876,9 @@ int launch_fast_pipeline(const DevJob &J, cudaStream_t st, const FastConfig &cfg
     if (cfg.mixed) k_unit_small<true><<<gSmall, 32, sSmall, st>>>(K);
     else k_unit_small<false><<<gSmall, 32, sSmall, st>>>(K);
     K.take = takeLarge;
-    if (cfg.mixed) k_unit_large<true><<<gLarge, 32, sLarge, st>>>(K);
-    else k_unit_large<false><<<gLarge, 32, sLarge, st>>>(K);
+    const int nw = J.few ? 2 : 1;
+    (cfg.mixed ? nw > 1 ? k_unit_large<true, 2> : k_unit_large<true, 1>
+               : nw > 1 ? k_unit_large<false, 2> : k_unit_large<false, 1>)<<<gLarge, 32 * nw, sLarge, st>>>(K);
     k_unit_link<<<units, link_threads(sLink), sLink, st>>>(K);
   });
   if (u1) record_timing(u1, st);

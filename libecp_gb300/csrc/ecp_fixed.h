@@ -264,9 +264,8 @@ ECPGB_HD i64 fx_q53(double x) {
 // z d^2 in Q53 (z > 0), saturating at 2^62.
 ECPGB_HD u64 fx_gauss(double z, double d) {
   const xf D = xf_from(d), v = xf_mul(xf_from(z), xf_mul(D, D));
-  const int sh = v.e + 53;
-  const u64 E = sh <= 0 ? shr64(v.m, -sh) : (v.m >> (63 - (sh > 63 ? 63 : sh)) ? ~0ull : v.m << sh);
-  return E < 1ull << 62 ? E : 1ull << 62;
+  const u64 E = shr64(v.m, -(v.e + 53));  // v.m >= 2^61 or 0
+  return v.e + 53 <= 0 && E < 1ull << 62 ? E : 1ull << 62;
 }
 
 // A signed number m * 2^e, |m| < 2^62: the running values of a quadrature.
@@ -321,13 +320,17 @@ struct xf_run {
   ECPGB_HD xs sum() const { return xs_fit({m, e}); }
 };
 
-// A signed sum of any number of terms (the ECP channels).
-struct xf_sum {
-  xs v;
-  ECPGB_HD void add(xf t, uint32_t sign) {
-    const i64 tm = (i64)(t.m >> 4);
-    v = xs_add(v, {sign ? -tm : tm, t.e + 4});
-  }
+// An ECP term d r^n exp(-a r^2), laid out by the host: normalised mantissas and
+// exponents of a and d, d's sign in the top bit, n (3: any other power).
+struct FxTerm {
+  u64 am, dm;
+  int ae, de;
+  uint32_t sign;
+  int n;
 };
+inline FxTerm fx_term(double a, double d, double n) {
+  const xf A = xf_from(a), D = xf_from(d);
+  return {A.m, D.m, A.e, D.e, sign_of(d), n == 0 ? 0 : n == 1 ? 1 : n == 2 ? 2 : 3};
+}
 
 }  // namespace ecpgb

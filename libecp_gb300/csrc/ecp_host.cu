@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "ecp_engine.h"
+#include "ecp_fixed.h"
 #include "ecp_host.h"
 #include "ecp_tables.h"
 
@@ -632,7 +633,7 @@ size_t job_device_bytes(const Parsed &P, int mode, size_t budget, size_t *scratc
   const size_t angLam = P.maxLECP + LB + 1, angC = (LB + 1) * (LB + 2) * (LB + 3) / 6;
   size_t in = 8 * (P.geom.size() + P.primA.size() + P.primD.size() + 3 * P.termL.size() + P.pairOff.size()) +
               4 * (5 * P.shL.size() + P.atomMaxL.size() + 4 * P.ctrAtom.size() + P.termL.size() + 3 * P.pairA.size()) +
-              36 * (P.nPairs + 1) + 8 * nc + 4 * P.chanT0.size() + (mode == ECPGB_MIXED ? 16 * P.termL.size() : 0) +
+              36 * (P.nPairs + 1) + 8 * nc + 4 * P.chanT0.size() + (32 + (mode == ECPGB_MIXED ? 16 : 0)) * P.termL.size() +
               32 * 256;
   size_t work = 8 * (ns + nc * O * LE * nk + nc * O + nc * ns * (1 + P.deriv) * O * nF + nc * na * 4 + nc * na * D * D * D +
                      nc * na * angLam * LE * LE * angC + nc * (size_t)P.centreStride + (size_t)P.dim * P.dim) +
@@ -690,6 +691,9 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   make_plan(P, scratchCap, J.single, B.plan, orders, offs, chunkPairs, ctr);
   size_t iOrd = add(orders.data(), 4 * orders.size()), iOff = add(offs.data(), 8 * offs.size()),
          iChk = add(chunkPairs.data(), 4 * chunkPairs.size()), iCtr = add(ctr.data(), 4 * ctr.size());
+  std::vector<FxTerm> terms;
+  for (size_t t = 0; t < P.termL.size() && !J.plain; t++) terms.push_back(fx_term(P.termA[t], P.termD[t], P.termN[t]));
+  size_t iFx = add(terms.data(), sizeof(FxTerm) * terms.size());
   const std::vector<unsigned> zeros(P.nCentres);
   size_t iTk = add(zeros.data(), 4 * zeros.size());
   // the ECP terms' exponents and coefficients as float pairs (mixed path)
@@ -718,6 +722,7 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.pairShift = (const int *)dp(iPS);
   J.chanT0 = (const int *)dp(iCh);
   J.tickets = (unsigned *)dp(iTk);
+  J.termFx = (const FxTerm *)dp(iFx);
   J.termAf = mode == ECPGB_MIXED ? (const ff *)dp(iTAf) : nullptr;
   J.termDf = mode == ECPGB_MIXED ? (const ff *)dp(iTDf) : nullptr;
   J.deriv = P.deriv;

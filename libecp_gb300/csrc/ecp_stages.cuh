@@ -16,7 +16,8 @@
 
 namespace ecpgb {
 
-constexpr int kWalkCap = 128;  // large-grid quadratures per warp and pass
+constexpr int kWalkCap = 128;  // large-grid quadratures per pass
+constexpr int kLargeWarps = 2; // most warps a CTA of the batched large-grid stage
 constexpr int kLargeWords = (kMaxLargeOrder + 1) / 32;  // bitmap words over the large grid (128, even)
 static_assert(kLargeWords * 32 >= kMaxLargeOrder && kLargeWords % 2 == 0, "large-grid bitmap size");
 
@@ -203,7 +204,7 @@ __host__ __device__ inline SmallSmem small_layout(int LB, int rows, int cap) {
 // the weight), the walkers' state, the needed-slot bitmap
 // with word prefixes, the pending slots and the failed items.
 struct LargeSmem {
-  int tab, I, P, Q, E, part, act, bits, pend, pref, fail, total, tabStride, expStride;
+  int tab, tabT1, I, P, Q, E, part, act, bits, pend, pref, fail, red, total, tabStride, expStride;
 };
 __host__ __device__ inline LargeSmem large_layout(int LB, int LE, bool exact) {
   LargeSmem s{};
@@ -211,20 +212,22 @@ __host__ __device__ inline LargeSmem large_layout(int LB, int LE, bool exact) {
   s.tabStride = (nE + nA + 2 * LBE + (exact ? 2 : 0)) | 1;  // odd: conflict-free lane strides
   // 16-bit exponents of U, Ka, Kb and r^l (batched path): an odd number of words a lane
   s.expStride = 2 * (((nE + 2 * LBE + nA + 1) / 2) | 1);
-  int o = 32 * s.tabStride + (exact ? 0 : 8 * s.expStride), t1 = 32 * (2 * nA + 3);
+  s.tabT1 = 32 * (2 * nA + 3);  // type-1 table of one warp
+  int o = 32 * s.tabStride + (exact ? 0 : 8 * s.expStride), t1 = (exact ? 1 : kLargeWarps) * s.tabT1;
   s.tab = 0;
   if (t1 > o) o = t1;
   s.I = o; o += kWalkCap;
   s.P = o; o += kWalkCap;
   s.Q = o; o += kWalkCap;
   s.part = o; o += kWalkCap;
-  s.pend = o; o += 32;
+  s.pend = o; o += 32 * (exact ? 1 : kLargeWarps);
   if (exact) {  // needed-slot bitmap and word prefixes
     s.bits = o; o += kLargeWords / 2;
     s.pref = o; o += kLargeWords / 2;
   } else {  // exponents and list of the running items
     s.E = o; o += kWalkCap;
     s.act = o; o += kWalkCap / 8;
+    s.red = o; o += 2 * kLargeWarps;
   }
   s.fail = o; o += kWalkCap / 2;
   s.total = o;
