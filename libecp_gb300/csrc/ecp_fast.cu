@@ -864,12 +864,19 @@ static __device__ void t2_small(const DevJob &J, const Unit &U, const LevelTab &
         const double *src = g == 0 ? Fa + (size_t)m * nF : g == 1 ? Fb + (size_t)m * nF : Ut + ((size_t)m * LE + g - 2) * nk;
         const int cntR = g == 0 ? nA : g == 1 ? nB : n3;
 #pragma unroll 1
-        for (int r = 0; r < cntR; r++, i++) {
-          const double x = __ldg(src + r);
-          xf v = xf_from(x);
-          if (g >= 2) v = norm1(xf_mul(v, w));
-          M[i] = v.m;
-          E[i] = (short)(v.e * 4 + (int)(sign_of(x) >> 31));
+        for (int r = 0; r < cntR; r += 4) {
+          double x[4];
+#pragma unroll
+          for (int j = 0; j < 4; j++) x[j] = r + j < cntR ? __ldg(src + r + j) : 0.0;
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            if (r + j >= cntR) break;
+            xf v = xf_from(x[j]);
+            if (g >= 2) v = norm1(xf_mul(v, w));
+            M[i] = v.m;
+            E[i] = (short)(v.e * 4 + (int)(sign_of(x[j]) >> 31));
+            i++;
+          }
         }
       }
     }
