@@ -129,6 +129,7 @@ struct DevJob {
   struct T1Fail *listFail;
   bool plain;                    // runs the plain path's stages
   bool few, single;              // few primitive pairs in all; one primitive pair a type-2 part
+  bool twoWarps;                 // two warps a large-grid entry (batched path)
   int take;                      // work-list entries a warp takes before it exits
   int gcap;                      // type-1 step-table width cap (doubles per slot)
   int balance;                   // 1: narrower type-1 groups for units with few primitive pairs

@@ -1883,7 +1883,7 @@ int launch_fast_pipeline(const DevJob &J, cudaStream_t st, const FastConfig &cfg
     if (cfg.mixed) k_unit_small<true><<<gSmall, 32, sSmall, st>>>(K);
     else k_unit_small<false><<<gSmall, 32, sSmall, st>>>(K);
     K.take = takeLarge;
-    const int nw = J.few ? 2 : 1;
+    const int nw = J.twoWarps ? 2 : 1;
     (cfg.mixed ? nw > 1 ? k_unit_large<true, 2> : k_unit_large<true, 1>
                : nw > 1 ? k_unit_large<false, 2> : k_unit_large<false, 1>)<<<gLarge, 32 * nw, sLarge, st>>>(K);
     k_unit_link<<<units, link_threads(sLink), sLink, st>>>(K);

@@ -513,13 +513,18 @@ static PairPlan plan_of_pair(const Parsed &P, int p, bool single) {
 
 // Jobs of at most kFewPairs primitive pairs over all units: every warp of the
 // GPU gets at most a few work-list entries and the longest one sets a stage's
-// time, so an entry is one primitive pair (the 702-pair example's large-grid
-// stage takes 0.25 instead of 0.52 ms).
-constexpr long long kFewPairs = 4864;  // 32 a streaming multiprocessor
-static bool few_pairs(const Parsed &P) {
+// time, so an entry is one primitive pair (unit stages of 702 pairs 0.33 instead of
+// 0.58 ms, of 5148 pairs 0.42 instead of 0.66; of 38,300 pairs 1.55 instead of 1.40).
+constexpr long long kFewPairs = 9728;  // 64 a streaming multiprocessor
+// Up to kTwoWarpPairs the batched large grid gives an entry to two warps, which
+// halves its latency (38,300 pairs: 1.40 instead of 1.60 ms, a Hessian job of 51,480:
+// 1.83 instead of 2.23); with more the SMs are full and the two warps' different
+// code costs instruction fetches (150,792 pairs: 3.67 instead of 3.34 ms).
+constexpr long long kTwoWarpPairs = 58368;  // 384 a streaming multiprocessor
+static long long primitive_pairs(const Parsed &P) {
   long long n = 0;
   for (int p = 0; p < P.nPairs; p++) n += (long long)P.nCentres * P.shK[P.pairA[p]] * P.shK[P.pairB[p]];
-  return n <= kFewPairs;
+  return n;
 }
 
 // Whether a batched job runs the plain path's stages.  The batched path's
@@ -642,7 +647,7 @@ size_t job_device_bytes(const Parsed &P, int mode, size_t budget, size_t *scratc
   // other buffers fit is never refused for it
   const size_t base = in + work, cap = base < budget ? std::min(kScratchCap, budget - base) : 0;
   if (scratchCap) *scratchCap = cap;
-  return base > budget ? base : std::min(budget, base + scratch_bytes(P, cap, plain_stages(P, mode) || few_pairs(P)));
+  return base > budget ? base : std::min(budget, base + scratch_bytes(P, cap, plain_stages(P, mode) || primitive_pairs(P) <= kFewPairs));
 }
 
 int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int mode, cudaStream_t stream,
@@ -650,7 +655,9 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   const HostTables &h = T->host;
   std::memset(&J, 0, sizeof J);
   J.plain = plain_stages(P, mode);
-  J.few = few_pairs(P);
+  const long long np = primitive_pairs(P);
+  J.few = np <= kFewPairs;
+  J.twoWarps = np <= kTwoWarpPairs;
   J.single = J.few || J.plain;
   J.nAtoms = P.nAtoms; J.nShells = P.nShells; J.nPrims = P.nPrims; J.nCentres = P.nCentres;
   J.nPairs = P.nPairs; J.dim = P.dim;
