@@ -126,7 +126,6 @@ static __device__ __noinline__ double bessel_row(const DevJob &J, int l, double 
 static __device__ __noinline__ xf channel(const DevJob &J, int c, int l, double r, uint32_t &sign) {
   const xf R = xf_from(r), R2 = norm1(xf_mul(R, R));
   xs acc;
-  int top = -100000;  // every term so far is below 2^top
   const int *ch = J.chanT0 + c * (kMaxLEcp + 2) + l, t1 = ch[1];
 #pragma unroll 1
   for (int t = ch[0]; t < t1; t++) {
@@ -137,11 +136,8 @@ static __device__ __noinline__ xf channel(const DevJob &J, int c, int l, double 
     // 2^b above the term, b = log2 |d| + log2 r^n - a r^2 log2 e rounded up
     // (n <= 2; r^n otherwise unknown: never left out)
     const xf Rn = T.n == 1 ? R : R2;
-    const int b = T.de + 64 - (int)(((u64)(uint32_t)(E >> 32) * 1477) >> 31) + (T.n == 0 ? 0 : T.n < 3 ? Rn.e + 64 : 100000);
-    if (b < top - 70) continue;
     xf v = xf_mul(fx_exp(-(i64)E), {T.dm, T.de});
     if (T.n) v = xf_mul(v, T.n < 3 ? Rn : xf_from(rpow_rare(r, J.termN[t])));
-    top = v.e + 64 > top ? v.e + 64 : top;
     const i64 m = (i64)(v.m >> 4), s = (i64)(int)T.sign >> 31;
     acc = xs_add(acc, {(m ^ s) - s, v.e + 4});
   }

@@ -214,7 +214,8 @@ ECPGB_HD xf fx_bessel(const i64 *besX, const i64 *besXA, int HL1, int lmax, xf z
   } else {
     W += 1ull << 51;
     X = (W & ((1ull << 52) - 1)) << 11;
-    q += (size_t)(W >> 52) * HL1 * 8;
+    // (z = 0, a shell on the ECP centre: a block of its own, exactly 1, 0, 0, ...)
+    q += (size_t)(z100.m ? W >> 52 : 1601) * HL1 * 8;
   }
   const fxmul x = fx_split(X);
 ECPGB_NOUNROLL
@@ -229,10 +230,7 @@ ECPGB_NOUNROLL
     v = c23.x + mul_hi_s(v, x);
     v = c01.y + mul_hi_s(v, x);
     v = c01.x + mul_hi_s(v, x);
-    // (z = 0, a shell on the ECP centre: exactly 1, 0, 0, ...)
-    const bool zero = z100.m == 0;
-    if (zero) v = l == 0 ? (1ll << 62) - 1 : 0;
-    row(l, (u64)(v > 0 ? v : 0), zero ? 62 : (int)ld_one(q + scaleAt));
+    row(l, (u64)(v > 0 ? v : 0), (int)ld_one(q + scaleAt));
   }
   return c;
 }

@@ -474,7 +474,10 @@ static void fixed_row(const long double *c, int deg, long long *out, long long &
 void bessel_fixed(HostTables &t) {
   const int N = t.besselN + 1, HL = t.besselHL, AS = HL + 1 < 6 ? 6 : HL + 1;
   const long double h = 16.0L / t.besselN;
-  t.besselX.assign((size_t)N * (HL + 1) * 8, 0);
+  t.besselX.assign((size_t)(N + 1) * (HL + 1) * 8, 0);
+  // the rows of z = 0 (a shell on the ECP centre): 1, 0, 0, ...
+  t.besselX[(size_t)N * (HL + 1) * 8] = (1ll << 62) - 1;
+  for (int l = 0; l <= HL; l++) t.besselX[((size_t)N * (HL + 1) + l) * 8 + 6] = 62;
   for (int i = 0; i < N; i++)
     for (int l = 0; l <= HL; l++) {
       const double *q = &t.besselH[((size_t)i * (HL + 1) + l) * 6];

@@ -82,7 +82,7 @@ struct HostTables {
   std::vector<double> besselA;
   // The polynomials of besselH and besselA as 64-bit integers for Horner passes
   // in fixed point (ecp_fixed.h), both in a variable X in [0, 1/2]:
-  // besselX [i][l][8]: X = x / 2, z = z_i + (x - 1/2) h, h = 16/besselN, degree
+  // besselX [i][l][8] (and i = besselN + 1: z = 0 exactly): X = x / 2, z = z_i + (x - 1/2) h, h = 16/besselN, degree
   // 5, coefficients in [0..5]; besselXA [l][16]: X = 16 a, coefficients with
   // their signs in [0..l].  A row's value is v * 2^-scale, the scale in [6]
   // ([15] of besselXA).
