@@ -939,7 +939,7 @@ static __device__ void t2_small(const DevJob &J, const Unit &U, const LevelTab &
 // One warp a CTA; each takes up to J.take entries of the type-1 groups, then
 // of the type-2 batches (one kind of work at a time on the whole GPU).
 template <bool kMixed>
-__global__ void __launch_bounds__(32, 20) k_unit_small(DevJob J) {
+__global__ void __launch_bounds__(32, 24) k_unit_small(DevJob J) {
   extern __shared__ double sm[];
   __shared__ LevelTab V;
   level_tab(V, c93_3n, c93_nLevels, J.tol);
