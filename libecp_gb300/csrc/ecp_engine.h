@@ -126,6 +126,7 @@ struct DevJob {
   int chunk, nChunks, chunk0, chunk1;  // queue positions [chunk0, chunk1)
   long long scrBase;
   int2 *listT1, *listT2, *listPart;
+  int capT1;                     // entries listT1 has room for
   struct T1Fail *listFail;
   bool plain;                    // runs the plain path's stages
   bool few, single;              // few primitive pairs in all; one primitive pair a type-2 part

@@ -38,24 +38,17 @@ static __device__ inline bool ps93_exact(int k, double tol, int cnt, double I, d
 // A group of G primitive pairs of one kind (perm[p0 ..]) on the small grid
 // (src/type1.c:63-148), by one warp; lane = (pair, quadrature).
 template <bool kZero>
-static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem &L, double *sm, int pos, int p0,
+static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem &L, double *sm, int off, int p0,
                                 int G) {
-  const int lane = threadIdx.x & 31, lab = U.lab, lq = lab + 1, O = kSmallOrder, Nb = U.Nb, ws = U.ws, we = U.we;
+  const int lane = threadIdx.x & 31, lab = U.lab, lq = lab + 1, O = kSmallOrder, ws = U.ws, we = U.we;
   const int TS = 1 + 2 * lq, nq = t1_items(lab);
-  double *sc = sm + L.sc, *tab = sm + L.tab;
+  double *rec = sm + L.rec, *tab = sm + L.tab;  // the pairs' records
   const unsigned char *perm = (const unsigned char *)(U.scr + U.L.perm);
   const double *uL = J.uL + (size_t)U.c * O;
   __syncwarp();
-  if (lane < G) {
-    const int k = perm[p0 + lane];
-    const double za = U.pzA[k / Nb], zb = U.pzB[k % Nb];
-    const double ca = zeta_times(U.pcA[k / Nb], za, U.pa0), cb = zeta_times(U.pcB[k % Nb], zb, U.pb0);
-    double P[3];
-    for (int i = 0; i < 3; i++) P[i] = 2.0 * (za * U.gA[i] + zb * U.gB[i]);
-    sc[lane * 3 + 0] = sqrt(P[0] * P[0] + P[1] * P[1] + P[2] * P[2]);
-    sc[lane * 3 + 1] = ca * cb * exp(-za * U.gA[3] * U.gA[3] - zb * U.gB[3] * U.gB[3]);
-    sc[lane * 3 + 2] = -za - zb;
-  }
+#pragma unroll 1
+  for (int e = lane; e < G * kPairWords; e += 32)
+    rec[e] = ((const double *)(U.scr + U.L.pair))[perm[p0 + e / kPairWords] * kPairWords + e % kPairWords];
   __syncwarp();
   const bool mine = lane < G * nq;
   const int g = mine ? lane / nq : 0, qi = mine ? lane % nq : 0;
@@ -71,7 +64,7 @@ static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem 
   int k = -2, cnt = 0, lvEnd = 1;
   if (kZero) {
     if (mine) {
-      done = t1_zero_walk(J, sc[g * 3], sc[g * 3 + 2], ws, we);
+      done = t1_zero_walk(J, rec[g * kPairWords], rec[g * kPairWords + 2], ws, we);
       if (done) *Qout = 0.0;
     }
   } else
@@ -97,7 +90,8 @@ static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem 
                 t = tn & 0xffff, n = tn >> 16;
       // entry: K_l, then (C1 r^l) U, then the exponential
       double *ent = tab + ((t - s0) * G + gg) * TS, *WR = ent + lq;
-      const double r = J.xSmall[n], s = sc[gg * 3], C1 = sc[gg * 3 + 1], ex = (sc[gg * 3 + 2] * r + s) * r, u = uL[n];
+      const PairRec &P = *(const PairRec *)(rec + gg * kPairWords);
+      const double r = J.xSmall[n], s = P.s, C1 = P.C1, ex = (P.z * r + s) * r, u = uL[n];
       if (ex >= J.lnAcc1) {
         bessel_rows(J, lab, s * r, ent);
         double R = 1.0;
@@ -149,7 +143,7 @@ static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem 
 #pragma unroll 1
   for (int gg = 0; fail && gg < G; gg++) {
     const unsigned m = fail >> (gg * nq) & (nq >= 32 ? ~0u : (1u << nq) - 1u);
-    if (m && lane == 0) J.listFail[atomicAdd(J.counters + kCntFail, 1u)] = {pos, perm[p0 + gg], m, 0, sc[gg * 3]};
+    if (m && lane == 0) J.listFail[atomicAdd(J.counters + kCntFail, 1u)] = {off, perm[p0 + gg], m, 0, rec[gg * kPairWords]};
   }
 }
 
@@ -195,13 +189,13 @@ static __device__ void x2_small(const DevJob &J, const Unit &U, int q0) {
 __global__ void __launch_bounds__(32, 16) k_exact_small(DevJob J) {
   extern __shared__ double sm[];
   const SmallSmem L = small_layout(J.maxLBS, 0, J.gcap);
-  const int n1 = (int)J.counters[kCntT1], n = n1 + (int)J.counters[kCntT2];
+  const int n0 = (int)J.counters[kCntT1], n1 = n0 + (int)J.counters[kCntRest], n = n1 + (int)J.counters[kCntT2];
 #pragma unroll 1
   for (int taken = 0; taken < J.take; taken++) {
     const int i = next_item(J.counters + kHeadSmall);
     if (i >= n) return;
-    const int2 it = i < n1 ? J.listT1[i] : J.listT2[i - n1];
-    const Unit U = unit_load(J, it.x);
+    const int2 it = small_entry(J, i, n0, n1);
+    const Unit &U = unit_get(J, it.x);
     if (i >= n1) {
       x2_small(J, U, it.y);
       continue;
@@ -600,11 +594,11 @@ __global__ void __launch_bounds__(32, 14) k_exact_large(DevJob J) {
     if (i >= n) return;
     if (i < n2) {
       const int2 it = J.listPart[i];
-      const Unit U = unit_load(J, it.x);
+      const Unit &U = unit_get(J, it.x);
       x2_large(J, U, L, sm, it.y);
     } else {
       const T1Fail it = J.listFail[i - n2];
-      const Unit U = unit_load(J, it.pos);
+      const Unit &U = unit_get(J, it.off);
       x1_large(J, U, L, sm, it.k, it.mask, it.s);
     }
   }

@@ -549,44 +549,24 @@ static __device__ __noinline__ EntInfo t1_large_entry(const DevJob &J, int c, in
 
 // --------------------------------------------------- stage 2: the small grid
 
-// A primitive pair's scalars for the small grid, out of line (one copy for the
-// kinds): |P| (as src/util.c:75-106), the prefactor, -za - zb, and for the
-// normal kind s and Z r (r inside the window) as integers times 2^q, both
-// below 2^62.
-static __device__ __noinline__ void t1_pair_setup(const DevJob &J, const Unit &U, int k, double *sc, PairFx *fx) {
-  const int i = k / U.Nb, j = k - i * U.Nb;
-  // derivative blocks: coefficients times zeta^max(0, shift) (src/type1.c:239-246)
-  const double za = U.pzA[i], ca = zeta_times(U.pcA[i], za, U.pa0), zb = U.pzB[j], cb = zeta_times(U.pcB[j], zb, U.pb0);
-  double P[3];
-  for (int x = 0; x < 3; x++) P[x] = 2.0 * (za * U.gA[x] + zb * U.gB[x]);
-  const double s = sqrt(P[0] * P[0] + P[1] * P[1] + P[2] * P[2]);
-  sc[0] = s;
-  sc[1] = t1_prefactor(za, ca, zb, cb, U.gA[3], U.gB[3]);
-  sc[2] = -za - zb;
-  if (fx) {
-    const xf S = xf_from(s), Z = xf_from(za + zb), s100 = xf_times100(S);
-    const int zr = Z.e + xf_from(J.xSmall[U.we - 1]).e + 64, q = -3 - (S.e > zr ? S.e : zr);
-    *fx = {(i64)shr64(S.m, -(S.e + q)), Z.m, s100.m, Z.e, s100.e, q};
-  }
-}
-
 // A group of G primitive pairs of one kind (perm[p0 ..]) of a unit's type-1
 // quadratures on the small grid (src/type1.c:95-148), by one warp; lane =
 // (pair, quadrature).  Converged quadratures are written to the unit's Q, the
 // pairs with a failed one to the fallback list.
 template <bool kMixed, int kKind>
 static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem &L, double *sm, const LevelTab &V,
-                                int pos, int p0, int G) {
+                                int off, int p0, int G) {
   const int lane = threadIdx.x & 31, lab = U.lab, lq = lab + 1, O = kSmallOrder, ws = U.ws, we = U.we;
   // odd entry strides: lanes touching neighbouring entries hit distinct banks
   const int TS = 1 + 2 * lq, nq = t1_items(lab);
   const u64 thr = (u64)(i64)(-J.lnAcc1 * 0x1p53);
-  double *sc = sm + L.sc, *tab = sm + L.tab;
-  PairFx *fx = (PairFx *)(sm + L.fx);
+  double *rec = sm + L.rec, *tab = sm + L.tab;  // the pairs' records
   const unsigned char *perm = (const unsigned char *)(U.scr + U.L.perm);
   const double *uL = J.uL + (size_t)U.c * O;
   __syncwarp();
-  if (lane < G) t1_pair_setup(J, U, perm[p0 + lane], sc + lane * 3, kKind == kPairNormal ? fx + lane : nullptr);
+#pragma unroll 1
+  for (int e = lane; e < G * kPairWords; e += 32)
+    rec[e] = ((const double *)(U.scr + U.L.pair))[perm[p0 + e / kPairWords] * kPairWords + e % kPairWords];
   __syncwarp();
   // (2) PS93: lane = (pair g, quadrature (l1, l2))
   const bool mine = lane < G * nq;
@@ -607,7 +587,7 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
   if constexpr (kKind == kPairZero) {
     // converged quadratures give 0; failed ones go to the fallback
     if (mine) {
-      done = t1_zero_walk(J, sc[g * 3], sc[g * 3 + 2], ws, we);
+      done = t1_zero_walk(J, rec[g * kPairWords], rec[g * kPairWords + 2], ws, we);
       if (done) *Qout = 0.0;
     }
   } else
@@ -651,10 +631,11 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
       const int i = slot_of(e);
       const int gg = live_pair(e, i), tn = __ldg(J.byN93 + s0 + lo + i), t = tn & 0xffff, n = tn >> 16;
       double *ent = tab + ((t - s0) * G + gg) * TS, *WR = ent + lq;
-      const double s = sc[gg * 3], C1 = sc[gg * 3 + 1];
+      const PairRec &P = *(const PairRec *)(rec + gg * kPairWords);
+      const double s = P.s, C1 = P.C1;
       if constexpr (kKind == kPairBand) {
         // row l: (C1 r^l) U; the walk multiplies by K, exp(e) and w in turn
-        const double r = J.xSmall[n], ex = t1_exponent(sc[gg * 3 + 2], s, r);
+        const double r = J.xSmall[n], ex = t1_exponent(P.z, s, r);
         bessel_fx(J, lab, xf_mul(xf_times100(xf_from(s)), xf_from(r)), {0, 0}, 0, ent);
         double R = 1.0;
 #pragma unroll 1
@@ -668,7 +649,7 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
         // w C1 U_L exp(e) r^l with 60-bit mantissas
         const double w = J.wSmall[n], u = uL[n];
         const xf R = xf_from(J.xSmall[n]);
-        const PairFx F = fx[gg];
+        const PairFx F = P.fx;
         const u64 zr = shr64(mul_hi(F.Zm, R.m), -(F.Ze + R.e + 64 + F.q));
         const i64 tt = F.S - (i64)zr;
         u64 E = mul_hi(tt < 0 ? (u64)-tt : (u64)tt, R.m);
@@ -808,7 +789,7 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
     if (!m) continue;
     int ffp = 0;
     if constexpr (kMixed) ffp = __reduce_max_sync(0xffffffffu, g == gg ? est : 0u) < lim;
-    if (lane == 0) J.listFail[atomicAdd(J.counters + kCntFail, 1u)] = {pos, perm[p0 + gg] | ffp << 16, m, 0, sc[gg * 3]};
+    if (lane == 0) J.listFail[atomicAdd(J.counters + kCntFail, 1u)] = {off, perm[p0 + gg] | ffp << 16, m, 0, rec[gg * kPairWords]};
   }
 }
 
@@ -944,13 +925,13 @@ __global__ void __launch_bounds__(32, 24) k_unit_small(DevJob J) {
   __shared__ LevelTab V;
   level_tab(V, c93_3n, c93_nLevels, J.tol);
   const SmallSmem L = small_layout(J.maxLBS, J.t2Rows, J.gcap);
-  const int n1 = (int)J.counters[kCntT1], n = n1 + (int)J.counters[kCntT2];
+  const int n0 = (int)J.counters[kCntT1], n1 = n0 + (int)J.counters[kCntRest], n = n1 + (int)J.counters[kCntT2];
 #pragma unroll 1
   for (int taken = 0; taken < J.take; taken++) {
     const int i = next_item(J.counters + kHeadSmall);
     if (i >= n) return;
-    const int2 it = i < n1 ? J.listT1[i] : J.listT2[i - n1];
-    const Unit U = unit_load(J, it.x);
+    const int2 it = small_entry(J, i, n0, n1);
+    const Unit &U = unit_get(J, it.x);
     if (i >= n1) {
       t2_small<kMixed>(J, U, V, (u64 *)(sm + L.tab), (int *)(sm + L.quad), it.y);
       continue;
@@ -1602,7 +1583,7 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) k_unit_large(DevJob 
     }
     if (i >= n2) break;
     const int2 it = J.listPart[i];
-    const Unit U = unit_load(J, it.x);
+    const Unit &U = unit_get(J, it.x);
     t2_large<kMixed, kWarps>(J, U, L, sm, V, it.y);
   }
 #pragma unroll 1
@@ -1611,7 +1592,7 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) k_unit_large(DevJob 
     if (i >= n || threadIdx.x >= 32) i = next_item(J.counters + kHeadLarge);
     if (i >= n) return;
     const T1Fail it = J.listFail[i - n2];
-    const Unit U = unit_load(J, it.pos);
+    const Unit &U = unit_get(J, it.off);
     t1_large<kMixed>(J, U, L, sm, V, it.k & 0xffff, it.k >> 16, it.mask, it.s);
   }
 }

@@ -133,24 +133,51 @@ __host__ __device__ inline int t2_parts(int NP, bool single) {
   return (NP + n - 1) / n;
 }
 
-// Global scratch of one unit between the stages (byte offsets): a header,
-// per primitive pair the FM06 map (i1, i2) and {break index, window}, the
-// type-1 quadratures [pair][t1_index], the type-2 quadratures of the class's
-// items, their partial sums [part][item] when there are several parts, the
-// bitmap of failed items, and the primitive pairs ordered by kind.
+// A unit as the stages see it: the pair's shells and derivative shift, the
+// screened window, its scratch (byte offsets L).  The plan leaves it in the
+// scratch, where the work-list entries point.
+struct UnitScratch {
+  int map, win, pair, Q, T, part, mask, perm, total;
+};
+struct Unit {
+  int c, pr, sa, sb, A, B, la, lb, lab, lpa, lpb, pa0, pb0, ws, we, Nb, NP, Lc, cls, nItems;
+  const double *gA, *gB, *pzA, *pcA, *pzB, *pcB;
+  char *scr;
+  UnitScratch L;
+  bool live;
+};
 struct UnitHead {
   u64 est;   // mixed path: largest |estimate| of a failed small-grid item (bits)
   int warn;  // 1: a type-1, 2: a type-2 quadrature ran out of levels
-  int pad;
+  int off;   // the scratch's offset in 16 bytes, for the work lists
+  Unit unit;
 };
-struct UnitScratch {
-  int map, win, Q, T, part, mask, perm, total;
+// A normal-kind primitive pair's scalars in fixed point: s = |P| as S 2^-q,
+// Z = za + zb (mantissa and exponent), 100 s.
+struct PairFx {
+  i64 S;
+  u64 Zm, sm;
+  int Ze, se, q;
 };
+// What the small grid reads of a primitive pair: s = |P|, the prefactor C1,
+// -za - zb.
+struct PairRec {
+  double s, C1, z;
+  PairFx fx;
+};
+constexpr int kPairWords = sizeof(PairRec) / sizeof(double);
+
+// Global scratch of one unit between the stages (byte offsets): the head, per
+// primitive pair the FM06 map (i1, i2), {break index, window} and the record
+// above, the type-1 quadratures [pair][t1_index], the type-2 quadratures of the
+// class's items, their partial sums [part][item] when there are several parts, the
+// bitmap of failed items, and the primitive pairs ordered by kind.
 __host__ __device__ inline UnitScratch unit_scratch(int NP, int lab, int nItems, bool single) {
   UnitScratch s;
-  int o = (int)sizeof(UnitHead);
+  int o = ((int)sizeof(UnitHead) + 15) & ~15;
   s.map = o; o += 16 * NP;
   s.win = o; o += 16 * NP;
+  s.pair = o; o += (int)sizeof(PairRec) * NP;
   s.Q = o; o += 8 * NP * t1_items(lab);
   s.T = o; o += 8 * nItems;
   s.part = o; o += t2_parts(NP, single) > 1 ? 8 * t2_parts(NP, single) * nItems : 0;
@@ -162,7 +189,7 @@ __host__ __device__ inline UnitScratch unit_scratch(int NP, int lab, int nItems,
 // Work-list entries a unit can add: type-1 groups (at most one per pair),
 // type-2 small-grid batches, type-2 parts, failed type-1 pairs.
 struct T1Fail {
-  int pos, k;  // queue position, primitive pair (bit 16: double-single tables)
+  int off, k;  // the unit's scratch, primitive pair (bit 16: double-single tables)
   unsigned mask;
   int pad;
   double s;  // |P|
@@ -171,18 +198,10 @@ __host__ __device__ inline size_t unit_list_bytes(int NP, int nItems, bool singl
   return 8 * (size_t)NP + 8 * (size_t)((nItems + 31) / 32) + 8 * (size_t)t2_parts(NP, single) + sizeof(T1Fail) * (size_t)NP;
 }
 
-// A normal-kind primitive pair's scalars in fixed point: s = |P| as S 2^-q,
-// Z = za + zb (mantissa and exponent), 100 s.
-struct PairFx {
-  i64 S;
-  u64 Zm, sm;
-  int Ze, se, q;
-};
-
 // Shared memory of the stages, in doubles.  Small grid (one warp a CTA): the
 // group's pair scalars and step table.
 struct SmallSmem {
-  int sc, fx, quad, tab, total;
+  int rec, quad, tab, total;
 };
 __host__ __device__ inline SmallSmem small_layout(int LB, int rows, int cap) {
   SmallSmem s;
@@ -192,9 +211,8 @@ __host__ __device__ inline SmallSmem small_layout(int LB, int rows, int cap) {
     const int w = 33 * t1_group(lab, cap) * (2 * lab + 3);
     if (w > tt) tt = w;
   }
-  s.sc = 0;
-  s.fx = 24;  // 3 scalars of up to 8 pairs
-  s.quad = s.fx + 8 * (int)(sizeof(PairFx) / sizeof(double));  // 32 ints
+  s.rec = 0;                      // up to 8 pairs
+  s.quad = 8 * kPairWords;        // 32 ints
   s.tab = s.quad + 16;
   s.total = s.tab + tt;
   return s;
@@ -262,16 +280,6 @@ __host__ __device__ inline LinkSmem link_layout(int LB, int LE) {
   return s;
 }
 
-// A unit as the stages see it: queue position pos = (sorted pair, centre),
-// the pair's shells and derivative shift, the screened window, its scratch.
-struct Unit {
-  int c, pr, sa, sb, A, B, la, lb, lab, lpa, lpb, pa0, pb0, ws, we, Nb, NP, Lc, cls, nItems;
-  const double *gA, *gB, *pzA, *pcA, *pzB, *pcB;
-  char *scr;
-  UnitScratch L;
-  bool live;
-};
-
 // Unit id of queue position pos (pairs in the plan's order, centres innermost).
 static __device__ inline long long unit_at(const DevJob &J, int pos) {
   const int c = J.ctrOrder[pos % J.nCentres], pr = J.pairOrder[pos / J.nCentres];
@@ -285,6 +293,12 @@ static __device__ inline int class_items(const DevJob &J, int ncls, int l) {
   return n;
 }
 
+// The unit a work-list entry points to.
+static __device__ inline const Unit &unit_get(const DevJob &J, int off) {
+  return ((const UnitHead *)(J.scr + (size_t)off * 16))->unit;
+}
+
+// The unit at queue position pos = (sorted pair, centre).
 static __device__ inline Unit unit_load(const DevJob &J, int pos) {
   Unit U;
   const int ps = pos / J.nCentres, ci = pos % J.nCentres;
@@ -336,7 +350,7 @@ static __device__ inline int unit_item(const DevJob &J, const Unit &U, int q) {
 }
 
 // Work lists of a chunk and their counters (zeroed before the chunk).
-enum { kCntT1, kCntT2, kCntFail, kCntPart, kHeadSmall, kHeadLarge, kCounters };
+enum { kCntT1, kCntRest, kCntT2, kCntFail, kCntPart, kHeadSmall, kHeadLarge, kCounters };
 
 // The next entry of a list for a warp; its index to every lane.
 static __device__ inline int next_item(unsigned *head) {
@@ -398,7 +412,8 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
   unsigned *mask = (unsigned *)(U.scr + U.L.mask);
 #pragma unroll 1
   for (int w = lane; w < (U.nItems + 31) / 32; w += 32) mask[w] = 0u;
-  if (lane == 0) *(UnitHead *)U.scr = {0ull, 0, 0};
+  const int off = (int)((U.scr - J.scr) >> 4);
+  if (lane == 0) *(UnitHead *)U.scr = {0ull, 0, off, U};
   int cnt[3] = {0, 0, 0};
   unsigned kinds = 0;  // the lane's pairs' kinds, 2 bits each (at most 8)
 #pragma unroll 1
@@ -414,6 +429,17 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
       const double s2 = P[0] * P[0] + P[1] * P[1] + P[2] * P[2];
       kind = C1 == 0.0 ? kPairZero
                        : (kExact || fabs(C1) < 0x1p-900 || s2 > 2800.0 * (za + zb)) ? kPairBand : kPairNormal;
+      PairRec rec;
+      rec.s = sqrt(s2);
+      rec.C1 = C1;
+      rec.z = -za - zb;
+      if (!kExact && kind == kPairNormal) {
+        // s and Z r (r inside the window) as integers times 2^q, both below 2^62
+        const xf S = xf_from(rec.s), Z = xf_from(za + zb), s100 = xf_times100(S);
+        const int zr = Z.e + xf_from(J.xSmall[U.we - 1]).e + 64, q = -3 - (S.e > zr ? S.e : zr);
+        rec.fx = {(i64)shr64(S.m, -(S.e + q)), Z.m, s100.m, Z.e, s100.e, q};
+      }
+      ((PairRec *)(U.scr + U.L.pair))[k] = rec;
       double i1, i2;
       fm06(za, zb, dAC, dBC, i1, i2);
       map[k] = make_double2(i1, i2);
@@ -516,23 +542,33 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
     nGroups += n[kd];
   }
   const int nBatch = (U.nItems + 31) / 32, nPart = U.nItems > 0 ? t2_parts(NP, J.single) : 0;
+  // the type-1 list holds the groups of normal kind from its front and the others
+  // from its end: warps that run at the same time run the same code
   int base = 0;
-  if (lane < 3) base = (int)atomicAdd(J.counters + (lane == 0 ? kCntT1 : lane == 1 ? kCntT2 : kCntPart),
-                                      (unsigned)(lane == 0 ? nGroups : lane == 1 ? nBatch : nPart));
-  const int b1 = __shfl_sync(0xffffffffu, base, 0), b2 = __shfl_sync(0xffffffffu, base, 1),
-            b3 = __shfl_sync(0xffffffffu, base, 2);
+  if (lane < 4)
+    base = (int)atomicAdd(J.counters + (lane == 0 ? kCntT1 : lane == 1 ? kCntRest : lane == 2 ? kCntT2 : kCntPart),
+                          (unsigned)(lane == 0 ? n[0] : lane == 1 ? n[1] + n[2] : lane == 2 ? nBatch : nPart));
+  const int b1 = __shfl_sync(0xffffffffu, base, 0), br = __shfl_sync(0xffffffffu, base, 1),
+            b2 = __shfl_sync(0xffffffffu, base, 2), b3 = __shfl_sync(0xffffffffu, base, 3);
 #pragma unroll 1
   for (int g = lane; g < nGroups; g += 32) {
     int kd = 0, gj = g, p0 = 0;
     while (gj >= n[kd]) { gj -= n[kd]; p0 += cnt[kd]; kd++; }
     p0 += gj * G[kd];
     const int left = cnt[kd] - gj * G[kd];
-    J.listT1[b1 + g] = make_int2(pos, p0 | (left < G[kd] ? left : G[kd]) << 10 | kd << 16);
+    J.listT1[kd == 0 ? b1 + g : J.capT1 - 1 - (br + g - n[0])] =
+        make_int2(off, p0 | (left < G[kd] ? left : G[kd]) << 10 | kd << 16);
   }
 #pragma unroll 1
-  for (int q = lane; q < nBatch; q += 32) J.listT2[b2 + q] = make_int2(pos, 32 * q);
+  for (int q = lane; q < nBatch; q += 32) J.listT2[b2 + q] = make_int2(off, 32 * q);
 #pragma unroll 1
-  for (int q = lane; q < nPart; q += 32) J.listPart[b3 + q] = make_int2(pos, q);
+  for (int q = lane; q < nPart; q += 32) J.listPart[b3 + q] = make_int2(off, q);
+}
+
+// Entry i of the small-grid stage: the type-1 groups of normal kind, the other
+// groups, the type-2 batches.
+static __device__ inline int2 small_entry(const DevJob &J, int i, int n0, int n1) {
+  return i < n0 ? J.listT1[i] : i < n1 ? J.listT1[J.capT1 - 1 - (i - n0)] : J.listT2[i - n1];
 }
 
 // The blocks of a unit from its combined-index block H (type 1) and its radial
@@ -814,6 +850,7 @@ static void launch_chunks(DevJob J, const JobPlan::Order &ord, cudaStream_t st, 
     J.scrBase = ch.base;
     char *lists = J.scr + ch.scratch;
     J.listT1 = (int2 *)lists;
+    J.capT1 = (int)ch.groups;
     J.listT2 = J.listT1 + ch.groups;
     J.listPart = J.listT2 + ch.batches;
     J.listFail = (T1Fail *)(J.listPart + ch.parts);
