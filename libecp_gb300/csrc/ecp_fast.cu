@@ -955,9 +955,8 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, const LargeSmem 
   double *tab = sm + Ls.tab + (threadIdx.x >> 5) * Ls.tabT1;
   int *quad = (int *)(sm + Ls.fail) + (threadIdx.x >> 5) * 32;  // the running quadratures, by rank
   const int lane = threadIdx.x & 31, lab = U.lab, lq = lab + 1, O = kSmallOrder, OL = J.largeOrder, TSf = 3 + 2 * lq;
-  const int Nb = U.Nb, ws = U.ws, we = U.we, c = U.c, Lc = U.Lc;
+  const int ws = U.ws, we = U.we, c = U.c, Lc = U.Lc;
   const double *uL = J.uL + (size_t)c * O;
-  const double dAC = U.gA[3], dBC = U.gB[3];
   const bool fail = mask >> lane & 1u;
   int l1 = 0, l2 = 0;
   {
@@ -965,40 +964,12 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, const LargeSmem 
     while (l1 <= lab && rem >= l1 / 2 + 1) { rem -= l1 / 2 + 1; l1++; }
     l2 = l1 - 2 * rem;
   }
-  const double za = U.pzA[kk / Nb], ca = zeta_times(U.pcA[kk / Nb], za, U.pa0), zb = U.pzB[kk % Nb],
-               cb = zeta_times(U.pcB[kk % Nb], zb, U.pb0);
-  const double z = -za - zb, zd2 = -za * dAC * dAC - zb * dBC * dBC;
-  const double C2 = ca * cb;
+  const PairRec &P = ((const PairRec *)(U.scr + U.L.pair))[kk];
+  const double z = P.z, zd2 = P.zd2, C2 = P.C2;
   const double2 map = ((const double2 *)(U.scr + U.L.map))[kk];
   const double i1 = map.x, i2 = map.y;
   const ff C2f = ff_from_double(C2), sf = ff_from_double(s), i1f = ff_from_double(i1);
-  // first point past both centres whose exponent is below the screen
-  // (src/type1.c:168-176).  Past both centres the exponent falls as r
-  // grows, so the predicate is monotone in the index: a 32-way search,
-  // first over the last points of 32 chunks, then inside the first chunk
-  // whose last point qualifies.
-  auto brk = [&](int n) {
-    const double r = i1 * J.xLarge[n] + i2, e = (z * r + s) * r + zd2;
-    return r > dAC && r > dBC && e < J.lnAcc1;
-  };
-  const int chunk = (OL + 31) / 32;
-  int nb = OL;
-  {
-    const int n = lane * chunk + chunk - 1 < OL ? lane * chunk + chunk - 1 : OL - 1;
-    const unsigned b = __ballot_sync(0xffffffffu, brk(n));
-    if (b) {
-      const int n0 = (__ffs(b) - 1) * chunk;
-#pragma unroll 1
-      for (int c0 = n0; c0 < n0 + chunk && c0 < OL; c0 += 32) {
-        const int m = c0 + lane;
-        const unsigned b2 = __ballot_sync(0xffffffffu, m < n0 + chunk && m < OL && brk(m));
-        if (b2) {
-          nb = c0 + __ffs(b2) - 1;
-          break;
-        }
-      }
-    }
-  }
+  const int nb = ((const int4 *)(U.scr + U.L.win))[kk].w;
   const int end = nb - 1;
   double I2 = 0, p2 = 0, q2 = 0, res2 = 0;  // double-single sums (mixed path)
   Psm92 S;
@@ -1204,10 +1175,10 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
   int *pend = (int *)(sm + L.pend) + warp * 64;
   int *red = (int *)(sm + L.red);
   (void)red;
-  const double za = pzA[k / Nb], ca = U.pcA[k / Nb], zb = pzB[k % Nb], cb = U.pcB[k % Nb];
-  // derivative blocks: the product times zeta_a^max(0, shifta), then
-  // zeta_b^max(0, shiftb) (src/type2.c:456-462)
-  const double Ck = zeta_times(zeta_times(ca * cb, za, U.pa0), zb, U.pb0);
+  // derivative blocks: the product times zeta_a^max(0, shifta), zeta_b^max(0, shiftb)
+  // (src/type2.c:456-462)
+  const PairRec &P = ((const PairRec *)(U.scr + U.L.pair))[k];
+  const double za = P.za, zb = P.zb, Ck = P.C2;
   const double i1 = map[k].x;
   const double iCk = i1 * Ck;
   const ff i1f = ff_from_double(i1), Ckf = ff_from_double(Ck);

@@ -80,6 +80,18 @@ static __device__ inline long long ordered_bits(double x) {
   return b ^ (long long)((unsigned long long)(b >> 63) >> 1);
 }
 
+// The first large-grid point with abscissa x >= b, and the first with x > b.
+static __device__ __noinline__ int first_key(const DevJob &J, long long key) {
+  int lo = 0, hi = J.largeOrder;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (ordered_bits(J.xLarge[mid]) >= key) hi = mid; else lo = mid + 1;
+  }
+  return lo;
+}
+static __device__ inline int first_from(const DevJob &J, double b) { return first_key(J, ordered_bits(b)); }
+static __device__ inline int first_after(const DevJob &J, double b) { return first_key(J, ordered_bits(b) + 1); }
+
 // FM06 map parameters (src/gc_integrators.c:317-331).
 static __device__ inline void fm06(double za, double zb, double dAC, double dBC, double &i1, double &i2) {
   double zp = za + zb, P = (za * dAC + zb * dBC) / zp;
@@ -159,10 +171,11 @@ struct PairFx {
   u64 Zm, sm;
   int Ze, se, q;
 };
-// What the small grid reads of a primitive pair: s = |P|, the prefactor C1,
-// -za - zb.
+// What the stages read of a primitive pair: s = |P|, the prefactor C1, -za - zb
+// and, on the batched path, the exponents, the coefficients' product C2 and
+// zd2 = -za dAC^2 - zb dBC^2.
 struct PairRec {
-  double s, C1, z;
+  double s, C1, z, za, zb, C2, zd2;
   PairFx fx;
 };
 constexpr int kPairWords = sizeof(PairRec) / sizeof(double);
@@ -433,6 +446,10 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
       rec.s = sqrt(s2);
       rec.C1 = C1;
       rec.z = -za - zb;
+      rec.za = za;
+      rec.zb = zb;
+      rec.C2 = ca * cb;
+      rec.zd2 = -za * dAC * dAC - zb * dBC * dBC;
       if (!kExact && kind == kPairNormal) {
         // s and Z r (r inside the window) as integers times 2^q, both below 2^62
         const xf S = xf_from(rec.s), Z = xf_from(za + zb), s100 = xf_times100(S);
@@ -443,6 +460,14 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
       double i1, i2;
       fm06(za, zb, dAC, dBC, i1, i2);
       map[k] = make_double2(i1, i2);
+      int t1Break = 0;
+      if constexpr (!kExact) {
+        // first point past both centres whose type-1 exponent (z r + s) r + zd2 is
+        // below the screen (src/type1.c:168-176): the root of the parabola
+        const double zp = za + zb, q = rec.s * rec.s - 4.0 * zp * (J.lnAcc1 - rec.zd2);
+        const double root = q > 0.0 ? 0.5 * (rec.s + sqrt(q)) / zp : 0.0, far = dAC > dBC ? dAC : dBC;
+        t1Break = first_after(J, ((root > far ? root : far) - i2) / i1);
+      }
       if (U.nItems > 0) {
         // break index, and the point-index interval in which the pair's
         // exponent passes the screen: past both centres the exponent falls with
@@ -456,21 +481,11 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
           // -> 69 us for 6048 units)
           const double zp = za + zb, mu = za * zb / zp * (dAC - dBC) * (dAC - dBC), q = (-J.lnAcc2 - mu) / zp;
           const double h = sqrt(q > 0.0 ? q : 0.0), m = 1.0 / i1;
-          // first point with x >= b, or x > b
-          auto first = [&](double b, bool after) {
-            const long long key = ordered_bits(b) + (after ? 1 : 0);
-            int lo = 0, hi = J.largeOrder;
-            while (lo < hi) {
-              const int mid = (lo + hi) >> 1;
-              if (ordered_bits(J.xLarge[mid]) >= key) hi = mid; else lo = mid + 1;
-            }
-            return lo;
-          };
-          const int n0 = first((V - h - i2) * m, false), n1 = first((V + h - i2) * m, true),
-                    n2 = first(((dAC > dBC ? dAC : dBC) - i2) * m, true);
+          const int n0 = first_from(J, (V - h - i2) * m), n1 = first_after(J, (V + h - i2) * m),
+                    n2 = first_after(J, ((dAC > dBC ? dAC : dBC) - i2) * m);
           const int brk = q >= 0.0 && n1 > n2 ? n1 : n2;
-          win[k] = q >= 0.0 ? make_int4(brk < J.largeOrder ? brk : INT_MAX, n0, n1 - 1, 0)
-                            : make_int4(brk < J.largeOrder ? brk : INT_MAX, 1, 0, 0);
+          win[k] = q >= 0.0 ? make_int4(brk < J.largeOrder ? brk : INT_MAX, n0, n1 - 1, t1Break)
+                            : make_int4(brk < J.largeOrder ? brk : INT_MAX, 1, 0, t1Break);
         } else {
           // (the stage tests every slot of the interval itself: a margin of 1)
           const double thr = J.lnAcc2 - 1.0;
@@ -508,6 +523,8 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
           }
           win[k] = make_int4(brk, nLo, a - 1, 0);
         }
+      } else {
+        win[k] = make_int4(INT_MAX, 1, 0, t1Break);
       }
     }
     kinds |= (unsigned)kind << (2 * j);
