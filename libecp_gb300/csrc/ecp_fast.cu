@@ -77,15 +77,6 @@ static __device__ __noinline__ RowBase bessel_rows2(const DevJob &J, int lmax, x
   b.odd = base[1];
   return b;
 }
-// The rows as normalised mantissas and exponents for the type-2 tables.
-static __device__ __noinline__ xf bessel_me(const DevJob &J, int lmax, xf z100, u64 *K, short *E) {
-  return fx_bessel(J.besX, J.besXA, J.besHL + 1, lmax, z100, [&](int l, u64 v, int scale) {
-    const xf k = xf_norm({v, -scale});
-    K[l] = k.m;
-    E[l] = (short)k.e;
-  });
-}
-
 // Powers of r other than 0, 1, 2: rare, out of line.
 static __device__ __noinline__ double rpow_rare(double r, double n) { return rpow(r, n); }
 
@@ -1135,10 +1126,25 @@ static __device__ __noinline__ i64 t2_exponent(double za, double zb, double dA, 
   for (int side = 0; side < 2; side++) E += fx_gauss(side ? zb : za, (side ? dB : dA) - r);
   return -(i64)E;
 }
-// 100 times the Bessel argument 2 zeta d r without its r.
-static __device__ __noinline__ xf t2_argument(double zeta, double d) {
-  const xf z = xf_mul(xf_from(zeta), xf_from(d));
-  return xf_times100({z.m, z.e + 1});
+// A slot's rows K_l1 and K_l2 as normalised mantissas and exponents; returns their
+// common factors (large arguments).
+static __device__ __noinline__ xf t2_bessel(const DevJob &J, double za, double zb, double dA, double dB, double r,
+                                            u64 *Ka, u64 *Kb, short *Ea, short *Eb, int la, int lb) {
+  xf f = {1ull << 63, -63};
+#pragma unroll 1
+  for (int side = 0; side < 2; side++) {
+    const xf z = xf_mul(xf_from(side ? zb : za), xf_from(side ? dB : dA));  // 2 zeta d r: exponent + 1
+    u64 *K = side ? Kb : Ka;
+    short *E = side ? Eb : Ea;
+    const xf c = fx_bessel(J.besX, J.besXA, J.besHL + 1, side ? lb : la,
+                           xf_mul(xf_times100({z.m, z.e + 1}), xf_from(r)), [&](int l, u64 v, int scale) {
+                             const xf k = xf_norm({v, -scale});
+                             K[l] = k.m;
+                             E[l] = (short)k.e;
+                           });
+    f = norm1(xf_mul(f, c));
+  }
+  return f;
 }
 
 // One primitive pair of the type-2 large-grid fallback, by the CTA's one or two
@@ -1284,12 +1290,7 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
         short *Ue = (short *)(tab + 32 * TS) + lane * ES, *Ae = Ue + LE, *Be = Ae + LBE, *Re = Be + LBE;
         const xf Rx = xf_from(r);
         if (role == 0) {
-          // through one copy of the Bessel code
-#pragma unroll 1
-          for (int side = 0; side < 2; side++) {
-            const xf z = t2_argument(side ? zbj : zaj, side ? dBC : dAC);
-            f = norm1(xf_mul(f, bessel_me(J, side ? pL2 : pL1, xf_mul(z, Rx), side ? Kb : Ka, side ? Be : Ae)));
-          }
+          f = t2_bessel(J, zaj, zbj, dAC, dBC, r, Ka, Kb, Ae, Be, pL1, pL2);
           if constexpr (kWarps > 1) {  // the other warp has the potential
 #pragma unroll 1
             for (int l = 0; l <= pL2; l++) {
