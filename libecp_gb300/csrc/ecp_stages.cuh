@@ -279,15 +279,16 @@ __host__ __device__ inline LinkSmem link_layout(int LB, int LE) {
   const int ncAB = (2 * LB + 1) * (2 * LB + 2) * (2 * LB + 3) / 6;
   int o = 0;
   s.chi = o; o += nc * nc;
-  s.J = o; o += nct * nc;
-  s.T = o; o += nE * LBE * LBE * nA;
-  {  // S_lm of a batch, later the half-contracted gamma of one (l, alpha)
-    const int r = kLinkBatch * nA * nA, y = (2 * nE - 1) * (LB + 1) * nc;
-    s.rsh = o; o += r > y ? r : y;
+  {  // W, later the radial table
+    const int t = nE * LBE * LBE * (LB + 1);
+    s.T = s.W = o; o += t > ncAB ? t : ncAB;
+  }
+  {  // S_lm of a batch, later the half-contracted gamma of one (l, alpha) or the half-shifted block
+    const int r = kLinkBatch * nA * nA, y = (2 * nE - 1) * (LB + 1) * nc, h = nct * nc;
+    s.rsh = s.J = o; o += r > y ? (r > h ? r : h) : (y > h ? y : h);
   }
   s.fac = o; o += 2 * kShiftTerms * nct;
   s.dir = o; o += kLinkBatch * 4;
-  s.W = o; o += ncAB;
   s.H = o; o += ncAB;
   s.total = o;
   return s;
@@ -599,7 +600,8 @@ template <bool kExact>
 static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSmem &Lm, double *sm) {
   const int tid = threadIdx.x, NT = blockDim.x, la = U.la, lb = U.lb, lpa = U.lpa, lpb = U.lpb, nca = NCUM(la),
             ncb = NCUM(lb), Lc = U.Lc;
-  const int nA = 2 * J.maxLBS + 1, LE = J.maxLECP > 0 ? J.maxLECP : 1, LBE = J.maxLBS + LE;
+  // (l1 + l2 + l3 is even: every other l3 in a row)
+  const int nT = J.maxLBS + 1, LE = J.maxLECP > 0 ? J.maxLECP : 1, LBE = J.maxLBS + LE;
   const size_t cA = (size_t)U.c * J.nAtoms + U.A, cB = (size_t)U.c * J.nAtoms + U.B;
   double *chi = sm + Lm.chi, *Jsh = sm + Lm.J, *T = sm + Lm.T, *H = sm + Lm.H;
   double *out1 = J.out + (size_t)U.c * J.centreStride + J.pairOff[U.pr];
@@ -611,9 +613,9 @@ static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSme
     chi[e] = H[J.ijkIdx[((ei[0] + ej[0]) * dd + (ei[1] + ej[1])) * dd + ei[2] + ej[2]]];
   }
   // the radial table of type 2
-  auto tidx = [&](int l, int l1, int l2, int l3) { return ((l * LBE + l1) * LBE + l2) * nA + l3; };
+  auto tidx = [&](int l, int l1, int l2, int l3) { return ((l * LBE + l1) * LBE + l2) * nT + (l3 >> 1); };
 #pragma unroll 1
-  for (int e = tid; e < LE * LBE * LBE * nA; e += NT) T[e] = 0.0;
+  for (int e = tid; e < LE * LBE * LBE * nT; e += NT) T[e] = 0.0;
   __syncthreads();
   {
     const double *Tq = (const double *)(U.scr + U.L.T), *part = (const double *)(U.scr + U.L.part);
@@ -797,7 +799,7 @@ static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSme
             const double *t = T + tidx(l, l1, lo2, alpha + beta);
             double v = 0.0;
 #pragma unroll 1
-            for (int l2 = lo2; l2 <= l + beta; l2 += 2, B += 2 * (size_t)LMd * AC, t += 2 * nA) v = fma(*B, *t, v);
+            for (int l2 = lo2; l2 <= l + beta; l2 += 2, B += 2 * (size_t)LMd * AC, t += 2 * nT) v = fma(*B, *t, v);
             Y[e] = v;
           }
           __syncthreads();
