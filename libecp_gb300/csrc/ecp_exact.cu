@@ -60,6 +60,7 @@ static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem 
   }
   double *Qout = (double *)(U.scr + U.L.Q) + (size_t)perm[p0 + g] * nq + qi;
   double I = 0, p = 0, q = 0, T = 0;
+  int *quad = (int *)(sm + L.quad);  // the running quadratures, by rank
   bool done = !mine;
   int k = -2, cnt = 0, lvEnd = 1;
   if (kZero) {
@@ -106,34 +107,52 @@ static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem 
       }
     }
     __syncwarp();
+    // the lanes dealt to the running quadratures: P points' products side by side,
+    // added in the reference's order by the quadrature's own lane
+    const unsigned act = __ballot_sync(0xffffffffu, !done);
+    const LaneDeal D = deal_lanes(__popc(act));
+    const int rank = __popc(act & ((1u << lane) - 1u)), src = rank * D.P;
+    if (!done) quad[rank] = g | l1 << 8 | l2 << 16;
+    __syncwarp();
+    const bool work = D.rank < __popc(act);
+    const int qd = work ? quad[D.rank] : 0;
+    const int oW = lq + ((qd >> 8) & 255), oK = qd >> 16;
 #pragma unroll 1
-    for (int t = s0; t < s1; t++) {
-      const int n = c93_slot[t];
-      if (!done && n >= ws && n < we) {
-        const double *e = tab + ((t - s0) * G + g) * TS;
-        if (e[2 * lq] != 0.0) T += J.wSmall[n] * (e[lq + l1] * e[l2] * e[2 * lq]);
-      }
-      cnt += (t & 1) ? n >= ws : n <= we;
-      if (t > 2 && !(t & 1)) {  // the reference's order: pair by pair
-        I += T;
-        T = 0.0;
-      }
-      if (t + 1 < lvEnd) continue;
-      if (!done) {
-        double res;
-        if (k == -2) p = T;
-        else if (k == -1) {
-          q = T;
-          I = p + q;
-        } else if (ps93_exact(k, J.tol, cnt, I, p, q, res)) {
-          done = true;
-          *Qout = res;
+    for (int t0 = s0; t0 < s1; t0 += D.P) {
+      double v = 0.0;
+      if (work && t0 + D.part < s1) {
+        const int n = __ldg(J.s93 + t0 + D.part);
+        if (n >= ws && n < we) {
+          const double *e = tab + ((t0 + D.part - s0) * G + (qd & 255)) * TS;
+          if (e[2 * lq] != 0.0) v = J.wSmall[n] * (e[oW] * e[oK] * e[2 * lq]);
         }
       }
-      T = 0.0;
-      k++;
-      lvEnd = k < 0 ? 3 : c93_lvEnd[k];  // k <= the level count, inside the 32-entry table
-      cnt = 0;
+#pragma unroll 1
+      for (int j = 0; j < D.P && t0 + j < s1; j++) {
+        const int t = t0 + j, n = c93_slot[t];
+        if (n >= ws && n < we) T += __shfl_sync(0xffffffffu, v, (src + j) & 31);
+        cnt += (t & 1) ? n >= ws : n <= we;
+        if (t > 2 && !(t & 1)) {  // the reference's order: pair by pair
+          I += T;
+          T = 0.0;
+        }
+        if (t + 1 < lvEnd) continue;
+        if (!done) {
+          double res;
+          if (k == -2) p = T;
+          else if (k == -1) {
+            q = T;
+            I = p + q;
+          } else if (ps93_exact(k, J.tol, cnt, I, p, q, res)) {
+            done = true;
+            *Qout = res;
+          }
+        }
+        T = 0.0;
+        k++;
+        lvEnd = k < 0 ? 3 : c93_lvEnd[k];  // k <= the level count, inside the 32-entry table
+        cnt = 0;
+      }
     }
     __syncwarp();
     s0 = s1;
@@ -208,15 +227,18 @@ __global__ void __launch_bounds__(32, 16) k_exact_small(DevJob J) {
 
 // --------------------------------------------------- stage 3: the large grid
 
-// PSM92 walk (src/gc_integrators.c:39-86) over the slots [s0, s1) whose bit is
-// set in `bits`, in the reference's operation order.  The other slots
-// integrate to exactly zero, and adding zero changes no sum.
+// PSM92 walk (src/gc_integrators.c:39-86) over the slots [s0, s1), of which
+// slots[0 .. nE) have an integrand that is not zero (adding zero changes no sum), in
+// the reference's operation order.  D.P lanes evaluate a quadrature's points side by
+// side, val(x) of entry x for the quadrature of the lane's deal; the lane that holds
+// the quadrature of rank src / D.P adds them up.
 template <class V, class Vis>
-static __device__ inline void psm92_exact(int s0, int s1, const unsigned *bits, double tol, V val, Vis vis, double &I,
-                                          double &p, double &q, bool &done, double &res) {
-  int pos = s0, k = s0 == 0 ? -1 : level_of(s0);
+static __device__ inline void psm92_exact(int s0, int s1, const int *slots, int nE, const LaneDeal &D, int src,
+                                          double tol, V val, Vis vis, double &I, double &p, double &q, bool &done,
+                                          double &res) {
+  int pos = s0, i = 0, k = s0 == 0 ? -1 : level_of(s0);
 #pragma unroll 1
-  while (pos < s1 && !done) {
+  while (pos < s1) {
     const int lvStart = k <= 0 ? 1 : c92_lvEnd[k - 1], lvE = k < 0 ? 1 : c92_lvEnd[k];
     if (pos == lvStart && k >= 0) {
       q = 2 * p;
@@ -226,26 +248,27 @@ static __device__ inline void psm92_exact(int s0, int s1, const unsigned *bits, 
     double T = 0.0;
     int last = -1;  // the (lower, upper) pair T belongs to
 #pragma unroll 1
-    for (int w = pos >> 5; (w << 5) < stop; w++) {
-      unsigned word = bits[w];
-      if (w == (pos >> 5)) word &= ~0u << (pos & 31);
-      if ((w << 5) + 32 > stop) word &= ~(~0u << (stop & 31));
+    while (i < nE && slots[i] < stop) {
+      int m = 1;
+      while (m < D.P && i + m < nE && slots[i + m] < stop) m++;
+      const double v = D.part < m ? val(i + D.part) : 0.0;
 #pragma unroll 1
-      for (; word; word &= word - 1u) {
-        const int t = (w << 5) + __ffs(word) - 1, pr = (t + 1) >> 1;
+      for (int j = 0; j < m; j++, i++) {
+        const int t = slots[i], pr = (t + 1) >> 1;
         if (pr != last) {
           I += T;
           T = 0.0;
           last = pr;
         }
-        if ((t & 1) || t == 0 || vis(t)) T += val(t);
+        const double x = __shfl_sync(0xffffffffu, v, (src + j) & 31);
+        if ((t & 1) || t == 0 || vis(t)) T += x;
       }
     }
     I += T;
     pos = stop;
     if (pos == lvE) {
       if (k < 0) p = I;
-      else {
+      else if (!done) {
         const double N3 = c92_3N[k], e = I - p;
         if (16 * e * e <= N3 * fabs(I - q) * tol) {
           res = 16 * I / N3;
@@ -254,6 +277,7 @@ static __device__ inline void psm92_exact(int s0, int s1, const unsigned *bits, 
       }
       k++;
     }
+    if (__all_sync(0xffffffffu, done)) break;
   }
 }
 
@@ -264,7 +288,7 @@ static __device__ void x1_large(const DevJob &J, const Unit &U, const LargeSmem 
   const int lane = threadIdx.x & 31, lab = U.lab, lq = lab + 1, O = kSmallOrder, OL = J.largeOrder, TS = 1 + 2 * lq;
   const int Nb = U.Nb, ws = U.ws, we = U.we, c = U.c, Lc = U.Lc;
   double *tab = sm + L.tab;
-  unsigned *bits = (unsigned *)(sm + L.bits);
+  int *slots = (int *)(sm + L.pend), *quad = (int *)(sm + L.fail);  // the step's entries; the running quadratures
   const double *uL = J.uL + (size_t)c * O;
   const double dAC = U.gA[3], dBC = U.gB[3];
   const bool fail = mask >> lane & 1u;
@@ -355,21 +379,23 @@ static __device__ void x1_large(const DevJob &J, const Unit &U, const LargeSmem 
         }
       }
     }
-    // bits of the step, at its slots' positions
-    const unsigned b = __ballot_sync(0xffffffffu, any);
-    if (lane == 0) {
-      bits[s0 >> 5] = s0 & 31 ? (bits[s0 >> 5] & ((1u << (s0 & 31)) - 1u)) | b << (s0 & 31) : b;
-      if (s0 & 31) bits[(s0 >> 5) + 1] = b >> (32 - (s0 & 31));
-    }
+    const unsigned b = __ballot_sync(0xffffffffu, any), act = __ballot_sync(0xffffffffu, !done);
+    const unsigned below = (1u << lane) - 1u;
+    const LaneDeal D = deal_lanes(__popc(act));
+    const int rank = __popc(act & below), src = rank * D.P;
+    if (any) slots[__popc(b & below)] = t;
+    if (!done) quad[rank] = l1 | l2 << 16;
     __syncwarp();
-    if (!done) {
-      auto vis = [&](int t) { return c92_slot[t] <= end; };
-      auto val = [&](int t) {
-        const double *e = tab + (t - s0) * TS;
-        return J.wLarge[c92_slot[t]] * i1 * (e[lq + l1] * e[l2] * e[2 * lq]);
-      };
-      psm92_exact(s0, s1, bits, J.tol, val, vis, I, p, q, done, res);
-    }
+    const bool work = D.rank < __popc(act);
+    const int qd = work ? quad[D.rank] : 0;
+    const int oW = lq + (qd & 0xffff), oK = qd >> 16;
+    auto vis = [&](int t) { return c92_slot[t] <= end; };
+    auto val = [&](int x) {
+      const int t = slots[x];
+      const double *e = tab + (t - s0) * TS;
+      return work ? J.wLarge[__ldg(J.s92 + t)] * i1 * (e[oW] * e[oK] * e[2 * lq]) : 0.0;
+    };
+    psm92_exact(s0, s1, slots, __popc(b), D, src, J.tol, val, vis, I, p, q, done, res);
     __syncwarp();
     s0 = s1;
     if (__all_sync(0xffffffffu, done)) break;
@@ -396,8 +422,8 @@ static __device__ void x2_large(const DevJob &J, const Unit &U, const LargeSmem 
   double *dst = U.NP == 1 ? (double *)(U.scr + U.L.T)
                           : (double *)(U.scr + U.L.part) + (size_t)k * class_items(J, U.cls * LE, LE);
   double *tab = sm + L.tab, *sI = sm + L.I, *sP = sm + L.P, *sQ = sm + L.Q;
-  int *fail = (int *)(sm + L.fail), *pend = (int *)(sm + L.pend), *pref = (int *)(sm + L.pref);
-  unsigned *needBits = (unsigned *)(sm + L.bits);
+  int *fail = (int *)(sm + L.fail), *pend = (int *)(sm + L.pend);
+  unsigned char *act = (unsigned char *)(sm + L.act);  // the running items
   const double dAC = U.gA[3], dBC = U.gB[3];
   const double za = U.pzA[k / Nb], zb = U.pzB[k % Nb];
   const double Ck = zeta_times(zeta_times(U.pcA[k / Nb] * U.pcB[k % Nb], za, U.pa0), zb, U.pb0);
@@ -456,12 +482,12 @@ static __device__ void x2_large(const DevJob &J, const Unit &U, const LargeSmem 
     pL2 = __reduce_max_sync(0xffffffffu, pL2);
     pL3 = __reduce_max_sync(0xffffffffu, pL3);
 #pragma unroll 1
-    for (int q = lane; q < nf; q += 32) { sI[q] = 0; sP[q] = 0; sQ[q] = 0; }
-#pragma unroll 1
-    for (int w = lane; w < (OL + 31) / 32; w += 32) needBits[w] = 0u;
+    for (int q = lane; q < nf; q += 32) {
+      act[q] = (unsigned char)q;
+      sI[q] = sP[q] = sQ[q] = 0;
+    }
     __syncwarp();
-    unsigned doneBits[kWalkCap / 32] = {0u, 0u, 0u, 0u};
-    int cpos = 0, wpos = 0, nPend = 0;
+    int cpos = 0, wpos = 0, nPend = 0, nAct = nf;
 #pragma unroll 1
     while (wpos < OL) {
       // classify slots step by step, queue the needed ones
@@ -479,10 +505,7 @@ static __device__ void x2_large(const DevJob &J, const Unit &U, const LargeSmem 
           }
         }
         const unsigned m = __ballot_sync(0xffffffffu, need);
-        if (need) {
-          pend[nPend + __popc(m & below)] = t;
-          atomicOr(&needBits[t >> 5], 1u << (t & 31));
-        }
+        if (need) pend[nPend + __popc(m & below)] = t;
         nPend += __popc(m);
         cpos = c1;
       }
@@ -512,44 +535,50 @@ static __device__ void x2_large(const DevJob &J, const Unit &U, const LargeSmem 
 #pragma unroll 1
         for (int l = 1; l <= pL3; l++) R[l] = r * R[l - 1];
       }
-      if (lane == 0) {  // entry of slot t: queued slots in [wpos, t)
-        const int w0 = wpos >> 5, w1 = (b - 1) >> 5;
-        int acc = -__popc(needBits[w0] & ((1u << (wpos & 31)) - 1u));
-#pragma unroll 1
-        for (int w = w0; w <= w1; w++) {
-          pref[w] = acc;
-          acc += __popc(needBits[w]);
-        }
-      }
       __syncwarp();
-      bool all = true;
       unsigned nMask = 0u;
-      int n1 = 0, n2 = 0, n3 = 0;
+      int n1 = 0, n2 = 0, n3 = 0, left = 0;
+      // the running items, 32 at a time, the last ones by several lanes each
 #pragma unroll 1
-      for (int q = lane, qi = 0; q < nf; q += 32, qi++) {
-        if (doneBits[qi] & (1u << lane)) continue;
-        const int v = fail[q], l = v & 255, l1 = (v >> 8) & 255, l2 = (v >> 16) & 255, l3 = v >> 24;
-        auto val = [&](int t) {
-          const double *Uc = tab + (pref[t >> 5] + __popc(needBits[t >> 5] & ((1u << (t & 31)) - 1u))) * TS,
-                       *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
-          return Kb[LBE + 1] * (Uc[l] * R[l3] * Ka[l1] * Kb[l2] * Kb[LBE]);
+      for (int i0 = 0; i0 < nAct;) {
+        const LaneDeal D = deal_lanes(nAct - i0);
+        const bool work = i0 + D.rank < nAct;  // the item the lane evaluates
+        const int v = work ? fail[act[i0 + D.rank]] : 0;
+        const double *eU = tab + (v & 255), *eR = tab + LE + (v >> 24), *eA = tab + LE + nA + ((v >> 8) & 255),
+                     *eB = tab + LE + nA + LBE + ((v >> 16) & 255), *eK = tab + LE + nA + 2 * LBE;
+        auto val = [&](int x) {
+          const int o = x * TS;
+          return work ? eK[o + 1] * (eU[o] * eR[o] * eA[o] * eB[o] * eK[o]) : 0.0;
         };
         auto vis = [&](int t) { return c92_slot[t] <= end; };
+        // the item whose sums the lane holds
+        const bool mine = lane < 32 / D.P && i0 + lane < nAct;
+        const int q = mine ? act[i0 + lane] : 0;
         double I = sI[q], p = sP[q], qv = sQ[q], res = 0;
-        bool done = false;
-        psm92_exact(wpos, b, needBits, J.tol, val, vis, I, p, qv, done, res);
-        sI[q] = done ? res : I;
-        sP[q] = p;
-        sQ[q] = qv;
-        if (done) doneBits[qi] |= 1u << lane;
-        else {
-          all = false;
-          nMask |= 1u << l;
+        bool done = !mine;
+        psm92_exact(wpos, b, pend, nE, D, lane * D.P, J.tol, val, vis, I, p, qv, done, res);
+        __syncwarp();
+        if (mine) {
+          sI[q] = done ? res : I;
+          sP[q] = p;
+          sQ[q] = qv;
+        }
+        const bool keep = mine && !done;
+        if (keep) {
+          const int u = fail[q], l1 = (u >> 8) & 255, l2 = (u >> 16) & 255, l3 = u >> 24;
+          nMask |= 1u << (u & 255);
           n1 = l1 > n1 ? l1 : n1;
           n2 = l2 > n2 ? l2 : n2;
           n3 = l3 > n3 ? l3 : n3;
         }
+        // the list shrinks in place
+        const unsigned km = __ballot_sync(0xffffffffu, keep);
+        if (keep) act[left + __popc(km & below)] = (unsigned char)q;
+        left += __popc(km);
+        i0 += 32 / D.P;
+        __syncwarp();
       }
+      nAct = left;
       pMask = __reduce_or_sync(0xffffffffu, nMask);
       pL1 = __reduce_max_sync(0xffffffffu, n1);
       pL2 = __reduce_max_sync(0xffffffffu, n2);
@@ -563,15 +592,14 @@ static __device__ void x2_large(const DevJob &J, const Unit &U, const LargeSmem 
       nPend = rest;
       wpos = b;
       __syncwarp();
-      if (__all_sync(0xffffffffu, all)) break;
+      if (nAct == 0) break;
     }
     const double N3 = c92_3N[c92_nLevels - 1];
 #pragma unroll 1
-    for (int q = lane, qi = 0; q < nf; q += 32, qi++)
-      if (!(doneBits[qi] & (1u << lane))) {
-        sI[q] = 16 * sI[q] / N3;
-        atomicOr(&((UnitHead *)U.scr)->warn, 2);
-      }
+    for (int i = lane; i < nAct; i += 32) {
+      sI[act[i]] = 16 * sI[act[i]] / N3;
+      atomicOr(&((UnitHead *)U.scr)->warn, 2);
+    }
     __syncwarp();
     int at = 0;
 #pragma unroll 1

@@ -302,18 +302,6 @@ static __device__ inline double ps93_result(const Ps93 &S, const LevelTab &L, in
   return xs_scaled(S.q, {L.rm[k], L.re[k]});
 }
 
-// Lanes of a warp dealt to n running quadratures: P = 2^b lanes each, so that
-// a run of points is summed by P lanes side by side (the sums of 57-bit
-// integers then combine by shuffles).
-struct LaneDeal {
-  int P;     // lanes per quadrature
-  int rank;  // the quadrature this lane works for, n or more: none
-  int part;  // which of its P lanes
-};
-static __device__ inline LaneDeal deal_lanes(int n) {
-  const int b = n > 16 ? 0 : n > 8 ? 1 : n > 4 ? 2 : 3, lane = threadIdx.x & 31;
-  return {1 << b, lane >> b, lane & ((1 << b) - 1)};
-}
 static __device__ inline xs combine(xs a, int P) {
 #pragma unroll 1
   for (int o = 1; o < P; o <<= 1) {

@@ -18,8 +18,6 @@ namespace ecpgb {
 
 constexpr int kWalkCap = 128;  // large-grid quadratures per pass
 constexpr int kLargeWarps = 2; // most warps a CTA of the batched large-grid stage
-constexpr int kLargeWords = (kMaxLargeOrder + 1) / 32;  // bitmap words over the large grid (128, even)
-static_assert(kLargeWords * 32 >= kMaxLargeOrder && kLargeWords % 2 == 0, "large-grid bitmap size");
 
 // Small-grid prefactor of a type-1 primitive pair, C1 = ca cb exp(zd2) with
 // zd2 = -za dAC^2 - zb dBC^2 (src/type1.c:235-246), rounded as the reference
@@ -230,12 +228,12 @@ __host__ __device__ inline SmallSmem small_layout(int LB, int rows, int cap) {
   s.total = s.tab + tt;
   return s;
 }
-// Large grid (one warp a CTA): type 1 a 32-slot table; type 2 a 32-slot table
-// (U[nE], R[nA], Ka[LBE], Kb[LBE], and on the plain path the exponential and
-// the weight), the walkers' state, the needed-slot bitmap
-// with word prefixes, the pending slots and the failed items.
+// Large grid: type 1 a 32-slot table a warp; type 2 a 32-slot table (U[nE],
+// R[nA], Ka[LBE], Kb[LBE], on the plain path the exponential and the weight, on the
+// batched path 16-bit exponents after it), the quadratures' state, the running
+// ones, the pending slots and the failed items.
 struct LargeSmem {
-  int tab, tabT1, I, P, Q, E, part, act, bits, pend, pref, fail, red, total, tabStride, expStride;
+  int tab, tabT1, I, P, Q, E, part, act, pend, fail, red, total, tabStride, expStride;
 };
 __host__ __device__ inline LargeSmem large_layout(int LB, int LE, bool exact) {
   LargeSmem s{};
@@ -252,12 +250,9 @@ __host__ __device__ inline LargeSmem large_layout(int LB, int LE, bool exact) {
   s.Q = o; o += kWalkCap;
   s.part = o; o += kWalkCap;
   s.pend = o; o += 32 * (exact ? 1 : kLargeWarps);
-  if (exact) {  // needed-slot bitmap and word prefixes
-    s.bits = o; o += kLargeWords / 2;
-    s.pref = o; o += kLargeWords / 2;
-  } else {  // exponents and list of the running items
+  s.act = o; o += kWalkCap / 8;
+  if (!exact) {  // exponents of the running items, what two warps tell each other
     s.E = o; o += kWalkCap;
-    s.act = o; o += kWalkCap / 8;
     s.red = o; o += 2 * kLargeWarps;
   }
   s.fail = o; o += kWalkCap / 2;
@@ -365,6 +360,19 @@ static __device__ inline int unit_item(const DevJob &J, const Unit &U, int q) {
 
 // Work lists of a chunk and their counters (zeroed before the chunk).
 enum { kCntT1, kCntRest, kCntT2, kCntFail, kCntPart, kHeadSmall, kHeadLarge, kCounters };
+
+// Lanes of a warp dealt to n running quadratures: P = 2^b lanes each, which
+// evaluate P points side by side (the batched path's integer sums then combine by
+// shuffles; the plain path's values are added in order).
+struct LaneDeal {
+  int P;     // lanes per quadrature
+  int rank;  // the quadrature this lane works for, n or more: none
+  int part;  // which of its P lanes
+};
+static __device__ inline LaneDeal deal_lanes(int n) {
+  const int b = n > 16 ? 0 : n > 8 ? 1 : n > 4 ? 2 : 3, lane = threadIdx.x & 31;
+  return {1 << b, lane >> b, lane & ((1 << b) - 1)};
+}
 
 // The next entry of a list for a warp; its index to every lane.
 static __device__ inline int next_item(unsigned *head) {
