@@ -205,11 +205,32 @@ static __device__ inline UnitShift unit_shift(const DevJob &J, int pr, int la, i
 }
 
 // r^n for the ECP exponent n (a double in the interface; integers are the norm).
+// 0, 1 and 2 are told apart by their bits: a comparison of doubles is an
+// instruction of the FP64 pipe.
 static __device__ inline double rpow(double r, double n) {
-  if (n == 0.0) return 1.0;
-  if (n == 1.0) return r;
-  if (n == 2.0) return r * r;
+  const long long b = __double_as_longlong(n);
+  if (b << 1 == 0) return 1.0;
+  if (b == 0x3ff0000000000000ll) return r;
+  if (b == 0x4000000000000000ll) return r * r;
   return pow(r, n);
+}
+
+// Whether a term D r^n exp(-x) leaves pot as it is, bit for bit: D r^n below 2^u,
+// exp(-x) at most 2^-q by x's high word, and the product below a 2^-58th of pot
+// (or of the smallest double).  By integers, beside the 20-odd FP64 instructions of
+// the exponential that it saves.
+static __device__ inline bool ecp_term_lost(double pot, double D, double x, double n, double r, double r2) {
+  const unsigned hx = (unsigned)__double2hiint(x), hD = (unsigned)__double2hiint(D) & 0x7fffffffu;
+  const long long nb = __double_as_longlong(n);
+  if (hx >= 0x7ff00000u || hD >= 0x7ff00000u) return false;  // negative, infinite, NaN
+  int u = (int)(hD >> 20) - 1022;
+  if (nb == 0x3ff0000000000000ll) u += (__double2hiint(r) >> 20) - 1022;
+  else if (nb == 0x4000000000000000ll) u += (__double2hiint(r2) >> 20) - 1022;
+  else if (nb << 1 != 0) return false;
+  const int e = (int)(hx >> 20) - 1023;
+  const unsigned y = ((hx & 0xfffffu) | 0x100000u) * 1477u;  // log2(e) from below, Q30 2^-e
+  const int q = e < 0 ? 0 : e > 10 ? 4096 : (int)(y >> (30 - e));
+  return u - q < (__double2hiint(pot) >> 20 & 0x7ff) - 1023 - 58;
 }
 
 // U_l(r) of centre c (src/ecp.c:42-60).
@@ -218,7 +239,10 @@ static __device__ double eval_ecp(const DevJob &J, int c, int l, double r) {
   if (J.chanT0) {  // the channel's terms, in order
     const int *ch = J.chanT0 + c * (kMaxLEcp + 2) + l;
 #pragma unroll 1
-    for (int t = ch[0], t1 = ch[1]; t < t1; t++) pot += rpow(r, J.termN[t]) * J.termD[t] * exp(-J.termA[t] * r2);
+    for (int t = ch[0], t1 = ch[1]; t < t1; t++) {
+      const double D = J.termD[t], n = J.termN[t], x = J.termA[t] * r2;
+      if (!ecp_term_lost(pot, D, x, n, r, r2)) pot += rpow(r, n) * D * exp(-x);
+    }
     return pot;
   }
   int t0 = J.ctrT0[c], t1 = t0 + J.ctrNT[c];
