@@ -1610,7 +1610,7 @@ __global__ void __launch_bounds__(kLinkThreadsMax) k_unit_link(DevJob J) {
         while (r >= 2 * l + 1) { r -= 2 * l + 1; l -= 2; }
         const double *q = Q + (size_t)b0 * nq + t1_index(Lm1, l), *s = rsh + l * l + r;
         double v = W[e];
-#pragma unroll 1
+#pragma unroll 4
         for (int g = 0; g < nb; g++) v += s[g * RQ] * q[(size_t)g * nq];
         W[e] = v;
       }
@@ -1625,7 +1625,7 @@ __global__ void __launch_bounds__(kLinkThreadsMax) k_unit_link(DevJob J) {
       double acc = 0.0;
 #pragma unroll 1
       for (int l = lmax; l >= 0; l -= 2) {
-#pragma unroll 1
+#pragma unroll 4
         for (int m = 0; m < 2 * l + 1; m++) acc += p2s[l * l + m] * w[m];
         w += 2 * l + 1;
       }

@@ -799,14 +799,14 @@ static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSme
           __syncthreads();
 #pragma unroll 1
           for (int e = tid; e < M * n1 * ncb; e += NT) {
-            const int q = e % ncb, r = e / ncb, l1 = lo1 + 2 * (r % n1), m = r / n1;
+            const int q = e % ncb, r = e / ncb, l1 = lo1 + 2 * (r / M), m = r % M;
             int beta = 0;
             while (NCUM(beta) <= q) beta++;
             const int lo2 = l > beta ? l - beta : (beta + l) & 1;
             const double *B = angB + ((size_t)lo2 * LMd + l * l + m) * AC + q;
             const double *t = T + tidx(l, l1, lo2, alpha + beta);
             double v = 0.0;
-#pragma unroll 1
+#pragma unroll 4
             for (int l2 = lo2; l2 <= l + beta; l2 += 2, B += 2 * (size_t)LMd * AC, t += 2 * nT) v = fma(*B, *t, v);
             Y[e] = v;
           }
@@ -816,11 +816,11 @@ static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSme
           for (int e = tid; e < NCART(alpha) * ncb; e += NT) {
             const int p = p0 + e / ncb, q = e % ncb;
             double v = 0.0;
+            const double *A = angA + ((size_t)lo1 * LMd + l * l) * AC + p, *y = Y + q;
 #pragma unroll 1
-            for (int m = 0; m < M; m++)
-#pragma unroll 1
-              for (int i = 0; i < n1; i++)
-                v = fma(angA[((size_t)(lo1 + 2 * i) * LMd + l * l + m) * AC + p], Y[(m * n1 + i) * ncb + q], v);
+            for (int i = 0; i < n1; i++, A += 2 * (size_t)LMd * AC, y += M * ncb)
+#pragma unroll 4
+              for (int m = 0; m < M; m++) v = fma(A[(size_t)m * AC], y[m * ncb], v);
             chi[p * ncb + q] += v;
           }
         }
