@@ -481,57 +481,32 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
         // break index, and the point-index interval in which the pair's
         // exponent passes the screen: past both centres the exponent falls with
         // the index; it is a parabola in r with its vertex at V, and r grows with
-        // the index.
-        const double V = (za * dAC + zb * dBC) / (za + zb);
+        // the index.  r within h of the vertex, -zp h^2 - mu = the threshold: bisections
+        // of the abscissae, whose bits are compared as integers (five of the
+        // exponent, at eight FP64 operations a step, were most of this kernel: 190
+        // -> 69 us for 6048 units).  The plain path's stage tests every slot of the
+        // interval itself (a margin of 1), and its break is settled by the exponent as
+        // the reference rounds it.
+        const double V = (za * dAC + zb * dBC) / (za + zb), zp = za + zb, mu = za * zb / zp * (dAC - dBC) * (dAC - dBC);
+        const double m = 1.0 / i1, far = dAC > dBC ? dAC : dBC;
+        const double q = ((kExact ? 1.0 : 0.0) - J.lnAcc2 - mu) / zp, h = sqrt(q > 0.0 ? q : 0.0);
+        const int n0 = first_from(J, (V - h - i2) * m), n1 = first_after(J, (V + h - i2) * m);
+        int brk = first_after(J, (far - i2) * m);
         if constexpr (!kExact) {
-          // r within h of the vertex, -zp h^2 - mu = the threshold: two bisections of
-          // the abscissae, whose bits are compared as integers (five of the
-          // exponent, at eight FP64 operations a step, were most of this kernel: 190
-          // -> 69 us for 6048 units)
-          const double zp = za + zb, mu = za * zb / zp * (dAC - dBC) * (dAC - dBC), q = (-J.lnAcc2 - mu) / zp;
-          const double h = sqrt(q > 0.0 ? q : 0.0), m = 1.0 / i1;
-          const int n0 = first_from(J, (V - h - i2) * m), n1 = first_after(J, (V + h - i2) * m),
-                    n2 = first_after(J, ((dAC > dBC ? dAC : dBC) - i2) * m);
-          const int brk = q >= 0.0 && n1 > n2 ? n1 : n2;
-          win[k] = q >= 0.0 ? make_int4(brk < J.largeOrder ? brk : INT_MAX, n0, n1 - 1, t1Break)
-                            : make_int4(brk < J.largeOrder ? brk : INT_MAX, 1, 0, t1Break);
+          if (q >= 0.0 && n1 > brk) brk = n1;
         } else {
-          // (the stage tests every slot of the interval itself: a margin of 1)
-          const double thr = J.lnAcc2 - 1.0;
-          auto exq = [&](int n, double &r) {
-            r = i1 * J.xLarge[n] + i2;
-            const double d1 = dAC - r, d2 = dBC - r;
-            return -za * d1 * d1 - zb * d2 * d2;
+          const double qb = (-J.lnAcc2 - mu) / zp;
+          const int nb = qb >= 0.0 ? first_after(J, (V + sqrt(qb) - i2) * m) : 0;
+          if (nb > brk) brk = nb;
+          auto past = [&](int n) {
+            const double r = i1 * J.xLarge[n] + i2, d1 = dAC - r, d2 = dBC - r;
+            return r > dAC && r > dBC && -za * d1 * d1 - zb * d2 * d2 < J.lnAcc2;
           };
-          double r;
-          int lo = 0, hi = J.largeOrder;
-          while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            const double e = exq(mid, r);
-            if (r > dAC && r > dBC && e < J.lnAcc2) hi = mid; else lo = mid + 1;
-          }
-          const int brk = lo < J.largeOrder ? lo : INT_MAX;
-          int a = 0, b = J.largeOrder;
-          while (a < b) {
-            const int mid = (a + b) >> 1;
-            if (i1 * J.xLarge[mid] + i2 >= V) b = mid; else a = mid + 1;
-          }
-          const int nv = a;
-          a = 0;
-          b = nv;
-          while (a < b) {
-            const int mid = (a + b) >> 1;
-            if (exq(mid, r) >= thr) b = mid; else a = mid + 1;
-          }
-          const int nLo = a;
-          a = nv;
-          b = J.largeOrder;
-          while (a < b) {
-            const int mid = (a + b) >> 1;
-            if (exq(mid, r) < thr) b = mid; else a = mid + 1;
-          }
-          win[k] = make_int4(brk, nLo, a - 1, 0);
+          while (brk < J.largeOrder && !past(brk)) brk++;
+          while (brk > 0 && past(brk - 1)) brk--;
         }
+        if (brk >= J.largeOrder) brk = INT_MAX;
+        win[k] = q >= 0.0 ? make_int4(brk, n0, n1 - 1, t1Break) : make_int4(brk, 1, 0, t1Break);
       } else {
         win[k] = make_int4(INT_MAX, 1, 0, t1Break);
       }
