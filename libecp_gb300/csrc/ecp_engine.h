@@ -90,7 +90,7 @@ struct DevJob {
   const int *byN93;            // small-grid slots (with point << 16) step by step in ascending point order
   // mixed path: tables as float pairs (ecp_ff.h)
   const ff *besHf, *besAf, *besZf;  // besH, besA, besZ
-  const ff *xLf, *wLf;              // large grid abscissae and weights
+  const ff *wLf;                    // large grid weights
   const ff *termAf, *termDf;        // ECP term exponents and coefficients
   const double *besZ;          // Bessel table abscissae i / (besselN / 16)
   int besHL;

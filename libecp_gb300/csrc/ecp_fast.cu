@@ -211,17 +211,7 @@ static __device__ inline ff ecp_term_ff(const DevJob &J, int t, ff r, ff r2) {
   return ff_mul(v, ff_from_double(rpow(ff_to_double(r), n)));  // other powers: rare
 }
 
-// U_l(r) in ff for the channels set in mask (the others untouched).
-static __device__ __noinline__ void channels_ff(const DevJob &J, int c, ff r, unsigned mask, ff *U) {
-  const ff r2 = ff_mul(r, r);
-  for (unsigned m = mask; m; m &= m - 1) U[__ffs(m) - 1] = {0.0f, 0.0f};
-  const int t0 = J.ctrT0[c], t1 = t0 + J.ctrNT[c];
-  for (int t = t0; t < t1; t++) {
-    const int l = J.termL[t];
-    if (mask >> l & 1u) U[l] = ff_add(U[l], ecp_term_ff(J, t, r, r2));
-  }
-}
-
+// U_l(r) in ff.
 static __device__ __noinline__ ff channel_ff(const DevJob &J, int c, int l, ff r) {
   const ff r2 = ff_mul(r, r);
   ff pot = {0.0f, 0.0f};
@@ -354,38 +344,6 @@ static __device__ inline void psm92_advance_ff(int s0, int s1, double tol, V val
     }
   }
   I += acc.value();
-}
-
-// psm92_advance_ff over the queued slots pend[0 .. nE), which lie in [s0, s1);
-// val(i) of entry i.
-template <class V>
-static __device__ inline void psm92_queue_ff(int s0, int s1, const int *pend, int nE, double tol, V val, double &I,
-                                             double &p, double &q, bool &done, double &res) {
-  int i = 0, pos = s0, k = s0 == 0 ? -1 : level_of(s0);
-#pragma unroll 1
-  while (pos < s1 && !done) {
-    const int lvStart = k <= 0 ? 1 : c92_lvEnd[k - 1], lvE = k < 0 ? 1 : c92_lvEnd[k];
-    if (pos == lvStart && k >= 0) {
-      q = 2 * p;
-      p = 2 * I;
-    }
-    pos = lvE < s1 ? lvE : s1;
-    ff_acc acc;
-#pragma unroll 1
-    for (; i < nE && pend[i] < pos; i++) acc.add(val(i));
-    I += acc.value();
-    if (pos == lvE) {
-      if (k < 0) p = I;
-      else {
-        const double N3 = c92_3N[k], e = I - p;
-        if (16 * e * e <= N3 * fabs(I - q) * tol) {
-          res = 16 * I / N3;
-          done = true;
-        }
-      }
-      k++;
-    }
-  }
 }
 
 PairPlan pair_plan(int NP, int la, int lb, int nItems, bool single) {
@@ -779,7 +737,6 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
 // sign: three signs fit the low bits of a sum), so a point costs a quadrature
 // two products and one sum.  The lanes are dealt to the running quadratures,
 // again whenever half of them have converged.
-template <bool kMixed>
 static __device__ void t2_small(const DevJob &J, const Unit &U, const LevelTab &V, u64 *tab, int *quad, int q0) {
   const int lane = threadIdx.x & 31, O = kSmallOrder, nF = J.nF, nk = J.nk, LE = J.maxLECP > 0 ? J.maxLECP : 1,
             nRuns = J.nRuns > 0 ? J.nRuns : 1, ws = U.ws, we = U.we;
@@ -891,8 +848,6 @@ static __device__ void t2_small(const DevJob &J, const Unit &U, const LevelTab &
   }
   if (!done && D.part == 0) {
     atomicOr((unsigned *)(U.scr + U.L.mask) + (q >> 5), 1u << (q & 31));
-    if (kMixed)
-      atomicMax(&((UnitHead *)U.scr)->est, (u64)__double_as_longlong(fabs(ps93_result(S, V, c93_nLevels - 1))));
   }
 }
 
@@ -912,7 +867,7 @@ __global__ void __launch_bounds__(32, 24) k_unit_small(DevJob J) {
     const int2 it = small_entry(J, i, n0, n1);
     const Unit &U = unit_get(J, it.x);
     if (i >= n1) {
-      t2_small<kMixed>(J, U, V, (u64 *)(sm + L.tab), (int *)(sm + L.quad), it.y);
+      t2_small(J, U, V, (u64 *)(sm + L.tab), (int *)(sm + L.quad), it.y);
       continue;
     }
     const long long t0 = J.classCycles ? clock64() : 0;
@@ -1148,20 +1103,16 @@ struct T2Pass {
   unsigned mask;     // channels they read
   int l1, l2, l3;    // highest Ka, Kb and r^l rows
 };
-template <bool kMixed, int kWarps>
+template <int kWarps>
 static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &L, double *sm, const LevelTab &V,
-                               const T2Pass &S0, int k, int mb, const double2 *map, const int4 *win, bool useFF, int &warn) {
-  // mixed path: useFF picks the double-single tables and sums for this pass
-  // (one copy of the common code for both precisions)
-  const bool inFF = kMixed && useFF;
+                               const T2Pass &S0, int k, int mb, const double2 *map, const int4 *win, int &warn) {
   const int lane = threadIdx.x & 31, warp = kWarps > 1 ? threadIdx.x >> 5 : 0, nA = 2 * J.maxLBS + 1, Nb = U.Nb, c = U.c, nf = S0.nf;
   const int LE = J.maxLECP > 0 ? J.maxLECP : 1, LBE = J.maxLBS + LE, OL = J.largeOrder;
   const int TS = L.tabStride, ES = L.expStride;
   const double *pzA = U.pzA, *pzB = U.pzB;
   const double dAC = U.gA[3], dBC = U.gB[3];
   double *tab = sm + L.tab, *part = sm + L.part;
-  // an item's state: three mantissas (or, in double-single, I, p, q) and the
-  // exponents, 16 bits each
+  // an item's state: three mantissas and the exponents, 16 bits each
   i64 *s0m = (i64 *)(sm + L.I), *s1m = (i64 *)(sm + L.P), *s2m = (i64 *)(sm + L.Q);
   short4 *sE = (short4 *)(sm + L.E);
   const int *fail = (const int *)(sm + L.fail);
@@ -1175,14 +1126,13 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
   const double za = P.za, zb = P.zb, Ck = P.C2;
   const double i1 = map[k].x;
   const double iCk = i1 * Ck;
-  const ff i1f = ff_from_double(i1), Ckf = ff_from_double(Ck);
   const int4 wk = win[k];
   const int nb = wk.x, nLo = wk.y, nHi = wk.z;
 #pragma unroll 1
   for (int i = lane; i * kWarps + warp < nf; i += 32) {
     const int q = i * kWarps + warp;
     act[i] = (unsigned char)q;
-    s0m[q] = s1m[q] = s2m[q] = 0;  // (also 0.0)
+    s0m[q] = s1m[q] = s2m[q] = 0;
     sE[q] = make_short4(kNoExp, kNoExp, kNoExp, 0);
   }
   __syncwarp();
@@ -1251,27 +1201,6 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
       // the Bessel rows of both centres, then the rest: a warp each, or both by one
 #pragma unroll 1
       for (int role = warp; role < 2; role += kWarps) {
-        if (inFF) {
-          // the same rows in double-single
-          ff *Uc = (ff *)e, *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
-          const ff rf = ff_from_double(r);
-          if (role == 0) {
-#pragma unroll 1
-            for (int side = 0; side < 2; side++)
-              bessel_ff(J, side ? pL2 : pL1, ff_mul(ff_from_double(side ? 2.0 * zbj * dBC : 2.0 * zaj * dAC), rf),
-                        side ? Kb : Ka, 1);
-          } else {
-            const ff wB = ff_mul(ff_mul(J.wLf[n], i1f),
-                                 ff_mul(Ckf, ff_exp(ff_from_double((double)exponent(zaj, zbj, r) * 0x1p-53))));
-            channels_ff(J, c, rf, pMask, Uc);
-#pragma unroll 1
-            for (unsigned m = pMask; m; m &= m - 1u) Uc[__ffs(m) - 1] = ff_mul(Uc[__ffs(m) - 1], wB);
-            R[0] = {1.0f, 0.0f};
-#pragma unroll 1
-            for (int l = 1; l <= pL3; l++) R[l] = ff_mul(rf, R[l - 1]);
-          }
-          continue;
-        }
         // mantissas of w Ck e^ex U_l, r^l, K_l1 and K_l2, the
         // exponents in 16 bits, U's with its sign
         u64 *Um = (u64 *)e, *R = Um + LE, *Ka = R + nA, *Kb = Ka + LBE;
@@ -1328,63 +1257,48 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
       const int v = fail[q], l = v & 255, l1 = (v >> 8) & 255, l2 = (v >> 16) & 255, l3 = v >> 24;
       bool done = !work;
       double res = 0;
-      if (inFF) {
-        double I = __longlong_as_double(s0m[q]), p = __longlong_as_double(s1m[q]), qv = __longlong_as_double(s2m[q]);
-        auto val = [&](int i) {
-          const ff *Uc = (const ff *)(tab + i * TS), *R = Uc + LE, *Ka = R + nA, *Kb = Ka + LBE;
-          return ff_mul(ff_mul(ff_mul(Ka[l1], Kb[l2]), Uc[l]), R[l3]);
-        };
-        psm92_queue_ff(wpos, b, pend, nE, J.tol, val, I, p, qv, done, res);
-        __syncwarp();
-        if (work && D.part == 0) {
-          s0m[q] = __double_as_longlong(done ? res : I);
-          s1m[q] = __double_as_longlong(p);
-          s2m[q] = __double_as_longlong(qv);
-        }
-      } else {
-        const short4 e = sE[q];
-        Psm92 S;
-        S.I = {s0m[q], e.x};
-        S.I1 = {s1m[q], e.y};
-        S.I2 = {s2m[q], e.z};
-        const u64 *eU = (const u64 *)tab + l, *eR = (const u64 *)tab + LE + l3, *eA = (const u64 *)tab + LE + nA + l1,
-                  *eB = (const u64 *)tab + LE + nA + LBE + l2;
-        const short *xT = (const short *)(tab + 32 * TS);
-        const int xA = LE + l1, xB = LE + LBE + l2, xR = LE + 2 * LBE + l3;
-        int i = 0, pos = wpos, k = wpos == 0 ? -1 : level_of(wpos);
+      const short4 e = sE[q];
+      Psm92 S;
+      S.I = {s0m[q], e.x};
+      S.I1 = {s1m[q], e.y};
+      S.I2 = {s2m[q], e.z};
+      const u64 *eU = (const u64 *)tab + l, *eR = (const u64 *)tab + LE + l3, *eA = (const u64 *)tab + LE + nA + l1,
+                *eB = (const u64 *)tab + LE + nA + LBE + l2;
+      const short *xT = (const short *)(tab + 32 * TS);
+      const int xA = LE + l1, xB = LE + LBE + l2, xR = LE + 2 * LBE + l3;
+      int i = 0, pos = wpos, k = wpos == 0 ? -1 : level_of(wpos);
 #pragma unroll 1
-        while (pos < b) {
-          const int lvE = k < 0 ? 1 : c92_lvEnd[k];
-          pos = lvE < b ? lvE : b;
-          const int ie = __popc(__ballot_sync(0xffffffffu, myPend < pos));
-          xf_run run;
+      while (pos < b) {
+        const int lvE = k < 0 ? 1 : c92_lvEnd[k];
+        pos = lvE < b ? lvE : b;
+        const int ie = __popc(__ballot_sync(0xffffffffu, myPend < pos));
+        xf_run run;
 #pragma unroll 1
-          for (int x = i + D.part; x < ie; x += D.P) {
-            const short *xe = xT + x * ES;
-            const int ue = xe[l];
-            run.add({mul_hi(mul_hi(eA[x * TS], eB[x * TS]), mul_hi(eU[x * TS], eR[x * TS])),
-                     (ue >> 1) + xe[xA] + xe[xB] + xe[xR] + 3 * 64},
-                    (uint32_t)ue << 31);
-          }
-          i = ie;
-          S.I = xs_plus(S.I, combine(run.sum(), D.P));
-          if (pos == lvE) {
-            if (k < 0) psm92_head(S);
-            else if (!done && psm92_end(S, V, k)) {
-              done = true;
-              res = psm92_result(S, V, k);
-            }
-            k++;
-          }
-          if (__all_sync(0xffffffffu, done)) break;
+        for (int x = i + D.part; x < ie; x += D.P) {
+          const short *xe = xT + x * ES;
+          const int ue = xe[l];
+          run.add({mul_hi(mul_hi(eA[x * TS], eB[x * TS]), mul_hi(eU[x * TS], eR[x * TS])),
+                   (ue >> 1) + xe[xA] + xe[xB] + xe[xR] + 3 * 64},
+                  (uint32_t)ue << 31);
         }
-        __syncwarp();
-        if (work && D.part == 0) {
-          s0m[q] = done ? __double_as_longlong(res) : S.I.m;
-          s1m[q] = S.I1.m;
-          s2m[q] = S.I2.m;
-          sE[q] = make_short4(exp16(S.I.e), exp16(S.I1.e), exp16(S.I2.e), 0);
+        i = ie;
+        S.I = xs_plus(S.I, combine(run.sum(), D.P));
+        if (pos == lvE) {
+          if (k < 0) psm92_head(S);
+          else if (!done && psm92_end(S, V, k)) {
+            done = true;
+            res = psm92_result(S, V, k);
+          }
+          k++;
         }
+        if (__all_sync(0xffffffffu, done)) break;
+      }
+      __syncwarp();
+      if (work && D.part == 0) {
+        s0m[q] = done ? __double_as_longlong(res) : S.I.m;
+        s1m[q] = S.I1.m;
+        s2m[q] = S.I2.m;
+        sE[q] = make_short4(exp16(S.I.e), exp16(S.I1.e), exp16(S.I2.e), 0);
       }
       if (!done) {
         nMask |= 1u << l;
@@ -1433,12 +1347,9 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
 #pragma unroll 1
   for (int i = lane; i < nAct; i += 32) {
     const int q = act[i];
-    if (inFF) part[q] += 16 * __longlong_as_double(s0m[q]) / c92_3N[c92_nLevels - 1];
-    else {
-      Psm92 S;
-      S.I1 = {s1m[q], sE[q].y};
-      part[q] += psm92_result(S, V, c92_nLevels - 1);
-    }
+    Psm92 S;
+    S.I1 = {s1m[q], sE[q].y};
+    part[q] += psm92_result(S, V, c92_nLevels - 1);
     warn = 1;
   }
   __syncwarp();
@@ -1446,7 +1357,7 @@ static __device__ void t2_pair(const DevJob &J, const Unit &U, const LargeSmem &
 
 // The failed type-2 quadratures of a unit over the primitive pairs of one part
 // (src/type2.c:418-528), in passes of up to kWalkCap of them.
-template <bool kMixed, int kWarps>
+template <int kWarps>
 static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem &L, double *sm, const LevelTab &V,
                                 int part) {
   const int lane = threadIdx.x & 31, nIt = U.nItems, LE = J.maxLECP > 0 ? J.maxLECP : 1;
@@ -1458,9 +1369,6 @@ static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem 
   // partial sums of the part, or the results themselves when it is the only one
   double *dst = single ? (double *)(U.scr + U.L.T)
                        : (double *)(U.scr + U.L.part) + (size_t)part * class_items(J, U.cls * LE, LE);
-  // mixed path: double-single tables only where their sums can take the
-  // reference's decisions (ff_limit); larger integrals in FP64
-  const bool useFF = kMixed && __longlong_as_double((i64)((const UnitHead *)U.scr)->est) < ff_limit(J.tol);
   const double2 *map = (const double2 *)(U.scr + U.L.map);
   const int4 *win = (const int4 *)(U.scr + U.L.win);
   // the latest break of the pairs before the part: beyond it no earlier
@@ -1503,7 +1411,7 @@ static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem 
     int mb = mb0, warn = 0;
 #pragma unroll 1
     for (int k = k0; k < k1; k++) {
-      t2_pair<kMixed, kWarps>(J, U, L, sm, V, S, k, mb, map, win, useFF, warn);
+      t2_pair<kWarps>(J, U, L, sm, V, S, k, mb, map, win, warn);
       mb = win[k].x > mb ? win[k].x : mb;
     }
     if (warn) atomicOr(&((UnitHead *)U.scr)->warn, 2);
@@ -1544,7 +1452,7 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) k_unit_large(DevJob 
     if (i >= n2) break;
     const int2 it = J.listPart[i];
     const Unit &U = unit_get(J, it.x);
-    t2_large<kMixed, kWarps>(J, U, L, sm, V, it.y);
+    t2_large<kWarps>(J, U, L, sm, V, it.y);
   }
 #pragma unroll 1
   for (; taken < J.take; taken++, i = n) {

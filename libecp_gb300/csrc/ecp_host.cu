@@ -232,7 +232,7 @@ int parse_system(const ecpgb_system &s, Parsed &P) {
 struct DevTables {
   TableKey key{};
   HostTables host;
-  DBuf<float> besHf, besAf, besZf, xlf, wlf;  // float pairs (mixed path)
+  DBuf<float> besHf, besAf, besZf, wlf;  // float pairs (mixed path)
   DBuf<double> xs, ws, xl, wl, besT, besC, besH, besA, besZ, shNorm, p2s, fac, dfac, omega, c2s;
   DBuf<int> ijk, ijkIdx, itemOff, itemCnt, items, s93, s92, byN93;
   DBuf<long long> besX, besXA;  // fixed-point Bessel rows
@@ -316,7 +316,7 @@ struct Engine {
               t->omega.upload(h.omega, stream) && t->ijk.upload(h.ijk, stream) &&
               t->ijkIdx.upload(h.ijkIndex, stream) && t->besH.upload(h.besselH, stream) && t->besA.upload(h.besselA, stream) && t->besHf.upload(h.besselHf, stream) &&
               t->besAf.upload(h.besselAf, stream) && t->besZf.upload(h.besselZf, stream) &&
-              t->xlf.upload(h.xlf, stream) && t->wlf.upload(h.wlf, stream) &&
+              t->wlf.upload(h.wlf, stream) &&
               t->besZ.upload(h.besselZ, stream) && t->besX.upload(h.besselX, stream) &&
               t->besXA.upload(h.besselXA, stream) &&
               t->c2s.upload(h.cart2sph, stream) && t->s93.upload(h.s93.slot, stream) &&
@@ -786,7 +786,6 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.besHf = (const ff *)T->besHf.p;
   J.besAf = (const ff *)T->besAf.p;
   J.besZf = (const ff *)T->besZf.p;
-  J.xLf = (const ff *)T->xlf.p;
   J.wLf = (const ff *)T->wlf.p;
   J.s93 = T->s93.p;
   J.s92 = T->s92.p;

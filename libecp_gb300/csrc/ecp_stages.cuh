@@ -157,9 +157,8 @@ struct Unit {
   bool live;
 };
 struct UnitHead {
-  u64 est;   // mixed path: largest |estimate| of a failed small-grid item (bits)
   int warn;  // 1: a type-1, 2: a type-2 quadrature ran out of levels
-  int off;   // the scratch's offset in 16 bytes, for the work lists
+  int pad;
   Unit unit;
 };
 // A normal-kind primitive pair's scalars in fixed point: s = |P| as S 2^-q,
@@ -435,7 +434,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
 #pragma unroll 1
   for (int w = lane; w < (U.nItems + 31) / 32; w += 32) mask[w] = 0u;
   const int off = (int)((U.scr - J.scr) >> 4);
-  if (lane == 0) *(UnitHead *)U.scr = {0ull, 0, off, U};
+  if (lane == 0) *(UnitHead *)U.scr = {0, 0, U};
   int cnt[3] = {0, 0, 0};
   unsigned kinds = 0;  // the lane's pairs' kinds, 2 bits each (at most 8)
 #pragma unroll 1

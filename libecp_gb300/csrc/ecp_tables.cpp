@@ -381,7 +381,6 @@ void build_tables(const TableKey &key, HostTables &t) {
   grid_ps93(128, t.xs, t.ws);
   schedule_ps93(128, t.s93);
   grid_psm92(key.largeGridOrder, t.xl, t.wl);
-  split_pairs(t.xl, t.xlf);
   split_pairs(t.wl, t.wlf);
   schedule_psm92((int)t.xl.size(), t.s92);
   t.tabL = t.maxLECP + t.maxAlpha + 6;

@@ -89,7 +89,7 @@ struct HostTables {
   std::vector<long long> besselX, besselXA;
   // mixed-precision path: the tables above split into float pairs (hi, lo)
   // with hi + lo = the double to 48 bits (ecp_ff.h), interleaved
-  std::vector<float> besselHf, besselAf, besselZf, xlf, wlf;
+  std::vector<float> besselHf, besselAf, besselZf, wlf;
   std::vector<double> besselZ;   // table abscissae z_i = i / (besselN / 16), the reference's division
   // Normalisation of the real spherical harmonics, [l][m] for l, m <= tmDim:
   // sqrt((2l+1)/(2 pi)) and sqrt((l-m)!/(l+m)!) times that, computed as
