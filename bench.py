@@ -27,12 +27,12 @@ value   : device-resident job (inputs in HBM before the timed region); per step
 e2e     : ecpgb_getIntegrals (the getIntegrals call with the path chosen) with
           host buffers: one packed H2D copy of the inputs and a D2H copy of the
           matrix per step.
-roofline: the unit kernel against the FP64 FMA pipe measured live (the path is
-          FP64-latency bound; DRAM traffic is a few hundred bytes per unit):
-          achieved = FP64 operations the kernel executed per emitted unit (ncu
-          counts on the cluster's first 8 centres, profiles/roofline_inputs.txt;
-          cluster workload only) x emitted units / the unit kernel's CUDA-event
-          time; alg_* = the reference's algorithmic FLOPs counted by the oracle
+roofline: the unit stages against the FP64 FMA pipe measured live (DRAM traffic
+          is some ten kilobytes per unit; the batched path keeps most of its
+          arithmetic on the integer pipes): achieved = FP64 operations the
+          stages executed per emitted unit (ncu counts on the cluster's first 8
+          centres, profiles/roofline_inputs.txt; cluster workload only) x emitted
+          units / the stages' CUDA-event time; alg_* = the reference's algorithmic FLOPs counted by the oracle
           on its control flow over the CPU-baseline sample.
 cpu_baseline: the oracle restatement (or the reference build where one exists
           on the machine) on a bounded sample of the workload, on all host cores
@@ -369,12 +369,11 @@ def ours(args, rank, world):
         f_unit = algorithmic_flops(st) / max(st["blocks"], 1)
         alg_achieved = f_unit * emitted / (t_unit / 1e3) / 1e12
         peak = peaks["fp64_fma_tflops"]
-        if mode == eg.ECPGB_FP64:
-            kernel = "k_unit"
-        else:
-            kernel = "k_unit_queue" if tuned["chosen"]["queue"] else "k_unit_fast"
-        # executed work: FP64 operations the unit kernel executed per emitted
-        # unit (ncu: 2 DFMA + DMUL + DADD thread instructions of one launch on
+        key = {eg.ECPGB_FP64: "stages_plain", eg.ECPGB_MIXED: "stages_mixed"}.get(mode, "stages_batched")
+        kernel = ("k_unit_plan + k_exact_small + k_exact_large + k_exact_link" if mode == eg.ECPGB_FP64
+                  else "k_unit_plan + k_unit_small + k_unit_large + k_unit_link")
+        # executed work: FP64 operations the unit stages executed per emitted
+        # unit (ncu: 2 DFMA + DMUL + DADD thread instructions of one run on
         # the cluster's first 8 centres, divided by its emitted units), FP64
         # pipe utilisation and DRAM bytes, from profiles/roofline_inputs.txt
         # (measured on the cluster: other workloads have no executed-work figure)
@@ -382,9 +381,7 @@ def ours(args, rank, world):
         prof = os.path.join(ROOT, "profiles", "roofline_inputs.txt")
         if os.path.exists(prof) and args.workload == "cluster":
             with open(prof) as f:
-                inputs = json.load(f)
-            key = {"k_unit": "k_unit", "k_unit_queue": "k_unit_queue", "k_unit_fast": "k_unit_queue"}[kernel]
-            entry = inputs.get(key + ("_mixed" if mode == eg.ECPGB_MIXED else ""), {})
+                entry = json.load(f).get(key, {})
         f_exec = entry.get("fp64_flops_per_emitted_unit")
         achieved = f_exec * emitted / (t_unit / 1e3) / 1e12 if f_exec else None
         traffic = entry["dram_bytes_per_emitted_unit"] * emitted if entry.get("dram_bytes_per_emitted_unit") else None
@@ -416,11 +413,11 @@ def ours(args, rank, world):
                          "alg_flops_per_unit": f_unit, "alg_achieved": alg_achieved,
                          "alg_frac": alg_achieved / peak,
                          "inputs": entry.get("source"),
-                         "note": ("achieved = FP64 operations the kernel executed (ncu counts per emitted "
-                                  "unit on the cluster's first 8 centres) x emitted units / the unit kernel's "
+                         "note": ("achieved = FP64 operations the unit stages executed (ncu counts per emitted "
+                                  "unit on the cluster's first 8 centres) x emitted units / their "
                                   "CUDA-event time; alg_* = the reference's work counted by the oracle on its "
                                   "control flow, which includes the full 1023-point tabulation of every "
-                                  "large-grid fallback the kernel skips, so alg_frac can exceed 1")},
+                                  "large-grid fallback the stages skip, so alg_frac can exceed 1")},
             "cpu_baseline": {"value": cpu_v, "unit": UNIT, "cores": cores, "kind": kind,
                              "sample": f"{text}: {s_units} units in {s_time:.1f} s on {cores} threads "
                                        + ("(jobs taken by threads as they free up)"

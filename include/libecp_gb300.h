@@ -128,7 +128,7 @@ int ecpgb_gradient(const ecpgb_system *s, int mode, const double *D, int ldD, do
 /* Device-resident job: inputs are copied to HBM once; ecpgb_job_run then
  * re-runs the whole pipeline (all kernels) nRuns times without host traffic,
  * writing one device-time per run (CUDA events on the engine's stream) to
- * msRun and the per-unit kernel's time to msUnit (either may be NULL).  With
+ * msRun and the unit stages' time to msUnit (either may be NULL).  With
  * flushL2 != 0 a 256 MiB buffer is written between runs, outside the timed
  * spans, so no run starts with a warm L2. */
 typedef struct ecpgb_job ecpgb_job;
@@ -139,28 +139,27 @@ long long ecpgb_job_units(const ecpgb_job *j, long long *emitted);
 int ecpgb_job_kernel_launches(const ecpgb_job *j);           /* kernels per run */
 void ecpgb_job_free(ecpgb_job *j);
 
-/* Launch configuration of the batched path (ECPGB_FAST).  queue: 1 = a
- * persistent launch whose CTAs pull units from a work queue, 0 = one CTA per
- * unit; sorted: 1 = the queue holds the units by descending estimated cost
- * (primitive pairs x (la + lb + 2) x (L + 2)), 2 = grouped by (la, lb, L)
- * class (largest la + lb first), by that cost within a class, 0 = the
- * reference's order;
+/* Launch configuration of the batched path (ECPGB_FAST).  queue: 1 = with
+ * screen, only the units that compute blocks enter the unit stages (a screening
+ * stage compacts them first), 0 = every unit does; sorted: 1 = the shell pairs by
+ * descending estimated cost (primitive pairs x (la + lb + 2)), 2 = grouped by
+ * (la, lb) class (largest la + lb first), by that cost within a class (the
+ * default), 0 = the reference's order; a pair's centres by descending L;
  * gcap: width cap of the type-1 step table in doubles per slot, which sets
- * the primitive pairs per warp and the CTAs per SM; balance: 1 = a unit with
- * few primitive pairs gets narrower type-1 groups so that all its warps
- * work; screen: 1 = with the queue launch, a screening stage first compacts
- * the queue to the units that compute blocks.  perClass: 1 = the autotuner
+ * the primitive pairs per warp and the CTAs per SM (default 33); balance: 1 = a
+ * unit with few primitive pairs gets narrower type-1 groups, so that more warps
+ * share them; screen: see queue.  perClass: 1 = the autotuner
  * chose the type-1 cap and balance per (la, lb) class (see
  * ecpgb_job_class_config; gcap is then the cap the shared memory is sized
  * for); configurations set with ecpgb_job_config have none.  msUnit: the
- * unit kernel's time when the autotuner measured it, else 0. */
+ * unit stages' time when the autotuner measured it, else 0. */
 typedef struct {
   int queue, sorted, gcap, balance, screen, perClass;
   float msUnit;
 } ecpgb_launch_config;
 
 /* Autotuner: times each candidate configuration on the job (one untimed and
- * two timed runs each, unit kernel only), keeps the fastest for this job and
+ * two timed runs each, unit stages only), keeps the fastest for this job and
  * for later jobs of the same (max basis l, max ECP L) in this process, and
  * reports it in *chosen.  trials (may be NULL) receives up to maxTrials
  * candidates with their times; *nTrials the number written.  queue and sorted

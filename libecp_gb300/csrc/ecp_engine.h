@@ -1,5 +1,5 @@
 // ecp_engine.h -- device-side job description shared by the host driver
-// (ecp_engine.cu) and the kernels (ecp_fp64.cu).
+// (ecp_host.cu) and the kernels.
 //
 // HBM layout of one job (all arrays device-resident, FP64 unless noted):
 //   inputs      geometry[3*nAtoms]; per shell l, K, first primitive, atom,
@@ -255,12 +255,11 @@ int upload_schedules(const int *s93slot, int s93n, const int *s93lvEnd, const in
 // recorded around the per-unit kernel.
 int launch_fp64_pipeline(const DevJob &job, cudaStream_t stream, size_t smemBytes, cudaEvent_t u0,
                          cudaEvent_t u1);
-// The four per-job kernels before the unit kernel (radii, centre potentials,
-// centre-atom angular tables, windows + F tables) and the AO scatter after it.
-void launch_prologue(const DevJob &job, cudaStream_t stream, bool withF);
+// The AO scatter after the blocks.
 void launch_epilogue(const DevJob &job, cudaStream_t stream);
 
-// The first three of those kernels and the run's first warning word in one launch.
+// Radii, centre potentials, centre-atom angular tables and the run's first warning
+// word in one launch; then the windows and F tables of the plain path.
 void launch_stage1(const DevJob &job, cudaStream_t stream);
 
 void launch_shell_F(const DevJob &job, cudaStream_t stream);
@@ -290,7 +289,6 @@ int fast_ctas_per_sm(size_t smemBytes);
 // before any graph capture).
 void fast_prepare();
 // Resets the per-run words (first warning, input errors).
-void launch_reset(const DevJob &job, cudaStream_t stream);
 int launch_fast_pipeline(const DevJob &job, cudaStream_t stream, const FastConfig &cfg, cudaEvent_t u0,
                          cudaEvent_t u1);
 

@@ -1,33 +1,33 @@
-// ecp_fast.cu -- batched unit kernel for sm_103a (the fast FP64 path).
+// ecp_fast.cu -- the batched path's unit stages for sm_103a (FP64 and mixed).
 //
-// Same results as the drop-in kernel (same quadrature schedules, windows,
-// convergence tests, stale-buffer semantics of the reference's fallbacks);
-// the work is organised for GB300, where FP64 runs at 1/62 of the FP32 rate
-// and every FP64 operation counts:
-//   * a warp per primitive pair (pairs dealt round-robin to the 4 warps):
-//     no CTA barrier inside the type-1 loop or the type-2 fallback;
+// Same results as the plain path (same quadrature schedules, windows,
+// convergence tests, stale-buffer semantics of the reference's fallbacks),
+// organised for two properties of GB300: its FP64 pipe takes one warp instruction
+// per 16 to 19 cycles and SM, however many lanes are active, and its instruction
+// cache holds little more than one of these loops.
+//   * stages instead of a unit a CTA: a plan (one warp a unit) lists the type-1
+//     groups, type-2 batches and fallback parts; one-warp CTAs take entries
+//     from the lists, so warps that run at the same time run the same code, no
+//     barrier waits for a slow primitive pair, and a chunk of units bounds the
+//     scratch between the stages;
+//   * tables, walks and convergence tests on the integer pipes with 64-bit
+//     mantissas (ecp_fixed.h), eleven bits more than FP64; FP64 where a value is
+//     rounded once (quadrature results) and in the angular linking;
 //   * level-granular tabulation: grid points are tabulated 32 schedule slots
 //     at a time (one slot per lane) and a primitive pair stops as soon as all
-//     its quadratures have converged -- on the 50-centre cluster the type-2
-//     fallback's quadratures stop after ~280 of the 1023 large-grid slots,
-//     where the reference tabulates all 1023;
-//   * K_l(z) as one Horner pass over precomputed Taylor coefficients (the
-//     reference's 5-step derivative recurrence, done once per table point on
-//     the host); exp by the table-driven method of ecp_fastmath.h; no FP64
-//     divide or trigonometric call in the hot loops (tabulated abscissae and
-//     reciprocals, division-free convergence tests, the k-vector direction
-//     from ratios);
-//   * only what is read is computed: type-1 tabulation for the pairs with a
-//     quadrature still running, fallback rows for the quadratures still
-//     running, and in the type-2 fallback only the slots whose value passes
-//     the screen (a pair's own points through its index interval), walked
-//     pair by pair with the empty slot pairs skipped;
+//     its quadratures have converged -- the type-2 fallback's stop after ~280 of
+//     the 1023 large-grid slots, where the reference tabulates all 1023;
+//   * only what is read is computed: slots whose value passes the screen (a pair's
+//     own points through its index interval), the rows and channels of the
+//     quadratures still running, kept in a dense list and dealt to the lanes;
 //   * the type-1 block accumulated per combined Cartesian index: chi[i][j]
 //     depends on (i, j) only through the index of a_i + b_j
 //     (src/type1.c:323-345), so one accumulator per combined index receives
 //     exactly the terms the reference adds to each chi[i][j];
-//   * the precision mode a template parameter: the FP64 kernels carry no
-//     mixed-precision code (instruction fetch is one of the kernel's stalls).
+//   * little code in the hot loops (no unrolling, one copy of what is used
+//     twice): a kilobyte more costs the large-grid stage 1 to 9 %.
+// 50-centre cluster (90,976 units): 37.0 ms in these stages; one FP64 kernel
+// with a unit a CTA took 116.3.
 #include <algorithm>
 
 #include "ecp_stages.cuh"
@@ -138,17 +138,17 @@ static __device__ __noinline__ xf channel(const DevJob &J, int c, int l, double 
 
 // ------------------------------------------- double-single (mixed path)
 //
-// The mixed path evaluates the large-grid fallbacks' tables -- Bessel rows,
-// ECP channels, powers of r, the Gaussian prefactor -- and their integrand
+// The mixed path evaluates the type-1 large-grid fallback's tables -- Bessel
+// rows, ECP channels, powers of r, the Gaussian prefactor -- and its integrand
 // products in double-single arithmetic (ecp_ff.h: FP32 pairs on the FMA
 // pipes), sums each level of a quadrature with a compensated FP32 sum and
-// adds it to the FP64 running sum at the level's end.  The convergence
-// tests, the level recurrences and every accumulation into T, Q and the
-// blocks stay FP64.  The fallbacks' test (PSM92, 16 e^2 <= 3 N |I - q| tol)
-// compares level differences far above the double-single rounding, so it
-// takes the FP64 path's decisions; the small-grid quadratures, whose
-// absolute test (err < tol) sits at the FP64 rounding level for large
-// integrals, are not touched.
+// adds it to the FP64 running sum at the level's end.  The fallback's test
+// (PSM92, 16 e^2 <= 3 N |I - q| tol) compares level differences far above the
+// double-single rounding, so it takes the FP64 path's decisions; the
+// small-grid quadratures, whose absolute test (err < tol) sits at the FP64
+// rounding level for large integrals, are not touched.  The type-2 fallback
+// runs on the integer tables: in double-single it took 45.1 ms of unit stages on
+// the cluster against 38.7, and 65.6 against 48.2 on the 150-shell sweep.
 
 // 1 / z: the float reciprocal refined by one Newton step in ff.
 static __device__ inline ff ff_recip(ff z) {
@@ -157,7 +157,7 @@ static __device__ inline ff ff_recip(ff z) {
   return ff_norm(y, __fmul_rn(y, e));
 }
 
-// K_0..K_lmax(z) in ff: the branches of bessel_fast over the tables' float
+// K_0..K_lmax(z) in ff: the branches of fx_bessel over the tables' float
 // pairs (Taylor coefficients, table abscissae, large-argument polynomial).
 static __device__ __noinline__ void bessel_ff(const DevJob &J, int lmax, ff z, ff *K, int stride) {
   if (__builtin_expect(z.hi < 1.0e-7f, 0)) {  // rare: the small-argument formula in FP64
@@ -309,7 +309,7 @@ static __device__ inline xs from_lane(xs a, int src) {
   return b;
 }
 
-// psm92_advance with val(pos) in ff: each level summed with a compensated
+// The PSM92 walk of slots s0 to s1 with val(pos) in ff: each level summed with a compensated
 // FP32 sum and added to the FP64 running sum I at the level's end (and at
 // the end of the slots walked, so that I is complete between calls).
 template <class V, class Vis>
@@ -488,7 +488,8 @@ static __device__ __noinline__ EntInfo t1_large_entry(const DevJob &J, int c, in
 
 // A group of G primitive pairs of one kind (perm[p0 ..]) of a unit's type-1
 // quadratures on the small grid (src/type1.c:95-148), by one warp; lane =
-// (pair, quadrature).  Converged quadratures are written to the unit's Q, the
+// (pair, quadrature).  G fills the lanes of the tabulation's entries as far as the
+// step table's width allows.  Converged quadratures are written to the unit's Q, the
 // pairs with a failed one to the fallback list.
 template <bool kMixed, int kKind>
 static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem &L, double *sm, const LevelTab &V,
@@ -853,6 +854,12 @@ static __device__ void t2_small(const DevJob &J, const Unit &U, const LevelTab &
 
 // One warp a CTA; each takes up to J.take entries of the type-1 groups, then
 // of the type-2 batches (one kind of work at a time on the whole GPU).
+// Bound by instruction latency: 56 % of the issue slots at 16 warps an SM, the
+// stalls fixed latencies (2.0 warps an issue), table rows from L2 (1.5) and
+// instruction fetch (0.4); the FP64 pipe is 6 % busy.  80 registers let 24 CTAs
+// share an SM (at 96 the cluster's stages took 46.5 instead of 45.3 ms, at 64
+// 45.8, with spills).  8 centres of the cluster: 1.53 ms (2.46 with doubles and
+// per-entry set-up).
 template <bool kMixed>
 __global__ void __launch_bounds__(32, 24) k_unit_small(DevJob J) {
   extern __shared__ double sm[];
@@ -1428,7 +1435,13 @@ static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem 
 }
 
 // The type-2 parts first (the longer ones), one at a time by the whole CTA, then
-// the failed type-1 pairs, one a warp.
+// the failed type-1 pairs, one a warp.  Bound by instruction latency like the
+// small grid: 49 % of the issue slots at 13 warps an SM, fixed latencies 2.0
+// warps an issue, table rows 1.5, fetch 0.4, FP64 pipe 4 %.  128 registers and the
+// tables' shared memory admit 14 to 16 warps; fewer registers spill in the walks
+// (18 warps: 48.8 against 46.5 ms on the cluster), two Bessel rows or two walk
+// entries at a time overflow the instruction cache (39.6 and 39.7 against 37.4).
+// 8 centres of the cluster: 3.25 ms.
 template <bool kMixed, int kWarps>
 __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) k_unit_large(DevJob J) {
   extern __shared__ double sm[];
@@ -1469,7 +1482,11 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) k_unit_large(DevJob 
 
 // One unit a CTA: the type-1 block from the quadratures of its primitive
 // pairs (src/type1.c:323-345), the type-2 block from its radial table
-// (src/type2.c:583-623), both shifted onto A and B (src/util.c:247-334).
+// (src/type2.c:583-623), both shifted onto A and B (src/util.c:247-334).  Bound by
+// the FP64 pipe (69 % busy) and the barriers between its short phases; 44 KB of
+// shared memory at g shells let five CTAs share an SM (61 KB, three CTAs: the
+// 150-shell sweep's stages took 50.6 instead of 47.9 ms).  8 centres of the
+// cluster: 0.39 ms.
 __global__ void __launch_bounds__(kLinkThreadsMax) k_unit_link(DevJob J) {
   extern __shared__ double sm[];
   int pos = J.chunk0 + blockIdx.x;
@@ -1652,16 +1669,12 @@ __global__ void __launch_bounds__(kScreenThreads) k_screen_scatter(DevJob J, lon
       if (J.chunkPair[k] == (int)i / J.nCentres) J.liveStart[k] = at;
 }
 
-__global__ void k_reset(int *errWord) {
-  errWord[0] = INT_MAX;
-  errWord[1] = 0;
-}
-
 // --------------------------------------------------------------- launchers
 
 int upload_schedules_fast(const int *s93slot, int s93n, const int *s93lvEnd, const int *s93lvJ,
                           const int *s93lvN, int s93levels, const int *s92slot, int s92n,
                           const int *s92lvEnd, const int *s92lvN, int s92levels, void *stream) {
+  if (s93levels > kMaxLevels || s92levels > kMaxLevels) return 1;
   return upload_stage_schedules(s93slot, s93n, s93lvEnd, s93lvJ, s93lvN, s93levels, s92slot, s92n, s92lvEnd, s92lvN,
                                 s92levels, stream);
 }
@@ -1691,8 +1704,6 @@ int fast_ctas_per_sm(size_t smemBytes) {
     return 0;
   return n;
 }
-
-void launch_reset(const DevJob &J, cudaStream_t st) { k_reset<<<1, 1, 0, st>>>(J.errWord); }
 
 int launch_fast_pipeline(const DevJob &J, cudaStream_t st, const FastConfig &cfg, cudaEvent_t u0, cudaEvent_t u1) {
   fast_prepare();

@@ -286,9 +286,6 @@ ECPGB_HD xs xs_add(xs a, xs b) {
 ECPGB_HD xs xs_neg(xs a) { return {-a.m, a.e}; }
 ECPGB_HD xs xs_shl(xs a, int k) { return {a.m, a.e + k}; }  // a 2^k
 ECPGB_HD xf xs_abs(xs a) { return xf_norm({a.m < 0 ? (u64)-a.m : (u64)a.m, a.e}); }
-ECPGB_HD double xs_to_double(xs a) {
-  return xf_to_double(a.m < 0 ? (u64)-a.m : (u64)a.m, a.e, a.m < 0 ? 0x80000000u : 0u);
-}
 // a * c rounded to double (c positive).
 ECPGB_HD double xs_times(xs a, xf c) {
   const xf v = xf_mul(xs_abs(a), c);

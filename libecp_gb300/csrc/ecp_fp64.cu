@@ -795,6 +795,24 @@ int upload_schedules(const int *s93slot, int s93n, const int *s93lvEnd, const in
   return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
+// Few CTAs leave SMs idle and the slowest sets the time: 32 points a CTA there
+// (12 shells: 27 instead of 51 us batched, 35 instead of 72 plain); with more the
+// window search and the centre's distance are worth sharing.
+int point_threads(const DevJob &J) { return (long long)J.nShells * J.nCentres <= 256 ? 32 : kPointThreads; }
+
+void launch_shell_F(const DevJob &J, cudaStream_t st) {
+  const int nt = point_threads(J);
+  k_shell_F<<<dim3(J.nShells, J.nCentres, (kSmallOrder + nt - 1) / nt), nt, 0, st>>>(J);
+}
+
+// The per-job stages one by one, for the entry point that allocates nothing.
+static void launch_prologue(const DevJob &J, cudaStream_t st) {
+  k_radius<<<(J.nShells + 127) / 128, 128, 0, st>>>(J);
+  k_centre<<<J.nCentres, 128, 0, st>>>(J);
+  k_centre_atom<<<dim3(J.nAtoms, J.nCentres), 64, 0, st>>>(J);
+  launch_shell_F(J, st);
+}
+
 int launch_fp64_pipeline(const DevJob &J, cudaStream_t st, size_t smemBytes, cudaEvent_t u0,
                          cudaEvent_t u1) {
   // function attributes are per device; callers hold the engine lock
@@ -806,7 +824,7 @@ int launch_fp64_pipeline(const DevJob &J, cudaStream_t st, size_t smemBytes, cud
     attr[dev] = true;
   }
   if (smemBytes > 200 * 1024) return 3;
-  launch_prologue(J, st, true);
+  launch_prologue(J, st);
   long long nUnits = (long long)J.nCentres * J.nPairs;
   if (u0) record_timing(u0, st);
   if (nUnits > 0) k_unit<<<(unsigned)nUnits, kUnitThreads, smemBytes, st>>>(J);
@@ -814,25 +832,6 @@ int launch_fp64_pipeline(const DevJob &J, cudaStream_t st, size_t smemBytes, cud
   launch_epilogue(J, st);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : kLaunchErrorBase + (int)e;
-}
-
-// Few CTAs leave SMs idle and the slowest sets the time: 32 points a CTA there
-// (12 shells: 27 instead of 51 us batched, 35 instead of 72 plain); with more the
-// window search and the centre's distance are worth sharing.
-int point_threads(const DevJob &J) { return (long long)J.nShells * J.nCentres <= 256 ? 32 : kPointThreads; }
-
-void launch_shell_F(const DevJob &J, cudaStream_t st) {
-  const int nt = point_threads(J);
-  k_shell_F<<<dim3(J.nShells, J.nCentres, (kSmallOrder + nt - 1) / nt), nt, 0, st>>>(J);
-}
-
-// Per-job stages before and after the unit kernel; shared by both paths
-// (the batched path launches its own F-table kernel: withF false).
-void launch_prologue(const DevJob &J, cudaStream_t st, bool withF) {
-  k_radius<<<(J.nShells + 127) / 128, 128, 0, st>>>(J);
-  k_centre<<<J.nCentres, 128, 0, st>>>(J);
-  k_centre_atom<<<dim3(J.nAtoms, J.nCentres), 64, 0, st>>>(J);
-  if (withF) launch_shell_F(J, st);
 }
 
 void launch_bessel_rows(const DevJob &J, double *D, cudaStream_t st) {

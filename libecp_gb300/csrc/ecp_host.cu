@@ -2,8 +2,9 @@
 // buffers, the run sequence, the device-resident job and the pipe probe.
 //
 // One run of a job on the engine's stream:
-//   one H2D copy of all inputs (packed into a pinned staging buffer), memsets
-//   of the AO matrix / block buffer / error words, the mode's pipeline, one D2H copy of the result (matrix or blocks) and the error
+//   one H2D copy of all inputs and of the queue orders and chunks of the unit
+//   stages (packed into a pinned staging buffer), a memset of the AO matrix, the
+//   mode's pipeline, one D2H copy of the result (matrix or blocks) and the error
 //   words.  Tables (grids, Bessel table, angular table, ...) are built once
 //   per key on the host and stay resident on the device.
 #include <cuda_runtime.h>
@@ -1209,8 +1210,8 @@ int job_tune(void *vj, ecpgb_launch_config *chosen, ecpgb_launch_config *trials,
   if (nTrials) *nTrials = 0;
   if (R->mode == ECPGB_FP64) { set_error("the autotuner applies to the batched path only"); return 3; }
   if (E.use_schedules(R->T, &lk)) return 1;
-  // candidates: queue or CTA-per-unit, cost order or the reference's, and
-  // the step-table cap (pairs per warp against CTAs per SM)
+  // candidates: live units only or all, the queue's orders, and the
+  // step-table cap (pairs per warp against CTAs per SM)
   std::vector<FastConfig> cand;
   auto mk = [](int queue, int sorted, int gcap, int balance) {
     FastConfig c;
@@ -1259,7 +1260,7 @@ int job_tune(void *vj, ecpgb_launch_config *chosen, ecpgb_launch_config *trials,
     n++;
     if (ms < best) { best = ms; bestCfg = c; }
   }
-  // per-class refinement on the best persistent configuration: each
+  // per-class refinement on the best configuration of live units: each
   // (la, lb) class takes the type-1 cap (at most the launch's) and balance
   // under which its own units took the fewest cycles, measured with every
   // class on one setting at a time; the combination is kept if the whole job

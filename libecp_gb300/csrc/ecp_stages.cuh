@@ -5,7 +5,7 @@
 // work lists that the plan writes (small grid, large grid) or over the units
 // (plan, blocks).  Independent warps take list entries, so no CTA barrier waits
 // for the slowest primitive pair and a launch's warps run the same code.
-// Included by ecp_fast.cu (batched FP64 and mixed) and ecp_fp64.cu (the plain
+// Included by ecp_fast.cu (batched FP64 and mixed) and ecp_exact.cu (the plain
 // path, --fmad=false), each with its own __constant__ schedules.
 #pragma once
 #include <algorithm>
@@ -405,8 +405,10 @@ static __device__ inline double binom_tab(int n, int k) { return __ldg(&kBinom.v
 // --------------------------------------------------------- stage 1: the plan
 
 // A unit by one warp: its primitive pairs by kind (kind-major, each kind in
-// pair order), the FM06 map, break index and point window of every pair, its
-// work-list entries; a dead unit is marked skipped.
+// pair order), the FM06 map, break index, point window and scalars of every pair,
+// its work-list entries; a dead unit is marked skipped.  A lane a pair: bound by
+// the FP64 pipe (81 % busy), some 200 instructions a unit, most of them square
+// roots and divides.  8 centres of the cluster: 0.20 ms (0.22 on the plain path).
 constexpr int kPlanThreads = 128;
 template <bool kExact>
 __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
@@ -576,7 +578,8 @@ static __device__ inline int2 small_entry(const DevJob &J, int i, int n0, int n1
 // (src/util.c:247-334), and its status.
 constexpr int kLinkThreadsMax = 256;
 // Threads a CTA: 256 where the shared memory (g shells) lets only a few CTAs
-// share a multiprocessor.
+// share a multiprocessor (the 150-shell sweep's unit stages: 47.9 ms, at 128 threads
+// 48.7; with less shared memory 128 and 256 measure the same).
 static inline int link_threads(size_t smem) { return smem > 40 * 1024 ? 256 : 128; }
 template <bool kExact>
 static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSmem &Lm, double *sm) {
@@ -836,8 +839,8 @@ static const JobPlan::Order &use_order(DevJob &J, int sorted) {
 
 // The unit stages of every chunk: sets the chunk's fields and clears its
 // counters, then `stages` launches the four kernels.  A warp takes up to 8
-// list entries where there are many (fewer CTAs to start), one where there
-// are few (every SM gets work).
+// list entries where there are at least 64 a multiprocessor for each (fewer CTAs
+// to start), one where there are few (every SM gets work).
 template <class Stages>
 static void launch_chunks(DevJob J, const JobPlan::Order &ord, cudaStream_t st, Stages stages) {
   int dev = 0, sms = 0;

@@ -3,9 +3,9 @@
 
     python -m libecp_gb300.profile_job fast|mixed|plain
 
-The batched modes use a fixed launch configuration (persistent queue,
-class-major order, step-table cap 45, screening stage), so that the unit
-kernel launches exactly once; no CUDA graph.  Prints the run's times and the
+The batched modes use a fixed launch configuration (class-major order,
+step-table cap 45, screening stage), and the job is one chunk, so that every
+unit stage launches exactly once; no CUDA graph.  Prints the run's times and the
 job's unit counts as one JSON line.
 """
 from __future__ import annotations

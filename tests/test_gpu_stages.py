@@ -92,6 +92,22 @@ def test_plain_stages_equal_the_single_kernel_bit_for_bit(eg, name):
     assert np.array_equal(np.triu(I), np.triu(_noalloc(eg, s)))
 
 
+@pytest.mark.parametrize("mode_name", ["ECPGB_FAST", "ECPGB_MIXED"])
+@pytest.mark.parametrize("centres, atoms", [(1, 9), (1, 10), (1, 21), (2, 21)])
+def test_job_sizes_on_both_sides_of_the_entry_rules(eg, mode_name, centres, atoms):
+    """Primitive pairs: up to 9728 an entry is one pair, up to 58368 two warps
+    take a large-grid entry; (1, 9) and (1, 10), (1, 21) and (2, 21) straddle the
+    lines."""
+    s = W.batched_cluster(5, n_centres=centres, n_basis_atoms=atoms)
+    k = np.asarray(s.KBS, dtype=int)
+    pairs = centres * (k.sum() ** 2 + (k ** 2).sum()) // 2
+    assert (pairs <= 9728) == (atoms == 9) and (pairs <= 58368) == (centres == 1), pairs
+    v0, o0, st0, _ = eg.raw_blocks(s, eg.ECPGB_FP64)
+    v1, o1, st1, _ = eg.raw_blocks(s, getattr(eg, mode_name))
+    assert np.array_equal(st0, st1) and np.array_equal(o0, o1)
+    assert np.abs(v1 - v0).max() <= TOL_ABS
+
+
 ODD = {
     "nan_coefficient": lambda s: s.dBS.__setitem__(0, np.nan),
     "infinite_ecp_coefficient": lambda s: s.dECP.__setitem__(1, np.inf),
