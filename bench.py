@@ -457,7 +457,7 @@ def serving_run(eg, rate, seconds, mode=None, slots=32):
             "units_per_s": r["units_per_s"], "latency_ms": r["latency_ms"], "queued_ms": r["queued_ms"],
             "gpu_ms": r["gpu_ms"], "hbm_budget_bytes": 64 << 30, "slots": slots,
             "max_inflight": r["stats"]["maxInflight"],
-            "batching": "continuous: jobs overlap on per-slot streams; each CTA takes at most 8 units, "
+            "batching": "continuous: jobs overlap on per-slot streams; each CTA takes at most 8 work-list entries, "
                         "jobs under 100k units on high-priority streams"}
 
 

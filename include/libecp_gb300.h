@@ -53,15 +53,11 @@ enum {
                        points tabulated level by level until convergence,
                        Horner-form Bessel rows, table-driven exp; same
                        schedules and decisions, rounding-level differences */
-  ECPGB_MIXED = 2,  /* the batched path with the bulk radial arithmetic in
-                       FP32: Bessel rows below the large-argument branch
-                       (Horner in FP32 over FP32 Taylor coefficients) and the
-                       ECP channel terms d r^n exp(-a r^2) (FP32 exp).  FP64
-                       stays for the large-argument Bessel rows, the Gaussian
-                       product exp prefactors, the quadrature sums and their
-                       convergence tests, and every accumulation.  Errors are
-                       those of FP32 (about 1e-7 relative to a block's
-                       largest element): it does not meet the FP64 bar */
+  ECPGB_MIXED = 2,  /* the batched path with the type-1 large-grid fallback
+                       in double-single FP32 pairs (about 48 bits) where its
+                       sums can still take the FP64 path's convergence
+                       decisions; within 1e-10 on the 50-centre cluster and
+                       2^-44 of a block's scale beyond                   */
 };
 
 /* Unit status.  A large-grid (PSM92) quadrature that exhausts its levels keeps
@@ -82,7 +78,7 @@ typedef struct {
   long long firstFailed;  /* first unit with a warning status, -1 if none */
   long long values;       /* doubles in the block layout                 */
   double msGpu;           /* device time of the last run (CUDA events)   */
-  double msUnitKernel;    /* of which the per-unit kernel                */
+  double msUnitKernel;    /* of which the unit stages                    */
   long long h2dBytes, d2hBytes;
 } ecpgb_info;
 
