@@ -167,7 +167,11 @@ struct JobPlan {
   size_t bytes = 0;            // scratch buffer, work lists included
 };
 
-// Launch configuration of the batched path (picked by the autotuner).
+// Launch configuration of the batched path (picked by the autotuner).  The
+// defaults are the fastest on all three of (unit stages, ms) 50-centre cluster,
+// 83-shell mixed batch and 150-shell sweep: 37.1, 30.6, 47.6; gcap 24: 37.8, 31.1, 47.9,
+// 45: 37.7, 30.9, 47.9, 64: 38.7, 31.8, 49.5; by cost: 37.2, 30.8, 49.6, the reference's
+// order: 37.3, 31.4, 50.5; balance: 37.8, 30.7, 47.8.
 struct FastConfig {
   int queue = 1;   // 1: the units that compute blocks (with screen); 0: every unit
   int sorted = 2;  // pairs 1: by descending estimated cost; 2: class-major; 0: the reference's order
