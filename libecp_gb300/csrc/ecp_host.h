@@ -194,7 +194,8 @@ bool valid_mode(int mode);
 struct DevTables;
 // Packs P's inputs into B's pinned buffer, copies them to the device on
 // `stream` and fills J (B's buffers grow as needed).
-// A job's units run in chunks whose scratch stays within scratchCap.
+// A job's units run in chunks whose scratch stays within scratchCap (1 or 4 GiB
+// take 0.3 % off the largest jobs' unit stages, 47.5 -> 47.3 ms).
 constexpr size_t kScratchCap = 512ull << 20;
 int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int mode, cudaStream_t stream,
               size_t scratchCap = kScratchCap);
