@@ -645,6 +645,7 @@ __global__ void __launch_bounds__(kLinkThreadsMax) k_exact_link(DevJob J) {
   const Unit U = unit_load(J, J.chunk0 + blockIdx.x);
   if (!U.live) return;
   const LinkSmem Lm = link_layout(J.maxLBS, J.maxLECP);
+  const bool one = blockIdx.y == 0, two = blockIdx.y == gridDim.y - 1;  // the blocks this CTA makes
   const int tid = threadIdx.x, NT = blockDim.x, lab = U.lab, lq = lab + 1, Nb = U.Nb, RQ = lq * lq;
   double *rsh = sm + Lm.rsh, *dir = sm + Lm.dir, *H = sm + Lm.H;
   const int dd = J.tmDim + 1, tmW = (J.tmDim + 1) * (J.tmDim + 1), nq = t1_items(lab), nH = NCUM(lab);
@@ -652,7 +653,7 @@ __global__ void __launch_bounds__(kLinkThreadsMax) k_exact_link(DevJob J) {
 #pragma unroll 1
   for (int e = tid; e < nH; e += NT) H[e] = 0.0;
 #pragma unroll 1
-  for (int b0 = 0; b0 < U.NP; b0 += kLinkBatch) {
+  for (int b0 = one ? 0 : U.NP; b0 < U.NP; b0 += kLinkBatch) {
     const int nb = U.NP - b0 < kLinkBatch ? U.NP - b0 : kLinkBatch;
     __syncthreads();
     // cos(theta), phi and its sine and cosine, then S_lm a column a thread
@@ -696,7 +697,7 @@ __global__ void __launch_bounds__(kLinkThreadsMax) k_exact_link(DevJob J) {
     }
   }
   __syncthreads();
-  link_finish<true>(J, U, Lm, sm);
+  link_finish<true>(J, U, Lm, sm, one, two);
 }
 
 // --------------------------------------------------------------- launchers
@@ -743,7 +744,7 @@ int launch_exact_pipeline(const DevJob &J, cudaStream_t st, cudaEvent_t u0, cuda
     k_exact_small<<<gSmall, 32, sSmall, st>>>(K);
     K.take = takeLarge;
     k_exact_large<<<gLarge, 32, sLarge, st>>>(K);
-    k_exact_link<<<units, link_threads(sLink), sLink, st>>>(K);
+    k_exact_link<<<dim3(units, link_parts(units)), link_threads(sLink), sLink, st>>>(K);
   });
   if (u1) record_timing(u1, st);
   launch_epilogue(Jc, st);

@@ -1480,7 +1480,7 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) k_unit_large(DevJob 
 
 // -------------------------------------------------------- stage 4: the blocks
 
-// One unit a CTA: the type-1 block from the quadratures of its primitive
+// One unit a CTA (in small jobs one of its blocks): the type-1 block from the quadratures of its primitive
 // pairs (src/type1.c:323-345), the type-2 block from its radial table
 // (src/type2.c:583-623), both shifted onto A and B (src/util.c:247-334).  Bound by
 // the FP64 pipe (69 % busy) and the barriers between its short phases; 44 KB of
@@ -1498,13 +1498,14 @@ __global__ void __launch_bounds__(kLinkThreadsMax) k_unit_link(DevJob J) {
   const Unit U = unit_load(J, pos);
   if (!U.live) return;
   const LinkSmem Lm = link_layout(J.maxLBS, J.maxLECP);
+  const bool one = blockIdx.y == 0, two = blockIdx.y == gridDim.y - 1;  // the blocks this CTA makes
   const int tid = threadIdx.x, NT = blockDim.x, lab = U.lab, lq = lab + 1, Nb = U.Nb;
   double *rsh = sm + Lm.rsh, *dir = sm + Lm.dir, *W = sm + Lm.W, *H = sm + Lm.H;
   const int dd = J.tmDim + 1, tmW = (J.tmDim + 1) * (J.tmDim + 1), RQ = lq * lq, nq = t1_items(lab);
   // type 1: W[L][l][m] = sum over the primitive pairs of S_lm Q[L][l] (the
   // pairs in order), then H[p] = sum_lm poly2sph[p][lm] W[|p|][l][m]: the
   // angular coefficients once per unit instead of once per pair
-  {
+  if (one) {
     const double *Q = (const double *)(U.scr + U.L.Q);
     const int nW = NCUM(lab);  // sum over L of (L+1)(L+2)/2 entries (l, m)
 #pragma unroll 1
@@ -1558,7 +1559,7 @@ __global__ void __launch_bounds__(kLinkThreadsMax) k_unit_link(DevJob J) {
     }
     __syncthreads();
   }
-  link_finish<false>(J, U, Lm, sm);
+  link_finish<false>(J, U, Lm, sm, one, two);
 }
 
 // The screening window and F table of every (shell, centre) -- k_shell_F of
@@ -1742,7 +1743,7 @@ int launch_fast_pipeline(const DevJob &J, cudaStream_t st, const FastConfig &cfg
     const int nw = J.twoWarps ? 2 : 1;
     (cfg.mixed ? nw > 1 ? k_unit_large<true, 2> : k_unit_large<true, 1>
                : nw > 1 ? k_unit_large<false, 2> : k_unit_large<false, 1>)<<<gLarge, 32 * nw, sLarge, st>>>(K);
-    k_unit_link<<<units, link_threads(sLink), sLink, st>>>(K);
+    k_unit_link<<<dim3(units, link_parts(units)), link_threads(sLink), sLink, st>>>(K);
   });
   if (u1) record_timing(u1, st);
   launch_epilogue(Jc, st);

@@ -573,16 +573,20 @@ static __device__ inline int2 small_entry(const DevJob &J, int i, int n0, int n1
   return i < n0 ? J.listT1[i] : i < n1 ? J.listT1[J.capT1 - 1 - (i - n0)] : J.listT2[i - n1];
 }
 
-// The blocks of a unit from its combined-index block H (type 1) and its radial
-// table (type 2, src/type2.c:583-623), both shifted onto A and B
-// (src/util.c:247-334), and its status.
+// The blocks of a unit from its combined-index block H (type 1: `one`) and its
+// radial table (type 2, src/type2.c:583-623: `two`), both shifted onto A and B
+// (src/util.c:247-334), and its status (with `two`).
 constexpr int kLinkThreadsMax = 256;
+// CTAs a unit: in small jobs one for each block, which halves a unit's chain (78
+// units: 42 instead of 55 us, plain path 47 instead of 80; unit stages of 2016 units
+// 1.19 instead of 1.25 ms, of 6048 2.68 instead of 2.67, of 100,800 37.3 instead of 37.0).
+static inline unsigned link_parts(unsigned units) { return units <= 4096 ? 2 : 1; }
 // Threads a CTA: 256 where the shared memory (g shells) lets only a few CTAs
 // share a multiprocessor (the 150-shell sweep's unit stages: 47.9 ms, at 128 threads
 // 48.7; with less shared memory 128 and 256 measure the same).
 static inline int link_threads(size_t smem) { return smem > 40 * 1024 ? 256 : 128; }
 template <bool kExact>
-static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSmem &Lm, double *sm) {
+static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSmem &Lm, double *sm, bool one, bool two) {
   const int tid = threadIdx.x, NT = blockDim.x, la = U.la, lb = U.lb, lpa = U.lpa, lpb = U.lpb, nca = NCUM(la),
             ncb = NCUM(lb), Lc = U.Lc;
   // (l1 + l2 + l3 is even: every other l3 in a row)
@@ -593,7 +597,7 @@ static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSme
   double *out2 = out1 + NCART(lpa) * NCART(lpb);
   const int dd = J.tmDim + 1;
 #pragma unroll 1
-  for (int e = tid; e < nca * ncb; e += NT) {
+  for (int e = one ? tid : nca * ncb; e < nca * ncb; e += NT) {
     const int *ei = J.ijk + 3 * (e / ncb), *ej = J.ijk + 3 * (e % ncb);
     chi[e] = H[J.ijkIdx[((ei[0] + ej[0]) * dd + (ei[1] + ej[1])) * dd + ei[2] + ej[2]]];
   }
@@ -602,7 +606,7 @@ static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSme
 #pragma unroll 1
   for (int e = tid; e < LE * LBE * LBE * nT; e += NT) T[e] = 0.0;
   __syncthreads();
-  {
+  if (two) {
     const double *Tq = (const double *)(U.scr + U.L.T), *part = (const double *)(U.scr + U.L.part);
     const unsigned *mask = (const unsigned *)(U.scr + U.L.mask);
     const int nParts = t2_parts(U.NP, J.single), nIt = class_items(J, U.cls * LE, LE);
@@ -674,7 +678,8 @@ static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSme
       }
       __syncthreads();
     };
-    poly_shift(norm1, out1);
+    if (one) poly_shift(norm1, out1);
+    if (!two) return;
     // gamma (src/type2.c:583-623)
     {
       const double *angA = J.ang + cA * J.angLam * J.angLM * J.angC;
@@ -756,7 +761,8 @@ static __device__ void link_finish(const DevJob &J, const Unit &U, const LinkSme
       }
     };
     __syncthreads();
-    shift(norm1, out1);
+    if (one) shift(norm1, out1);
+    if (!two) return;
     // gamma (src/type2.c:583-623), for every channel l and bra degree alpha in
     // two steps: Y[m][l1][q] = sum over l2 of Omega_B T, then the sum over
     // (m, l1) of Omega_A Y -- the radial table enters once per (l1, q) instead of
