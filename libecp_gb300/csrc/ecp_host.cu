@@ -544,19 +544,6 @@ static bool plain_stages(const Parsed &P, int mode) {
            P.tol >= 1e-300 && P.tol <= 1e100);
 }
 
-// Scratch of a job with chunks of at most `cap` bytes (at least one
-// pair's units a chunk).
-static size_t scratch_bytes(const Parsed &P, size_t cap, bool single) {
-  size_t tot = 0, one = 0;
-  for (int p = 0; p < P.nPairs; p++) {
-    const PairPlan q = plan_of_pair(P, p, single);
-    const size_t b = (size_t)P.nCentres * (q.scratch + q.lists);
-    tot += b;
-    one = std::max(one, b);
-  }
-  return std::min(tot, std::max(cap, one));
-}
-
 // The queue orders of a job -- shell pairs in the reference's order,
 // by descending estimated cost, and class-major (largest la + lb first, then
 // la; within a class by that cost), ties in the reference's order; every
@@ -630,27 +617,56 @@ static void make_plan(const Parsed &P, size_t cap, bool single, JobPlan &plan, s
   }
 }
 
-// Packs the inputs into the pinned staging buffer, copies them to the device
-// and fills the DevJob's input and work pointers.
-size_t job_device_bytes(const Parsed &P, int mode, size_t budget, size_t *scratchCap) {
-  const size_t nc = P.nCentres, ns = P.nShells, na = P.nAtoms, O = kSmallOrder;
+// The bytes of the packed inputs, alignment included (upper bound); of which the
+// unit stages' plan and integer terms: *stages.
+static size_t input_bytes(const Parsed &P, int mode, size_t chunks, size_t *stages) {
+  const size_t nc = P.nCentres, np = P.nPairs, nt = P.termL.size();
+  *stages = 36 * (np + 1) + 12 * chunks + 8 * nc + 4 * P.chanT0.size() + 32 * nt + 8 * 256;
+  return 8 * (P.geom.size() + P.primA.size() + P.primD.size() + 3 * nt + np) +
+         4 * (5 * P.shL.size() + P.atomMaxL.size() + 4 * nc + nt + 3 * np) + (mode == ECPGB_MIXED ? 16 * nt : 0) +
+         24 * 256 + *stages;
+}
+
+// The bytes of a job's device buffers under its plan.
+static JobBytes job_bytes(const Parsed &P, int mode, const JobPlan &plan, size_t *stages) {
+  const size_t nc = P.nCentres, ns = P.nShells, na = P.nAtoms, O = kSmallOrder, nu = nc * P.nPairs;
   const size_t LE = P.maxLECP > 0 ? P.maxLECP : 1, LB = P.maxLBS + P.deriv;
   const size_t nk = std::max(LB + LE, 2 * LB) + 1, nF = LB + LE + 1, D = LB + 1;  // table ranks (upper bounds)
   const size_t angLam = P.maxLECP + LB + 1, angC = (LB + 1) * (LB + 2) * (LB + 3) / 6;
-  size_t in = 8 * (P.geom.size() + P.primA.size() + P.primD.size() + 3 * P.termL.size() + P.pairOff.size()) +
-              4 * (5 * P.shL.size() + P.atomMaxL.size() + 4 * P.ctrAtom.size() + P.termL.size() + 3 * P.pairA.size()) +
-              36 * (P.nPairs + 1) + 8 * nc + 4 * P.chanT0.size() + (32 + (mode == ECPGB_MIXED ? 16 : 0)) * P.termL.size() +
-              32 * 256;
-  size_t work = 8 * (ns + nc * O * LE * nk + nc * O + nc * ns * (1 + P.deriv) * O * nF + nc * na * 4 + nc * na * D * D * D +
-                     nc * na * angLam * LE * LE * angC + nc * (size_t)P.centreStride + (size_t)P.dim * P.dim) +
-                4 * (nc + nc * ns * 3 + nc * (size_t)P.nPairs + 2) + 8;
-  // the scratch between the stages takes what the budget leaves: a job whose
-  // other buffers fit is never refused for it
-  const size_t base = in + work, cap = base < budget ? std::min(kScratchCap, budget - base) : 0;
-  if (scratchCap) *scratchCap = cap;
-  return base > budget ? base : std::min(budget, base + scratch_bytes(P, cap, plain_stages(P, mode) || primitive_pairs(P) <= kFewPairs));
+  size_t chunks = 0;
+  for (const JobPlan::Order &o : plan.order) chunks = std::max(chunks, o.chunks.size());
+  const bool screen = mode != ECPGB_FP64;
+  return {{input_bytes(P, mode, chunks, stages), 8 * (ns + 1), 8 * (nc * O * LE * nk + 1), 8 * (nc * O + 1),
+           8 * (nc * ns * (1 + P.deriv) * O * nF + 1), 8 * (nc * na * 4 + 1), 8 * (nc * na * D * D * D + 1),
+           8 * (nc * na * angLam * LE * LE * angC + 1), 8 * (nc * (size_t)P.centreStride + 1),
+           8 * ((size_t)P.dim * P.dim + 1), 4 * (nc + 1), 4 * (nc * ns * 3 + 1), 4 * (nu + 1), 4 * 16,
+           screen ? 4 * (nu + 1) : 0, screen ? 4 * (nu / 256 + 2) : 0, screen ? 4 * (chunks + 1) : 0, plan.bytes + 16}};
 }
 
+static bool single_pair_parts(const Parsed &P, int mode) {
+  return plain_stages(P, mode) || primitive_pairs(P) <= kFewPairs;
+}
+
+bool job_device_bytes(const Parsed &P, int mode, size_t budget, JobBytes *need, size_t *scratchCap) {
+  JobPlan plan;
+  std::vector<int> orders, chunkPairs, ctr;
+  std::vector<long long> offs;
+  const bool single = single_pair_parts(P, mode);
+  size_t stages;
+  // (a smaller scratch means more chunks, whose list takes a little more of the inputs)
+  for (size_t cap = kScratchCap;;) {
+    make_plan(P, cap, single, plan, orders, offs, chunkPairs, ctr);
+    *need = job_bytes(P, mode, plan, &stages);
+    *scratchCap = cap;
+    const size_t base = need->total() - need->b[kJobBufs - 1];
+    if (base - stages > budget) return false;
+    if (need->total() <= budget || plan.bytes > cap) return true;
+    cap = std::min(budget > base + 16 ? budget - base - 16 : 0, cap - cap / 16 - 1);
+  }
+}
+
+// Packs the inputs into the pinned staging buffer, copies them to the device
+// and fills the DevJob's input and work pointers.
 int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int mode, cudaStream_t stream,
               size_t scratchCap) {
   const HostTables &h = T->host;
@@ -659,7 +675,7 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   const long long np = primitive_pairs(P);
   J.few = np <= kFewPairs;
   J.twoWarps = np <= kTwoWarpPairs;
-  J.single = J.few || J.plain;
+  J.single = single_pair_parts(P, mode);
   J.nAtoms = P.nAtoms; J.nShells = P.nShells; J.nPrims = P.nPrims; J.nCentres = P.nCentres;
   J.nPairs = P.nPairs; J.dim = P.dim;
   J.maxLECP = h.maxLECP; J.maxLBS = h.maxLBS; J.maxLambda = h.maxLambda; J.nk = h.nk; J.nF = h.nF;
@@ -710,9 +726,14 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
     split_pairs(P.termA, tAf);
     split_pairs(P.termD, tDf);
   }
-  size_t iTAf = add(tAf.data(), 4 * tAf.size()), iTDf = add(tDf.data(), 4 * tDf.size());
-  if (!B.pinned.ensure(tot) || !B.in.ensure(tot)) {
+  size_t iTAf = add(tAf.data(), 4 * tAf.size()), iTDf = add(tDf.data(), 4 * tDf.size()), stages;
+  const JobBytes need = job_bytes(P, mode, B.plan, &stages);
+  if (tot > need.b[0] || !B.pinned.ensure(tot)) {
     set_error("allocation of %zu input bytes failed", tot);
+    return -1;
+  }
+  if (!B.reserve(need)) {
+    set_error("device allocation of the job's %zu bytes failed", need.total());
     return -1;
   }
   for (auto &p : pcs)
@@ -742,41 +763,20 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.besT = T->besT.p; J.besC = T->besC.p; J.p2s = T->p2s.p; J.fac = T->fac.p; J.dfac = T->dfac.p;
   J.ijk = T->ijk.p; J.ijkIdx = T->ijkIdx.p; J.omega = T->omega.p;
   // --- work arrays
-  const size_t nc = P.nCentres, ns = P.nShells, na = P.nAtoms, O = kSmallOrder;
-  bool ok = B.radius.ensure(ns + 1) && B.utab.ensure(nc * O * LE * h.nk + 1) && B.uL.ensure(nc * O + 1) &&
-            B.gridEnd.ensure(nc + 1) && B.win.ensure(nc * ns * 3 + 1) && B.F.ensure(nc * ns * (1 + P.deriv) * O * h.nF + 1) &&
-            B.cgeo.ensure(nc * na * 4 + 1) && B.usp.ensure(nc * na * J.uspD * J.uspD * J.uspD + 1) &&
-            B.ang.ensure(nc * na * (size_t)J.angLam * J.angLM * J.angC + 1) &&
-            B.out.ensure(nc * (size_t)P.centreStride + 1) && B.status.ensure(nc * (size_t)P.nPairs + 1) &&
-            B.mat.ensure((size_t)P.dim * P.dim + 1) && B.err.ensure(16);
-  if (!ok) {
-    set_error("device allocation failed for the job's work arrays");
-    return -1;
-  }
   J.radius = B.radius.p; J.utab = B.utab.p; J.uL = B.uL.p; J.gridEnd = B.gridEnd.p; J.win = B.win.p;
   J.F = B.F.p; J.cgeo = B.cgeo.p; J.usp = B.usp.p; J.ang = B.ang.p; J.out = B.out.p;
   J.status = B.status.p; J.mat = B.mat.p; J.errWord = B.err.p;
-  {  // the plan, the scratch and the batched path's screening stage
-    const size_t nu = nc * (size_t)P.nPairs;
-    size_t chunks = 0;
-    for (const JobPlan::Order &o : B.plan.order) chunks = std::max(chunks, o.chunks.size());
-    if ((mode != ECPGB_FP64 && !(B.live.ensure(nu + 1) && B.screenBlocks.ensure(nu / 256 + 2) &&
-                                 B.liveStart.ensure(chunks + 1))) ||
-        !B.scr.ensure(B.plan.bytes + 16)) {
-      set_error("device allocation failed for the job's scratch");
-      return -1;
-    }
-    J.live = B.live.p;
-    J.liveStart = B.liveStart.p;
-    J.screenBlocks = B.screenBlocks.p;
-    J.scr = B.scr.p;
-    J.counters = (unsigned *)(B.err.p + 2);
-    J.plan = &B.plan;
-    J.pairOrders = (const int *)dp(iOrd);
-    J.scrOffs = (const long long *)dp(iOff);
-    J.chunkPairs = (const int *)dp(iChk);
-    J.ctrOrder = (const int *)dp(iCtr);
-  }
+  // --- the plan, the scratch and the batched path's screening stage
+  J.live = B.live.p;
+  J.liveStart = B.liveStart.p;
+  J.screenBlocks = B.screenBlocks.p;
+  J.scr = B.scr.p;
+  J.counters = (unsigned *)(B.err.p + 2);
+  J.plan = &B.plan;
+  J.pairOrders = (const int *)dp(iOrd);
+  J.scrOffs = (const long long *)dp(iOff);
+  J.chunkPairs = (const int *)dp(iChk);
+  J.ctrOrder = (const int *)dp(iCtr);
   J.gcap = FastConfig{}.gcap;
   J.besH = T->besH.p;
   J.besA = T->besA.p;

@@ -125,6 +125,17 @@ struct PinnedBuf {
   PinnedBuf &operator=(const PinnedBuf &) = delete;
 };
 
+// Bytes of each of a job's device buffers, in the order of JobBuffers::each.
+constexpr int kJobBufs = 18;
+struct JobBytes {
+  size_t b[kJobBufs] = {};
+  size_t total() const {
+    size_t t = 0;
+    for (size_t x : b) t += x;
+    return t;
+  }
+};
+
 // Device allocations of one job.
 struct JobBuffers {
   DBuf<char> in;
@@ -139,17 +150,32 @@ struct JobBuffers {
   int *pinnedErr = nullptr;
   long long h2dBytes = 0;
   JobBuffers() { cudaMallocHost((void **)&pinnedErr, 4 * sizeof(int)); }
-  // device bytes held by the buffers
-  size_t device_bytes() const {
-    return in.cap + scr.cap + 8 * (radius.cap + utab.cap + uL.cap + F.cap + cgeo.cap + usp.cap + ang.cap + out.cap + mat.cap) +
-           4 * (gridEnd.cap + win.cap + status.cap + err.cap + live.cap + screenBlocks.cap + liveStart.cap);
+  // Every buffer that staging a job grows.
+  template <class F_>
+  void each(F_ f) {
+    f(in); f(radius); f(utab); f(uL); f(F); f(cgeo); f(usp); f(ang); f(out); f(mat);
+    f(gridEnd); f(win); f(status); f(err); f(live); f(screenBlocks); f(liveStart); f(scr);
+  }
+  // Device bytes held, and what they will be once a job of `need` is staged (a
+  // buffer keeps the larger size).
+  size_t device_bytes_with(const JobBytes &need) {
+    size_t t = 0;
+    int i = 0;
+    each([&](auto &d) { t += std::max(d.cap * sizeof(*d.p), need.b[i++]); });
+    return t;
+  }
+  size_t device_bytes() { return device_bytes_with(JobBytes{}); }
+  // Grows every buffer to at least its bytes in `need`.
+  bool reserve(const JobBytes &need) {
+    bool ok = true;
+    int i = 0;
+    each([&](auto &d) { ok = d.ensure((need.b[i++] + sizeof(*d.p) - 1) / sizeof(*d.p)) && ok; });
+    return ok;
   }
   // Releases the device buffers (ordered on stream s); they grow again on use.
   void release(cudaStream_t s) {
-    in.release(s);
-    for (DBuf<double> *b : {&radius, &utab, &uL, &F, &cgeo, &usp, &ang, &out, &mat, &sout}) b->release(s);
-    for (DBuf<int> *b : {&gridEnd, &win, &status, &err, &live, &screenBlocks, &liveStart}) b->release(s);
-    scr.release(s);
+    each([&](auto &d) { d.release(s); });
+    sout.release(s);
     sphOff.release(s);
   }
   ~JobBuffers() {
@@ -203,9 +229,11 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
 // cfg null = the tuned configuration for the job's (l, L).
 int run_pipeline(JobBuffers &B, const DevJob &J, int mode, cudaEvent_t u0, cudaEvent_t u1,
                  const FastConfig *cfg, cudaStream_t stream);
-// Device bytes a job of P will hold (inputs, work arrays, scratch) where at
-// most `budget` may be held; scratchCap: the scratch cap to stage it with.
-size_t job_device_bytes(const Parsed &P, int mode, size_t budget, size_t *scratchCap);
+// Device bytes of a job of P where at most `budget` may be held, and the scratch
+// cap to stage it with; false where its buffers without the unit stages' plan and
+// scratch are above the budget.  The scratch takes what the budget leaves, down to
+// one pair's units (which a job within that distance of the budget holds above it).
+bool job_device_bytes(const Parsed &P, int mode, size_t budget, JobBytes *need, size_t *scratchCap);
 // With the engine lock held: the tables of the request and, unless requests
 // in flight pin other level schedules (returns 4: retry after they finish),
 // its schedules made current and pinned.  0 ok, 1 error.

@@ -52,7 +52,8 @@ double now_ms() {
 struct Request {
   long long id = 0;
   Parsed P;
-  size_t need = 0;  // device bytes estimate
+  JobBytes need;      // of its device buffers
+  bool fits = false;  // in the budget
   size_t scratchCap = kScratchCap;
   int state = 0;    // 0 queued, 1 running, 2 done, 3 failed
   int rc = 0;       // like ecpgb_getIntegrals: 0 ok, 2 unit warnings, 1 failure
@@ -202,19 +203,7 @@ struct Server {
           if (queue.empty()) break;
           r = queue.front();
         }
-        // the free slot that fits best: the smallest that holds the job
-        // without growing, else the largest
-        int k = -1;
-        for (size_t i = 0; i < slots.size(); i++) {
-          if (slots[i]->req) continue;
-          if (k < 0) { k = (int)i; continue; }
-          const size_t bi = slots[i]->B.device_bytes(), bk = slots[k]->B.device_bytes();
-          const bool fi = bi >= r->need, fk = bk >= r->need;
-          if ((fi && (!fk || bi < bk)) || (!fi && !fk && bi > bk)) k = (int)i;
-        }
-        if (k < 0) break;
-        size_t mine = slots[k]->B.device_bytes();
-        if (r->need > budget) {
+        if (!r->fits) {
           {
             std::lock_guard<std::mutex> lk(mu);
             queue.pop_front();
@@ -223,19 +212,34 @@ struct Server {
           finish(*r, 3);
           continue;
         }
-        // over the budget: release the buffers of idle slots, largest first
-        while (held() - mine + std::max(mine, r->need) > budget) {
+        // the free slot whose buffers grow least, of those the smallest
+        int k = -1;
+        size_t grow = 0;
+        for (size_t i = 0; i < slots.size(); i++) {
+          if (slots[i]->req) continue;
+          const size_t have = slots[i]->B.device_bytes(), g = slots[i]->B.device_bytes_with(r->need) - have;
+          if (k < 0 || g < grow || (g == grow && have < slots[k]->B.device_bytes())) {
+            k = (int)i;
+            grow = g;
+          }
+        }
+        if (k < 0) break;
+        // over the budget: release the buffers of idle slots, largest first, the
+        // chosen slot's own last (its buffers may have other jobs' shapes)
+        while (held() + slots[k]->B.device_bytes_with(r->need) - slots[k]->B.device_bytes() > budget) {
           int v = -1;
           for (size_t i = 0; i < slots.size(); i++)
             if ((int)i != k && !slots[i]->req && slots[i]->B.device_bytes() > 0 &&
                 (v < 0 || slots[i]->B.device_bytes() > slots[v]->B.device_bytes()))
               v = (int)i;
+          if (v < 0 && slots[k]->B.device_bytes() > 0) v = k;
           if (v < 0) break;
           slots[v]->B.release(slots[v]->stream);
           std::lock_guard<std::mutex> lk(mu);
           slotBytes[v] = 0;
         }
-        if (held() - mine + std::max(mine, r->need) > budget) break;  // wait for memory
+        // wait for memory while other jobs hold it
+        if (busy && held() + slots[k]->B.device_bytes_with(r->need) - slots[k]->B.device_bytes() > budget) break;
         int rc = start(k, r);
         if (rc == 4) break;  // other level schedules in flight
         {
@@ -304,7 +308,7 @@ long long server_submit(void *sv, const ecpgb_system &s) {
     set_error("job has no units");
     return -1;
   }
-  r->need = job_device_bytes(r->P, S->mode, S->budget, &r->scratchCap);
+  r->fits = job_device_bytes(r->P, S->mode, S->budget, &r->need, &r->scratchCap);
   r->tSubmit = now_ms();
   std::lock_guard<std::mutex> lk(S->mu);
   if (S->stop) {
