@@ -670,6 +670,12 @@ bool job_device_bytes(const Parsed &P, int mode, size_t budget, JobBytes *need, 
 int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int mode, cudaStream_t stream,
               size_t scratchCap) {
   const HostTables &h = T->host;
+  // queue positions and unit numbers on the device are ints
+  const long long units = (long long)P.nCentres * P.nPairs;
+  if (units > INT_MAX) {
+    set_error("job has %lld units; at most %d run in one job", units, INT_MAX);
+    return -1;
+  }
   std::memset(&J, 0, sizeof J);
   J.plain = plain_stages(P, mode);
   const long long np = primitive_pairs(P);

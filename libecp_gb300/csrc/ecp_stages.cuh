@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
     const int l0 = J.liveStart[J.chunk];
     if (l0 + idx >= J.liveStart[J.chunk + 1]) return;
     pos = J.live[l0 + idx];
-  } else if (pos >= J.chunk1) {
+  } else if (idx >= J.chunk1 - J.chunk0) {
     return;
   }
   const Unit U = unit_load(J, pos);
