@@ -115,13 +115,13 @@ struct DevJob {
   // between the stages, work lists and their counters (ecp_fast.cu)
   const int *pairOrders;          // [3][nPairs], by FastConfig::sorted
   const long long *scrOffs;       // [3][nPairs + 1] scratch bytes before a pair's units
-  const int *chunkPairs;          // first sorted pair of every chunk, order after order
+  const int *chunkUnits;          // first queue position of every chunk, order after order
   const int *ctrOrder;
   const struct JobPlan *plan;     // host side
   char *scr;
   unsigned *counters;
   // the launch's order and chunk
-  const int *pairOrder, *chunkPair;
+  const int *pairOrder, *chunkUnit;
   const long long *scrOff;
   int chunk, nChunks, chunk0, chunk1;  // queue positions [chunk0, chunk1)
   long long scrBase;
@@ -152,17 +152,17 @@ struct PairPlan {
 };
 PairPlan pair_plan(int NP, int la, int lb, int nItems, bool single);
 
-// A batched job's queue orders, cut into chunks of consecutive sorted pairs
-// whose units' scratch fits the scratch buffer.
+// A job's queue orders, cut into chunks of consecutive units whose scratch fits
+// the scratch buffer.
 struct JobPlan {
   struct Chunk {
-    int p0, p1;                // sorted pairs
-    long long base, scratch;   // scratch offset of p0, bytes of the chunk's units
+    int u0, u1;                // queue positions
+    long long base, scratch;   // scratch offset of u0, bytes of the chunk's units
     long long groups, batches, parts;
   };
   struct Order {
     std::vector<Chunk> chunks;
-    int chunkAt;               // position of the order in DevJob::chunkPairs
+    int chunkAt;               // position of the order in DevJob::chunkUnits
   } order[3];
   size_t bytes = 0;            // scratch buffer, work lists included
 };

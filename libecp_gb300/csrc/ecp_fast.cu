@@ -1664,10 +1664,13 @@ __global__ void __launch_bounds__(kScreenThreads) k_screen_scatter(DevJob J, lon
   for (int w = 0; w < warp; w++) at += warpCnt[w];
   if (live) J.live[at] = (int)i;
   else J.status[unit_at(J, (int)i)] = kUnitSkipped;
-  if ((int)i % J.nCentres == 0)
+  int k = 0;  // the chunk that starts here, if one does
 #pragma unroll 1
-    for (int k = 0; k < J.nChunks; k++)
-      if (J.chunkPair[k] == (int)i / J.nCentres) J.liveStart[k] = at;
+  for (int hi = J.nChunks; hi - k > 1;) {
+    const int mid = (k + hi) >> 1;
+    if (J.chunkUnit[mid] <= (int)i) k = mid; else hi = mid;
+  }
+  if (J.chunkUnit[k] == (int)i) J.liveStart[k] = at;
 }
 
 // --------------------------------------------------------------- launchers

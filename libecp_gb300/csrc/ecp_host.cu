@@ -549,8 +549,9 @@ static bool plain_stages(const Parsed &P, int mode) {
 // la; within a class by that cost), ties in the reference's order; every
 // pair's units consecutive, centres by descending L -- and their chunks.
 static void make_plan(const Parsed &P, size_t cap, bool single, JobPlan &plan, std::vector<int> &orders,
-                      std::vector<long long> &offs, std::vector<int> &chunkPairs, std::vector<int> &ctr) {
+                      std::vector<long long> &offs, std::vector<int> &chunkUnits, std::vector<int> &ctr) {
   const int n = P.nPairs;
+  cap = std::max(cap, kScratchFloor);
   std::vector<int> cost(n), cls(n);
   std::vector<PairPlan> pp(n);
   for (int p = 0; p < n; p++) {
@@ -564,7 +565,7 @@ static void make_plan(const Parsed &P, size_t cap, bool single, JobPlan &plan, s
   std::stable_sort(ctr.begin(), ctr.end(), [&](int a, int b) { return P.ctrL[a] > P.ctrL[b]; });
   orders.resize(3 * (size_t)n);
   offs.resize(3 * (size_t)(n + 1));
-  chunkPairs.clear();
+  chunkUnits.clear();
   plan.bytes = 0;
   // a stable counting sort by cost serves both sorted orders
   std::vector<int> byCost(n), start;
@@ -589,31 +590,39 @@ static void make_plan(const Parsed &P, size_t cap, bool single, JobPlan &plan, s
     long long *off = offs.data() + (size_t)o * (n + 1);
     JobPlan::Order &O = plan.order[o];
     O.chunks.clear();
-    O.chunkAt = (int)chunkPairs.size();
+    O.chunkAt = (int)chunkUnits.size();
     long long at = 0, lists = 0;
     JobPlan::Chunk ch{0, 0, 0, 0, 0, 0, 0};
     const long long nc = P.nCentres;
-    auto close = [&](int p) {
-      ch.p1 = p;
+    auto close = [&](int u) {
+      ch.u1 = u;
       ch.scratch = at - ch.base;
       O.chunks.push_back(ch);
-      chunkPairs.push_back(ch.p0);
+      chunkUnits.push_back(ch.u0);
       plan.bytes = std::max(plan.bytes, (size_t)(ch.scratch + lists));
-      ch = {p, 0, at, 0, 0, 0, 0};
+      ch = {u, 0, at, 0, 0, 0, 0};
       lists = 0;
     };
     for (int i = 0; i < n; i++) {
       const PairPlan &q = pp[ord[i]];
-      if (i > ch.p0 && (size_t)(at - ch.base + lists + nc * (q.scratch + q.lists)) > cap) close(i);
+      const long long b = q.scratch + q.lists, u = i * nc;
       off[i] = at;
-      at += nc * q.scratch;
-      lists += nc * q.lists;
-      ch.groups += nc * q.groups;
-      ch.batches += nc * q.batches;
-      ch.parts += nc * q.parts;
+      // a pair's units stay in one chunk where they fit one
+      if (u > ch.u0 && (size_t)(at - ch.base + lists + nc * b) > cap) close((int)u);
+      const long long most = std::max(1ll, (long long)cap / b);
+      for (long long c = 0; c < nc;) {
+        const long long m = std::min(most, nc - c);
+        at += m * q.scratch;
+        lists += m * q.lists;
+        ch.groups += m * q.groups;
+        ch.batches += m * q.batches;
+        ch.parts += m * q.parts;
+        c += m;
+        if (c < nc) close((int)(u + c));
+      }
     }
     off[n] = at;
-    if (n) close(n);
+    if (n) close((int)(n * nc));
   }
 }
 
@@ -649,13 +658,13 @@ static bool single_pair_parts(const Parsed &P, int mode) {
 
 bool job_device_bytes(const Parsed &P, int mode, size_t budget, JobBytes *need, size_t *scratchCap) {
   JobPlan plan;
-  std::vector<int> orders, chunkPairs, ctr;
+  std::vector<int> orders, chunkUnits, ctr;
   std::vector<long long> offs;
   const bool single = single_pair_parts(P, mode);
   size_t stages;
   // (a smaller scratch means more chunks, whose list takes a little more of the inputs)
   for (size_t cap = kScratchCap;;) {
-    make_plan(P, cap, single, plan, orders, offs, chunkPairs, ctr);
+    make_plan(P, cap, single, plan, orders, offs, chunkUnits, ctr);
     *need = job_bytes(P, mode, plan, &stages);
     *scratchCap = cap;
     const size_t base = need->total() - need->b[kJobBufs - 1];
@@ -716,11 +725,11 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
          iTL = add(P.termL.data(), 4 * P.termL.size()), iPrA = add(P.pairA.data(), 4 * P.pairA.size()),
          iPrB = add(P.pairB.data(), 4 * P.pairB.size()), iPO = add(P.pairOff.data(), 8 * P.pairOff.size()),
          iPS = add(P.pairShift.data(), 4 * P.pairShift.size()), iCh = add(P.chanT0.data(), 4 * P.chanT0.size());
-  std::vector<int> orders, chunkPairs, ctr;
+  std::vector<int> orders, chunkUnits, ctr;
   std::vector<long long> offs;
-  make_plan(P, scratchCap, J.single, B.plan, orders, offs, chunkPairs, ctr);
+  make_plan(P, scratchCap, J.single, B.plan, orders, offs, chunkUnits, ctr);
   size_t iOrd = add(orders.data(), 4 * orders.size()), iOff = add(offs.data(), 8 * offs.size()),
-         iChk = add(chunkPairs.data(), 4 * chunkPairs.size()), iCtr = add(ctr.data(), 4 * ctr.size());
+         iChk = add(chunkUnits.data(), 4 * chunkUnits.size()), iCtr = add(ctr.data(), 4 * ctr.size());
   std::vector<FxTerm> terms;
   for (size_t t = 0; t < P.termL.size() && !J.plain; t++) terms.push_back(fx_term(P.termA[t], P.termD[t], P.termN[t]));
   size_t iFx = add(terms.data(), sizeof(FxTerm) * terms.size());
@@ -781,7 +790,7 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.plan = &B.plan;
   J.pairOrders = (const int *)dp(iOrd);
   J.scrOffs = (const long long *)dp(iOff);
-  J.chunkPairs = (const int *)dp(iChk);
+  J.chunkUnits = (const int *)dp(iChk);
   J.ctrOrder = (const int *)dp(iCtr);
   J.gcap = FastConfig{}.gcap;
   J.besH = T->besH.p;

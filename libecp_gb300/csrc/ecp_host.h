@@ -223,6 +223,9 @@ struct DevTables;
 // A job's units run in chunks whose scratch stays within scratchCap (1 or 4 GiB
 // take 0.3 % off the largest jobs' unit stages, 47.5 -> 47.3 ms).
 constexpr size_t kScratchCap = 512ull << 20;
+// No cap makes chunks smaller than this (or than one unit): their list and their
+// launches would cost more than the scratch they save.
+constexpr size_t kScratchFloor = 256ull << 10;
 int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int mode, cudaStream_t stream,
               size_t scratchCap = kScratchCap);
 // Resets the run's words and launches the pipeline of the mode on `stream`;
@@ -232,7 +235,7 @@ int run_pipeline(JobBuffers &B, const DevJob &J, int mode, cudaEvent_t u0, cudaE
 // Device bytes of a job of P where at most `budget` may be held, and the scratch
 // cap to stage it with; false where its buffers without the unit stages' plan and
 // scratch are above the budget.  The scratch takes what the budget leaves, down to
-// one pair's units (which a job within that distance of the budget holds above it).
+// kScratchFloor or one unit's (which a job that close to the budget holds above it).
 bool job_device_bytes(const Parsed &P, int mode, size_t budget, JobBytes *need, size_t *scratchCap);
 // With the engine lock held: the tables of the request and, unless requests
 // in flight pin other level schedules (returns 4: retry after they finish),

@@ -838,7 +838,7 @@ static const JobPlan::Order &use_order(DevJob &J, int sorted) {
   const JobPlan::Order &ord = J.plan->order[sorted];
   J.pairOrder = J.pairOrders + (size_t)sorted * J.nPairs;
   J.scrOff = J.scrOffs + (size_t)sorted * (J.nPairs + 1);
-  J.chunkPair = J.chunkPairs + ord.chunkAt;
+  J.chunkUnit = J.chunkUnits + ord.chunkAt;
   J.nChunks = (int)ord.chunks.size();
   return ord;
 }
@@ -855,8 +855,8 @@ static void launch_chunks(DevJob J, const JobPlan::Order &ord, cudaStream_t st, 
   for (int k = 0; k < J.nChunks; k++) {
     const JobPlan::Chunk &ch = ord.chunks[k];
     J.chunk = k;
-    J.chunk0 = ch.p0 * J.nCentres;
-    J.chunk1 = ch.p1 * J.nCentres;
+    J.chunk0 = ch.u0;
+    J.chunk1 = ch.u1;
     J.scrBase = ch.base;
     char *lists = J.scr + ch.scratch;
     J.listT1 = (int2 *)lists;

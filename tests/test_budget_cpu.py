@@ -76,3 +76,22 @@ def test_a_job_stays_within_its_budget(probe, name, mode):
         # within the budget, but where the scratch is at its smallest (one entry)
         assert ok and (need <= budget or scr > cap + 16), (k, need, budget, scr, cap)
     assert not probe(s, mode, other // 2)[0]
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_the_smallest_scratch_is_one_unit(probe, mode):
+    """40 centres on one shell pair of 16 x 16 primitives: a chunk may be a single
+    unit of the 40."""
+    b = W._Builder()
+    shell = (4, [(0.1 + 0.05 * i, 0.05 * 1.7 ** i) for i in range(16)])
+    for i in range(40):
+        b.atom([0.5 * i, 0.1, 0.0], ecp=[(l, [(2.0, 1.0, 1.0)]) for l in range(4)], shells=[shell] if i == 0 else [])
+    s = b.build("one_pair")
+    ok, full, scratch, _ = probe(s, mode, 1 << 40)
+    other = full - scratch
+    one = -(-(scratch - 16) // 40)
+    # the screening stage's and the plan's lists of 40 chunks take some more
+    ok, need, scr, _ = probe(s, mode, other + one + 8192)
+    assert ok and need <= other + one + 8192 and scr <= one + 4096
+    ok, need, scr, _ = probe(s, mode, other)
+    assert ok and scr <= one + 4096
