@@ -636,11 +636,18 @@ static size_t input_bytes(const Parsed &P, int mode, size_t chunks, size_t *stag
          24 * 256 + *stages;
 }
 
+// Ranks of the r^k U_l and F tables (HostTables::nk, nF).
+static int table_nk(const Parsed &P) {
+  const int LB = P.maxLBS + P.deriv;
+  return std::max(P.maxLECP - 1 + LB, 2 * LB) + 1;
+}
+static int table_nF(const Parsed &P) { return std::max(P.maxLECP + P.maxLBS + P.deriv, 1); }
+
 // The bytes of a job's device buffers under its plan.
 static JobBytes job_bytes(const Parsed &P, int mode, const JobPlan &plan, size_t *stages) {
   const size_t nc = P.nCentres, ns = P.nShells, na = P.nAtoms, O = kSmallOrder, nu = nc * P.nPairs;
   const size_t LE = P.maxLECP > 0 ? P.maxLECP : 1, LB = P.maxLBS + P.deriv;
-  const size_t nk = std::max(LB + LE, 2 * LB) + 1, nF = LB + LE + 1, D = LB + 1;  // table ranks (upper bounds)
+  const size_t nk = table_nk(P), nF = table_nF(P), D = LB + 1;
   const size_t angLam = P.maxLECP + LB + 1, angC = (LB + 1) * (LB + 2) * (LB + 3) / 6;
   size_t chunks = 0;
   for (const JobPlan::Order &o : plan.order) chunks = std::max(chunks, o.chunks.size());
@@ -685,6 +692,10 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
     set_error("job has %lld units; at most %d run in one job", units, INT_MAX);
     return -1;
   }
+  if (h.nk != table_nk(P) || h.nF != table_nF(P)) {
+    set_error("table ranks %d, %d differ from the job's", h.nk, h.nF);
+    return -1;
+  }
   std::memset(&J, 0, sizeof J);
   J.plain = plain_stages(P, mode);
   const long long np = primitive_pairs(P);
@@ -705,6 +716,20 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.tol = P.tol; J.acc = P.acc;
   J.lnAcc1 = std::log(P.acc) - 2;
   J.lnAcc2 = std::log(1.0E-14) - 2;
+  // --- the plan and the device buffers: where they cannot be had, with less scratch
+  std::vector<int> orders, chunkUnits, ctr;
+  std::vector<long long> offs;
+  JobBytes need;
+  for (size_t cap = scratchCap, stages;; cap /= 4) {
+    make_plan(P, cap, J.single, B.plan, orders, offs, chunkUnits, ctr);
+    need = job_bytes(P, mode, B.plan, &stages);
+    if (B.reserve(need)) break;
+    cudaGetLastError();  // the launches' own check must not find it
+    if (cap <= kScratchFloor) {
+      set_error("device allocation of the job's %zu bytes failed", need.total());
+      return -1;
+    }
+  }
   // --- inputs: one packed H2D copy
   struct Piece { const void *src; size_t bytes; size_t off; };
   std::vector<Piece> pcs;
@@ -725,9 +750,6 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
          iTL = add(P.termL.data(), 4 * P.termL.size()), iPrA = add(P.pairA.data(), 4 * P.pairA.size()),
          iPrB = add(P.pairB.data(), 4 * P.pairB.size()), iPO = add(P.pairOff.data(), 8 * P.pairOff.size()),
          iPS = add(P.pairShift.data(), 4 * P.pairShift.size()), iCh = add(P.chanT0.data(), 4 * P.chanT0.size());
-  std::vector<int> orders, chunkUnits, ctr;
-  std::vector<long long> offs;
-  make_plan(P, scratchCap, J.single, B.plan, orders, offs, chunkUnits, ctr);
   size_t iOrd = add(orders.data(), 4 * orders.size()), iOff = add(offs.data(), 8 * offs.size()),
          iChk = add(chunkUnits.data(), 4 * chunkUnits.size()), iCtr = add(ctr.data(), 4 * ctr.size());
   std::vector<FxTerm> terms;
@@ -741,14 +763,9 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
     split_pairs(P.termA, tAf);
     split_pairs(P.termD, tDf);
   }
-  size_t iTAf = add(tAf.data(), 4 * tAf.size()), iTDf = add(tDf.data(), 4 * tDf.size()), stages;
-  const JobBytes need = job_bytes(P, mode, B.plan, &stages);
+  size_t iTAf = add(tAf.data(), 4 * tAf.size()), iTDf = add(tDf.data(), 4 * tDf.size());
   if (tot > need.b[0] || !B.pinned.ensure(tot)) {
     set_error("allocation of %zu input bytes failed", tot);
-    return -1;
-  }
-  if (!B.reserve(need)) {
-    set_error("device allocation of the job's %zu bytes failed", need.total());
     return -1;
   }
   for (auto &p : pcs)
