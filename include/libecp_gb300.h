@@ -124,7 +124,12 @@ int ecpgb_gradient(const ecpgb_system *s, int mode, const double *D, int ldD, do
 /* Device-resident job: inputs are copied to HBM once; ecpgb_job_run then
  * re-runs the whole pipeline (all kernels) nRuns times without host traffic,
  * writing one device-time per run (CUDA events on the engine's stream) to
- * msRun and the unit stages' time to msUnit (either may be NULL).  With
+ * msRun and the unit stages' time to msUnit (either may be NULL).  Device
+ * memory: a job holds its inputs and work arrays; the scratch between the unit
+ * stages (at most 512 MiB, or one unit's where that is more; smaller chunks of
+ * units where it cannot be allocated) is one for all resident jobs and one-shot
+ * calls of the process and is given back with the last resident job, unless
+ * one-shot calls, which keep their buffers, have used as much.  With
  * flushL2 != 0 a 256 MiB buffer is written between runs, outside the timed
  * spans, so no run starts with a warm L2. */
 typedef struct ecpgb_job ecpgb_job;
@@ -184,8 +189,12 @@ int ecpgb_job_blocks(ecpgb_job *j, double *values, int *status);
  * jobs in arrival order as slots and device memory free up: each admitted
  * job is staged and run on its own CUDA stream while earlier ones are still
  * on the GPU, so their kernels overlap; the device-resident tables are shared
- * by all of them.  hbmBudgetBytes caps the device bytes the slots hold (a job
- * larger than the budget fails); slots caps the jobs in flight (1..64).  mode
+ * by all of them.  hbmBudgetBytes caps the device bytes the slots hold, the
+ * scratch between the unit stages included: a job takes up to 512 MiB of it,
+ * or what the budget leaves, in smaller chunks.  A job whose other buffers are
+ * above the budget fails; one that leaves less than the smallest scratch (256
+ * KiB or one unit's) runs alone and holds that much more.  slots caps the jobs
+ * in flight (1..64).  mode
  * is ECPGB_FP64 or ECPGB_FAST for every job of the server.  Results are those
  * of ecpgb_getIntegrals for the same system, mode and launch configuration,
  * bit for bit: a job runs the same kernels in the mix as alone. */

@@ -276,7 +276,13 @@ struct Engine {
   }
   std::vector<std::unique_ptr<DevTables>> tables;
   const DevTables *schedOwner = nullptr;
-  JobBuffers shared;
+  // the scratch of every job on `stream` -- one-shot calls and resident jobs run one
+  // after another there; it only grows, until the last resident job gives it back
+  DBuf<char> scr;
+  size_t oneShotScr = 0;  // the most that one-shot calls took of it
+  int residents = 0;
+  JobBuffers shared;  // of the one-shot calls
+  Engine() { shared.scr = &scr; }
   DBuf<char> flush;
   DBuf<unsigned long long> classCycles;  // autotuner: per-class cycle counts
   DBuf<double> dens, gradBuf;  // density matrix and gradient of run_gradient
@@ -802,7 +808,8 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.live = B.live.p;
   J.liveStart = B.liveStart.p;
   J.screenBlocks = B.screenBlocks.p;
-  J.scr = B.scr.p;
+  J.scr = B.scr->p;
+  if (&B == &engine().shared) engine().oneShotScr = std::max(engine().oneShotScr, B.plan.bytes);
   J.counters = (unsigned *)(B.err.p + 2);
   J.plan = &B.plan;
   J.pairOrders = (const int *)dp(iOrd);
@@ -1115,6 +1122,13 @@ struct ResidentJob {
   }
 };
 
+// The shared scratch as it is now: another job may have had it grown (engine lock held).
+static void bind_scratch(Engine &E, ResidentJob *R) {
+  if (R->J.scr == E.scr.p) return;
+  R->J.scr = E.scr.p;
+  R->drop_graph();
+}
+
 // Captures the job's pipeline into R->graph (engine lock held).
 static int capture_graph(Engine &E, ResidentJob *R) {
   if (R->graph) return 0;
@@ -1148,6 +1162,7 @@ void *job_create(const ecpgb_system &s, int mode) {
   if (E.ensure_init()) return nullptr;
   auto *R = new ResidentJob();
   R->mode = mode;
+  R->B.scr = &E.scr;
   if (parse_system(s, R->P)) { delete R; return nullptr; }
   if (R->P.nCentres == 0 || R->P.nPairs == 0) { set_error("job has no units"); delete R; return nullptr; }
   R->T = E.get_tables(table_key(R->P));
@@ -1157,6 +1172,7 @@ void *job_create(const ecpgb_system &s, int mode) {
   // skipped units are never written: their values read as zero
   cudaMemsetAsync(R->B.out.p, 0, sizeof(double) * (size_t)R->P.nCentres * R->P.centreStride, E.stream);
   if (cudaStreamSynchronize(E.stream) != cudaSuccess) { set_error("staging failed"); delete R; return nullptr; }
+  E.residents++;
   return R;
 }
 
@@ -1165,6 +1181,7 @@ int job_run(void *vj, int nRuns, int flushL2, float *msRun, float *msUnit) {
   std::unique_lock<std::mutex> lk(E.mu);
   auto *R = (ResidentJob *)vj;
   if (E.use_schedules(R->T, &lk)) return 1;
+  bind_scratch(E, R);
   const size_t flushBytes = 256u << 20;
   if (flushL2 && !E.flush.ensure(flushBytes)) { set_error("flush buffer allocation failed"); return 1; }
   if (R->useGraph) {
@@ -1242,6 +1259,7 @@ int job_tune(void *vj, ecpgb_launch_config *chosen, ecpgb_launch_config *trials,
   if (nTrials) *nTrials = 0;
   if (R->mode == ECPGB_FP64) { set_error("the autotuner applies to the batched path only"); return 3; }
   if (E.use_schedules(R->T, &lk)) return 1;
+  bind_scratch(E, R);
   // candidates: live units only or all, the queue's orders, and the
   // step-table cap (pairs per warp against CTAs per SM)
   std::vector<FastConfig> cand;
@@ -1454,6 +1472,8 @@ void job_free(void *vj) {
   std::lock_guard<std::mutex> lk(E.mu);
   cudaStreamSynchronize(E.stream);
   delete (ResidentJob *)vj;
+  // one-shot calls keep theirs, as they keep their other buffers
+  if (--E.residents == 0 && E.scr.cap > 2 * E.oneShotScr) E.scr.release(nullptr);
 }
 
 }  // namespace ecpgb

@@ -70,6 +70,16 @@ struct DBuf {
     cap = n;
     return true;
   }
+  // Like ensure, but the memory held stays until the larger one is there.
+  bool grow(size_t n) {
+    if (n <= cap) return true;
+    T *q = nullptr;
+    if (cudaMalloc((void **)&q, n * sizeof(T)) != cudaSuccess) return false;
+    if (p) cudaFree(p);
+    p = q;
+    cap = n;
+    return true;
+  }
   // Releases the memory, ordered on stream s (null: cudaFree).
   void release(cudaStream_t s) {
     if (p) {
@@ -142,7 +152,8 @@ struct JobBuffers {
   DBuf<double> radius, utab, uL, F, cgeo, usp, ang, out, mat;
   DBuf<int> gridEnd, win, status, err;
   DBuf<int> live, screenBlocks, liveStart;  // screening stage of the batched path
-  DBuf<char> scr;                // scratch between the unit stages
+  DBuf<char> ownScr;             // scratch between the unit stages: a server slot's own,
+  DBuf<char> *scr = &ownScr;     // or the one that all jobs of the engine's stream share
   JobPlan plan;
   DBuf<double> sout;       // spherical blocks
   DBuf<long long> sphOff;  // their per-entry offsets
@@ -154,7 +165,7 @@ struct JobBuffers {
   template <class F_>
   void each(F_ f) {
     f(in); f(radius); f(utab); f(uL); f(F); f(cgeo); f(usp); f(ang); f(out); f(mat);
-    f(gridEnd); f(win); f(status); f(err); f(live); f(screenBlocks); f(liveStart); f(scr);
+    f(gridEnd); f(win); f(status); f(err); f(live); f(screenBlocks); f(liveStart); f(*scr);
   }
   // Device bytes held, and what they will be once a job of `need` is staged (a
   // buffer keeps the larger size).
@@ -169,7 +180,11 @@ struct JobBuffers {
   bool reserve(const JobBytes &need) {
     bool ok = true;
     int i = 0;
-    each([&](auto &d) { ok = d.ensure((need.b[i++] + sizeof(*d.p) - 1) / sizeof(*d.p)) && ok; });
+    each([&](auto &d) {
+      const size_t n = (need.b[i++] + sizeof(*d.p) - 1) / sizeof(*d.p);
+      // (resident jobs are planned for the shared scratch as it is)
+      ok = ((void *)&d == (void *)scr && scr != &ownScr ? d.grow(n) : d.ensure(n)) && ok;
+    });
     return ok;
   }
   // Releases the device buffers (ordered on stream s); they grow again on use.
@@ -220,8 +235,10 @@ bool valid_mode(int mode);
 struct DevTables;
 // Packs P's inputs into B's pinned buffer, copies them to the device on
 // `stream` and fills J (B's buffers grow as needed).
-// A job's units run in chunks whose scratch stays within scratchCap (1 or 4 GiB
-// take 0.3 % off the largest jobs' unit stages, 47.5 -> 47.3 ms).
+// A job's units run in chunks whose scratch stays within scratchCap.  Unit stages
+// of the 50-centre cluster, the 83-shell g batch and the 150-shell sweep (ms) with
+// 512 MiB: 36.9, 30.5, 47.4; 256: 37.0, 31.2, 48.2; 128: 37.4, 34.6, 51.5; 64: 38.6,
+// 38.0, 58.4 (a chunk's last entries leave the GPU idle); 1 and 4 GiB take 0.3 % off.
 constexpr size_t kScratchCap = 512ull << 20;
 // No cap makes chunks smaller than this (or than one unit): their list and their
 // launches would cost more than the scratch they save.

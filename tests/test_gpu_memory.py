@@ -68,3 +68,55 @@ def test_scratch_that_cannot_be_had(tmp_path, mode):
     r = subprocess.run([sys.executable, "-c", SCRIPT, mode], cwd=ROOT, capture_output=True, text=True, timeout=300,
                        env=dict(os.environ, PYTHONPATH=ROOT, LD_PRELOAD=so))
     assert r.returncode == 0 and "same" in r.stdout, r.stderr[-2000:]
+
+
+SHARED = """
+import ctypes as ct, sys
+import numpy as np
+import libecp_gb300 as eg
+from libecp_gb300 import workloads as W
+rt = ct.CDLL("libcudart.so.13")
+def free_bytes():
+    f, t = ct.c_size_t(0), ct.c_size_t(0)
+    assert rt.cudaMemGetInfo(ct.byref(f), ct.byref(t)) == 0
+    return f.value
+mode = getattr(eg, sys.argv[1])
+small, large = (W.batched_cluster(0, n_centres=8, n_basis_atoms=n) for n in (12, 20))
+eg.get_integrals_info(W.batched_cluster(0, n_centres=1, n_basis_atoms=3), mode=mode)
+jobs = [eg.Job(small, mode=mode)]
+def run(job):
+    job.run(1, flush_l2=False)
+    return job.matrix()
+first = run(jobs[0])
+f0 = free_bytes()
+job = eg.Job(large, mode=mode)
+run(job)
+assert free_bytes() < f0 - (50 << 20)  # grown by 62 MB (batched) or more
+job.close()
+jobs[0].close()  # the last one gives the scratch back
+assert free_bytes() > f0 - (8 << 20)
+jobs[0] = eg.Job(small, mode=mode)
+assert np.array_equal(run(jobs[0]), first)
+jobs.append(eg.Job(large, mode=mode))  # the scratch grows under the first job's captured graph
+second = run(jobs[1])
+assert np.array_equal(run(jobs[0]), first)
+f0 = free_bytes()
+for _ in range(4):
+    jobs.append(eg.Job(large, mode=mode))
+per_job = (f0 - free_bytes()) / 4
+assert all(np.array_equal(run(j), second) for j in jobs[2:])
+assert np.array_equal(eg.get_integrals_info(large, mode=mode)[1], second)
+assert np.array_equal(run(jobs[0]), first) and np.array_equal(run(jobs[1]), second)
+for j in jobs:
+    j.close()
+# inputs and work arrays are 18 MB, the scratch 99 (batched) or 174 MB (plain)
+assert per_job <= 40 << 20, per_job
+print("shared")
+"""
+
+
+@pytest.mark.parametrize("mode", ["ECPGB_FP64", "ECPGB_FAST"])
+def test_resident_jobs_share_the_scratch(mode):
+    r = subprocess.run([sys.executable, "-c", SHARED, mode], cwd=ROOT, capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, PYTHONPATH=ROOT))
+    assert r.returncode == 0 and "shared" in r.stdout, r.stderr[-2000:]
