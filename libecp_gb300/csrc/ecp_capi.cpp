@@ -108,7 +108,7 @@ libECPHandle *libECP_init(int nrAtoms, double *geometry, int *shellsECP, int *lE
     return nullptr;
   }
   ecpgb::HostTables t;
-  ecpgb::build_tables(ecpgb::table_key(P), t);
+  ecpgb::build_tables(ecpgb::table_key(P), t, false);
   if (t.status) {  // e.g. the Bessel series does not converge (src/libecp.c:181-185)
     delete h;
     return nullptr;

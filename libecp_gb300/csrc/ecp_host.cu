@@ -263,6 +263,8 @@ static bool same_schedules(const DevTables *a, const DevTables *b) {
          a->host.s93.lvEnd == b->host.s93.lvEnd && a->host.s92.lvEnd == b->host.s92.lvEnd;
 }
 
+static bool plain_stages(const Parsed &P, int mode);
+
 struct Engine {
   std::mutex mu;
   cudaStream_t stream = nullptr;
@@ -301,7 +303,20 @@ struct Engine {
     return 0;
   }
 
-  const DevTables *get_tables(const TableKey &key) {
+  // The tables of a job; the batched path's fixed-point rows from its first job on.
+  const DevTables *get_tables(const Parsed &P, int mode) {
+    DevTables *t = plain_tables(table_key(P));
+    if (!t || plain_stages(P, mode) || t->besXA.p) return t;
+    bessel_fixed(t->host);
+    if (!t->besX.upload(t->host.besselX, stream) || !t->besXA.upload(t->host.besselXA, stream)) {
+      t->besXA.release(nullptr);
+      set_error("device allocation failed for tables");
+      return nullptr;
+    }
+    return t;
+  }
+
+  DevTables *plain_tables(const TableKey &key) {
     for (auto &t : tables)
       if (t->key == key) return t.get();
     if (tables.size() >= 256) {
@@ -310,7 +325,7 @@ struct Engine {
     }
     auto t = std::make_unique<DevTables>();
     t->key = key;
-    build_tables(key, t->host);
+    build_tables(key, t->host, false);
     if (t->host.status) {
       set_error(t->host.status == 1 ? "Bessel series did not converge" : "table sizes out of range");
       return nullptr;
@@ -324,8 +339,7 @@ struct Engine {
               t->ijkIdx.upload(h.ijkIndex, stream) && t->besH.upload(h.besselH, stream) && t->besA.upload(h.besselA, stream) && t->besHf.upload(h.besselHf, stream) &&
               t->besAf.upload(h.besselAf, stream) && t->besZf.upload(h.besselZf, stream) &&
               t->wlf.upload(h.wlf, stream) &&
-              t->besZ.upload(h.besselZ, stream) && t->besX.upload(h.besselX, stream) &&
-              t->besXA.upload(h.besselXA, stream) &&
+              t->besZ.upload(h.besselZ, stream) &&
               t->c2s.upload(h.cart2sph, stream) && t->s93.upload(h.s93.slot, stream) &&
               t->s92.upload(h.s92.slot, stream) && t->byN93.upload(by_point_order(h.s93.slot), stream) &&
               t->shNorm.upload(h.shNorm, stream);
@@ -437,10 +451,10 @@ static Engine &engine() {
 
 std::mutex &engine_mutex() { return engine().mu; }
 void schedules_overwritten() { engine().schedOwner = nullptr; }
-int engine_pin_request(const Parsed &P, const DevTables **T) {
+int engine_pin_request(const Parsed &P, int mode, const DevTables **T) {
   Engine &E = engine();
   if (E.ensure_init()) return 1;
-  const DevTables *t = E.get_tables(table_key(P));
+  const DevTables *t = E.get_tables(P, mode);
   if (!t) return 1;
   if (E.schedPins > 0 && E.schedOwner != t && !(E.schedOwner && same_schedules(E.schedOwner, t))) return 4;
   if (E.use_schedules(t)) return 1;
@@ -871,7 +885,7 @@ int run_matrix(const ecpgb_system &s, int mode, int rowdim, double *I, ecpgb_inf
     if (info) { std::memset(info, 0, sizeof *info); info->firstFailed = -1; }
     return 0;
   }
-  const DevTables *T = E.get_tables(table_key(P));
+  const DevTables *T = E.get_tables(P, mode);
   if (!T || E.use_schedules(T, &lk)) return 1;
   JobBuffers &B = E.shared;
   DevJob J;
@@ -921,7 +935,7 @@ int run_blocks(const ecpgb_system &s, int mode, double *values, long long *offse
     if (info) { std::memset(info, 0, sizeof *info); info->firstFailed = -1; }
     return 0;
   }
-  const DevTables *T = E.get_tables(table_key(P));
+  const DevTables *T = E.get_tables(P, mode);
   if (!T || E.use_schedules(T, &lk)) return 1;
   JobBuffers &B = E.shared;
   DevJob J;
@@ -988,7 +1002,7 @@ int run_gradient(const ecpgb_system &s0, int mode, const double *D, int ldD, dou
       else std::memset(grad, 0, sizeof(double) * 3 * P.nAtoms);
       continue;
     }
-    const DevTables *T = E.get_tables(table_key(P));
+    const DevTables *T = E.get_tables(P, mode);
     if (!T || E.use_schedules(T, &lk)) return 1;
     JobBuffers &B = E.shared;
     DevJob J;
@@ -1049,7 +1063,7 @@ int run_blocks_sph(const ecpgb_system &s, int mode, double *values, long long *o
   if (parse_system(s, P)) return 1;
   const long long nUnits = (long long)P.nCentres * P.nPairs;
   if (nUnits == 0) return 0;
-  const DevTables *T = E.get_tables(table_key(P));
+  const DevTables *T = E.get_tables(P, mode);
   if (!T || E.use_schedules(T, &lk)) return 1;
   JobBuffers &B = E.shared;
   DevJob J;
@@ -1080,7 +1094,7 @@ int run_blocks_sph(const ecpgb_system &s, int mode, double *values, long long *o
 int cart2sph_table(int l, double *out) {
   if (l < 0 || l > kMaxLBasis) { set_error("l %d outside 0..%d", l, kMaxLBasis); return 1; }
   HostTables t;
-  build_tables({1, kMaxLBasis, 1024, 1e-12, 1e-14, {}}, t);
+  build_tables({1, kMaxLBasis, 1024, 1e-12, 1e-14, {}}, t, false);
   if (t.status) { set_error("table build failed"); return 1; }
   size_t o = 0;
   for (int k = 0; k < l; k++) o += (size_t)(2 * k + 1) * ncart(k);
@@ -1165,7 +1179,7 @@ void *job_create(const ecpgb_system &s, int mode) {
   R->B.scr = &E.scr;
   if (parse_system(s, R->P)) { delete R; return nullptr; }
   if (R->P.nCentres == 0 || R->P.nPairs == 0) { set_error("job has no units"); delete R; return nullptr; }
-  R->T = E.get_tables(table_key(R->P));
+  R->T = E.get_tables(R->P, mode);
   if (!R->T || stage_job(R->P, R->T, R->B, R->J, mode, E.stream)) { delete R; return nullptr; }
   R->cfg = E.config_for(R->J.maxLBS, R->J.maxLECP);
 

@@ -257,7 +257,7 @@ bool job_device_bytes(const Parsed &P, int mode, size_t budget, JobBytes *need, 
 // With the engine lock held: the tables of the request and, unless requests
 // in flight pin other level schedules (returns 4: retry after they finish),
 // its schedules made current and pinned.  0 ok, 1 error.
-int engine_pin_request(const Parsed &P, const DevTables **T);
+int engine_pin_request(const Parsed &P, int mode, const DevTables **T);
 // With the engine lock held: releases one pin.
 void engine_unpin_request();
 // Server objects (ecp_serve.cpp).

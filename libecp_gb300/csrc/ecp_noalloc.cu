@@ -89,7 +89,7 @@ int run_matrix_noalloc(const ecpgb_system &s, int rowdim, double *I) {
   if (P.deriv) { set_error("the AO matrix exists for derivative order 0 only"); return 1; }
   if (P.nCentres == 0 || P.nPairs == 0) return 0;
   HostTables h;
-  build_tables(table_key(P), h);
+  build_tables(table_key(P), h, false);
   if (h.status) {
     set_error(h.status == 1 ? "Bessel series did not converge" : "table sizes out of range");
     return 1;

@@ -109,7 +109,7 @@ struct Server {
     Slot &s = *slots[k];
     const DevTables *T = nullptr;
     std::unique_lock<std::mutex> lk(engine_mutex());
-    int rc = engine_pin_request(r->P, &T);
+    int rc = engine_pin_request(r->P, mode, &T);
     if (rc == 4) return 4;
     if (rc) {
       r->err = last_error();

@@ -338,7 +338,7 @@ static void omega_table(HostTables &t) {
     }
 }
 
-void build_tables(const TableKey &key, HostTables &t) {
+void build_tables(const TableKey &key, HostTables &t, bool fixed) {
   t = HostTables();
   t.key = key;
   t.maxLECP = key.maxLECP;
@@ -392,7 +392,7 @@ void build_tables(const TableKey &key, HostTables &t) {
   if (t.maxLECP > 0) omega_table(t);
   else t.omega.assign(1, 0.0);
   bessel_horner(t);
-  bessel_fixed(t);
+  if (fixed) bessel_fixed(t);
   const int W = t.tmDim + 1;
   t.shNorm.assign((size_t)W * W, 0.0);
   for (int l = 0; l < W; l++) {
@@ -477,15 +477,17 @@ void bessel_fixed(HostTables &t) {
   // the rows of z = 0 (a shell on the ECP centre): 1, 0, 0, ...
   t.besselX[(size_t)N * (HL + 1) * 8] = (1ll << 62) - 1;
   for (int l = 0; l <= HL; l++) t.besselX[((size_t)N * (HL + 1) + l) * 8 + 6] = 62;
+  // sum_j q_j (h (2 X - 1/2))^j in powers of X: m[j][k] of X^k in the j-th power
+  long double m[6][6] = {{1.0L}};
+  for (int j = 1; j < 6; j++)
+    for (int k = 0; k <= j; k++) m[j][k] = (k ? 2 * h * m[j - 1][k - 1] : 0.0L) - 0.5L * h * m[j - 1][k];
   for (int i = 0; i < N; i++)
     for (int l = 0; l <= HL; l++) {
       const double *q = &t.besselH[((size_t)i * (HL + 1) + l) * 6];
-      // sum_j q_j (h (2 X - 1/2))^j in powers of X
-      long double c[6] = {0, 0, 0, 0, 0, 0}, d[6];
-      for (int j = 5; j >= 0; j--) {  // c = c * (2 h X - h/2) + q_j
-        for (int k = 5; k >= 0; k--) d[k] = (k ? 2 * h * c[k - 1] : 0.0L) - 0.5L * h * c[k];
-        for (int k = 0; k < 6; k++) c[k] = d[k];
-        c[0] += q[j];
+      long double c[6];
+      for (int k = 0; k < 6; k++) {
+        c[k] = q[k] * m[k][k];
+        for (int j = k + 1; j < 6; j++) c[k] += q[j] * m[j][k];
       }
       long long *out = &t.besselX[((size_t)i * (HL + 1) + l) * 8];
       fixed_row(c, 5, out, out[6]);

@@ -100,8 +100,10 @@ struct HostTables {
   int status = 0;                // 0 ok, 1 Bessel series did not converge, 3 sizes out of range
 };
 
-// Builds every table for the key.  status != 0 reports a failure.
-void build_tables(const TableKey &key, HostTables &t);
+// Builds every table for the key.  status != 0 reports a failure.  fixed = false
+// leaves out the fixed-point rows of the batched path (bessel_fixed; extended
+// precision, which takes an Arm host 10 ms in software).
+void build_tables(const TableKey &key, HostTables &t, bool fixed = true);
 void bessel_horner(HostTables &t);
 void bessel_fixed(HostTables &t);
 void split_pairs(const std::vector<double> &d, std::vector<float> &out);
