@@ -52,30 +52,9 @@ static __device__ __noinline__ void bessel_fx(const DevJob &J, int lmax, xf z100
   fx_bessel_rows(J.besX, J.besXA, J.besHL + 1, lmax, z100, mul, sign, K);
 }
 
-// The rows for the type-1 tables, K_l / c = K[l] 2^base with one base for the
-// even rows (K_0 normalised) and one for the odd rows (K_1 normalised): a
-// quadrature (l1, l2) and those it is added to read rows of one parity.
-struct RowBase {
-  xf c;
-  int even, odd;
-};
+// The rows for the type-1 tables.
 static __device__ __noinline__ RowBase bessel_rows2(const DevJob &J, int lmax, xf z100, u64 *K) {
-  RowBase b;
-  int base[2] = {0, 0};
-  b.c = fx_bessel(J.besX, J.besXA, J.besHL + 1, lmax, z100, [&](int l, u64 v, int scale) {
-    if (l < 2) {
-      const int n = clz64(v | 1u);
-      K[l] = v << n;
-      if (l == 0) base[0] = base[1] = -scale - n;
-      else if (v) base[1] = -scale - n;
-    } else {
-      const int sh = (l & 1 ? base[1] : base[0]) + scale;  // K_l <= K_(l-2)
-      K[l] = sh < 0 ? v << -sh : shr64(v, sh);
-    }
-  });
-  b.even = base[0];
-  b.odd = base[1];
-  return b;
+  return fx_bessel_packed(J.besX, J.besXA, J.besHL + 1, lmax, z100, K);
 }
 // Powers of r other than 0, 1, 2: rare, out of line.
 static __device__ __noinline__ double rpow_rare(double r, double n) { return rpow(r, n); }
@@ -436,12 +415,12 @@ static __device__ void rsh_column(const DevJob &J, int lmax, int m, double x, do
   }
 }
 
-// Type-1 table entries, 2 lq + 1 words: K_l (bessel_rows2), then normalised
-// mantissas of v r^l, then the exponents: of row l times K_l2's parity,
-// e + l er - (leading bits won back up to row l) - (l odd: odd).
+// Type-1 table entries, 2 lq + 1 words: K_l (fx_bessel_packed), then normalised
+// mantissas of v r^l, then the exponents: of row l1 times K_l2,
+// e + l1 er - (leading bits won back up to row l1) - l2 t - (K's low bits).
 struct EntInfo {
   int e;       // 2 e + sign
-  int packed;  // er (8 bits, signed), odd (8 bits), a bit per row whose product was shifted
+  int packed;  // er (8 bits, signed), t (16 bits), a bit per row l = 1..8 whose product was shifted
 };
 constexpr EntInfo kNoEntry = {-2000000, 0};
 // A point past the break: the entry holds doubles.
@@ -456,17 +435,18 @@ static __device__ inline EntInfo t1_entry_rows(u64 *WR, xf v, const RowBase &b, 
     m = mul_hi(m, R.m);
     if ((i64)m >= 0) {
       m += m;
-      won |= 1u << l;
+      won |= 1u << (23 + l);
     }
     WR[l] = m;
   }
-  const int odd = b.even - b.odd;
-  return {(v.e + b.even + 64) * 2 + (int)(sign >> 31), ((R.e + 64) & 255) | (odd > 255 ? 255 : odd) << 8 | (int)(won << 16)};
+  return {(v.e + b.e0 + 64) * 2 + (int)(sign >> 31), ((R.e + 64) & 255) | b.t << 8 | (int)won};
 }
 // The product of row l1 and K_l2 of an entry into a run.
-static __device__ inline void t1_entry_add(xf_run &run, u64 wr, u64 k, EntInfo f, int l1) {
-  const int er = (int)(signed char)f.packed, odd = l1 & 1 ? (f.packed >> 8) & 255 : 0;
-  run.add({mul_hi(wr, k), (f.e >> 1) + l1 * er - odd - __popc((unsigned)f.packed >> 16 & ((2u << l1) - 1u))},
+static __device__ inline void t1_entry_add(xf_run &run, u64 wr, u64 k, EntInfo f, int l1, int l2) {
+  const int er = (int)(signed char)f.packed, t = (f.packed >> 8) & 0xffff;
+  const xf K = row_packed(k);
+  run.add({mul_hi(wr, K.m),
+           (f.e >> 1) + l1 * er - l2 * t + K.e - __popc((unsigned)f.packed >> 24 & ((1u << l1) - 1u))},
           (uint32_t)f.e << 31);
 }
 
@@ -679,7 +659,7 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
           // the points inside the window (the entries outside it are zero)
           if (work && (inw >> (x - s0) & 1u)) {
             const u64 *e = eT + (x - s0) * G * TS;
-            t1_entry_add(run, e[oW], e[oK], *(const EntInfo *)(e + 2 * lq), q1);
+            t1_entry_add(run, e[oW], e[oK], *(const EntInfo *)(e + 2 * lq), q1, oK);
           }
         xs sum = combine(run.sum(), D.P);
         sum = from_lane(sum, (mine_rank * D.P) & 31);
@@ -1021,7 +1001,7 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, const LargeSmem 
               const double a = ((const double *)e)[oW], b = ((const double *)e)[oK];
               run.add(xf_mul(xf_from(a), xf_from(b)), ent_h(a) ^ ent_h(b));
             } else {
-              t1_entry_add(run, e[oW], e[oK], f, q1);
+              t1_entry_add(run, e[oW], e[oK], f, q1, oK);
             }
           }
         xs sum = combine(run.sum(), D.P);

@@ -235,6 +235,32 @@ ECPGB_NOUNROLL
   return c;
 }
 
+// The rows packed one word each for the type-1 tables: a mantissa of 58 bits (2^63
+// <= m < 2^64, 0 for a row that is 0) with the row's exponent in the low 6 bits, as
+// K_l / c = m 2^(e0 - l t - low bits).  2^t is z's size below 1 (z 2^t in 0.3 to 2.6):
+// then K_l 2^(l t) <= K_0, and no less than 2^-42 of it for l <= 8.  One exponent for
+// all rows cut l = 8 to 47 bits at z = 2 and to none below 0.01.
+struct RowBase {
+  xf c;
+  int e0, t;
+};
+ECPGB_HD RowBase fx_bessel_packed(const i64 *besX, const i64 *besXA, int HL1, int lmax, xf z100, u64 *K) {
+  RowBase b;
+  b.t = z100.e < -56 ? -56 - z100.e : 0;
+  int e0 = 0, lt = 0;
+  b.c = fx_bessel(besX, besXA, HL1, lmax, z100, [&](int l, u64 v, int scale) {
+    const int n = clz64(v | 1u), e = -scale - n;
+    if (l == 0) e0 = e;
+    const int d = e0 - lt - e;  // (above 63: a row's cut series near its root)
+    K[l] = d > 63 ? 0 : ((v << n) & ~63ull) | (u64)(d > 0 ? d : 0);
+    lt += b.t;
+  });
+  b.e0 = e0;
+  return b;
+}
+// Mantissa and exponent (over c and e0 - l t) of a packed row.
+ECPGB_HD xf row_packed(u64 k) { return {k & ~63ull, -(int)(k & 63u)}; }
+
 // The rows as doubles, each times mul (mul.m = 0: times 1) with the sign bit `sign`.
 ECPGB_HD void fx_bessel_rows(const i64 *besX, const i64 *besXA, int HL1, int lmax, xf z100, xf mul, uint32_t sign,
                              double *K) {
