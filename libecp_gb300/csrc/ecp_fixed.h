@@ -180,6 +180,9 @@ ECPGB_HD i64 ld_one(const i64 *p) {
 #endif
 }
 
+// Octaves of z tabulated below 1/200, down to 1e-60; what is smaller counts as 0.
+constexpr int kBesselOctaves = 192;
+
 // 100 z for z = f * r, f already times 100 (xf_times100): the argument of fx_bessel_rows.
 ECPGB_HD xf xf_times100(xf f) { return {mul_hi(f.m, 100ull << 57), f.e + 7}; }
 
@@ -189,14 +192,15 @@ ECPGB_HD xf xf_times100(xf f) { return {mul_hi(f.m, 100ull << 57), f.e + 7}; }
 // src/bessel.c:102-199: the 5-term Taylor polynomial about the nearest table
 // point (z < 16) and the large-argument polynomial are both one Horner pass
 // per row over 64-bit coefficients (besX, besXA), so lanes on either branch
-// run the same instructions.  The small-argument branch (z < 1e-7) agrees with
-// the first table point's polynomial to 1e-14 of K_0 and needs no code; z = 0
-// gives exactly (1, 0, ...).
+// run the same instructions.  The first table point's polynomial, z < 1/200, is
+// tabulated once per octave of z, each row at the octave's scale: K_l falls as z^l,
+// and at one scale l = 3 had 10 bits left at z = 1e-6.  (The reference's branch for
+// z < 1e-7 is that polynomial's first two terms.)  z = 0 gives exactly 1, 0, 0, ...
 template <class Row>
 ECPGB_HD xf fx_bessel(const i64 *besX, const i64 *besXA, int HL1, int lmax, xf z100, Row row) {
   z100 = xf_norm(z100);
   const int sh = -(z100.e + 52);  // 100 z in Q52 = z100.m >> sh; sh < 0 only above 1600
-  u64 W = sh < 0 ? ~0ull : shr64(z100.m, sh);
+  const u64 W = sh < 0 ? ~0ull : shr64(z100.m, sh);
   const bool asy = W >= 1600ull << 52;
   const i64 *q = besX;
   int rowStride = 8, scaleAt = 6;
@@ -212,10 +216,16 @@ ECPGB_HD xf fx_bessel(const i64 *besX, const i64 *besXA, int HL1, int lmax, xf z
     rowStride = 16;
     scaleAt = 15;
   } else {
-    W += 1ull << 51;
-    X = (W & ((1ull << 52) - 1)) << 11;
-    // (z = 0, a shell on the ECP centre: a block of its own, exactly 1, 0, 0, ...)
-    q += (size_t)(z100.m ? W >> 52 : 1601) * HL1 * 8;
+    int i = (int)((W + (1ull << 51)) >> 52);
+    if (i == 0) {
+      X = z100.m & ((1ull << 63) - 1);
+      i = -65 - z100.e;  // octaves below 1/2
+      i = 1601 + (z100.m && i < kBesselOctaves ? i : kBesselOctaves);
+    } else {
+      X = sh < 11 ? z100.m << (11 - sh) : z100.m >> (sh - 11);  // 100 z / 2 in Q64
+      X = (X + (1ull << 62)) & ((1ull << 63) - 1);
+    }
+    q += (size_t)i * HL1 * 8;
   }
   const fxmul x = fx_split(X);
 ECPGB_NOUNROLL
@@ -251,8 +261,8 @@ ECPGB_HD RowBase fx_bessel_packed(const i64 *besX, const i64 *besXA, int HL1, in
   b.c = fx_bessel(besX, besXA, HL1, lmax, z100, [&](int l, u64 v, int scale) {
     const int n = clz64(v | 1u), e = -scale - n;
     if (l == 0) e0 = e;
-    const int d = e0 - lt - e;  // (above 63: a row's cut series near its root)
-    K[l] = d > 63 ? 0 : ((v << n) & ~63ull) | (u64)(d > 0 ? d : 0);
+    const int d = e0 - lt - e;  // (above 63: 0, and a row's cut series near its root)
+    K[l] = d > 63 ? 63ull : ((v << n) & ~63ull) | (u64)(d > 0 ? d : 0);
     lt += b.t;
   });
   b.e0 = e0;
@@ -271,7 +281,7 @@ ECPGB_HD void fx_bessel_rows(const i64 *besX, const i64 *besXA, int HL1, int lma
 ECPGB_NOUNROLL
   for (int l = 0; l <= lmax; l++) {
     const xf v = one ? xf{k[l].m, k[l].e + c.e + 63} : xf_mul(k[l], c);
-    K[l] = z100.m == 0 && l == 0 ? xf_to_double(c.m, c.e, sign) : xf_to_double(v.m, v.e, sign);
+    K[l] = xf_to_double(v.m, v.e, sign);
   }
 }
 

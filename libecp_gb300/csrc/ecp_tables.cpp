@@ -3,6 +3,7 @@
 // Each builder states the reference code whose table it reproduces; the
 // arithmetic is kept in the same operation order so that the device sees the
 // same table values the reference computes.
+#include "ecp_fixed.h"
 #include "ecp_tables.h"
 
 #include <algorithm>
@@ -461,7 +462,7 @@ static void fixed_row(const long double *c, int deg, long long *out, long long &
     s = 0.5L * s + std::fabs(c[k]);
     top = std::max(top, s);
   }
-  scale = 0;
+  scale = 4096;  // (a zero's exponent is below every other row's: sums align to the largest)
   if (!(top > 1e-300L)) {
     for (int k = 0; k <= deg; k++) out[k] = 0;
     return;
@@ -473,15 +474,27 @@ static void fixed_row(const long double *c, int deg, long long *out, long long &
 void bessel_fixed(HostTables &t) {
   const int N = t.besselN + 1, HL = t.besselHL, AS = HL + 1 < 6 ? 6 : HL + 1;
   const long double h = 16.0L / t.besselN;
-  t.besselX.assign((size_t)(N + 1) * (HL + 1) * 8, 0);
-  // the rows of z = 0 (a shell on the ECP centre): 1, 0, 0, ...
-  t.besselX[(size_t)N * (HL + 1) * 8] = (1ll << 62) - 1;
-  for (int l = 0; l <= HL; l++) t.besselX[((size_t)N * (HL + 1) + l) * 8 + 6] = 62;
+  t.besselX.assign((size_t)(N + kBesselOctaves + 1) * (HL + 1) * 8, 0);
+  // z < h/2 by octaves, z = 2^-k (h/2) (1/2 + X): sum_j q_j z^j in powers of X; then
+  // z = 0
+  for (int k = 0; k <= kBesselOctaves; k++)
+    for (int l = 0; l <= HL; l++) {
+      const double *q = &t.besselH[(size_t)l * 6];
+      const long double f = k < kBesselOctaves ? std::ldexp(0.5L * h, -k) : 0.0L;
+      long double c[6] = {0, 0, 0, 0, 0, 0}, d[6];
+      for (int j = 5; j >= 0; j--) {  // c = c * (f / 2 + f X) + q_j
+        for (int i = 5; i >= 0; i--) d[i] = f * (0.5L * c[i] + (i ? c[i - 1] : 0.0L));
+        for (int i = 0; i < 6; i++) c[i] = d[i];
+        c[0] += q[j];
+      }
+      long long *out = &t.besselX[((size_t)(N + k) * (HL + 1) + l) * 8];
+      fixed_row(c, 5, out, out[6]);
+    }
   // sum_j q_j (h (2 X - 1/2))^j in powers of X: m[j][k] of X^k in the j-th power
   long double m[6][6] = {{1.0L}};
   for (int j = 1; j < 6; j++)
     for (int k = 0; k <= j; k++) m[j][k] = (k ? 2 * h * m[j - 1][k - 1] : 0.0L) - 0.5L * h * m[j - 1][k];
-  for (int i = 0; i < N; i++)
+  for (int i = 1; i < N; i++)
     for (int l = 0; l <= HL; l++) {
       const double *q = &t.besselH[((size_t)i * (HL + 1) + l) * 6];
       long double c[6];

@@ -82,8 +82,9 @@ struct HostTables {
   std::vector<double> besselA;
   // The polynomials of besselH and besselA as 64-bit integers for Horner passes
   // in fixed point (ecp_fixed.h), both in a variable X in [0, 1/2]:
-  // besselX [i][l][8] (and i = besselN + 1: z = 0 exactly): X = x / 2, z = z_i + (x - 1/2) h, h = 16/besselN, degree
-  // 5, coefficients in [0..5]; besselXA [l][16]: X = 16 a, coefficients with
+  // besselX [i][l][8]: X = x / 2, z = z_i + (x - 1/2) h, h = 16/besselN, degree
+  // 5, coefficients in [0..5]; z < h/2 (i = 0) by octaves in blocks besselN + 1 + k,
+  // z = 2^-k (h/2) (1/2 + X), and z = 0 last; besselXA [l][16]: X = 16 a, coefficients with
   // their signs in [0..l].  A row's value is v * 2^-scale, the scale in [6]
   // ([15] of besselXA).
   std::vector<long long> besselX, besselXA;
