@@ -420,7 +420,7 @@ static __device__ void rsh_column(const DevJob &J, int lmax, int m, double x, do
 // e + l1 er - (leading bits won back up to row l1) - l2 t - (K's low bits).
 struct EntInfo {
   int e;       // 2 e + sign
-  int packed;  // er (8 bits, signed), t (16 bits), a bit per row l = 1..8 whose product was shifted
+  int packed;  // er (8 bits, signed), t (8 bits), from bit 16 a bit per row l = 1.. whose product was shifted
 };
 constexpr EntInfo kNoEntry = {-2000000, 0};
 // A point past the break: the entry holds doubles.
@@ -435,19 +435,22 @@ static __device__ inline EntInfo t1_entry_rows(u64 *WR, xf v, const RowBase &b, 
     m = mul_hi(m, R.m);
     if ((i64)m >= 0) {
       m += m;
-      won |= 1u << (23 + l);
+      won |= 1u << (15 + l);
     }
     WR[l] = m;
   }
   return {(v.e + b.e0 + 64) * 2 + (int)(sign >> 31), ((R.e + 64) & 255) | b.t << 8 | (int)won};
 }
-// The product of row l1 and K_l2 of an entry into a run.
-static __device__ inline void t1_entry_add(xf_run &run, u64 wr, u64 k, EntInfo f, int l1, int l2) {
-  const int er = (int)(signed char)f.packed, t = (f.packed >> 8) & 0xffff;
+// What a quadrature (l1, l2) reads of an entry's exponents: their factors, a byte
+// each, and the mask of the products up to row l1.
+struct EntRow {
+  int l, won;
+};
+static __device__ inline EntRow t1_entry_row(int l1, int l2) { return {l1 | (-l2 & 255) << 8, (1 << (16 + l1)) - (1 << 16)}; }
+// The product of row l1 and K_l2 of an entry into a run (l1 er - l2 t in one instruction).
+static __device__ inline void t1_entry_add(xf_run &run, u64 wr, u64 k, EntInfo f, EntRow q) {
   const xf K = row_packed(k);
-  run.add({mul_hi(wr, K.m),
-           (f.e >> 1) + l1 * er - l2 * t + K.e - __popc((unsigned)f.packed >> 24 & ((1u << l1) - 1u))},
-          (uint32_t)f.e << 31);
+  run.add({mul_hi(wr, K.m), __dp4a(f.packed, q.l, f.e >> 1) + K.e - __popc(f.packed & q.won)}, (uint32_t)f.e << 31);
 }
 
 // One live entry of the type-1 large-grid tables: K_l(s r) and w C2 U_L(r) e^ex
@@ -648,6 +651,7 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
       const int q1 = (qd >> 8) & 255;
       const u64 *eT = (const u64 *)tab + (qd & 255) * TS;
       const int oW = lq + q1, oK = qd >> 16;
+      const EntRow qr = t1_entry_row(q1, oK);
 #pragma unroll 1
       for (int t = s0; t < s1;) {
         const int te = lvEnd < s1 ? lvEnd : s1;
@@ -659,7 +663,7 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
           // the points inside the window (the entries outside it are zero)
           if (work && (inw >> (x - s0) & 1u)) {
             const u64 *e = eT + (x - s0) * G * TS;
-            t1_entry_add(run, e[oW], e[oK], *(const EntInfo *)(e + 2 * lq), q1, oK);
+            t1_entry_add(run, e[oW], e[oK], *(const EntInfo *)(e + 2 * lq), qr);
           }
         xs sum = combine(run.sum(), D.P);
         sum = from_lane(sum, (mine_rank * D.P) & 31);
@@ -988,6 +992,7 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, const LargeSmem 
       const bool work = D.rank < __popc(act);
       const int qd = work ? quad[D.rank] : 0;
       const int q1 = qd & 0xffff, oW = lq + q1, oK = qd >> 16;
+      const EntRow qr = t1_entry_row(q1, oK);
 #pragma unroll 1
       for (int t = s0; t < s1;) {
         const int te = lvEnd < s1 ? lvEnd : s1;
@@ -1001,7 +1006,7 @@ static __device__ void t1_large(const DevJob &J, const Unit &U, const LargeSmem 
               const double a = ((const double *)e)[oW], b = ((const double *)e)[oK];
               run.add(xf_mul(xf_from(a), xf_from(b)), ent_h(a) ^ ent_h(b));
             } else {
-              t1_entry_add(run, e[oW], e[oK], f, q1, oK);
+              t1_entry_add(run, e[oW], e[oK], f, qr);
             }
           }
         xs sum = combine(run.sum(), D.P);

@@ -256,7 +256,7 @@ struct RowBase {
 };
 ECPGB_HD RowBase fx_bessel_packed(const i64 *besX, const i64 *besXA, int HL1, int lmax, xf z100, u64 *K) {
   RowBase b;
-  b.t = z100.e < -56 ? -56 - z100.e : 0;
+  b.t = z100.e < -56 ? (z100.e > -183 ? -56 - z100.e : 127) : 0;  // (a byte of the entry)
   int e0 = 0, lt = 0;
   b.c = fx_bessel(besX, besXA, HL1, lmax, z100, [&](int l, u64 v, int scale) {
     const int n = clz64(v | 1u), e = -scale - n;
