@@ -96,12 +96,13 @@ ECPGB_HD xf xf_norm(xf a) {
   return {a.m << lz, a.e - lz};
 }
 
-// m * 2^e rounded to the nearest double, with a sign; 0 below the normal range.
+// m * 2^e rounded to the nearest double, with a sign; 0 below the normal range,
+// infinity above it.
 ECPGB_HD double xf_to_double(u64 m, int e, uint32_t sign) {
   const int lz = clz64(m);
   const int be = e + 63 + 1023 - lz;  // biased exponent
   m <<= (lz & 63);
-  const u64 b = ((u64)(uint32_t)be << 52) + ((m << 1) >> 12) + ((m >> 10) & 1u);
+  const u64 b = be < 0x7ff ? ((u64)(uint32_t)be << 52) + ((m << 1) >> 12) + ((m >> 10) & 1u) : 0x7ffull << 52;
   return lz < 64 && be > 0 ? bits_d((i64)(b | (u64)sign << 32)) : 0.0;
 }
 

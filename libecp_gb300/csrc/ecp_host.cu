@@ -548,10 +548,33 @@ static long long primitive_pairs(const Parsed &P) {
   return n;
 }
 
+// log2 of a bound of every product of the integrands: two contraction
+// coefficients (times zeta^order), a potential, powers of r.  Points reach from
+// 9e-12 (small grid) or 9e-14 of an interval of 9/sqrt(za + zb) (large grid; with
+// more than 1023 points its first abscissa is -1, r = 0) to a distance plus that interval.
+static double product_bits(const Parsed &P) {
+  double zMin = INFINITY, zMax = 0.0, c = -INFINITY, u = -INFINITY, far = 0.0;
+  for (double z : P.primA) {
+    zMin = std::min(zMin, z);
+    zMax = std::max(zMax, z);
+  }
+  for (double d : P.primD) c = std::max(c, std::log2(std::fabs(d)));
+  for (double x : P.geom) far = std::max(far, std::fabs(x));
+  const double top = std::log2(std::max(64.0, 4.0 * far + 9.0 / std::sqrt(2.0 * zMin)));
+  const double low = P.largeGridOrder < 2047 ? std::max(37.0, 44.0 - std::log2(4.5 / std::sqrt(2.0 * zMax))) : INFINITY;
+  for (size_t t = 0; t < P.termN.size(); t++) {
+    const double n = P.termN[t];
+    u = std::max(u, std::log2(std::fabs(P.termD[t])) + (n > 0.0 ? n * top : n < 0.0 ? -n * low : 0.0));
+  }
+  // (r^l, l <= 8, the interval's length and the map's weight; sums)
+  return 2.0 * (c + P.deriv * std::max(0.0, std::log2(zMax))) + u + std::log2(1.0 + P.termN.size()) + 11.0 * top + 64.0;
+}
+
 // Whether a batched job runs the plain path's stages.  The batched path's
 // integer arithmetic takes finite inputs of the magnitudes that basis sets and
 // potentials have, decaying primitives and thresholds below 1; outside that
-// (NaN, infinities, ECP exponents below 0, ...) FP64 decides what comes out.
+// (NaN, infinities, ECP exponents below 0, products that FP64 cannot hold, ...) FP64
+// decides what comes out.
 static bool plain_stages(const Parsed &P, int mode) {
   if (mode == ECPGB_FP64) return true;
   auto within = [](const std::vector<double> &v, double lo, double hi) {
@@ -561,7 +584,7 @@ static bool plain_stages(const Parsed &P, int mode) {
   };
   return !(within(P.primA, 1e-30, 1e30) && within(P.primD, -1e60, 1e60) && within(P.termA, 0.0, 1e30) &&
            within(P.termD, -1e100, 1e100) && within(P.termN, -16.0, 16.0) && P.acc >= 1e-300 && P.acc <= 1.0 &&
-           P.tol >= 1e-300 && P.tol <= 1e100);
+           P.tol >= 1e-300 && P.tol <= 1e100 && product_bits(P) <= 1000.0);
 }
 
 // The queue orders of a job -- shell pairs in the reference's order,
