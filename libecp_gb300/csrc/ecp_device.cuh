@@ -227,6 +227,7 @@ static __device__ inline bool ecp_term_lost(double pot, double D, double x, doub
   if (nb == 0x3ff0000000000000ll) u += (__double2hiint(r) >> 20) - 1022;
   else if (nb == 0x4000000000000000ll) u += (__double2hiint(r2) >> 20) - 1022;
   else if (nb << 1 != 0) return false;
+  if (u > 1024) return false;  // D r^n may be infinite, and the term NaN
   const int e = (int)(hx >> 20) - 1023;
   const unsigned y = ((hx & 0xfffffu) | 0x100000u) * 1477u;  // log2(e) from below, Q30 2^-e
   const int q = e < 0 ? 0 : e > 10 ? 4096 : (int)(y >> (30 - e));
