@@ -48,11 +48,13 @@ typedef struct {
 } ecpgb_system;
 
 enum {
-  ECPGB_FP64 = 0,   /* plain FP64 kernels, one unit per CTA (the drop-in path) */
-  ECPGB_FAST = 1,   /* batched FP64 path: a warp per primitive pair, quadrature
-                       points tabulated level by level until convergence,
-                       Horner-form Bessel rows, table-driven exp; same
-                       schedules and decisions, rounding-level differences */
+  ECPGB_FP64 = 0,   /* plain FP64 path (the drop-in path): the reference's
+                       operations in their order, unit stages over work lists */
+  ECPGB_FAST = 1,   /* batched path: the same stages and schedules, tables and
+                       sums in 64-bit integer arithmetic where the inputs'
+                       magnitudes allow (else the plain path's stages); the
+                       differences are of rounding, also in the convergence
+                       tests that sit at FP64's rounding level */
   ECPGB_MIXED = 2,  /* the batched path with the type-1 large-grid fallback
                        in double-single FP32 pairs (about 48 bits) where its
                        sums can still take the FP64 path's convergence

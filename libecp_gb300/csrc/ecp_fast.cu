@@ -91,8 +91,8 @@ static __device__ __noinline__ double bessel_row(const DevJob &J, int l, double 
 }
 
 // U_l(r) of centre c (src/ecp.c:42-60): its terms of channel l, summed with
-// 60-bit mantissas; normalised, with its sign.  A term below 2^-70 of the
-// largest one before it is left out, and one whose exponential underflows.
+// 60-bit mantissas; normalised, with its sign.  A term whose exponential is below
+// e^-700 is left out.
 static __device__ __noinline__ xf channel(const DevJob &J, int c, int l, double r, uint32_t &sign) {
   const xf R = xf_from(r), R2 = norm1(xf_mul(R, R));
   xs acc;
@@ -103,8 +103,6 @@ static __device__ __noinline__ xf channel(const DevJob &J, int c, int l, double 
     const xf a = xf_mul({T.am, T.ae}, R2);
     const u64 E = shr64(a.m, -(a.e + 53));  // a r^2 in Q53
     if (a.e + 53 > 0 || E > (u64)(700ll << 53)) continue;
-    // 2^b above the term, b = log2 |d| + log2 r^n - a r^2 log2 e rounded up
-    // (n <= 2; r^n otherwise unknown: never left out)
     const xf Rn = T.n == 1 ? R : R2;
     xf v = xf_mul(fx_exp(-(i64)E), {T.dm, T.de});
     if (T.n) v = xf_mul(v, T.n < 3 ? Rn : xf_from(rpow_rare(r, J.termN[t])));

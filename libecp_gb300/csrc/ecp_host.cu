@@ -534,14 +534,20 @@ static PairPlan plan_of_pair(const Parsed &P, int p, bool single) {
 
 // Jobs of at most kFewPairs primitive pairs over all units: every warp of the
 // GPU gets at most a few work-list entries and the longest one sets a stage's
-// time, so an entry is one primitive pair (unit stages of 702 pairs 0.33 instead of
-// 0.58 ms, of 5148 pairs 0.42 instead of 0.66; of 38,300 pairs 1.55 instead of 1.40).
-constexpr long long kFewPairs = 9728;  // 64 a streaming multiprocessor
+// time, so an entry is one primitive pair.  Unit stages with an entry a pair and with
+// entries of several (ms): 702 pairs 0.33 and 0.58, 5,308 0.53 and 0.77, 9,236 0.64 and
+// 0.88; beyond the line 10,490 0.69 and 0.92, 14,421 0.76 and 0.95, 24,374 1.13 and
+// 1.33, 38,300 1.55 and 1.40; the plain path's small grid, 9,236 pairs: 1.84 and 1.78.
+// The line is below the crossing: a part a pair takes a partial sum per pair and
+// quadrature of scratch.  (The partial sums' number, and with it a unit's last bits,
+// follow the job's size.)
+constexpr long long kFewPairs = 64 * 152;  // 64 a streaming multiprocessor
 // Up to kTwoWarpPairs the batched large grid gives an entry to two warps, which
-// halves its latency (38,300 pairs: 1.40 instead of 1.60 ms, a Hessian job of 51,480:
-// 1.83 instead of 2.23); with more the SMs are full and the two warps' different
-// code costs instruction fetches (150,792 pairs: 3.67 instead of 3.34 ms).
-constexpr long long kTwoWarpPairs = 58368;  // 384 a streaming multiprocessor
+// halves its latency; with more the SMs are full and the two warps' different code
+// costs instruction fetches.  Unit stages with two warps and with one (ms): 19,170
+// pairs 1.17 and 1.35, 50,110 1.73 and 1.89; beyond the line 60,920 1.86 and 1.98,
+// 94,458 2.32 and 2.43, 118,395 2.78 and 2.67, 163,264 3.61 and 3.16.
+constexpr long long kTwoWarpPairs = 384 * 152;  // 384 a streaming multiprocessor
 static long long primitive_pairs(const Parsed &P) {
   long long n = 0;
   for (int p = 0; p < P.nPairs; p++) n += (long long)P.nCentres * P.shK[P.pairA[p]] * P.shK[P.pairB[p]];
