@@ -100,9 +100,13 @@ ECPGB_HD xf xf_norm(xf a) {
 // infinity above it.
 ECPGB_HD double xf_to_double(u64 m, int e, uint32_t sign) {
   const int lz = clz64(m);
-  const int be = e + 63 + 1023 - lz;  // biased exponent
+  int be = e + 63 + 1023 - lz;  // biased exponent
   m <<= (lz & 63);
-  const u64 b = be < 0x7ff ? ((u64)(uint32_t)be << 52) + ((m << 1) >> 12) + ((m >> 10) & 1u) : 0x7ffull << 52;
+  if (be >= 0x7ff) {
+    be = 0x7ff;
+    m = 0;
+  }
+  const u64 b = ((u64)(uint32_t)be << 52) + ((m << 1) >> 12) + ((m >> 10) & 1u);
   return lz < 64 && be > 0 ? bits_d((i64)(b | (u64)sign << 32)) : 0.0;
 }
 
@@ -197,7 +201,10 @@ ECPGB_HD xf xf_times100(xf f) { return {mul_hi(f.m, 100ull << 57), f.e + 7}; }
 // tabulated once per octave of z, each row at the octave's scale: K_l falls as z^l,
 // and at one scale l = 3 had 10 bits left at z = 1e-6.  (The reference's branch for
 // z < 1e-7 is that polynomial's first two terms.)  z = 0 gives exactly 1, 0, 0, ...
-template <class Row>
+// kLate: a row is handed out while the next one's coefficients are on their way
+// (the small grid, whose warps wait for them; in the large grid the second copy of
+// `row` costs more in instruction fetch than it hides).
+template <bool kLate = false, class Row>
 ECPGB_HD xf fx_bessel(const i64 *besX, const i64 *besXA, int HL1, int lmax, xf z100, Row row) {
   z100 = xf_norm(z100);
   const int sh = -(z100.e + 52);  // 100 z in Q52 = z100.m >> sh; sh < 0 only above 1600
@@ -229,20 +236,27 @@ ECPGB_HD xf fx_bessel(const i64 *besX, const i64 *besXA, int HL1, int lmax, xf z
     q += (size_t)i * HL1 * 8;
   }
   const fxmul x = fx_split(X);
+  u64 vp = 0;
+  int sp = 0;
 ECPGB_NOUNROLL
   for (int l = 0; l <= lmax; l++, q += rowStride) {
+    const fxpair c45 = ld_pair(q + 4), c23 = ld_pair(q + 2), c01 = ld_pair(q);
+    const int sc = (int)ld_one(q + scaleAt);
+    if (kLate && l) row(l - 1, vp, sp);
     i64 v = 0;
 ECPGB_NOUNROLL
     for (int k = asy ? l : 5; k > 5; k--) v = ld_one(q + k) + mul_hi_s(v, x);
-    const fxpair c45 = ld_pair(q + 4), c23 = ld_pair(q + 2), c01 = ld_pair(q);
     v = c45.y + mul_hi_s(v, x);
     v = c45.x + mul_hi_s(v, x);
     v = c23.y + mul_hi_s(v, x);
     v = c23.x + mul_hi_s(v, x);
     v = c01.y + mul_hi_s(v, x);
     v = c01.x + mul_hi_s(v, x);
-    row(l, (u64)(v > 0 ? v : 0), (int)ld_one(q + scaleAt));
+    vp = (u64)(v > 0 ? v : 0);
+    sp = sc;
+    if (!kLate) row(l, vp, sp);
   }
+  if (kLate) row(lmax, vp, sp);
   return c;
 }
 
@@ -255,15 +269,16 @@ struct RowBase {
   xf c;
   int e0, t;
 };
+template <bool kLate = false>
 ECPGB_HD RowBase fx_bessel_packed(const i64 *besX, const i64 *besXA, int HL1, int lmax, xf z100, u64 *K) {
   RowBase b;
   b.t = z100.e < -56 ? (z100.e > -183 ? -56 - z100.e : 127) : 0;  // (a byte of the entry)
   int e0 = 0, lt = 0;
-  b.c = fx_bessel(besX, besXA, HL1, lmax, z100, [&](int l, u64 v, int scale) {
+  b.c = fx_bessel<kLate>(besX, besXA, HL1, lmax, z100, [&](int l, u64 v, int scale) {
     const int n = clz64(v | 1u), e = -scale - n;
     if (l == 0) e0 = e;
     const int d = e0 - lt - e;  // (above 63: 0, and a row's cut series near its root)
-    K[l] = d > 63 ? 63ull : ((v << n) & ~63ull) | (u64)(d > 0 ? d : 0);
+    K[l] = (unsigned)d > 63u ? 63ull : ((v << n) & ~63ull) | (u64)(unsigned)d;
     lt += b.t;
   });
   b.e0 = e0;
