@@ -59,6 +59,7 @@ struct DevJob {
   int largeOrder;
   int t2Rows;                  // most table rows a batch of type-2 quadratures reads
   double tol, acc, lnAcc1, lnAcc2;
+  unsigned long long lnAcc1Q53;  // -lnAcc1 2^53 (batched path)
   // inputs
   const double *geom;
   const int *shL, *shK, *shP, *shAtom, *shAO;

@@ -480,7 +480,7 @@ static __device__ void t1_small(const DevJob &J, const Unit &U, const SmallSmem 
   const int lane = threadIdx.x & 31, lab = U.lab, lq = lab + 1, O = kSmallOrder, ws = U.ws, we = U.we;
   // odd entry strides: lanes touching neighbouring entries hit distinct banks
   const int TS = 1 + 2 * lq, nq = t1_items(lab);
-  const u64 thr = (u64)(i64)(-J.lnAcc1 * 0x1p53);
+  const u64 thr = J.lnAcc1Q53;
   double *rec = sm + L.rec, *tab = sm + L.tab;  // the pairs' records
   const unsigned char *perm = (const unsigned char *)(U.scr + U.L.perm);
   const double *uL = J.uL + (size_t)U.c * O;

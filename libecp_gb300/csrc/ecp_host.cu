@@ -764,6 +764,7 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   J.t2Rows = T->t2Rows;
   J.tol = P.tol; J.acc = P.acc;
   J.lnAcc1 = std::log(P.acc) - 2;
+  J.lnAcc1Q53 = J.plain ? 0 : (unsigned long long)(-J.lnAcc1 * 0x1p53);
   J.lnAcc2 = std::log(1.0E-14) - 2;
   // --- the plan and the device buffers: where they cannot be had, with less scratch
   std::vector<int> orders, chunkUnits, ctr;
