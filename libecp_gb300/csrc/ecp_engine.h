@@ -130,6 +130,7 @@ struct DevJob {
   int capT1;                     // entries listT1 has room for
   struct T1Fail *listFail;
   bool plain;                    // runs the plain path's stages
+  bool inRange;                  // no product of the integrands leaves FP64's range: 0 times one is 0
   bool few, single;              // few primitive pairs in all; one primitive pair a type-2 part
   bool twoWarps;                 // two warps a large-grid entry (batched path)
   int take;                      // work-list entries a warp takes before it exits

@@ -97,7 +97,9 @@ static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem 
       double *ent = tab + ((t - s0) * G + gg) * TS, *WR = ent + lq;
       const PairRec &P = *(const PairRec *)(rec + gg * kPairWords);
       const double r = J.xSmall[n], s = P.s, C1 = P.C1, ex = (P.z * r + s) * r, u = uL[n];
-      if (ex >= J.lnAcc1) {
+      // below the screen the exponential is 0, and so is the product where it is finite
+      const bool seen = ex >= J.lnAcc1;
+      if (seen || !J.inRange) {
         bessel_rows(J, lab, s * r, ent);
         double R = 1.0;
 #pragma unroll 1
@@ -105,7 +107,7 @@ static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem 
           WR[l] = C1 * R * u;
           R = r * R;
         }
-        ent[2 * lq] = exp(ex);
+        ent[2 * lq] = seen ? exp(ex) : 0.0;
       } else {
         ent[2 * lq] = 0.0;  // marks a zero point
       }
@@ -128,7 +130,7 @@ static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem 
         const int n = __ldg(J.s93 + t0 + D.part);
         if (n >= ws && n < we) {
           const double *e = tab + ((t0 + D.part - s0) * G + (qd & 255)) * TS;
-          if (e[2 * lq] != 0.0) v = J.wSmall[n] * (e[oW] * e[oK] * e[2 * lq]);
+          if (e[2 * lq] != 0.0 || !J.inRange) v = J.wSmall[n] * (e[oW] * e[oK] * e[2 * lq]);
         }
       }
 #pragma unroll 1

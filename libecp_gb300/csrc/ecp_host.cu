@@ -746,7 +746,8 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
     return -1;
   }
   std::memset(&J, 0, sizeof J);
-  J.plain = plain_stages(P, mode);
+  J.inRange = !plain_stages(P, ECPGB_FAST);
+  J.plain = mode == ECPGB_FP64 || !J.inRange;
   const long long np = primitive_pairs(P);
   J.few = np <= kFewPairs;
   J.twoWarps = np <= kTwoWarpPairs;

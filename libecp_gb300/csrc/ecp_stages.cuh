@@ -37,8 +37,8 @@ static __device__ inline double t1_prefactor(double za, double ca, double zb, do
 //  * band: C1 below 2^-900 but not 0, or exp(e) may overflow: partial
 //    products underflow (or overflow) where a regrouped product would not, so
 //    the integrand is evaluated in the reference's order;
-//  * zero: C1 = 0, so every integrand value is 0 * (finite) = 0, or NaN where
-//    exp(e) overflows -- no table is needed.
+//  * zero: C1 = 0 in a job whose products stay in FP64's range, so every integrand
+//    value is 0 * (finite) = 0, or NaN where exp(e) overflows -- no table is needed.
 constexpr int kPairNormal = 0, kPairBand = 1, kPairZero = 2;
 constexpr double kLnDblMax = 0x1.62e42fefa39efp+9;  // exp overflows above it
 
@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_unit_plan(DevJob J) {
       double P[3];
       for (int i = 0; i < 3; i++) P[i] = 2.0 * (za * U.gA[i] + zb * U.gB[i]);
       const double s2 = P[0] * P[0] + P[1] * P[1] + P[2] * P[2];
-      kind = C1 == 0.0 ? kPairZero
+      kind = C1 == 0.0 && J.inRange ? kPairZero
                        : (kExact || fabs(C1) < 0x1p-900 || s2 > 2800.0 * (za + zb)) ? kPairBand : kPairNormal;
       PairRec rec;
       rec.s = sqrt(s2);
