@@ -39,6 +39,14 @@ static __device__ inline bool ps93_exact(int k, double tol, int cnt, double I, d
   return true;
 }
 
+// Whether the walk adds slot t, grid point n (src/gc_integrators.c:157-217): the head
+// always, then the lower halves from the window's start and the upper ones to its end.
+// Outside the window the reference's tables are 0, and so is the integrand unless
+// another factor is infinite or NaN.
+static __device__ inline bool ps93_adds(int t, int n, int ws, int we) {
+  return t < 3 || ((t & 1) ? n >= ws : n <= we);
+}
+
 // A group of G primitive pairs of one kind (perm[p0 ..]) on the small grid
 // (src/type1.c:63-148), by one warp; lane = (pair, quadrature).
 template <bool kZero>
@@ -131,12 +139,15 @@ static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem 
         if (n >= ws && n < we) {
           const double *e = tab + ((t0 + D.part - s0) * G + (qd & 255)) * TS;
           if (e[2 * lq] != 0.0 || !J.inRange) v = J.wSmall[n] * (e[oW] * e[oK] * e[2 * lq]);
+        } else if (!J.inRange) {
+          v = J.wSmall[n] * (((const PairRec *)(rec + (qd & 255) * kPairWords))->C1 * 0.0);
         }
       }
 #pragma unroll 1
       for (int j = 0; j < D.P && t0 + j < s1; j++) {
         const int t = t0 + j, n = c93_slot[t];
-        if (n >= ws && n < we) T += __shfl_sync(0xffffffffu, v, (src + j) & 31);
+        if ((n >= ws && n < we) || (!J.inRange && ps93_adds(t, n, ws, we)))
+          T += __shfl_sync(0xffffffffu, v, (src + j) & 31);
         cnt += (t & 1) ? n >= ws : n <= we;
         if (t > 2 && !(t & 1)) {  // the reference's order: pair by pair
           I += T;
@@ -186,8 +197,8 @@ static __device__ void x2_small(const DevJob &J, const Unit &U, int q0) {
 #pragma unroll 1
   for (int t = 0;; t++) {
     const int n = c93_slot[t];
-    // (F is zero outside both windows)
-    if (n >= U.ws && n < U.we)
+    // (F is zero outside the windows)
+    if ((n >= U.ws && n < U.we) || (!J.inRange && ps93_adds(t, n, U.ws, U.we)))
       T += J.wSmall[n] * (__ldg(Fa + n * nF) * __ldg(Fb + n * nF) * __ldg(Ut + (size_t)n * LE * nk));
     cnt += (t & 1) ? n >= U.ws : n <= U.we;
     if (t > 2 && !(t & 1)) {
