@@ -27,13 +27,15 @@ value   : device-resident job (inputs in HBM before the timed region); per step
 e2e     : ecpgb_getIntegrals (the getIntegrals call with the path chosen) with
           host buffers: one packed H2D copy of the inputs and a D2H copy of the
           matrix per step.
-roofline: the unit stages against the FP64 FMA pipe measured live (DRAM traffic
-          is some ten kilobytes per unit; the batched path keeps most of its
-          arithmetic on the integer pipes): achieved = FP64 operations the
-          stages executed per emitted unit (ncu counts on the cluster's first 8
-          centres, profiles/roofline_inputs.txt; cluster workload only) x emitted
-          units / the stages' CUDA-event time; alg_* = the reference's algorithmic FLOPs counted by the oracle
-          on its control flow over the CPU-baseline sample.
+roofline: the unit stages against what bounds them (DRAM traffic is some ten
+          kilobytes per unit): the plain path against the FP64 FMA pipe, the
+          batched paths, whose arithmetic is on the integer pipes, against the
+          issue rate; both rates measured live (a warp instruction is 32 lanes'
+          FP32 FMA).  achieved = FP64 operations or warp instructions the stages
+          executed per emitted unit (ncu counts on the cluster's first 8 centres,
+          profiles/roofline_inputs.txt; cluster workload only) x emitted units /
+          the stages' CUDA-event time; alg_* = the reference's algorithmic FLOPs
+          counted by the oracle on its control flow over the CPU-baseline sample.
 cpu_baseline: the oracle restatement (or the reference build where one exists
           on the machine) on a bounded sample of the workload, on all host cores
           the process may use and on one core.
@@ -372,10 +374,10 @@ def ours(args, rank, world):
         key = {eg.ECPGB_FP64: "stages_plain", eg.ECPGB_MIXED: "stages_mixed"}.get(mode, "stages_batched")
         kernel = ("k_unit_plan + k_exact_small + k_exact_large + k_exact_link" if mode == eg.ECPGB_FP64
                   else "k_unit_plan + k_unit_small + k_unit_large + k_unit_link")
-        # executed work: FP64 operations the unit stages executed per emitted
-        # unit (ncu: 2 DFMA + DMUL + DADD thread instructions of one run on
-        # the cluster's first 8 centres, divided by its emitted units), FP64
-        # pipe utilisation and DRAM bytes, from profiles/roofline_inputs.txt
+        # executed work: FP64 operations and warp instructions the unit stages
+        # executed per emitted unit (ncu: 2 DFMA + DMUL + DADD thread instructions
+        # of one run on the cluster's first 8 centres, divided by its emitted
+        # units), FP64 pipe utilisation and DRAM bytes, from profiles/roofline_inputs.txt
         # (measured on the cluster: other workloads have no executed-work figure)
         entry = {}
         prof = os.path.join(ROOT, "profiles", "roofline_inputs.txt")
@@ -383,7 +385,13 @@ def ours(args, rank, world):
             with open(prof) as f:
                 entry = json.load(f).get(key, {})
         f_exec = entry.get("fp64_flops_per_emitted_unit")
-        achieved = f_exec * emitted / (t_unit / 1e3) / 1e12 if f_exec else None
+        i_exec = entry.get("warp_insts_per_emitted_unit")
+        fp64_achieved = f_exec * emitted / (t_unit / 1e3) / 1e12 if f_exec else None
+        issue_achieved = i_exec * emitted / (t_unit / 1e3) / 1e9 if i_exec else None
+        issue_peak = peaks["fp32_fma_tflops"] * 1e3 / 64
+        bound, achieved, top, top_unit, source = (
+            ("fp64", fp64_achieved, peak, "TFLOP/s", "FP64 FMA pipe") if mode == eg.ECPGB_FP64 else
+            ("issue", issue_achieved, issue_peak, "G warp instructions/s", "FP32 FMA rate / 64 FLOP a warp instruction,"))
         traffic = entry["dram_bytes_per_emitted_unit"] * emitted if entry.get("dram_bytes_per_emitted_unit") else None
         pipe = entry.get("fp64_pipe_active")
         line = {
@@ -402,20 +410,24 @@ def ours(args, rank, world):
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                     "d2h_bytes_per_step": int(d2h),
                     "api": "ecpgb_getIntegrals (the getIntegrals call, host buffers, path = mode)"},
-            "roofline": {"bound": "fp64", "kernel": kernel,
-                         "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                         "frac": achieved / peak if achieved else None,
+            "roofline": {"bound": bound, "kernel": kernel,
+                         "achieved": achieved, "peak": top, "unit": top_unit,
+                         "frac": achieved / top if achieved else None,
                          "traffic": traffic,
-                         "peak_source": "FP64 FMA pipe measured live by ecpgb_measure_peaks (of measured)",
+                         "peak_source": f"{source} measured live by ecpgb_measure_peaks (of measured)",
+                         "executed_warp_insts_per_unit": i_exec,
                          "executed_fp64_flops_per_unit": f_exec,
+                         "fp64_achieved_tflops": fp64_achieved, "fp64_peak_tflops": peak,
+                         "fp64_frac": fp64_achieved / peak if fp64_achieved else None,
                          "fp64_pipe_active_ncu": pipe,
                          "unit_kernel_ms": t_unit,
                          "alg_flops_per_unit": f_unit, "alg_achieved": alg_achieved,
                          "alg_frac": alg_achieved / peak,
                          "inputs": entry.get("source"),
-                         "note": ("achieved = FP64 operations the unit stages executed (ncu counts per emitted "
-                                  "unit on the cluster's first 8 centres) x emitted units / their "
-                                  "CUDA-event time; alg_* = the reference's work counted by the oracle on its "
+                         "note": ("achieved = warp instructions (batched) or FP64 operations (plain) the unit "
+                                  "stages executed (ncu counts per emitted unit on the cluster's first 8 "
+                                  "centres) x emitted units / their CUDA-event time; alg_* = the reference's "
+                                  "work in FP64 operations counted by the oracle on its "
                                   "control flow, which includes the full 1023-point tabulation of every "
                                   "large-grid fallback the stages skip, so alg_frac can exceed 1")},
             "cpu_baseline": {"value": cpu_v, "unit": UNIT, "cores": cores, "kind": kind,

@@ -13,7 +13,7 @@
 // instructions make them faster.  So quadratures of several primitive pairs
 // share a warp, tables are computed a point a lane, the running quadratures stay
 // packed and the products of the last ones are spread over the idle lanes.
-// 8 centres of the cluster (14,564 units): small grid 5.3 ms, large grid 8.5, blocks
+// 8 centres of the cluster (14,564 units): small grid 5.4 ms, large grid 8.5, blocks
 // 1.4; one kernel with a unit a CTA took 155.6.
 #include "ecp_stages.cuh"
 

@@ -26,7 +26,7 @@
 //     exactly the terms the reference adds to each chi[i][j];
 //   * little code in the hot loops (no unrolling, one copy of what is used
 //     twice): a kilobyte more costs the large-grid stage 1 to 9 %.
-// 50-centre cluster (90,976 units): 37.0 ms in these stages; one FP64 kernel
+// 50-centre cluster (90,976 units): 37.1 ms in these stages; one FP64 kernel
 // with a unit a CTA took 116.3.
 #include <algorithm>
 
@@ -839,10 +839,10 @@ static __device__ void t2_small(const DevJob &J, const Unit &U, const LevelTab &
 // One warp a CTA; each takes up to J.take entries of the type-1 groups, then
 // of the type-2 batches (one kind of work at a time on the whole GPU).
 // Bound by instruction latency: 56 % of the issue slots at 16 warps an SM, the
-// stalls fixed latencies (2.0 warps an issue), table rows from L2 (1.5) and
-// instruction fetch (0.4); the FP64 pipe is 6 % busy.  80 registers let 24 CTAs
+// stalls fixed latencies (1.9 warps an issue), table rows from L2 (1.4) and
+// instruction fetch (0.5); the FP64 pipe is 6 % busy.  80 registers let 24 CTAs
 // share an SM (at 96 the cluster's stages took 46.5 instead of 45.3 ms, at 64
-// 45.8, with spills).  8 centres of the cluster: 1.53 ms (2.46 with doubles and
+// 45.8, with spills).  8 centres of the cluster: 1.55 ms (2.46 with doubles and
 // per-entry set-up).
 template <bool kMixed>
 __global__ void __launch_bounds__(32, 24) k_unit_small(DevJob J) {
@@ -1421,12 +1421,12 @@ static __device__ void t2_large(const DevJob &J, const Unit &U, const LargeSmem 
 
 // The type-2 parts first (the longer ones), one at a time by the whole CTA, then
 // the failed type-1 pairs, one a warp.  Bound by instruction latency like the
-// small grid: 49 % of the issue slots at 13 warps an SM, fixed latencies 2.0
+// small grid: 48 % of the issue slots at 13 warps an SM, fixed latencies 2.0
 // warps an issue, table rows 1.5, fetch 0.4, FP64 pipe 4 %.  128 registers and the
 // tables' shared memory admit 14 to 16 warps; fewer registers spill in the walks
 // (18 warps: 48.8 against 46.5 ms on the cluster), two Bessel rows or two walk
 // entries at a time overflow the instruction cache (39.6 and 39.7 against 37.4).
-// 8 centres of the cluster: 3.25 ms.
+// 8 centres of the cluster: 3.27 ms.
 template <bool kMixed, int kWarps>
 __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps) k_unit_large(DevJob J) {
   extern __shared__ double sm[];

@@ -539,15 +539,15 @@ static PairPlan plan_of_pair(const Parsed &P, int p, bool single) {
 // 0.88; beyond the line 10,490 0.69 and 0.92, 14,421 0.76 and 0.95, 24,374 1.13 and
 // 1.33, 38,300 1.55 and 1.40; the plain path's small grid, 9,236 pairs: 1.84 and 1.78.
 // The line is below the crossing: a part a pair takes a partial sum per pair and
-// quadrature of scratch.  (The partial sums' number, and with it a unit's last bits,
-// follow the job's size.)
-constexpr long long kFewPairs = 64 * 152;  // 64 a streaming multiprocessor
+// quadrature of scratch.  (The groups and the partial sums, and with them a unit's
+// last bits, follow the job's size.)
+constexpr long long kFewPairs = 64 * 152;  // 64 for each of GB300's 152 multiprocessors
 // Up to kTwoWarpPairs the batched large grid gives an entry to two warps, which
 // halves its latency; with more the SMs are full and the two warps' different code
 // costs instruction fetches.  Unit stages with two warps and with one (ms): 19,170
 // pairs 1.17 and 1.35, 50,110 1.73 and 1.89; beyond the line 60,920 1.86 and 1.98,
 // 94,458 2.32 and 2.43, 118,395 2.78 and 2.67, 163,264 3.61 and 3.16.
-constexpr long long kTwoWarpPairs = 384 * 152;  // 384 a streaming multiprocessor
+constexpr long long kTwoWarpPairs = 384 * 152;  // 384 for each multiprocessor
 static long long primitive_pairs(const Parsed &P) {
   long long n = 0;
   for (int p = 0; p < P.nPairs; p++) n += (long long)P.nCentres * P.shK[P.pairA[p]] * P.shK[P.pairB[p]];
