@@ -49,7 +49,7 @@ static __device__ inline bool ps93_adds(int t, int n, int ws, int we) {
 
 // A group of G primitive pairs of one kind (perm[p0 ..]) on the small grid
 // (src/type1.c:63-148), by one warp; lane = (pair, quadrature).
-template <bool kZero>
+template <bool kInRange, bool kZero>
 static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem &L, double *sm, int off, int p0,
                                 int G) {
   const int lane = threadIdx.x & 31, lab = U.lab, lq = lab + 1, O = kSmallOrder, ws = U.ws, we = U.we;
@@ -107,7 +107,7 @@ static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem 
       const double r = J.xSmall[n], s = P.s, C1 = P.C1, ex = (P.z * r + s) * r, u = uL[n];
       // below the screen the exponential is 0, and so is the product where it is finite
       const bool seen = ex >= J.lnAcc1;
-      if (seen || !J.inRange) {
+      if (seen || !kInRange) {
         bessel_rows(J, lab, s * r, ent);
         double R = 1.0;
 #pragma unroll 1
@@ -138,15 +138,15 @@ static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem 
         const int n = __ldg(J.s93 + t0 + D.part);
         if (n >= ws && n < we) {
           const double *e = tab + ((t0 + D.part - s0) * G + (qd & 255)) * TS;
-          if (e[2 * lq] != 0.0 || !J.inRange) v = J.wSmall[n] * (e[oW] * e[oK] * e[2 * lq]);
-        } else if (!J.inRange) {
+          if (e[2 * lq] != 0.0 || !kInRange) v = J.wSmall[n] * (e[oW] * e[oK] * e[2 * lq]);
+        } else if (!kInRange) {
           v = J.wSmall[n] * (((const PairRec *)(rec + (qd & 255) * kPairWords))->C1 * 0.0);
         }
       }
 #pragma unroll 1
       for (int j = 0; j < D.P && t0 + j < s1; j++) {
         const int t = t0 + j, n = c93_slot[t];
-        if ((n >= ws && n < we) || (!J.inRange && ps93_adds(t, n, ws, we)))
+        if ((n >= ws && n < we) || (!kInRange && ps93_adds(t, n, ws, we)))
           T += __shfl_sync(0xffffffffu, v, (src + j) & 31);
         cnt += (t & 1) ? n >= ws : n <= we;
         if (t > 2 && !(t & 1)) {  // the reference's order: pair by pair
@@ -184,6 +184,7 @@ static __device__ void x1_small(const DevJob &J, const Unit &U, const SmallSmem 
 }
 
 // A batch of 32 type-2 small-grid quadratures, one per lane (src/type2.c:337-387).
+template <bool kInRange>
 static __device__ void x2_small(const DevJob &J, const Unit &U, int q0) {
   const int qx = q0 + (threadIdx.x & 31), O = kSmallOrder;
   if (qx >= U.nItems) return;
@@ -198,7 +199,7 @@ static __device__ void x2_small(const DevJob &J, const Unit &U, int q0) {
   for (int t = 0;; t++) {
     const int n = c93_slot[t];
     // (F is zero outside the windows)
-    if ((n >= U.ws && n < U.we) || (!J.inRange && ps93_adds(t, n, U.ws, U.we)))
+    if ((n >= U.ws && n < U.we) || (!kInRange && ps93_adds(t, n, U.ws, U.we)))
       T += J.wSmall[n] * (__ldg(Fa + n * nF) * __ldg(Fb + n * nF) * __ldg(Ut + (size_t)n * LE * nk));
     cnt += (t & 1) ? n >= U.ws : n <= U.we;
     if (t > 2 && !(t & 1)) {
@@ -222,6 +223,8 @@ static __device__ void x2_small(const DevJob &J, const Unit &U, int q0) {
   atomicOr((unsigned *)(U.scr + U.L.mask) + (qx >> 5), 1u << (qx & 31));
 }
 
+// kInRange: no product leaves FP64's range, so what has a factor 0 is 0 (DevJob::inRange).
+template <bool kInRange>
 __global__ void __launch_bounds__(32, 16) k_exact_small(DevJob J) {
   extern __shared__ double sm[];
   const SmallSmem L = small_layout(J.maxLBS, 0, J.gcap);
@@ -233,12 +236,12 @@ __global__ void __launch_bounds__(32, 16) k_exact_small(DevJob J) {
     const int2 it = small_entry(J, i, n0, n1);
     const Unit &U = unit_get(J, it.x);
     if (i >= n1) {
-      x2_small(J, U, it.y);
+      x2_small<kInRange>(J, U, it.y);
       continue;
     }
     const int p0 = it.y & 1023, G = (it.y >> 10) & 63;
-    if (it.y >> 16 == kPairZero) x1_small<true>(J, U, L, sm, it.x, p0, G);
-    else x1_small<false>(J, U, L, sm, it.x, p0, G);
+    if (it.y >> 16 == kPairZero) x1_small<kInRange, true>(J, U, L, sm, it.x, p0, G);
+    else x1_small<kInRange, false>(J, U, L, sm, it.x, p0, G);
   }
 }
 
@@ -728,7 +731,8 @@ void exact_prepare() {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || attr[dev]) return;
-  for (const void *k : {(const void *)k_exact_small, (const void *)k_exact_large, (const void *)k_exact_link}) {
+  for (const void *k : {(const void *)k_exact_small<true>, (const void *)k_exact_small<false>,
+                        (const void *)k_exact_large, (const void *)k_exact_link}) {
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   }
@@ -754,7 +758,7 @@ int launch_exact_pipeline(const DevJob &J, cudaStream_t st, cudaEvent_t u0, cuda
     DevJob K = C;
     k_unit_plan<true><<<(units + 3) / 4, kPlanThreads, 0, st>>>(K);
     K.take = takeSmall;
-    k_exact_small<<<gSmall, 32, sSmall, st>>>(K);
+    (J.inRange ? k_exact_small<true> : k_exact_small<false>)<<<gSmall, 32, sSmall, st>>>(K);
     K.take = takeLarge;
     k_exact_large<<<gLarge, 32, sLarge, st>>>(K);
     k_exact_link<<<dim3(units, link_parts(units)), link_threads(sLink), sLink, st>>>(K);

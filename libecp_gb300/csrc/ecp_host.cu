@@ -306,7 +306,7 @@ struct Engine {
   // The tables of a job; the batched path's fixed-point rows from its first job on.
   const DevTables *get_tables(const Parsed &P, int mode) {
     DevTables *t = plain_tables(table_key(P));
-    if (!t || plain_stages(P, mode) || t->besXA.p) return t;
+    if (!t || t->besXA.p || plain_stages(P, mode)) return t;
     bessel_fixed(t->host);
     if (!t->besX.upload(t->host.besselX, stream) || !t->besXA.upload(t->host.besselXA, stream)) {
       t->besXA.release(nullptr);
@@ -559,12 +559,12 @@ static long long primitive_pairs(const Parsed &P) {
 // 9e-12 (small grid) or 9e-14 of an interval of 9/sqrt(za + zb) (large grid; with
 // more than 1023 points its first abscissa is -1, r = 0) to a distance plus that interval.
 static double product_bits(const Parsed &P) {
-  double zMin = INFINITY, zMax = 0.0, c = -INFINITY, u = -INFINITY, far = 0.0;
+  double zMin = INFINITY, zMax = 0.0, dMax = 0.0, u = -INFINITY, far = 0.0;
   for (double z : P.primA) {
     zMin = std::min(zMin, z);
     zMax = std::max(zMax, z);
   }
-  for (double d : P.primD) c = std::max(c, std::log2(std::fabs(d)));
+  for (double d : P.primD) dMax = std::max(dMax, std::fabs(d));
   for (double x : P.geom) far = std::max(far, std::fabs(x));
   const double top = std::log2(std::max(64.0, 4.0 * far + 9.0 / std::sqrt(2.0 * zMin)));
   const double low = P.largeGridOrder < 2047 ? std::max(37.0, 44.0 - std::log2(4.5 / std::sqrt(2.0 * zMax))) : INFINITY;
@@ -573,7 +573,7 @@ static double product_bits(const Parsed &P) {
     u = std::max(u, std::log2(std::fabs(P.termD[t])) + (n > 0.0 ? n * top : n < 0.0 ? -n * low : 0.0));
   }
   // (r^l, l <= 8, the interval's length and the map's weight; sums)
-  return 2.0 * (c + P.deriv * std::max(0.0, std::log2(zMax))) + u + std::log2(1.0 + P.termN.size()) + 11.0 * top + 64.0;
+  return 2.0 * (std::log2(dMax) + P.deriv * std::max(0.0, std::log2(zMax))) + u + std::log2(1.0 + P.termN.size()) + 11.0 * top + 64.0;
 }
 
 // Whether a batched job runs the plain path's stages.  The batched path's
@@ -708,15 +708,13 @@ static JobBytes job_bytes(const Parsed &P, int mode, const JobPlan &plan, size_t
            screen ? 4 * (nu + 1) : 0, screen ? 4 * (nu / 256 + 2) : 0, screen ? 4 * (chunks + 1) : 0, plan.bytes + 16}};
 }
 
-static bool single_pair_parts(const Parsed &P, int mode) {
-  return plain_stages(P, mode) || primitive_pairs(P) <= kFewPairs;
-}
+static bool single_pair_parts(const Parsed &P, bool plain) { return plain || primitive_pairs(P) <= kFewPairs; }
 
 bool job_device_bytes(const Parsed &P, int mode, size_t budget, JobBytes *need, size_t *scratchCap) {
   JobPlan plan;
   std::vector<int> orders, chunkUnits, ctr;
   std::vector<long long> offs;
-  const bool single = single_pair_parts(P, mode);
+  const bool single = single_pair_parts(P, plain_stages(P, mode));
   size_t stages;
   // (a smaller scratch means more chunks, whose list takes a little more of the inputs)
   for (size_t cap = kScratchCap;;) {
@@ -751,7 +749,7 @@ int stage_job(const Parsed &P, const DevTables *T, JobBuffers &B, DevJob &J, int
   const long long np = primitive_pairs(P);
   J.few = np <= kFewPairs;
   J.twoWarps = np <= kTwoWarpPairs;
-  J.single = single_pair_parts(P, mode);
+  J.single = single_pair_parts(P, J.plain);
   J.nAtoms = P.nAtoms; J.nShells = P.nShells; J.nPrims = P.nPrims; J.nCentres = P.nCentres;
   J.nPairs = P.nPairs; J.dim = P.dim;
   J.maxLECP = h.maxLECP; J.maxLBS = h.maxLBS; J.maxLambda = h.maxLambda; J.nk = h.nk; J.nF = h.nF;
